@@ -697,6 +697,13 @@ static void check_same_extent(std::vector<APR*>& aprs, const std::vector<int>& d
     }
 }
 
+static torch::Tensor image_workspace(std::vector<APR*>& aprs, const std::vector<int>& dl, const torch::Tensor& like) {
+    int64_t bytes = 256;
+    for (size_t i = 0; i < aprs.size(); ++i)
+        bytes = std::max<int64_t>(bytes, aprnet_image_workspace_bytes(aprs[i]->handle(like), dl[i], dtype_id(like), (int) like.size(1)));
+    return torch::empty({bytes}, like.options().dtype(torch::kUInt8));
+}
+
 torch::Tensor reconstruct_forward(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor level_delta) {
     CHECK_INPUT(input);
     check_batch(aprs, input);
@@ -706,9 +713,10 @@ torch::Tensor reconstruct_forward(std::vector<APR*>& aprs, torch::Tensor input, 
     const auto e = image_extent(aprs, dl, input);
     check_same_extent(aprs, dl, input, e);
     auto output = torch::empty({input.size(0), input.size(1), e[0], e[1], e[2]}, input.options());
+    auto ws = image_workspace(aprs, dl, input);
     for (int64_t b = 0; b < input.size(0); ++b)
-        check(aprnet_reconstruct_forward(aprs[b]->handle(input), dl[b], dtype_id(input), (int) input.size(1), row(input, b), input.size(2),
-                                         row(output, b), stream_of(input)), "reconstruct_forward");
+        check(aprnet_cells_to_image(aprs[b]->handle(input), dl[b], dtype_id(input), (int) input.size(1), row(input, b), input.size(2),
+                                    row(output, b), 0, ws.data_ptr(), stream_of(input)), "reconstruct_forward");
     return output;
 }
 
@@ -721,9 +729,10 @@ torch::Tensor reconstruct_backward(std::vector<APR*>& aprs, torch::Tensor grad_o
     for (size_t i = 0; i < aprs.size(); ++i) { check_level_delta(*aprs[i], dl[i]); max_size = std::max(max_size, aprs[i]->number_parts(dl[i])); }
     check_same_extent(aprs, dl, grad_output, {grad_output.size(2), grad_output.size(3), grad_output.size(4)});
     auto grad_input = torch::empty({grad_output.size(0), grad_output.size(1), max_size}, grad_output.options());
+    auto ws = image_workspace(aprs, dl, grad_output);
     for (int64_t b = 0; b < grad_output.size(0); ++b) {
-        check(aprnet_reconstruct_backward(aprs[b]->handle(grad_output), dl[b], dtype_id(grad_output), (int) grad_output.size(1), row(grad_output, b),
-                                          row(grad_input, b), max_size, stream_of(grad_output)), "reconstruct_backward");
+        check(aprnet_image_to_cells(aprs[b]->handle(grad_output), dl[b], dtype_id(grad_output), (int) grad_output.size(1), row(grad_output, b),
+                                    row(grad_input, b), max_size, 0, ws.data_ptr(), stream_of(grad_output)), "reconstruct_backward");
         zero_padding(grad_input, b, aprs[b]->number_parts(dl[b]));
     }
     return grad_input;
@@ -738,9 +747,10 @@ torch::Tensor sample_particles_forward(std::vector<APR*>& aprs, torch::Tensor in
     for (size_t i = 0; i < aprs.size(); ++i) { check_level_delta(*aprs[i], dl[i]); max_size = std::max(max_size, aprs[i]->number_parts(dl[i])); }
     check_same_extent(aprs, dl, input, {input.size(2), input.size(3), input.size(4)});
     auto output = torch::empty({input.size(0), input.size(1), max_size}, input.options());
+    auto ws = image_workspace(aprs, dl, input);
     for (int64_t b = 0; b < input.size(0); ++b) {
-        check(aprnet_sample_particles_forward(aprs[b]->handle(input), dl[b], dtype_id(input), (int) input.size(1), row(input, b),
-                                              row(output, b), max_size, stream_of(input)), "sample_particles_forward");
+        check(aprnet_image_to_cells(aprs[b]->handle(input), dl[b], dtype_id(input), (int) input.size(1), row(input, b),
+                                    row(output, b), max_size, 1, ws.data_ptr(), stream_of(input)), "sample_particles_forward");
         zero_padding(output, b, aprs[b]->number_parts(dl[b]));
     }
     return output;
@@ -755,10 +765,10 @@ torch::Tensor sample_particles_backward(std::vector<APR*>& aprs, torch::Tensor g
     const auto e = image_extent(aprs, dl, grad_output);
     check_same_extent(aprs, dl, grad_output, e);
     auto grad_input = torch::empty({grad_output.size(0), grad_output.size(1), e[0], e[1], e[2]}, grad_output.options());
+    auto ws = image_workspace(aprs, dl, grad_output);
     for (int64_t b = 0; b < grad_output.size(0); ++b)
-        check(aprnet_sample_particles_backward(aprs[b]->handle(grad_output), dl[b], dtype_id(grad_output), (int) grad_output.size(1),
-                                               row(grad_output, b), grad_output.size(2), row(grad_input, b), stream_of(grad_output)),
-              "sample_particles_backward");
+        check(aprnet_cells_to_image(aprs[b]->handle(grad_output), dl[b], dtype_id(grad_output), (int) grad_output.size(1), row(grad_output, b),
+                                    grad_output.size(2), row(grad_input, b), 1, ws.data_ptr(), stream_of(grad_output)), "sample_particles_backward");
     return grad_input;
 }
 
