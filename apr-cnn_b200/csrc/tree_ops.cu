@@ -8,6 +8,7 @@
 // Arithmetic follows pyapr/aprnet/src/helpers.hpp:156-350 (tree mean and its adjoint),
 // pyapr/aprnet/src/maxpool.hpp:70-230 and pyapr/aprnet/src/upsample.hpp:70-236.
 #include "apr_device.cuh"
+#include <algorithm>
 
 namespace {
 
@@ -19,48 +20,69 @@ template<typename T> struct DT;
 template<> struct DT<float> { static constexpr int id = APRNET_F32; };
 template<> struct DT<double> { static constexpr int id = APRNET_F64; };
 
-// parent level lp: tree[t] = scale[t] * sum(children).  All child values of the block's channels are
-// requested before any is used (CH_PER_BLOCK x 8 independent loads in flight per thread).
-template<typename T>
-__global__ void __launch_bounds__(TPB) tree_mean_level_kernel(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree,
-                                       ll tb, ll te, const T* __restrict__ in, ll ld_in, T* __restrict__ tree,
-                                       ll ld_tree, int C, ll up_off, int use_up) {
-    const ll t = tb + (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= te) return;
-    // resolve the eight child slots once: pointer to the child's value in channel c0 and the channel stride
-    const int c0 = blockIdx.y * CH_PER_BLOCK;
-    const T* src[8];
-    unsigned coded = 0;                 // slots whose child is a tree node (summed after the particles)
-    const unsigned in_tree = use_up ? 0u : 0xffu;      // coded children live in the tree scratch unless they are upgraded nodes
+// One tree level: node t = scale[t] * sum(children) (MAX: their maximum).  A thread owns a node and CH channels; the
+// block's channel group is the fast grid axis, so that the groups of the same nodes run together and find the 36-byte
+// table entries of a node in L2.  All CH x 8 child values are requested before any is used.
+template<typename T, int CH, bool MAX>
+__device__ __forceinline__ void tree_node(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree, ll t,
+                                          const T* __restrict__ in, ll ld_in, T* tree, ll ld_tree, int c0, int nch, ll up_off, int use_up) {
+    int32_t v[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) v[s] = __ldg(child + (ll) s * n_tree + t);
+    const T f = MAX ? T(1) : (T) __ldg(scale + t);
+    const T* xin = in + (ll) c0 * ld_in;
+    const T* xtree = use_up ? xin + up_off : tree + (ll) c0 * ld_tree;     // coded children: upgraded nodes in the features, else the tree scratch
+    const ll ld_coded = use_up ? ld_in : ld_tree;
+    T vals[CH][8];
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
-        const int32_t v = child[(ll) s * n_tree + t];
-        src[s] = nullptr;
-        if (v >= 0) src[s] = in + (ll) c0 * ld_in + v;
-        else if (v != APRNET_NONE) {
-            coded |= 1u << s;
-            src[s] = use_up ? in + (ll) c0 * ld_in + aprnet_dec_tree(v) + up_off : tree + (ll) c0 * ld_tree + aprnet_dec_tree(v);
-        }
-    }
-    const T f = (T) scale[t];
-    const int nch = min(CH_PER_BLOCK, C - c0);
-    T vals[CH_PER_BLOCK][8];
+        const T* src = v[s] >= 0 ? xin + v[s] : xtree + aprnet_dec_tree(v[s]);
+        const ll ld = v[s] >= 0 ? ld_in : ld_coded;
 #pragma unroll
-    for (int k = 0; k < CH_PER_BLOCK; ++k) {
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            vals[k][s] = (src[s] && k < nch) ? *src[s] : T(0);
-            src[s] += (coded & in_tree) >> s & 1 ? ld_tree : ld_in;
-        }
+        for (int k = 0; k < CH; ++k) vals[k][s] = (v[s] != APRNET_NONE && k < nch) ? src[k * ld] : T(0);
     }
     T* dst = tree + (ll) c0 * ld_tree + t;
 #pragma unroll
-    for (int k = 0; k < CH_PER_BLOCK; ++k) {
+    for (int k = 0; k < CH; ++k) {
         if (k >= nch) break;
-        T s_part = 0, s_tree = 0;       // particles first, then tree children (fixed order)
+        if (MAX) {
+            bool seen = false;
+            T best = 0;
 #pragma unroll
-        for (int s = 0; s < 8; ++s) { if (coded >> s & 1) s_tree += vals[k][s]; else s_part += vals[k][s]; }
-        dst[(ll) k * ld_tree] = f * (s_part + s_tree);
+            for (int s = 0; s < 8; ++s)
+                if (v[s] != APRNET_NONE && (!seen || vals[k][s] > best)) { best = vals[k][s]; seen = true; }
+            dst[(ll) k * ld_tree] = best;
+        } else {
+            T s_part = 0, s_tree = 0;       // particles first, then tree children (fixed order)
+#pragma unroll
+            for (int s = 0; s < 8; ++s) { if (v[s] < 0) s_tree += vals[k][s]; else s_part += vals[k][s]; }
+            dst[(ll) k * ld_tree] = f * (s_part + s_tree);
+        }
+    }
+}
+
+template<typename T, int CH, bool MAX>
+__global__ void __launch_bounds__(TPB) tree_level_kernel(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree,
+                                                         ll tb, ll te, const T* __restrict__ in, ll ld_in, T* tree,
+                                                         ll ld_tree, int C, ll up_off, int use_up) {
+    const ll t = tb + (ll) blockIdx.y * TPB + threadIdx.x;
+    const int c0 = blockIdx.x * CH;
+    if (t < te) tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, use_up);
+}
+
+// The coarse end of the tree in one launch: a block owns CH channels and walks the levels [0, n) of `lv` (fine to coarse), whose
+// nodes are few; what it reads of a finer level it has written itself before the barrier.
+struct LevelList { int n; ll begin[APRNET_MAX_LEVELS], end[APRNET_MAX_LEVELS]; int use_up[APRNET_MAX_LEVELS]; };
+constexpr int COARSE_TPB = 512;
+
+template<typename T, int CH, bool MAX>
+__global__ void __launch_bounds__(COARSE_TPB) tree_coarse_kernel(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree,
+                                                                 LevelList lv, const T* __restrict__ in, ll ld_in, T* tree, ll ld_tree, int C, ll up_off) {
+    const int c0 = blockIdx.x * CH;
+    for (int i = 0; i < lv.n; ++i) {
+        for (ll t = lv.begin[i] + threadIdx.x; t < lv.end[i]; t += COARSE_TPB)
+            tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
+        __syncthreads();
     }
 }
 
@@ -71,11 +93,8 @@ __global__ void __launch_bounds__(TPB) tree_mean_level_kernel(const int32_t* __r
 // gradient half at a time and ran at half this speed.  dst and gtree may be the same array (node levels): a level only
 // reads the level above it.
 template<typename T>
-__global__ void __launch_bounds__(TPB) tree_mean_backward_children_kernel(const int32_t* __restrict__ parent, const float* __restrict__ scale,
-                                                                          ll ub, ll ue, T* dst, ll ld_dst, const T* gtree, ll ld_tree, int C) {
-    const ll u = ub + (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= ue) return;
-    const int c0 = blockIdx.y * CH_PER_BLOCK;
+__device__ __forceinline__ void tree_backward_child(const int32_t* __restrict__ parent, const float* __restrict__ scale, ll u, T* dst, ll ld_dst,
+                                                    const T* gtree, ll ld_tree, int c0, int C) {
     T old[CH_PER_BLOCK];
 #pragma unroll
     for (int k = 0; k < CH_PER_BLOCK; ++k) old[k] = dst[(ll) min(c0 + k, C - 1) * ld_dst + u];        // independent of the parent
@@ -91,27 +110,20 @@ __global__ void __launch_bounds__(TPB) tree_mean_backward_children_kernel(const 
 }
 
 template<typename T>
-__global__ void tree_max_level_kernel(const int32_t* __restrict__ child, ll n_tree, ll tb, ll te,
-                                      const T* __restrict__ in, ll ld_in, T* __restrict__ tree, ll ld_tree, int C) {
-    const ll t = tb + (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= te) return;
-    int32_t ch[8];
-#pragma unroll
-    for (int s = 0; s < 8; ++s) ch[s] = child[(ll) s * n_tree + t];
-    const int c0 = blockIdx.y * CH_PER_BLOCK, c1 = min(C, c0 + CH_PER_BLOCK);
-    for (int c = c0; c < c1; ++c) {
-        const T* x = in + (ll) c * ld_in;
-        const T* tr = tree + (ll) c * ld_tree;
-        bool seen = false;
-        T best = 0;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            const int32_t v = ch[s];
-            if (v == APRNET_NONE) continue;
-            const T val = v >= 0 ? x[v] : tr[aprnet_dec_tree(v)];
-            if (!seen || val > best) { best = val; seen = true; }
-        }
-        tree[(ll) c * ld_tree + t] = best;
+__global__ void __launch_bounds__(TPB) tree_mean_backward_children_kernel(const int32_t* __restrict__ parent, const float* __restrict__ scale,
+                                                                          ll ub, ll ue, T* dst, ll ld_dst, const T* gtree, ll ld_tree, int C) {
+    const ll u = ub + (ll) blockIdx.x * blockDim.x + threadIdx.x;
+    if (u < ue) tree_backward_child<T>(parent, scale, u, dst, ld_dst, gtree, ld_tree, blockIdx.y * CH_PER_BLOCK, C);
+}
+
+// the coarse tree levels of `lv` (coarse to fine) in one launch, a block per channel group (see tree_coarse_kernel)
+template<typename T>
+__global__ void __launch_bounds__(COARSE_TPB) tree_mean_backward_coarse_kernel(const int32_t* __restrict__ parent, const float* __restrict__ scale,
+                                                                               LevelList lv, T* gtree, ll ld_tree, int C) {
+    for (int i = 0; i < lv.n; ++i) {
+        for (ll u = lv.begin[i] + threadIdx.x; u < lv.end[i]; u += COARSE_TPB)
+            tree_backward_child<T>(parent, scale, u, gtree, ld_tree, gtree, ld_tree, blockIdx.x * CH_PER_BLOCK, C);
+        __syncthreads();
     }
 }
 
@@ -203,18 +215,39 @@ int copy_rows(T* dst, ll ld_dst, const T* src, ll ld_src, ll count, int C, cudaS
     return APRNET_OK;
 }
 
-template<typename T>
-int fill_tree_mean_fwd(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree, ll ld_tree, cudaStream_t st) {
+// Fills the tree bottom-up.  A level of more than COARSE_NODES nodes is a launch of its own; the levels above the first one
+// with fewer (the coarser, the fewer) share one launch: a level costs about 2 us as a launch and about 1.5 us plus 1 us per
+// COARSE_TPB nodes inside the shared one.
+constexpr ll COARSE_NODES = 1024;
+
+template<typename T, bool MAX>
+int fill_tree(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree, ll ld_tree, const char* pname, cudaStream_t st) {
+    constexpr int CH = 4;
     const LevelMeta& m = a->meta;
     const int cml = a->cml(dl);
     const ll up = (dl > 0) ? a->tree_offset(cml) : 0;
+    const unsigned gx = (unsigned) aprnet_ceil_div(C, CH);
+    LevelList coarse;
+    coarse.n = 0;
     for (int lp = cml - 1; lp >= m.level_min - 1; --lp) {
         const ll tb = m.tlvl_begin[lp], te = m.tlvl_begin[lp + 1];
         if (te <= tb) continue;
-        { AprnetProfScope _prof("tree_mean_fwd", st);
-        tree_mean_level_kernel<T><<<node_grid(te - tb, C), TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, tb, te, in,
-                                                                          ld_in, tree, ld_tree, C, up, (dl > 0 && lp + 1 == cml) ? 1 : 0);
+        const int use_up = (dl > 0 && lp + 1 == cml) ? 1 : 0;
+        if (te - tb <= COARSE_NODES || coarse.n > 0) {
+            coarse.begin[coarse.n] = tb; coarse.end[coarse.n] = te; coarse.use_up[coarse.n] = use_up;
+            ++coarse.n;
+            continue;
         }
+        for (ll b = tb; b < te; b += 65535ll * TPB) {              // grid.y holds 65535 blocks
+            AprnetProfScope _prof(pname, st);
+            const ll e = std::min(te, b + 65535ll * TPB);
+            tree_level_kernel<T, CH, MAX><<<dim3(gx, (unsigned) aprnet_ceil_div(e - b, TPB)), TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, b, e, in, ld_in,
+                                                                                                          tree, ld_tree, C, up, use_up);
+        }
+    }
+    if (coarse.n > 0) {
+        AprnetProfScope _prof(pname, st);
+        tree_coarse_kernel<T, CH, MAX><<<gx, COARSE_TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, coarse, in, ld_in, tree, ld_tree, C, up);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -228,7 +261,16 @@ int fill_tree_mean_bwd(const aprnet_apr* a, int dl, int C, T* gin, ll ld_in, T* 
     const int32_t* loc_parent = aprnet_loc_parent_table(a, dl, st);
     if (!node_parent || !loc_parent) return APRNET_ERR_CUDA;
     // tree nodes, coarse to fine: level l receives from level l - 1, whose gradient is complete by then
-    for (int l = m.level_min; l <= cml - 1; ++l) {
+    LevelList coarse;
+    coarse.n = 0;
+    int l = m.level_min;
+    for (; l <= cml - 1 && m.tlvl_begin[l + 1] - m.tlvl_begin[l] <= COARSE_NODES; ++l)
+        if (m.tlvl_begin[l + 1] > m.tlvl_begin[l]) { coarse.begin[coarse.n] = m.tlvl_begin[l]; coarse.end[coarse.n] = m.tlvl_begin[l + 1]; ++coarse.n; }
+    if (coarse.n > 0) {
+        AprnetProfScope _prof("tree_mean_bwd", st);
+        tree_mean_backward_coarse_kernel<T><<<(unsigned) aprnet_ceil_div(C, CH_PER_BLOCK), COARSE_TPB, 0, st>>>(node_parent, a->tree_scale, coarse, gtree, ld_tree, C);
+    }
+    for (; l <= cml - 1; ++l) {
         const ll ub = m.tlvl_begin[l], ue = m.tlvl_begin[l + 1];
         if (ue <= ub) continue;
         AprnetProfScope _prof("tree_mean_bwd", st);
@@ -239,20 +281,6 @@ int fill_tree_mean_bwd(const aprnet_apr* a, int dl, int C, T* gin, ll ld_in, T* 
     if (n > 0) {
         AprnetProfScope _prof("tree_mean_bwd", st);
         tree_mean_backward_children_kernel<T><<<node_grid(n, C), TPB, 0, st>>>(loc_parent, a->tree_scale, 0, n, gin, ld_in, gtree, ld_tree, C);
-    }
-    APRNET_LAUNCH_CHECK();
-    return APRNET_OK;
-}
-
-template<typename T>
-int fill_tree_max_impl(const aprnet_apr* a, int C, const T* in, ll ld_in, T* tree, ll ld_tree, cudaStream_t st) {
-    const LevelMeta& m = a->meta;
-    for (int lp = m.level_max - 1; lp >= m.level_min - 1; --lp) {
-        const ll tb = m.tlvl_begin[lp], te = m.tlvl_begin[lp + 1];
-        if (te <= tb) continue;
-        { AprnetProfScope _prof("tree_max", st);
-        tree_max_level_kernel<T><<<node_grid(te - tb, C), TPB, 0, st>>>(a->child, a->n_tree, tb, te, in, ld_in, tree, ld_tree, C);
-        }
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -324,8 +352,8 @@ extern "C" int aprnet_fill_tree_mean_forward(const aprnet_apr* a, int dl, int dt
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), "leading dimension too small");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, fill_tree_mean_fwd<float>(a, dl, C, (const float*) in, ld_in, (float*) tree, ld_tree, st),
-             fill_tree_mean_fwd<double>(a, dl, C, (const double*) in, ld_in, (double*) tree, ld_tree, st));
+    DISPATCH(dtype, (fill_tree<float, false>(a, dl, C, (const float*) in, ld_in, (float*) tree, ld_tree, "tree_mean_fwd", st)),
+             (fill_tree<double, false>(a, dl, C, (const double*) in, ld_in, (double*) tree, ld_tree, "tree_mean_fwd", st)));
 }
 
 extern "C" int aprnet_fill_tree_mean_full(const aprnet_apr* a, int dtype, int C, const void* in, int64_t ld_in, void* tree,
@@ -349,8 +377,8 @@ extern "C" int aprnet_fill_tree_max(const aprnet_apr* a, int dtype, int C, const
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->n_particles && ld_tree >= a->n_tree, "leading dimension too small");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, fill_tree_max_impl<float>(a, C, (const float*) in, ld_in, (float*) tree, ld_tree, st),
-             fill_tree_max_impl<double>(a, C, (const double*) in, ld_in, (double*) tree, ld_tree, st));
+    DISPATCH(dtype, (fill_tree<float, true>(a, 0, C, (const float*) in, ld_in, (float*) tree, ld_tree, "tree_max", st)),
+             (fill_tree<double, true>(a, 0, C, (const double*) in, ld_in, (double*) tree, ld_tree, "tree_max", st)));
 }
 
 extern "C" int aprnet_maxpool_forward(const aprnet_apr* a, int dl, int dtype, int C, const void* in, int64_t ld_in,
