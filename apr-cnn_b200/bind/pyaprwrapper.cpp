@@ -183,53 +183,141 @@ inline void check_level_delta(const APR& apr, int dl) {
 inline size_t esize(const torch::Tensor& t) { return t.element_size(); }
 inline char* row(const torch::Tensor& t, int64_t b) { return (char*) t.data_ptr() + b * t.stride(0) * (int64_t) esize(t); }
 
-// zero the padding behind the valid entries of batch item b
-inline void zero_padding(torch::Tensor& t, int64_t b, int64_t valid) {
-    if (valid < t.size(2)) t.select(0, b).narrow(1, valid, t.size(2) - valid).zero_();
+// entries behind the valid ones of every batch item: zero, or the channel's bias
+inline void fill_padding(torch::Tensor& t, const std::vector<int64_t>& valid, const torch::Tensor& bias = torch::Tensor()) {
+    bool any = false;
+    for (int64_t v : valid) any = any || v < t.size(2);
+    if (any)
+        check(aprnet_fill_padding(dtype_id(t), (int) t.size(0), (int) t.size(1), t.size(2), valid.data(), bias.defined() ? bias.data_ptr() : nullptr,
+                                  t.data_ptr(), stream_of(t)), "fill_padding");
+}
+
+inline std::vector<int64_t> valid_of(const std::vector<APR*>& aprs, const std::vector<int>& dl, int step = 0) {
+    std::vector<int64_t> n(aprs.size());
+    for (size_t i = 0; i < aprs.size(); ++i) n[i] = aprs[i]->number_parts(dl[i] + step);
+    return n;
 }
 
 // ---- 3x3x3 convolution ------------------------------------------------------------------------
+// What every call needs of its batch: handles, valid entries, tree scratch, checked against the tensor.
+struct Batch {
+    std::vector<int> dl;
+    std::vector<aprnet_apr*> h;
+    std::vector<int64_t> n;
+    int64_t max_tree = 1;
+    Batch(std::vector<APR*>& aprs, const torch::Tensor& like, const torch::Tensor& level_delta) {
+        check_batch(aprs, like);
+        dl = read_level_delta(level_delta, aprs.size());
+        for (size_t i = 0; i < aprs.size(); ++i) {
+            check_level_delta(*aprs[i], dl[i]);
+            h.push_back(aprs[i]->handle(like));
+            n.push_back(aprs[i]->number_parts(dl[i]));
+            TORCH_CHECK(n.back() <= like.size(2), "input has fewer particles than the APR at this level delta");
+            max_tree = std::max<int64_t>(max_tree, aprnet_tree_size(h.back(), dl[i]));
+        }
+    }
+    template<typename F> int64_t most_bytes(F f) const {
+        int64_t b = 256;
+        for (size_t i = 0; i < h.size(); ++i) b = std::max<int64_t>(b, f(h[i], dl[i]));
+        return b;
+    }
+};
+
+static void check_conv333(const torch::Tensor& input, const torch::Tensor& weights) {
+    TORCH_CHECK(weights.dim() == 6 && weights.size(3) == 3 && weights.size(4) == 3 && weights.size(5) == 3, "weights must be (levels, Cout, Cin, 3, 3, 3)");
+    TORCH_CHECK(input.dim() == 3 && input.size(1) == weights.size(2), "input tensor shape does not match weights tensor");
+    TORCH_CHECK(input.scalar_type() == weights.scalar_type(), "input and weights must have the same dtype");
+}
+
+inline torch::Tensor bytes_like(int64_t bytes, const torch::Tensor& like) { return torch::empty({bytes}, like.options().dtype(torch::kUInt8)); }
+inline const float* opt_bias(const c10::optional<torch::Tensor>& bias, int64_t cout) {
+    if (!bias.has_value() || !bias->defined()) return nullptr;
+    TORCH_CHECK(bias->is_cuda() && bias->is_contiguous() && bias->numel() == cout && bias->scalar_type() == torch::kFloat32, "bias must be (Cout) float32 on the device");
+    return bias->data_ptr<float>();
+}
+
+// float32: {output, tree, rows} with the parts that are wanted kept per batch item (the others are one item's scratch)
+static std::vector<torch::Tensor> conv333_forward_rows(std::vector<APR*>& aprs, const torch::Tensor& input, const torch::Tensor& weights, const torch::Tensor& level_delta,
+                                                       int mode, bool keep_tree, bool keep_rows, const torch::Tensor& given_tree = torch::Tensor(),
+                                                       const c10::optional<torch::Tensor>& bias = c10::nullopt) {
+    const Batch B(aprs, input, level_delta);
+    const int cin = (int) input.size(1), cout = (int) weights.size(1), slots = (int) weights.size(0);
+    const int64_t n = input.size(2), nb = input.size(0);
+    const float* bp = opt_bias(bias, cout);
+    auto output = torch::empty({nb, cout, n}, input.options());
+    auto tree = given_tree.defined() ? given_tree : torch::empty({keep_tree ? nb : 1, cin, B.max_tree}, input.options());
+    const int64_t bytes = B.most_bytes([&](aprnet_apr* h, int dl) { return aprnet_conv333_rows_forward_workspace_bytes(h, dl, mode, cin, cout, slots); });
+    auto ws = torch::empty({keep_rows ? nb : 1, (bytes + 255) / 256 * 256}, input.options().dtype(torch::kUInt8));
+    for (int64_t b = 0; b < nb; ++b)
+        check(aprnet_conv333_rows_forward(B.h[b], B.dl[b], mode, cin, cout, slots, (const float*) row(input, b), n, weights.data_ptr<float>(), bp,
+                                          (float*) row(output, b), n, (float*) row(tree, given_tree.defined() || keep_tree ? b : 0), tree.size(2), given_tree.defined() ? 1 : 0,
+                                          row(ws, keep_rows ? b : 0), stream_of(input)), mode == APRNET_PREC_BF16 ? "conv333_forward (tensor cores)" : "conv333_forward");
+    fill_padding(output, B.n, bp ? *bias : torch::Tensor());
+    return {output, tree, ws};
+}
+
+// float32 backward from the packed rows (B, bytes): {grad_input or undefined, grad_weights, grad_tree}
+static std::vector<torch::Tensor> conv333_backward_rows(std::vector<APR*>& aprs, const torch::Tensor& rows, const torch::Tensor& weights, const torch::Tensor& grad_output,
+                                                        const torch::Tensor& level_delta, int mode, bool need_grad_input, bool fold_tree, int64_t ld_tree = 0) {
+    const Batch B(aprs, grad_output, level_delta);
+    TORCH_CHECK(grad_output.size(1) == weights.size(1) && grad_output.scalar_type() == torch::kFloat32, "grad_output shape does not match");
+    const int cin = (int) weights.size(2), cout = (int) weights.size(1), slots = (int) weights.size(0);
+    const int64_t n = grad_output.size(2), nb = grad_output.size(0);
+    TORCH_CHECK(rows.dim() == 2 && rows.size(0) == nb && rows.scalar_type() == torch::kUInt8 &&
+                rows.size(1) >= B.most_bytes([&](aprnet_apr* h, int dl) { return aprnet_conv333_rows_bytes(h, dl, mode, cin); }), "rows buffer too small for this APR");
+    // the cached edge lists fix the size of the workspace
+    if (need_grad_input)
+        for (int64_t b = 0; b < nb; ++b)
+            if (27 * B.n[b] + 1 < (1ll << 31)) check(aprnet_edge_plan_build(B.h[b], B.dl[b], stream_of(grad_output)), "edge plan");
+    const int64_t bytes = B.most_bytes([&](aprnet_apr* h, int dl) { return aprnet_conv333_rows_backward_workspace_bytes(h, dl, mode, cin, cout, slots, need_grad_input ? 1 : 0); });
+    ld_tree = std::max(ld_tree, B.max_tree);
+    auto grad_tree = need_grad_input ? torch::empty({fold_tree ? 1 : nb, cin, ld_tree}, grad_output.options()) : torch::Tensor();
+    auto grad_input = need_grad_input ? torch::empty({nb, cin, n}, grad_output.options()) : torch::Tensor();
+    auto grad_weights = torch::zeros_like(weights);
+    auto ws = bytes_like(bytes, grad_output);
+    auto partial = torch::empty({aprnet_conv333_rows_partial_elems(mode, cin, cout)}, grad_output.options());
+    for (int64_t b = 0; b < nb; ++b)
+        check(aprnet_conv333_rows_backward(B.h[b], B.dl[b], mode, cin, cout, slots, row(rows, b), (const float*) row(grad_output, b), n, weights.data_ptr<float>(),
+                                           need_grad_input ? (float*) row(grad_input, b) : nullptr, n, grad_weights.data_ptr<float>(),
+                                           need_grad_input ? (float*) row(grad_tree, fold_tree ? 0 : b) : nullptr, ld_tree, fold_tree ? 1 : 0,
+                                           partial.data_ptr<float>(), ws.data_ptr(), stream_of(grad_output)),
+              mode == APRNET_PREC_BF16 ? "conv333_backward (tensor cores)" : "conv333_backward");
+    if (need_grad_input) fill_padding(grad_input, B.n);
+    return {grad_input, grad_weights, grad_tree};
+}
+
+// packed rows of an input whose forward call did not keep them (tree: its tree means per batch item, or undefined)
+static torch::Tensor conv333_pack(std::vector<APR*>& aprs, const torch::Tensor& input, const torch::Tensor& level_delta, int mode, const torch::Tensor& tree) {
+    const Batch B(aprs, input, level_delta);
+    const int cin = (int) input.size(1);
+    const int64_t bytes = B.most_bytes([&](aprnet_apr* h, int dl) { return aprnet_conv333_rows_bytes(h, dl, mode, cin); });
+    auto rows = torch::empty({input.size(0), (bytes + 255) / 256 * 256}, input.options().dtype(torch::kUInt8));
+    auto means = tree.defined() ? tree : torch::empty({1, cin, B.max_tree}, input.options());
+    for (int64_t b = 0; b < input.size(0); ++b)
+        check(aprnet_conv333_rows_pack(B.h[b], B.dl[b], mode, cin, (const float*) row(input, b), input.size(2), (float*) row(means, tree.defined() ? b : 0), means.size(2),
+                                       tree.defined() ? 1 : 0, row(rows, b), stream_of(input)), "conv333_backward (packing)");
+    return rows;
+}
+
 static std::vector<torch::Tensor> conv333_forward_impl(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights, torch::Tensor level_delta, bool keep_tree,
                                                        const std::string& precision = "") {
     CHECK_INPUT(input); CHECK_INPUT(weights);
-    check_batch(aprs, input);
-    TORCH_CHECK(weights.dim() == 6 && weights.size(3) == 3 && weights.size(4) == 3 && weights.size(5) == 3, "weights must be (levels, Cout, Cin, 3, 3, 3)");
-    TORCH_CHECK(input.size(1) == weights.size(2), "input tensor shape does not match weights tensor");
-    TORCH_CHECK(input.scalar_type() == weights.scalar_type(), "input and weights must have the same dtype");
+    check_conv333(input, weights);
     c10::cuda::CUDAGuard guard(input.device());
-    const auto dl = read_level_delta(level_delta, aprs.size());
-    int64_t max_tree = 1;
-    for (size_t i = 0; i < aprs.size(); ++i) {
-        check_level_delta(*aprs[i], dl[i]);
-        max_tree = std::max<int64_t>(max_tree, aprnet_tree_size(aprs[i]->handle(input), dl[i]));
-        TORCH_CHECK(aprs[i]->number_parts(dl[i]) <= input.size(2), "input has fewer particles than the APR at this level delta");
+    if (dtype_id(input) == APRNET_F32) {
+        auto r = conv333_forward_rows(aprs, input, weights, level_delta, resolve_mode(precision), keep_tree, false);
+        return {r[0], r[1]};
     }
+    const Batch B(aprs, input, level_delta);
     const int64_t cin = input.size(1), cout = weights.size(1), n = input.size(2);
     auto output = torch::empty({input.size(0), cout, n}, input.options());
     // one tree buffer per batch item when the caller keeps it for the backward pass, else one shared scratch
-    auto tree_all = torch::empty({keep_tree ? input.size(0) : 1, cin, max_tree}, input.options());
-    const int dt = dtype_id(input);
-    const bool tc = resolve_mode(precision) == 1 && dt == APRNET_F32;
-    torch::Tensor ws;
-    if (tc) {
-        int64_t bytes = 256;
-        for (size_t i = 0; i < aprs.size(); ++i)
-            bytes = std::max<int64_t>(bytes, aprnet_conv333_tc_forward_workspace_bytes(aprs[i]->handle(input), dl[i], (int) cin, (int) cout, (int) weights.size(0)));
-        ws = torch::empty({bytes}, input.options().dtype(torch::kUInt8));
-    }
-    for (int64_t b = 0; b < input.size(0); ++b) {
-        auto tree = tree_all.select(0, keep_tree ? b : 0);
-        if (tc)
-            check(aprnet_conv333_forward_tc(aprs[b]->handle(input), dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n,
-                                            (const float*) weights.data_ptr(), (float*) row(output, b), n, (float*) tree.data_ptr(), max_tree,
-                                            ws.data_ptr(), stream_of(input)), "conv333_forward (tensor cores)");
-        else
-            check(aprnet_conv333_forward(aprs[b]->handle(input), dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
-                                         weights.data_ptr(), row(output, b), n, tree.data_ptr(), max_tree, stream_of(input)),
-                  "conv333_forward");
-        zero_padding(output, b, aprs[b]->number_parts(dl[b]));
-    }
-    return {output, tree_all};
+    auto tree = torch::empty({keep_tree ? input.size(0) : 1, cin, B.max_tree}, input.options());
+    for (int64_t b = 0; b < input.size(0); ++b)
+        check(aprnet_conv333_forward(B.h[b], B.dl[b], APRNET_F64, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
+                                     weights.data_ptr(), row(output, b), n, row(tree, keep_tree ? b : 0), B.max_tree, stream_of(input)), "conv333_forward");
+    fill_padding(output, B.n);
+    return {output, tree};
 }
 
 torch::Tensor conv333_forward(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights, torch::Tensor level_delta) {
@@ -242,71 +330,24 @@ std::vector<torch::Tensor> conv333_forward_keep_tree(std::vector<APR*>& aprs, to
     return conv333_forward_impl(aprs, input, weights, level_delta, true, precision);
 }
 
-// Tensor-core forward that keeps the packed bf16 rows of the input (particles, tree means, zero row) for the
-// backward pass instead of the fp32 input and the tree means: returns {output, rows (B, bytes) uint8}.
-std::vector<torch::Tensor> conv333_forward_keep_rows(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights, torch::Tensor level_delta) {
+// float32 forward that keeps the packed rows of the input (particles, tree means, zero row) for the backward pass instead
+// of the input and the tree means: returns {output, rows (B, bytes) uint8}.  bias: added to the output, padding included.
+std::vector<torch::Tensor> conv333_forward_keep_rows(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights, torch::Tensor level_delta,
+                                                     const std::string& precision, c10::optional<torch::Tensor> bias) {
     CHECK_INPUT(input); CHECK_INPUT(weights);
-    check_batch(aprs, input);
-    TORCH_CHECK(weights.dim() == 6 && weights.size(3) == 3 && weights.size(4) == 3 && weights.size(5) == 3, "weights must be (levels, Cout, Cin, 3, 3, 3)");
-    TORCH_CHECK(input.size(1) == weights.size(2), "input tensor shape does not match weights tensor");
-    TORCH_CHECK(input.scalar_type() == torch::kFloat32 && weights.scalar_type() == torch::kFloat32, "the tensor-core path takes float32 tensors");
+    check_conv333(input, weights);
+    TORCH_CHECK(input.scalar_type() == torch::kFloat32, "the packed-row path takes float32 tensors");
     c10::cuda::CUDAGuard guard(input.device());
-    const auto dl = read_level_delta(level_delta, aprs.size());
-    const int64_t cin = input.size(1), cout = weights.size(1), n = input.size(2);
-    int64_t max_tree = 1, rows_bytes = 256, w_bytes = 256;
-    for (size_t i = 0; i < aprs.size(); ++i) {
-        check_level_delta(*aprs[i], dl[i]);
-        aprnet_apr* h = aprs[i]->handle(input);
-        TORCH_CHECK(aprs[i]->number_parts(dl[i]) <= n, "input has fewer particles than the APR at this level delta");
-        max_tree = std::max<int64_t>(max_tree, aprnet_tree_size(h, dl[i]));
-        const int64_t rb = aprnet_conv333_tc_packed_rows_bytes(h, dl[i], (int) cin);
-        rows_bytes = std::max(rows_bytes, rb);
-        w_bytes = std::max(w_bytes, aprnet_conv333_tc_forward_workspace_bytes(h, dl[i], (int) cin, (int) cout, (int) weights.size(0)) - rb);
-    }
-    auto output = torch::empty({input.size(0), cout, n}, input.options());
-    auto tree = torch::empty({cin, max_tree}, input.options());
-    // per batch item: [packed rows | packed weights]; only the rows part is handed back (the view keeps the buffer)
-    auto ws = torch::empty({input.size(0), rows_bytes + w_bytes}, input.options().dtype(torch::kUInt8));
-    for (int64_t b = 0; b < input.size(0); ++b) {
-        check(aprnet_conv333_forward_tc(aprs[b]->handle(input), dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n,
-                                        (const float*) weights.data_ptr(), (float*) row(output, b), n, (float*) tree.data_ptr(), max_tree,
-                                        row(ws, b), stream_of(input)), "conv333_forward (tensor cores)");
-        zero_padding(output, b, aprs[b]->number_parts(dl[b]));
-    }
-    return {output, ws};
+    auto r = conv333_forward_rows(aprs, input, weights, level_delta, resolve_mode(precision), false, true, torch::Tensor(), bias);
+    return {r[0], r[2]};
 }
 
 std::vector<torch::Tensor> conv333_backward_with_rows(std::vector<APR*>& aprs, torch::Tensor rows, torch::Tensor weights, torch::Tensor grad_output,
-                                                      torch::Tensor level_delta, bool need_grad_input) {
+                                                      torch::Tensor level_delta, bool need_grad_input, const std::string& precision) {
     CHECK_INPUT(weights); CHECK_INPUT(grad_output); CHECK_INPUT(rows);
-    check_batch(aprs, grad_output);
-    TORCH_CHECK(rows.dim() == 2 && rows.size(0) == grad_output.size(0) && rows.scalar_type() == torch::kUInt8, "rows must be the (batch, bytes) buffer of conv333_forward_keep_rows");
-    TORCH_CHECK(grad_output.dim() == 3 && grad_output.size(1) == weights.size(1) && grad_output.scalar_type() == torch::kFloat32, "grad_output shape does not match");
     c10::cuda::CUDAGuard guard(grad_output.device());
-    const auto dl = read_level_delta(level_delta, aprs.size());
-    const int64_t cin = weights.size(2), cout = weights.size(1), n = grad_output.size(2);
-    int64_t max_tree = 1, bytes = 256;
-    for (size_t i = 0; i < aprs.size(); ++i) {
-        check_level_delta(*aprs[i], dl[i]);
-        aprnet_apr* h = aprs[i]->handle(grad_output);
-        max_tree = std::max<int64_t>(max_tree, aprnet_tree_size(h, dl[i]));
-        TORCH_CHECK(rows.size(1) >= aprnet_conv333_tc_packed_rows_bytes(h, dl[i], (int) cin), "rows buffer too small for this APR");
-        bytes = std::max<int64_t>(bytes, aprnet_conv333_tc_workspace_bytes(h, dl[i], (int) cin, (int) cout, (int) weights.size(0)));
-    }
-    auto grad_tree = torch::empty({cin, max_tree}, grad_output.options());
-    auto grad_input = need_grad_input ? torch::empty({grad_output.size(0), cin, n}, grad_output.options()) : torch::Tensor();
-    auto grad_weights = torch::zeros_like(weights);
-    auto ws = torch::empty({bytes}, grad_output.options().dtype(torch::kUInt8));
-    auto partial = torch::empty({aprnet_conv333_tc_dw_partial_elems((int) cin, (int) cout)}, grad_output.options());
-    for (int64_t b = 0; b < grad_output.size(0); ++b) {
-        check(aprnet_conv333_backward_tc_rows(aprs[b]->handle(grad_output), dl[b], (int) cin, (int) cout, (int) weights.size(0), row(rows, b),
-                                              (const float*) row(grad_output, b), n, (const float*) weights.data_ptr(),
-                                              need_grad_input ? (float*) row(grad_input, b) : nullptr, n, (float*) grad_weights.data_ptr(),
-                                              (float*) grad_tree.data_ptr(), max_tree, (float*) partial.data_ptr(), ws.data_ptr(), stream_of(grad_output)),
-              "conv333_backward (tensor cores, packed rows)");
-        if (need_grad_input) zero_padding(grad_input, b, aprs[b]->number_parts(dl[b]));
-    }
-    return {grad_input, grad_weights};
+    auto r = conv333_backward_rows(aprs, rows, weights, grad_output, level_delta, resolve_mode(precision), need_grad_input, true);
+    return {r[0], r[1]};
 }
 
 static std::vector<torch::Tensor> conv333_backward_impl(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights,
@@ -318,55 +359,32 @@ static std::vector<torch::Tensor> conv333_backward_impl(std::vector<APR*>& aprs,
                 grad_output.size(2) == input.size(2), "grad_output shape does not match");
     TORCH_CHECK(input.size(1) == weights.size(2), "input tensor shape does not match weights tensor");
     c10::cuda::CUDAGuard guard(input.device());
-    const auto dl = read_level_delta(level_delta, aprs.size());
-    int64_t max_tree = 1;
-    for (size_t i = 0; i < aprs.size(); ++i) {
-        check_level_delta(*aprs[i], dl[i]);
-        max_tree = std::max<int64_t>(max_tree, aprnet_tree_size(aprs[i]->handle(input), dl[i]));
-    }
-    const int64_t cin = input.size(1), cout = weights.size(1), n = input.size(2);
-    const int dt = dtype_id(input);
-    void* st = stream_of(input);
-    const bool tc = resolve_mode(precision) == 1 && dt == APRNET_F32;
-    const bool skip_gin = tc && !need_grad_input;        // only the tensor-core driver can leave the input gradient out
+    const Batch B(aprs, input, level_delta);
+    const int64_t cin = input.size(1), cout = weights.size(1), n = input.size(2), max_tree = B.max_tree;
     const bool have_tree = saved_tree.has_value() && saved_tree->defined() && saved_tree->dim() == 3 && saved_tree->size(0) == input.size(0) &&
                            saved_tree->size(1) == cin && saved_tree->size(2) == max_tree && saved_tree->is_contiguous() &&
                            saved_tree->scalar_type() == input.scalar_type();
+    if (dtype_id(input) == APRNET_F32) {
+        const int mode = resolve_mode(precision);
+        auto rows = conv333_pack(aprs, input, level_delta, mode, have_tree ? *saved_tree : torch::Tensor());
+        // without a need for it only the tensor-core arithmetic leaves the input gradient out here
+        auto r = conv333_backward_rows(aprs, rows, weights, grad_output, level_delta, mode, need_grad_input || mode != APRNET_PREC_BF16, true);
+        return {r[0], r[1]};
+    }
+    void* st = stream_of(input);
     auto tree_all = have_tree ? *saved_tree : torch::empty({1, cin, max_tree}, input.options());
     auto grad_tree = torch::empty({cin, max_tree}, input.options());
-    // the tensor-core path writes every valid entry of grad_input; the CUDA-core path accumulates into zeros
-    auto grad_input = skip_gin ? torch::Tensor() : (tc ? torch::empty_like(input) : torch::zeros_like(input));
+    auto grad_input = torch::zeros_like(input);          // the double kernels accumulate into zeros
     auto grad_weights = torch::zeros_like(weights);
-    torch::Tensor partial;
-    if (!tc) partial = torch::empty({aprnet_conv333_partial_elems((int) cin, (int) cout)}, input.options());
-    torch::Tensor ws;
-    if (tc) {
-        int64_t bytes = 256;
-        for (size_t i = 0; i < aprs.size(); ++i)
-            bytes = std::max<int64_t>(bytes, aprnet_conv333_tc_workspace_bytes(aprs[i]->handle(input), dl[i], (int) cin, (int) cout, (int) weights.size(0)));
-        ws = torch::empty({bytes}, input.options().dtype(torch::kUInt8));
-    }
-    torch::Tensor partial_tc;
-    if (tc) partial_tc = torch::empty({aprnet_conv333_tc_dw_partial_elems((int) cin, (int) cout)}, input.options());
+    auto partial = torch::empty({aprnet_conv333_partial_elems((int) cin, (int) cout)}, input.options());
     for (int64_t b = 0; b < input.size(0); ++b) {
-        aprnet_apr* h = aprs[b]->handle(input);
-        auto tree = tree_all.select(0, have_tree ? b : 0);
-        if (tc) {
-            check(aprnet_conv333_backward_tc(h, dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n,
-                                             (const float*) row(grad_output, b), n, (const float*) weights.data_ptr(),
-                                             skip_gin ? nullptr : (float*) row(grad_input, b), (float*) grad_weights.data_ptr(), (float*) tree.data_ptr(),
-                                             have_tree ? 1 : 0, (float*) grad_tree.data_ptr(), max_tree, (float*) partial_tc.data_ptr(),
-                                             ws.data_ptr(), st),
-                  "conv333_backward (tensor cores)");
-            if (!skip_gin) zero_padding(grad_input, b, aprs[b]->number_parts(dl[b]));
-            continue;
-        }
+        char* tree = row(tree_all, have_tree ? b : 0);
         if (!have_tree)
-        check(aprnet_fill_tree_mean_forward(h, dl[b], dt, (int) cin, row(input, b), n, tree.data_ptr(), max_tree, st), "fill_tree_mean");
-        check(aprnet_conv333_backward_weights(h, dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
-                                              tree.data_ptr(), max_tree, row(grad_output, b), n, grad_weights.data_ptr(),
+            check(aprnet_fill_tree_mean_forward(B.h[b], B.dl[b], APRNET_F64, (int) cin, row(input, b), n, tree, max_tree, st), "fill_tree_mean");
+        check(aprnet_conv333_backward_weights(B.h[b], B.dl[b], APRNET_F64, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
+                                              tree, max_tree, row(grad_output, b), n, grad_weights.data_ptr(),
                                               partial.data_ptr(), st), "conv333_backward_weights");
-        check(aprnet_conv333_backward_input(h, dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(grad_output, b), n,
+        check(aprnet_conv333_backward_input(B.h[b], B.dl[b], APRNET_F64, (int) cin, (int) cout, (int) weights.size(0), row(grad_output, b), n,
                                             weights.data_ptr(), row(grad_input, b), n, grad_tree.data_ptr(), max_tree, st),
               "conv333_backward_input");
     }
@@ -395,34 +413,22 @@ std::vector<torch::Tensor> conv333_forward_pretree(std::vector<APR*>& aprs, torc
     TORCH_CHECK(tree.dim() == 3 && tree.size(0) == input.size(0) && tree.size(1) == input.size(1) && tree.scalar_type() == input.scalar_type(),
                 "tree must be (batch, Cin, tree nodes) of the input's dtype");
     c10::cuda::CUDAGuard guard(input.device());
-    const auto dl = read_level_delta(level_delta, aprs.size());
-    const int64_t cin = input.size(1), cout = weights.size(1), n = input.size(2), ldt = tree.size(2);
-    const int dt = dtype_id(input);
-    const bool tc = resolve_mode(precision) == 1 && dt == APRNET_F32;
-    int64_t rows_bytes = 256, w_bytes = 256;
-    for (size_t i = 0; i < aprs.size(); ++i) {
-        check_level_delta(*aprs[i], dl[i]);
-        aprnet_apr* h = aprs[i]->handle(input);
-        TORCH_CHECK(aprs[i]->number_parts(dl[i]) <= n && aprnet_tree_size(h, dl[i]) <= ldt, "input or tree has fewer entries than the APR at this level delta");
-        if (tc) {
-            const int64_t rb = aprnet_conv333_tc_packed_rows_bytes(h, dl[i], (int) cin);
-            rows_bytes = std::max(rows_bytes, rb);
-            w_bytes = std::max(w_bytes, aprnet_conv333_tc_forward_workspace_bytes(h, dl[i], (int) cin, (int) cout, (int) weights.size(0)) - rb);
-        }
+    if (dtype_id(input) == APRNET_F32) {
+        const Batch B(aprs, input, level_delta);
+        TORCH_CHECK(B.max_tree <= std::max<int64_t>(tree.size(2), 1), "tree has fewer entries than the APR at this level delta");
+        const int mode = resolve_mode(precision);
+        auto r = conv333_forward_rows(aprs, input, weights, level_delta, mode, true, mode == APRNET_PREC_BF16, tree);
+        return {r[0], mode == APRNET_PREC_BF16 ? r[2] : torch::empty({0}, input.options().dtype(torch::kUInt8))};
     }
+    const Batch B(aprs, input, level_delta);
+    TORCH_CHECK(B.max_tree <= std::max<int64_t>(tree.size(2), 1), "tree has fewer entries than the APR at this level delta");
+    const int64_t cin = input.size(1), cout = weights.size(1), n = input.size(2);
     auto output = torch::empty({input.size(0), cout, n}, input.options());
-    torch::Tensor ws = tc ? torch::empty({input.size(0), rows_bytes + w_bytes}, input.options().dtype(torch::kUInt8)) : torch::Tensor();
-    for (int64_t b = 0; b < input.size(0); ++b) {
-        if (tc)
-            check(aprnet_conv333_forward_tc_pretree(aprs[b]->handle(input), dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n,
-                                                    (const float*) weights.data_ptr(), (float*) row(output, b), n, (const float*) row(tree, b), ldt,
-                                                    row(ws, b), stream_of(input)), "conv333_forward_pretree (tensor cores)");
-        else
-            check(aprnet_conv333_forward_pretree(aprs[b]->handle(input), dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
-                                                 weights.data_ptr(), row(output, b), n, row(tree, b), ldt, stream_of(input)), "conv333_forward_pretree");
-        zero_padding(output, b, aprs[b]->number_parts(dl[b]));
-    }
-    return {output, tc ? ws : torch::empty({0}, input.options().dtype(torch::kUInt8))};
+    for (int64_t b = 0; b < input.size(0); ++b)
+        check(aprnet_conv333_forward_pretree(B.h[b], B.dl[b], APRNET_F64, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
+                                             weights.data_ptr(), row(output, b), n, row(tree, b), tree.size(2), stream_of(input)), "conv333_forward_pretree");
+    fill_padding(output, B.n);
+    return {output, torch::empty({0}, input.options().dtype(torch::kUInt8))};
 }
 
 // backward without the tree adjoint: returns {grad_input (direct contributions), grad_tree (B, Cin, T), grad_weights}.
@@ -430,49 +436,30 @@ std::vector<torch::Tensor> conv333_forward_pretree(std::vector<APR*>& aprs, torc
 std::vector<torch::Tensor> conv333_backward_pretree(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor tree, torch::Tensor kept, torch::Tensor weights,
                                                     torch::Tensor grad_output, torch::Tensor level_delta, bool need_grad_input) {
     CHECK_INPUT(weights); CHECK_INPUT(grad_output); CHECK_INPUT(tree);
-    check_batch(aprs, grad_output);
     c10::cuda::CUDAGuard guard(grad_output.device());
-    const auto dl = read_level_delta(level_delta, aprs.size());
-    const int64_t cin = weights.size(2), cout = weights.size(1), n = grad_output.size(2), ldt = tree.size(2), B = grad_output.size(0);
+    const Batch B(aprs, grad_output, level_delta);
+    const int64_t cin = weights.size(2), cout = weights.size(1), n = grad_output.size(2), ldt = tree.size(2), nb = grad_output.size(0);
+    TORCH_CHECK(grad_output.size(1) == cout && tree.dim() == 3 && tree.size(0) == nb && tree.size(1) == cin, "shapes do not match");
     const int dt = dtype_id(grad_output);
-    const bool tc = dt == APRNET_F32 && kept.numel() > 0;          // a rows buffer exists only when the forward call ran on the tensor cores
-    TORCH_CHECK(grad_output.size(1) == cout && tree.dim() == 3 && tree.size(0) == B && tree.size(1) == cin, "shapes do not match");
-    if (!tc) { CHECK_INPUT(input); TORCH_CHECK(input.dim() == 3 && input.size(1) == cin && input.size(2) == n, "input shape does not match"); }
-    auto grad_tree = torch::zeros({B, cin, ldt}, grad_output.options());
-    auto grad_weights = torch::zeros_like(weights);
-    torch::Tensor grad_input;
+    const bool bf16 = dt == APRNET_F32 && kept.numel() > 0;          // a rows buffer exists only when the forward call ran on the tensor cores
+    if (!bf16) { CHECK_INPUT(input); TORCH_CHECK(input.dim() == 3 && input.size(1) == cin && input.size(2) == n, "input shape does not match"); }
+    if (dt == APRNET_F32) {
+        const int mode = bf16 ? APRNET_PREC_BF16 : APRNET_PREC_F32;
+        auto rows = bf16 ? kept : conv333_pack(aprs, input, level_delta, mode, tree);
+        auto r = conv333_backward_rows(aprs, rows, weights, grad_output, level_delta, mode, need_grad_input, false, ldt);
+        return {r[0], need_grad_input ? r[2] : torch::zeros({nb, cin, ldt}, grad_output.options()), r[1]};
+    }
     void* st = stream_of(grad_output);
-    if (tc) {
-        int64_t bytes = 256;
-        for (size_t i = 0; i < aprs.size(); ++i) {
-            check_level_delta(*aprs[i], dl[i]);
-            aprnet_apr* h = aprs[i]->handle(grad_output);
-            TORCH_CHECK(kept.dim() == 2 && kept.size(0) == B && kept.size(1) >= aprnet_conv333_tc_packed_rows_bytes(h, dl[i], (int) cin), "rows buffer too small for this APR");
-            bytes = std::max<int64_t>(bytes, aprnet_conv333_tc_workspace_bytes(h, dl[i], (int) cin, (int) cout, (int) weights.size(0)));
-        }
-        if (need_grad_input) grad_input = torch::empty({B, cin, n}, grad_output.options());
-        auto ws = torch::empty({bytes}, grad_output.options().dtype(torch::kUInt8));
-        auto partial = torch::empty({aprnet_conv333_tc_dw_partial_elems((int) cin, (int) cout)}, grad_output.options());
-        for (int64_t b = 0; b < B; ++b) {
-            check(aprnet_conv333_backward_tc_rows_pretree(aprs[b]->handle(grad_output), dl[b], (int) cin, (int) cout, (int) weights.size(0), row(kept, b),
-                                                          (const float*) row(grad_output, b), n, (const float*) weights.data_ptr(),
-                                                          need_grad_input ? (float*) row(grad_input, b) : nullptr, n, (float*) grad_weights.data_ptr(),
-                                                          (float*) row(grad_tree, b), ldt, (float*) partial.data_ptr(), ws.data_ptr(), st),
-                  "conv333_backward_pretree (tensor cores)");
-            if (need_grad_input) zero_padding(grad_input, b, aprs[b]->number_parts(dl[b]));
-        }
-    } else {
-        auto partial = torch::empty({aprnet_conv333_partial_elems((int) cin, (int) cout)}, grad_output.options());
-        grad_input = torch::zeros({B, cin, n}, grad_output.options());
-        for (int64_t b = 0; b < B; ++b) {
-            check_level_delta(*aprs[b], dl[b]);
-            aprnet_apr* h = aprs[b]->handle(grad_output);
-            check(aprnet_conv333_backward_weights(h, dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n, row(tree, b), ldt,
-                                                  row(grad_output, b), n, grad_weights.data_ptr(), partial.data_ptr(), st), "conv333_backward_weights");
-            if (need_grad_input)
-                check(aprnet_conv333_backward_input_pretree(h, dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(grad_output, b), n,
-                                                            weights.data_ptr(), row(grad_input, b), n, row(grad_tree, b), ldt, st), "conv333_backward_input_pretree");
-        }
+    auto grad_tree = torch::zeros({nb, cin, ldt}, grad_output.options());
+    auto grad_weights = torch::zeros_like(weights);
+    auto partial = torch::empty({aprnet_conv333_partial_elems((int) cin, (int) cout)}, grad_output.options());
+    auto grad_input = torch::zeros({nb, cin, n}, grad_output.options());
+    for (int64_t b = 0; b < nb; ++b) {
+        check(aprnet_conv333_backward_weights(B.h[b], B.dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n, row(tree, b), ldt,
+                                              row(grad_output, b), n, grad_weights.data_ptr(), partial.data_ptr(), st), "conv333_backward_weights");
+        if (need_grad_input)
+            check(aprnet_conv333_backward_input_pretree(B.h[b], B.dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(grad_output, b), n,
+                                                        weights.data_ptr(), row(grad_input, b), n, row(grad_tree, b), ldt, st), "conv333_backward_input_pretree");
     }
     return {grad_input, grad_tree, grad_weights};
 }
@@ -531,8 +518,8 @@ torch::Tensor conv111_forward(std::vector<APR*>& aprs, torch::Tensor input, torc
         if (rc == APRNET_ERR_UNSUPPORTED)
         check(aprnet_conv111_forward(aprs[b]->handle(input), dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
                                      weights.data_ptr(), row(output, b), n, stream_of(input)), "conv111_forward");
-        zero_padding(output, b, aprs[b]->number_parts(dl[b]));
     }
+    fill_padding(output, valid_of(aprs, dl));
     return output;
 }
 
@@ -562,7 +549,6 @@ std::vector<torch::Tensor> conv111_backward(std::vector<APR*>& aprs, torch::Tens
         if (rc == APRNET_ERR_UNSUPPORTED)
         check(aprnet_conv111_backward_input(h, dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(grad_output, b), n,
                                             weights.data_ptr(), row(grad_input, b), n, st), "conv111_backward_input");
-        zero_padding(grad_input, b, aprs[b]->number_parts(dl[b]));
         rc = APRNET_ERR_UNSUPPORTED;
         if (tc) {
             rc = aprnet_conv111_backward_weights_tc(h, dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n,
@@ -575,6 +561,7 @@ std::vector<torch::Tensor> conv111_backward(std::vector<APR*>& aprs, torch::Tens
                                               row(grad_output, b), n, grad_weights.data_ptr(), partial.data_ptr(), st),
               "conv111_backward_weights");
     }
+    fill_padding(grad_input, valid_of(aprs, dl));
     return {grad_input, grad_weights};
 }
 
@@ -618,8 +605,8 @@ std::vector<torch::Tensor> maxpool_forward_cuda(std::vector<APR*>& aprs, torch::
     for (int64_t b = 0; b < input.size(0); ++b) {
         check(aprnet_maxpool_forward(aprs[b]->handle(input), dl[b], dt, (int) input.size(1), row(input, b), input.size(2), row(output, b),
                                      (int64_t*) row(max_indices, b), max_size, stream_of(input)), "maxpool_forward");
-        zero_padding(output, b, aprs[b]->number_parts(dl[b] + 1));
     }
+    fill_padding(output, valid_of(aprs, dl, +1));
     return {output, max_indices};
 }
 
@@ -654,8 +641,8 @@ torch::Tensor upsample_const_forward(std::vector<APR*>& aprs, torch::Tensor inpu
     for (int64_t b = 0; b < input.size(0); ++b) {
         check(aprnet_upsample_forward(aprs[b]->handle(input), dl[b], dt, (int) input.size(1), row(input, b), input.size(2), row(output, b),
                                       max_size, stream_of(input)), "upsample_const_forward");
-        zero_padding(output, b, aprs[b]->number_parts(dl[b] - 1));
     }
+    fill_padding(output, valid_of(aprs, dl, -1));
     return output;
 }
 
@@ -672,8 +659,8 @@ torch::Tensor upsample_const_backward(std::vector<APR*>& aprs, torch::Tensor gra
     for (int64_t b = 0; b < grad_output.size(0); ++b) {
         check(aprnet_upsample_backward(aprs[b]->handle(grad_output), dl[b], dt, (int) grad_output.size(1), row(grad_output, b),
                                        grad_output.size(2), row(grad_input, b), max_size, stream_of(grad_output)), "upsample_const_backward");
-        zero_padding(grad_input, b, aprs[b]->number_parts(dl[b]));
     }
+    fill_padding(grad_input, valid_of(aprs, dl));
     return grad_input;
 }
 
@@ -733,8 +720,8 @@ torch::Tensor reconstruct_backward(std::vector<APR*>& aprs, torch::Tensor grad_o
     for (int64_t b = 0; b < grad_output.size(0); ++b) {
         check(aprnet_image_to_cells(aprs[b]->handle(grad_output), dl[b], dtype_id(grad_output), (int) grad_output.size(1), row(grad_output, b),
                                     row(grad_input, b), max_size, 0, ws.data_ptr(), stream_of(grad_output)), "reconstruct_backward");
-        zero_padding(grad_input, b, aprs[b]->number_parts(dl[b]));
     }
+    fill_padding(grad_input, valid_of(aprs, dl));
     return grad_input;
 }
 
@@ -751,8 +738,8 @@ torch::Tensor sample_particles_forward(std::vector<APR*>& aprs, torch::Tensor in
     for (int64_t b = 0; b < input.size(0); ++b) {
         check(aprnet_image_to_cells(aprs[b]->handle(input), dl[b], dtype_id(input), (int) input.size(1), row(input, b),
                                     row(output, b), max_size, 1, ws.data_ptr(), stream_of(input)), "sample_particles_forward");
-        zero_padding(output, b, aprs[b]->number_parts(dl[b]));
     }
+    fill_padding(output, valid_of(aprs, dl));
     return output;
 }
 
@@ -981,8 +968,8 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
     cuda.def("conv333_forward_keep_tree", &conv333_forward_keep_tree, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "");
     cuda.def("conv333_backward_with_tree", &conv333_backward_with_tree, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "tree"_a, "need_grad_input"_a = true,
              "precision"_a = "");
-    cuda.def("conv333_forward_keep_rows", &conv333_forward_keep_rows, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a);
-    cuda.def("conv333_backward_with_rows", &conv333_backward_with_rows, "aprs"_a, "rows"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "need_grad_input"_a = true);
+    cuda.def("conv333_forward_keep_rows", &conv333_forward_keep_rows, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "bf16", "bias"_a = py::none());
+    cuda.def("conv333_backward_with_rows", &conv333_backward_with_rows, "aprs"_a, "rows"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "need_grad_input"_a = true, "precision"_a = "bf16");
     cuda.def("upsample_const_forward", &upsample_const_forward, "aprs"_a, "input"_a, "level_delta"_a);
     cuda.def("upsample_const_backward", &upsample_const_backward, "aprs"_a, "grad_output"_a, "level_delta"_a);
     cuda.def("reconstruct_forward", &reconstruct_forward, "aprs"_a, "input"_a, "level_delta"_a);

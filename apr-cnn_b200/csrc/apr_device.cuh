@@ -145,11 +145,11 @@ void aprnet_free_edge_plan(EdgePlan& ep);
 int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* vrows, int gpad, long long zero_row,
                              const void* wp_packed, const EdgePlan* ep, long long a0, long long a1,
                              float* gin, long long ld_in, float* gtree, long long ld_tree, cudaStream_t st);
-// CUDA-core fp32 kernels for Cin <= 4 (conv333_small.cu), used by the tensor-core drivers for such layers:
+// CUDA-core fp32 kernels for Cin <= 4 (conv333_small.cu), used in either arithmetic for such layers:
 // vals = channel-major staging buffer [cin][N + T + 1] (particles, tree means, zero)
 bool aprnet_small_cin(int cin);
 int aprnet_small_stage(const float* x, long long ld_x, long long n, const float* tree, long long ld_tree, long long t, int cin, float* vals, cudaStream_t st);
-int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, float* out, long long ld_out, cudaStream_t st);
+int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, const float* bias, float* out, long long ld_out, cudaStream_t st);
 int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* gout, long long ld_out,
                                   float* gw, float* partial, cudaStream_t st);
 int aprnet_tc_pack_weights(const float* w, int slots, int cin, int cout, int mode, void* wp, cudaStream_t st);
@@ -165,3 +165,29 @@ extern "C" int aprnet_conv333_backward_input_cross_level_tc(aprnet_apr* a, int d
 int aprnet_cross_level_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* grows, int gpad, const float* w, float* gin,
                           long long ld_in, float* gtree, long long ld_tree, void* wp_ws, void* edge_ws, long long edge_ws_bytes, void* stream,
                           bool tree_adjoint);
+
+// fp32 path (conv333_f32.cu): the same steps over packed fp32 rows
+size_t aprnet_f32_rows_bytes(const aprnet_apr* a, int dl, int cin);
+size_t aprnet_f32_forward_bytes(const aprnet_apr* a, int dl, int cin, int cout, int slots);        // packed input rows + packed weights
+size_t aprnet_f32_backward_bytes(const aprnet_apr* a, int dl, int cin, int cout, int slots);       // packed grad_output rows, weights, edge sums
+int64_t aprnet_f32_partial_elems(int cin, int cout);
+int aprnet_f32_pack_input(const aprnet_apr* a, int dl, int cin, const float* in, long long ld_in, const float* tree, long long ld_tree, void* rows, cudaStream_t st);
+int aprnet_f32_pack_grad(const aprnet_apr* a, int dl, int cout, const float* gout, long long ld_out, void* grows, cudaStream_t st);
+int aprnet_f32_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* w, const float* bias, float* out, long long ld_out, void* workspace, cudaStream_t st);
+int aprnet_f32_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* rows, const float* gout, long long ld_out, const void* grows,
+                                float* gw, float* partial, cudaStream_t st);
+int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* gout, long long ld_out, const float* w, float* gin, long long ld_in,
+                              float* gtree, long long ld_tree, void* workspace, bool tree_adjoint, cudaStream_t st);
+
+// stream-ordered scratch of one call, for entry points whose signature has no workspace
+struct StreamScratch {
+    void* p = nullptr;
+    cudaStream_t st;
+    explicit StreamScratch(cudaStream_t s) : st(s) {}
+    ~StreamScratch() { if (p) cudaFreeAsync(p, st); }
+    int get(size_t bytes) {
+        const cudaError_t e = cudaMallocAsync(&p, bytes, st);
+        if (e != cudaSuccess) { p = nullptr; cudaGetLastError(); aprnet_set_error("allocation of %zu bytes of scratch failed: %s", bytes, cudaGetErrorString(e)); return APRNET_ERR_CUDA; }
+        return APRNET_OK;
+    }
+};

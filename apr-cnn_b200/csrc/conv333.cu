@@ -1,10 +1,8 @@
-// 3x3x3 particle convolution: forward, input gradient and weight gradient (CUDA-core path,
-// float and double).
+// 3x3x3 particle convolution in double precision (forward, input gradient, weight gradient), the C entry points that
+// take either dtype, and the atomic scatter of the cross-level input gradient for structures beyond the edge plan.
 //
-// Replaces pyapr/aprnet/cuda/src/conv333_gpu.cu and conv333_gpu_backward.cu.  The reference puts the
-// input channel in grid.z and combines channels with atomicAdd into a zero-filled output, re-stages a
-// dense (z, x, y) patch per block and re-enumerates non-empty tiles on every call.  Here the cell
-// resolution is a cached neighbour table (27 int32 per output location, apr_handle.cu), and
+// float32 tensors go to the row drivers (conv333_rows.cu).  The double kernels gather straight from the channel-major
+// tensors through the cached neighbour table (27 int32 per output location, apr_handle.cu):
 //   * forward: one thread owns one output location and a block of output channels, loops over all
 //     input channels and taps, and writes each output exactly once;
 //   * input gradient: same-level taps are gathered through the mirrored table entry; cross-level taps (parent-level
@@ -354,7 +352,6 @@ __global__ void reduce_partial_kernel(const T* __restrict__ partial, int nchunks
 // host side
 // ---------------------------------------------------------------------------------------------
 template<typename T> struct FwdCfg;
-template<> struct FwdCfg<float> { static constexpr int OB = 32, IB = 8, TPB = 256; };
 template<> struct FwdCfg<double> { static constexpr int OB = 16, IB = 8, TPB = 128; };
 
 template<typename T, int OB, int IB, int TPB>
@@ -383,10 +380,6 @@ int conv333_fwd(aprnet_apr* a, int dl, int cin, int cout, int slots, const T* in
     snprintf(pname, sizeof(pname), "conv333_fwd:ci%d:co%d:dl%d", cin, cout, dl);
     const SegTable segs = make_seg_table(aprnet_segments(a, dl, slots, false), C::TPB);
     if (segs.tile_begin[segs.n] == 0) return APRNET_OK;
-    if (cout <= 4 && sizeof(T) == 4)
-        return launch_forward<T, 4, C::IB, C::TPB>(segs, plan, in, ld_in, tree, ld_tree, w, out, ld_out, cin, cout, st, pname);
-    if (cout <= 16)
-        return launch_forward<T, 16, C::IB, C::TPB>(segs, plan, in, ld_in, tree, ld_tree, w, out, ld_out, cin, cout, st, pname);
     return launch_forward<T, C::OB, C::IB, C::TPB>(segs, plan, in, ld_in, tree, ld_tree, w, out, ld_out, cin, cout, st, pname);
 }
 
@@ -484,16 +477,7 @@ int conv333_bwd_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, con
         const ll len = s.end - s.begin;
         const int nranges = (int) std::min<ll>(max_ranges, (len + 511) / 512);
         const ll range_len = (len + nranges - 1) / nranges;
-        int rc;
-        if (sizeof(T) == 8) {
-            rc = launch_dw<T, 16, 16, 1, 16, 256>(s.begin, s.end, nranges, range_len, plan, in, ld_in, tree, ld_tree, gout, ld_out, partial, cin, cout, st, pname);
-        } else if (cin >= 24) {
-            rc = launch_dw<T, 32, 32, 4, 32, 256>(s.begin, s.end, nranges, range_len, plan, in, ld_in, tree, ld_tree, gout, ld_out, partial, cin, cout, st, pname);
-        } else if (cin > 2) {
-            rc = launch_dw<T, 8, 32, 4, 32, 256>(s.begin, s.end, nranges, range_len, plan, in, ld_in, tree, ld_tree, gout, ld_out, partial, cin, cout, st, pname);
-        } else {
-            rc = launch_dw<T, 2, 32, 4, 64, 256>(s.begin, s.end, nranges, range_len, plan, in, ld_in, tree, ld_tree, gout, ld_out, partial, cin, cout, st, pname);
-        }
+        const int rc = launch_dw<T, 16, 16, 1, 16, 256>(s.begin, s.end, nranges, range_len, plan, in, ld_in, tree, ld_tree, gout, ld_out, partial, cin, cout, st, pname);
         if (rc) return rc;
         { AprnetProfScope _prof("conv333_dw_reduce", st);
         reduce_partial_kernel<T><<<aprnet_ceil_div(elems, 256), 256, 0, st>>>(partial, nranges, elems, gw + (ll) s.slot * elems);
@@ -518,13 +502,46 @@ int conv333_bwd_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, con
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), \
                      "leading dimension too small")
 
+// float32 through the row drivers, with stream-ordered scratch where the signature has no workspace
+namespace {
+
+int forward_f32(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* in, ll ld_in, const float* w, float* out, ll ld_out, float* tree, ll ld_tree,
+                int tree_valid, cudaStream_t st) {
+    StreamScratch ws(st);
+    const int rc = ws.get((size_t) aprnet_conv333_rows_forward_workspace_bytes(a, dl, APRNET_PREC_F32, cin, cout, slots));
+    return rc ? rc : aprnet_conv333_rows_forward(a, dl, APRNET_PREC_F32, cin, cout, slots, in, ld_in, w, nullptr, out, ld_out, tree, ld_tree, tree_valid, ws.p, st);
+}
+
+int backward_input_f32(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* gout, ll ld_out, const float* w, float* gin, ll ld_in,
+                       float* gtree, ll ld_tree, int fold_tree, cudaStream_t st) {
+    // the plan fixes the size of the workspace
+    if (27 * a->number_parts(dl) + 1 < (1ll << 31) && !aprnet_get_edge_plan(a, dl, st)) return APRNET_ERR_CUDA;
+    StreamScratch ws(st);
+    const int rc = ws.get((size_t) aprnet_conv333_rows_backward_workspace_bytes(a, dl, APRNET_PREC_F32, cin, cout, slots, 1));
+    return rc ? rc : aprnet_conv333_rows_backward(a, dl, APRNET_PREC_F32, cin, cout, slots, nullptr, gout, ld_out, w, gin, ld_in, nullptr, gtree, ld_tree,
+                                                  fold_tree, nullptr, ws.p, st);
+}
+
+int backward_weights_f32(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* in, ll ld_in, const float* tree, ll ld_tree, const float* gout, ll ld_out,
+                         float* gw, float* partial, cudaStream_t st) {
+    StreamScratch rows(st), ws(st);
+    int rc;
+    if ((rc = rows.get((size_t) aprnet_conv333_rows_bytes(a, dl, APRNET_PREC_F32, cin)))) return rc;
+    if ((rc = ws.get((size_t) aprnet_conv333_rows_backward_workspace_bytes(a, dl, APRNET_PREC_F32, cin, cout, slots, 0)))) return rc;
+    if ((rc = aprnet_conv333_rows_pack(a, dl, APRNET_PREC_F32, cin, in, ld_in, const_cast<float*>(tree), ld_tree, 1, rows.p, st))) return rc;
+    return aprnet_conv333_rows_backward(a, dl, APRNET_PREC_F32, cin, cout, slots, rows.p, gout, ld_out, nullptr, nullptr, 0, gw, const_cast<float*>(tree), ld_tree,
+                                        0, partial, ws.p, st);
+}
+
+} // namespace
+
 extern "C" int aprnet_conv333_forward(aprnet_apr* a, int dl, int dtype, int cin, int cout, int slots, const void* in,
                                       int64_t ld_in, const void* w, void* out, int64_t ld_out, void* tree, int64_t ld_tree,
                                       void* stream) {
     CONV_CHECKS();
     APRNET_ARG_CHECK(in && w && out && tree, "null pointer");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, conv333_fwd<float>(a, dl, cin, cout, slots, (const float*) in, ld_in, (const float*) w, (float*) out, ld_out, (float*) tree, ld_tree, st),
+    DISPATCH(dtype, forward_f32(a, dl, cin, cout, slots, (const float*) in, ld_in, (const float*) w, (float*) out, ld_out, (float*) tree, ld_tree, 0, st),
              conv333_fwd<double>(a, dl, cin, cout, slots, (const double*) in, ld_in, (const double*) w, (double*) out, ld_out, (double*) tree, ld_tree, st));
 }
 
@@ -534,7 +551,7 @@ extern "C" int aprnet_conv333_backward_input(aprnet_apr* a, int dl, int dtype, i
     CONV_CHECKS();
     APRNET_ARG_CHECK(gout && w && gin && gtree, "null pointer");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, conv333_bwd_input<float>(a, dl, cin, cout, slots, (const float*) gout, ld_out, (const float*) w, (float*) gin, ld_in, (float*) gtree, ld_tree, st),
+    DISPATCH(dtype, backward_input_f32(a, dl, cin, cout, slots, (const float*) gout, ld_out, (const float*) w, (float*) gin, ld_in, (float*) gtree, ld_tree, 1, st),
              conv333_bwd_input<double>(a, dl, cin, cout, slots, (const double*) gout, ld_out, (const double*) w, (double*) gin, ld_in, (double*) gtree, ld_tree, st));
 }
 
@@ -546,7 +563,7 @@ extern "C" int aprnet_conv333_forward_pretree(aprnet_apr* a, int dl, int dtype, 
     CONV_CHECKS();
     APRNET_ARG_CHECK(in && w && out && tree, "null pointer");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, conv333_fwd<float>(a, dl, cin, cout, slots, (const float*) in, ld_in, (const float*) w, (float*) out, ld_out, (float*) tree, ld_tree, st, true),
+    DISPATCH(dtype, forward_f32(a, dl, cin, cout, slots, (const float*) in, ld_in, (const float*) w, (float*) out, ld_out, (float*) tree, ld_tree, 1, st),
              conv333_fwd<double>(a, dl, cin, cout, slots, (const double*) in, ld_in, (const double*) w, (double*) out, ld_out, (double*) tree, ld_tree, st, true));
 }
 
@@ -556,11 +573,11 @@ extern "C" int aprnet_conv333_backward_input_pretree(aprnet_apr* a, int dl, int 
     CONV_CHECKS();
     APRNET_ARG_CHECK(gout && w && gin && gtree, "null pointer");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, conv333_bwd_input<float>(a, dl, cin, cout, slots, (const float*) gout, ld_out, (const float*) w, (float*) gin, ld_in, (float*) gtree, ld_tree, st, 0, false),
+    DISPATCH(dtype, backward_input_f32(a, dl, cin, cout, slots, (const float*) gout, ld_out, (const float*) w, (float*) gin, ld_in, (float*) gtree, ld_tree, 0, st),
              conv333_bwd_input<double>(a, dl, cin, cout, slots, (const double*) gout, ld_out, (const double*) w, (double*) gin, ld_in, (double*) gtree, ld_tree, st, 0, false));
 }
 
-extern "C" int64_t aprnet_conv333_partial_elems(int cin, int cout) { return (int64_t) dw_max_ranges(cin, cout) * 27 * cin * cout; }
+extern "C" int64_t aprnet_conv333_partial_elems(int cin, int cout) { return std::max<int64_t>((int64_t) dw_max_ranges(cin, cout) * 27 * cin * cout, aprnet_conv333_rows_partial_elems(APRNET_PREC_F32, cin, cout)); }
 
 extern "C" int aprnet_conv333_backward_weights(aprnet_apr* a, int dl, int dtype, int cin, int cout, int slots, const void* in,
                                                int64_t ld_in, const void* tree, int64_t ld_tree, const void* gout,
@@ -568,7 +585,7 @@ extern "C" int aprnet_conv333_backward_weights(aprnet_apr* a, int dl, int dtype,
     CONV_CHECKS();
     APRNET_ARG_CHECK(in && tree && gout && gw && partial, "null pointer");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, conv333_bwd_weights<float>(a, dl, cin, cout, slots, (const float*) in, ld_in, (const float*) tree, ld_tree, (const float*) gout, ld_out, (float*) gw, (float*) partial, st),
+    DISPATCH(dtype, backward_weights_f32(a, dl, cin, cout, slots, (const float*) in, ld_in, (const float*) tree, ld_tree, (const float*) gout, ld_out, (float*) gw, (float*) partial, st),
              conv333_bwd_weights<double>(a, dl, cin, cout, slots, (const double*) in, ld_in, (const double*) tree, ld_tree, (const double*) gout, ld_out, (double*) gw, (double*) partial, st));
 }
 

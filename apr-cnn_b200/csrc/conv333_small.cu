@@ -1,5 +1,5 @@
 // 3x3x3 convolution for very few input channels (Cin <= 4: the first layer of a network) on CUDA cores,
-// fp32, used by the tensor-core drivers instead of the implicit GEMM: with Cin = 1 a packed bf16 row would
+// fp32, used in either arithmetic instead of the implicit GEMM: with Cin = 1 a packed bf16 row would
 // carry one useful value in 32 bytes and the 27 x Cin x Cout products per location are far too few to
 // amortise a gathered operand tile.  Values are read from a channel-major buffer
 //     vals[ci][r],  r in [0, N) particles, [N, N + T) tree means, r = N + T: zero
@@ -52,7 +52,7 @@ __global__ void small_stage_kernel(const float* __restrict__ x, ll ld_x, ll n, c
 template<int CIN>
 __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable segs, const int32_t* __restrict__ nbr, ll N, ll T,
                                                                     const float* __restrict__ vals, const float* __restrict__ w,
-                                                                    int cout, float* __restrict__ out, ll ld_out) {
+                                                                    int cout, const float* __restrict__ bias, float* __restrict__ out, ll ld_out) {
     __shared__ F4 ws[27 * CIN * 8];
     int seg = 0;
     while (seg + 1 < segs.n && (int) blockIdx.x >= segs.tile_begin[seg + 1]) ++seg;
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable seg
     }
 #pragma unroll
     for (int o = 0; o < 32; ++o)
-        if (co0 + o < cout) out[(ll) (co0 + o) * ld_out + p] = acc[o];
+        if (co0 + o < cout) out[(ll) (co0 + o) * ld_out + p] = bias ? acc[o] + __ldg(bias + co0 + o) : acc[o];
 }
 
 // weight gradient of one level: block = range of locations x block of 32 output channels.  The 27 x CIN
@@ -196,7 +196,7 @@ int aprnet_small_stage(const float* x, ll ld_x, ll n, const float* tree, ll ld_t
     return APRNET_OK;
 }
 
-int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, float* out, ll ld_out, cudaStream_t st) {
+int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, const float* bias, float* out, ll ld_out, cudaStream_t st) {
     const AprPlan* plan = aprnet_get_plan(a, dl, st);
     if (!plan) return APRNET_ERR_CUDA;
     const SegTable segs = make_seg_table(aprnet_segments(a, dl, slots, false), 128);
@@ -207,10 +207,10 @@ int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, co
     snprintf(pname, sizeof(pname), "conv333_small_fwd:ci%d:co%d:dl%d", cin, cout, dl);
     AprnetProfScope _prof(pname, st);
     switch (cin) {
-        case 1: conv333_small_forward_kernel<1><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, out, ld_out); break;
-        case 2: conv333_small_forward_kernel<2><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, out, ld_out); break;
-        case 3: conv333_small_forward_kernel<3><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, out, ld_out); break;
-        case 4: conv333_small_forward_kernel<4><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, out, ld_out); break;
+        case 1: conv333_small_forward_kernel<1><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
+        case 2: conv333_small_forward_kernel<2><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
+        case 3: conv333_small_forward_kernel<3><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
+        case 4: conv333_small_forward_kernel<4><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
         default: aprnet_set_error("small-Cin path called with cin = %d", cin); return APRNET_ERR_ARG;
     }
     APRNET_LAUNCH_CHECK();

@@ -131,6 +131,7 @@ struct TcParams {
     ll tree_base, zero_row;                // row index of tree node 0 and of the zero row
     const __nv_bfloat16* wp;               // packed weights
     float* out; ll ld_out; int n_dim;      // output (n_dim, ld_out)
+    const float* bias;                     // added to every output channel (null: none)
     int n_tiles;
     int same_level_only;                   // input-gradient mode: mask entries outside the tile's level
     int* error_flag;
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
 #pragma unroll
                     for (int jj = 0; jj < 32; ++jj) {
                         const int n = ti.ntile * NT + c0 + jj;
-                        if (n < P.n_dim) P.out[(ll) n * P.ld_out + p] = __uint_as_float(r[jj]);
+                        if (n < P.n_dim) P.out[(ll) n * P.ld_out + p] = P.bias ? __uint_as_float(r[jj]) + __ldg(P.bias + n) : __uint_as_float(r[jj]);
                     }
                 } else if (valid) {          // this thread is the only writer of its target: read all, then add and write
 #pragma unroll
@@ -613,7 +614,7 @@ int aprnet_tc_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_
 // Gather-GEMM over packed rows.  backward == 0: out[n = co] from rows of the input (k = ci);
 // backward == 1: out[n = ci] from rows of grad_output (k = co), same-level neighbours only, mirrored taps.
 int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout, int slots, const void* rows, int kpad,
-                          ll tree_base, ll zero_row, const float* w, void* wp_ws, float* out, ll ld_out, cudaStream_t st) {
+                          ll tree_base, ll zero_row, const float* w, void* wp_ws, const float* bias, float* out, ll ld_out, cudaStream_t st) {
     int rc = ensure_error_flag();
     if (rc) return rc;
     if (*g_error_flag_host) { aprnet_set_error("a previous tensor-core kernel gave up waiting on a barrier"); return APRNET_ERR_CUDA; }
@@ -632,7 +633,7 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
     P.segs = make_seg_table(aprnet_segments(a, dl, slots, false), TILE_M);
     P.nbr = plan->nbr; P.N = plan->n; P.rows = reinterpret_cast<const __nv_bfloat16*>(rows); P.kpad = g.kpad;
     P.tree_base = tree_base; P.zero_row = zero_row;
-    P.wp = wp; P.out = out; P.ld_out = ld_out; P.n_dim = n_dim; P.n_tiles = g.n_tiles; P.same_level_only = backward;
+    P.wp = wp; P.out = out; P.ld_out = ld_out; P.bias = bias; P.n_dim = n_dim; P.n_tiles = g.n_tiles; P.same_level_only = backward;
     P.error_flag = g_error_flag_dev;
     P.out_map = nullptr; P.out_split = 0; P.out2 = nullptr; P.ld_out2 = 0;
 
@@ -750,111 +751,3 @@ extern "C" int64_t aprnet_conv333_tc_forward_workspace_bytes(const aprnet_apr* a
     return (int64_t) (aprnet_tc_rows_bytes(a->number_parts(dl) + a->tree_size(dl) + 1, cin) + aprnet_tc_weight_bytes(cin, cout, slots));
 }
 
-// forward: out = conv(in) with bf16 operands / fp32 accumulation; tree_scratch receives the fp32 tree means
-static int conv333_forward_tc_impl(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* in, int64_t ld_in,
-                                   const float* w, float* out, int64_t ld_out, float* tree, int64_t ld_tree,
-                                   void* workspace, void* stream, bool tree_valid) {
-    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && in && w && out && tree && workspace, "bad argument");
-    APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), "leading dimension too small");
-    cudaStream_t st = (cudaStream_t) stream;
-    int rc = tree_valid ? APRNET_OK : aprnet_fill_tree_mean_forward(a, dl, APRNET_F32, cin, in, ld_in, tree, ld_tree, st);
-    if (rc) return rc;
-    const ll n = a->number_parts(dl), t = a->tree_size(dl);
-    const int kpad = aprnet_tc_pad(cin);
-    char* ws = (char*) workspace;
-    void* rows = ws;
-    void* wp = ws + aprnet_tc_rows_bytes(n + t + 1, cin);
-    if (aprnet_small_cin(cin)) {         // first-layer widths: fp32 CUDA-core kernels; the rows area holds the fp32 staging buffer instead
-        if ((rc = aprnet_small_stage(in, ld_in, n, tree, ld_tree, t, cin, (float*) rows, st))) return rc;
-        return aprnet_small_forward(a, dl, cin, cout, slots, (const float*) rows, w, out, ld_out, st);
-    }
-    rc = aprnet_tc_pack_rows(in, ld_in, n, tree, ld_tree, t, cin, kpad, rows, st);
-    if (rc) return rc;
-    return aprnet_tc_gather_conv(a, dl, 0, cin, cout, slots, rows, kpad, n, n + t, w, wp, out, ld_out, st);
-}
-
-extern "C" int aprnet_conv333_forward_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* in, int64_t ld_in,
-                                         const float* w, float* out, int64_t ld_out, float* tree, int64_t ld_tree,
-                                         void* workspace, void* stream) {
-    return conv333_forward_tc_impl(a, dl, cin, cout, slots, in, ld_in, w, out, ld_out, tree, ld_tree, workspace, stream, false);
-}
-
-// Split form (see aprnet_conv333_forward_pretree): the tree means are taken as given.
-extern "C" int aprnet_conv333_forward_tc_pretree(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* in, int64_t ld_in,
-                                                 const float* w, float* out, int64_t ld_out, const float* tree, int64_t ld_tree,
-                                                 void* workspace, void* stream) {
-    return conv333_forward_tc_impl(a, dl, cin, cout, slots, in, ld_in, w, out, ld_out, const_cast<float*>(tree), ld_tree, workspace, stream, true);
-}
-
-// Backward pass of the 3x3x3 convolution with the contractions on the tensor cores, from the packed
-// bf16 rows of the input that the forward call left at the start of its workspace
-// (aprnet_conv333_tc_packed_rows_bytes() bytes: particles, tree means, zero row; for Cin <= 4 the same
-// area holds an fp32 channel-major copy instead, see conv333_small.cu): nothing of the fp32 input is needed.  grad_weights is accumulated into, grad_input (float32 (Cin, ld_in)) written; null: skipped.
-//   packed dO rows -> weight gradient (tcgen05, deterministic) -> same-level input gradient (tcgen05 gather)
-//   -> cross-level part (per-(target, tap) sums + gather over the targets) and tree adjoint.
-// workspace: aprnet_conv333_tc_workspace_bytes() bytes (its leading part is not touched, so the forward
-// workspace itself may be passed as packed_input_rows).
-static int conv333_backward_tc_rows_impl(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* packed_input_rows,
-                                         const float* gout, int64_t ld_out, const float* w, float* gin, int64_t ld_in, float* gw,
-                                         float* gtree, int64_t ld_tree, float* partial, void* workspace, void* stream, bool tree_adjoint) {
-    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && packed_input_rows && gout && w && gw && gtree && partial && workspace, "bad argument");
-    APRNET_ARG_CHECK(ld_out >= a->number_parts(dl) && (!gin || ld_in >= a->number_parts(dl)) && ld_tree >= a->tree_size(dl), "leading dimension too small");
-    cudaStream_t st = (cudaStream_t) stream;
-    const ll n = a->number_parts(dl), t = a->tree_size(dl);
-    const int xpad = aprnet_tc_pad(cin), gpad = aprnet_tc_pad(cout);
-    char* ws = (char*) workspace;
-    void* grows = ws + aprnet_tc_rows_bytes(n + t + 1, cin);
-    void* wp = (char*) grows + aprnet_tc_rows_bytes(n + 1, cout);
-    int rc;
-    if (!(aprnet_small_cin(cin) && !gin) && (rc = aprnet_tc_pack_rows(gout, ld_out, n, nullptr, 0, 0, cout, gpad, grows, st))) return rc;
-    if (aprnet_small_cin(cin)) {
-        if ((rc = aprnet_small_backward_weights(a, dl, cin, cout, slots, (const float*) packed_input_rows, gout, ld_out, gw, partial, st))) return rc;
-    } else if ((rc = aprnet_conv333_backward_weights_tc(a, dl, cin, cout, slots, packed_input_rows, xpad, grows, gpad, gw, partial, st))) return rc;
-    if (!gin) return APRNET_OK;          // the caller does not need the input gradient (first layer of a network)
-    if ((rc = aprnet_tc_gather_conv(a, dl, 1, cin, cout, slots, grows, gpad, n, n, w, wp, gin, ld_in, st))) return rc;
-    void* edge_ws = (char*) wp + aprnet_tc_weight_bytes(cout, cin, slots);
-    if (27 * n + 1 >= (1ll << 31)) {
-        // more than 79.5 M locations: the 32-bit edge ids of the edge plan run out.  The cross-level part then runs on the
-        // fp32 scatter kernel (atomic adds: correct, but the summation order is no longer fixed).
-        if (!tree_adjoint) { aprnet_set_error("the split backward form needs the edge plan, which supports up to 79.5 M locations"); return APRNET_ERR_UNSUPPORTED; }
-        return aprnet_conv333_backward_input_cross_level(a, dl, APRNET_F32, cin, cout, slots, gout, ld_out, w, gin, ld_in, gtree, ld_tree, stream);
-    }
-    return aprnet_cross_level_tc(a, dl, cin, cout, slots, grows, gpad, w, gin, ld_in, gtree, ld_tree, wp, edge_ws,
-                                 aprnet_edge_workspace_bytes(a, dl, cout), st, tree_adjoint);
-}
-
-extern "C" int aprnet_conv333_backward_tc_rows(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* packed_input_rows,
-                                               const float* gout, int64_t ld_out, const float* w, float* gin, int64_t ld_in, float* gw,
-                                               float* gtree, int64_t ld_tree, float* partial, void* workspace, void* stream) {
-    return conv333_backward_tc_rows_impl(a, dl, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, gtree, ld_tree, partial, workspace, stream, true);
-}
-
-// Split form: grad_input holds the direct contributions only and grad_tree the gradient of the tree means; the
-// caller folds them with aprnet_fill_tree_mean_backward after it has exchanged the halo parts.
-extern "C" int aprnet_conv333_backward_tc_rows_pretree(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* packed_input_rows,
-                                                       const float* gout, int64_t ld_out, const float* w, float* gin, int64_t ld_in, float* gw,
-                                                       float* gtree, int64_t ld_tree, float* partial, void* workspace, void* stream) {
-    return conv333_backward_tc_rows_impl(a, dl, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, gtree, ld_tree, partial, workspace, stream, false);
-}
-
-extern "C" int64_t aprnet_conv333_tc_packed_rows_bytes(const aprnet_apr* a, int dl, int cin) {
-    if (!a || !a->valid_dl(dl)) return -1;
-    return (int64_t) aprnet_tc_rows_bytes(a->number_parts(dl) + a->tree_size(dl) + 1, cin);
-}
-
-// Complete backward pass from the fp32 input: fills the tree means (unless tree_valid), packs the input
-// rows into the workspace and continues as aprnet_conv333_backward_tc_rows.
-extern "C" int aprnet_conv333_backward_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* in, int64_t ld_in,
-                                          const float* gout, int64_t ld_out, const float* w, float* gin, float* gw,
-                                          float* tree, int tree_valid, float* gtree, int64_t ld_tree, float* partial,
-                                          void* workspace, void* stream) {
-    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && in && gout && w && gw && tree && gtree && partial && workspace, "bad argument");
-    APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), "leading dimension too small");
-    cudaStream_t st = (cudaStream_t) stream;
-    int rc = tree_valid ? APRNET_OK : aprnet_fill_tree_mean_forward(a, dl, APRNET_F32, cin, in, ld_in, tree, ld_tree, st);
-    if (rc) return rc;
-    const ll n = a->number_parts(dl), t = a->tree_size(dl);
-    if (aprnet_small_cin(cin)) { if ((rc = aprnet_small_stage(in, ld_in, n, tree, ld_tree, t, cin, (float*) workspace, st))) return rc; }
-    else if ((rc = aprnet_tc_pack_rows(in, ld_in, n, tree, ld_tree, t, cin, aprnet_tc_pad(cin), workspace, st))) return rc;
-    return aprnet_conv333_backward_tc_rows(a, dl, cin, cout, slots, workspace, gout, ld_out, w, gin, ld_in, gw, gtree, ld_tree, partial, workspace, stream);
-}

@@ -1,0 +1,41 @@
+// Entries behind the valid ones of a padded batch: (batch, channels, ld) tensors whose items hold fewer than ld locations.
+#include "apr_device.cuh"
+#include <algorithm>
+
+namespace {
+
+typedef long long ll;
+constexpr int ITEMS = 64;             // batch items per launch (their sizes travel as kernel arguments)
+
+struct Valid { ll n[ITEMS]; };
+
+// One launch for all items and channels; HBM-bound by the bytes written.  (A strided fill per item and tensor, from the host,
+// took 2.4 of the 36.8 ms of a forward pass over four images of 0.3 to 1.8 M particles.)
+template<typename T>
+__global__ void __launch_bounds__(256) fill_padding_kernel(Valid valid, int channels, ll ld, const T* __restrict__ bias, T* __restrict__ out) {
+    const int b = blockIdx.z, c = blockIdx.y;
+    const T v = bias ? bias[c] : T(0);
+    T* row = out + ((ll) b * channels + c) * ld;
+    for (ll i = valid.n[b] + (ll) blockIdx.x * 256 + threadIdx.x; i < ld; i += (ll) gridDim.x * 256) row[i] = v;
+}
+
+} // namespace
+
+extern "C" int aprnet_fill_padding(int dtype, int batch, int channels, int64_t ld, const int64_t* host_valid, const void* bias, void* out, void* stream) {
+    APRNET_ARG_CHECK(batch > 0 && channels > 0 && channels <= 65535 && ld >= 0 && host_valid && out, "bad argument");
+    APRNET_ARG_CHECK(dtype == APRNET_F32 || dtype == APRNET_F64, "unknown dtype");
+    for (int b0 = 0; b0 < batch; b0 += ITEMS) {
+        const int nb = std::min(ITEMS, batch - b0);
+        Valid v;
+        ll most = 0;
+        for (int b = 0; b < nb; ++b) { v.n[b] = host_valid[b0 + b]; most = std::max<ll>(most, ld - v.n[b]); }
+        if (most <= 0) continue;
+        const dim3 grid((unsigned) std::min<ll>(1024, (most + 2047) / 2048), (unsigned) channels, (unsigned) nb);
+        const ll off = (ll) b0 * channels * ld;
+        AprnetProfScope _prof("fill_padding", (cudaStream_t) stream);
+        if (dtype == APRNET_F32) fill_padding_kernel<float><<<grid, 256, 0, (cudaStream_t) stream>>>(v, channels, ld, (const float*) bias, (float*) out + off);
+        else fill_padding_kernel<double><<<grid, 256, 0, (cudaStream_t) stream>>>(v, channels, ld, (const double*) bias, (double*) out + off);
+    }
+    APRNET_LAUNCH_CHECK();
+    return APRNET_OK;
+}

@@ -26,19 +26,19 @@ class Conv333Function(Function):
         expanded = restrict_kernel333_forward(weights, num_levels)
         ctx.aprs = aprs
         ctx.num_stencils = weights.shape[0]
-        # arithmetic of this layer: the module's own setting, else the process-wide one
-        ctx.packed = (precision or get_conv_precision()) == "bf16" and inputs.dtype == torch.float32
+        # float32: the backward pass works from the packed rows of the input (particles + tree means, bf16 or fp32 as the
+        # layer's arithmetic wants them) that the forward pass produced anyway; they replace the input among the saved
+        # tensors and spare the backward pass the tree fill and the packing.  The bias is added where the output is written.
+        ctx.packed = inputs.dtype == torch.float32
         if ctx.packed:
-            # tensor-core path: the backward pass works from the packed bf16 rows of the input (particles + tree
-            # means) that the forward pass produced anyway; they replace the fp32 input among the saved tensors
-            # (half the bytes) and spare the backward pass the tree fill and the packing
-            out, rows = conv333_forward_keep_rows(APRPtrVector(aprs), inputs, expanded, level_deltas)
+            ctx.precision = precision or get_conv_precision()
+            out, rows = conv333_forward_keep_rows(APRPtrVector(aprs), inputs, expanded, level_deltas, ctx.precision, bias)
             ctx.save_for_backward(expanded, bias, level_deltas.clone(), rows)
-        else:
-            # the tree means computed by the forward pass are kept (1/7 of the input's size) so that the
-            # backward pass does not have to fill the tree again
-            out, tree = conv333_forward_keep_tree(APRPtrVector(aprs), inputs, expanded, level_deltas, "fp32")
-            ctx.save_for_backward(inputs, expanded, bias, level_deltas.clone(), tree)
+            return out
+        # float64: the tree means computed by the forward pass are kept (1/7 of the input's size) so that the
+        # backward pass does not have to fill the tree again
+        out, tree = conv333_forward_keep_tree(APRPtrVector(aprs), inputs, expanded, level_deltas)
+        ctx.save_for_backward(inputs, expanded, bias, level_deltas.clone(), tree)
         if bias is not None:
             out = out + bias.view(1, -1, 1)
         return out
@@ -49,14 +49,12 @@ class Conv333Function(Function):
         if ctx.packed:
             expanded, bias, level_deltas, rows = ctx.saved_tensors
             grad_input, grad_expanded = conv333_backward_with_rows(APRPtrVector(ctx.aprs), rows, expanded, grad_output, level_deltas,
-                                                                   bool(ctx.needs_input_grad[0]))
+                                                                   bool(ctx.needs_input_grad[0]), ctx.precision)
             grad_weights = restrict_kernel333_backward(grad_expanded, ctx.num_stencils)
             grad_bias = grad_output.sum(dim=(0, 2)) if bias is not None else None
             return grad_input, grad_weights, grad_bias, None, None, None
         inputs, expanded, bias, level_deltas, tree = ctx.saved_tensors
-        # the input gradient of a first layer (features that do not require grad) is not computed
-        grad_input, grad_expanded = conv333_backward_with_tree(APRPtrVector(ctx.aprs), inputs, expanded, grad_output, level_deltas, tree,
-                                                               bool(ctx.needs_input_grad[0]), "fp32")
+        grad_input, grad_expanded = conv333_backward_with_tree(APRPtrVector(ctx.aprs), inputs, expanded, grad_output, level_deltas, tree)
         grad_weights = restrict_kernel333_backward(grad_expanded, ctx.num_stencils)
         grad_bias = grad_output.sum(dim=(0, 2)) if bias is not None else None
         return grad_input, grad_weights, grad_bias, None, None, None

@@ -31,6 +31,10 @@ extern "C" {
 #define APRNET_F32 0
 #define APRNET_F64 1
 
+/* arithmetic of a 3x3x3 convolution on float32 tensors */
+#define APRNET_PREC_F32 0        /* exact fp32 multiply-adds on the CUDA cores */
+#define APRNET_PREC_BF16 1       /* bf16 operands, fp32 accumulation, on the tensor cores */
+
 #define APRNET_OK 0
 #define APRNET_ERR_ARG (-1)      /* bad argument (null pointer, level_delta out of range, size mismatch) */
 #define APRNET_ERR_CUDA (-2)     /* a CUDA runtime call failed; aprnet_last_error() has the text */
@@ -83,6 +87,10 @@ int aprnet_plan_build(aprnet_apr* apr, int level_delta, void* stream);
 /* Test hooks: copy the cached tables to host memory.  nbr: int32[27][N]; child: int32[8][T]. */
 int aprnet_plan_copy_nbr_table(aprnet_apr* apr, int level_delta, int32_t* host_out);
 int aprnet_copy_child_table(aprnet_apr* apr, int32_t* host_out);
+
+/* out[b][c][i] = bias[c] (0 for a null bias) for host_valid[b] <= i < ld: the entries behind the valid ones of every batch
+ * item of a contiguous (batch, channels, ld) tensor. */
+int aprnet_fill_padding(int dtype, int batch, int channels, int64_t ld, const int64_t* host_valid, const void* bias, void* out, void* stream);
 
 /* ---- tree fill -------------------------------------------------------------------------------
  * pyapr/aprnet/cuda/src/fill_tree_gpu.hpp:15-32 (apply_fill_tree_mean / _backward); arithmetic of
@@ -145,6 +153,30 @@ int aprnet_conv333_backward_input_pretree(aprnet_apr* apr, int level_delta, int 
                                           const void* grad_output, int64_t ld_out, const void* weights,
                                           void* grad_input, int64_t ld_in, void* grad_tree, int64_t ld_tree,
                                           void* stream);
+
+/* ---- 3x3x3 convolution over packed rows, in either arithmetic (float32 tensors) -----------------
+ * The forward call leaves the packed rows of the input (particles, tree means, zero row;
+ * aprnet_conv333_rows_bytes() bytes) at the start of its workspace; they are all that the backward call needs of the
+ * input.  bias: (Cout) floats added to the output, or NULL.  tree: (Cin, ld_tree), filled by the call unless
+ * tree_is_valid.  aprnet_conv333_rows_pack writes the packed rows alone. */
+int64_t aprnet_conv333_rows_bytes(const aprnet_apr* apr, int level_delta, int precision, int cin);
+int64_t aprnet_conv333_rows_forward_workspace_bytes(const aprnet_apr* apr, int level_delta, int precision, int cin, int cout, int num_slots);
+int aprnet_conv333_rows_forward(aprnet_apr* apr, int level_delta, int precision, int cin, int cout, int num_slots,
+                                const float* input, int64_t ld_in, const float* weights, const float* bias,
+                                float* output, int64_t ld_out, float* tree, int64_t ld_tree, int tree_is_valid,
+                                void* workspace, void* stream);
+int aprnet_conv333_rows_pack(aprnet_apr* apr, int level_delta, int precision, int cin, const float* input, int64_t ld_in,
+                             float* tree, int64_t ld_tree, int tree_is_valid, void* packed_rows, void* stream);
+/* grad_input (Cin, ld_in) is written (NULL: not computed); grad_weights (num_slots, Cout, Cin, 27) is accumulated into
+ * (NULL: not computed; deterministic); grad_tree (Cin, ld_tree) is zero-filled, receives the gradient of the tree means and, with
+ * fold_tree, is folded into grad_input.  partial: aprnet_conv333_rows_partial_elems() floats. */
+int64_t aprnet_conv333_rows_backward_workspace_bytes(const aprnet_apr* apr, int level_delta, int precision, int cin, int cout, int num_slots,
+                                                     int with_grad_input);
+int64_t aprnet_conv333_rows_partial_elems(int precision, int cin, int cout);
+int aprnet_conv333_rows_backward(aprnet_apr* apr, int level_delta, int precision, int cin, int cout, int num_slots,
+                                 const void* packed_rows, const float* grad_output, int64_t ld_out, const float* weights,
+                                 float* grad_input, int64_t ld_in, float* grad_weights, float* grad_tree, int64_t ld_tree,
+                                 int fold_tree, float* partial, void* workspace, void* stream);
 
 /* ---- 3x3x3 convolution on the tensor cores (bf16 operands, fp32 accumulation) ------------------
  * No counterpart in the reference (its kernels are CUDA-core only).  Same contract as
