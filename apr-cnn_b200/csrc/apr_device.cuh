@@ -57,6 +57,15 @@ struct EdgePlan {
     std::vector<long long> chunk_a, chunk_v;
 };
 
+// Output locations of a level delta in runs along y (run_plan.cu): slot s is a cell of its level, loc[s] the location it holds
+// (-1: none), src[d][s] what fills the cell (dz, dx) = (d / 3 - 1, d % 3 - 1) away (encoded like the neighbour table).
+struct RunPlan {
+    long long n_slots = 0;
+    std::vector<long long> level_begin;      // first slot of each level ([l + 1] = end of l)
+    int32_t* loc = nullptr;                  // [n_slots]
+    int32_t* src = nullptr;                  // [9][n_slots]
+};
+
 struct aprnet_apr {
     int device = 0;
     LevelMeta meta;
@@ -69,6 +78,7 @@ struct aprnet_apr {
     float* tree_scale = nullptr;         // [n_tree] weight of each child in its parent's mean
     std::map<int, AprPlan> plans;
     std::map<int, EdgePlan> edge_plans;
+    std::map<int, RunPlan> run_plans;
     // parent tree node of every tree node (-1: none) and, per level delta, of every feature location (particle or
     // upgraded node); built on first use by the tree-mean adjoint (aprnet_node_parent_table / aprnet_loc_parent_table)
     mutable int32_t* node_parent = nullptr;
@@ -138,6 +148,7 @@ extern "C" int aprnet_conv333_backward_input_cross_level(aprnet_apr* a, int dl, 
                                                          const void* gout, int64_t ld_out, const void* w, void* gin,
                                                          int64_t ld_in, void* gtree, int64_t ld_tree, void* stream);
 
+const RunPlan* aprnet_get_run_plan(aprnet_apr* apr, int dl, cudaStream_t stream);                // nullptr on failure
 EdgePlan* aprnet_get_edge_plan(aprnet_apr* apr, int dl, cudaStream_t stream);
 void aprnet_free_edge_plan(EdgePlan& ep);
 // gather GEMM over the active targets [a0, a1) of an edge plan: grad[target] += sum over taps of
@@ -152,6 +163,10 @@ int aprnet_small_stage(const float* x, long long ld_x, long long n, const float*
 int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, const float* bias, float* out, long long ld_out, cudaStream_t st);
 int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* gout, long long ld_out,
                                   float* gw, float* partial, cudaStream_t st);
+// tensor-core gather over runs (conv333_tc_runs.cu)
+int aprnet_tc_runs_order(int backward, int kpad, int nt, int ks);
+int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, long long tree_base, long long zero_row, const void* wp,
+                       const float* bias, float* out, long long ld_out, int n_dim, int* error_flag, cudaStream_t st, const char* pname);
 int aprnet_tc_pack_weights(const float* w, int slots, int cin, int cout, int mode, void* wp, cudaStream_t st);
 size_t aprnet_tc_weight_bytes(int k_dim, int n_dim, int slots);
 size_t aprnet_tc_rows_bytes(long long rows, int channels);

@@ -299,6 +299,7 @@ extern "C" void aprnet_apr_destroy(aprnet_apr* a) {
     cudaFree(a->node_parent);
     for (auto& kv : a->loc_parent) cudaFree(kv.second);
     for (auto& kv : a->edge_plans) aprnet_free_edge_plan(kv.second);
+    for (auto& kv : a->run_plans) { cudaFree(kv.second.loc); cudaFree(kv.second.src); }
     delete a;
     if (prev >= 0) cudaSetDevice(prev);
 }

@@ -393,11 +393,18 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
                 uint32_t r[32];
                 tmem_ld32(tmem_d + ((uint32_t) (q * 32) << 16) + acc * NT + c0, r);
                 tmem_ld_wait();
+                if (P.bias) {                // apart from the stores: a choice per element there cost the whole kernel 10 to 20 %
+#pragma unroll
+                    for (int jj = 0; jj < 32; ++jj) {
+                        const int n = ti.ntile * NT + c0 + jj;
+                        if (n < P.n_dim) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + __ldg(P.bias + n));
+                    }
+                }
                 if (valid && !P.out_map) {
 #pragma unroll
                     for (int jj = 0; jj < 32; ++jj) {
                         const int n = ti.ntile * NT + c0 + jj;
-                        if (n < P.n_dim) P.out[(ll) n * P.ld_out + p] = P.bias ? __uint_as_float(r[jj]) + __ldg(P.bias + n) : __uint_as_float(r[jj]);
+                        if (n < P.n_dim) P.out[(ll) n * P.ld_out + p] = __uint_as_float(r[jj]);
                     }
                 } else if (valid) {          // this thread is the only writer of its target: read all, then add and write
 #pragma unroll
@@ -453,6 +460,7 @@ inline int pick_nt(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 12
 
 struct TcGeom { int kpad, ks, nt, n_tiles; size_t rows_bytes, w_bytes; };
 
+int g_runs_off = 0;          // aprnet_tc_set_option("runs", 0 / 1): 0 = always this file's kernel, measurement switch
 int g_ks_override = 0;       // aprnet_tc_set_option("ks", n): channels per stage, measurement switch
 
 TcGeom tc_geometry(ll rows, int k_dim, int n_dim, int slots) {
@@ -629,6 +637,10 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
         w, slots, cin, cout, backward, n_dim, k_dim, g.nt, g.n_tiles, g.kpad, wp);
     }
     APRNET_LAUNCH_CHECK();
+    char pname[64];
+    snprintf(pname, sizeof(pname), "%s:ci%d:co%d:dl%d", backward ? "conv333_tc_bwd_gather" : "conv333_tc_fwd", cin, cout, dl);
+    const int run_order = g_runs_off ? 0 : aprnet_tc_runs_order(backward, g.kpad, g.nt, g.ks);
+    if (run_order) return aprnet_tc_run_conv(a, dl, backward, slots, g.nt, run_order, rows, g.kpad, tree_base, zero_row, wp, bias, out, ld_out, n_dim, g_error_flag_dev, st, pname);
     TcParams P;
     P.segs = make_seg_table(aprnet_segments(a, dl, slots, false), TILE_M);
     P.nbr = plan->nbr; P.N = plan->n; P.rows = reinterpret_cast<const __nv_bfloat16*>(rows); P.kpad = g.kpad;
@@ -639,8 +651,6 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
 
     const int total = P.segs.tile_begin[P.segs.n] * g.n_tiles;
     if (total == 0) return APRNET_OK;
-    char pname[64];
-    snprintf(pname, sizeof(pname), "%s:ci%d:co%d:dl%d", backward ? "conv333_tc_bwd_gather" : "conv333_tc_fwd", cin, cout, dl);
     return dispatch_tc(P, g, total, st, pname);
 }
 
@@ -726,6 +736,7 @@ extern "C" int aprnet_tc_set_option(const char* name, int value) {
     if (!strcmp(name, "wps")) { g_wps_override = value; return APRNET_OK; }
     if (!strcmp(name, "tma_taps")) { g_tma_taps_override = value; return APRNET_OK; }
     if (!strcmp(name, "dw_waves")) { g_dw_waves_override = value; return APRNET_OK; }
+    if (!strcmp(name, "runs")) { g_runs_off = value == 0; return APRNET_OK; }
     if (!strcmp(name, "ks")) {
         APRNET_ARG_CHECK(value == 0 || value == 16 || value == 32 || value == 64, "channels per stage must be 0 (automatic), 16, 32 or 64");
         g_ks_override = value;

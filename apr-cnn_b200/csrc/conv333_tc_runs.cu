@@ -1,0 +1,363 @@
+// 3x3x3 particle convolution on the tensor cores over runs of cells (bf16 operands, fp32 accumulation; forward pass and
+// same-level input gradient of layers with at most 128 result channels).
+//
+// The kernel of conv333_tc.cu gathers every source row once per tap, 27 rows per location.  Here the M dimension of a tile is not
+// 128 locations but 128 * H consecutive slots of the run plan (run_plan.cu).  For each of the 9 rows of cells (dz, dx) the tile's
+// sources are gathered once, one row per slot, and the three y taps read the same staged rows shifted by one: the A descriptor of
+// tap dy starts dy rows further.  (The swizzle of a K-major operand is a function of the shared-memory address, so a start address
+// inside the pattern is an ordinary one.)  That is 9 x 1.07 .. 1.27 gathered rows per location instead of 27; slots without a
+// location are the price, 7 to 27 % more multiply-adds.  Each weight tile that is fetched meets H blocks of 128 rows.
+// What bounds it now: rows and weights arrive from L2 at 6.5 to 7 TB/s (64 -> 64 channels), and the MMAs of narrow tiles read
+// shared memory for longer than they multiply.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
+// 32 -> 32 layer that takes 0.48.)
+//
+// Every result of the forward pass is the same sequence of MMAs (neighbour row, channel block, dy, 16 channels) as in
+// conv333_tc.cu, so the two kernels agree bit for bit: what follows a convolution (rounding to bf16, ReLU, max-pooling) turns a
+// difference in the last bit into another gate.
+#include "apr_device.cuh"
+#include "tc_ptx.cuh"
+#include <cuda_bf16.h>
+#include <algorithm>
+#include <cstring>
+
+namespace {
+
+using namespace tcptx;
+typedef long long ll;
+constexpr int MAX_SEGS = APRNET_MAX_LEVELS;
+constexpr int MAX_STAGES = 16;
+constexpr int MAX_ACC = 4;
+constexpr int NPROD = 8;                                 // producer warps
+constexpr int MMA_WARP = NPROD, EPI_WARP = NPROD + 2;    // two MMA warps, two sets of four epilogue warps
+constexpr int THREADS = (NPROD + 2 + 8) * 32;
+
+struct RunParams {
+    int n_segs;
+    ll slot_begin[MAX_SEGS], slot_end[MAX_SEGS];         // slots of the level
+    ll lo[MAX_SEGS], hi[MAX_SEGS];                       // its locations (same-level mask of the input gradient)
+    int wslot[MAX_SEGS];
+    int tile_begin[MAX_SEGS + 1];
+    const int32_t* src; ll S;                            // run plan: [9][S] sources, [S] locations
+    const int32_t* loc;
+    const __nv_bfloat16* rows; int kpad;
+    ll tree_base, zero_row;
+    const __nv_bfloat16* wp;                             // packed weights [slot][tap][k chunk][NT][8]
+    float* out; ll ld_out; int n_dim;
+    const float* bias;
+    int same_level_only;
+    int* error_flag;
+};
+
+template<int KS> __device__ __forceinline__ int swizzled_chunk(int row, int c) {      // position of 16-byte chunk c of row `row`
+    return KS == 64 ? (c ^ (row & 7)) : (KS == 32 ? (c ^ ((row >> 1) & 3)) : (c ^ ((row >> 2) & 1)));
+}
+
+struct Tile { ll s0, sb, se, lo, hi; int wslot; };       // s0: slot of staged row 0
+
+__device__ __forceinline__ Tile tile_of(const RunParams& P, int tile, int rows) {
+    int seg = 0;
+    while (seg + 1 < P.n_segs && tile >= P.tile_begin[seg + 1]) ++seg;
+    Tile t;
+    t.sb = P.slot_begin[seg]; t.se = P.slot_end[seg]; t.lo = P.lo[seg]; t.hi = P.hi[seg]; t.wslot = P.wslot[seg];
+    t.s0 = t.sb - 1 + (ll) (tile - P.tile_begin[seg]) * (rows - 2);      // the first and the last row have no neighbour on one side
+    return t;
+}
+
+// Roles of the warps of the persistent block:
+//   0-7         producers, in groups of WPS; a stage (neighbour row x KS channels x 128 H slots, and the weights of its three taps) belongs to one
+//               group, each warp copies its share of the rows with 16-byte cp.async into the swizzled K-major operand and attaches its
+//               arrival to the stage's barrier; a lane holds the table entries of its rows, requested one stage of the group ahead, and
+//               hands them round by shuffles; one lane streams the weights with bulk copies;
+//   8, 9        one thread each issues the MMAs of every second block of 128 rows (two issuers: a narrow MMA costs its thread more
+//               cycles than it costs the tensor pipe) and commits the stage's free barrier;
+//   10-17       epilogue, four warps per issuer: TMEM -> registers -> global;
+// All waits are bounded and poll the block's abort flag (see conv333_tc.cu).
+template<int NT, int KS, int KORD, int H, int WPS>
+__global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunParams P, const int stages) {
+    constexpr int NG = NPROD / WPS;                          // stages in issue at once
+    constexpr int CH = KS / 8;                               // 16-byte chunks per row piece
+    constexpr int RW = 32 / CH;                              // rows per copy instruction of a warp
+    constexpr int ROWS = 128 * H, WROWS = ROWS / WPS;        // slots of a tile, rows a producer warp copies
+    constexpr int NI = WROWS / RW, LR = (WROWS + 31) / 32;   // its copy instructions per stage, table entries per lane
+    constexpr int NACC = 512 / (H * NT) < MAX_ACC ? 512 / (H * NT) : MAX_ACC;      // accumulators in flight per block of 128 rows
+    constexpr int ISSUERS = H < 2 ? 1 : 2;
+    constexpr int ROW_BYTES = KS * 2;
+    constexpr uint32_t A_LAYOUT = KS == 64 ? 2u : (KS == 32 ? 4u : 6u);     // SWIZZLE_128B / 64B / 32B
+    constexpr int A_BYTES = ROWS * ROW_BYTES;
+    constexpr int B_TAP = NT * KS * 2;
+    constexpr int STAGE_BYTES = A_BYTES + 3 * B_TAP;
+    constexpr uint32_t IDESC = make_idesc(NT, false, false);
+    static_assert(STAGE_BYTES % 1024 == 0 && H * NT <= 512 && WROWS % 32 == 0, "stages keep the swizzle alignment; accumulators fit TMEM");
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    // ring at a multiple of 1024 bytes, with 1024 bytes in front of it (row -1 of the first stage is read, its results are not used)
+    unsigned char* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u) + 1024;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ring + (size_t) stages * STAGE_BYTES + 1024);
+    uint64_t* full = bars;                                   // [stages] copies of the stage landed
+    uint64_t* empty = bars + MAX_STAGES;                     // [stages] all MMAs that read the stage completed
+    uint64_t* tmem_full = empty + MAX_STAGES;                // [2][NACC] accumulators of an issuer complete
+    uint64_t* tmem_empty = tmem_full + 2 * MAX_ACC;          // [2][NACC] read back
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2 * MAX_ACC);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int kchunks = P.kpad / KS, steps = 9 * kchunks;
+    const int total_tiles = P.tile_begin[P.n_segs];
+    const int my_tiles = (int) blockIdx.x < total_tiles ? (total_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
+    const int ngroups = min(NG, stages);
+
+    if (tid == 0) {
+        for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), WPS * 32 + 1); mbar_init(smem_u32(empty + i), ISSUERS); }
+        for (int i = 0; i < 2 * MAX_ACC; ++i) { mbar_init(smem_u32(tmem_full + i), 1); mbar_init(smem_u32(tmem_empty + i), 4); }
+        *abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == MMA_WARP) { tmem_alloc(smem_u32(tmem_slot), H * NACC * NT); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_d = *tmem_slot;
+    bool failed = false, bulk_issued = false;
+
+    if (warp < NPROD) {
+        // ---------------- producers ----------------
+        const int grp = warp / WPS, sub = warp % WPS;
+        if (grp < ngroups) {
+            const int j = lane % CH, rsub = lane / CH;
+            const uint32_t total = (uint32_t) my_tiles * (uint32_t) steps;
+            const ll w_tap_stride = (ll) P.kpad * NT * 2;
+            uint32_t g = grp, slot = grp, use = 0;
+            int it = 0, step = grp, cur_it = -1;
+            Tile t;
+            int32_t raw[LR], cur[LR];
+            auto request = [&](int d) {                      // table entries of this lane's rows
+#pragma unroll
+                for (int i = 0; i < LR; ++i) {
+                    const ll s = t.s0 + sub * WROWS + 32 * i + lane;
+                    raw[i] = (s >= t.sb && s < t.se) ? __ldg(P.src + (ll) d * P.S + s) : APRNET_NONE;
+                }
+            };
+            auto locate = [&]() {                            // tile and stage of g
+                while (step >= steps) { step -= steps; ++it; }
+                if (it != cur_it) { cur_it = it; t = tile_of(P, blockIdx.x + it * gridDim.x, ROWS); }
+            };
+            if (g < total) { locate(); request(step / kchunks); }
+            while (g < total) {
+                const int d = step / kchunks, kc = step - d * kchunks;
+#pragma unroll
+                for (int i = 0; i < LR; ++i) {
+                    const int32_t v = raw[i];
+                    ll r = P.zero_row;
+                    if (P.same_level_only) { if (v >= t.lo && v < t.hi) r = v; }
+                    else if (v >= 0) r = v;
+                    else if (v != APRNET_NONE) r = P.tree_base + aprnet_dec_tree(v);
+                    cur[i] = (int32_t) r;
+                }
+                const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(P.wp) + (ll) t.wslot * 27 * w_tap_stride;
+                step += ngroups;
+                if (g + ngroups < total) { locate(); request(step / kchunks); }      // in flight while this stage is copied
+                if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
+                unsigned char* a_s = ring + (size_t) slot * STAGE_BYTES;
+                if (sub == 0 && lane == 0) {
+                    mbar_expect_tx(smem_u32(full + slot), 3 * B_TAP);
+#pragma unroll
+                    for (int dy = 0; dy < 3; ++dy)
+                        bulk_copy_g2s(smem_u32(a_s + A_BYTES + dy * B_TAP), wsrc + (3 * d + dy) * w_tap_stride + (ll) kc * KS * NT * 2, B_TAP, smem_u32(full + slot));
+                    bulk_issued = true;
+                }
+                const __nv_bfloat16* src0 = P.rows + kc * KS + j * 8;
+#pragma unroll
+                for (int i = 0; i < NI; ++i) {
+                    const int row = sub * WROWS + i * RW + rsub;
+                    const int32_t r = __shfl_sync(0xffffffffu, cur[i * RW / 32], (i * RW + rsub) & 31);
+                    cp_async16(smem_u32(a_s + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) r * P.kpad);
+                }
+                cp_async_arrive_noinc(smem_u32(full + slot));        // this thread's arrival when its copies have landed
+                g += ngroups; slot += ngroups;
+                if (slot >= (uint32_t) stages) { slot -= stages; ++use; }
+            }
+            cp_async_commit();
+            cp_async_wait<0>();
+        }
+    } else if (warp < EPI_WARP) {
+        // ---------------- MMA issue, every second block of 128 rows ----------------
+        const int h0 = warp - MMA_WARP;
+        if (lane == 0 && h0 < ISSUERS) {
+            uint32_t slot = 0, use = 0;
+            for (int it = 0; it < my_tiles && !failed; ++it) {
+                const uint32_t acc = (uint32_t) it % NACC, acc_use = (uint32_t) it / NACC;
+                if (acc_use > 0 && !mbar_wait(smem_u32(tmem_empty + h0 * MAX_ACC + acc), (acc_use - 1) & 1, abort_flag)) { failed = true; break; }
+                tc_fence_after();
+                for (int step = 0; step < steps; ++step) {
+                    if (!mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
+                    fence_proxy_async();          // generic-proxy writes of the cp.async copies -> tensor-core (async proxy) reads
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(ring + (size_t) slot * STAGE_BYTES);
+                    const uint64_t db0 = make_desc(a_addr + A_BYTES, NT * 16, 128, 0);
+#pragma unroll
+                    for (int h = 0; h < H; h += ISSUERS) {
+                        const uint64_t da0 = make_desc(a_addr + (h + h0) * 128 * ROW_BYTES - ROW_BYTES, 16, 8 * ROW_BYTES, A_LAYOUT);      // dy = -1
+                        const uint32_t d_addr = tmem_d + ((h + h0) * NACC + acc) * NT;
+#pragma unroll
+                        for (int ko = 0; ko < KS / KORD; ++ko)
+#pragma unroll
+                            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                                for (int kk = 0; kk < KORD / 16; ++kk) {
+                                    const int k = ko * (KORD / 16) + kk;
+                                    umma_bf16(d_addr, da0 + (uint64_t) ((dy * ROW_BYTES + k * 32) >> 4), db0 + (uint64_t) ((dy * B_TAP + k * 2 * (NT * 16)) >> 4),
+                                              IDESC, (step > 0 || ko > 0 || dy > 0 || kk > 0) ? 1u : 0u);
+                                }
+                    }
+                    umma_commit(smem_u32(empty + slot));
+                    if (++slot == (uint32_t) stages) { slot = 0; ++use; }
+                }
+                if (!failed) umma_commit(smem_u32(tmem_full + h0 * MAX_ACC + acc));
+            }
+        }
+    } else if ((warp - EPI_WARP) / 4 < ISSUERS) {
+        // ---------------- epilogue of one issuer's blocks ----------------
+        const int h0 = (warp - EPI_WARP) >> 2, q = warp & 3;         // q: TMEM lanes this warp may read
+        auto location = [&](int it, int h) {
+            const int m = h * 128 + q * 32 + lane;
+            if (it >= my_tiles || m == 0 || m == ROWS - 1) return (int32_t) -1;
+            const Tile t = tile_of(P, blockIdx.x + it * gridDim.x, ROWS);
+            const ll s = t.s0 + m;
+            return s >= t.sb && s < t.se ? __ldg(P.loc + s) : -1;
+        };
+        constexpr int BLOCKS = H / ISSUERS;
+        int32_t p_next[BLOCKS];
+#pragma unroll
+        for (int b = 0; b < BLOCKS; ++b) p_next[b] = location(0, h0 + b * ISSUERS);
+        for (int it = 0; it < my_tiles; ++it) {
+            int32_t p_cur[BLOCKS];
+#pragma unroll
+            for (int b = 0; b < BLOCKS; ++b) { p_cur[b] = p_next[b]; p_next[b] = location(it + 1, h0 + b * ISSUERS); }
+            const uint32_t acc = (uint32_t) it % NACC, acc_use = (uint32_t) it / NACC;
+            if (!mbar_wait_warp(smem_u32(tmem_full + h0 * MAX_ACC + acc), acc_use & 1, abort_flag)) { failed = true; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int b = 0; b < BLOCKS; ++b) {
+                const int32_t p = p_cur[b];
+#pragma unroll 1
+                for (int c0 = 0; c0 < NT; c0 += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(tmem_d + ((uint32_t) (q * 32) << 16) + ((h0 + b * ISSUERS) * NACC + acc) * NT + c0, r);
+                    tmem_ld_wait();
+                    if (P.bias) {
+#pragma unroll
+                        for (int jj = 0; jj < 32; ++jj)
+                            if (c0 + jj < P.n_dim) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + __ldg(P.bias + c0 + jj));
+                    }
+                    if (p >= 0) {
+                        float* dst = P.out + (ll) c0 * P.ld_out + p;
+#pragma unroll
+                        for (int jj = 0; jj < 32; ++jj)
+                            if (c0 + jj < P.n_dim) dst[(ll) jj * P.ld_out] = __uint_as_float(r[jj]);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(tmem_empty + h0 * MAX_ACC + acc));
+        }
+    }
+
+    // teardown (also the error path): the gather copies were drained above; after a failure the bulk copies still in flight get
+    // time to land before the block's shared memory is released
+    if (failed) {
+        *abort_flag = 1;
+        if (P.error_flag) *P.error_flag = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (bulk_issued && *abort_flag) for (int i = 0; i < 2000; ++i) __nanosleep(100);
+    if (warp == MMA_WARP) tmem_dealloc(tmem_d, H * NACC * NT);
+}
+
+// ---- host side ----------------------------------------------------------------------------------------
+constexpr size_t FIXED = (2 * MAX_STAGES + 4 * MAX_ACC) * 8 + 16 + 2048 + 1024;      // barriers, the rows in front of and behind the ring, alignment
+
+inline size_t stage_bytes(int nt, int ks, int h) { return (size_t) 128 * h * ks * 2 + 3 * (size_t) nt * ks * 2; }
+inline int run_stages(int nt, int ks, int h) { return (int) std::min<size_t>(MAX_STAGES, (227 * 1024 - FIXED) / stage_bytes(nt, ks, h)); }
+
+template<int NT, int KS, int KORD, int H, int WPS>
+int launch_runs(RunParams& P, int sms, cudaStream_t st, const char* pname) {
+    auto kern = conv333_tc_runs_kernel<NT, KS, KORD, H, WPS>;
+    const int stages = run_stages(NT, KS, H);
+    const size_t smem = (size_t) stages * stage_bytes(NT, KS, H) + FIXED;
+    APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    for (int i = 0; i < P.n_segs; ++i) P.tile_begin[i + 1] = P.tile_begin[i] + aprnet_ceil_div(P.slot_end[i] - P.slot_begin[i], 128 * H - 2);
+    if (P.tile_begin[P.n_segs] == 0) return APRNET_OK;
+    AprnetProfScope _prof(pname, st);
+    kern<<<std::min(P.tile_begin[P.n_segs], sms), THREADS, smem, st>>>(P, stages);
+    APRNET_LAUNCH_CHECK();
+    return APRNET_OK;
+}
+
+// Blocks of 128 rows per tile.  Cycles of a stage as fitted to the measurements below: the MMAs read their operands from shared
+// memory at 128 bytes per clock (32 cycles for A, nt / 4 for B each), the copies write it, and about 550 cycles pass between the
+// roles whatever the stage holds.  Tall tiles spread that and the weights over more rows; few rows want short tiles on all SMs.
+// (16 -> 16, 32 -> 32, 64 -> 32 at level delta 0 and 64 -> 64 at level delta 1 of 1.8 M particles, forward: H = 2: 0.22, 0.30,
+// 0.45, 0.26 ms; H = 4: 0.16, 0.24, 0.39, 0.25 ms; conv333_tc.cu: 0.52 for 32 -> 32, 0.48 for 64 -> 64.)
+inline int pick_h(const RunParams& P, int nt, int ks, int max_h, int sms) {
+    int best = 1;
+    double cost = 0;
+    for (int h = 1; h <= max_h; h *= 2) {
+        ll tiles = 0;
+        for (int i = 0; i < P.n_segs; ++i) tiles += aprnet_ceil_div(P.slot_end[i] - P.slot_begin[i], 128 * h - 2);
+        const double stage = 550 + h * 3 * (ks / 16) * (32 + nt / 4) + 1.3 * stage_bytes(nt, ks, h) / 128;
+        const double c = (double) ((tiles + sms - 1) / sms) * (9 * P.kpad / ks) * stage;
+        if (h == 1 || c < cost) { cost = c; best = h; }
+    }
+    return best;
+}
+
+} // namespace
+
+// Channels between two changes of dy (the order of the products) of this kernel for kpad source channels and a tile of nt result
+// channels; 0: not this kernel.  The forward pass keeps the order of conv333_tc.cu, whose stages of `ks` channels hold three taps for
+// nt <= 64 (the same order as here) but one tap for nt = 128 (the same only when all channels are in one stage).  The input gradient is
+// free: nothing that follows depends on its last bit.
+int aprnet_tc_runs_order(int backward, int kpad, int nt, int ks) {
+    if (nt > 128) return 0;
+    if (nt <= 64) return ks;
+    if (!backward) return kpad == ks ? ks : 0;
+    return kpad % 32 == 0 ? 32 : 16;
+}
+
+int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, ll tree_base, ll zero_row, const void* wp,
+                       const float* bias, float* out, ll ld_out, int n_dim, int* error_flag, cudaStream_t st, const char* pname) {
+    const RunPlan* rp = aprnet_get_run_plan(a, dl, st);
+    if (!rp) return APRNET_ERR_CUDA;
+    RunParams P;
+    memset(&P, 0, sizeof(P));
+    for (const Segment& sg : aprnet_segments(a, dl, slots, false)) {
+        const int i = P.n_segs++;
+        P.slot_begin[i] = rp->level_begin[sg.level]; P.slot_end[i] = rp->level_begin[sg.level + 1];
+        P.lo[i] = sg.begin; P.hi[i] = sg.end; P.wslot[i] = sg.slot;
+    }
+    if (P.n_segs == 0) return APRNET_OK;
+    P.src = rp->src; P.S = rp->n_slots; P.loc = rp->loc;
+    P.rows = (const __nv_bfloat16*) rows; P.kpad = kpad; P.tree_base = tree_base; P.zero_row = zero_row;
+    P.wp = (const __nv_bfloat16*) wp; P.out = out; P.ld_out = ld_out; P.n_dim = n_dim; P.bias = bias; P.same_level_only = backward;
+    P.error_flag = error_flag;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // channels per stage: whole 128-byte rows where the width allows (64 -> 64: 0.25 instead of 0.29 ms with 32)
+    const int ks = kpad % 64 == 0 && order >= 32 ? 64 : order;
+    const int h = pick_h(P, nt, ks, nt == 128 ? 2 : (nt == 32 && ks == 16 ? 8 : 4), sms);
+#define RUN_CASE(NT_, KS_, KORD_, H_, WPS_) if (nt == NT_ && ks == KS_ && order == KORD_ && h == H_) return launch_runs<NT_, KS_, KORD_, H_, WPS_>(P, sms, st, pname);
+    // warps per stage: two, so that four stages are in issue at once; four where the ring holds only two or three stages
+    RUN_CASE(32, 16, 16, 1, 2) RUN_CASE(32, 16, 16, 2, 2) RUN_CASE(32, 16, 16, 4, 2) RUN_CASE(32, 16, 16, 8, 4)
+    RUN_CASE(32, 32, 32, 1, 2) RUN_CASE(32, 32, 32, 2, 2) RUN_CASE(32, 32, 32, 4, 2)
+    RUN_CASE(32, 64, 64, 1, 2) RUN_CASE(32, 64, 64, 2, 2) RUN_CASE(32, 64, 64, 4, 4)
+    RUN_CASE(64, 16, 16, 1, 2) RUN_CASE(64, 16, 16, 2, 2) RUN_CASE(64, 16, 16, 4, 2)
+    RUN_CASE(64, 32, 32, 1, 2) RUN_CASE(64, 32, 32, 2, 2) RUN_CASE(64, 32, 32, 4, 2)
+    RUN_CASE(64, 64, 32, 1, 2) RUN_CASE(64, 64, 32, 2, 4) RUN_CASE(64, 64, 32, 4, 4)
+    RUN_CASE(128, 16, 16, 1, 2) RUN_CASE(128, 16, 16, 2, 2) RUN_CASE(128, 32, 32, 1, 2) RUN_CASE(128, 32, 32, 2, 2)
+    RUN_CASE(128, 64, 32, 1, 4) RUN_CASE(128, 64, 32, 2, 4) RUN_CASE(128, 64, 64, 1, 4) RUN_CASE(128, 64, 64, 2, 4)
+#undef RUN_CASE
+    aprnet_set_error("conv333 tensor-core path: unsupported run geometry nt=%d ks=%d order=%d h=%d", nt, ks, order, h);
+    return APRNET_ERR_UNSUPPORTED;
+}

@@ -234,6 +234,8 @@ int aprnet_conv333_backward_input_cross_level(aprnet_apr* apr, int level_delta, 
  * Limit: 27 * N(level_delta) < 2^31, i.e. up to 79.5 M locations (32-bit edge ids); beyond it
  * aprnet_conv333_backward_tc(_rows) falls back to aprnet_conv333_backward_input_cross_level (atomic adds). */
 int aprnet_edge_plan_build(aprnet_apr* apr, int level_delta, void* stream);
+/* The same for the run plan of the tensor-core gather kernels (output locations in runs along y; built once per level delta). */
+int aprnet_run_plan_build(aprnet_apr* apr, int level_delta, void* stream);
 int64_t aprnet_edge_workspace_bytes(const aprnet_apr* apr, int level_delta, int cout);
 int aprnet_conv333_backward_input_cross_level_tc(aprnet_apr* apr, int level_delta, int cin, int cout, int num_slots,
                                                  const void* packed_grad_output_rows, int grad_output_row_width,
@@ -250,7 +252,7 @@ int aprnet_tc_selftest_wait_timeout(int max_polls, void* stream);
  * stage, "wps" = producer warps that fill one stage together (both must be set, and the pair must be a compiled
  * shape whose ring fits shared memory, else the automatic choice stays), "tma_taps" = how many of a stage's taps the TMA
  * unit fetches (tile::gather4) instead of cp.async (with "taps" and "wps"), "ks" = channels per stage (16, 32, 64),
- * "dw_waves" = waves of blocks of the weight-gradient kernel. */
+ * "runs" = 0: gather every tap by itself instead of runs of cells, "dw_waves" = waves of blocks of the weight-gradient kernel. */
 int aprnet_tc_set_option(const char* name, int value);
 
 /* ---- 1x1x1 convolution -----------------------------------------------------------------------
