@@ -194,6 +194,10 @@ int aprnet_f32_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int sl
 int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* gout, long long ld_out, const float* w, float* gin, long long ld_in,
                               float* gtree, long long ld_tree, void* workspace, bool tree_adjoint, cudaStream_t st);
 
+// ranges of block partial sums [range][27][cin][cout] per stencil slot: slot[g] owns [first[g], first[g + 1]), g < n
+struct SlotRanges { int n; int first[APRNET_MAX_LEVELS + 1]; int slot[APRNET_MAX_LEVELS]; };
+int aprnet_dw_reduce(const float* partial, const SlotRanges& sr, int cin, int cout, float* gw, cudaStream_t st);      // grad_weights += sums, fixed order
+
 // stream-ordered scratch of one call, for entry points whose signature has no workspace
 struct StreamScratch {
     void* p = nullptr;

@@ -449,8 +449,6 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
 
 // grad_weights[slot][co][ci][tap] += the block sums of the slot's ranges.  Eight threads share a result and take every eighth
 // range; their sums are combined in a fixed order.
-struct SlotRanges { int first[MAX_SEGS + 1]; int slot[MAX_SEGS]; };      // ranges of the g-th slot: [first[g], first[g + 1])
-
 __global__ void __launch_bounds__(256) dw_reduce_f32_kernel(const float* __restrict__ partial, SlotRanges sr, int cin, int cout, float* __restrict__ gw) {
     __shared__ float sums[8][33];
     const ll elems = (ll) 27 * cin * cout;
@@ -595,14 +593,14 @@ int run_dw(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* xro
     ll per_block = std::max<ll>(2, (total_units + budget - 1) / budget);
     while (blocks_for(per_block) > budget) ++per_block;
     SlotRanges sr;
-    int n_slots = 0;
+    sr.n = 0;
     P.range_first[0] = 0;
     for (int i = 0; i < P.n_segs; ++i) {
         P.seg_begin[i] = segs[i].begin; P.seg_end[i] = segs[i].end;
         P.range_first[i + 1] = P.range_first[i] + (int) (((segs[i].end - segs[i].begin + DW_UNIT - 1) / DW_UNIT + per_block - 1) / per_block);
         // levels are listed coarse to fine, so those that share a slot (the last one) are neighbours
-        if (n_slots == 0 || sr.slot[n_slots - 1] != segs[i].slot) { sr.first[n_slots] = P.range_first[i]; sr.slot[n_slots++] = segs[i].slot; }
-        sr.first[n_slots] = P.range_first[i + 1];
+        if (sr.n == 0 || sr.slot[sr.n - 1] != segs[i].slot) { sr.first[sr.n] = P.range_first[i]; sr.slot[sr.n++] = segs[i].slot; }
+        sr.first[sr.n] = P.range_first[i + 1];
     }
     P.nbr = plan->nbr; P.N = plan->n;
     P.xrows = xrows; P.xpad = pad4(cin); P.tree_base = plan->n; P.zero_row = plan->n + plan->tree_size;
@@ -617,11 +615,7 @@ int run_dw(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* xro
     DW_CASE(16, 64, 1, 4, 16) DW_CASE(16, 32, 2, 2, 16) DW_CASE(16, 16, 2, 2, 8) DW_CASE(16, 8, 2, 2, 4)
     DW_CASE(8, 64, 1, 4, 16) DW_CASE(8, 32, 2, 2, 16) DW_CASE(8, 16, 2, 2, 8) DW_CASE(8, 8, 2, 2, 4)
 #undef DW_CASE
-    if (rc) return rc;
-    AprnetProfScope _prof("conv333_dw_reduce", st);
-    dw_reduce_f32_kernel<<<dim3((unsigned) aprnet_ceil_div((ll) 27 * cin * cout, 32), (unsigned) n_slots), 256, 0, st>>>(partial, sr, cin, cout, gw);
-    APRNET_LAUNCH_CHECK();
-    return APRNET_OK;
+    return rc ? rc : aprnet_dw_reduce(partial, sr, cin, cout, gw, st);
 }
 
 // cross-level part of the input gradient (see edge_plan.cu): sums per (target, tap), then the gather over the targets
@@ -676,6 +670,13 @@ inline size_t edge_bytes(const aprnet_apr* a, int dl, int cout) {
 }
 
 } // namespace
+
+int aprnet_dw_reduce(const float* partial, const SlotRanges& sr, int cin, int cout, float* gw, cudaStream_t st) {
+    AprnetProfScope _prof("conv333_dw_reduce", st);
+    dw_reduce_f32_kernel<<<dim3((unsigned) aprnet_ceil_div((ll) 27 * cin * cout, 32), (unsigned) sr.n), 256, 0, st>>>(partial, sr, cin, cout, gw);
+    APRNET_LAUNCH_CHECK();
+    return APRNET_OK;
+}
 
 // bytes of the packed rows of the input (particles, tree means, zero row), which a forward call leaves at the start of its workspace
 size_t aprnet_f32_rows_bytes(const aprnet_apr* a, int dl, int cin) {

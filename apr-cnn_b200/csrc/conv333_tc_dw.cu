@@ -1,20 +1,26 @@
 // Weight gradient of the 3x3x3 particle convolution on the tensor cores (tcgen05 + TMEM), bf16
 // operands with fp32 accumulation, deterministic.
 //
-//     dW[tap][ci][co] = sum over output locations p of  X[nbr(tap, p)][ci] * dO[p][co]
+//     dW[d, dy][ci][co] = sum over locations p of  X[cell (dz, dx, dy) of p][ci] * dO[p][co]
+//                       = sum over slots s of      X_d[s][ci] * dO[location of slot s - dy][co]
 //
-// is a GEMM whose contraction index is the particle.  One block owns a contiguous range of locations of
-// one level, a group of taps, a block of CIB input channels and up to 256 output channels.  Its
-// accumulators D[(tap, ci)][co] stay in TMEM for the whole range: 128-row tiles of 128 / CIB taps x CIB
-// channels, NCOL fp32 columns each, side by side in the 512 columns; the tap group is as large as the
-// columns allow, so the gathered rows are read once (CIB = all channels) and only the small dO rows are
-// re-read per tap group.  Both operands are MN-major with the 128-byte hardware swizzle: a gathered
-// neighbour row piece (CIB channels) and a dO row are contiguous in shared memory as they are in global
-// memory, with K = particles.  Warp roles: 8 producer warps (two stages in issue at once, four warps of
-// 32 particles each per stage; table entries are loaded by the lane that owns the particle, one stage
-// ahead, and passed between lanes by shuffles; arrival on the stage barrier is asynchronous), one MMA
-// thread, epilogue by warps 0-3 after the last MMA.  Each block writes its partial sums once; a second
-// pass adds the ranges in ascending order (no atomics).
+// with the slots of the run plan (run_plan.cu): X_d[s] is what fills the cell one step of d = (dz, dx) beside slot s, and the cell of
+// slot s is the y neighbour of slot s - dy.  So every neighbour row is gathered once per slot (9 x 1.07 .. 1.27 rows per location)
+// and meets dO three times, shifted by one slot each.  The product contracts over the slots; both operands are MN-major with a hardware
+// swizzle, rows of channels in shared memory as they lie in global memory.  M = TPT = 128 / CIB neighbours x CIB input channels; the
+// three shifts lie side by side in N: the B operand's blocks of NCOL columns start one slot (one row) further each (their stride in
+// the descriptor is a row), which makes one MMA of 3 * NCOL <= 192 columns; for NCOL = 128 they are three MMAs.
+// A block owns every cnt-th chunk of 128 slots of one level, a group of neighbours, CIB input and NCOL output channels; its
+// accumulators stay in the 512 TMEM columns for all its chunks.  Blocks that run together walk through the level side by side, so the
+// rows one of them gathers for the neighbouring z planes are still in L2 for the others.
+//
+// What bounds it: rows arriving from L2 (6 to 7 TB/s).  Gathering all 27 taps of a location by themselves, as this kernel did before,
+// took 1.15 ms for 64 -> 64 channels at level delta 1 (1.86 M locations) and 1.03 ms for 32 -> 32 at level delta 0 (3.5 M).
+//
+// Warp roles: 16 producer warps (four stages in issue at once, four warps of 32 slots each per stage; table entries are loaded by the
+// lane that owns the slot, one stage ahead, and passed between lanes by shuffles; arrival on the stage barrier is asynchronous), one
+// MMA thread, epilogue by warps 0-3 after the last MMA.  Each block writes its partial sums once; a second pass adds the ranges in
+// a fixed order (no atomics).
 // Reference arithmetic: pyapr/aprnet/src/helpers.hpp:624-702 (accumulate_convolution_backward, dW part).
 #include "apr_device.cuh"
 #include "tc_ptx.cuh"
@@ -27,38 +33,43 @@ namespace {
 
 using namespace tcptx;
 typedef long long ll;
-constexpr int PT = 128;                       // particles per stage (K extent of one stage)
-constexpr int DW_THREADS = 9 * 32;            // 8 producer warps + 1 MMA warp
+constexpr int PT = 128;                       // slots per stage (K extent of one stage)
+constexpr int NGROUP = 4;                     // producer groups of four warps = stages in issue at once
+constexpr int MMA_WARP = 4 * NGROUP;
+constexpr int DW_THREADS = (4 * NGROUP + 1) * 32;
 constexpr int DW_MAX_STAGES = 6;
-constexpr int A_STAGE = 2 * PT * 128;         // 128 accumulator rows = two 64-element swizzle atoms per particle
+constexpr int A_STAGE = 2 * PT * 128;         // 128 accumulator rows = two 64-element swizzle atoms per slot
+constexpr int G_ROWS = PT + 8;                // dO of slots -1 .. 128 of the chunk, whole 8-row groups
 
 constexpr int DW_MAX_SEGS = APRNET_MAX_LEVELS;
 struct DwParams {
-    // the levels of the level delta, each cut into chunks of PT locations that its blocks take in turn: block r
-    // with range_first[i] <= r < range_first[i + 1] belongs to level i and takes that level's chunks
-    // r - range_first[i], + cnt, + 2 cnt, ... (cnt = blocks of the level).  Blocks that run at the same time
-    // thus walk through the level side by side, and the rows one of them gathers for the neighbouring z planes
-    // are still in L2 when the others (and the blocks of the other tap groups) ask for them.
+    // the levels of the level delta, each cut into chunks of PT slots that its blocks take in turn: block r with
+    // range_first[i] <= r < range_first[i + 1] belongs to level i and takes that level's chunks r - range_first[i], + cnt, + 2 cnt, ...
     int n_segs;
     ll seg_begin[DW_MAX_SEGS], seg_end[DW_MAX_SEGS];
     int range_first[DW_MAX_SEGS + 1];
-    const int32_t* nbr; ll N;
+    const int32_t* src; ll S;              // run plan
+    const int32_t* loc;
     const __nv_bfloat16* xrows; int xpad;  // packed inputs [N + T + 1][xpad]; tree rows start at tree_base, zeros at zero_row
     ll tree_base, zero_row;
     const __nv_bfloat16* grows; int gpad;  // packed dO [N + 1][gpad], zeros at row g_zero_row
     ll g_zero_row;
-    float* partial;                        // [range][cout][cin][27]
-    int cin, cout, ci_blocks, groups, taps_per_group;
+    float* partial;                        // [range][27][cin][cout]
+    int cin, cout, ci_blocks, groups, d_per_group;
     int* error_flag;
 };
 
 template<int CIB, int NCOL>
 __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwParams P, const int nstage) {
-    constexpr int TPT = 128 / CIB;                      // taps per 128-row accumulator tile
+    constexpr int TPT = 128 / CIB;                      // neighbours per 128-row accumulator tile
     constexpr int PC = CIB / 8;                         // 16-byte chunks per gathered row piece
-    constexpr int G_BYTES = (NCOL / 64) * PT * 128;     // one dO chunk: NCOL / 64 swizzle atoms per particle
-    constexpr uint32_t IDESC = make_idesc(NCOL, true, true);
-    constexpr uint32_t ATOM_STRIDE = PT * 128;          // between 64-element atoms along M (or N)
+    constexpr int G_ROW = NCOL == 32 ? 64 : 128;        // bytes of a dO row in one swizzle atom
+    constexpr int G_ATOM = G_ROWS * G_ROW;              // one atom (32 or 64 columns) of a dO chunk
+    constexpr int G_BYTES = (G_ATOM * (NCOL == 128 ? 2 : 1) + 1023) / 1024 * 1024;
+    constexpr int COLS = 3 * NCOL;                      // accumulator columns of a tile
+    constexpr int MMAS = NCOL == 128 ? 3 : 1;
+    constexpr uint32_t IDESC = make_idesc(COLS / MMAS, true, true);
+    constexpr uint32_t ATOM_STRIDE = PT * 128;          // between 64-element atoms along M
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -75,22 +86,19 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = blockIdx.y % P.groups, cib = (blockIdx.y / P.groups) % P.ci_blocks, cob = blockIdx.y / (P.groups * P.ci_blocks);
-    const int tap0 = grp * P.taps_per_group;
-    const int ntaps = min(P.taps_per_group, 27 - tap0);
-    const int MT = (ntaps + TPT - 1) / TPT;             // accumulator tiles of this block
+    const int d0 = grp * P.d_per_group;
+    const int nd = min(P.d_per_group, 9 - d0);
+    const int MT = (nd + TPT - 1) / TPT;                // accumulator tiles of this block
     int seg = 0;
     while (seg + 1 < P.n_segs && (int) blockIdx.x >= P.range_first[seg + 1]) ++seg;
     const int rl = (int) blockIdx.x - P.range_first[seg], cnt = P.range_first[seg + 1] - P.range_first[seg];
-    const ll pb = P.seg_begin[seg] + (ll) rl * PT, pe = P.seg_end[seg];
-    const ll pstride = (ll) cnt * PT;                   // between two chunks of this block
-    const ll seg_chunks = (pe - P.seg_begin[seg] + PT - 1) / PT;
+    const ll sb = P.seg_begin[seg], se = P.seg_end[seg];
+    const ll seg_chunks = (se - sb + PT - 1) / PT;
     const int nchunks = rl < seg_chunks ? (int) ((seg_chunks - rl + cnt - 1) / cnt) : 0;
     const int total_stages = nchunks * MT;
-    const int gpiece = min(256, P.gpad - cob * 256);    // dO channels of this block
+    const int cpieces = min(PC, (P.xpad - cib * CIB) / 8);            // 16-byte pieces that exist of a row (the others are never used)
+    const int gpieces = min(NCOL, P.gpad - cob * NCOL) / 8;
 
-    // dO columns beyond gpiece are never copied: they must read as zeros
-    for (int e = tid; e < 2 * G_BYTES / 16; e += DW_THREADS) reinterpret_cast<uint4*>(g_ring)[e] = make_uint4(0, 0, 0, 0);
-    fence_proxy_async();
     if (tid == 0) {
         for (int i = 0; i < nstage; ++i) { mbar_init(smem_u32(full + i), 128); mbar_init(smem_u32(empty + i), 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(dfull + i), 128); mbar_init(smem_u32(dempty + i), 1); }
@@ -98,56 +106,73 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 8) { tmem_alloc(smem_u32(tmem_slot), 512); tmem_relinquish(); }
+    if (warp == MMA_WARP) { tmem_alloc(smem_u32(tmem_slot), 512); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_d = *tmem_slot;
     bool failed = false;
 
-    if (warp < 8 && total_stages > 0) {
+    if (warp < MMA_WARP && total_stages > 0) {
         // ---------------- producers ----------------
-        const int gq = warp >> 2, wq = warp & 3;        // stage parity handled / 32-particle quarter of the stage
+        const int gq = warp >> 2, wq = warp & 3;        // stage (modulo NGROUP) / 32-slot quarter of the stage
         const int c = lane % PC, r0 = lane / PC;
-        constexpr int RPI = 32 / PC;                    // particles covered by one copy instruction
+        constexpr int RPI = 32 / PC;                    // slots covered by one copy instruction
         int32_t rows_cur[TPT], raw_nxt[TPT];
-        // table entries of this lane's particle for the taps of stage s: requested here, decoded only when the
-        // stage is issued, so that the load latency overlaps the copies of the stage in between
-        auto request_rows = [&](int s, int32_t (&raw)[TPT]) {
+        int32_t loc_nxt = -1, loc_extra = -1, g_row = 0, g_extra = 0;
+        // table entries of this lane's slot for stage s: requested here, decoded only when the stage is issued, so that the load
+        // latency overlaps the copies of the stage in between; with a chunk's first stage also the locations of its dO rows (row r of
+        // the dO chunk is slot r - 1; the last two rows belong to the last quarter)
+        auto request = [&](int s) {
             const int chunk = s / MT, mt = s - chunk * MT;
-            const ll p = pb + (ll) chunk * pstride + wq * 32 + lane;
+            const ll c0 = sb + ((ll) rl + (ll) chunk * cnt) * PT, slot = c0 + wq * 32 + lane;
 #pragma unroll
             for (int tl = 0; tl < TPT; ++tl) {
-                const int t = mt * TPT + tl;
-                raw[tl] = (p < pe && t < ntaps) ? __ldg(P.nbr + (ll) (tap0 + t) * P.N + p) : APRNET_NONE;
+                const int d = mt * TPT + tl;
+                raw_nxt[tl] = (slot < se && d < nd) ? __ldg(P.src + (ll) (d0 + d) * P.S + slot) : APRNET_NONE;
+            }
+            if (mt == 0) {
+                const ll p = slot - 1, q = c0 + PT - 1 + lane;
+                loc_nxt = p >= sb && p < se ? __ldg(P.loc + p) : -1;
+                loc_extra = wq == 3 && lane < 2 && q < se ? __ldg(P.loc + q) : -1;
             }
         };
-        auto decode_rows = [&](const int32_t (&raw)[TPT], int32_t (&rows)[TPT]) {
+        auto decode = [&]() {
 #pragma unroll
             for (int tl = 0; tl < TPT; ++tl) {
-                const int32_t v = raw[tl];
-                rows[tl] = (int32_t) (v >= 0 ? (ll) v : (v == APRNET_NONE ? P.zero_row : P.tree_base + aprnet_dec_tree(v)));
+                const int32_t v = raw_nxt[tl];
+                rows_cur[tl] = (int32_t) (v >= 0 ? (ll) v : (v == APRNET_NONE ? P.zero_row : P.tree_base + aprnet_dec_tree(v)));
             }
+            g_row = loc_nxt >= 0 ? loc_nxt : (int32_t) P.g_zero_row;
+            g_extra = loc_extra >= 0 ? loc_extra : (int32_t) P.g_zero_row;
         };
         int s = gq;
-        if (s < total_stages) { request_rows(s, raw_nxt); decode_rows(raw_nxt, rows_cur); }
+        if (s < total_stages) { request(s); decode(); }
         while (s < total_stages) {
-            const int s_nxt = s + 2;
-            if (s_nxt < total_stages) request_rows(s_nxt, raw_nxt);      // in flight while this stage is issued
+            const int s_nxt = s + NGROUP;
+            if (s_nxt < total_stages) request(s_nxt);      // in flight while this stage is issued
             const int chunk = s / MT, mt = s - chunk * MT;
             const uint32_t slot = (uint32_t) s % (uint32_t) nstage, use = (uint32_t) s / (uint32_t) nstage;
             if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
             if (mt == 0) {
-                // this warp's 32 rows of the dO chunk
+                // this warp's rows of the dO chunk
                 const uint32_t db = chunk & 1, duse = chunk >> 1;
                 if (duse > 0 && !mbar_wait_warp(smem_u32(dempty + db), (duse - 1) & 1, abort_flag)) { failed = true; break; }
                 unsigned char* g_s = g_ring + db * G_BYTES;
-                const int gc = gpiece / 8;
-                for (int e = lane; e < 32 * gc; e += 32) {
-                    const int pl = e / gc, cc = e - pl * gc, k = wq * 32 + pl;
-                    const ll p = pb + (ll) chunk * pstride + k;
-                    cp_async16(smem_u32(g_s + (cc >> 3) * ATOM_STRIDE + k * 128 + (((cc & 7) ^ (k & 7)) << 4)),
-                               P.grows + (p < pe ? p : P.g_zero_row) * P.gpad + cob * 256 + cc * 8);
+                constexpr int GP = NCOL / 8;                           // 16-byte pieces of a dO row
+                const int cc = lane % GP;
+#pragma unroll
+                for (int i = 0; i < GP; ++i) {
+                    const int pl = i * (32 / GP) + lane / GP, r = wq * 32 + pl;
+                    const int32_t a = __shfl_sync(0xffffffffu, g_row, pl);
+                    const uint32_t off = NCOL == 32 ? r * 64 + ((cc ^ ((r >> 1) & 3)) << 4) : (cc >> 3) * G_ATOM + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
+                    if (cc < gpieces) cp_async16(smem_u32(g_s) + off, P.grows + (ll) a * P.gpad + cob * NCOL + cc * 8);
+                }
+                if (wq == 3) {                                         // rows 128 and 129
+                    const int pl = lane / GP, r = PT + pl;
+                    const int32_t a = __shfl_sync(0xffffffffu, g_extra, pl & 1);
+                    const uint32_t off = NCOL == 32 ? r * 64 + ((cc ^ ((r >> 1) & 3)) << 4) : (cc >> 3) * G_ATOM + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
+                    if (pl < 2 && cc < gpieces) cp_async16(smem_u32(g_s) + off, P.grows + (ll) a * P.gpad + cob * NCOL + cc * 8);
                 }
                 cp_async_arrive_noinc(smem_u32(dfull + db));
             }
@@ -155,6 +180,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
             const __nv_bfloat16* src0 = P.xrows + cib * CIB + c * 8;
 #pragma unroll
             for (int tl = 0; tl < TPT; ++tl) {
+                if (mt * TPT + tl >= nd) break;
                 const int m = tl * CIB + c * 8;                        // accumulator row of this chunk's first channel
                 const uint32_t dst0 = smem_u32(a_s + (m >> 6) * ATOM_STRIDE);
                 const int cc = (m & 63) >> 3;
@@ -163,17 +189,17 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                     const int pl = pi * RPI + r0;
                     const int32_t r = __shfl_sync(0xffffffffu, rows_cur[tl], pl);
                     const int k = wq * 32 + pl;
-                    cp_async16(dst0 + k * 128 + ((cc ^ (k & 7)) << 4), src0 + (ll) r * P.xpad);
+                    if (c < cpieces) cp_async16(dst0 + k * 128 + ((cc ^ (k & 7)) << 4), src0 + (ll) r * P.xpad);
                 }
             }
             // the stage's barrier receives this thread's arrival when the copies above have landed
             cp_async_arrive_noinc(smem_u32(full + slot));
-            if (s_nxt < total_stages) decode_rows(raw_nxt, rows_cur);
+            if (s_nxt < total_stages) decode();
             s = s_nxt;
         }
         cp_async_commit();
         cp_async_wait<0>();
-    } else if (warp == 8 && total_stages > 0) {
+    } else if (warp == MMA_WARP && total_stages > 0) {
         // ---------------- MMA issue ----------------
         if (lane == 0) {
             uint32_t slot = 0, use = 0;
@@ -188,10 +214,15 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                     const uint32_t a_addr = smem_u32(a_ring + (size_t) slot * A_STAGE);
 #pragma unroll
                     for (int k = 0; k < PT / 16; ++k) {
-                        // 16 particles = two 8-row groups of 1024 bytes; atoms along M / N are ATOM_STRIDE apart
+                        // 16 slots = two 8-row groups; atoms along M are ATOM_STRIDE apart, along N one row (the next shift) or, for
+                        // 128 columns, one atom
                         const uint64_t da = make_desc(a_addr + k * 2048, ATOM_STRIDE, 1024, 2);
-                        const uint64_t dbd = make_desc(b_addr + k * 2048, ATOM_STRIDE, 1024, 2);
-                        umma_bf16(tmem_d + mt * NCOL, da, dbd, IDESC, (chunk > 0 || k > 0) ? 1u : 0u);
+#pragma unroll
+                        for (int i = 0; i < MMAS; ++i) {
+                            const uint64_t dbd = NCOL == 32 ? make_desc(b_addr + k * 1024, 64, 512, 4)
+                                                            : make_desc(b_addr + k * 2048 + i * 128, NCOL == 64 ? 128 : G_ATOM, 1024, 2);
+                            umma_bf16(tmem_d + mt * COLS + i * NCOL, da, dbd, IDESC, (chunk > 0 || k > 0) ? 1u : 0u);
+                        }
                     }
                     umma_commit(smem_u32(empty + slot));
                     if (mt == MT - 1) umma_commit(smem_u32(dempty + db));
@@ -208,30 +239,25 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
         if (!mbar_wait_warp(smem_u32(done), 0, abort_flag)) failed = true;
         if (!failed) {
             tc_fence_after();
-            const int row = warp * 32 + lane;                 // accumulator row = (tap within tile) * CIB + ci
+            const int row = warp * 32 + lane;                 // accumulator row = (neighbour within tile) * CIB + ci
             const int tl = row / CIB, ci = cib * CIB + row % CIB;
             for (int mt = 0; mt < MT; ++mt) {
-                const int t = mt * TPT + tl;
-#pragma unroll
-                for (int c0 = 0; c0 < NCOL; c0 += 32) {
+                const int d = mt * TPT + tl;
+#pragma unroll 1
+                for (int c0 = 0; c0 < COLS; c0 += 32) {
                     uint32_t r[32];
-                    tmem_ld32(tmem_d + ((uint32_t) (warp * 32) << 16) + mt * NCOL + c0, r);
+                    tmem_ld32(tmem_d + ((uint32_t) (warp * 32) << 16) + mt * COLS + c0, r);
                     tmem_ld_wait();
-                    if (t < ntaps && ci < P.cin) {
+                    if (d < nd && ci < P.cin) {
+                        const int tap = (d0 + d) * 3 + 2 - c0 / NCOL;      // block i of the columns holds dy = 1 - i
+                        const int co0 = cob * NCOL + c0 % NCOL;
+                        float* o = dst + ((ll) tap * P.cin + ci) * P.cout + co0;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const int co = cob * 256 + c0 + j;
-                            if (co < P.cout) dst[((ll) co * P.cin + ci) * 27 + tap0 + t] = __uint_as_float(r[j]);
-                        }
+                        for (int j = 0; j < 32; ++j)
+                            if (co0 + j < P.cout) o[j] = __uint_as_float(r[j]);
                     }
                 }
             }
-        }
-    } else if (total_stages == 0) {
-        // empty range: this block still owns its slice of the partial buffer
-        for (int e = tid; e < CIB * 256 * ntaps; e += DW_THREADS) {
-            const int t = e % ntaps, ci = cib * CIB + (e / ntaps) % CIB, co = cob * 256 + e / (ntaps * CIB);
-            if (ci < P.cin && co < P.cout) dst[((ll) co * P.cin + ci) * 27 + tap0 + t] = 0.f;
         }
     }
 
@@ -241,24 +267,19 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) tmem_dealloc(tmem_d, 512);
-}
-
-template<typename T>
-__global__ void reduce_partial_kernel(const T* __restrict__ partial, int nchunks, ll elems, T* __restrict__ dst) {
-    const ll e = (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= elems) return;
-    T s = 0;
-    for (int c = 0; c < nchunks; ++c) s += partial[(ll) c * elems + e];
-    dst[e] += s;
+    if (warp == MMA_WARP) tmem_dealloc(tmem_d, 512);
 }
 
 template<int CIB, int NCOL>
 int launch_dw(const DwParams& P, int nranges, int blocks_y, cudaStream_t st, const char* pname) {
-    constexpr size_t G_BYTES = (size_t) (NCOL / 64) * PT * 128;
+    constexpr size_t G_BYTES = ((size_t) G_ROWS * (NCOL == 32 ? 64 : 128) * (NCOL == 128 ? 2 : 1) + 1023) / 1024 * 1024;
     const size_t fixed = 2 * G_BYTES + (2 * DW_MAX_STAGES + 5) * 8 + 16 + 1024;
-    const int nstage = (int) std::min<size_t>(DW_MAX_STAGES, (227 * 1024 - 1024 - fixed) / A_STAGE);
-    if (nstage < 2) { aprnet_set_error("conv333 tensor-core weight gradient: tile does not fit shared memory"); return APRNET_ERR_UNSUPPORTED; }
+    // Every wait on a barrier must find the phase before the awaited one complete (its parity test cannot tell two phases apart).  For
+    // the ring that holds with at least NGROUP stages; for the two dO buffers, filled for chunk c after chunk c - 2 has been read, also
+    // when a chunk is one stage only if the ring has at most four: chunk c - 4 has then been read when stage c is filled.
+    const bool one_tile = (9 - P.d_per_group * (P.groups - 1)) * CIB <= 128 || P.d_per_group * CIB <= 128;
+    const int nstage = (int) std::min<size_t>(one_tile ? 4 : DW_MAX_STAGES, (227 * 1024 - fixed) / A_STAGE);
+    if (nstage < NGROUP) { aprnet_set_error("conv333 tensor-core weight gradient: ring of %d stages", nstage); return APRNET_ERR_UNSUPPORTED; }
     const size_t smem = (size_t) nstage * A_STAGE + fixed;
     auto kern = conv333_tc_dw_kernel<CIB, NCOL>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
@@ -288,18 +309,15 @@ extern "C" int aprnet_conv333_backward_weights_tc(aprnet_apr* a, int dl, int cin
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && xrows && grows && gw && partial, "bad argument");
     APRNET_ARG_CHECK(xpad % 16 == 0 && gpad % 16 == 0 && xpad >= cin && gpad >= cout, "packed row widths must be multiples of 16");
     cudaStream_t st = (cudaStream_t) stream;
-    const AprPlan* plan = aprnet_get_plan(a, dl, st);
-    if (!plan) return APRNET_ERR_CUDA;
-    const ll n = plan->n, t = plan->tree_size;
-    // input-channel block: the widest of 128 / 64 / 32 / 16 that divides the padded width (gathered once when it covers all channels)
-    const int cibk = (xpad % 128 == 0) ? 128 : ((xpad % 64 == 0) ? 64 : ((xpad % 32 == 0) ? 32 : 16));
-    const int ci_blocks = xpad / cibk;
-    const int co_blocks = (gpad + 255) / 256;
-    const int ncol = (std::min(gpad, 256) + 63) / 64 * 64;                 // accumulator columns per tile
-    const int tpt = 128 / cibk;
-    const int max_taps = (512 / ncol) * tpt;                               // taps whose accumulators fit the 512 TMEM columns
-    const int groups = (27 + max_taps - 1) / max_taps;
-    const int taps_per_group = ((27 + groups - 1) / groups + tpt - 1) / tpt * tpt;
+    const RunPlan* rp = aprnet_get_run_plan(a, dl, st);
+    if (!rp) return APRNET_ERR_CUDA;
+    const ll n = a->number_parts(dl), t = a->tree_size(dl);
+    // one block of input channels where they fit (rows are then gathered once per neighbour), 128 at a time beyond
+    const int cib = xpad <= 16 ? 16 : (xpad <= 32 ? 32 : (xpad <= 64 ? 64 : 128));
+    const int ncol = gpad <= 32 ? 32 : (gpad <= 64 ? 64 : 128);
+    const int ci_blocks = (xpad + cib - 1) / cib, co_blocks = (gpad + ncol - 1) / ncol;
+    const int max_d = 512 / (3 * ncol) * (128 / cib);                      // neighbours whose accumulators fit the 512 TMEM columns
+    const int groups = (9 + max_d - 1) / max_d, d_per_group = (9 + groups - 1) / groups;
     const int blocks_y = groups * ci_blocks * co_blocks;
     const ll elems = (ll) 27 * cin * cout;
     const ll max_ranges = aprnet_conv333_tc_dw_partial_elems(cin, cout) / elems;
@@ -309,48 +327,49 @@ extern "C" int aprnet_conv333_backward_weights_tc(aprnet_apr* a, int dl, int cin
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_tc_dw:ci%d:co%d:dl%d", cin, cout, dl);
     // one launch over all levels, blocks for `waves` waves of one block per SM where the partial buffer and the number
-    // of levels allow it: every level gets blocks in proportion to its chunks (at most `per_block` chunks each, at least 4
-    // where the level has that many); a level's partial sums are added into the slot of that level afterwards
+    // of levels allow it: every level gets blocks in proportion to its chunks (at most `per_block` chunks each); a level's partial
+    // sums are added into the slot of that level afterwards
     const std::vector<Segment> segs = aprnet_segments(a, dl, slots, false);
+    DwParams P;
+    P.n_segs = 0;
+    SlotRanges sr;
+    sr.n = 0;
     ll total_chunks = 0;
-    for (const Segment& sg : segs) total_chunks += (sg.end - sg.begin + PT - 1) / PT;
+    for (const Segment& sg : segs) {
+        P.seg_begin[P.n_segs] = rp->level_begin[sg.level]; P.seg_end[P.n_segs] = rp->level_begin[sg.level + 1];
+        total_chunks += (P.seg_end[P.n_segs] - P.seg_begin[P.n_segs] + PT - 1) / PT;
+        ++P.n_segs;
+    }
     if (total_chunks == 0) return APRNET_OK;
     // two waves: a short level then costs a short block rather than an idle SM (1 to 4 waves measured within 5 % of each other)
     const int waves = g_dw_waves_override > 0 ? g_dw_waves_override : 2;
-    ll budget = std::max<ll>((ll) segs.size(), ((ll) waves * sms + blocks_y - 1) / blocks_y);
-    budget = std::max<ll>(1, std::min<ll>(budget, max_ranges));
-    auto blocks_for = [&](ll per_block) { ll b = 0; for (const Segment& sg : segs) b += ((sg.end - sg.begin + PT - 1) / PT + per_block - 1) / per_block; return b; };
-    ll per_block = std::max<ll>(4, (total_chunks + budget - 1) / budget);
+    ll budget = std::max<ll>(P.n_segs, ((ll) waves * sms + blocks_y - 1) / blocks_y);
+    budget = std::max<ll>(P.n_segs, std::min<ll>(budget, max_ranges));
+    auto blocks_of = [&](int i, ll per_block) { return ((P.seg_end[i] - P.seg_begin[i] + PT - 1) / PT + per_block - 1) / per_block; };
+    auto blocks_for = [&](ll per_block) { ll b = 0; for (int i = 0; i < P.n_segs; ++i) b += blocks_of(i, per_block); return b; };
+    ll per_block = std::max<ll>(1, (total_chunks + budget - 1) / budget);
     while (blocks_for(per_block) > budget) ++per_block;
-    DwParams P;
-    P.n_segs = (int) segs.size();
     P.range_first[0] = 0;
     for (int i = 0; i < P.n_segs; ++i) {
-        P.seg_begin[i] = segs[i].begin; P.seg_end[i] = segs[i].end;
-        P.range_first[i + 1] = P.range_first[i] + (int) (((segs[i].end - segs[i].begin + PT - 1) / PT + per_block - 1) / per_block);
+        P.range_first[i + 1] = P.range_first[i] + (int) blocks_of(i, per_block);
+        // levels are listed coarse to fine, so those that share a slot (the last one) are neighbours
+        if (sr.n == 0 || sr.slot[sr.n - 1] != segs[i].slot) { sr.first[sr.n] = P.range_first[i]; sr.slot[sr.n++] = segs[i].slot; }
+        sr.first[sr.n] = P.range_first[i + 1];
     }
     const int nranges = P.range_first[P.n_segs];
     if (nranges > max_ranges) { aprnet_set_error("conv333 tensor-core weight gradient: %d ranges exceed the partial buffer", nranges); return APRNET_ERR_ARG; }
-    P.nbr = plan->nbr; P.N = n;
+    P.src = rp->src; P.S = rp->n_slots; P.loc = rp->loc;
     P.xrows = (const __nv_bfloat16*) xrows; P.xpad = xpad; P.tree_base = n; P.zero_row = n + t;
     P.grows = (const __nv_bfloat16*) grows; P.gpad = gpad; P.g_zero_row = n;
-    P.partial = partial; P.cin = cin; P.cout = cout; P.ci_blocks = ci_blocks; P.groups = groups; P.taps_per_group = taps_per_group;
+    P.partial = partial; P.cin = cin; P.cout = cout; P.ci_blocks = ci_blocks; P.groups = groups; P.d_per_group = d_per_group;
     P.error_flag = aprnet_tc_error_flag_device();
     int rc;
-#define DW_CASE(CIB_, NCOL_) if (cibk == CIB_ && ncol == NCOL_) rc = launch_dw<CIB_, NCOL_>(P, nranges, blocks_y, st, pname); else
-    DW_CASE(16, 64) DW_CASE(16, 128) DW_CASE(16, 192) DW_CASE(16, 256)
-    DW_CASE(32, 64) DW_CASE(32, 128) DW_CASE(32, 192) DW_CASE(32, 256)
-    DW_CASE(64, 64) DW_CASE(64, 128) DW_CASE(64, 192) DW_CASE(64, 256)
-    DW_CASE(128, 64) DW_CASE(128, 128) DW_CASE(128, 192) DW_CASE(128, 256)
+#define DW_CASE(CIB_, NCOL_) if (cib == CIB_ && ncol == NCOL_) rc = launch_dw<CIB_, NCOL_>(P, nranges, blocks_y, st, pname); else
+    DW_CASE(16, 32) DW_CASE(16, 64) DW_CASE(16, 128)
+    DW_CASE(32, 32) DW_CASE(32, 64) DW_CASE(32, 128)
+    DW_CASE(64, 32) DW_CASE(64, 64) DW_CASE(64, 128)
+    DW_CASE(128, 32) DW_CASE(128, 64) DW_CASE(128, 128)
     { aprnet_set_error("conv333 tensor-core weight gradient: unsupported blocking"); return APRNET_ERR_UNSUPPORTED; }
 #undef DW_CASE
-    if (rc) return rc;
-    for (int i = 0; i < P.n_segs; ++i) {
-        const int cnt = P.range_first[i + 1] - P.range_first[i];
-        if (cnt == 0) continue;
-        AprnetProfScope _prof("conv333_dw_reduce", st);
-        reduce_partial_kernel<float><<<aprnet_ceil_div(elems, 256), 256, 0, st>>>(partial + (ll) P.range_first[i] * elems, cnt, elems, gw + (ll) segs[i].slot * elems);
-    }
-    APRNET_LAUNCH_CHECK();
-    return APRNET_OK;
+    return rc ? rc : aprnet_dw_reduce(partial, sr, cin, cout, gw, st);
 }
