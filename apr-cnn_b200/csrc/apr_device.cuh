@@ -126,6 +126,11 @@ struct Segment { long long begin, end; int slot; int level; };
 // With merge=true, consecutive levels that share a slot are fused into one range (1x1x1 conv).
 std::vector<Segment> aprnet_segments(const aprnet_apr* apr, int dl, int num_slots, bool merge);
 
+// memory of the cached tables and of their construction (one pool per device)
+int aprnet_pool_alloc(void** p, size_t bytes, cudaStream_t st);
+void aprnet_pool_free(void* p, cudaStream_t st);
+
+int aprnet_fill_nbr_table(aprnet_apr* a, int dl, int32_t* nbr, long long n, cudaStream_t st);
 const AprPlan* aprnet_get_plan(aprnet_apr* apr, int dl, cudaStream_t stream);
 const int32_t* aprnet_node_parent_table(const aprnet_apr* apr, cudaStream_t stream);            // nullptr on failure
 const int32_t* aprnet_loc_parent_table(const aprnet_apr* apr, int dl, cudaStream_t stream);     // nullptr on failure
@@ -150,7 +155,7 @@ extern "C" int aprnet_conv333_backward_input_cross_level(aprnet_apr* a, int dl, 
 
 const RunPlan* aprnet_get_run_plan(aprnet_apr* apr, int dl, cudaStream_t stream);                // nullptr on failure
 EdgePlan* aprnet_get_edge_plan(aprnet_apr* apr, int dl, cudaStream_t stream);
-void aprnet_free_edge_plan(EdgePlan& ep);
+void aprnet_free_edge_plan(EdgePlan& ep, cudaStream_t st);
 // gather GEMM over the active targets [a0, a1) of an edge plan: grad[target] += sum over taps of
 // W[slot][:, :, tap]^T times virtual row vnbr[tap][a] (rows: bf16 [.. ][gpad], row index relative to `vrows`)
 int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* vrows, int gpad, long long zero_row,

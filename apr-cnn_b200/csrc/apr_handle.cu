@@ -7,6 +7,7 @@
 // index-driven gathers.
 #include "apr_device.cuh"
 #include <cstring>
+#include <mutex>
 #include <algorithm>
 
 static thread_local std::string g_last_error;
@@ -21,6 +22,56 @@ void aprnet_set_error(const char* fmt, ...) {
 }
 
 extern "C" const char* aprnet_last_error(void) { return g_last_error.c_str(); }
+
+// ---- memory of the cached tables and of their construction ------------------------------------------
+// One stream-ordered pool per device, shared by all handles.  cudaMalloc / cudaFree cost about 0.9 and 0.5 ms per table, which was
+// most of the time it took to prepare an access structure.  What is freed (temporaries, the tables of a destroyed handle) stays for
+// the next structure up to POOL_SPARE bytes above what is in use; the driver gives the rest back at the next synchronisation.
+// The driver's allocator is safe with several threads and streams.
+namespace {
+constexpr unsigned long long POOL_SPARE = 2ull << 30;
+constexpr int POOL_DEVICES = 64;
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pools[POOL_DEVICES] = {};
+
+cudaMemPool_t pool_of_device() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= POOL_DEVICES) { cudaGetLastError(); return nullptr; }
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (!g_pools[dev]) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        if (cudaMemPoolCreate(&g_pools[dev], &props) != cudaSuccess) { cudaGetLastError(); g_pools[dev] = nullptr; }
+    }
+    return g_pools[dev];
+}
+
+void pool_keep(cudaMemPool_t pool) {          // reserved memory the pool may hold: what is in use and POOL_SPARE on top
+    unsigned long long used = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) { cudaGetLastError(); return; }
+    used += POOL_SPARE;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &used);
+}
+}
+
+int aprnet_pool_alloc(void** p, size_t bytes, cudaStream_t st) {
+    *p = nullptr;
+    cudaMemPool_t pool = pool_of_device();
+    if (!pool) { aprnet_set_error("no memory pool on this device"); return APRNET_ERR_CUDA; }
+    const cudaError_t e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st);
+    if (e != cudaSuccess) { *p = nullptr; cudaGetLastError(); aprnet_set_error("allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e)); return APRNET_ERR_CUDA; }
+    pool_keep(pool);
+    return APRNET_OK;
+}
+
+void aprnet_pool_free(void* p, cudaStream_t st) {
+    if (!p) return;
+    cudaFreeAsync(p, st);
+    if (cudaMemPool_t pool = pool_of_device()) pool_keep(pool);
+}
 
 // ---- per-kernel event timing -----------------------------------------------------------------
 namespace {
@@ -84,11 +135,6 @@ __device__ __forceinline__ ll lower_bound_y(const uint16_t* __restrict__ y, ll b
     return b;
 }
 
-__device__ __forceinline__ ll find_y(const uint16_t* __restrict__ y, ll b, ll e, int target) {
-    const ll p = lower_bound_y(y, b, e, target);
-    return (p < e && (int) y[p] == target) ? p : -1;
-}
-
 // One warp per tree row of level `l`; lanes stride over the row's nodes.
 __global__ void build_child_table_kernel(LevelMeta m, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y,
                                          const ll* __restrict__ trow_ptr, const uint16_t* __restrict__ ty,
@@ -134,80 +180,10 @@ __global__ void build_child_table_kernel(LevelMeta m, const ll* __restrict__ row
     }
 }
 
-// One warp per output row of level `l`.  Output locations are the APR particles of the row
-// (outputs_are_tree == 0) or, at the current max level of a pooled tensor, its tree nodes
-// (outputs_are_tree == 1, stored at tree index + tree_off).  Cell resolution order follows
-// pyapr/aprnet/src/helpers.hpp:373-408: same-level particle, else the covering particle one level
-// coarser, else the tree node of that cell (stored value at l == cml, tree mean below), else nothing.
-__global__ void build_nbr_table_kernel(LevelMeta m, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y,
-                                       const ll* __restrict__ trow_ptr, const uint16_t* __restrict__ ty,
-                                       int32_t* __restrict__ nbr, ll N, int l, int cml, ll tree_off, int outputs_are_tree) {
-    const ll row = ((ll) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const int xn = m.x_num[l], zn = m.z_num[l], yn = m.y_num[l];
-    if (row >= (ll) zn * xn) return;
-    const int z = (int) (row / xn), x = (int) (row % xn);
-
-    ll ob, oe;
-    const uint16_t* oy;
-    ll shift;
-    if (outputs_are_tree) {
-        const ll tr = m.trow_off[l] + row;
-        ob = trow_ptr[tr]; oe = trow_ptr[tr + 1]; oy = ty; shift = tree_off;
-    } else {
-        const ll r = m.row_off[l] + row;
-        ob = row_ptr[r]; oe = row_ptr[r + 1]; oy = y; shift = 0;
-    }
-    if (ob == oe) return;
-    const bool has_parent = l > m.level_min;
-    const bool has_tree = l <= m.level_max - 1;
-
-    for (int dz = -1; dz <= 1; ++dz) {
-        for (int dx = -1; dx <= 1; ++dx) {
-            const int nz = z + dz, nx = x + dx;
-            const int tap0 = ((dz + 1) * 3 + (dx + 1)) * 3;
-            const bool inside = nz >= 0 && nx >= 0 && nz < zn && nx < xn;
-            ll sb = 0, se = 0, pb = 0, pe = 0, tb = 0, te = 0;
-            if (inside) {
-                const ll r = m.row_off[l] + (ll) nz * xn + nx;
-                sb = row_ptr[r]; se = row_ptr[r + 1];
-                if (has_parent) {
-                    const ll pr = m.row_off[l - 1] + (ll) (nz >> 1) * m.x_num[l - 1] + (nx >> 1);
-                    pb = row_ptr[pr]; pe = row_ptr[pr + 1];
-                }
-                if (has_tree) {
-                    const ll tr = m.trow_off[l] + (ll) nz * xn + nx;
-                    tb = trow_ptr[tr]; te = trow_ptr[tr + 1];
-                }
-            }
-            for (ll i = ob + lane; i < oe; i += 32) {
-                const int yo = oy[i];
-                const ll p = i + shift;
-                for (int dy = -1; dy <= 1; ++dy) {
-                    const int yq = yo + dy;
-                    int32_t v = APRNET_NONE;
-                    if (inside && yq >= 0 && yq < yn) {
-                        ll f = find_y(y, sb, se, yq);
-                        if (f >= 0) v = (int32_t) f;
-                        else {
-                            f = has_parent ? find_y(y, pb, pe, yq >> 1) : -1;
-                            if (f >= 0) v = (int32_t) f;
-                            else {
-                                f = has_tree ? find_y(ty, tb, te, yq) : -1;
-                                if (f >= 0) v = (l == cml) ? (int32_t) (f + tree_off) : aprnet_enc_tree(f);
-                            }
-                        }
-                    }
-                    nbr[(ll) (tap0 + dy + 1) * N + p] = v;
-                }
-            }
-        }
-    }
-}
-
 template<typename T>
 int upload(T** dst, const T* src, size_t n, long long* bytes) {
-    APRNET_CUDA_CHECK(cudaMalloc((void**) dst, std::max<size_t>(n, 1) * sizeof(T)));
+    const int rc = aprnet_pool_alloc((void**) dst, std::max<size_t>(n, 1) * sizeof(T), 0);
+    if (rc) return rc;
     if (n) APRNET_CUDA_CHECK(cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice));
     *bytes += (long long) (std::max<size_t>(n, 1) * sizeof(T));
     return APRNET_OK;
@@ -267,14 +243,16 @@ extern "C" int aprnet_apr_create(aprnet_apr** out, int level_min, int level_max,
     }
     static_assert(sizeof(long long) == sizeof(int64_t), "int64 layout");
     int rc;
-    if ((rc = upload(&a->row_ptr, (const long long*) row_ptr, (size_t) a->n_rows + 1, &a->device_bytes))) { delete a; return rc; }
-    if ((rc = upload(&a->y, y, (size_t) a->n_particles, &a->device_bytes))) { delete a; return rc; }
-    if ((rc = upload(&a->tree_row_ptr, (const long long*) tree_row_ptr, (size_t) a->n_tree_rows + 1, &a->device_bytes))) { delete a; return rc; }
-    if ((rc = upload(&a->tree_y, tree_y, (size_t) a->n_tree, &a->device_bytes))) { delete a; return rc; }
+    if ((rc = upload(&a->row_ptr, (const long long*) row_ptr, (size_t) a->n_rows + 1, &a->device_bytes))) { aprnet_apr_destroy(a); return rc; }
+    if ((rc = upload(&a->y, y, (size_t) a->n_particles, &a->device_bytes))) { aprnet_apr_destroy(a); return rc; }
+    if ((rc = upload(&a->tree_row_ptr, (const long long*) tree_row_ptr, (size_t) a->n_tree_rows + 1, &a->device_bytes))) { aprnet_apr_destroy(a); return rc; }
+    if ((rc = upload(&a->tree_y, tree_y, (size_t) a->n_tree, &a->device_bytes))) { aprnet_apr_destroy(a); return rc; }
 
     const size_t nt = (size_t) std::max<long long>(a->n_tree, 1);
-    APRNET_CUDA_CHECK(cudaMalloc((void**) &a->child, 8 * nt * sizeof(int32_t)));
-    APRNET_CUDA_CHECK(cudaMalloc((void**) &a->tree_scale, nt * sizeof(float)));
+    if ((rc = aprnet_pool_alloc((void**) &a->child, 8 * nt * sizeof(int32_t), 0)) || (rc = aprnet_pool_alloc((void**) &a->tree_scale, nt * sizeof(float), 0))) {
+        aprnet_apr_destroy(a);
+        return rc;
+    }
     a->device_bytes += (long long) (8 * nt * sizeof(int32_t) + nt * sizeof(float));
     for (int l = level_min - 1; l <= level_max - 1; ++l) {
         const long long rows = (long long) m.z_num[l] * m.x_num[l];
@@ -293,13 +271,13 @@ extern "C" void aprnet_apr_destroy(aprnet_apr* a) {
     int prev = -1;
     if (cudaGetDevice(&prev) != cudaSuccess) { prev = -1; cudaGetLastError(); }
     cudaSetDevice(a->device);
-    cudaFree(a->row_ptr); cudaFree(a->y); cudaFree(a->tree_row_ptr); cudaFree(a->tree_y);
-    cudaFree(a->child); cudaFree(a->tree_scale);
-    for (auto& kv : a->plans) cudaFree(kv.second.nbr);
-    cudaFree(a->node_parent);
-    for (auto& kv : a->loc_parent) cudaFree(kv.second);
-    for (auto& kv : a->edge_plans) aprnet_free_edge_plan(kv.second);
-    for (auto& kv : a->run_plans) { cudaFree(kv.second.loc); cudaFree(kv.second.src); }
+    cudaDeviceSynchronize();          // no stream uses the tables any more
+    void* owned[] = {a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, a->child, a->tree_scale, a->node_parent};
+    for (void* p : owned) aprnet_pool_free(p, 0);
+    for (auto& kv : a->plans) aprnet_pool_free(kv.second.nbr, 0);
+    for (auto& kv : a->loc_parent) aprnet_pool_free(kv.second, 0);
+    for (auto& kv : a->edge_plans) aprnet_free_edge_plan(kv.second, 0);
+    for (auto& kv : a->run_plans) { aprnet_pool_free(kv.second.loc, 0); aprnet_pool_free(kv.second.src, 0); }
     delete a;
     if (prev >= 0) cudaSetDevice(prev);
 }
@@ -329,30 +307,10 @@ const AprPlan* aprnet_get_plan(aprnet_apr* a, int dl, cudaStream_t stream) {
     p.level_delta = dl;
     p.n = a->number_parts(dl);
     p.tree_size = a->tree_size(dl);
-    const size_t elems = 27 * (size_t) std::max<long long>(p.n, 1);
-    if (cudaMalloc((void**) &p.nbr, elems * sizeof(int32_t)) != cudaSuccess) {
-        aprnet_set_error("aprnet_plan_build: cudaMalloc of %zu bytes failed", elems * sizeof(int32_t));
-        cudaGetLastError();
-        return nullptr;
-    }
-    a->device_bytes += (long long) (elems * sizeof(int32_t));
-    const LevelMeta& m = a->meta;
-    const int cml = a->cml(dl);
-    const long long toff = (cml <= m.level_max - 1) ? a->tree_offset(cml) : 0;
-    for (int l = m.level_min; l <= cml; ++l) {
-        const long long rows = (long long) m.z_num[l] * m.x_num[l];
-        const int blocks = aprnet_ceil_div(rows * 32, 128);
-        build_nbr_table_kernel<<<blocks, 128, 0, stream>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, p.nbr,
-                                                           p.n, l, cml, toff, 0);
-        if (l == cml && dl > 0)
-            build_nbr_table_kernel<<<blocks, 128, 0, stream>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, p.nbr,
-                                                               p.n, l, cml, toff, 1);
-    }
-    if (cudaGetLastError() != cudaSuccess) {
-        aprnet_set_error("aprnet_plan_build: kernel launch failed");
-        cudaFree(p.nbr);
-        return nullptr;
-    }
+    const size_t bytes = 27 * (size_t) std::max<long long>(p.n, 1) * sizeof(int32_t);
+    if (aprnet_pool_alloc((void**) &p.nbr, bytes, stream)) return nullptr;
+    if (aprnet_fill_nbr_table(a, dl, p.nbr, p.n, stream)) { aprnet_pool_free(p.nbr, stream); return nullptr; }
+    a->device_bytes += (long long) bytes;
     auto res = a->plans.emplace(dl, p);
     return &res.first->second;
 }
@@ -375,14 +333,10 @@ __global__ void build_parent_tables_kernel(const int32_t* __restrict__ child, lo
     }
 }
 
-static int32_t* alloc_minus_one(const aprnet_apr* a, long long n, cudaStream_t stream, const char* what) {
+static int32_t* alloc_minus_one(const aprnet_apr* a, long long n, cudaStream_t stream) {
     int32_t* p = nullptr;
     n = std::max<long long>(n, 1);
-    if (cudaMalloc((void**) &p, (size_t) n * sizeof(int32_t)) != cudaSuccess) {
-        aprnet_set_error("%s: cudaMalloc of %zu bytes failed", what, (size_t) n * sizeof(int32_t));
-        cudaGetLastError();
-        return nullptr;
-    }
+    if (aprnet_pool_alloc((void**) &p, (size_t) n * sizeof(int32_t), stream)) return nullptr;
     a->device_bytes += n * (long long) sizeof(int32_t);
     cudaMemsetAsync(p, 0xFF, (size_t) n * sizeof(int32_t), stream);
     return p;
@@ -390,14 +344,15 @@ static int32_t* alloc_minus_one(const aprnet_apr* a, long long n, cudaStream_t s
 
 const int32_t* aprnet_node_parent_table(const aprnet_apr* a, cudaStream_t stream) {
     if (a->node_parent) return a->node_parent;
-    int32_t* tab = alloc_minus_one(a, a->n_tree, stream, "aprnet_node_parent_table");
+    int32_t* tab = alloc_minus_one(a, a->n_tree, stream);
     if (!tab) return nullptr;
     const LevelMeta& m = a->meta;
     for (int lp = m.level_min - 1; lp <= m.level_max - 1; ++lp) {
         const long long tb = m.tlvl_begin[lp], te = m.tlvl_begin[lp + 1];
         if (te > tb) build_parent_tables_kernel<<<aprnet_ceil_div(te - tb, 256), 256, 0, stream>>>(a->child, a->n_tree, tb, te, 0, 0, nullptr, tab);
     }
-    if (cudaGetLastError() != cudaSuccess) { aprnet_set_error("aprnet_node_parent_table: kernel launch failed"); cudaFree(tab); return nullptr; }
+    if (cudaGetLastError() != cudaSuccess) { aprnet_set_error("aprnet_node_parent_table: kernel launch failed"); aprnet_pool_free(tab, stream); return nullptr; }
+    if (cudaStreamSynchronize(stream) != cudaSuccess) return nullptr;          // usable on any stream from here on
     a->node_parent = tab;
     return tab;
 }
@@ -405,7 +360,7 @@ const int32_t* aprnet_node_parent_table(const aprnet_apr* a, cudaStream_t stream
 const int32_t* aprnet_loc_parent_table(const aprnet_apr* a, int dl, cudaStream_t stream) {
     auto it = a->loc_parent.find(dl);
     if (it != a->loc_parent.end()) return it->second;
-    int32_t* tab = alloc_minus_one(a, a->number_parts(dl), stream, "aprnet_loc_parent_table");
+    int32_t* tab = alloc_minus_one(a, a->number_parts(dl), stream);
     if (!tab) return nullptr;
     const LevelMeta& m = a->meta;
     const int cml = a->cml(dl);
@@ -415,7 +370,8 @@ const int32_t* aprnet_loc_parent_table(const aprnet_apr* a, int dl, cudaStream_t
         if (te > tb) build_parent_tables_kernel<<<aprnet_ceil_div(te - tb, 256), 256, 0, stream>>>(a->child, a->n_tree, tb, te, up,
                                                                                                  (dl > 0 && lp + 1 == cml) ? 1 : 0, tab, nullptr);
     }
-    if (cudaGetLastError() != cudaSuccess) { aprnet_set_error("aprnet_loc_parent_table: kernel launch failed"); cudaFree(tab); return nullptr; }
+    if (cudaGetLastError() != cudaSuccess) { aprnet_set_error("aprnet_loc_parent_table: kernel launch failed"); aprnet_pool_free(tab, stream); return nullptr; }
+    if (cudaStreamSynchronize(stream) != cudaSuccess) return nullptr;
     a->loc_parent.emplace(dl, tab);
     return tab;
 }

@@ -13,6 +13,7 @@
 #include <cub/cub.cuh>
 #include <cuda_bf16.h>
 #include <algorithm>
+#include <cstring>
 
 namespace {
 
@@ -176,16 +177,16 @@ __global__ void __launch_bounds__(256) vrow_reduce_kernel(const int32_t* __restr
 constexpr ll VROW_GRANULE = 4ll << 20;      // virtual rows per entry of the chunk map
 
 template<typename T>
-int dev_alloc(T** p, size_t n, long long* bytes) {
-    APRNET_CUDA_CHECK(cudaMalloc((void**) p, std::max<size_t>(n, 1) * sizeof(T)));
-    if (bytes) *bytes += (long long) (std::max<size_t>(n, 1) * sizeof(T));
-    return APRNET_OK;
+int dev_alloc(T** p, size_t n, long long* bytes, cudaStream_t st) {
+    const int rc = aprnet_pool_alloc((void**) p, std::max<size_t>(n, 1) * sizeof(T), st);
+    if (!rc && bytes) *bytes += (long long) (std::max<size_t>(n, 1) * sizeof(T));
+    return rc;
 }
 
 } // namespace
 
-void aprnet_free_edge_plan(EdgePlan& ep) {
-    cudaFree(ep.vsrc); cudaFree(ep.vstart); cudaFree(ep.active); cudaFree(ep.vnbr);
+void aprnet_free_edge_plan(EdgePlan& ep, cudaStream_t st) {
+    aprnet_pool_free(ep.vsrc, st); aprnet_pool_free(ep.vstart, st); aprnet_pool_free(ep.active, st); aprnet_pool_free(ep.vnbr, st);
     ep = EdgePlan();
 }
 
@@ -203,33 +204,33 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
     ll *keys = nullptr, *found = nullptr;
     void* temp = nullptr;
     int rc = APRNET_OK;
-    auto cleanup = [&]() { cudaFree(scan); cudaFree(src); cudaFree(tgt); cudaFree(count); cudaFree(tgt_ptr); cudaFree(tgt_edge);
-                           cudaFree(vfirst); cudaFree(keys); cudaFree(found); cudaFree(temp); };
+    auto cleanup = [&]() { void* all[] = {scan, src, tgt, count, tgt_ptr, tgt_edge, vfirst, keys, found, temp}; for (void* p : all) aprnet_pool_free(p, st); };
+#define EP_ALLOC(p, n) do { if ((rc = dev_alloc(&(p), (size_t) (n), nullptr, st))) { cleanup(); return rc; } } while (0)
 #define EP_CHECK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) { aprnet_set_error("%s failed: %s", #expr, cudaGetErrorString(_e)); cleanup(); return APRNET_ERR_CUDA; } } while (0)
 
-    EP_CHECK(cudaMalloc((void**) &scan, (size_t) (F + 1) * sizeof(int32_t)));
+    EP_ALLOC(scan, F + 1);
     edge_flag_kernel<<<aprnet_ceil_div(F + 1, 256), 256, 0, st>>>(plan->nbr, N, lr, scan);
     size_t temp_bytes = 0, temp2 = 0;
     EP_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, scan, scan, (int) (F + 1), st));
     EP_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, temp2, scan, scan, (int) (NT + 2), st));
     temp_bytes = std::max(temp_bytes, temp2);
-    EP_CHECK(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 1)));
+    if ((rc = aprnet_pool_alloc(&temp, std::max<size_t>(temp_bytes, 1), st))) { cleanup(); return rc; }
     EP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, scan, scan, (int) (F + 1), st));
 
     // first edge id of every tap
     TapBegin tb;
-    for (int tap = 0; tap <= 27; ++tap)
-        EP_CHECK(cudaMemcpyAsync(&tb.b[tap], scan + (ll) tap * N, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    if (N > 0) EP_CHECK(cudaMemcpy2DAsync(tb.b, sizeof(int32_t), scan, (size_t) N * sizeof(int32_t), sizeof(int32_t), 28, cudaMemcpyDeviceToHost, st));
+    else memset(&tb, 0, sizeof(tb));
     EP_CHECK(cudaStreamSynchronize(st));
     const ll E = tb.b[27];
     ep.n_edges = E; ep.n_targets = NT;
 
     // per-edge source and target, per-target ascending edge lists, active targets
-    EP_CHECK(cudaMalloc((void**) &src, std::max<size_t>(E, 1) * sizeof(int32_t)));
-    EP_CHECK(cudaMalloc((void**) &tgt, std::max<size_t>(E, 1) * sizeof(int32_t)));
-    EP_CHECK(cudaMalloc((void**) &tgt_edge, std::max<size_t>(E, 1) * sizeof(int32_t)));
-    EP_CHECK(cudaMalloc((void**) &tgt_ptr, (size_t) (NT + 1) * sizeof(int32_t)));
-    EP_CHECK(cudaMalloc((void**) &count, (size_t) (NT + 1) * sizeof(int32_t)));
+    EP_ALLOC(src, E);
+    EP_ALLOC(tgt, E);
+    EP_ALLOC(tgt_edge, E);
+    EP_ALLOC(tgt_ptr, NT + 1);
+    EP_ALLOC(count, NT + 1);
     EP_CHECK(cudaMemsetAsync(count, 0, (size_t) (NT + 1) * sizeof(int32_t), st));
     edge_emit_kernel<<<aprnet_ceil_div(F, 256), 256, 0, st>>>(plan->nbr, N, scan, src, tgt, count);
     EP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, count, tgt_ptr, (int) (NT + 1), st));
@@ -241,21 +242,21 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
     EP_CHECK(cudaMemcpyAsync(&n_active, count + NT, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     EP_CHECK(cudaStreamSynchronize(st));
     ep.n_active = n_active;
-    if ((rc = dev_alloc(&ep.active, (size_t) n_active, &a->device_bytes))) { cleanup(); return rc; }
+    if ((rc = dev_alloc(&ep.active, (size_t) n_active, &a->device_bytes, st))) { cleanup(); return rc; }
     if (NT) edge_compact_active_kernel<<<aprnet_ceil_div(NT, 256), 256, 0, st>>>(count, NT, ep.active);
-    cudaFree(scan); scan = nullptr;
-    cudaFree(tgt); tgt = nullptr;
+    aprnet_pool_free(scan, st); scan = nullptr;
+    aprnet_pool_free(tgt, st); tgt = nullptr;
 
     // virtual rows: runs of equal tap in every active target's list
-    EP_CHECK(cudaMalloc((void**) &vfirst, (size_t) (n_active + 1) * sizeof(int32_t)));
+    EP_ALLOC(vfirst, n_active + 1);
     vrow_count_kernel<<<aprnet_ceil_div((ll) n_active + 1, 128), 128, 0, st>>>(ep.active, n_active, tgt_ptr, tgt_edge, tb, vfirst);
     EP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, vfirst, vfirst, n_active + 1, st));
     int32_t n_vrows = 0;
     EP_CHECK(cudaMemcpyAsync(&n_vrows, vfirst + n_active, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     EP_CHECK(cudaStreamSynchronize(st));
     ep.n_vrows = n_vrows;
-    if ((rc = dev_alloc(&ep.vsrc, (size_t) E, &a->device_bytes)) || (rc = dev_alloc(&ep.vstart, (size_t) n_vrows + 1, &a->device_bytes)) ||
-        (rc = dev_alloc(&ep.vnbr, (size_t) 27 * std::max(n_active, 1), &a->device_bytes))) { cleanup(); return rc; }
+    if ((rc = dev_alloc(&ep.vsrc, (size_t) E, &a->device_bytes, st)) || (rc = dev_alloc(&ep.vstart, (size_t) n_vrows + 1, &a->device_bytes, st)) ||
+        (rc = dev_alloc(&ep.vnbr, (size_t) 27 * std::max(n_active, 1), &a->device_bytes, st))) { cleanup(); return rc; }
     EP_CHECK(cudaMemsetAsync(ep.vnbr, 0xFF, (size_t) 27 * std::max(n_active, 1) * sizeof(int32_t), st));       // APRNET_NONE
     EP_CHECK(cudaMemsetAsync(ep.vstart, 0, ((size_t) n_vrows + 1) * sizeof(int32_t), st));
     if (n_active) vrow_fill_kernel<<<aprnet_ceil_div(n_active, 128), 128, 0, st>>>(ep.active, n_active, tgt_ptr, tgt_edge, src, tb, vfirst, E,
@@ -274,8 +275,8 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
     key_h.push_back(NT); key_level.push_back(-1);
     const int nkeys = (int) key_h.size();
     const int nchunk = (int) (n_vrows / VROW_GRANULE) + 1;
-    EP_CHECK(cudaMalloc((void**) &keys, (size_t) std::max(nkeys, nchunk + 1) * sizeof(ll)));
-    EP_CHECK(cudaMalloc((void**) &found, (size_t) std::max(nkeys, nchunk + 1) * sizeof(ll)));
+    EP_ALLOC(keys, std::max(nkeys, nchunk + 1));
+    EP_ALLOC(found, std::max(nkeys, nchunk + 1));
     std::vector<ll> found_h(std::max(nkeys, nchunk + 1));
     EP_CHECK(cudaMemcpyAsync(keys, key_h.data(), nkeys * sizeof(ll), cudaMemcpyHostToDevice, st));
     lower_bound_kernel<<<1, 64, 0, st>>>(ep.active, n_active, keys, nkeys, found);
@@ -308,6 +309,7 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
     EP_CHECK(cudaGetLastError());
     EP_CHECK(cudaStreamSynchronize(st));
 #undef EP_CHECK
+#undef EP_ALLOC
     cleanup();
     return APRNET_OK;
 }
@@ -318,7 +320,7 @@ EdgePlan* aprnet_get_edge_plan(aprnet_apr* a, int dl, cudaStream_t st) {
     const AprPlan* plan = aprnet_get_plan(a, dl, st);
     if (!plan) return nullptr;
     EdgePlan ep;
-    if (build_edge_plan(a, dl, plan, ep, st) != APRNET_OK) { aprnet_free_edge_plan(ep); return nullptr; }
+    if (build_edge_plan(a, dl, plan, ep, st) != APRNET_OK) { aprnet_free_edge_plan(ep, st); return nullptr; }
     auto res = a->edge_plans.emplace(dl, ep);
     return &res.first->second;
 }

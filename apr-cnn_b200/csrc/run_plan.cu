@@ -108,6 +108,22 @@ __global__ void run_sources_kernel(LevelMeta m, const ll* __restrict__ row_ptr, 
     }
 }
 
+// the neighbour table from the run plan: the three y neighbours of a location are its slot and the slots beside it, in the nine rows
+__global__ void nbr_from_runs_kernel(const int32_t* __restrict__ loc, const int32_t* __restrict__ src, ll S, int32_t* __restrict__ nbr, ll N) {
+    const ll s = (ll) blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= S) return;
+    const int32_t p = loc[s];
+    if (p < 0) return;                 // a location has a slot on either side, so s - 1 and s + 1 exist
+    int32_t v[27];
+#pragma unroll
+    for (int t = 0; t < 27; ++t) v[t] = src[(ll) (t / 3) * S + s + t % 3 - 1];
+#pragma unroll
+    for (int t = 0; t < 27; ++t) nbr[(ll) t * N + p] = v[t];
+}
+
+struct Picks { ll at[APRNET_MAX_LEVELS + 2]; };
+__global__ void pick_kernel(const int32_t* __restrict__ v, Picks at, int n, int32_t* __restrict__ out) { if ((int) threadIdx.x < n) out[threadIdx.x] = v[at.at[threadIdx.x]]; }
+
 int build_run_plan(aprnet_apr* a, int dl, RunPlan& rp, cudaStream_t st) {
     const LevelMeta& m = a->meta;
     const int cml = a->cml(dl);
@@ -116,30 +132,34 @@ int build_run_plan(aprnet_apr* a, int dl, RunPlan& rp, cudaStream_t st) {
     std::vector<ll> row_begin(cml + 2, 0);
     for (int l = m.level_min; l <= cml; ++l) { row_begin[l] = rows; rows += (ll) m.z_num[l] * m.x_num[l]; }
     row_begin[cml + 1] = rows;
-    int32_t *first = nullptr, *slot_y = nullptr;
+    int32_t *first = nullptr, *slot_y = nullptr, *picked = nullptr;
+    int rc = APRNET_OK;
     void* temp = nullptr;
     size_t temp_bytes = 0;
-    auto cleanup = [&]() { cudaFree(first); cudaFree(slot_y); cudaFree(temp); };
+    auto cleanup = [&]() { aprnet_pool_free(first, st); aprnet_pool_free(slot_y, st); aprnet_pool_free(picked, st); aprnet_pool_free(temp, st); };
+#define RP_ALLOC(p, bytes) do { if ((rc = aprnet_pool_alloc((void**) &(p), (bytes), st))) { cleanup(); return rc; } } while (0)
 #define RP_CHECK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) { aprnet_set_error("%s failed: %s", #expr, cudaGetErrorString(_e)); cudaGetLastError(); cleanup(); return APRNET_ERR_CUDA; } } while (0)
-    RP_CHECK(cudaMalloc((void**) &first, (size_t) (rows + 1) * sizeof(int32_t)));
+    RP_ALLOC(first, (size_t) (rows + 1) * sizeof(int32_t));
     RP_CHECK(cudaMemsetAsync(first + rows, 0, sizeof(int32_t), st));
     for (int l = m.level_min; l <= cml; ++l)
         run_slots_kernel<<<aprnet_ceil_div((ll) m.z_num[l] * m.x_num[l], 128), 128, 0, st>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, l, dl > 0 && l == cml, toff,
                                                                                        first + row_begin[l], nullptr, nullptr, nullptr);
     RP_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, first, first, (int) (rows + 1), st));
-    RP_CHECK(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 1)));
+    RP_ALLOC(temp, std::max<size_t>(temp_bytes, 1));
     RP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, first, first, (int) (rows + 1), st));
     std::vector<int32_t> at(cml + 2, 0);
-    for (int l = m.level_min; l <= cml + 1; ++l)
-        RP_CHECK(cudaMemcpyAsync(&at[l], first + row_begin[l], sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    Picks picks;
+    for (int l = m.level_min; l <= cml + 1; ++l) picks.at[l - m.level_min] = row_begin[l];
+    RP_ALLOC(picked, sizeof(int32_t) * (APRNET_MAX_LEVELS + 2));
+    pick_kernel<<<1, 32, 0, st>>>(first, picks, cml + 2 - m.level_min, picked);
+    RP_CHECK(cudaMemcpyAsync(at.data() + m.level_min, picked, sizeof(int32_t) * (cml + 2 - m.level_min), cudaMemcpyDeviceToHost, st));
     RP_CHECK(cudaStreamSynchronize(st));
     const ll S = at[cml + 1];
     rp.n_slots = S;
     rp.level_begin.assign(at.begin(), at.end());
-    RP_CHECK(cudaMalloc((void**) &slot_y, (size_t) std::max<ll>(S, 1) * sizeof(int32_t)));
-    RP_CHECK(cudaMalloc((void**) &rp.loc, (size_t) std::max<ll>(S, 1) * sizeof(int32_t)));
-    RP_CHECK(cudaMalloc((void**) &rp.src, (size_t) std::max<ll>(S, 1) * 9 * sizeof(int32_t)));
-    a->device_bytes += std::max<ll>(S, 1) * 10 * (ll) sizeof(int32_t);
+    RP_ALLOC(slot_y, (size_t) std::max<ll>(S, 1) * sizeof(int32_t));
+    RP_ALLOC(rp.loc, (size_t) std::max<ll>(S, 1) * sizeof(int32_t));
+    RP_ALLOC(rp.src, (size_t) std::max<ll>(S, 1) * 9 * sizeof(int32_t));
     for (int l = m.level_min; l <= cml; ++l) {
         const ll n = (ll) m.z_num[l] * m.x_num[l];
         run_slots_kernel<<<aprnet_ceil_div(n, 128), 128, 0, st>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, l, dl > 0 && l == cml, toff, nullptr,
@@ -149,6 +169,7 @@ int build_run_plan(aprnet_apr* a, int dl, RunPlan& rp, cudaStream_t st) {
     RP_CHECK(cudaGetLastError());
     RP_CHECK(cudaStreamSynchronize(st));
 #undef RP_CHECK
+#undef RP_ALLOC
     cleanup();
     return APRNET_OK;
 }
@@ -160,8 +181,24 @@ const RunPlan* aprnet_get_run_plan(aprnet_apr* a, int dl, cudaStream_t st) {
     if (it != a->run_plans.end()) return &it->second;
     if (aprnet_check_device(a) != APRNET_OK) return nullptr;
     RunPlan rp;
-    if (build_run_plan(a, dl, rp, st) != APRNET_OK) { cudaFree(rp.loc); cudaFree(rp.src); return nullptr; }
+    if (build_run_plan(a, dl, rp, st) != APRNET_OK) { aprnet_pool_free(rp.loc, st); aprnet_pool_free(rp.src, st); return nullptr; }
+    a->device_bytes += std::max<ll>(rp.n_slots, 1) * 10 * (ll) sizeof(int32_t);
     return &a->run_plans.emplace(dl, rp).first->second;
+}
+
+// nbr: [27][n].  Nine searches per slot and a copy instead of 27 searches per location; a run plan that is not cached is built for it.
+int aprnet_fill_nbr_table(aprnet_apr* a, int dl, int32_t* nbr, ll n, cudaStream_t st) {
+    const auto it = a->run_plans.find(dl);
+    RunPlan own;
+    const RunPlan* rp = it != a->run_plans.end() ? &it->second : &own;
+    int rc = APRNET_OK;
+    if (rp == &own) rc = build_run_plan(a, dl, own, st);
+    if (!rc && rp->n_slots > 0) {
+        nbr_from_runs_kernel<<<aprnet_ceil_div(rp->n_slots, 256), 256, 0, st>>>(rp->loc, rp->src, rp->n_slots, nbr, n);
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) { aprnet_set_error("aprnet_fill_nbr_table: kernel failed"); rc = APRNET_ERR_CUDA; }
+    }
+    aprnet_pool_free(own.loc, st); aprnet_pool_free(own.src, st);
+    return rc;
 }
 
 // Builds (once; cached) the run plan of a level delta.  Allocates; call it up front.
