@@ -495,7 +495,7 @@ void fill_tree_mean_backward_inplace(std::vector<APR*>& aprs, torch::Tensor grad
 
 // ---- 1x1x1 convolution ------------------------------------------------------------------------
 torch::Tensor conv111_forward(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights, torch::Tensor level_delta,
-                              const std::string& precision) {
+                              const std::string& precision, c10::optional<torch::Tensor> bias) {
     CHECK_INPUT(input); CHECK_INPUT(weights);
     check_batch(aprs, input);
     TORCH_CHECK(weights.dim() == 6 && weights.size(3) == 1 && weights.size(4) == 1 && weights.size(5) == 1, "weights must be (stencils, Cout, Cin, 1, 1, 1)");
@@ -505,21 +505,24 @@ torch::Tensor conv111_forward(std::vector<APR*>& aprs, torch::Tensor input, torc
     const int64_t cin = input.size(1), cout = weights.size(1), n = input.size(2);
     auto output = torch::empty({input.size(0), cout, n}, input.options());
     const int dt = dtype_id(input);
+    const bool has_bias = bias.has_value() && bias->defined();
+    if (has_bias) TORCH_CHECK(bias->is_cuda() && bias->is_contiguous() && bias->numel() == cout && bias->scalar_type() == input.scalar_type(), "bias must be (Cout) of the input's dtype on the device");
+    const void* bp = has_bias ? bias->data_ptr() : nullptr;
     const bool tc = resolve_mode(precision) == 1 && dt == APRNET_F32;
     for (int64_t b = 0; b < input.size(0); ++b) {
         check_level_delta(*aprs[b], dl[b]);
         // tensor cores where the layer asks for bf16 arithmetic and the weights fit shared memory; CUDA cores otherwise
         int rc = APRNET_ERR_UNSUPPORTED;
         if (tc) {
-            rc = aprnet_conv111_forward_tc(aprs[b]->handle(input), dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n,
-                                           (const float*) weights.data_ptr(), (float*) row(output, b), n, stream_of(input));
+            rc = aprnet_conv111_forward_tc_bias(aprs[b]->handle(input), dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n,
+                                           (const float*) weights.data_ptr(), (const float*) bp, (float*) row(output, b), n, stream_of(input));
             if (rc != APRNET_ERR_UNSUPPORTED) check(rc, "conv111_forward (tensor cores)");
         }
         if (rc == APRNET_ERR_UNSUPPORTED)
-        check(aprnet_conv111_forward(aprs[b]->handle(input), dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
-                                     weights.data_ptr(), row(output, b), n, stream_of(input)), "conv111_forward");
+        check(aprnet_conv111_forward_bias(aprs[b]->handle(input), dl[b], dt, (int) cin, (int) cout, (int) weights.size(0), row(input, b), n,
+                                     weights.data_ptr(), bp, row(output, b), n, stream_of(input)), "conv111_forward");
     }
-    fill_padding(output, valid_of(aprs, dl));
+    fill_padding(output, valid_of(aprs, dl), has_bias ? *bias : torch::Tensor());
     return output;
 }
 
@@ -961,7 +964,7 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
     py::module cuda = aprnet.def_submodule("cuda");
     cuda.def("maxpool_forward_cuda", &maxpool_forward_cuda, "aprs"_a, "input"_a, "level_delta"_a);
     cuda.def("maxpool_backward_cuda", &maxpool_backward_cuda, "aprs"_a, "grad_output"_a, "max_indices"_a, "level_delta"_a);
-    cuda.def("conv111_forward", &conv111_forward, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "");
+    cuda.def("conv111_forward", &conv111_forward, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "", "bias"_a = py::none());
     cuda.def("conv111_backward", &conv111_backward, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "precision"_a = "");
     cuda.def("conv333_forward", &conv333_forward, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a);
     cuda.def("conv333_backward", &conv333_backward, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a);

@@ -172,7 +172,9 @@ int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int 
 int aprnet_tc_runs_order(int backward, int kpad, int nt, int ks);
 int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, long long tree_base, long long zero_row, const void* wp,
                        const float* bias, float* out, long long ld_out, int n_dim, int* error_flag, cudaStream_t st, const char* pname);
-int aprnet_tc_pack_weights(const float* w, int slots, int cin, int cout, int mode, void* wp, cudaStream_t st);
+int aprnet_pack_weights(const aprnet_apr* a, int dl, bool bf16, const float* w, int slots, int cin, int cout, int transposed, int nt, int n_tiles, int kpad,
+                        void* out, cudaStream_t st);
+int aprnet_tc_pack_weights(const aprnet_apr* a, int dl, const float* w, int slots, int cin, int cout, int transposed, void* wp, cudaStream_t st);
 size_t aprnet_tc_weight_bytes(int k_dim, int n_dim, int slots);
 size_t aprnet_tc_rows_bytes(long long rows, int channels);
 int aprnet_tc_pad(int channels);

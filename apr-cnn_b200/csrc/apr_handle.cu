@@ -316,10 +316,10 @@ const AprPlan* aprnet_get_plan(aprnet_apr* a, int dl, cudaStream_t stream) {
 }
 
 // Parent tables from the child table: every child slot of tree node t names a particle (v >= 0), a tree node (coded) or,
-// at the finest tree level of a level delta > 0 (use_up), an upgraded node that lives in the feature vector at
+// from the node up_from on (the finest tree level of a level delta > 0), an upgraded node that lives in the feature vector at
 // up_off + index.  Either output may be null.
 __global__ void build_parent_tables_kernel(const int32_t* __restrict__ child, long long n_tree, long long tb, long long te,
-                                           long long up_off, int use_up, int32_t* __restrict__ loc_parent, int32_t* __restrict__ node_parent) {
+                                           long long up_off, long long up_from, int32_t* __restrict__ loc_parent, int32_t* __restrict__ node_parent) {
     const long long t = tb + (long long) blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= te) return;
 #pragma unroll
@@ -327,7 +327,7 @@ __global__ void build_parent_tables_kernel(const int32_t* __restrict__ child, lo
         const int32_t v = child[(long long) s * n_tree + t];
         if (v >= 0) { if (loc_parent) loc_parent[v] = (int32_t) t; }
         else if (v != APRNET_NONE) {
-            if (use_up) { if (loc_parent) loc_parent[aprnet_dec_tree(v) + up_off] = (int32_t) t; }
+            if (t >= up_from) { if (loc_parent) loc_parent[aprnet_dec_tree(v) + up_off] = (int32_t) t; }
             else if (node_parent) node_parent[aprnet_dec_tree(v)] = (int32_t) t;
         }
     }
@@ -346,11 +346,7 @@ const int32_t* aprnet_node_parent_table(const aprnet_apr* a, cudaStream_t stream
     if (a->node_parent) return a->node_parent;
     int32_t* tab = alloc_minus_one(a, a->n_tree, stream);
     if (!tab) return nullptr;
-    const LevelMeta& m = a->meta;
-    for (int lp = m.level_min - 1; lp <= m.level_max - 1; ++lp) {
-        const long long tb = m.tlvl_begin[lp], te = m.tlvl_begin[lp + 1];
-        if (te > tb) build_parent_tables_kernel<<<aprnet_ceil_div(te - tb, 256), 256, 0, stream>>>(a->child, a->n_tree, tb, te, 0, 0, nullptr, tab);
-    }
+    if (a->n_tree > 0) build_parent_tables_kernel<<<aprnet_ceil_div(a->n_tree, 256), 256, 0, stream>>>(a->child, a->n_tree, 0, a->n_tree, 0, a->n_tree, nullptr, tab);
     if (cudaGetLastError() != cudaSuccess) { aprnet_set_error("aprnet_node_parent_table: kernel launch failed"); aprnet_pool_free(tab, stream); return nullptr; }
     if (cudaStreamSynchronize(stream) != cudaSuccess) return nullptr;          // usable on any stream from here on
     a->node_parent = tab;
@@ -364,12 +360,9 @@ const int32_t* aprnet_loc_parent_table(const aprnet_apr* a, int dl, cudaStream_t
     if (!tab) return nullptr;
     const LevelMeta& m = a->meta;
     const int cml = a->cml(dl);
-    const long long up = (dl > 0) ? a->tree_offset(cml) : 0;
-    for (int lp = m.level_min - 1; lp <= cml - 1; ++lp) {
-        const long long tb = m.tlvl_begin[lp], te = m.tlvl_begin[lp + 1];
-        if (te > tb) build_parent_tables_kernel<<<aprnet_ceil_div(te - tb, 256), 256, 0, stream>>>(a->child, a->n_tree, tb, te, up,
-                                                                                                 (dl > 0 && lp + 1 == cml) ? 1 : 0, tab, nullptr);
-    }
+    const long long te = m.tlvl_begin[cml];          // nodes of levels below cml
+    if (te > 0) build_parent_tables_kernel<<<aprnet_ceil_div(te, 256), 256, 0, stream>>>(a->child, a->n_tree, 0, te, dl > 0 ? a->tree_offset(cml) : 0,
+                                                                                       dl > 0 ? m.tlvl_begin[cml - 1] : te, tab, nullptr);
     if (cudaGetLastError() != cudaSuccess) { aprnet_set_error("aprnet_loc_parent_table: kernel launch failed"); aprnet_pool_free(tab, stream); return nullptr; }
     if (cudaStreamSynchronize(stream) != cudaSuccess) return nullptr;
     a->loc_parent.emplace(dl, tab);

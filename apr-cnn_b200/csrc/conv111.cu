@@ -1,6 +1,6 @@
-// 1x1x1 particle convolution (per-level channel mixing) and stencil restriction.
+// 1x1x1 particle convolution (per-level channel mixing).
 //
-// Replaces pyapr/aprnet/cuda/src/conv111_gpu.cu:9-232 and restrict_gpu.cu:5-235.  The reference
+// Replaces pyapr/aprnet/cuda/src/conv111_gpu.cu:9-232.  The reference
 // splits input channels over grid.z and combines them with atomicAdd into a zero-filled output; here
 // one thread owns a particle and a block of output channels, loops over all input channels and
 // writes each output once (no atomics, deterministic).  Weight gradients are block-local partial
@@ -46,7 +46,7 @@ template<> struct Vec16<double> { typedef double2 type; static constexpr int N =
 template<typename T, int OB, int TPB, int PPT>
 __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 2 : 1) conv111_kernel(SegTable segs, const T* __restrict__ in, ll ld_in,
                                                       const T* __restrict__ w, ll ws, ll wo, ll wi,
-                                                      T* __restrict__ out, ll ld_out, int n_in, int n_out) {
+                                                      const T* __restrict__ bias, T* __restrict__ out, ll ld_out, int n_in, int n_out) {
     typedef typename Vec16<T>::type V;
     constexpr int VN = Vec16<T>::N;
     static_assert(OB % VN == 0, "output block is a whole number of 16-byte vectors");
@@ -97,6 +97,14 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 2 : 1) conv111_kernel(Se
 #pragma unroll
         for (int q = 0; q < PPT; ++q) v[q] = (p0 + (ll) q * TPB < pend) ? in[(ll) i * ld_in + p0 + (ll) q * TPB] : T(0);
         mix(v, i);
+    }
+    if (bias) {
+#pragma unroll
+        for (int o = 0; o < OB; ++o) {
+            const T b = o0 + o < n_out ? bias[o0 + o] : T(0);
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) acc[q][o] += b;
+        }
     }
 #pragma unroll
     for (int q = 0; q < PPT; ++q) {
@@ -226,7 +234,7 @@ __global__ void reduce_partial_kernel(const T* __restrict__ partial, int nchunks
 inline int dw_max_chunks(int cin, int cout) { return (int) std::max<ll>(128, std::min<ll>(2048, (16ll << 20) / ((ll) cin * cout))); }
 
 template<typename T, int OB, int TPB, int PPT>
-int conv111_launch(const aprnet_apr* a, int dl, int S, const T* in, ll ld_in, const T* w, ll ws, ll wo, ll wi, T* out, ll ld_out,
+int conv111_launch(const aprnet_apr* a, int dl, int S, const T* in, ll ld_in, const T* w, ll ws, ll wo, ll wi, const T* bias, T* out, ll ld_out,
                    int n_in, int n_out, cudaStream_t st) {
     const SegTable segs = make_seg_table(aprnet_segments(a, dl, S, true), TPB * PPT);
     const int tiles = segs.tile_begin[segs.n];
@@ -236,7 +244,7 @@ int conv111_launch(const aprnet_apr* a, int dl, int S, const T* in, ll ld_in, co
         APRNET_CUDA_CHECK(cudaFuncSetAttribute(conv111_kernel<T, OB, TPB, PPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     dim3 grid((unsigned) tiles, (unsigned) aprnet_ceil_div(n_out, OB));
     { AprnetProfScope _prof("conv111", st);
-    conv111_kernel<T, OB, TPB, PPT><<<grid, TPB, smem, st>>>(segs, in, ld_in, w, ws, wo, wi, out, ld_out, n_in, n_out);
+    conv111_kernel<T, OB, TPB, PPT><<<grid, TPB, smem, st>>>(segs, in, ld_in, w, ws, wo, wi, bias, out, ld_out, n_in, n_out);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -244,13 +252,13 @@ int conv111_launch(const aprnet_apr* a, int dl, int S, const T* in, ll ld_in, co
 
 template<typename T>
 int conv111_apply(const aprnet_apr* a, int dl, int n_in, int n_out, int S, const T* in, ll ld_in, const T* w,
-                  ll ws, ll wo, ll wi, T* out, ll ld_out, cudaStream_t st) {
+                  ll ws, ll wo, ll wi, const T* bias, T* out, ll ld_out, cudaStream_t st) {
     constexpr int TPB = 256;
-    if (n_out <= 4) return conv111_launch<T, 4, TPB, 4>(a, dl, S, in, ld_in, w, ws, wo, wi, out, ld_out, n_in, n_out, st);      // e.g. a classification head
-    if (n_out <= 16) return conv111_launch<T, 16, TPB, 2>(a, dl, S, in, ld_in, w, ws, wo, wi, out, ld_out, n_in, n_out, st);
+    if (n_out <= 4) return conv111_launch<T, 4, TPB, 4>(a, dl, S, in, ld_in, w, ws, wo, wi, bias, out, ld_out, n_in, n_out, st);      // e.g. a classification head
+    if (n_out <= 16) return conv111_launch<T, 16, TPB, 2>(a, dl, S, in, ld_in, w, ws, wo, wi, bias, out, ld_out, n_in, n_out, st);
     // the input is read once per 32 outputs; two locations per thread (fp32) halve the shared-memory reads per multiply-add
-    if (sizeof(T) == 4) return conv111_launch<T, 32, TPB, 2>(a, dl, S, in, ld_in, w, ws, wo, wi, out, ld_out, n_in, n_out, st);
-    return conv111_launch<T, 32, TPB, 1>(a, dl, S, in, ld_in, w, ws, wo, wi, out, ld_out, n_in, n_out, st);
+    if (sizeof(T) == 4) return conv111_launch<T, 32, TPB, 2>(a, dl, S, in, ld_in, w, ws, wo, wi, bias, out, ld_out, n_in, n_out, st);
+    return conv111_launch<T, 32, TPB, 1>(a, dl, S, in, ld_in, w, ws, wo, wi, bias, out, ld_out, n_in, n_out, st);
 }
 
 template<typename T>
@@ -277,91 +285,6 @@ int conv111_dw(const aprnet_apr* a, int dl, int cin, int cout, int S, const T* i
     return APRNET_OK;
 }
 
-// Stencil restriction.  pyapr/aprnet/src/kernel.hpp:54-128: slots < S are copied; slot k >= S is the
-// last given stencil box-averaged onto a grid 2^(k-S+1) times coarser (overlap lengths per axis,
-// divided by step^3).  One thread per (extra level, filter); 27x27 overlap products each.
-// overlap weight between fine tap ti and coarse tap to along one axis, for a grid `step` times coarser
-__device__ __forceinline__ float restrict_overlap(int step, int fine_tap, int coarse_tap) {
-    const int off = step - 1;
-    return (float) (min((coarse_tap + 1) * step, off + fine_tap + step) - max(coarse_tap * step, off + fine_tap));
-}
-
-// forward: one thread per (extra slot k, filter f): dst[k][f][to] = sum_ti ov(ti, to) * src[S-1][f][ti]
-template<typename T>
-__global__ void restrict333_forward_kernel(int S, ll filters, const T* __restrict__ src, T* __restrict__ dst) {
-    const ll f = (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= filters) return;
-    const int k = S + blockIdx.y;
-    const int step = 1 << (k - (S - 1));
-    const float factor = (float) step * (float) step * (float) step;
-    const T* fine = src + ((ll) (S - 1) * filters + f) * 27;
-    T* coarse = dst + ((ll) k * filters + f) * 27;
-    for (int zo = 0; zo < 3; ++zo) for (int xo = 0; xo < 3; ++xo) for (int yo = 0; yo < 3; ++yo) {
-        T acc = 0;
-        for (int zi = 0; zi < 3; ++zi) {
-            const float oz = restrict_overlap(step, zi, zo);
-            if (oz <= 0) continue;
-            for (int xi = 0; xi < 3; ++xi) {
-                const float ox = restrict_overlap(step, xi, xo);
-                if (ox <= 0) continue;
-                for (int yi = 0; yi < 3; ++yi) {
-                    const float oy = restrict_overlap(step, yi, yo);
-                    if (oy <= 0) continue;
-                    acc += (T) (ox * oy * oz / factor) * fine[(zi * 3 + xi) * 3 + yi];
-                }
-            }
-        }
-        coarse[(zo * 3 + xo) * 3 + yo] = acc;
-    }
-}
-
-// backward (transpose): one thread per filter folds every extra slot into slot S-1, slots in
-// ascending order, so the sum order is fixed.
-template<typename T>
-__global__ void restrict333_backward_kernel(int S, int L, ll filters, const T* __restrict__ src, T* __restrict__ dst) {
-    // one thread per (filter, fine tap): 27 times the parallelism of one thread per filter, same summation order
-    const ll e = (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= filters * 27) return;
-    const ll f = e / 27;
-    const int tap = (int) (e - f * 27);
-    const int zi = tap / 9, xi = (tap / 3) % 3, yi = tap % 3;
-    T acc = src[((ll) (S - 1) * filters + f) * 27 + tap];
-    for (int k = S; k < L; ++k) {
-        const int step = 1 << (k - (S - 1));
-        const float factor = (float) step * (float) step * (float) step;
-        const T* coarse = src + ((ll) k * filters + f) * 27;
-        for (int zo = 0; zo < 3; ++zo) {
-            const float oz = restrict_overlap(step, zi, zo);
-            if (oz <= 0) continue;
-            for (int xo = 0; xo < 3; ++xo) {
-                const float ox = restrict_overlap(step, xi, xo);
-                if (ox <= 0) continue;
-                for (int yo = 0; yo < 3; ++yo) {
-                    const float oy = restrict_overlap(step, yi, yo);
-                    if (oy <= 0) continue;
-                    acc += (T) (ox * oy * oz / factor) * coarse[(zo * 3 + xo) * 3 + yo];
-                }
-            }
-        }
-    }
-    dst[((ll) (S - 1) * filters + f) * 27 + tap] = acc;
-}
-
-template<typename T>
-int restrict333(int S, int L, ll filters, const T* src, T* dst, bool backward, cudaStream_t st) {
-    APRNET_CUDA_CHECK(cudaMemcpyAsync(dst, src, (size_t) S * filters * 27 * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    if (L > S) {
-        if (backward) {
-            restrict333_backward_kernel<T><<<aprnet_ceil_div(filters * 27, 128), 128, 0, st>>>(S, L, filters, src, dst);
-        } else {
-            dim3 grid((unsigned) aprnet_ceil_div(filters, 128), (unsigned) (L - S));
-            restrict333_forward_kernel<T><<<grid, 128, 0, st>>>(S, filters, src, dst);
-        }
-        APRNET_LAUNCH_CHECK();
-    }
-    return APRNET_OK;
-}
-
 } // namespace
 
 #define DISPATCH(dtype, CALL_F, CALL_D)                                                   \
@@ -371,15 +294,20 @@ int restrict333(int S, int L, ll filters, const T* src, T* dst, bool backward, c
         default: aprnet_set_error("%s: unknown dtype %d", __func__, dtype); return APRNET_ERR_ARG; \
     }
 
-extern "C" int aprnet_conv111_forward(const aprnet_apr* a, int dl, int dtype, int cin, int cout, int S, const void* in,
-                                      int64_t ld_in, const void* w, void* out, int64_t ld_out, void* stream) {
+extern "C" int aprnet_conv111_forward_bias(const aprnet_apr* a, int dl, int dtype, int cin, int cout, int S, const void* in,
+                                           int64_t ld_in, const void* w, const void* bias, void* out, int64_t ld_out, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && in && w && out && cin > 0 && cout > 0 && S > 0, "bad argument");
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl), "leading dimension too small");
     cudaStream_t st = (cudaStream_t) stream;
     const ll ws = (ll) cin * cout;
-    DISPATCH(dtype, conv111_apply<float>(a, dl, cin, cout, S, (const float*) in, ld_in, (const float*) w, ws, cin, 1, (float*) out, ld_out, st),
-             conv111_apply<double>(a, dl, cin, cout, S, (const double*) in, ld_in, (const double*) w, ws, cin, 1, (double*) out, ld_out, st));
+    DISPATCH(dtype, conv111_apply<float>(a, dl, cin, cout, S, (const float*) in, ld_in, (const float*) w, ws, cin, 1, (const float*) bias, (float*) out, ld_out, st),
+             conv111_apply<double>(a, dl, cin, cout, S, (const double*) in, ld_in, (const double*) w, ws, cin, 1, (const double*) bias, (double*) out, ld_out, st));
+}
+
+extern "C" int aprnet_conv111_forward(const aprnet_apr* a, int dl, int dtype, int cin, int cout, int S, const void* in,
+                                      int64_t ld_in, const void* w, void* out, int64_t ld_out, void* stream) {
+    return aprnet_conv111_forward_bias(a, dl, dtype, cin, cout, S, in, ld_in, w, nullptr, out, ld_out, stream);
 }
 
 extern "C" int aprnet_conv111_backward_input(const aprnet_apr* a, int dl, int dtype, int cin, int cout, int S,
@@ -390,8 +318,8 @@ extern "C" int aprnet_conv111_backward_input(const aprnet_apr* a, int dl, int dt
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl), "leading dimension too small");
     cudaStream_t st = (cudaStream_t) stream;
     const ll ws = (ll) cin * cout;
-    DISPATCH(dtype, conv111_apply<float>(a, dl, cout, cin, S, (const float*) gout, ld_out, (const float*) w, ws, 1, cin, (float*) gin, ld_in, st),
-             conv111_apply<double>(a, dl, cout, cin, S, (const double*) gout, ld_out, (const double*) w, ws, 1, cin, (double*) gin, ld_in, st));
+    DISPATCH(dtype, conv111_apply<float>(a, dl, cout, cin, S, (const float*) gout, ld_out, (const float*) w, ws, 1, cin, nullptr, (float*) gin, ld_in, st),
+             conv111_apply<double>(a, dl, cout, cin, S, (const double*) gout, ld_out, (const double*) w, ws, 1, cin, nullptr, (double*) gin, ld_in, st));
 }
 
 extern "C" int64_t aprnet_conv111_partial_elems(int cin, int cout) { return (int64_t) dw_max_chunks(cin, cout) * cin * cout; }
@@ -405,18 +333,4 @@ extern "C" int aprnet_conv111_backward_weights(const aprnet_apr* a, int dl, int 
     cudaStream_t st = (cudaStream_t) stream;
     DISPATCH(dtype, conv111_dw<float>(a, dl, cin, cout, S, (const float*) in, ld_in, (const float*) gout, ld_out, (float*) gw, (float*) partial, st),
              conv111_dw<double>(a, dl, cin, cout, S, (const double*) in, ld_in, (const double*) gout, ld_out, (double*) gw, (double*) partial, st));
-}
-
-extern "C" int aprnet_restrict333_forward(int dtype, int S, int L, int64_t filters, const void* w, void* expanded, void* stream) {
-    APRNET_ARG_CHECK(w && expanded && S > 0 && L >= S && filters > 0, "requires num_levels >= num_stencils");
-    cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, restrict333<float>(S, L, filters, (const float*) w, (float*) expanded, false, st),
-             restrict333<double>(S, L, filters, (const double*) w, (double*) expanded, false, st));
-}
-
-extern "C" int aprnet_restrict333_backward(int dtype, int S, int L, int64_t filters, const void* gexp, void* gw, void* stream) {
-    APRNET_ARG_CHECK(gexp && gw && S > 0 && L >= S && filters > 0, "requires num_stencils <= expanded levels");
-    cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, restrict333<float>(S, L, filters, (const float*) gexp, (float*) gw, true, st),
-             restrict333<double>(S, L, filters, (const double*) gexp, (double*) gw, true, st));
 }

@@ -5,16 +5,17 @@
 // level; with 2 * Cin * Cout flops against 4 * (Cin + Cout) bytes per location the CUDA-core kernel sits at the
 // fp32 multiply-add bound, the tensor-core kernel at the HBM bound.
 //
-// One persistent block per SM, 17 warps:
-//   warps 0-7   producers, two groups of 128 threads on alternate tiles of 128 locations.  A thread owns one location:
+// One persistent block per SM, 25 warps:
+//   warps 0-15  producers, four groups of 128 threads that take the tiles of 128 locations in turn.  (With two groups, 32 KB of loads in
+//               flight per SM, 64 -> 128 channels on 3.5 M locations took 0.84 ms against 0.42 ms at the HBM rate.)  A thread owns one location:
 //               it requests up to 32 input channels at a time (4-byte loads, coalesced across the warp along the location
 //               axis of the channel-major tensor), rounds them to bf16 and writes them as 16-byte pieces of the K-major,
 //               hardware-swizzled A operand (the transposition happens in registers), then one arrival per thread on the
 //               stage's barrier;
-//   warp 8      one thread waits for the stage, fences the generic-proxy writes against the tensor core's reads and
+//   warp 16     one thread waits for the stage, fences the generic-proxy writes against the tensor core's reads and
 //               issues the Cin / 16 tcgen05.mma (M = 128, N = padded Cout) of each tile and commits the
 //               stage's "slot free" barrier and the accumulator's "complete" barrier;
-//   warps 9-16  epilogue, two sets of four warps on alternate tiles: TMEM -> registers -> coalesced fp32 stores of out[o][p].
+//   warps 17-24 epilogue, two sets of four warps on alternate tiles: TMEM -> registers (+ bias) -> coalesced fp32 stores of out[o][p].
 // The weights of one level (B operand, bf16, all of Cin x Cout) stay in shared memory; the block walks the levels one
 // after the other and converts the next level's weights from the fp32 tensor between two block-wide barriers.
 // Every wait is bounded and polls a block-wide abort flag; after an expiry the block raises the library's error flag,
@@ -31,8 +32,10 @@ namespace {
 using namespace tcptx;
 typedef long long ll;
 constexpr int TILE_M = 128;
-constexpr int C1_THREADS = 17 * 32;
-constexpr int C1_THREADS_DW = 13 * 32;
+constexpr int C1_GROUPS = 4, C1_MMA = 4 * C1_GROUPS;
+constexpr int C1_THREADS = (C1_MMA + 9) * 32;
+constexpr int DW_GROUPS = 2, DW_MMA = 8 * DW_GROUPS;
+constexpr int C1_THREADS_DW = (DW_MMA + 5) * 32;
 constexpr int C1_MAX_STAGES = 8;
 constexpr int C1_MAX_ACC = 4;
 constexpr int C1_MAX_SEGS = APRNET_MAX_LEVELS;
@@ -44,6 +47,7 @@ struct C1Params {
     const float* in; ll ld_in; int n_in;           // K = n_in channels
     const float* w; ll ws, wo, wi;                 // element (slot, o, i) at w[slot * ws + o * wo + i * wi]
     float* out; ll ld_out; int n_out;
+    const float* bias;                             // added to every output channel (null: none)
     int kpad;                                      // n_in padded to 16, 32 or a multiple of 64
     int* error_flag;
 };
@@ -68,6 +72,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     constexpr int KB = KS < 32 ? KS : 32;                       // channels a producer thread requests together
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ float bias_s[ACC_COLS];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int kchunks = P.kpad / KS;
     const int a_stage = kchunks * A_SUB;
@@ -82,18 +87,20 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int c = tid; c < ACC_COLS; c += C1_THREADS) bias_s[c] = P.bias && c < P.n_out ? P.bias[c] : 0.f;
     if (tid == 0) {
         for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), 128); mbar_init(smem_u32(empty + i), 1); }
         for (int i = 0; i < NACC; ++i) { mbar_init(smem_u32(tmem_full + i), 1); mbar_init(smem_u32(tmem_empty + i), 4); }
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 8) { tmem_alloc(smem_u32(tmem_slot), NACC * ACC_COLS); tmem_relinquish(); }
+    if (warp == C1_MMA) { tmem_alloc(smem_u32(tmem_slot), NACC * ACC_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_d = *tmem_slot;
     bool failed = false;
+    const int ngroups = min(C1_GROUPS, stages);      // (a ring at least as long as the groups keeps the phases that a wait can meet apart)
     uint32_t j_base = 0;                    // tiles this block has been given in the levels before the current one
 
     for (int seg = 0; seg < P.n_segs; ++seg) {
@@ -122,10 +129,10 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
         __syncthreads();
         tc_fence_after();
 
-        if (warp < 8) {
+        if (warp < C1_MMA) {
             // ---------------- producers ----------------
             const int grp = tid >> 7, row = tid & 127;
-            for (int it = grp; it < mine && !failed; it += 2) {
+            for (int it = grp; grp < ngroups && it < mine && !failed; it += ngroups) {
                 const uint32_t j = j_base + (uint32_t) it, slot = j % (uint32_t) stages, use = j / (uint32_t) stages;
                 const ll p = sb + ((ll) blockIdx.x + (ll) it * gridDim.x) * TILE_M + row;
                 const bool valid = p < se;
@@ -153,7 +160,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
                 // (no proxy fence here: the MMA thread fences after its wait)
                 mbar_arrive(smem_u32(full + slot));
             }
-        } else if (warp == 8) {
+        } else if (warp == C1_MMA) {
             // ---------------- MMA issue ----------------
             if (lane == 0) {
                 for (int it = 0; it < mine && !failed; ++it) {
@@ -181,7 +188,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
             // two sets of four warps on alternate tiles (twice the stores in flight)
             const int q = warp & 3;                           // TMEM lane group this warp may read
             const int row = q * 32 + lane;
-            for (int it = (warp - 9) >> 2; it < mine && !failed; it += 2) {
+            for (int it = (warp - C1_MMA - 1) >> 2; it < mine && !failed; it += 2) {
                 const uint32_t j = j_base + (uint32_t) it, acc = j % NACC, acc_use = j / NACC;
                 const ll p = sb + ((ll) blockIdx.x + (ll) it * gridDim.x) * TILE_M + row;
                 if (!mbar_wait_warp(smem_u32(tmem_full + acc), acc_use & 1, abort_flag)) { failed = true; break; }
@@ -191,6 +198,10 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
                     uint32_t r[32];
                     tmem_ld32(tmem_d + ((uint32_t) (q * 32) << 16) + acc * ACC_COLS + c0, r);
                     tmem_ld_wait();
+                    if (P.bias) {
+#pragma unroll
+                        for (int jj = 0; jj < 32; ++jj) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + bias_s[c0 + jj]);
+                    }
                     if (p < se) {
 #pragma unroll
                         for (int jj = 0; jj < 32; ++jj)
@@ -212,7 +223,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) tmem_dealloc(tmem_d, NACC * ACC_COLS);
+    if (warp == C1_MMA) tmem_dealloc(tmem_d, NACC * ACC_COLS);
 }
 
 inline int pad_k(int c) { return c <= 16 ? 16 : (c <= 32 ? 32 : (c + 63) / 64 * 64); }
@@ -222,8 +233,8 @@ template<int NT, int KS>
 int launch_c1(const C1Params& P, ll total_tiles, cudaStream_t st, const char* pname) {
     const size_t a_stage = (size_t) TILE_M * P.kpad * 2, b_bytes = (size_t) NT * P.kpad * 2;
     const size_t fixed = b_bytes + (2 * C1_MAX_STAGES + 2 * C1_MAX_ACC) * 8 + 16 + 1024;
-    if (fixed + 2 * a_stage > 227 * 1024 - 1024) return APRNET_ERR_UNSUPPORTED;
-    const int stages = (int) std::min<size_t>(C1_MAX_STAGES, (227 * 1024 - 1024 - fixed) / a_stage);
+    if (fixed + 2 * a_stage > 226 * 1024 - 1024) return APRNET_ERR_UNSUPPORTED;
+    const int stages = (int) std::min<size_t>(C1_MAX_STAGES, (226 * 1024 - 1024 - fixed) / a_stage);
     const size_t smem = (size_t) stages * a_stage + fixed;
     auto kern = conv111_tc_kernel<NT, KS>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
@@ -240,7 +251,7 @@ int launch_c1(const C1Params& P, ll total_tiles, cudaStream_t st, const char* pn
 
 // out[o][p] = sum_i w[slot][o][i] in[i][p] over the locations of level delta dl
 int run_conv111_tc(const aprnet_apr* a, int dl, int n_in, int n_out, int slots, const float* in, ll ld_in, const float* w, ll ws, ll wo, ll wi,
-                   float* out, ll ld_out, cudaStream_t st, const char* pname) {
+                   const float* bias, float* out, ll ld_out, cudaStream_t st, const char* pname) {
     // narrow layers (a classifier head) are bound by their one wide tensor either way and run faster on the CUDA cores
     if (n_out > 256 || n_in > 256 || n_in < 8 || n_out < 8) return APRNET_ERR_UNSUPPORTED;
     const std::vector<Segment> segs = aprnet_segments(a, dl, slots, true);
@@ -255,7 +266,7 @@ int run_conv111_tc(const aprnet_apr* a, int dl, int n_in, int n_out, int slots, 
         ++P.n_segs;
     }
     if (P.n_segs == 0) return APRNET_OK;
-    P.in = in; P.ld_in = ld_in; P.n_in = n_in; P.w = w; P.ws = ws; P.wo = wo; P.wi = wi; P.out = out; P.ld_out = ld_out; P.n_out = n_out;
+    P.in = in; P.ld_in = ld_in; P.n_in = n_in; P.w = w; P.ws = ws; P.wo = wo; P.wi = wi; P.out = out; P.ld_out = ld_out; P.n_out = n_out; P.bias = bias;
     P.kpad = pad_k(n_in);
     P.error_flag = aprnet_tc_error_flag_device();
     const int nt = pick_nt(n_out), ks = std::min(64, P.kpad);
@@ -273,11 +284,11 @@ int run_conv111_tc(const aprnet_apr* a, int dl, int n_in, int n_out, int slots, 
 // to 128 per accumulator), N = input channels, K = locations.  Both tensors are channel-major, i.e. K-major operands
 // as they lie in memory; they only have to be rounded to bf16.  One persistent block per SM walks its share of the
 // 128-location tiles of ONE level range and keeps the accumulators in TMEM until the end:
-//   warps 0-7   producers: a warp takes channel rows of both tensors in turn, 32 consecutive locations per load
+//   warps 0-15  producers, two groups of eight warps on alternate tiles: a warp takes channel rows of both tensors in turn, 32 consecutive locations per load
 //               instruction (coalesced), and writes each value as a 2-byte piece of the swizzled K-major operand row
 //               (conflict-free: the 32 lanes fill 64 bytes of one 128-byte row); locations past the end are zeros;
-//   warp 8      one thread issues 8 tcgen05.mma per accumulator and stage;
-//   warps 9-12  after the last tile: TMEM -> partial sums of this block; a second kernel adds the blocks in fixed order.
+//   warp 16     one thread issues 8 tcgen05.mma per accumulator and stage;
+//   warps 17-20 after the last tile: TMEM -> partial sums of this block; a second kernel adds the blocks in fixed order.
 struct C1DwParams {
     ll seg_begin, seg_end;
     const float* in; ll ld_in; int cin;
@@ -295,7 +306,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
     const int a_rows = mtiles * 128;
     const int stage_bytes = (a_rows + NT) * 256;             // two 64-location halves of 128 bytes per channel row
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t) stages * stage_bytes);
-    uint64_t* full = bars;                                   // [stages] operands written (256 producer threads)
+    uint64_t* full = bars;                                   // [stages] operands written (the 256 threads of a group)
     uint64_t* empty = bars + C1_MAX_STAGES;                  // [stages] MMAs that read the stage completed
     uint64_t* done = empty + C1_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
@@ -308,7 +319,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 8) { tmem_alloc(smem_u32(tmem_slot), tmem_cols); tmem_relinquish(); }
+    if (warp == DW_MMA) { tmem_alloc(smem_u32(tmem_slot), tmem_cols); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -318,15 +329,15 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
     const int seg_tiles = (int) ((se - sb + TILE_M - 1) / TILE_M);
     const int mine = (int) blockIdx.x < seg_tiles ? (seg_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
 
-    if (warp < 8) {
+    if (warp < DW_MMA) {
         // ---------------- producers ----------------
         const int nrows = P.cout + P.cin;                    // channel rows of a stage: gout rows, then in rows
-        for (int it = 0; it < mine && !failed; ++it) {
+        for (int it = warp >> 3; it < mine && !failed; it += DW_GROUPS) {
             const uint32_t slot = (uint32_t) it % (uint32_t) stages, use = (uint32_t) it / (uint32_t) stages;
             const ll p0 = sb + ((ll) blockIdx.x + (ll) it * gridDim.x) * TILE_M;
             if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
             unsigned char* st = smem + (size_t) slot * stage_bytes;
-            for (int r0 = warp; r0 < nrows; r0 += 8 * 8) {   // 8 rows of this warp x 4 quarters of 32 locations in flight
+            for (int r0 = warp & 7; r0 < nrows; r0 += 8 * 8) {   // 8 rows of this warp x 4 quarters of 32 locations in flight
                 float v[8][4];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
@@ -356,7 +367,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
             }
             mbar_arrive(smem_u32(full + slot));               // the MMA thread fences the generic-proxy writes after its wait
         }
-    } else if (warp == 8) {
+    } else if (warp == DW_MMA) {
         // ---------------- MMA issue ----------------
         if (lane == 0) {
             for (int it = 0; it < mine && !failed; ++it) {
@@ -381,9 +392,9 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
             if (!failed) umma_commit(smem_u32(done));
         }
     }
-    // ---------------- epilogue: warps 9-12 ----------------
+    // ---------------- epilogue: the last four warps ----------------
     float* dst = P.partial + (ll) blockIdx.x * P.cout * P.cin;
-    if (warp >= 9 && mine > 0 && !failed) {
+    if (warp > DW_MMA && mine > 0 && !failed) {
         if (!mbar_wait_warp(smem_u32(done), 0, abort_flag)) failed = true;
         if (!failed) {
             tc_fence_after();
@@ -412,7 +423,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) tmem_dealloc(tmem_d, tmem_cols);
+    if (warp == DW_MMA) tmem_dealloc(tmem_d, tmem_cols);
 }
 
 __global__ void c1_reduce_partial_kernel(const float* __restrict__ partial, int nblocks, ll elems, float* __restrict__ dst) {
@@ -438,14 +449,19 @@ int launch_c1_dw(const C1DwParams& P, int grid, int mtiles, cudaStream_t st) {
 
 } // namespace
 
-extern "C" int aprnet_conv111_forward_tc(const aprnet_apr* a, int dl, int cin, int cout, int S, const float* in, int64_t ld_in,
-                                         const float* w, float* out, int64_t ld_out, void* stream) {
+extern "C" int aprnet_conv111_forward_tc_bias(const aprnet_apr* a, int dl, int cin, int cout, int S, const float* in, int64_t ld_in,
+                                              const float* w, const float* bias, float* out, int64_t ld_out, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && in && w && out && cin > 0 && cout > 0 && S > 0, "bad argument");
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl), "leading dimension too small");
     char pname[64];
     snprintf(pname, sizeof(pname), "conv111_tc:ci%d:co%d:dl%d", cin, cout, dl);
-    return run_conv111_tc(a, dl, cin, cout, S, in, ld_in, w, (ll) cin * cout, cin, 1, out, ld_out, (cudaStream_t) stream, pname);
+    return run_conv111_tc(a, dl, cin, cout, S, in, ld_in, w, (ll) cin * cout, cin, 1, bias, out, ld_out, (cudaStream_t) stream, pname);
+}
+
+extern "C" int aprnet_conv111_forward_tc(const aprnet_apr* a, int dl, int cin, int cout, int S, const float* in, int64_t ld_in,
+                                         const float* w, float* out, int64_t ld_out, void* stream) {
+    return aprnet_conv111_forward_tc_bias(a, dl, cin, cout, S, in, ld_in, w, nullptr, out, ld_out, stream);
 }
 
 extern "C" int aprnet_conv111_backward_input_tc(const aprnet_apr* a, int dl, int cin, int cout, int S, const float* gout, int64_t ld_out,
@@ -455,7 +471,7 @@ extern "C" int aprnet_conv111_backward_input_tc(const aprnet_apr* a, int dl, int
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl), "leading dimension too small");
     char pname[64];
     snprintf(pname, sizeof(pname), "conv111_tc:ci%d:co%d:dl%d", cout, cin, dl);
-    return run_conv111_tc(a, dl, cout, cin, S, gout, ld_out, w, (ll) cin * cout, 1, cin, gin, ld_in, (cudaStream_t) stream, pname);
+    return run_conv111_tc(a, dl, cout, cin, S, gout, ld_out, w, (ll) cin * cout, 1, cin, nullptr, gin, ld_in, (cudaStream_t) stream, pname);
 }
 
 extern "C" int aprnet_conv111_backward_weights_tc(const aprnet_apr* a, int dl, int cin, int cout, int S, const float* in, int64_t ld_in,

@@ -105,35 +105,13 @@ __global__ void __launch_bounds__(256) pack_rows_f32_kernel(const float* __restr
     }
 }
 
-// packed weights [slot][tap][n tile][k][NT], zero where k or n exceed their extents.  mode 0: n = co, k = ci, w[tap];
-// mode 1: n = ci, k = co, w[26 - tap] (same-level input gradient); mode 2: n = ci, k = co, w[tap] (cross-level part)
-__global__ void pack_weights_f32_kernel(const float* __restrict__ w, int slots, int cin, int cout, int mode, int nt, int n_tiles, int kpad,
-                                        float* __restrict__ out) {
-    const int n_dim = mode ? cin : cout, k_dim = mode ? cout : cin;
-    const ll total = (ll) slots * 27 * n_tiles * kpad * nt;
-    for (ll e = (ll) blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (ll) gridDim.x * blockDim.x) {
-        ll r = e;
-        const int nn = (int) (r % nt); r /= nt;
-        const int k = (int) (r % kpad); r /= kpad;
-        const int tile = (int) (r % n_tiles); r /= n_tiles;
-        const int tap = (int) (r % 27); r /= 27;
-        const int n = tile * nt + nn;
-        float v = 0.f;
-        if (n < n_dim && k < k_dim) {
-            const int co = mode ? k : n, ci = mode ? n : k;
-            v = w[((r * cout + co) * cin + ci) * 27 + (mode == 1 ? 26 - tap : tap)];
-        }
-        out[e] = v;
-    }
-}
-
 // ---- gather product ---------------------------------------------------------------------------------
 struct F32Params {
     SegTable segs;
     const int32_t* nbr; ll N;              // neighbour table [27][N]
     const float* rows; int kpad;           // packed source rows [R][kpad]
     ll tree_base, zero_row;                // row of tree node 0 and of the zero row
-    const float* wp;                       // packed weights
+    const float* wp; int mirror;           // packed weights (weights.cu); mirror: tap t meets the weights of tap 26 - t
     int n_dim, n_tiles;
     int same_level_only;                   // mask table entries outside the tile's own level
     float* out; ll ld_out;
@@ -217,7 +195,7 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
         } else {
             if (ikc == 0) { decode(); request(itap + 1); }
             copy_rows(a_s, ikc * KS + piece * 4);
-            const float* w = wtile + itap * wtap + (ll) ikc * KS * NT;
+            const float* w = wtile + (P.mirror ? 26 - itap : itap) * wtap + (ll) ikc * KS * NT;
             const int wpieces = min(KS, P.kpad - ikc * KS) * (NT / 4);
             for (int e = tid; e < wpieces; e += T) cp_async16(smem_u32(a_s + A_ELEMS + e * 4), w + e * 4);
             if (++ikc == kchunks) { ikc = 0; ++itap; }
@@ -447,26 +425,37 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
     }
 }
 
-// grad_weights[slot][co][ci][tap] += the block sums of the slot's ranges.  Eight threads share a result and take every eighth
-// range; their sums are combined in a fixed order.
-__global__ void __launch_bounds__(256) dw_reduce_f32_kernel(const float* __restrict__ partial, SlotRanges sr, int cin, int cout, float* __restrict__ gw) {
-    __shared__ float sums[8][33];
-    const ll elems = (ll) 27 * cin * cout;
-    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
-    const ll e = (ll) blockIdx.x * 32 + x;
-    float s = 0.f;
-    if (e < elems) {
-        const int r1 = sr.first[blockIdx.y + 1];
-#pragma unroll 4
-        for (int r = sr.first[blockIdx.y] + y; r < r1; r += 8) s += partial[(ll) r * elems + e];
-    }
-    sums[y][x] = s;
-    __syncthreads();
-    if (y == 0 && e < elems) {
+// grad_weights[slot][co][ci][tap] += the block sums [range][tap][ci][co] of the slot's ranges.  Block = one input channel, 32 output
+// channels, one slot: warp y takes every eighth range, 27 independent coalesced loads at a time; the warps' sums are combined in a
+// fixed order and leave transposed, 27 contiguous values per filter.
+__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, SlotRanges sr, int cin, int cout, float* __restrict__ gw) {
+    __shared__ float sums[8][27][33];
+    const int lane = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int ci = blockIdx.x, co0 = blockIdx.y * 32, co = co0 + lane;
+    const int r0 = sr.first[blockIdx.z], r1 = sr.first[blockIdx.z + 1], ny = min(8, r1 - r0);
+    const ll tap_stride = (ll) cin * cout, range_stride = 27 * tap_stride;
+    float s[27];
 #pragma unroll
-        for (int k = 1; k < 8; ++k) s += sums[k][x];
-        const int co = (int) (e % cout), ci = (int) (e / cout % cin), tap = (int) (e / ((ll) cout * cin));
-        gw[(((ll) sr.slot[blockIdx.y] * cout + co) * cin + ci) * 27 + tap] += s;
+    for (int t = 0; t < 27; ++t) s[t] = 0.f;
+    if (co < cout) {
+        for (int r = r0 + y; r < r1; r += 8) {
+            const float* p = partial + r * range_stride + (ll) ci * cout + co;
+#pragma unroll
+            for (int t = 0; t < 27; ++t) s[t] += __ldg(p + t * tap_stride);
+        }
+    }
+    if (y < ny) {
+#pragma unroll
+        for (int t = 0; t < 27; ++t) sums[y][t][lane] = s[t];
+    }
+    __syncthreads();
+    const int n = min(32, cout - co0) * 27;
+    float* dst = gw + (((ll) sr.slot[blockIdx.z] * cout + co0) * cin + ci) * 27;
+    for (int e = threadIdx.x; e < n; e += 256) {
+        const int c = e / 27, t = e - c * 27;
+        float v = 0.f;
+        for (int k = 0; k < ny; ++k) v += sums[k][t][c];
+        dst[(ll) c * cin * 27 + t] += v;
     }
 }
 
@@ -506,13 +495,9 @@ int run_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, 
     return APRNET_OK;
 }
 
-int run_pack_weights(const float* w, int slots, int cin, int cout, int mode, float* wp, cudaStream_t st) {
-    const int n_dim = mode ? cin : cout, k_dim = mode ? cout : cin, nt = pick_nt(n_dim), n_tiles = (n_dim + nt - 1) / nt;
-    AprnetProfScope _prof("pack_weights_f32", st);
-    pack_weights_f32_kernel<<<std::min(1184, aprnet_ceil_div((ll) slots * 27 * n_tiles * pad4(k_dim) * nt, 256)), 256, 0, st>>>(
-        w, slots, cin, cout, mode, nt, n_tiles, pad4(k_dim), wp);
-    APRNET_LAUNCH_CHECK();
-    return APRNET_OK;
+int run_pack_weights(const aprnet_apr* a, int dl, const float* w, int slots, int cin, int cout, int transposed, float* wp, cudaStream_t st) {
+    const int n_dim = transposed ? cin : cout, nt = pick_nt(n_dim);
+    return aprnet_pack_weights(a, dl, false, w, slots, cin, cout, transposed, nt, (n_dim + nt - 1) / nt, pad4(transposed ? cout : cin), wp, st);
 }
 
 template<int WM, int WN, int TN, bool KMAJOR>
@@ -618,15 +603,14 @@ int run_dw(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* xro
     return rc ? rc : aprnet_dw_reduce(partial, sr, cin, cout, gw, st);
 }
 
-// cross-level part of the input gradient (see edge_plan.cu): sums per (target, tap), then the gather over the targets
-int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* grows, const float* w, float* gin, ll ld_in, float* gtree, ll ld_tree,
+// cross-level part of the input gradient (see edge_plan.cu; wp: the transposed weights as packed for the same-level part): sums per (target, tap), then the gather over the targets
+int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* grows, float* gin, ll ld_in, float* gtree, ll ld_tree,
               float* wp, float* vrows, ll vrow_bytes, cudaStream_t st) {
     EdgePlan* ep = aprnet_get_edge_plan(a, dl, st);
     if (!ep) return APRNET_ERR_CUDA;
     if (ep->n_active == 0) return APRNET_OK;
     const int gpad = pad4(cout), cml = a->cml(dl);
-    int rc = run_pack_weights(w, slots, cin, cout, 2, wp, st);
-    if (rc) return rc;
+    int rc = APRNET_OK;
     APRNET_CUDA_CHECK(cudaMemsetAsync(vrows, 0, (size_t) gpad * sizeof(float), st));          // row 0: zeros
     const ll cap_rows = vrow_bytes / ((ll) gpad * 4) - 1;
     const int nk = (int) ep->chunk_a.size() - 1;
@@ -673,7 +657,7 @@ inline size_t edge_bytes(const aprnet_apr* a, int dl, int cout) {
 
 int aprnet_dw_reduce(const float* partial, const SlotRanges& sr, int cin, int cout, float* gw, cudaStream_t st) {
     AprnetProfScope _prof("conv333_dw_reduce", st);
-    dw_reduce_f32_kernel<<<dim3((unsigned) aprnet_ceil_div((ll) 27 * cin * cout, 32), (unsigned) sr.n), 256, 0, st>>>(partial, sr, cin, cout, gw);
+    dw_reduce_kernel<<<dim3((unsigned) cin, (unsigned) aprnet_ceil_div(cout, 32), (unsigned) sr.n), 256, 0, st>>>(partial, sr, cin, cout, gw);
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
@@ -713,7 +697,7 @@ int aprnet_f32_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, cons
     const AprPlan* plan = aprnet_get_plan(a, dl, st);
     if (!plan) return APRNET_ERR_CUDA;
     float* wp = (float*) ((char*) workspace + aprnet_f32_rows_bytes(a, dl, cin));
-    int rc = run_pack_weights(w, slots, cin, cout, 0, wp, st);
+    int rc = run_pack_weights(a, dl, w, slots, cin, cout, 0, wp, st);
     if (rc) return rc;
     F32Params P;
     memset(&P, 0, sizeof(P));
@@ -741,11 +725,11 @@ int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slot
     float* grows = (float*) workspace;
     float* wp = (float*) ((char*) workspace + rows_bytes(n + 1, cout));
     float* vrows = (float*) ((char*) wp + weight_bytes(cout, cin, slots));
-    int rc = run_pack_weights(w, slots, cin, cout, 1, wp, st);
+    int rc = run_pack_weights(a, dl, w, slots, cin, cout, 1, wp, st);
     if (rc) return rc;
     F32Params P;
     memset(&P, 0, sizeof(P));
-    P.nbr = plan->nbr; P.N = n; P.rows = grows; P.kpad = pad4(cout); P.tree_base = n; P.zero_row = n; P.same_level_only = 1;
+    P.nbr = plan->nbr; P.N = n; P.rows = grows; P.kpad = pad4(cout); P.tree_base = n; P.zero_row = n; P.same_level_only = 1; P.mirror = 1;
     P.wp = wp; P.n_dim = cin; P.out = gin; P.ld_out = ld_in;
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_bwd_input:ci%d:co%d:dl%d", cin, cout, dl);
@@ -757,6 +741,6 @@ int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slot
         return aprnet_conv333_backward_input_cross_level(a, dl, APRNET_F32, cin, cout, slots, gout, ld_out, w, gin, ld_in, gtree, ld_tree, st);
     }
     if (ts > 0) APRNET_CUDA_CHECK(cudaMemset2DAsync(gtree, (size_t) ld_tree * sizeof(float), 0, (size_t) ts * sizeof(float), (size_t) cin, st));
-    if ((rc = run_cross(a, dl, cin, cout, slots, grows, w, gin, ld_in, gtree, ld_tree, wp, vrows, (ll) edge_bytes(a, dl, cout), st))) return rc;
+    if ((rc = run_cross(a, dl, cin, cout, slots, grows, gin, ld_in, gtree, ld_tree, wp, vrows, (ll) edge_bytes(a, dl, cout), st))) return rc;
     return tree_adjoint ? aprnet_fill_tree_mean_backward(a, dl, APRNET_F32, cin, gin, ld_in, gtree, ld_tree, st) : APRNET_OK;
 }

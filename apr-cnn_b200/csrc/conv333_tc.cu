@@ -98,38 +98,13 @@ __global__ void __launch_bounds__(256) pack_rows_bf16_kernel(const float* __rest
     }
 }
 
-// Packed weights: [slot][tap][n_tile][k chunk j][n][8] bf16 (canonical K-major operand per (slot,tap,n_tile)).
-// forward:  B[n = co][k = ci] = w[slot][co][ci][tap]
-// backward == 1: B[n = ci][k = co] = w[slot][co][ci][26 - tap];  backward == 2: B[n = ci][k = co] = w[slot][co][ci][tap]
-__global__ void pack_weights_bf16_kernel(const float* __restrict__ w, int slots, int cin, int cout, int backward,
-                                         int n_dim, int k_dim, int nt, int n_tiles, int kpad, __nv_bfloat16* __restrict__ out) {
-    const ll total = (ll) slots * 27 * n_tiles * (kpad / 8) * nt * 8;
-    for (ll e = (ll) blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (ll) gridDim.x * blockDim.x) {
-        ll r = e;
-        const int k8 = (int) (r % 8); r /= 8;
-        const int nn = (int) (r % nt); r /= nt;
-        const int j = (int) (r % (kpad / 8)); r /= (kpad / 8);
-        const int ntile = (int) (r % n_tiles); r /= n_tiles;
-        const int tap = (int) (r % 27); r /= 27;
-        const int slot = (int) r;
-        const int nidx = ntile * nt + nn, kidx = j * 8 + k8;
-        float v = 0.f;
-        if (nidx < n_dim && kidx < k_dim) {
-            const int co = backward ? kidx : nidx, ci = backward ? nidx : kidx;
-            const int tp = (backward == 1) ? 26 - tap : tap;
-            v = w[(((ll) slot * cout + co) * cin + ci) * 27 + tp];
-        }
-        out[e] = __float2bfloat16(v);
-    }
-}
-
 // ---- kernel parameters -------------------------------------------------------------------------------
 struct TcParams {
     SegTable segs;
     const int32_t* nbr; ll N;              // neighbour table [27][N]
     const __nv_bfloat16* rows; int kpad;   // packed source rows [R][kpad]
     ll tree_base, zero_row;                // row index of tree node 0 and of the zero row
-    const __nv_bfloat16* wp;               // packed weights
+    const __nv_bfloat16* wp; int mirror;   // packed weights (weights.cu); mirror: tap t meets the weights of tap 26 - t
     float* out; ll ld_out; int n_dim;      // output (n_dim, ld_out)
     const float* bias;                     // added to every output channel (null: none)
     int n_tiles;
@@ -272,7 +247,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
                     const int nt = min(TAPS, 27 - t0);
                     mbar_expect_tx(smem_u32(full + slot), nt * B_TAP + max(0, nt - (TAPS - TT)) * A_TAP);
                     for (int t = 0; t < nt; ++t)
-                        bulk_copy_g2s(smem_u32(a_s + TAPS * A_TAP + t * B_TAP), wsrc + (ll) (t0 + t) * w_tap_stride + (ll) kc * KS * NT * 2,
+                        bulk_copy_g2s(smem_u32(a_s + TAPS * A_TAP + t * B_TAP), wsrc + (ll) (P.mirror ? 26 - t0 - t : t0 + t) * w_tap_stride + (ll) kc * KS * NT * 2,
                                       B_TAP, smem_u32(full + slot));
                     bulk_issued = true;
                 }
@@ -458,25 +433,32 @@ int ensure_error_flag() {
 inline int pad_to(int v, int m) { return (v + m - 1) / m * m; }
 inline int pick_nt(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256)); }
 
-struct TcGeom { int kpad, ks, nt, n_tiles; size_t rows_bytes, w_bytes; };
+struct TcGeom { int kpad, ks, nt, n_tiles, order_nt; size_t rows_bytes, w_bytes; };
 
 int g_runs_off = 0;          // aprnet_tc_set_option("runs", 0 / 1): 0 = always this file's kernel, measurement switch
 int g_ks_override = 0;       // aprnet_tc_set_option("ks", n): channels per stage, measurement switch
 
-TcGeom tc_geometry(ll rows, int k_dim, int n_dim, int slots) {
+// tiles: tiles of 128 locations of the layer.  The width of the result tiles also fixes the channels and taps of a stage, that is the
+// order of the products; few locations get narrower tiles, so that all SMs work, in the order of the wide ones (order_nt).
+// 256 -> 256 channels on 1.9 k locations: 71 us with one 256-wide tile per 128 locations (15 blocks).
+TcGeom tc_geometry(ll rows, int k_dim, int n_dim, int slots, ll tiles, bool free_order) {
     TcGeom g;
     g.kpad = pad_to(k_dim, 16);
-    g.nt = pick_nt(n_dim);
+    g.nt = g.order_nt = free_order ? std::min(128, pick_nt(n_dim)) : pick_nt(n_dim);
     g.ks = (g.kpad % 64 == 0 && g.nt <= 128) ? 64 : ((g.kpad % 32 == 0) ? 32 : 16);
     // 64 output channels: stages of 3 taps x 32 channels (5 ring slots, 4 producer groups) measured 3-10 % faster than
     // 2 taps x 64 channels (3 slots, 2 groups); for 32 and 128 outputs the 64-channel stages win
     if (g.nt == 64 && g.ks == 64) g.ks = 32;
     if (g_ks_override > 0 && g.kpad % g_ks_override == 0 && (g_ks_override < 64 || g.nt <= 128)) g.ks = g_ks_override;
+    while (g.nt > 32 && tiles * ((n_dim + g.nt - 1) / g.nt) < 148) g.nt /= 2;
+    if (free_order) { g.order_nt = g.nt; if (g.nt == 64 && g.ks == 64) g.ks = 32; }
     g.n_tiles = (n_dim + g.nt - 1) / g.nt;
     g.rows_bytes = ((size_t) rows * g.kpad * 2 + 255) / 256 * 256;
-    g.w_bytes = ((size_t) slots * 27 * g.n_tiles * g.kpad * g.nt * 2 + 255) / 256 * 256;
+    g.w_bytes = ((size_t) slots * 27 * pad_to(n_dim, pick_nt(n_dim)) * g.kpad * 2 + 255) / 256 * 256;      // for any split
     return g;
 }
+
+inline ll tiles_of(const aprnet_apr* a, int dl) { return (a->number_parts(dl) + TILE_M - 1) / TILE_M; }
 
 // Stage geometry per tile shape: (taps per stage, producer warps per stage).  The ring needs one slot per producer
 // group plus one for the tensor core; stages are as large as that allows, because the MMA thread pays a fixed
@@ -494,8 +476,8 @@ inline int ws_stages(int nt, int ks, int taps) {
 // (output tile width, channels per stage, taps per stage, warps per stage) combinations that are compiled
 #define TC_VARIANTS(X) \
     X(32, 16, 1, 1) X(32, 16, 3, 1) X(32, 16, 9, 2) X(32, 32, 1, 1) X(32, 32, 3, 1) X(32, 32, 3, 2) X(32, 32, 9, 4) \
-    X(32, 64, 1, 1) X(32, 64, 3, 2) X(32, 64, 3, 4) \
-    X(64, 16, 1, 1) X(64, 16, 3, 1) X(64, 16, 9, 2) X(64, 32, 1, 1) X(64, 32, 3, 2) X(64, 64, 1, 1) X(64, 64, 2, 2) X(64, 64, 2, 4) X(64, 64, 3, 4) \
+    X(32, 64, 1, 1) X(32, 64, 1, 2) X(32, 32, 2, 2) X(32, 64, 3, 2) X(32, 64, 3, 4) \
+    X(64, 16, 1, 1) X(64, 16, 3, 1) X(64, 16, 9, 2) X(64, 32, 1, 1) X(64, 32, 3, 2) X(64, 32, 2, 2) X(64, 64, 1, 1) X(64, 64, 1, 2) X(64, 64, 2, 2) X(64, 64, 2, 4) X(64, 64, 3, 4) \
     X(128, 16, 1, 1) X(128, 16, 3, 2) X(128, 32, 1, 1) X(128, 32, 2, 2) X(128, 32, 3, 4) X(128, 64, 1, 1) X(128, 64, 1, 2) X(128, 64, 2, 4) \
     X(256, 16, 1, 1) X(256, 16, 3, 2) X(256, 32, 1, 1) X(256, 32, 2, 2) X(256, 32, 2, 4)
 
@@ -591,7 +573,9 @@ int launch_tc_ws(const TcParams& P, int total_tiles, cudaStream_t st, const char
 int dispatch_tc(const TcParams& P, const TcGeom& g, int total_tiles, cudaStream_t st, const char* pname) {
     int taps = 1, wps = 1, tt = 0;
     // the rows of the cross-level pass are addressed from a shifted base with the zero row in front: no tensor map for them
-    pick_stage_shape(g.nt, g.ks, P.out_map == nullptr, &taps, &wps, &tt);
+    pick_stage_shape(g.order_nt, g.ks, P.out_map == nullptr && g.nt == g.order_nt, &taps, &wps, &tt);
+    if (g.nt != g.order_nt)          // a narrower tile in the order of the wide one: the same taps per stage
+        for (int w = 4; w >= 1; w /= 2) if (tc_variant_ok(g.nt, g.ks, taps, w)) wps = w;
 #define X(NT_, KS_, TAPS_, WPS_) if (tt == 0 && g.nt == NT_ && g.ks == KS_ && taps == TAPS_ && wps == WPS_) return launch_tc_ws<NT_, KS_, TAPS_, WPS_, 0>(P, total_tiles, st, pname);
     TC_VARIANTS(X)
 #undef X
@@ -629,23 +613,19 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
     const AprPlan* plan = aprnet_get_plan(a, dl, st);
     if (!plan) return APRNET_ERR_CUDA;
     const int k_dim = backward ? cout : cin, n_dim = backward ? cin : cout;
-    const TcGeom g = tc_geometry(1, k_dim, n_dim, slots);
+    const TcGeom g = tc_geometry(1, k_dim, n_dim, slots, tiles_of(a, dl), backward != 0);
     if (g.kpad != kpad) { aprnet_set_error("packed row width %d does not match the padded channel count %d", kpad, g.kpad); return APRNET_ERR_ARG; }
     __nv_bfloat16* wp = reinterpret_cast<__nv_bfloat16*>(wp_ws);
-    { AprnetProfScope _prof("pack_weights_bf16", st);
-    pack_weights_bf16_kernel<<<std::min(1024, aprnet_ceil_div((ll) slots * 27 * g.n_tiles * g.kpad * g.nt, 256)), 256, 0, st>>>(
-        w, slots, cin, cout, backward, n_dim, k_dim, g.nt, g.n_tiles, g.kpad, wp);
-    }
-    APRNET_LAUNCH_CHECK();
+    if ((rc = aprnet_pack_weights(a, dl, true, w, slots, cin, cout, backward, g.nt, g.n_tiles, g.kpad, wp, st))) return rc;
     char pname[64];
     snprintf(pname, sizeof(pname), "%s:ci%d:co%d:dl%d", backward ? "conv333_tc_bwd_gather" : "conv333_tc_fwd", cin, cout, dl);
-    const int run_order = g_runs_off ? 0 : aprnet_tc_runs_order(backward, g.kpad, g.nt, g.ks);
+    const int run_order = g_runs_off ? 0 : aprnet_tc_runs_order(backward, g.kpad, g.order_nt, g.ks);
     if (run_order) return aprnet_tc_run_conv(a, dl, backward, slots, g.nt, run_order, rows, g.kpad, tree_base, zero_row, wp, bias, out, ld_out, n_dim, g_error_flag_dev, st, pname);
     TcParams P;
     P.segs = make_seg_table(aprnet_segments(a, dl, slots, false), TILE_M);
     P.nbr = plan->nbr; P.N = plan->n; P.rows = reinterpret_cast<const __nv_bfloat16*>(rows); P.kpad = g.kpad;
     P.tree_base = tree_base; P.zero_row = zero_row;
-    P.wp = wp; P.out = out; P.ld_out = ld_out; P.bias = bias; P.n_dim = n_dim; P.n_tiles = g.n_tiles; P.same_level_only = backward;
+    P.wp = wp; P.mirror = backward; P.out = out; P.ld_out = ld_out; P.bias = bias; P.n_dim = n_dim; P.n_tiles = g.n_tiles; P.same_level_only = backward;
     P.error_flag = g_error_flag_dev;
     P.out_map = nullptr; P.out_split = 0; P.out2 = nullptr; P.ld_out2 = 0;
 
@@ -654,25 +634,19 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
     return dispatch_tc(P, g, total, st, pname);
 }
 
-int aprnet_tc_pack_weights(const float* w, int slots, int cin, int cout, int mode, void* wp, cudaStream_t st) {
-    const int k_dim = mode ? cout : cin, n_dim = mode ? cin : cout;
-    const TcGeom g = tc_geometry(1, k_dim, n_dim, slots);
-    { AprnetProfScope _prof("pack_weights_bf16", st);
-    pack_weights_bf16_kernel<<<std::min(1024, aprnet_ceil_div((ll) slots * 27 * g.n_tiles * g.kpad * g.nt, 256)), 256, 0, st>>>(
-        w, slots, cin, cout, mode, n_dim, k_dim, g.nt, g.n_tiles, g.kpad, reinterpret_cast<__nv_bfloat16*>(wp));
-    }
-    APRNET_LAUNCH_CHECK();
-    return APRNET_OK;
+int aprnet_tc_pack_weights(const aprnet_apr* a, int dl, const float* w, int slots, int cin, int cout, int transposed, void* wp, cudaStream_t st) {
+    const TcGeom g = tc_geometry(1, transposed ? cout : cin, transposed ? cin : cout, slots, tiles_of(a, dl), transposed != 0);
+    return aprnet_pack_weights(a, dl, true, w, slots, cin, cout, transposed, g.nt, g.n_tiles, g.kpad, wp, st);
 }
 
-// Gather GEMM over the active targets [a0, a1) of an edge plan (weights already packed with mode 2).
+// Gather GEMM over the active targets [a0, a1) of an edge plan (transposed weights as packed by aprnet_tc_gather_conv).
 int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* vrows, int gpad, ll zero_row,
                              const void* wp_packed, const EdgePlan* ep, ll a0, ll a1,
                              float* gin, ll ld_in, float* gtree, ll ld_tree, cudaStream_t st) {
     int rc = ensure_error_flag();
     if (rc) return rc;
     if (*g_error_flag_host) { aprnet_set_error("a previous tensor-core kernel gave up waiting on a barrier"); return APRNET_ERR_CUDA; }
-    const TcGeom g = tc_geometry(1, cout, cin, slots);
+    const TcGeom g = tc_geometry(1, cout, cin, slots, tiles_of(a, dl), true);
     if (g.kpad != gpad) { aprnet_set_error("packed row width %d does not match the padded channel count %d", gpad, g.kpad); return APRNET_ERR_ARG; }
     const int cml = a->cml(dl);
     std::vector<Segment> segs;
@@ -697,8 +671,8 @@ int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots
     return dispatch_tc(P, g, total, st, pname);
 }
 
-size_t aprnet_tc_rows_bytes(ll rows, int channels) { return tc_geometry(rows, channels, 16, 1).rows_bytes; }
-size_t aprnet_tc_weight_bytes(int k_dim, int n_dim, int slots) { return tc_geometry(1, k_dim, n_dim, slots).w_bytes; }
+size_t aprnet_tc_rows_bytes(ll rows, int channels) { return tc_geometry(rows, channels, 16, 1, rows, false).rows_bytes; }
+size_t aprnet_tc_weight_bytes(int k_dim, int n_dim, int slots) { return tc_geometry(1, k_dim, n_dim, slots, 1 << 20, false).w_bytes; }
 int aprnet_tc_pad(int channels) { return pad_to(channels, 16); }
 
 extern "C" int aprnet_tc_error_flag(void) { return g_error_flag_host ? *g_error_flag_host : 0; }

@@ -347,7 +347,8 @@ extern "C" int aprnet_conv333_backward_weights_tc(aprnet_apr* a, int dl, int cin
     budget = std::max<ll>(P.n_segs, std::min<ll>(budget, max_ranges));
     auto blocks_of = [&](int i, ll per_block) { return ((P.seg_end[i] - P.seg_begin[i] + PT - 1) / PT + per_block - 1) / per_block; };
     auto blocks_for = [&](ll per_block) { ll b = 0; for (int i = 0; i < P.n_segs; ++i) b += blocks_of(i, per_block); return b; };
-    ll per_block = std::max<ll>(1, (total_chunks + budget - 1) / budget);
+    // (at least four chunks per block: the block sums of 256 x 256 channels are 7 MB per range)
+    ll per_block = std::max<ll>(4, (total_chunks + budget - 1) / budget);
     while (blocks_for(per_block) > budget) ++per_block;
     P.range_first[0] = 0;
     for (int i = 0; i < P.n_segs; ++i) {

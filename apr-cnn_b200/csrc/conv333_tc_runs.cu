@@ -27,6 +27,7 @@ typedef long long ll;
 constexpr int MAX_SEGS = APRNET_MAX_LEVELS;
 constexpr int MAX_STAGES = 16;
 constexpr int MAX_ACC = 4;
+constexpr int MAX_N = 256;                               // result channels of all tiles, where a bias is added
 constexpr int NPROD = 8;                                 // producer warps
 constexpr int MMA_WARP = NPROD, EPI_WARP = NPROD + 2;    // two MMA warps, two sets of four epilogue warps
 constexpr int THREADS = (NPROD + 2 + 8) * 32;
@@ -41,10 +42,10 @@ struct RunParams {
     const int32_t* loc;
     const __nv_bfloat16* rows; int kpad;
     ll tree_base, zero_row;
-    const __nv_bfloat16* wp;                             // packed weights [slot][tap][k chunk][NT][8]
-    float* out; ll ld_out; int n_dim;
+    const __nv_bfloat16* wp;                             // packed weights [slot][tap][n tile][k chunk][NT][8]
+    float* out; ll ld_out; int n_dim, n_tiles;           // results, tiles of NT channels
     const float* bias;
-    int same_level_only;
+    int same_level_only;                                 // input gradient: sources of the tile's own level, taps mirrored
     int* error_flag;
 };
 
@@ -52,13 +53,14 @@ template<int KS> __device__ __forceinline__ int swizzled_chunk(int row, int c) {
     return KS == 64 ? (c ^ (row & 7)) : (KS == 32 ? (c ^ ((row >> 1) & 3)) : (c ^ ((row >> 2) & 1)));
 }
 
-struct Tile { ll s0, sb, se, lo, hi; int wslot; };       // s0: slot of staged row 0
+struct Tile { ll s0, sb, se, lo, hi; int wslot, ntile; };       // s0: slot of staged row 0
 
-__device__ __forceinline__ Tile tile_of(const RunParams& P, int tile, int rows) {
+__device__ __forceinline__ Tile tile_of(const RunParams& P, int work, int rows) {
+    const int tile = work / P.n_tiles;
     int seg = 0;
     while (seg + 1 < P.n_segs && tile >= P.tile_begin[seg + 1]) ++seg;
     Tile t;
-    t.sb = P.slot_begin[seg]; t.se = P.slot_end[seg]; t.lo = P.lo[seg]; t.hi = P.hi[seg]; t.wslot = P.wslot[seg];
+    t.sb = P.slot_begin[seg]; t.se = P.slot_end[seg]; t.lo = P.lo[seg]; t.hi = P.hi[seg]; t.wslot = P.wslot[seg]; t.ntile = work - tile * P.n_tiles;
     t.s0 = t.sb - 1 + (ll) (tile - P.tile_begin[seg]) * (rows - 2);      // the first and the last row have no neighbour on one side
     return t;
 }
@@ -89,6 +91,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     constexpr uint32_t IDESC = make_idesc(NT, false, false);
     static_assert(STAGE_BYTES % 1024 == 0 && H * NT <= 512 && WROWS % 32 == 0, "stages keep the swizzle alignment; accumulators fit TMEM");
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ float bias_s[MAX_N];
     // ring at a multiple of 1024 bytes, with 1024 bytes in front of it (row -1 of the first stage is read, its results are not used)
     unsigned char* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u) + 1024;
     uint64_t* bars = reinterpret_cast<uint64_t*>(ring + (size_t) stages * STAGE_BYTES + 1024);
@@ -101,10 +104,11 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kchunks = P.kpad / KS, steps = 9 * kchunks;
-    const int total_tiles = P.tile_begin[P.n_segs];
+    const int total_tiles = P.tile_begin[P.n_segs] * P.n_tiles;
     const int my_tiles = (int) blockIdx.x < total_tiles ? (total_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
     const int ngroups = min(NG, stages);
 
+    if (P.bias) for (int c = tid; c < min(MAX_N, P.n_tiles * NT); c += THREADS) bias_s[c] = c < P.n_dim ? P.bias[c] : 0.f;
     if (tid == 0) {
         for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), WPS * 32 + 1); mbar_init(smem_u32(empty + i), ISSUERS); }
         for (int i = 0; i < 2 * MAX_ACC; ++i) { mbar_init(smem_u32(tmem_full + i), 1); mbar_init(smem_u32(tmem_empty + i), 4); }
@@ -124,7 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
         if (grp < ngroups) {
             const int j = lane % CH, rsub = lane / CH;
             const uint32_t total = (uint32_t) my_tiles * (uint32_t) steps;
-            const ll w_tap_stride = (ll) P.kpad * NT * 2;
+            const ll w_tile = (ll) P.kpad * NT * 2, w_tap_stride = P.n_tiles * w_tile;
             uint32_t g = grp, slot = grp, use = 0;
             int it = 0, step = grp, cur_it = -1;
             Tile t;
@@ -152,7 +156,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
                     else if (v != APRNET_NONE) r = P.tree_base + aprnet_dec_tree(v);
                     cur[i] = (int32_t) r;
                 }
-                const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(P.wp) + (ll) t.wslot * 27 * w_tap_stride;
+                const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(P.wp) + (ll) t.wslot * 27 * w_tap_stride + t.ntile * w_tile;
                 step += ngroups;
                 if (g + ngroups < total) { locate(); request(step / kchunks); }      // in flight while this stage is copied
                 if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
                     mbar_expect_tx(smem_u32(full + slot), 3 * B_TAP);
 #pragma unroll
                     for (int dy = 0; dy < 3; ++dy)
-                        bulk_copy_g2s(smem_u32(a_s + A_BYTES + dy * B_TAP), wsrc + (3 * d + dy) * w_tap_stride + (ll) kc * KS * NT * 2, B_TAP, smem_u32(full + slot));
+                        bulk_copy_g2s(smem_u32(a_s + A_BYTES + dy * B_TAP), wsrc + (P.same_level_only ? 26 - 3 * d - dy : 3 * d + dy) * w_tap_stride + (ll) kc * KS * NT * 2, B_TAP, smem_u32(full + slot));
                     bulk_issued = true;
                 }
                 const __nv_bfloat16* src0 = P.rows + kc * KS + j * 8;
@@ -229,6 +233,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
 #pragma unroll
         for (int b = 0; b < BLOCKS; ++b) p_next[b] = location(0, h0 + b * ISSUERS);
         for (int it = 0; it < my_tiles; ++it) {
+            const int n0 = (int) ((blockIdx.x + it * gridDim.x) % (unsigned) P.n_tiles) * NT;
             int32_t p_cur[BLOCKS];
 #pragma unroll
             for (int b = 0; b < BLOCKS; ++b) { p_cur[b] = p_next[b]; p_next[b] = location(it + 1, h0 + b * ISSUERS); }
@@ -246,13 +251,13 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
                     if (P.bias) {
 #pragma unroll
                         for (int jj = 0; jj < 32; ++jj)
-                            if (c0 + jj < P.n_dim) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + __ldg(P.bias + c0 + jj));
+                            r[jj] = __float_as_uint(__uint_as_float(r[jj]) + bias_s[n0 + c0 + jj]);
                     }
                     if (p >= 0) {
-                        float* dst = P.out + (ll) c0 * P.ld_out + p;
+                        float* dst = P.out + (ll) (n0 + c0) * P.ld_out + p;
 #pragma unroll
                         for (int jj = 0; jj < 32; ++jj)
-                            if (c0 + jj < P.n_dim) dst[(ll) jj * P.ld_out] = __uint_as_float(r[jj]);
+                            if (n0 + c0 + jj < P.n_dim) dst[(ll) jj * P.ld_out] = __uint_as_float(r[jj]);
                     }
                 }
             }
@@ -278,7 +283,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
 constexpr size_t FIXED = (2 * MAX_STAGES + 4 * MAX_ACC) * 8 + 16 + 2048 + 1024;      // barriers, the rows in front of and behind the ring, alignment
 
 inline size_t stage_bytes(int nt, int ks, int h) { return (size_t) 128 * h * ks * 2 + 3 * (size_t) nt * ks * 2; }
-inline int run_stages(int nt, int ks, int h) { return (int) std::min<size_t>(MAX_STAGES, (227 * 1024 - FIXED) / stage_bytes(nt, ks, h)); }
+inline int run_stages(int nt, int ks, int h) { return (int) std::min<size_t>(MAX_STAGES, (226 * 1024 - FIXED) / stage_bytes(nt, ks, h)); }
 
 template<int NT, int KS, int KORD, int H, int WPS>
 int launch_runs(RunParams& P, int sms, cudaStream_t st, const char* pname) {
@@ -289,7 +294,7 @@ int launch_runs(RunParams& P, int sms, cudaStream_t st, const char* pname) {
     for (int i = 0; i < P.n_segs; ++i) P.tile_begin[i + 1] = P.tile_begin[i] + aprnet_ceil_div(P.slot_end[i] - P.slot_begin[i], 128 * H - 2);
     if (P.tile_begin[P.n_segs] == 0) return APRNET_OK;
     AprnetProfScope _prof(pname, st);
-    kern<<<std::min(P.tile_begin[P.n_segs], sms), THREADS, smem, st>>>(P, stages);
+    kern<<<std::min(P.tile_begin[P.n_segs] * P.n_tiles, sms), THREADS, smem, st>>>(P, stages);
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
@@ -306,7 +311,7 @@ inline int pick_h(const RunParams& P, int nt, int ks, int max_h, int sms) {
         ll tiles = 0;
         for (int i = 0; i < P.n_segs; ++i) tiles += aprnet_ceil_div(P.slot_end[i] - P.slot_begin[i], 128 * h - 2);
         const double stage = 550 + h * 3 * (ks / 16) * (32 + nt / 4) + 1.3 * stage_bytes(nt, ks, h) / 128;
-        const double c = (double) ((tiles + sms - 1) / sms) * (9 * P.kpad / ks) * stage;
+        const double c = (double) ((tiles * P.n_tiles + sms - 1) / sms) * (9 * P.kpad / ks) * stage;
         if (h == 1 || c < cost) { cost = c; best = h; }
     }
     return best;
@@ -314,15 +319,14 @@ inline int pick_h(const RunParams& P, int nt, int ks, int max_h, int sms) {
 
 } // namespace
 
-// Channels between two changes of dy (the order of the products) of this kernel for kpad source channels and a tile of nt result
-// channels; 0: not this kernel.  The forward pass keeps the order of conv333_tc.cu, whose stages of `ks` channels hold three taps for
-// nt <= 64 (the same order as here) but one tap for nt = 128 (the same only when all channels are in one stage).  The input gradient is
-// free: nothing that follows depends on its last bit.
-int aprnet_tc_runs_order(int backward, int kpad, int nt, int ks) {
-    if (nt > 128) return 0;
-    if (nt <= 64) return ks;
-    if (!backward) return kpad == ks ? ks : 0;
-    return kpad % 32 == 0 ? 32 : 16;
+// Channels between two changes of dy (the order of the products) of this kernel for kpad source channels; 0: not this kernel.
+// nt_order, ks: tile width and channels per stage that conv333_tc.cu takes for the layer.  The forward pass keeps its order: stages of
+// `ks` channels that hold three taps for nt_order <= 64 (the same order as here) but fewer for wider tiles (the same only when all
+// channels are in one stage of one tap).  The input gradient is free: nothing that follows depends on its last bit.
+int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int ks) {
+    if (backward) return kpad % 32 == 0 ? 32 : 16;
+    if (nt_order <= 64) return ks;
+    return nt_order == 128 && kpad == ks ? ks : 0;
 }
 
 int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, ll tree_base, ll zero_row, const void* wp,
@@ -339,7 +343,7 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     if (P.n_segs == 0) return APRNET_OK;
     P.src = rp->src; P.S = rp->n_slots; P.loc = rp->loc;
     P.rows = (const __nv_bfloat16*) rows; P.kpad = kpad; P.tree_base = tree_base; P.zero_row = zero_row;
-    P.wp = (const __nv_bfloat16*) wp; P.out = out; P.ld_out = ld_out; P.n_dim = n_dim; P.bias = bias; P.same_level_only = backward;
+    P.wp = (const __nv_bfloat16*) wp; P.out = out; P.ld_out = ld_out; P.n_dim = n_dim; P.n_tiles = (n_dim + nt - 1) / nt; P.bias = bias; P.same_level_only = backward;
     P.error_flag = error_flag;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -352,6 +356,7 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     RUN_CASE(32, 16, 16, 1, 2) RUN_CASE(32, 16, 16, 2, 2) RUN_CASE(32, 16, 16, 4, 2) RUN_CASE(32, 16, 16, 8, 4)
     RUN_CASE(32, 32, 32, 1, 2) RUN_CASE(32, 32, 32, 2, 2) RUN_CASE(32, 32, 32, 4, 2)
     RUN_CASE(32, 64, 64, 1, 2) RUN_CASE(32, 64, 64, 2, 2) RUN_CASE(32, 64, 64, 4, 4)
+    RUN_CASE(32, 64, 32, 1, 2) RUN_CASE(32, 64, 32, 2, 2) RUN_CASE(32, 64, 32, 4, 4) RUN_CASE(64, 64, 64, 1, 2) RUN_CASE(64, 64, 64, 2, 4) RUN_CASE(64, 64, 64, 4, 4)
     RUN_CASE(64, 16, 16, 1, 2) RUN_CASE(64, 16, 16, 2, 2) RUN_CASE(64, 16, 16, 4, 2)
     RUN_CASE(64, 32, 32, 1, 2) RUN_CASE(64, 32, 32, 2, 2) RUN_CASE(64, 32, 32, 4, 2)
     RUN_CASE(64, 64, 32, 1, 2) RUN_CASE(64, 64, 32, 2, 4) RUN_CASE(64, 64, 32, 4, 4)

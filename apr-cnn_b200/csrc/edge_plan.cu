@@ -342,8 +342,8 @@ extern "C" int64_t aprnet_edge_workspace_bytes(const aprnet_apr* a, int dl, int 
 
 // Cross-level part of the input gradient (added to grad_input, which holds the same-level part, and to
 // grad_tree, which the call zero-fills) followed by the tree adjoint.  packed_grad_output_rows:
-// channels-last bf16 dO rows; weights fp32 (slots, Cout, Cin, 27); wp_ws: space for the packed
-// transposed weights; edge_ws: aprnet_edge_workspace_bytes() bytes.
+// channels-last bf16 dO rows; weights fp32 (slots, Cout, Cin, 27); wp_ws: the packed transposed
+// weights; edge_ws: aprnet_edge_workspace_bytes() bytes.
 int aprnet_cross_level_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* grows, int gpad, const float* w, float* gin,
                           long long ld_in, float* gtree, long long ld_tree, void* wp_ws, void* edge_ws, long long edge_ws_bytes, void* stream,
                           bool tree_adjoint) {
@@ -355,8 +355,7 @@ int aprnet_cross_level_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, c
     const ll ts = a->tree_size(dl);
     if (ts > 0) APRNET_CUDA_CHECK(cudaMemset2DAsync(gtree, (size_t) ld_tree * sizeof(float), 0, (size_t) ts * sizeof(float), (size_t) cin, st));
     if (ep->n_active > 0) {
-        int rc = aprnet_tc_pack_weights(w, slots, cin, cout, 2, wp_ws, st);
-        if (rc) return rc;
+        int rc = APRNET_OK;
         __nv_bfloat16* vrows = reinterpret_cast<__nv_bfloat16*>(edge_ws);
         APRNET_CUDA_CHECK(cudaMemsetAsync(vrows, 0, (size_t) gpad * 2, st));          // row 0: zeros
         const ll cap_rows = edge_ws_bytes / ((ll) gpad * 2) - 1;
@@ -389,5 +388,7 @@ extern "C" int aprnet_conv333_backward_input_cross_level_tc(aprnet_apr* a, int d
                                                             const void* grows, int gpad, const float* w, float* gin,
                                                             int64_t ld_in, float* gtree, int64_t ld_tree, void* wp_ws,
                                                             void* edge_ws, int64_t edge_ws_bytes, void* stream) {
-    return aprnet_cross_level_tc(a, dl, cin, cout, slots, grows, gpad, w, gin, ld_in, gtree, ld_tree, wp_ws, edge_ws, edge_ws_bytes, stream, true);
+    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && w && wp_ws, "bad argument");
+    const int rc = aprnet_tc_pack_weights(a, dl, w, slots, cin, cout, 1, wp_ws, (cudaStream_t) stream);
+    return rc ? rc : aprnet_cross_level_tc(a, dl, cin, cout, slots, grows, gpad, w, gin, ld_in, gtree, ld_tree, wp_ws, edge_ws, edge_ws_bytes, stream, true);
 }

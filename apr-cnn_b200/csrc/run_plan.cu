@@ -14,6 +14,15 @@ namespace {
 
 typedef long long ll;
 
+// rows of all levels of the level delta, level by level
+struct RunLevels { int lmin, cml, dl; ll begin[APRNET_MAX_LEVELS + 2]; ll tree_off; };
+
+__device__ __forceinline__ int level_of_row(const RunLevels& R, ll row) {
+    int l = R.lmin;
+    while (l < R.cml && row >= R.begin[l + 1]) ++l;
+    return l;
+}
+
 struct RunRow {                 // the sorted y coordinates of one row: particles, and at the finest level of a pooled tensor tree nodes
     const uint16_t *a, *b;
     ll ia, ea, ib, eb;
@@ -37,16 +46,19 @@ __device__ __forceinline__ RunRow run_row(const LevelMeta& m, const ll* row_ptr,
 }
 
 // one thread per row; first pass (slot_y == null): count[row] = slots of the row; second pass: the slots from first[row] on
-__global__ void run_slots_kernel(LevelMeta m, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y, const ll* __restrict__ trow_ptr,
-                                 const uint16_t* __restrict__ ty, int l, int with_tree, ll tree_off, int32_t* __restrict__ count,
-                                 const int32_t* __restrict__ first, int32_t* __restrict__ slot_y, int32_t* __restrict__ slot_loc) {
-    const ll row = (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= (ll) m.z_num[l] * m.x_num[l]) return;
+__global__ void run_slots_kernel(LevelMeta m, RunLevels R, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y, const ll* __restrict__ trow_ptr,
+                                 const uint16_t* __restrict__ ty, int32_t* __restrict__ count, const int32_t* __restrict__ first,
+                                 int32_t* __restrict__ slot_y, int32_t* __restrict__ slot_loc) {
+    const ll g = (ll) blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= R.begin[R.cml + 1]) return;
+    const int l = level_of_row(R, g);
+    const ll row = g - R.begin[l], tree_off = R.tree_off;
+    const int with_tree = R.dl > 0 && l == R.cml;
     RunRow r = run_row(m, row_ptr, y, trow_ptr, ty, l, row, with_tree);
     int last = -3, n = 0, yy;
     ll index;
     bool from_b;
-    const ll base = slot_y ? first[row] : 0;
+    const ll base = slot_y ? first[g] : 0;
     while (r.next(&yy, &index, &from_b)) {
         for (int c = max(yy - 1, last + 1); c <= yy + 1; ++c) {
             if (slot_y) { slot_y[base + n] = c; slot_loc[base + n] = -1; }
@@ -55,7 +67,7 @@ __global__ void run_slots_kernel(LevelMeta m, const ll* __restrict__ row_ptr, co
         last = yy + 1;
         if (slot_y) slot_loc[base + n - 2] = (int32_t) (from_b ? index + tree_off : index);
     }
-    if (!slot_y) count[row] = n;
+    if (!slot_y) count[g] = n;
 }
 
 __device__ __forceinline__ ll find_cell(const uint16_t* __restrict__ y, ll b, ll e, int target) {
@@ -65,14 +77,16 @@ __device__ __forceinline__ ll find_cell(const uint16_t* __restrict__ y, ll b, ll
 }
 
 // one warp per row: what fills cell (z + dz, x + dx, y) for every slot of the row; resolution as in build_nbr_table_kernel
-__global__ void run_sources_kernel(LevelMeta m, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y, const ll* __restrict__ trow_ptr,
-                                   const uint16_t* __restrict__ ty, int l, int cml, ll tree_off, const int32_t* __restrict__ first,
-                                   const int32_t* __restrict__ slot_y, ll S, int32_t* __restrict__ src) {
-    const ll row = ((ll) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__global__ void run_sources_kernel(LevelMeta m, RunLevels R, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y, const ll* __restrict__ trow_ptr,
+                                   const uint16_t* __restrict__ ty, const int32_t* __restrict__ first, const int32_t* __restrict__ slot_y, ll S,
+                                   int32_t* __restrict__ src) {
+    const ll g = ((ll) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    if (g >= R.begin[R.cml + 1]) return;
+    const int l = level_of_row(R, g), cml = R.cml;
+    const ll row = g - R.begin[l], tree_off = R.tree_off;
     const int xn = m.x_num[l], zn = m.z_num[l], yn = m.y_num[l];
-    if (row >= (ll) zn * xn) return;
-    const ll sb = first[row], se = first[row + 1];
+    const ll sb = first[g], se = first[g + 1];
     if (sb == se) return;
     const int z = (int) (row / xn), x = (int) (row % xn);
     for (int d = 0; d < 9; ++d) {
@@ -127,11 +141,11 @@ __global__ void pick_kernel(const int32_t* __restrict__ v, Picks at, int n, int3
 int build_run_plan(aprnet_apr* a, int dl, RunPlan& rp, cudaStream_t st) {
     const LevelMeta& m = a->meta;
     const int cml = a->cml(dl);
-    const ll toff = dl > 0 ? a->tree_offset(cml) : 0;
+    RunLevels R;
+    R.lmin = m.level_min; R.cml = cml; R.dl = dl; R.tree_off = dl > 0 ? a->tree_offset(cml) : 0;
     ll rows = 0;
-    std::vector<ll> row_begin(cml + 2, 0);
-    for (int l = m.level_min; l <= cml; ++l) { row_begin[l] = rows; rows += (ll) m.z_num[l] * m.x_num[l]; }
-    row_begin[cml + 1] = rows;
+    for (int l = m.level_min; l <= cml; ++l) { R.begin[l] = rows; rows += (ll) m.z_num[l] * m.x_num[l]; }
+    R.begin[cml + 1] = rows;
     int32_t *first = nullptr, *slot_y = nullptr, *picked = nullptr;
     int rc = APRNET_OK;
     void* temp = nullptr;
@@ -141,15 +155,13 @@ int build_run_plan(aprnet_apr* a, int dl, RunPlan& rp, cudaStream_t st) {
 #define RP_CHECK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) { aprnet_set_error("%s failed: %s", #expr, cudaGetErrorString(_e)); cudaGetLastError(); cleanup(); return APRNET_ERR_CUDA; } } while (0)
     RP_ALLOC(first, (size_t) (rows + 1) * sizeof(int32_t));
     RP_CHECK(cudaMemsetAsync(first + rows, 0, sizeof(int32_t), st));
-    for (int l = m.level_min; l <= cml; ++l)
-        run_slots_kernel<<<aprnet_ceil_div((ll) m.z_num[l] * m.x_num[l], 128), 128, 0, st>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, l, dl > 0 && l == cml, toff,
-                                                                                       first + row_begin[l], nullptr, nullptr, nullptr);
+    run_slots_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, first, nullptr, nullptr, nullptr);
     RP_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, first, first, (int) (rows + 1), st));
     RP_ALLOC(temp, std::max<size_t>(temp_bytes, 1));
     RP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, first, first, (int) (rows + 1), st));
     std::vector<int32_t> at(cml + 2, 0);
     Picks picks;
-    for (int l = m.level_min; l <= cml + 1; ++l) picks.at[l - m.level_min] = row_begin[l];
+    for (int l = m.level_min; l <= cml + 1; ++l) picks.at[l - m.level_min] = R.begin[l];
     RP_ALLOC(picked, sizeof(int32_t) * (APRNET_MAX_LEVELS + 2));
     pick_kernel<<<1, 32, 0, st>>>(first, picks, cml + 2 - m.level_min, picked);
     RP_CHECK(cudaMemcpyAsync(at.data() + m.level_min, picked, sizeof(int32_t) * (cml + 2 - m.level_min), cudaMemcpyDeviceToHost, st));
@@ -160,12 +172,8 @@ int build_run_plan(aprnet_apr* a, int dl, RunPlan& rp, cudaStream_t st) {
     RP_ALLOC(slot_y, (size_t) std::max<ll>(S, 1) * sizeof(int32_t));
     RP_ALLOC(rp.loc, (size_t) std::max<ll>(S, 1) * sizeof(int32_t));
     RP_ALLOC(rp.src, (size_t) std::max<ll>(S, 1) * 9 * sizeof(int32_t));
-    for (int l = m.level_min; l <= cml; ++l) {
-        const ll n = (ll) m.z_num[l] * m.x_num[l];
-        run_slots_kernel<<<aprnet_ceil_div(n, 128), 128, 0, st>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, l, dl > 0 && l == cml, toff, nullptr,
-                                                                 first + row_begin[l], slot_y, rp.loc);
-        run_sources_kernel<<<aprnet_ceil_div(n * 32, 128), 128, 0, st>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, l, cml, toff, first + row_begin[l], slot_y, S, rp.src);
-    }
+    run_slots_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, nullptr, first, slot_y, rp.loc);
+    run_sources_kernel<<<aprnet_ceil_div(rows * 32, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, first, slot_y, S, rp.src);
     RP_CHECK(cudaGetLastError());
     RP_CHECK(cudaStreamSynchronize(st));
 #undef RP_CHECK

@@ -68,10 +68,7 @@ class Conv111Function(Function):
         ctx.aprs = aprs
         ctx.precision = precision or ""
         ctx.save_for_backward(inputs, weights, bias, level_deltas.clone())
-        out = conv111_forward(APRPtrVector(aprs), inputs, weights, level_deltas, ctx.precision)
-        if bias is not None:
-            out = out + bias.view(1, -1, 1)
-        return out
+        return conv111_forward(APRPtrVector(aprs), inputs, weights, level_deltas, ctx.precision, bias)
 
     @staticmethod
     def backward(ctx, grad_output):

@@ -261,6 +261,10 @@ int aprnet_tc_set_option(const char* name, int value);
 int aprnet_conv111_forward(const aprnet_apr* apr, int level_delta, int dtype, int cin, int cout, int num_stencils,
                            const void* input, int64_t ld_in, const void* weights, void* output, int64_t ld_out,
                            void* stream);
+/* the same with a bias (Cout) added to every output, or NULL */
+int aprnet_conv111_forward_bias(const aprnet_apr* apr, int level_delta, int dtype, int cin, int cout, int num_stencils,
+                                const void* input, int64_t ld_in, const void* weights, const void* bias, void* output,
+                                int64_t ld_out, void* stream);
 int aprnet_conv111_backward_input(const aprnet_apr* apr, int level_delta, int dtype, int cin, int cout,
                                   int num_stencils, const void* grad_output, int64_t ld_out, const void* weights,
                                   void* grad_input, int64_t ld_in, void* stream);
@@ -270,6 +274,9 @@ int aprnet_conv111_backward_input(const aprnet_apr* apr, int level_delta, int dt
  * above then. */
 int aprnet_conv111_forward_tc(const aprnet_apr* apr, int level_delta, int cin, int cout, int num_stencils,
                               const float* input, int64_t ld_in, const float* weights, float* output, int64_t ld_out, void* stream);
+int aprnet_conv111_forward_tc_bias(const aprnet_apr* apr, int level_delta, int cin, int cout, int num_stencils,
+                                   const float* input, int64_t ld_in, const float* weights, const float* bias, float* output,
+                                   int64_t ld_out, void* stream);
 int aprnet_conv111_backward_input_tc(const aprnet_apr* apr, int level_delta, int cin, int cout, int num_stencils,
                                      const float* grad_output, int64_t ld_out, const float* weights, float* grad_input, int64_t ld_in,
                                      void* stream);
