@@ -273,12 +273,12 @@ static std::vector<torch::Tensor> conv333_backward_rows(std::vector<APR*>& aprs,
     ld_tree = std::max(ld_tree, B.max_tree);
     auto grad_tree = need_grad_input ? torch::empty({fold_tree ? 1 : nb, cin, ld_tree}, grad_output.options()) : torch::Tensor();
     auto grad_input = need_grad_input ? torch::empty({nb, cin, n}, grad_output.options()) : torch::Tensor();
-    auto grad_weights = torch::zeros_like(weights);
+    auto grad_weights = nb > 0 ? torch::empty_like(weights) : torch::zeros_like(weights);
     auto ws = bytes_like(bytes, grad_output);
     auto partial = torch::empty({aprnet_conv333_rows_partial_elems(mode, cin, cout)}, grad_output.options());
     for (int64_t b = 0; b < nb; ++b)
         check(aprnet_conv333_rows_backward(B.h[b], B.dl[b], mode, cin, cout, slots, row(rows, b), (const float*) row(grad_output, b), n, weights.data_ptr<float>(),
-                                           need_grad_input ? (float*) row(grad_input, b) : nullptr, n, grad_weights.data_ptr<float>(),
+                                           need_grad_input ? (float*) row(grad_input, b) : nullptr, n, grad_weights.data_ptr<float>(), b > 0 ? 1 : 0,
                                            need_grad_input ? (float*) row(grad_tree, fold_tree ? 0 : b) : nullptr, ld_tree, fold_tree ? 1 : 0,
                                            partial.data_ptr<float>(), ws.data_ptr(), stream_of(grad_output)),
               mode == APRNET_PREC_BF16 ? "conv333_backward (tensor cores)" : "conv333_backward");

@@ -167,7 +167,7 @@ bool aprnet_small_cin(int cin);
 int aprnet_small_stage(const float* x, long long ld_x, long long n, const float* tree, long long ld_tree, long long t, int cin, float* vals, cudaStream_t st);
 int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, const float* bias, float* out, long long ld_out, cudaStream_t st);
 int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* gout, long long ld_out,
-                                  float* gw, float* partial, cudaStream_t st);
+                                  float* gw, int accumulate, float* partial, cudaStream_t st);
 // tensor-core gather over runs (conv333_tc_runs.cu)
 int aprnet_tc_runs_order(int backward, int kpad, int nt, int ks);
 int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, long long tree_base, long long zero_row, const void* wp,
@@ -197,13 +197,16 @@ int aprnet_f32_pack_input(const aprnet_apr* a, int dl, int cin, const float* in,
 int aprnet_f32_pack_grad(const aprnet_apr* a, int dl, int cout, const float* gout, long long ld_out, void* grows, cudaStream_t st);
 int aprnet_f32_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* w, const float* bias, float* out, long long ld_out, void* workspace, cudaStream_t st);
 int aprnet_f32_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* rows, const float* gout, long long ld_out, const void* grows,
-                                float* gw, float* partial, cudaStream_t st);
+                                float* gw, int accumulate, float* partial, cudaStream_t st);
 int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* gout, long long ld_out, const float* w, float* gin, long long ld_in,
                               float* gtree, long long ld_tree, void* workspace, bool tree_adjoint, cudaStream_t st);
 
 // ranges of block partial sums [range][27][cin][cout] per stencil slot: slot[g] owns [first[g], first[g + 1]), g < n
-struct SlotRanges { int n; int first[APRNET_MAX_LEVELS + 1]; int slot[APRNET_MAX_LEVELS]; };
-int aprnet_dw_reduce(const float* partial, const SlotRanges& sr, int cin, int cout, float* gw, cudaStream_t st);      // grad_weights += sums, fixed order
+struct SlotRanges { int n; int first[APRNET_MAX_LEVELS + 1]; int slot[APRNET_MAX_LEVELS]; unsigned empty; };      // empty: slots to zero (bit per slot)
+// grad_weights (slots, Cout, Cin, 27) += sums in a fixed order; without `accumulate` all of it is written (zeros in slots without ranges)
+int aprnet_dw_reduce(const float* partial, SlotRanges sr, int slots, int accumulate, int cin, int cout, float* gw, cudaStream_t st);
+int aprnet_tc_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* xrows, int xpad, const void* grows, int gpad, float* gw, int accumulate,
+                               float* partial, cudaStream_t st);
 
 // stream-ordered scratch of one call, for entry points whose signature has no workspace
 struct StreamScratch {

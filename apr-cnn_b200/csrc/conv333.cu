@@ -518,7 +518,7 @@ int backward_input_f32(aprnet_apr* a, int dl, int cin, int cout, int slots, cons
     if (27 * a->number_parts(dl) + 1 < (1ll << 31) && !aprnet_get_edge_plan(a, dl, st)) return APRNET_ERR_CUDA;
     StreamScratch ws(st);
     const int rc = ws.get((size_t) aprnet_conv333_rows_backward_workspace_bytes(a, dl, APRNET_PREC_F32, cin, cout, slots, 1));
-    return rc ? rc : aprnet_conv333_rows_backward(a, dl, APRNET_PREC_F32, cin, cout, slots, nullptr, gout, ld_out, w, gin, ld_in, nullptr, gtree, ld_tree,
+    return rc ? rc : aprnet_conv333_rows_backward(a, dl, APRNET_PREC_F32, cin, cout, slots, nullptr, gout, ld_out, w, gin, ld_in, nullptr, 1, gtree, ld_tree,
                                                   fold_tree, nullptr, ws.p, st);
 }
 
@@ -529,7 +529,7 @@ int backward_weights_f32(aprnet_apr* a, int dl, int cin, int cout, int slots, co
     if ((rc = rows.get((size_t) aprnet_conv333_rows_bytes(a, dl, APRNET_PREC_F32, cin)))) return rc;
     if ((rc = ws.get((size_t) aprnet_conv333_rows_backward_workspace_bytes(a, dl, APRNET_PREC_F32, cin, cout, slots, 0)))) return rc;
     if ((rc = aprnet_conv333_rows_pack(a, dl, APRNET_PREC_F32, cin, in, ld_in, const_cast<float*>(tree), ld_tree, 1, rows.p, st))) return rc;
-    return aprnet_conv333_rows_backward(a, dl, APRNET_PREC_F32, cin, cout, slots, rows.p, gout, ld_out, nullptr, nullptr, 0, gw, const_cast<float*>(tree), ld_tree,
+    return aprnet_conv333_rows_backward(a, dl, APRNET_PREC_F32, cin, cout, slots, rows.p, gout, ld_out, nullptr, nullptr, 0, gw, 1, const_cast<float*>(tree), ld_tree,
                                         0, partial, ws.p, st);
 }
 

@@ -428,11 +428,18 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
 // grad_weights[slot][co][ci][tap] += the block sums [range][tap][ci][co] of the slot's ranges.  Block = one input channel, 32 output
 // channels, one slot: warp y takes every eighth range, 27 independent coalesced loads at a time; the warps' sums are combined in a
 // fixed order and leave transposed, 27 contiguous values per filter.
-__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, SlotRanges sr, int cin, int cout, float* __restrict__ gw) {
+__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, SlotRanges sr, int accumulate, int cin, int cout, float* __restrict__ gw) {
     __shared__ float sums[8][27][33];
     const int lane = threadIdx.x & 31, y = threadIdx.x >> 5;
     const int ci = blockIdx.x, co0 = blockIdx.y * 32, co = co0 + lane;
-    const int r0 = sr.first[blockIdx.z], r1 = sr.first[blockIdx.z + 1], ny = min(8, r1 - r0);
+    int slot, r0 = 0, r1 = 0;
+    if ((int) blockIdx.z < sr.n) { slot = sr.slot[blockIdx.z]; r0 = sr.first[blockIdx.z]; r1 = sr.first[blockIdx.z + 1]; }
+    else {                                     // the k-th slot without ranges
+        unsigned left = sr.empty;
+        for (int k = (int) blockIdx.z - sr.n; k > 0; --k) left &= left - 1;
+        slot = __ffs(left) - 1;
+    }
+    const int ny = min(8, r1 - r0);
     const ll tap_stride = (ll) cin * cout, range_stride = 27 * tap_stride;
     float s[27];
 #pragma unroll
@@ -450,12 +457,13 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict_
     }
     __syncthreads();
     const int n = min(32, cout - co0) * 27;
-    float* dst = gw + (((ll) sr.slot[blockIdx.z] * cout + co0) * cin + ci) * 27;
+    float* dst = gw + (((ll) slot * cout + co0) * cin + ci) * 27;
     for (int e = threadIdx.x; e < n; e += 256) {
         const int c = e / 27, t = e - c * 27;
         float v = 0.f;
         for (int k = 0; k < ny; ++k) v += sums[k][t][c];
-        dst[(ll) c * cin * 27 + t] += v;
+        float* o = dst + (ll) c * cin * 27 + t;
+        *o = accumulate ? *o + v : v;
     }
 }
 
@@ -562,12 +570,12 @@ int launch_dw(const F32DwParams& P, int nranges, int blocks_y, cudaStream_t st, 
     return APRNET_OK;
 }
 
-int run_dw(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* xrows, const float* grows, float* gw, float* partial, cudaStream_t st) {
+int run_dw(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* xrows, const float* grows, float* gw, int accumulate, float* partial, cudaStream_t st) {
     const AprPlan* plan = aprnet_get_plan(a, dl, st);
     if (!plan) return APRNET_ERR_CUDA;
     const DwGeom g = dw_geometry(cin, cout);
     const std::vector<Segment> segs = aprnet_segments(a, dl, slots, false);
-    if (segs.empty()) return APRNET_OK;
+    if (segs.empty()) return accumulate ? APRNET_OK : (cudaMemsetAsync(gw, 0, (size_t) slots * 27 * cin * cout * sizeof(float), st), APRNET_OK);
     const int budget = dw_max_ranges(cin, cout);
     F32DwParams P;
     P.n_segs = (int) segs.size();
@@ -600,7 +608,7 @@ int run_dw(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* xro
     DW_CASE(16, 64, 1, 4, 16) DW_CASE(16, 32, 2, 2, 16) DW_CASE(16, 16, 2, 2, 8) DW_CASE(16, 8, 2, 2, 4)
     DW_CASE(8, 64, 1, 4, 16) DW_CASE(8, 32, 2, 2, 16) DW_CASE(8, 16, 2, 2, 8) DW_CASE(8, 8, 2, 2, 4)
 #undef DW_CASE
-    return rc ? rc : aprnet_dw_reduce(partial, sr, cin, cout, gw, st);
+    return rc ? rc : aprnet_dw_reduce(partial, sr, slots, accumulate, cin, cout, gw, st);
 }
 
 // cross-level part of the input gradient (see edge_plan.cu; wp: the transposed weights as packed for the same-level part): sums per (target, tap), then the gather over the targets
@@ -655,9 +663,20 @@ inline size_t edge_bytes(const aprnet_apr* a, int dl, int cout) {
 
 } // namespace
 
-int aprnet_dw_reduce(const float* partial, const SlotRanges& sr, int cin, int cout, float* gw, cudaStream_t st) {
+int aprnet_dw_reduce(const float* partial, SlotRanges sr, int slots, int accumulate, int cin, int cout, float* gw, cudaStream_t st) {
+    int nz = sr.n;
+    sr.empty = 0;
+    if (!accumulate) {
+        if (slots > 32) { APRNET_CUDA_CHECK(cudaMemsetAsync(gw, 0, (size_t) slots * 27 * cin * cout * sizeof(float), st)); accumulate = 1; }      // (more slots than any structure has levels)
+        else {
+            sr.empty = slots == 32 ? ~0u : (1u << slots) - 1;
+            for (int i = 0; i < sr.n; ++i) sr.empty &= ~(1u << sr.slot[i]);
+            nz += __builtin_popcount(sr.empty);
+        }
+    }
+    if (nz == 0) return APRNET_OK;
     AprnetProfScope _prof("conv333_dw_reduce", st);
-    dw_reduce_kernel<<<dim3((unsigned) cin, (unsigned) aprnet_ceil_div(cout, 32), (unsigned) sr.n), 256, 0, st>>>(partial, sr, cin, cout, gw);
+    dw_reduce_kernel<<<dim3((unsigned) cin, (unsigned) aprnet_ceil_div(cout, 32), (unsigned) nz), 256, 0, st>>>(partial, sr, accumulate, cin, cout, gw);
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
@@ -710,9 +729,9 @@ int aprnet_f32_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, cons
 }
 
 int aprnet_f32_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* rows, const float* gout, ll ld_out, const void* grows,
-                                float* gw, float* partial, cudaStream_t st) {
-    if (aprnet_small_cin(cin)) return aprnet_small_backward_weights(a, dl, cin, cout, slots, (const float*) rows, gout, ld_out, gw, partial, st);
-    return run_dw(a, dl, cin, cout, slots, (const float*) rows, (const float*) grows, gw, partial, st);
+                                float* gw, int accumulate, float* partial, cudaStream_t st) {
+    if (aprnet_small_cin(cin)) return aprnet_small_backward_weights(a, dl, cin, cout, slots, (const float*) rows, gout, ld_out, gw, accumulate, partial, st);
+    return run_dw(a, dl, cin, cout, slots, (const float*) rows, (const float*) grows, gw, accumulate, partial, st);
 }
 
 // input gradient from the packed grad_output rows at the start of `workspace` (aprnet_f32_backward_bytes): grad_input is written,

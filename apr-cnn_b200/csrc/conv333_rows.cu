@@ -47,7 +47,7 @@ int forward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int sl
 
 // `ws`: grad_bytes() bytes.  gin == null: no input gradient; gw == null: no weight gradient; fold_tree: grad_tree is folded into gin
 int backward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const void* rows, const float* gout, ll ld_out, const float* w,
-                  float* gin, ll ld_in, float* gw, float* gtree, ll ld_tree, float* partial, void* ws, bool fold_tree, cudaStream_t st) {
+                  float* gin, ll ld_in, float* gw, int accumulate, float* gtree, ll ld_tree, float* partial, void* ws, bool fold_tree, cudaStream_t st) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && gout && (gin || gw) && (!gin || (w && gtree)) && ws && (!gw || (rows && partial)), "bad argument");
     APRNET_ARG_CHECK(ld_out >= a->number_parts(dl) && (!gin || (ld_in >= a->number_parts(dl) && ld_tree >= a->tree_size(dl))), "leading dimension too small");
     const ll n = a->number_parts(dl);
@@ -60,8 +60,8 @@ int backward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int s
         if (rc) return rc;
     }
     if (gw) {
-        rc = bf16 && !aprnet_small_cin(cin) ? aprnet_conv333_backward_weights_tc(a, dl, cin, cout, slots, rows, aprnet_tc_pad(cin), ws, gpad, gw, partial, st)
-                                            : aprnet_f32_backward_weights(a, dl, cin, cout, slots, rows, gout, ld_out, ws, gw, partial, st);
+        rc = bf16 && !aprnet_small_cin(cin) ? aprnet_tc_backward_weights(a, dl, cin, cout, slots, rows, aprnet_tc_pad(cin), ws, gpad, gw, accumulate, partial, st)
+                                            : aprnet_f32_backward_weights(a, dl, cin, cout, slots, rows, gout, ld_out, ws, gw, accumulate, partial, st);
         if (rc) return rc;
     }
     if (!gin) return APRNET_OK;
@@ -124,10 +124,10 @@ extern "C" int aprnet_conv333_rows_pack(aprnet_apr* a, int dl, int precision, in
 }
 
 extern "C" int aprnet_conv333_rows_backward(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const void* rows, const float* gout, int64_t ld_out,
-                                            const float* w, float* gin, int64_t ld_in, float* gw, float* gtree, int64_t ld_tree, int fold_tree,
+                                            const float* w, float* gin, int64_t ld_in, float* gw, int accumulate, float* gtree, int64_t ld_tree, int fold_tree,
                                             float* partial, void* workspace, void* stream) {
     APRNET_ARG_CHECK(precision_ok(precision), "unknown precision");
-    return backward_rows(a, dl, precision, cin, cout, slots, rows, gout, ld_out, w, gin, ld_in, gw, gtree, ld_tree, partial, workspace, fold_tree != 0, (cudaStream_t) stream);
+    return backward_rows(a, dl, precision, cin, cout, slots, rows, gout, ld_out, w, gin, ld_in, gw, accumulate, gtree, ld_tree, partial, workspace, fold_tree != 0, (cudaStream_t) stream);
 }
 
 // ---- the tensor-core entry points ------------------------------------------------------------------------
@@ -160,7 +160,7 @@ extern "C" int aprnet_conv333_backward_tc_rows(aprnet_apr* a, int dl, int cin, i
                                                const float* gout, int64_t ld_out, const float* w, float* gin, int64_t ld_in, float* gw,
                                                float* gtree, int64_t ld_tree, float* partial, void* workspace, void* stream) {
     APRNET_ARG_CHECK(gw, "bad argument");
-    return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, gtree, ld_tree, partial,
+    return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, 1, gtree, ld_tree, partial,
                          grad_area(a, dl, cin, workspace), true, (cudaStream_t) stream);
 }
 
@@ -170,7 +170,7 @@ extern "C" int aprnet_conv333_backward_tc_rows_pretree(aprnet_apr* a, int dl, in
                                                        const float* gout, int64_t ld_out, const float* w, float* gin, int64_t ld_in, float* gw,
                                                        float* gtree, int64_t ld_tree, float* partial, void* workspace, void* stream) {
     APRNET_ARG_CHECK(gw, "bad argument");
-    return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, gtree, ld_tree, partial,
+    return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, 1, gtree, ld_tree, partial,
                          grad_area(a, dl, cin, workspace), false, (cudaStream_t) stream);
 }
 

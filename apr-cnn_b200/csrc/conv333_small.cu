@@ -96,12 +96,15 @@ __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable seg
         if (co0 + o < cout) out[(ll) (co0 + o) * ld_out + p] = bias ? acc[o] + __ldg(bias + co0 + o) : acc[o];
 }
 
-// weight gradient of one level: block = range of locations x block of 32 output channels.  The 27 x CIN
-// gathered values and the 32 dO values of KP locations are staged in shared memory; a thread owns a 4 x 4
+// weight gradient: block = range of locations of one level x block of 32 output channels, one launch over all levels.  The 27 x CIN
+// gathered values and the 32 dO values of KP locations are staged in shared memory (all table entries of a step, then all values, are
+// requested before any is used: the staging is bound by their latency); a thread owns a 4 x 4
 // tile of (tap, ci) x co products; the 4 thread groups of a block take different quarters of every staged
-// step and are combined in a fixed order.  partial[range][co][ci][tap].
+// step and are combined in a fixed order.  partial[range][tap][ci][co].
+struct SmallRanges { int n; ll begin[MAX_SEGS], end[MAX_SEGS], len[MAX_SEGS]; int first[MAX_SEGS + 1]; };
+
 template<int CIN>
-__global__ void __launch_bounds__(256) conv333_small_dw_kernel(ll seg_begin, ll seg_end, ll range_len, const int32_t* __restrict__ nbr, ll N, ll T,
+__global__ void __launch_bounds__(256) conv333_small_dw_kernel(SmallRanges rg, const int32_t* __restrict__ nbr, ll N, ll T,
                                                                const float* __restrict__ vals, const float* __restrict__ gout, ll ld_out,
                                                                int cout, float* __restrict__ partial) {
     constexpr int ROWS = 27 * CIN, RQ = (ROWS + 3) / 4;                 // (tap, ci) rows, row quads
@@ -111,7 +114,9 @@ __global__ void __launch_bounds__(256) conv333_small_dw_kernel(ll seg_begin, ll 
     __shared__ F4 gs[KP][8 + 1];
     __shared__ float red[RQ * 4 * 32];
     const int co0 = blockIdx.y * 32;
-    const ll pb = seg_begin + (ll) blockIdx.x * range_len, pe = min(seg_end, pb + range_len);
+    int seg = 0;
+    while (seg + 1 < rg.n && (int) blockIdx.x >= rg.first[seg + 1]) ++seg;
+    const ll pb = rg.begin[seg] + (ll) ((int) blockIdx.x - rg.first[seg]) * rg.len[seg], pe = min(rg.end[seg], pb + rg.len[seg]);
     const ll R = N + T + 1;
     const int grp = threadIdx.x >> 6, t64 = threadIdx.x & 63;
     const int rq = t64 >> 3, cq = t64 & 7;                             // 8 row quads per pass of 64 threads
@@ -124,19 +129,26 @@ __global__ void __launch_bounds__(256) conv333_small_dw_kernel(ll seg_begin, ll 
 #pragma unroll
             for (int b = 0; b < 4; ++b) acc[ps][a][b] = 0.f;
     for (ll p0 = pb; p0 < pe; p0 += KP) {
-        for (int e = threadIdx.x; e < KP * RQ * 4; e += 256) {          // consecutive threads take consecutive locations of one row
-            const int k = e % KP, row = e / KP;
-            float v = 0.f;
-            if (row < ROWS && p0 + k < pe) {
-                const int tap = row / CIN, ci = row % CIN;
-                v = __ldg(vals + (ll) ci * R + resolve_row(__ldg(nbr + (ll) tap * N + p0 + k), N, N + T));
-            }
-            xs[k][row >> 2].a[row & 3] = v;
+        constexpr int NX = (KP * RQ * 4 + 255) / 256, NG = KP * 32 / 256;       // consecutive threads take consecutive locations of one row
+        int32_t at[NX];
+        float gv[NG];
+#pragma unroll
+        for (int i = 0; i < NX; ++i) {
+            const int e = threadIdx.x + i * 256, k = e % KP, row = e / KP;
+            at[i] = row < ROWS && p0 + k < pe ? (int32_t) resolve_row(__ldg(nbr + (ll) (row / CIN) * N + p0 + k), N, N + T) : (int32_t) (N + T);
         }
-        for (int e = threadIdx.x; e < KP * 32; e += 256) {
-            const int k = e % KP, co = e / KP;
-            gs[k][co >> 2].a[co & 3] = (p0 + k < pe && co0 + co < cout) ? gout[(ll) (co0 + co) * ld_out + p0 + k] : 0.f;
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            const int e = threadIdx.x + i * 256, k = e % KP, co = e / KP;
+            gv[i] = (p0 + k < pe && co0 + co < cout) ? gout[(ll) (co0 + co) * ld_out + p0 + k] : 0.f;
         }
+#pragma unroll
+        for (int i = 0; i < NX; ++i) {
+            const int e = threadIdx.x + i * 256, k = e % KP, row = e / KP;
+            if (row < RQ * 4) xs[k][row >> 2].a[row & 3] = __ldg(vals + (ll) (row % CIN) * R + at[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < NG; ++i) { const int e = threadIdx.x + i * 256, k = e % KP, co = e / KP; gs[k][co >> 2].a[co & 3] = gv[i]; }
         __syncthreads();
 #pragma unroll 4
         for (int k = grp * (KP / 4); k < (grp + 1) * (KP / 4); ++k) {
@@ -173,16 +185,8 @@ __global__ void __launch_bounds__(256) conv333_small_dw_kernel(ll seg_begin, ll 
     float* dst = partial + (ll) blockIdx.x * cout * CIN * 27;
     for (int e = threadIdx.x; e < ROWS * 32; e += 256) {
         const int row = e >> 5, co = co0 + (e & 31);
-        if (co < cout) dst[((ll) co * CIN + row % CIN) * 27 + row / CIN] = red[e];
+        if (co < cout) dst[((ll) (row / CIN) * CIN + row % CIN) * cout + co] = red[e];
     }
-}
-
-__global__ void small_reduce_partial_kernel(const float* __restrict__ partial, int nchunks, ll elems, float* __restrict__ dst) {
-    const ll e = (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= elems) return;
-    float s = 0;
-    for (int c = 0; c < nchunks; ++c) s += partial[(ll) c * elems + e];
-    dst[e] += s;
 }
 
 } // namespace
@@ -217,33 +221,46 @@ int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, co
     return APRNET_OK;
 }
 
-// grad_weights (slots, Cout, Cin, 27) is accumulated into; partial: aprnet_conv333_tc_dw_partial_elems() floats
+// partial: aprnet_conv333_tc_dw_partial_elems() floats
 int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* gout, ll ld_out,
-                                  float* gw, float* partial, cudaStream_t st) {
+                                  float* gw, int accumulate, float* partial, cudaStream_t st) {
     const AprPlan* plan = aprnet_get_plan(a, dl, st);
     if (!plan) return APRNET_ERR_CUDA;
-    const ll elems = (ll) 27 * cin * cout;
-    const ll max_ranges = aprnet_conv333_tc_dw_partial_elems(cin, cout) / elems;
+    const ll max_ranges = aprnet_conv333_tc_dw_partial_elems(cin, cout) / ((ll) 27 * cin * cout);
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_small_dw:ci%d:co%d:dl%d", cin, cout, dl);
-    for (const Segment& s : aprnet_segments(a, dl, slots, false)) {
-        const ll len = s.end - s.begin;
-        const int nranges = (int) std::max<ll>(1, std::min<ll>(std::min<ll>(max_ranges, 1184), (len + 511) / 512));
-        const ll range_len = ((len + nranges - 1) / nranges + 63) / 64 * 64;
+    const std::vector<Segment> segs = aprnet_segments(a, dl, slots, false);
+    SmallRanges rg;
+    SlotRanges sr;
+    rg.n = (int) segs.size();
+    sr.n = 0;
+    ll total = 0;
+    for (const Segment& s : segs) total += s.end - s.begin;
+    // at least 512 locations per block, at most eight blocks per SM or what the partial buffer holds
+    const ll budget = std::max<ll>(rg.n, std::min<ll>(max_ranges, 1184) - rg.n);
+    ll len = std::max<ll>(512, (total + budget - 1) / budget + 63) / 64 * 64;
+    auto blocks = [&]() { ll b = 0; for (const Segment& s : segs) b += (s.end - s.begin + len - 1) / len; return b; };
+    while (blocks() > std::max<ll>(max_ranges, rg.n)) len *= 2;
+    rg.first[0] = 0;
+    for (int i = 0; i < rg.n; ++i) {
+        rg.begin[i] = segs[i].begin; rg.end[i] = segs[i].end; rg.len[i] = len;
+        rg.first[i + 1] = rg.first[i] + aprnet_ceil_div(segs[i].end - segs[i].begin, len);
+        if (sr.n == 0 || sr.slot[sr.n - 1] != segs[i].slot) { sr.first[sr.n] = rg.first[i]; sr.slot[sr.n++] = segs[i].slot; }
+        sr.first[sr.n] = rg.first[i + 1];
+    }
+    const int nranges = rg.n ? rg.first[rg.n] : 0;
+    if (nranges > max_ranges) { aprnet_set_error("first-layer weight gradient: %d ranges exceed the partial buffer", nranges); return APRNET_ERR_ARG; }
+    if (nranges > 0) {
         dim3 grid((unsigned) nranges, (unsigned) aprnet_ceil_div(cout, 32));
-        { AprnetProfScope _prof(pname, st);
+        AprnetProfScope _prof(pname, st);
         switch (cin) {
-            case 1: conv333_small_dw_kernel<1><<<grid, 256, 0, st>>>(s.begin, s.end, range_len, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
-            case 2: conv333_small_dw_kernel<2><<<grid, 256, 0, st>>>(s.begin, s.end, range_len, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
-            case 3: conv333_small_dw_kernel<3><<<grid, 256, 0, st>>>(s.begin, s.end, range_len, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
-            case 4: conv333_small_dw_kernel<4><<<grid, 256, 0, st>>>(s.begin, s.end, range_len, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
+            case 1: conv333_small_dw_kernel<1><<<grid, 256, 0, st>>>(rg, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
+            case 2: conv333_small_dw_kernel<2><<<grid, 256, 0, st>>>(rg, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
+            case 3: conv333_small_dw_kernel<3><<<grid, 256, 0, st>>>(rg, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
+            case 4: conv333_small_dw_kernel<4><<<grid, 256, 0, st>>>(rg, plan->nbr, plan->n, plan->tree_size, vals, gout, ld_out, cout, partial); break;
             default: aprnet_set_error("small-Cin path called with cin = %d", cin); return APRNET_ERR_ARG;
         }
-        }
-        { AprnetProfScope _prof("conv333_dw_reduce", st);
-        small_reduce_partial_kernel<<<aprnet_ceil_div(elems, 256), 256, 0, st>>>(partial, nranges, elems, gw + (ll) s.slot * elems);
-        }
+        APRNET_LAUNCH_CHECK();
     }
-    APRNET_LAUNCH_CHECK();
-    return APRNET_OK;
+    return aprnet_dw_reduce(partial, sr, slots, accumulate, cin, cout, gw, st);
 }

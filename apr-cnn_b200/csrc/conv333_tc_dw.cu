@@ -303,12 +303,11 @@ extern "C" int64_t aprnet_conv333_tc_dw_partial_elems(int cin, int cout) {
 
 // xrows / grows: channels-last bf16 copies of the input (+ tree means + zero row) and of grad_output
 // (+ zero row) as produced by aprnet_pack_rows_bf16.  grad_weights (slots, Cout, Cin, 27) fp32 is
-// accumulated into.
-extern "C" int aprnet_conv333_backward_weights_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* xrows, int xpad,
-                                                  const void* grows, int gpad, float* gw, float* partial, void* stream) {
+// accumulated into or written.
+int aprnet_tc_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* xrows, int xpad, const void* grows, int gpad, float* gw, int accumulate,
+                               float* partial, cudaStream_t st) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && xrows && grows && gw && partial, "bad argument");
     APRNET_ARG_CHECK(xpad % 16 == 0 && gpad % 16 == 0 && xpad >= cin && gpad >= cout, "packed row widths must be multiples of 16");
-    cudaStream_t st = (cudaStream_t) stream;
     const RunPlan* rp = aprnet_get_run_plan(a, dl, st);
     if (!rp) return APRNET_ERR_CUDA;
     const ll n = a->number_parts(dl), t = a->tree_size(dl);
@@ -340,7 +339,7 @@ extern "C" int aprnet_conv333_backward_weights_tc(aprnet_apr* a, int dl, int cin
         total_chunks += (P.seg_end[P.n_segs] - P.seg_begin[P.n_segs] + PT - 1) / PT;
         ++P.n_segs;
     }
-    if (total_chunks == 0) return APRNET_OK;
+    if (total_chunks == 0) return accumulate ? APRNET_OK : aprnet_dw_reduce(partial, sr, slots, 0, cin, cout, gw, st);
     // two waves: a short level then costs a short block rather than an idle SM (1 to 4 waves measured within 5 % of each other)
     const int waves = g_dw_waves_override > 0 ? g_dw_waves_override : 2;
     ll budget = std::max<ll>(P.n_segs, ((ll) waves * sms + blocks_y - 1) / blocks_y);
@@ -372,5 +371,10 @@ extern "C" int aprnet_conv333_backward_weights_tc(aprnet_apr* a, int dl, int cin
     DW_CASE(128, 32) DW_CASE(128, 64) DW_CASE(128, 128)
     { aprnet_set_error("conv333 tensor-core weight gradient: unsupported blocking"); return APRNET_ERR_UNSUPPORTED; }
 #undef DW_CASE
-    return rc ? rc : aprnet_dw_reduce(partial, sr, cin, cout, gw, st);
+    return rc ? rc : aprnet_dw_reduce(partial, sr, slots, accumulate, cin, cout, gw, st);
+}
+
+extern "C" int aprnet_conv333_backward_weights_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* xrows, int xpad,
+                                                  const void* grows, int gpad, float* gw, float* partial, void* stream) {
+    return aprnet_tc_backward_weights(a, dl, cin, cout, slots, xrows, xpad, grows, gpad, gw, 1, partial, (cudaStream_t) stream);
 }

@@ -78,15 +78,35 @@ __global__ void gn_finalize_stats_kernel(const double* __restrict__ partial, int
     rstd[g] = (T) (1.0 / sqrt(var + eps));
 }
 
+// Sums of the first stage, ascending (the order of gn_finalize_stats_kernel / gn_backward_rows_kernel): short rows have so few chunks
+// that every block of the apply kernels adds them by itself and the kernels in between are not launched.
+constexpr int GN_FUSE = 32;             // chunks of a group at most
+__device__ __forceinline__ void sum_chunks(const double* __restrict__ partial, int count, double* buf, double& a, double& b) {
+    for (int i = threadIdx.x; i < 2 * count; i += GN_TPB) buf[i] = partial[i];
+    __syncthreads();
+    a = 0.0; b = 0.0;
+    for (int i = 0; i < count; ++i) { a += buf[2 * i]; b += buf[2 * i + 1]; }
+}
+
+// partial (null: mean / rstd are given): [row][nchunks][2] of the first stage; the first block of a group's first row stores its statistics
 // y = max((x - mean) * rstd * gamma + beta, 0)
 template<typename T>
 __global__ void __launch_bounds__(GN_TPB) gn_relu_apply_kernel(const T* __restrict__ x, ll n, int C, int ch_per_group, const T* __restrict__ gamma,
-                                                               const T* __restrict__ beta, const T* __restrict__ mean, const T* __restrict__ rstd,
-                                                               T* __restrict__ y, int relu) {
+                                                               const T* __restrict__ beta, T* mean, T* rstd, const double* __restrict__ partial,
+                                                               int nchunks, double eps, T* __restrict__ y, int relu) {
+    __shared__ double buf[2 * GN_FUSE];
     const ll row = blockIdx.y;                       // b * C + c
     const int c = (int) (row % C);
     const ll g = row / ch_per_group;                 // (b * C + c) / ch_per_group = b * G + c / ch_per_group
-    const T mu = mean[g], rs = rstd[g];
+    T mu, rs;
+    if (partial) {
+        double s, ss;
+        sum_chunks(partial + g * ch_per_group * nchunks * 2, ch_per_group * nchunks, buf, s, ss);
+        const double m = (double) ch_per_group * (double) n;
+        const double mud = s / m, var = fmax(ss / m - mud * mud, 0.0);
+        mu = (T) mud; rs = (T) (1.0 / sqrt(var + eps));
+        if (blockIdx.x == 0 && threadIdx.x == 0 && row % ch_per_group == 0) { mean[g] = mu; rstd[g] = rs; }
+    } else { mu = mean[g]; rs = rstd[g]; }
     const T ga = gamma ? gamma[c] : T(1), be = beta ? beta[c] : T(0);
     const T* xr = x + row * n;
     T* yr = y + row * n;
@@ -163,16 +183,37 @@ __global__ void gn_backward_finalize_kernel(const double* __restrict__ row_sums,
     }
 }
 
-// backward stage 3: dx = rstd * (dy_eff * gamma - mA - xhat * mB)
+// backward stage 3: dx = rstd * (dy_eff * gamma - mA - xhat * mB).  partial (null: group_terms are given): sums of stage 1 of ONE batch item;
+// every block adds those of its group as stages 2a and 2b do, the first block of a row stores its dgamma and dbeta
 template<typename T>
 __global__ void __launch_bounds__(GN_TPB) gn_backward_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, ll n, int C, int ch_per_group,
                                                                    const T* __restrict__ gamma, const T* __restrict__ beta, const T* __restrict__ mean,
-                                                                   const T* __restrict__ rstd, const T* __restrict__ group_terms, T* __restrict__ dx, int relu) {
+                                                                   const T* __restrict__ rstd, const T* __restrict__ group_terms, const double* __restrict__ partial,
+                                                                   int nchunks, T* __restrict__ dgamma, T* __restrict__ dbeta, T* __restrict__ dx, int relu) {
+    __shared__ double buf[2 * GN_FUSE];
     const ll row = blockIdx.y;
     const int c = (int) (row % C);
     const ll g = row / ch_per_group;
-    const T mu = mean[g], rs = rstd[g], mA = group_terms[2 * g], mB = group_terms[2 * g + 1];
+    const T mu = mean[g], rs = rstd[g];
     const T ga = gamma ? gamma[c] : T(1), be = beta ? beta[c] : T(0);
+    T mA, mB;
+    if (partial) {
+        const int count = ch_per_group * nchunks;
+        const double* p = partial + g * count * 2;
+        for (int i = threadIdx.x; i < 2 * count; i += GN_TPB) buf[i] = p[i];
+        __syncthreads();
+        double a = 0.0, b = 0.0;
+        for (int k = 0; k < ch_per_group; ++k) {
+            double ra = 0.0, rb = 0.0;
+            for (int i = k * nchunks; i < (k + 1) * nchunks; ++i) { ra += buf[2 * i]; rb += buf[2 * i + 1]; }
+            const int ck = (int) (g * ch_per_group) + k;
+            const double gk = gamma ? (double) gamma[ck] : 1.0;
+            a += gk * ra; b += gk * rb;
+            if (ck == c && blockIdx.x == 0 && threadIdx.x == 0) { if (dbeta) dbeta[c] = (T) ra; if (dgamma) dgamma[c] = (T) rb; }
+        }
+        const double m = (double) ch_per_group * (double) n;
+        mA = (T) (a / m); mB = (T) (b / m);
+    } else { mA = group_terms[2 * g]; mB = group_terms[2 * g + 1]; }
     const T* xr = x + row * n;
     const T* dr = dy + row * n;
     T* o = dx + row * n;
@@ -196,13 +237,14 @@ int gn_forward(int B, int C, ll n, int groups, const T* x, const T* gamma, const
     const int cpg = C / groups;
     const int nchunks = gn_chunks(n, rows);
     const ll chunk_len = (n + nchunks - 1) / nchunks;
+    const bool fused = cpg * nchunks <= GN_FUSE;
     { AprnetProfScope _p("groupnorm_stats", st);
     gn_partial_stats_kernel<T><<<dim3(nchunks, (unsigned) rows), GN_TPB, 0, st>>>(x, n, chunk_len, ws, nchunks);
-    gn_finalize_stats_kernel<T><<<aprnet_ceil_div((ll) B * groups, 128), 128, 0, st>>>(ws, nchunks, cpg, n, B * groups, eps, mean, rstd);
+    if (!fused) gn_finalize_stats_kernel<T><<<aprnet_ceil_div((ll) B * groups, 128), 128, 0, st>>>(ws, nchunks, cpg, n, B * groups, eps, mean, rstd);
     }
     const int gx = (int) std::max<ll>(1, std::min<ll>((n + GN_TPB * 8 - 1) / (GN_TPB * 8), 4096));
     { AprnetProfScope _p("groupnorm_relu_apply", st);
-    gn_relu_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, n, C, cpg, gamma, beta, mean, rstd, y, relu);
+    gn_relu_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, n, C, cpg, gamma, beta, mean, rstd, fused ? ws : nullptr, nchunks, eps, y, relu);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -217,14 +259,15 @@ int gn_backward(int B, int C, ll n, int groups, const T* x, const T* dy, const T
     const ll chunk_len = (n + nchunks - 1) / nchunks;
     double* row_sums = ws + rows * nchunks * 2;
     T* group_terms = reinterpret_cast<T*>(row_sums + rows * 2);
+    const bool fused = B == 1 && cpg * nchunks <= GN_FUSE;
     { AprnetProfScope _p("groupnorm_bwd_reduce", st);
     gn_backward_partial_kernel<T><<<dim3(nchunks, (unsigned) rows), GN_TPB, 0, st>>>(x, dy, n, chunk_len, C, cpg, gamma, beta, mean, rstd, ws, nchunks, relu);
-    gn_backward_rows_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(ws, nchunks, rows, row_sums);
-    gn_backward_finalize_kernel<T><<<aprnet_ceil_div(std::max<ll>(C, (ll) B * groups), 128), 128, 0, st>>>(row_sums, B, C, cpg, n, gamma, dgamma, dbeta, group_terms);
+    if (!fused) gn_backward_rows_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(ws, nchunks, rows, row_sums);
+    if (!fused) gn_backward_finalize_kernel<T><<<aprnet_ceil_div(std::max<ll>(C, (ll) B * groups), 128), 128, 0, st>>>(row_sums, B, C, cpg, n, gamma, dgamma, dbeta, group_terms);
     }
     const int gx = (int) std::max<ll>(1, std::min<ll>((n + GN_TPB * 8 - 1) / (GN_TPB * 8), 4096));
     { AprnetProfScope _p("groupnorm_bwd_apply", st);
-    gn_backward_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, dy, n, C, cpg, gamma, beta, mean, rstd, group_terms, dx, relu);
+    gn_backward_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, dy, n, C, cpg, gamma, beta, mean, rstd, group_terms, fused ? ws : nullptr, nchunks, dgamma, dbeta, dx, relu);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -280,7 +323,7 @@ static int gn_apply(int B, int C, ll n, int groups, const T* x, const T* gamma, 
     const ll rows = (ll) B * C;
     const int gx = (int) std::max<ll>(1, std::min<ll>((n + GN_TPB * 8 - 1) / (GN_TPB * 8), 4096));
     { AprnetProfScope _p("groupnorm_relu_apply", st);
-    gn_relu_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, n, C, C / groups, gamma, beta, mean, rstd, y, relu);
+    gn_relu_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, n, C, C / groups, gamma, beta, const_cast<T*>(mean), const_cast<T*>(rstd), nullptr, 0, 0.0, y, relu);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -306,7 +349,7 @@ static int gn_bwd_apply(int B, int C, ll n, int groups, const T* x, const T* dy,
     const ll rows = (ll) B * C;
     const int gx = (int) std::max<ll>(1, std::min<ll>((n + GN_TPB * 8 - 1) / (GN_TPB * 8), 4096));
     { AprnetProfScope _p("groupnorm_bwd_apply", st);
-    gn_backward_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, dy, n, C, C / groups, gamma, beta, mean, rstd, group_terms, dx, relu);
+    gn_backward_apply_kernel<T><<<dim3(gx, (unsigned) rows), GN_TPB, 0, st>>>(x, dy, n, C, C / groups, gamma, beta, mean, rstd, group_terms, nullptr, 0, nullptr, nullptr, dx, relu);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;

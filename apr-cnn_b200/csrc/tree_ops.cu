@@ -70,17 +70,30 @@ __global__ void __launch_bounds__(TPB) tree_level_kernel(const int32_t* __restri
     if (t < te) tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, use_up);
 }
 
-// The coarse end of the tree in one launch: a block owns CH channels and walks the levels [0, n) of `lv` (fine to coarse), whose
-// nodes are few; what it reads of a finer level it has written itself before the barrier.
+// The coarse end of the tree in one launch: a cluster of blocks owns CH channels and walks the levels [0, n) of `lv` (fine to
+// coarse).  A level reads what the cluster has written for the finer ones: the cluster barrier orders the blocks' global writes.  It
+// costs about 2 us, so levels of at most ALONE_NODES nodes are left to the cluster's first block, between barriers of its own.
 struct LevelList { int n; ll begin[APRNET_MAX_LEVELS], end[APRNET_MAX_LEVELS]; int use_up[APRNET_MAX_LEVELS]; };
-constexpr int COARSE_TPB = 512;
+constexpr int COARSE_TPB = 512, CLUSTER = 8;
+constexpr ll ALONE_NODES = 1024;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
 
 template<typename T, int CH, bool MAX>
-__global__ void __launch_bounds__(COARSE_TPB) tree_coarse_kernel(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree,
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(COARSE_TPB) tree_coarse_kernel(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree,
                                                                  LevelList lv, const T* __restrict__ in, ll ld_in, T* tree, ll ld_tree, int C, ll up_off) {
-    const int c0 = blockIdx.x * CH;
-    for (int i = 0; i < lv.n; ++i) {
-        for (ll t = lv.begin[i] + threadIdx.x; t < lv.end[i]; t += COARSE_TPB)
+    const int c0 = (int) (blockIdx.x / CLUSTER) * CH, first = (int) (blockIdx.x % CLUSTER) * COARSE_TPB + threadIdx.x;
+    int i = 0;
+    for (; i < lv.n && lv.end[i] - lv.begin[i] > ALONE_NODES; ++i) {
+        for (ll t = lv.begin[i] + first; t < lv.end[i]; t += CLUSTER * COARSE_TPB)
+            tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
+        cluster_barrier();
+    }
+    if (first >= COARSE_TPB) return;
+    for (; i < lv.n; ++i) {
+        for (ll t = lv.begin[i] + first; t < lv.end[i]; t += COARSE_TPB)
             tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
         __syncthreads();
     }
@@ -116,14 +129,23 @@ __global__ void __launch_bounds__(TPB) tree_mean_backward_children_kernel(const 
     if (u < ue) tree_backward_child<T>(parent, scale, u, dst, ld_dst, gtree, ld_tree, blockIdx.y * CH_PER_BLOCK, C);
 }
 
-// the coarse tree levels of `lv` (coarse to fine) in one launch, a block per channel group (see tree_coarse_kernel)
+// the coarse tree levels of `lv` (coarse to fine) in one launch, a cluster per channel group (see tree_coarse_kernel)
 template<typename T>
-__global__ void __launch_bounds__(COARSE_TPB) tree_mean_backward_coarse_kernel(const int32_t* __restrict__ parent, const float* __restrict__ scale,
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(COARSE_TPB) tree_mean_backward_coarse_kernel(const int32_t* __restrict__ parent, const float* __restrict__ scale,
                                                                                LevelList lv, T* gtree, ll ld_tree, int C) {
-    for (int i = 0; i < lv.n; ++i) {
-        for (ll u = lv.begin[i] + threadIdx.x; u < lv.end[i]; u += COARSE_TPB)
-            tree_backward_child<T>(parent, scale, u, gtree, ld_tree, gtree, ld_tree, blockIdx.x * CH_PER_BLOCK, C);
-        __syncthreads();
+    const int c0 = (int) (blockIdx.x / CLUSTER) * CH_PER_BLOCK, first = (int) (blockIdx.x % CLUSTER) * COARSE_TPB + threadIdx.x;
+    int i = 0;
+    for (; i < lv.n && lv.end[i] - lv.begin[i] <= ALONE_NODES; ++i) {
+        if (first < COARSE_TPB) {
+            for (ll u = lv.begin[i] + first; u < lv.end[i]; u += COARSE_TPB)
+                tree_backward_child<T>(parent, scale, u, gtree, ld_tree, gtree, ld_tree, c0, C);
+            __syncthreads();
+        }
+    }
+    for (; i < lv.n; ++i) {
+        cluster_barrier();
+        for (ll u = lv.begin[i] + first; u < lv.end[i]; u += CLUSTER * COARSE_TPB)
+            tree_backward_child<T>(parent, scale, u, gtree, ld_tree, gtree, ld_tree, c0, C);
     }
 }
 
@@ -216,9 +238,9 @@ int copy_rows(T* dst, ll ld_dst, const T* src, ll ld_src, ll count, int C, cudaS
 }
 
 // Fills the tree bottom-up.  A level of more than COARSE_NODES nodes is a launch of its own; the levels above the first one
-// with fewer (the coarser, the fewer) share one launch: a level costs about 2 us as a launch and about 1.5 us plus 1 us per
-// COARSE_TPB nodes inside the shared one.
-constexpr ll COARSE_NODES = 1024;
+// with fewer (the coarser, the fewer) share one launch: a launch costs the host 4 us, which is what small structures wait for, and
+// the device about 2 us; inside the shared one a level costs about 2 us per CLUSTER * COARSE_TPB nodes.
+constexpr ll COARSE_NODES = 2 * CLUSTER * COARSE_TPB;
 
 template<typename T, bool MAX>
 int fill_tree(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree, ll ld_tree, const char* pname, cudaStream_t st) {
@@ -247,7 +269,7 @@ int fill_tree(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree
     }
     if (coarse.n > 0) {
         AprnetProfScope _prof(pname, st);
-        tree_coarse_kernel<T, CH, MAX><<<gx, COARSE_TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, coarse, in, ld_in, tree, ld_tree, C, up);
+        tree_coarse_kernel<T, CH, MAX><<<gx * CLUSTER, COARSE_TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, coarse, in, ld_in, tree, ld_tree, C, up);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -268,7 +290,7 @@ int fill_tree_mean_bwd(const aprnet_apr* a, int dl, int C, T* gin, ll ld_in, T* 
         if (m.tlvl_begin[l + 1] > m.tlvl_begin[l]) { coarse.begin[coarse.n] = m.tlvl_begin[l]; coarse.end[coarse.n] = m.tlvl_begin[l + 1]; ++coarse.n; }
     if (coarse.n > 0) {
         AprnetProfScope _prof("tree_mean_bwd", st);
-        tree_mean_backward_coarse_kernel<T><<<(unsigned) aprnet_ceil_div(C, CH_PER_BLOCK), COARSE_TPB, 0, st>>>(node_parent, a->tree_scale, coarse, gtree, ld_tree, C);
+        tree_mean_backward_coarse_kernel<T><<<(unsigned) aprnet_ceil_div(C, CH_PER_BLOCK) * CLUSTER, COARSE_TPB, 0, st>>>(node_parent, a->tree_scale, coarse, gtree, ld_tree, C);
     }
     for (; l <= cml - 1; ++l) {
         const ll ub = m.tlvl_begin[l], ue = m.tlvl_begin[l + 1];

@@ -167,16 +167,16 @@ int aprnet_conv333_rows_forward(aprnet_apr* apr, int level_delta, int precision,
                                 void* workspace, void* stream);
 int aprnet_conv333_rows_pack(aprnet_apr* apr, int level_delta, int precision, int cin, const float* input, int64_t ld_in,
                              float* tree, int64_t ld_tree, int tree_is_valid, void* packed_rows, void* stream);
-/* grad_input (Cin, ld_in) is written (NULL: not computed); grad_weights (num_slots, Cout, Cin, 27) is accumulated into
- * (NULL: not computed; deterministic); grad_tree (Cin, ld_tree) is zero-filled, receives the gradient of the tree means and, with
+/* grad_input (Cin, ld_in) is written (NULL: not computed); grad_weights (num_slots, Cout, Cin, 27) is written or, with
+ * accumulate, added to (NULL: not computed; deterministic); grad_tree (Cin, ld_tree) is zero-filled, receives the gradient of the tree means and, with
  * fold_tree, is folded into grad_input.  partial: aprnet_conv333_rows_partial_elems() floats. */
 int64_t aprnet_conv333_rows_backward_workspace_bytes(const aprnet_apr* apr, int level_delta, int precision, int cin, int cout, int num_slots,
                                                      int with_grad_input);
 int64_t aprnet_conv333_rows_partial_elems(int precision, int cin, int cout);
 int aprnet_conv333_rows_backward(aprnet_apr* apr, int level_delta, int precision, int cin, int cout, int num_slots,
                                  const void* packed_rows, const float* grad_output, int64_t ld_out, const float* weights,
-                                 float* grad_input, int64_t ld_in, float* grad_weights, float* grad_tree, int64_t ld_tree,
-                                 int fold_tree, float* partial, void* workspace, void* stream);
+                                 float* grad_input, int64_t ld_in, float* grad_weights, int accumulate, float* grad_tree,
+                                 int64_t ld_tree, int fold_tree, float* partial, void* workspace, void* stream);
 
 /* ---- 3x3x3 convolution on the tensor cores (bf16 operands, fp32 accumulation) ------------------
  * No counterpart in the reference (its kernels are CUDA-core only).  Same contract as
