@@ -39,15 +39,15 @@ struct AprPlan {                 // cached per level_delta
 
 // Cross-level edges of one level_delta: every (output location p, tap) whose source ("target" of the
 // gradient) is a coarser particle or a tree node.  Targets are numbered as particle index, or
-// N + tree index.  The edges of one (target, tap) form a "virtual row": their dO rows are summed before
-// the contraction, because they all meet the same weight matrix.  Virtual rows are numbered by
-// ascending target, then tap; vsrc[vstart[v] .. vstart[v + 1]) lists the locations p of row v in
-// ascending order.  active[] lists the targets that have at least one edge (ascending), vnbr[tap][a] is
-// the virtual row of (active[a], tap) or -1.
+// N + tree index.  The edges of one (target, tap) meet the same weight matrix: where there are several, their dO rows are summed
+// before the contraction into a "virtual row"; a single one (every tap of a tree node, most of a particle's) is that location's row
+// itself.  Virtual rows are numbered by ascending target, then tap; vsrc[vstart[v] .. vstart[v + 1]) lists the locations p of row v in
+// ascending order.  active[] lists the targets that have at least one edge (ascending), vnbr[tap][a] is the virtual row of
+// (active[a], tap), the location encoded like a tree node (<= -2), or -1.
 struct ActiveSeg { long long begin, end; int location_level; };     // range of active[] whose edges come from one level
 struct EdgePlan {
     long long n_edges = 0, n_targets = 0, n_active = 0, n_vrows = 0;
-    int32_t* vsrc = nullptr;       // [n_edges]
+    int32_t* vsrc = nullptr;       // [locations of all virtual rows]
     int32_t* vstart = nullptr;     // [n_vrows + 1]
     int32_t* active = nullptr;     // [n_active]
     int32_t* vnbr = nullptr;       // [27][n_active]
@@ -156,9 +156,9 @@ extern "C" int aprnet_conv333_backward_input_cross_level(aprnet_apr* a, int dl, 
 const RunPlan* aprnet_get_run_plan(aprnet_apr* apr, int dl, cudaStream_t stream);                // nullptr on failure
 EdgePlan* aprnet_get_edge_plan(aprnet_apr* apr, int dl, cudaStream_t stream);
 void aprnet_free_edge_plan(EdgePlan& ep, cudaStream_t st);
-// gather GEMM over the active targets [a0, a1) of an edge plan: grad[target] += sum over taps of
-// W[slot][:, :, tap]^T times virtual row vnbr[tap][a] (rows: bf16 [.. ][gpad], row index relative to `vrows`)
-int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* vrows, int gpad, long long zero_row,
+// gather GEMM over the active targets [a0, a1) of an edge plan: grad[target] += sum over taps of W[slot][:, :, tap]^T times the row
+// of vnbr[tap][a]; rows are addressed from grows: location p at row p (zeros at row n_split = N), virtual row v at row v + v_shift
+int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* grows, int gpad, long long v_shift,
                              const void* wp_packed, const EdgePlan* ep, long long a0, long long a1,
                              float* gin, long long ld_in, float* gtree, long long ld_tree, cudaStream_t st);
 // CUDA-core fp32 kernels for Cin <= 4 (conv333_small.cu), used in either arithmetic for such layers:

@@ -217,11 +217,11 @@ __global__ void __launch_bounds__(TPB) conv333_cross_pull_kernel(const int32_t* 
         const int ob = min(OB, cout - o0);
         for (int tap = 0; tap < 27; ++tap) {
             const int32_t v = vnbr[(ll) tap * n_active + a];
-            if (v < 0) continue;
+            if (v == APRNET_NONE) continue;
             const T* wt = wsm + tap * OB * IB;
-            const int e1 = vstart[v + 1];
-            for (int e = vstart[v]; e < e1; ++e) {
-                const T* g = gout + (ll) o0 * ld_out + vsrc[e];
+            const int e0 = v >= 0 ? vstart[v] : 0, e1 = v >= 0 ? vstart[v + 1] : 1;
+            for (int e = e0; e < e1; ++e) {
+                const T* g = gout + (ll) o0 * ld_out + (v >= 0 ? (ll) vsrc[e] : aprnet_dec_tree(v));
                 for (int o = 0; o < ob; ++o) {
                     const T d = g[(ll) o * ld_out];
 #pragma unroll

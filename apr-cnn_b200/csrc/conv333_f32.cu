@@ -120,6 +120,7 @@ struct F32Params {
     // out[:, t] for t < out_split and to out2[:, t - out_split] otherwise
     const int32_t* out_map; ll out_split;
     float* out2; ll ld_out2;
+    ll v_shift;                            // added to table entries >= 0 (virtual rows)
 };
 
 // Block = 128 * WM locations x NT = TN * WN output channels, WM x WN warps; a thread owns the locations lane + 32 i (i < 4) of its
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
             const int32_t v = raw[i];
             ll r = P.zero_row;
             if (P.same_level_only) { if (v >= lo && v < hi) r = v; }
-            else if (v >= 0) r = v;
+            else if (v >= 0) r = v + P.v_shift;
             else if (v != APRNET_NONE) r = P.tree_base + aprnet_dec_tree(v);
             src[i] = (int32_t) r;
         }
@@ -280,8 +281,8 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
     }
 }
 
-// per-(target, tap) sums of dO rows: virtual row v of [v0, v1) -> row 1 + v - v0 (row 0 is the zero row).  A thread owns one
-// row and four channels and requests up to four locations before it adds them in ascending order (runs are 1 to 4 long).
+// per-(target, tap) sums of dO rows: virtual row v of [v0, v1) -> row v - v0.  A thread owns one
+// row and four channels and requests up to four locations before it adds them in ascending order (runs are 2 to 4 long).
 __global__ void __launch_bounds__(256) vrow_reduce_f32_kernel(const int32_t* __restrict__ vstart, const int32_t* __restrict__ vsrc, ll v0, ll v1,
                                                               const float* __restrict__ grows, int gpad, float* __restrict__ out) {
     const int nch = gpad >> 2;
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(256) vrow_reduce_f32_kernel(const int32_t* __r
 #pragma unroll
         for (int k = 0; k < 4; ++k) { acc.x += q[k].x; acc.y += q[k].y; acc.z += q[k].z; acc.w += q[k].w; }
     }
-    *reinterpret_cast<float4*>(out + (1 + v - v0) * gpad + c) = acc;
+    *reinterpret_cast<float4*>(out + (v - v0) * gpad + c) = acc;
 }
 
 // ---- weight gradient ----------------------------------------------------------------------------------
@@ -619,8 +620,9 @@ int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* 
     if (ep->n_active == 0) return APRNET_OK;
     const int gpad = pad4(cout), cml = a->cml(dl);
     int rc = APRNET_OK;
-    APRNET_CUDA_CHECK(cudaMemsetAsync(vrows, 0, (size_t) gpad * sizeof(float), st));          // row 0: zeros
-    const ll cap_rows = vrow_bytes / ((ll) gpad * 4) - 1;
+    // virtual rows lie a whole number of rows behind the first dO row, so that the gather addresses both from there
+    const ll row = (ll) gpad * 4, off = ((char*) vrows - (char*) grows + row - 1) / row, cap_rows = ((char*) vrows + vrow_bytes - (char*) grows) / row - off;
+    vrows = const_cast<float*>(grows) + off * gpad;
     const int nk = (int) ep->chunk_a.size() - 1;
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_bwd_cross_pull:ci%d:co%d:dl%d", cin, cout, dl);
@@ -629,8 +631,7 @@ int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* 
         while (k1 < nk && ep->chunk_v[k1 + 1] - ep->chunk_v[k0] <= cap_rows) ++k1;
         const ll v0 = ep->chunk_v[k0], v1 = ep->chunk_v[k1], a0 = ep->chunk_a[k0], a1 = ep->chunk_a[k1];
         if (v1 - v0 > cap_rows) { aprnet_set_error("edge workspace too small for %lld virtual rows", v1 - v0); return APRNET_ERR_ARG; }
-        if (v1 == v0) continue;
-        {
+        if (v1 > v0) {
             AprnetProfScope _prof("edge_reduce", st);
             vrow_reduce_f32_kernel<<<aprnet_ceil_div((v1 - v0) * (gpad / 4), 256), 256, 0, st>>>(ep->vstart, ep->vsrc, v0, v1, grows, gpad, vrows);
         }
@@ -644,8 +645,7 @@ int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* 
         if (segs.empty()) continue;
         F32Params P;
         memset(&P, 0, sizeof(P));
-        // row of the gather = virtual row; the zero row is addressed as v0 - 1
-        P.nbr = ep->vnbr; P.N = ep->n_active; P.rows = vrows + (1 - v0) * gpad; P.kpad = gpad; P.zero_row = v0 - 1; P.tree_base = v0 - 1;
+        P.nbr = ep->vnbr; P.N = ep->n_active; P.rows = grows; P.kpad = gpad; P.zero_row = a->number_parts(dl); P.tree_base = 0; P.v_shift = off - v0;
         P.wp = wp; P.n_dim = cin;
         P.out = gin; P.ld_out = ld_in; P.out_map = ep->active; P.out_split = a->number_parts(dl); P.out2 = gtree; P.ld_out2 = ld_tree;
         if ((rc = run_gather<false>(P, segs, st, pname))) return rc;

@@ -114,6 +114,7 @@ struct TcParams {
     // added to out[:, t] for t < out_split and to out2[:, t - out_split] otherwise
     const int32_t* out_map; ll out_split;
     float* out2; ll ld_out2;
+    ll v_shift;                            // added to table entries >= 0 (virtual rows)
 };
 
 // ---- warp-specialised gather kernel ---------------------------------------------------------------
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
             for (int tap = 0; tap < 27; ++tap) {
                 ll r = P.zero_row;
                 if (P.same_level_only) { if (v[tap] >= ti.lo && v[tap] < ti.hi) r = v[tap]; }
-                else if (v[tap] >= 0) r = v[tap];
+                else if (v[tap] >= 0) r = v[tap] + P.v_shift;
                 else if (v[tap] != APRNET_NONE) r = P.tree_base + aprnet_dec_tree(v[tap]);
                 dst[tap * TILE_M + row] = (int32_t) r;
             }
@@ -572,7 +573,7 @@ int launch_tc_ws(const TcParams& P, int total_tiles, cudaStream_t st, const char
 
 int dispatch_tc(const TcParams& P, const TcGeom& g, int total_tiles, cudaStream_t st, const char* pname) {
     int taps = 1, wps = 1, tt = 0;
-    // the rows of the cross-level pass are addressed from a shifted base with the zero row in front: no tensor map for them
+    // the rows of the cross-level pass lie in two areas, with the zero row between them: no tensor map for them
     pick_stage_shape(g.order_nt, g.ks, P.out_map == nullptr && g.nt == g.order_nt, &taps, &wps, &tt);
     if (g.nt != g.order_nt)          // a narrower tile in the order of the wide one: the same taps per stage
         for (int w = 4; w >= 1; w /= 2) if (tc_variant_ok(g.nt, g.ks, taps, w)) wps = w;
@@ -627,7 +628,7 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
     P.tree_base = tree_base; P.zero_row = zero_row;
     P.wp = wp; P.mirror = backward; P.out = out; P.ld_out = ld_out; P.bias = bias; P.n_dim = n_dim; P.n_tiles = g.n_tiles; P.same_level_only = backward;
     P.error_flag = g_error_flag_dev;
-    P.out_map = nullptr; P.out_split = 0; P.out2 = nullptr; P.ld_out2 = 0;
+    P.out_map = nullptr; P.out_split = 0; P.out2 = nullptr; P.ld_out2 = 0; P.v_shift = 0;
 
     const int total = P.segs.tile_begin[P.segs.n] * g.n_tiles;
     if (total == 0) return APRNET_OK;
@@ -640,7 +641,7 @@ int aprnet_tc_pack_weights(const aprnet_apr* a, int dl, const float* w, int slot
 }
 
 // Gather GEMM over the active targets [a0, a1) of an edge plan (transposed weights as packed by aprnet_tc_gather_conv).
-int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* vrows, int gpad, ll zero_row,
+int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* grows, int gpad, ll v_shift,
                              const void* wp_packed, const EdgePlan* ep, ll a0, ll a1,
                              float* gin, ll ld_in, float* gtree, ll ld_tree, cudaStream_t st) {
     int rc = ensure_error_flag();
@@ -661,7 +662,7 @@ int aprnet_tc_gather_targets(aprnet_apr* a, int dl, int cin, int cout, int slots
     memset(&P, 0, sizeof(P));
     P.segs = make_seg_table(segs, TILE_M);
     P.nbr = ep->vnbr; P.N = ep->n_active;
-    P.rows = reinterpret_cast<const __nv_bfloat16*>(vrows); P.kpad = g.kpad; P.zero_row = zero_row; P.tree_base = zero_row;
+    P.rows = reinterpret_cast<const __nv_bfloat16*>(grows); P.kpad = g.kpad; P.zero_row = a->number_parts(dl); P.tree_base = 0; P.v_shift = v_shift;
     P.wp = reinterpret_cast<const __nv_bfloat16*>(wp_packed); P.n_dim = cin; P.n_tiles = g.n_tiles;
     P.same_level_only = 0; P.error_flag = g_error_flag_dev;
     P.out = gin; P.ld_out = ld_in; P.out_map = ep->active; P.out_split = a->number_parts(dl); P.out2 = gtree; P.ld_out2 = ld_tree;

@@ -81,40 +81,47 @@ __global__ void edge_compact_active_kernel(const int32_t* __restrict__ pos, ll n
 
 struct TapBegin { int32_t b[28]; };      // first edge id of every tap (edge ids are tap-major)
 
-// virtual rows of one active target = runs of equal tap in its ascending edge list
+// virtual rows of one active target = runs of equal tap, of more than one edge, in its ascending edge list
+template<typename F>
+__device__ __forceinline__ void for_each_run(const int32_t* __restrict__ tgt_edge, int begin, int end, const TapBegin& tb, F f) {
+    int tap = 0;
+    for (int i = begin; i < end;) {
+        while (tgt_edge[i] >= tb.b[tap + 1]) ++tap;
+        int j = i + 1;
+        while (j < end && tgt_edge[j] < tb.b[tap + 1]) ++j;
+        f(tap, i, j);
+        i = j;
+    }
+}
+
 __global__ void vrow_count_kernel(const int32_t* __restrict__ active, ll n_active, const int32_t* __restrict__ ptr,
-                                  const int32_t* __restrict__ tgt_edge, TapBegin tb, int32_t* __restrict__ nruns) {
+                                  const int32_t* __restrict__ tgt_edge, TapBegin tb, int32_t* __restrict__ nruns, int32_t* __restrict__ nedges) {
     const ll a = (ll) blockIdx.x * blockDim.x + threadIdx.x;
     if (a > n_active) return;
-    int runs = 0;
+    int runs = 0, edges = 0;
     if (a < n_active) {
         const int t = active[a];
-        int cur = -1, tap = 0;
-        for (int i = ptr[t]; i < ptr[t + 1]; ++i) {
-            const int32_t e = tgt_edge[i];
-            while (e >= tb.b[tap + 1]) ++tap;
-            if (tap != cur) { ++runs; cur = tap; }
-        }
+        for_each_run(tgt_edge, ptr[t], ptr[t + 1], tb, [&](int, int i, int j) { if (j - i > 1) { ++runs; edges += j - i; } });
     }
     nruns[a] = runs;
+    nedges[a] = edges;
 }
 
 __global__ void vrow_fill_kernel(const int32_t* __restrict__ active, ll n_active, const int32_t* __restrict__ ptr,
                                  const int32_t* __restrict__ tgt_edge, const int32_t* __restrict__ src, TapBegin tb,
-                                 const int32_t* __restrict__ vfirst, ll n_edges, int32_t* __restrict__ vstart,
+                                 const int32_t* __restrict__ vfirst, const int32_t* __restrict__ efirst, int32_t* __restrict__ vstart,
                                  int32_t* __restrict__ vnbr, int32_t* __restrict__ vsrc) {
     const ll a = (ll) blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= n_active) return;
-    if (a == 0) vstart[vfirst[n_active]] = (int32_t) n_edges;
+    if (a == 0) vstart[vfirst[n_active]] = efirst[n_active];
     const int t = active[a];
-    int cur = -1, tap = 0;
-    int32_t v = vfirst[a] - 1;
-    for (int i = ptr[t]; i < ptr[t + 1]; ++i) {
-        const int32_t e = tgt_edge[i];
-        while (e >= tb.b[tap + 1]) ++tap;
-        if (tap != cur) { cur = tap; ++v; vstart[v] = i; vnbr[(ll) tap * n_active + a] = v; }
-        vsrc[i] = src[e];
-    }
+    int32_t v = vfirst[a], at = efirst[a];
+    for_each_run(tgt_edge, ptr[t], ptr[t + 1], tb, [&](int tap, int i, int j) {
+        if (j - i == 1) { vnbr[(ll) tap * n_active + a] = aprnet_enc_tree(src[tgt_edge[i]]); return; }
+        vstart[v] = at;
+        vnbr[(ll) tap * n_active + a] = v++;
+        for (; i < j; ++i) vsrc[at++] = src[tgt_edge[i]];
+    });
 }
 
 // out[k] = first index i of sorted[0, n) with sorted[i] >= key[k]
@@ -127,9 +134,9 @@ __global__ void lower_bound_kernel(const int32_t* __restrict__ sorted, ll n, con
 }
 
 // pass 1: thread = (VPT consecutive virtual rows, 8-channel chunk); sums the dO rows of each row's locations in
-// ascending order (fp32) and writes the bf16 row 1 + v - v0 of the workspace (row 0 is the zero row).  The three
+// ascending order (fp32) and writes the bf16 row v - v0 of the workspace.  The three
 // dependent accesses (row starts -> source locations -> dO rows) are each requested for all VPT rows and up to four
-// locations per row before any is used (runs are 1-4 locations long; longer ones continue in a loop).
+// locations per row before any is used (runs are 2-4 locations long; longer ones continue in a loop).
 constexpr int VROW_VPT = 2;          // measured: 2 rows per thread 20 % faster than 1, 4 slower (registers)
 
 template<int VPT>
@@ -170,7 +177,7 @@ __global__ void __launch_bounds__(256) vrow_reduce_kernel(const int32_t* __restr
         __nv_bfloat162 o[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) o[k] = __floats2bfloat162_rn(acc[2 * k], acc[2 * k + 1]);
-        *reinterpret_cast<uint4*>(out + (1 + vb + u - v0) * gpad + c * 8) = *reinterpret_cast<const uint4*>(o);
+        *reinterpret_cast<uint4*>(out + (vb + u - v0) * gpad + c * 8) = *reinterpret_cast<const uint4*>(o);
     }
 }
 
@@ -200,11 +207,11 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
     for (int i = 0; i < lr.n; ++i) { lr.begin[i] = segs[i].begin; lr.end[i] = segs[i].end; }
 
     // temporaries: flags / scan, per-edge source and target, per-target lists
-    int32_t *scan = nullptr, *src = nullptr, *tgt = nullptr, *count = nullptr, *tgt_ptr = nullptr, *tgt_edge = nullptr, *vfirst = nullptr;
+    int32_t *scan = nullptr, *src = nullptr, *tgt = nullptr, *count = nullptr, *tgt_ptr = nullptr, *tgt_edge = nullptr, *vfirst = nullptr, *efirst = nullptr;
     ll *keys = nullptr, *found = nullptr;
     void* temp = nullptr;
     int rc = APRNET_OK;
-    auto cleanup = [&]() { void* all[] = {scan, src, tgt, count, tgt_ptr, tgt_edge, vfirst, keys, found, temp}; for (void* p : all) aprnet_pool_free(p, st); };
+    auto cleanup = [&]() { void* all[] = {scan, src, tgt, count, tgt_ptr, tgt_edge, vfirst, efirst, keys, found, temp}; for (void* p : all) aprnet_pool_free(p, st); };
 #define EP_ALLOC(p, n) do { if ((rc = dev_alloc(&(p), (size_t) (n), nullptr, st))) { cleanup(); return rc; } } while (0)
 #define EP_CHECK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) { aprnet_set_error("%s failed: %s", #expr, cudaGetErrorString(_e)); cleanup(); return APRNET_ERR_CUDA; } } while (0)
 
@@ -249,17 +256,20 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
 
     // virtual rows: runs of equal tap in every active target's list
     EP_ALLOC(vfirst, n_active + 1);
-    vrow_count_kernel<<<aprnet_ceil_div((ll) n_active + 1, 128), 128, 0, st>>>(ep.active, n_active, tgt_ptr, tgt_edge, tb, vfirst);
+    EP_ALLOC(efirst, n_active + 1);
+    vrow_count_kernel<<<aprnet_ceil_div((ll) n_active + 1, 128), 128, 0, st>>>(ep.active, n_active, tgt_ptr, tgt_edge, tb, vfirst, efirst);
     EP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, vfirst, vfirst, n_active + 1, st));
-    int32_t n_vrows = 0;
+    EP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, efirst, efirst, n_active + 1, st));
+    int32_t n_vrows = 0, n_summed = 0;
     EP_CHECK(cudaMemcpyAsync(&n_vrows, vfirst + n_active, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    EP_CHECK(cudaMemcpyAsync(&n_summed, efirst + n_active, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     EP_CHECK(cudaStreamSynchronize(st));
     ep.n_vrows = n_vrows;
-    if ((rc = dev_alloc(&ep.vsrc, (size_t) E, &a->device_bytes, st)) || (rc = dev_alloc(&ep.vstart, (size_t) n_vrows + 1, &a->device_bytes, st)) ||
+    if ((rc = dev_alloc(&ep.vsrc, (size_t) n_summed, &a->device_bytes, st)) || (rc = dev_alloc(&ep.vstart, (size_t) n_vrows + 1, &a->device_bytes, st)) ||
         (rc = dev_alloc(&ep.vnbr, (size_t) 27 * std::max(n_active, 1), &a->device_bytes, st))) { cleanup(); return rc; }
     EP_CHECK(cudaMemsetAsync(ep.vnbr, 0xFF, (size_t) 27 * std::max(n_active, 1) * sizeof(int32_t), st));       // APRNET_NONE
     EP_CHECK(cudaMemsetAsync(ep.vstart, 0, ((size_t) n_vrows + 1) * sizeof(int32_t), st));
-    if (n_active) vrow_fill_kernel<<<aprnet_ceil_div(n_active, 128), 128, 0, st>>>(ep.active, n_active, tgt_ptr, tgt_edge, src, tb, vfirst, E,
+    if (n_active) vrow_fill_kernel<<<aprnet_ceil_div(n_active, 128), 128, 0, st>>>(ep.active, n_active, tgt_ptr, tgt_edge, src, tb, vfirst, efirst,
                                                                                   ep.vstart, ep.vnbr, ep.vsrc);
 
     // ranges of active[] by level of the locations their edges come from, and the chunk map
@@ -356,9 +366,18 @@ int aprnet_cross_level_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, c
     if (ts > 0) APRNET_CUDA_CHECK(cudaMemset2DAsync(gtree, (size_t) ld_tree * sizeof(float), 0, (size_t) ts * sizeof(float), (size_t) cin, st));
     if (ep->n_active > 0) {
         int rc = APRNET_OK;
-        __nv_bfloat16* vrows = reinterpret_cast<__nv_bfloat16*>(edge_ws);
-        APRNET_CUDA_CHECK(cudaMemsetAsync(vrows, 0, (size_t) gpad * 2, st));          // row 0: zeros
-        const ll cap_rows = edge_ws_bytes / ((ll) gpad * 2) - 1;
+        // virtual rows lie a whole number of rows behind the first dO row, so that the gather addresses both from there
+        const ll row = (ll) gpad * 2, n = a->number_parts(dl);
+        StreamScratch joint(st);
+        const char *g0 = (const char*) grows, *e0 = (const char*) edge_ws, *e1 = e0 + edge_ws_bytes;
+        if (e0 < g0 + (n + 1) * row || (e1 - g0) / row >= (1ll << 31) - 2) {      // separate buffers of a caller: one joint copy
+            const ll rows = (n + 1) * row;
+            if ((rc = joint.get((size_t) (rows + edge_ws_bytes)))) return rc;
+            APRNET_CUDA_CHECK(cudaMemcpyAsync(joint.p, grows, (size_t) rows, cudaMemcpyDeviceToDevice, st));
+            g0 = (const char*) joint.p; e0 = g0 + rows; e1 = e0 + edge_ws_bytes;
+        }
+        const ll off = (e0 - g0 + row - 1) / row, cap_rows = (e1 - g0) / row - off;
+        __nv_bfloat16* vrows = (__nv_bfloat16*) (g0 + off * row);
         const int nk = (int) ep->chunk_a.size() - 1;
         int k0 = 0;
         while (k0 < nk) {
@@ -367,16 +386,12 @@ int aprnet_cross_level_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, c
             const ll v0 = ep->chunk_v[k0], v1 = ep->chunk_v[k1], a0 = ep->chunk_a[k0], a1 = ep->chunk_a[k1];
             if (v1 - v0 > cap_rows) { aprnet_set_error("edge workspace too small for %lld virtual rows", v1 - v0); return APRNET_ERR_ARG; }
             if (v1 > v0) {
-                { AprnetProfScope _prof("edge_reduce", st);
+                AprnetProfScope _prof("edge_reduce", st);
                 vrow_reduce_kernel<VROW_VPT><<<aprnet_ceil_div(aprnet_ceil_div(v1 - v0, VROW_VPT) * (gpad / 8), 256), 256, 0, st>>>(
-                    ep->vstart, ep->vsrc, v0, v1, (const __nv_bfloat16*) grows, gpad, vrows);
-                }
+                    ep->vstart, ep->vsrc, v0, v1, (const __nv_bfloat16*) g0, gpad, vrows);
                 APRNET_LAUNCH_CHECK();
-                // row index r of the gather = virtual row id; the zero row is addressed as v0 - 1
-                rc = aprnet_tc_gather_targets(a, dl, cin, cout, slots, vrows + (1 - v0) * gpad, gpad, v0 - 1, wp_ws, ep, a0, a1,
-                                              gin, ld_in, gtree, ld_tree, st);
-                if (rc) return rc;
             }
+            if (a1 > a0 && (rc = aprnet_tc_gather_targets(a, dl, cin, cout, slots, g0, gpad, off - v0, wp_ws, ep, a0, a1, gin, ld_in, gtree, ld_tree, st))) return rc;
             k0 = k1;
         }
     }

@@ -22,15 +22,25 @@ __device__ __forceinline__ float restrict_overlap(int step, int fine_tap, int co
     return fmaxf(0.f, (float) (min((coarse_tap + 1) * step, off + fine_tap + step) - max(coarse_tap * step, off + fine_tap)));
 }
 
-// coef[to][ti]: share of fine tap ti in coarse tap to of slot k (all products and the power of two divide exactly)
+// coef[to][ti]: share of fine tap ti in coarse tap to of slot k (products of small integers times a power of two: exact)
 template<typename T>
 __device__ __forceinline__ void restrict_table(int S, int k, T (*coef)[CROW]) {
     const int step = 1 << (k - (S - 1));
-    const float factor = (float) step * (float) step * (float) step;
-    for (int e = threadIdx.x; e < 27 * 27; e += FB) {
-        const int to = e / 27, ti = e - to * 27;
-        coef[to][ti] = (T) (restrict_overlap(step, (ti / 3) % 3, (to / 3) % 3) * restrict_overlap(step, ti % 3, to % 3) *
-                            restrict_overlap(step, ti / 9, to / 9) / factor);
+    const float inv = 1.0f / ((float) step * (float) step * (float) step);
+    float ov[3][3];
+#pragma unroll
+    for (int t = 0; t < 9; ++t) ov[t / 3][t % 3] = restrict_overlap(step, t % 3, t / 3);      // [coarse][fine]
+    if (threadIdx.x < 27) {              // thread = coarse tap; its row of 27 products is unrolled
+        const int z = threadIdx.x / 9, x = (threadIdx.x / 3) % 3, y = threadIdx.x % 3;
+        float oz[3], ox[3], oy[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            oz[i] = z == 0 ? ov[0][i] : (z == 1 ? ov[1][i] : ov[2][i]);
+            ox[i] = x == 0 ? ov[0][i] : (x == 1 ? ov[1][i] : ov[2][i]);
+            oy[i] = y == 0 ? ov[0][i] : (y == 1 ? ov[1][i] : ov[2][i]);
+        }
+#pragma unroll
+        for (int t = 0; t < 27; ++t) coef[threadIdx.x][t] = (T) (ox[(t / 3) % 3] * oy[t % 3] * oz[t / 9] * inv);
     }
 }
 
@@ -90,13 +100,19 @@ __global__ void __launch_bounds__(FB) restrict333_backward_kernel(int S, int L, 
     T acc[27];
 #pragma unroll
     for (int t = 0; t < 27; ++t) acc[t] = stage[threadIdx.x * 27 + t];
+    T next[27];                          // the next slot's values, requested while this one's are used
+    auto request = [&](int k) {
+#pragma unroll
+        for (int i = 0; i < 27; ++i) { const int e = threadIdx.x + i * FB; next[i] = e < n ? src[((ll) k * filters + f0) * 27 + e] : T(0); }
+    };
+    if (S < L) request(S);
     for (int k = S; k < L; ++k) {
         __syncthreads();
-        const T* coarse = src + ((ll) k * filters + f0) * 27;
-#pragma unroll 9
-        for (int e = threadIdx.x; e < n; e += FB) stage[e] = coarse[e];
+#pragma unroll
+        for (int i = 0; i < 27; ++i) stage[threadIdx.x + i * FB] = next[i];
         restrict_table<T>(S, k, coef);
         __syncthreads();
+        if (k + 1 < L) request(k + 1);
 #pragma unroll 3
         for (int o = 0; o < 27; ++o) {
             const T c = stage[threadIdx.x * 27 + o];
