@@ -201,7 +201,7 @@ int aprnet_f32_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int sl
 int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* gout, long long ld_out, const float* w, float* gin, long long ld_in,
                               float* gtree, long long ld_tree, void* workspace, bool tree_adjoint, cudaStream_t st);
 
-// ranges of block partial sums [range][27][cin][cout] per stencil slot: slot[g] owns [first[g], first[g + 1]), g < n
+// ranges of block partial sums [range][27][cout][cin] per stencil slot: slot[g] owns [first[g], first[g + 1]), g < n
 struct SlotRanges { int n; int first[APRNET_MAX_LEVELS + 1]; int slot[APRNET_MAX_LEVELS]; unsigned empty; };      // empty: slots to zero (bit per slot)
 // grad_weights (slots, Cout, Cin, 27) += sums in a fixed order; without `accumulate` all of it is written (zeros in slots without ranges)
 int aprnet_dw_reduce(const float* partial, SlotRanges sr, int slots, int accumulate, int cin, int cout, float* gw, cudaStream_t st);

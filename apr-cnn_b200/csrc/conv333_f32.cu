@@ -318,7 +318,7 @@ struct F32DwParams {
     const int32_t* nbr; ll N;
     const float* xrows; int xpad; ll tree_base, zero_row;
     const float* grows; int gpad; ll g_zero_row;
-    float* partial;                        // [range][27][cin][cout]
+    float* partial;                        // [range][27][cout][cin]
     int cin, cout, ci_blocks, groups;
 };
 
@@ -413,43 +413,46 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
     }
     cp_async_wait<0>();
 
-    float* dst = P.partial + (ll) blockIdx.x * 27 * P.cin * P.cout;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + i, tap = tap0 + m / CIB, ci = c0 + m % CIB;
-        if (tap >= 27 || ci >= P.cin) continue;
+    // a thread's four rows are four input channels of one tap, the lanes of a warp lie along them
+    const int tap = tap0 + m0 / CIB, ci = c0 + m0 % CIB;
+    if (tap < 27) {
+        float* dst = P.partial + ((ll) blockIdx.x * 27 + tap) * P.cin * P.cout + ci;
 #pragma unroll
         for (int n = 0; n < TN; ++n) {
             const int co = o0 + n_off + n;
-            if (co < P.cout) { const float2 pair = unpack2(acc[i][n / 2]); dst[((ll) tap * P.cin + ci) * P.cout + co] = n & 1 ? pair.y : pair.x; }
+            if (co >= P.cout) continue;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 pair = unpack2(acc[i][n / 2]);
+                if (ci + i < P.cin) dst[(ll) co * P.cin + i] = n & 1 ? pair.y : pair.x;
+            }
         }
     }
 }
 
-// grad_weights[slot][co][ci][tap] += the block sums [range][tap][ci][co] of the slot's ranges.  Block = one input channel, 32 output
-// channels, one slot: warp y takes every eighth range, 27 independent coalesced loads at a time; the warps' sums are combined in a
-// fixed order and leave transposed, 27 contiguous values per filter.
-__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, SlotRanges sr, int accumulate, int cin, int cout, float* __restrict__ gw) {
+// grad_weights[slot][filter][tap] = (+=) the block sums [range][tap][filter] of the slot's ranges, filter = co * cin + ci.  Block = 32
+// filters of one slot: warp y takes every eighth range, 27 independent coalesced loads at a time; the warps' sums are combined in a
+// fixed order and leave transposed, as contiguous filters.
+__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, SlotRanges sr, int accumulate, ll filters, float* __restrict__ gw) {
     __shared__ float sums[8][27][33];
     const int lane = threadIdx.x & 31, y = threadIdx.x >> 5;
-    const int ci = blockIdx.x, co0 = blockIdx.y * 32, co = co0 + lane;
+    const ll f0 = (ll) blockIdx.x * 32, f = f0 + lane;
     int slot, r0 = 0, r1 = 0;
-    if ((int) blockIdx.z < sr.n) { slot = sr.slot[blockIdx.z]; r0 = sr.first[blockIdx.z]; r1 = sr.first[blockIdx.z + 1]; }
+    if ((int) blockIdx.y < sr.n) { slot = sr.slot[blockIdx.y]; r0 = sr.first[blockIdx.y]; r1 = sr.first[blockIdx.y + 1]; }
     else {                                     // the k-th slot without ranges
         unsigned left = sr.empty;
-        for (int k = (int) blockIdx.z - sr.n; k > 0; --k) left &= left - 1;
+        for (int k = (int) blockIdx.y - sr.n; k > 0; --k) left &= left - 1;
         slot = __ffs(left) - 1;
     }
     const int ny = min(8, r1 - r0);
-    const ll tap_stride = (ll) cin * cout, range_stride = 27 * tap_stride;
     float s[27];
 #pragma unroll
     for (int t = 0; t < 27; ++t) s[t] = 0.f;
-    if (co < cout) {
+    if (f < filters) {
         for (int r = r0 + y; r < r1; r += 8) {
-            const float* p = partial + r * range_stride + (ll) ci * cout + co;
+            const float* p = partial + r * 27 * filters + f;
 #pragma unroll
-            for (int t = 0; t < 27; ++t) s[t] += __ldg(p + t * tap_stride);
+            for (int t = 0; t < 27; ++t) s[t] += __ldg(p + t * filters);
         }
     }
     if (y < ny) {
@@ -457,14 +460,13 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict_
         for (int t = 0; t < 27; ++t) sums[y][t][lane] = s[t];
     }
     __syncthreads();
-    const int n = min(32, cout - co0) * 27;
-    float* dst = gw + (((ll) slot * cout + co0) * cin + ci) * 27;
+    const int n = (int) min((ll) 32, filters - f0) * 27;
+    float* dst = gw + ((ll) slot * filters + f0) * 27;
     for (int e = threadIdx.x; e < n; e += 256) {
         const int c = e / 27, t = e - c * 27;
         float v = 0.f;
         for (int k = 0; k < ny; ++k) v += sums[k][t][c];
-        float* o = dst + (ll) c * cin * 27 + t;
-        *o = accumulate ? *o + v : v;
+        dst[e] = accumulate ? dst[e] + v : v;
     }
 }
 
@@ -676,7 +678,8 @@ int aprnet_dw_reduce(const float* partial, SlotRanges sr, int slots, int accumul
     }
     if (nz == 0) return APRNET_OK;
     AprnetProfScope _prof("conv333_dw_reduce", st);
-    dw_reduce_kernel<<<dim3((unsigned) cin, (unsigned) aprnet_ceil_div(cout, 32), (unsigned) nz), 256, 0, st>>>(partial, sr, accumulate, cin, cout, gw);
+    const ll filters = (ll) cin * cout;
+    dw_reduce_kernel<<<dim3((unsigned) aprnet_ceil_div(filters, 32), (unsigned) nz), 256, 0, st>>>(partial, sr, accumulate, filters, gw);
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable seg
 // gathered values and the 32 dO values of KP locations are staged in shared memory (all table entries of a step, then all values, are
 // requested before any is used: the staging is bound by their latency); a thread owns a 4 x 4
 // tile of (tap, ci) x co products; the 4 thread groups of a block take different quarters of every staged
-// step and are combined in a fixed order.  partial[range][tap][ci][co].
+// step and are combined in a fixed order.  partial[range][tap][co][ci].
 struct SmallRanges { int n; ll begin[MAX_SEGS], end[MAX_SEGS], len[MAX_SEGS]; int first[MAX_SEGS + 1]; };
 
 template<int CIN>
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) conv333_small_dw_kernel(SmallRanges rg, c
     float* dst = partial + (ll) blockIdx.x * cout * CIN * 27;
     for (int e = threadIdx.x; e < ROWS * 32; e += 256) {
         const int row = e >> 5, co = co0 + (e & 31);
-        if (co < cout) dst[((ll) (row / CIN) * CIN + row % CIN) * cout + co] = red[e];
+        if (co < cout) dst[((ll) (row / CIN) * cout + co) * CIN + row % CIN] = red[e];
     }
 }
 

@@ -54,7 +54,7 @@ struct DwParams {
     ll tree_base, zero_row;
     const __nv_bfloat16* grows; int gpad;  // packed dO [N + 1][gpad], zeros at row g_zero_row
     ll g_zero_row;
-    float* partial;                        // [range][27][cin][cout]
+    float* partial;                        // [range][27][cout][cin]
     int cin, cout, ci_blocks, groups, d_per_group;
     int* error_flag;
 };
@@ -251,10 +251,10 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                     if (d < nd && ci < P.cin) {
                         const int tap = (d0 + d) * 3 + 2 - c0 / NCOL;      // block i of the columns holds dy = 1 - i
                         const int co0 = cob * NCOL + c0 % NCOL;
-                        float* o = dst + ((ll) tap * P.cin + ci) * P.cout + co0;
+                        float* o = dst + ((ll) tap * P.cout + co0) * P.cin + ci;         // the lanes lie along ci
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (co0 + j < P.cout) o[j] = __uint_as_float(r[j]);
+                            if (co0 + j < P.cout) o[(ll) j * P.cin] = __uint_as_float(r[j]);
                     }
                 }
             }

@@ -152,8 +152,9 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(const float* __restri
     const int slot = used.slot[blockIdx.z], k0 = blockIdx.x * 8, n0 = blockIdx.y * PK_N;
     const int n_dim = transposed ? cin : cout, k_dim = transposed ? cout : cin;
     const float* ws = w + (ll) slot * cout * cin * 27;
-#pragma unroll 9
-    for (int e = threadIdx.x; e < PK_N * 8 * 27; e += 256) {
+#pragma unroll
+    for (int i = 0; i < PK_N * 8 * 27 / 256; ++i) {          // 27: all requested before any is stored
+        const int e = threadIdx.x + i * 256;
         int n, k, tap;
         if (transposed) { k = e / (PK_N * 27); n = (e / 27) % PK_N; tap = e % 27; }        // ci (n) and tap are contiguous in memory
         else { n = e / (8 * 27); k = (e / 27) % 8; tap = e % 27; }                         // ci (k) and tap
