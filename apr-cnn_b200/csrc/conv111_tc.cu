@@ -5,17 +5,22 @@
 // level; with 2 * Cin * Cout flops against 4 * (Cin + Cout) bytes per location the CUDA-core kernel sits at the
 // fp32 multiply-add bound, the tensor-core kernel at the HBM bound.
 //
-// One persistent block per SM, 25 warps:
-//   warps 0-15  producers, four groups of 128 threads that take the tiles of 128 locations in turn.  (With two groups, 32 KB of loads in
-//               flight per SM, 64 -> 128 channels on 3.5 M locations took 0.84 ms against 0.42 ms at the HBM rate.)  A thread owns one location:
+// One persistent block per SM, 21 warps:
+//   warps 0-11  producers, three groups of 128 threads that take the tiles of 128 locations in turn (a fourth leaves 72 registers per
+//               thread, and the epilogue spills).  A thread owns one location:
 //               it requests up to 32 input channels at a time (4-byte loads, coalesced across the warp along the location
 //               axis of the channel-major tensor), rounds them to bf16 and writes them as 16-byte pieces of the K-major,
-//               hardware-swizzled A operand (the transposition happens in registers), then one arrival per thread on the
+//               hardware-swizzled A operand (the transposition happens in registers), then one arrival per warp on the
 //               stage's barrier;
-//   warp 16     one thread waits for the stage, fences the generic-proxy writes against the tensor core's reads and
+//   warp 12     one thread waits for the stage, fences the generic-proxy writes against the tensor core's reads and
 //               issues the Cin / 16 tcgen05.mma (M = 128, N = padded Cout) of each tile and commits the
 //               stage's "slot free" barrier and the accumulator's "complete" barrier;
-//   warps 17-24 epilogue, two sets of four warps on alternate tiles: TMEM -> registers (+ bias) -> coalesced fp32 stores of out[o][p].
+//   warps 13-20 epilogue, two sets of four warps on the two tiles of a unit: TMEM -> registers (+ bias) -> shared memory ->
+//               fp32 stores of out[o][p].  The rows of the channel-major tensor start at any multiple of four bytes, and a store that
+//               straddles two 128-byte lines costs two partial writes: writing 128 rows of 3.5 M locations from 64 ran at 3.3 TB/s, with
+//               aligned rows at 5.  So two neighbouring tiles (256 locations) are written together, 16 channels at a time, and every store
+//               covers what one line holds of them: 64 -> 128 channels on 3.5 M locations 0.85 -> 0.55 ms
+//               (0.42 ms at the HBM rate; the chain TMEM -> shared memory -> line is what is left).
 // The weights of one level (B operand, bf16, all of Cin x Cout) stay in shared memory; the block walks the levels one
 // after the other and converts the next level's weights from the fp32 tensor between two block-wide barriers.
 // Every wait is bounded and polls a block-wide abort flag; after an expiry the block raises the library's error flag,
@@ -32,12 +37,14 @@ namespace {
 using namespace tcptx;
 typedef long long ll;
 constexpr int TILE_M = 128;
-constexpr int C1_GROUPS = 4, C1_MMA = 4 * C1_GROUPS;
+constexpr int C1_GROUPS = 3, C1_MMA = 4 * C1_GROUPS;
 constexpr int C1_THREADS = (C1_MMA + 9) * 32;
 constexpr int DW_GROUPS = 2, DW_MMA = 8 * DW_GROUPS;
 constexpr int C1_THREADS_DW = (DW_MMA + 5) * 32;
 constexpr int C1_MAX_STAGES = 8;
 constexpr int C1_MAX_ACC = 4;
+constexpr int C1_OUT_CH = 16, C1_OUT_BYTES = 2 * C1_OUT_CH * 2 * TILE_M * 4;    // staged output: two buffers of 16 channels x 256 locations
+constexpr int C1_SMEM = 227 * 1024 - 1024;                                       // (the biases are static)
 constexpr int C1_MAX_SEGS = APRNET_MAX_LEVELS;
 
 struct C1Params {
@@ -78,8 +85,9 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     const int a_stage = kchunks * A_SUB;
     unsigned char* a_ring = smem;                                                   // stages x [kchunks][128][KS] bf16, swizzled
     unsigned char* b_s = a_ring + (size_t) stages * a_stage;                        // [kpad / 8][NT][8] bf16
-    uint64_t* bars = reinterpret_cast<uint64_t*>(b_s + (size_t) NT * P.kpad * 2);
-    uint64_t* full = bars;                              // [stages] operand written (128 producer threads)
+    float* out_s = reinterpret_cast<float*>(b_s + (size_t) NT * P.kpad * 2);        // [2][C1_OUT_CH][256]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + C1_OUT_BYTES / 4);
+    uint64_t* full = bars;                              // [stages] operand written (4 producer warps)
     uint64_t* empty = bars + C1_MAX_STAGES;             // [stages] MMAs that read the stage completed
     uint64_t* tmem_full = empty + C1_MAX_STAGES;        // [NACC]   accumulator complete
     uint64_t* tmem_empty = tmem_full + C1_MAX_ACC;      // [NACC]   accumulator read back (4 epilogue warps)
@@ -89,7 +97,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int c = tid; c < ACC_COLS; c += C1_THREADS) bias_s[c] = P.bias && c < P.n_out ? P.bias[c] : 0.f;
     if (tid == 0) {
-        for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), 128); mbar_init(smem_u32(empty + i), 1); }
+        for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), 4); mbar_init(smem_u32(empty + i), 1); }
         for (int i = 0; i < NACC; ++i) { mbar_init(smem_u32(tmem_full + i), 1); mbar_init(smem_u32(tmem_empty + i), 4); }
         *abort_flag = 0;
         fence_mbar_init();
@@ -101,12 +109,18 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     const uint32_t tmem_d = *tmem_slot;
     bool failed = false;
     const int ngroups = min(C1_GROUPS, stages);      // (a ring at least as long as the groups keeps the phases that a wait can meet apart)
+    int piece = 0;                          // 16-channel pieces the epilogue has staged
     uint32_t j_base = 0;                    // tiles this block has been given in the levels before the current one
 
     for (int seg = 0; seg < P.n_segs; ++seg) {
         const ll sb = P.seg_begin[seg], se = P.seg_end[seg];
         const int seg_tiles = (int) ((se - sb + TILE_M - 1) / TILE_M);
-        const int mine = (int) blockIdx.x < seg_tiles ? (seg_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
+        // units of two neighbouring tiles, of one where every block gets at most one tile
+        const int pair = seg_tiles > (int) gridDim.x ? 1 : 0;
+        const int seg_units = (seg_tiles + pair) >> pair;
+        const int units = (int) blockIdx.x < seg_units ? (seg_units - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
+        const int mine = (units << pair) - (units > 0 && (seg_tiles & pair) && (seg_units - 1) % (int) gridDim.x == (int) blockIdx.x ? 1 : 0);
+        auto tile_begin = [&](int it) { return sb + ((((ll) blockIdx.x + (ll) (it >> pair) * gridDim.x) << pair) + (it & pair)) * TILE_M; };
         // ---- the level's weights -> B operand (every accumulator of the previous level has been read back) ----
         __syncthreads();
         {
@@ -134,13 +148,17 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
             const int grp = tid >> 7, row = tid & 127;
             for (int it = grp; grp < ngroups && it < mine && !failed; it += ngroups) {
                 const uint32_t j = j_base + (uint32_t) it, slot = j % (uint32_t) stages, use = j / (uint32_t) stages;
-                const ll p = sb + ((ll) blockIdx.x + (ll) it * gridDim.x) * TILE_M + row;
-                const bool valid = p < se;
-                const float* src = P.in + (valid ? p : sb);
+                const float* src = P.in + min(tile_begin(it) + row, se - 1);     // rows past the end repeat the last location and are not stored
                 float v[KB];
                 auto request = [&](int kb) {
+                    const float* s = src + (ll) kb * P.ld_in;
+                    if (kb + KB <= P.n_in) {                                     // no condition per load
 #pragma unroll
-                    for (int q = 0; q < KB; ++q) v[q] = (valid && kb + q < P.n_in) ? src[(ll) (kb + q) * P.ld_in] : 0.f;
+                        for (int q = 0; q < KB; ++q) { v[q] = *s; s += P.ld_in; }
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < KB; ++q) v[q] = kb + q < P.n_in ? s[(ll) q * P.ld_in] : 0.f;
+                    }
                 };
                 request(0);             // in flight while this warp waits for the ring slot
                 if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
@@ -158,7 +176,8 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
                     }
                 }
                 // (no proxy fence here: the MMA thread fences after its wait)
-                mbar_arrive(smem_u32(full + slot));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(full + slot));
             }
         } else if (warp == C1_MMA) {
             // ---------------- MMA issue ----------------
@@ -185,32 +204,58 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
             }
         } else {
             // ---------------- epilogue ----------------
-            // two sets of four warps on alternate tiles (twice the stores in flight)
             const int q = warp & 3;                           // TMEM lane group this warp may read
-            const int row = q * 32 + lane;
-            for (int it = (warp - C1_MMA - 1) >> 2; it < mine && !failed; it += 2) {
+            const int w8 = warp - C1_MMA - 1, set = w8 >> 2;
+            for (int u = 0; u < units; ++u) {                 // (a failed warp keeps the pace of the barriers)
+                const int it = (u << pair) + set;
+                const bool has = set <= pair && it < mine;
                 const uint32_t j = j_base + (uint32_t) it, acc = j % NACC, acc_use = j / NACC;
-                const ll p = sb + ((ll) blockIdx.x + (ll) it * gridDim.x) * TILE_M + row;
-                if (!mbar_wait_warp(smem_u32(tmem_full + acc), acc_use & 1, abort_flag)) { failed = true; break; }
+                const ll p0 = tile_begin(u << pair);
+                const int cnt = (int) min(se - p0, (ll) (TILE_M << pair));
+                if (has && !failed && !mbar_wait_warp(smem_u32(tmem_full + acc), acc_use & 1, abort_flag)) failed = true;
+                const bool live = has && !failed;
+                constexpr int LINES = 2 * TILE_M / 32 + 1;
                 tc_fence_after();
+                const uint32_t taddr = tmem_d + ((uint32_t) (q * 32) << 16) + acc * ACC_COLS;
+                uint32_t r[C1_OUT_CH];
+                if (live) tmem_ld16(taddr, r);
+#pragma unroll 1
+                for (int c0 = 0; c0 < P.n_out; c0 += C1_OUT_CH) {
+                    float* buf = out_s + (piece++ & 1 ? C1_OUT_CH * 2 * TILE_M : 0);
+                    if (live) {
+                        tmem_ld_wait();
+                        float* dst = buf + set * TILE_M + q * 32 + lane;
 #pragma unroll
-                for (int c0 = 0; c0 < NT; c0 += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(tmem_d + ((uint32_t) (q * 32) << 16) + acc * ACC_COLS + c0, r);
-                    tmem_ld_wait();
-                    if (P.bias) {
-#pragma unroll
-                        for (int jj = 0; jj < 32; ++jj) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + bias_s[c0 + jj]);
+                        for (int jj = 0; jj < C1_OUT_CH; ++jj) dst[jj * 2 * TILE_M] = __uint_as_float(r[jj]);
+                        if (c0 + C1_OUT_CH < P.n_out) tmem_ld16(taddr + c0 + C1_OUT_CH, r);      // read while this piece is stored
                     }
-                    if (p < se) {
+                    // the buffer is written again after the barrier of the other one
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    if (failed) continue;
 #pragma unroll
-                        for (int jj = 0; jj < 32; ++jj)
-                            if (c0 + jj < P.n_out) P.out[(ll) (c0 + jj) * P.ld_out + p] = __uint_as_float(r[jj]);
+                    for (int k = 0; k < C1_OUT_CH / 8; ++k) {
+                        const int c = k * 8 + w8;
+                        if (c0 + c >= P.n_out) break;
+                        float* o = P.out + (ll) (c0 + c) * P.ld_out + p0;
+                        const int e0 = lane - (int) ((reinterpret_cast<uintptr_t>(o) >> 2) & 31);
+                        const float* src = buf + c * 2 * TILE_M + e0;
+                        const float bias = bias_s[c0 + c];
+                        float v[LINES];
+#pragma unroll
+                        for (int i = 0; i < LINES; ++i) v[i] = e0 + i * 32 >= 0 && e0 + i * 32 < 2 * TILE_M ? src[i * 32] : 0.f;
+                        if (P.bias) {
+#pragma unroll
+                            for (int i = 0; i < LINES; ++i) v[i] += bias;
+                        }
+                        o += e0;
+#pragma unroll
+                        for (int i = 0; i < LINES; ++i)
+                            if (e0 + i * 32 >= 0 && e0 + i * 32 < cnt) o[i * 32] = v[i];
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(tmem_empty + acc));
+                if (live && lane == 0) mbar_arrive(smem_u32(tmem_empty + acc));
             }
         }
         if (failed) *abort_flag = 1;
@@ -232,9 +277,9 @@ inline int pick_nt(int n) { return n <= 16 ? 16 : (n <= 32 ? 32 : (n <= 64 ? 64 
 template<int NT, int KS>
 int launch_c1(const C1Params& P, ll total_tiles, cudaStream_t st, const char* pname) {
     const size_t a_stage = (size_t) TILE_M * P.kpad * 2, b_bytes = (size_t) NT * P.kpad * 2;
-    const size_t fixed = b_bytes + (2 * C1_MAX_STAGES + 2 * C1_MAX_ACC) * 8 + 16 + 1024;
-    if (fixed + 2 * a_stage > 226 * 1024 - 1024) return APRNET_ERR_UNSUPPORTED;
-    const int stages = (int) std::min<size_t>(C1_MAX_STAGES, (226 * 1024 - 1024 - fixed) / a_stage);
+    const size_t fixed = b_bytes + C1_OUT_BYTES + (2 * C1_MAX_STAGES + 2 * C1_MAX_ACC) * 8 + 16 + 1024;
+    if (fixed + 2 * a_stage > C1_SMEM) return APRNET_ERR_UNSUPPORTED;
+    const int stages = (int) std::min<size_t>(C1_MAX_STAGES, (C1_SMEM - fixed) / a_stage);
     const size_t smem = (size_t) stages * a_stage + fixed;
     auto kern = conv111_tc_kernel<NT, KS>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
@@ -306,7 +351,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
     const int a_rows = mtiles * 128;
     const int stage_bytes = (a_rows + NT) * 256;             // two 64-location halves of 128 bytes per channel row
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t) stages * stage_bytes);
-    uint64_t* full = bars;                                   // [stages] operands written (the 256 threads of a group)
+    uint64_t* full = bars;                                   // [stages] operands written (the eight warps of a group)
     uint64_t* empty = bars + C1_MAX_STAGES;                  // [stages] MMAs that read the stage completed
     uint64_t* done = empty + C1_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
@@ -314,7 +359,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t tmem_cols = mtiles * NT <= 32 ? 32u : (mtiles * NT <= 64 ? 64u : (mtiles * NT <= 128 ? 128u : (mtiles * NT <= 256 ? 256u : 512u)));
     if (tid == 0) {
-        for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), 256); mbar_init(smem_u32(empty + i), 1); }
+        for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), 8); mbar_init(smem_u32(empty + i), 1); }
         mbar_init(smem_u32(done), 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -337,16 +382,19 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
             const ll p0 = sb + ((ll) blockIdx.x + (ll) it * gridDim.x) * TILE_M;
             if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
             unsigned char* st = smem + (size_t) slot * stage_bytes;
+            const bool whole = p0 + TILE_M <= se;
             for (int r0 = warp & 7; r0 < nrows; r0 += 8 * 8) {   // 8 rows of this warp x 4 quarters of 32 locations in flight
                 float v[8][4];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const int r = r0 + u * 8;
-                    const float* src = r < P.cout ? P.gout + (ll) r * P.ld_out : P.in + (ll) (r - P.cout) * P.ld_in;
+                    const int r = min(r0 + u * 8, nrows - 1);     // (the rows that repeat are not stored)
+                    const float* src = (r < P.cout ? P.gout + (ll) r * P.ld_out : P.in + (ll) (r - P.cout) * P.ld_in) + p0 + lane;
+                    if (whole) {                                  // no condition per load: a branch each cost more than the load
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const ll p = p0 + q * 32 + lane;
-                        v[u][q] = (r < nrows && p < se) ? src[p] : 0.f;
+                        for (int q = 0; q < 4; ++q) v[u][q] = src[q * 32];
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) v[u][q] = p0 + q * 32 + lane < se ? src[q * 32] : 0.f;
                     }
                 }
 #pragma unroll
@@ -365,7 +413,8 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
                     }
                 }
             }
-            mbar_arrive(smem_u32(full + slot));               // the MMA thread fences the generic-proxy writes after its wait
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(full + slot));   // the MMA thread fences the generic-proxy writes after its wait
         }
     } else if (warp == DW_MMA) {
         // ---------------- MMA issue ----------------
