@@ -76,7 +76,7 @@ __device__ __forceinline__ ll find_cell(const uint16_t* __restrict__ y, ll b, ll
     return (lo < e && (int) y[lo] == target) ? lo : -1;
 }
 
-// one warp per row: what fills cell (z + dz, x + dx, y) for every slot of the row; resolution as in build_nbr_table_kernel
+// one warp per row: what fills cell (z + dz, x + dx, y) for every slot of the row; binary search of the neighbour row in particles, coarser particles and tree nodes
 __global__ void run_sources_kernel(LevelMeta m, RunLevels R, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y, const ll* __restrict__ trow_ptr,
                                    const uint16_t* __restrict__ ty, const int32_t* __restrict__ first, const int32_t* __restrict__ slot_y, ll S,
                                    int32_t* __restrict__ src) {

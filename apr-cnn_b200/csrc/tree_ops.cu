@@ -149,48 +149,85 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(COARSE_TPB) tr
     }
 }
 
-// Max pooling: one thread per tree node of level cml-1.  Visiting order = APR-particle children in
+// ---- pooling and up-sampling ---------------------------------------------------------------------------
+// One thread per tree node and CH_PER_BLOCK channels.  Bound by HBM once enough loads are in flight: the loads carry no conditions (a
+// child outside the volume stands for entry 0 and its value is not used) and those of several channels are requested before the first
+// value is looked at; one conditional load after the other, the adjoint of the
+// up-sampling took 4.9 ms in a training step on 28 M particles instead of 2.3, the max pooling 3.0 instead of 2.6.
+
+// where child s of a node is stored: particles as they are, tree nodes from `off` on; 0 where there is none
+template<typename T>
+struct Children {
+    ll at[8];
+    unsigned particle = 0, node = 0;             // which of the eight are particles / tree nodes
+    __device__ Children(const int32_t* __restrict__ child, ll n_tree, ll t, ll off) {
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const int32_t v = child[(ll) s * n_tree + t];
+            at[s] = v >= 0 ? v : (v == APRNET_NONE ? 0 : aprnet_dec_tree(v) + off);
+            particle |= (v >= 0 ? 1u : 0u) << s;
+            node |= (v < APRNET_NONE ? 1u : 0u) << s;
+        }
+    }
+    __device__ void load(const T* __restrict__ x, T (&v)[8]) const {
+#pragma unroll
+        for (int s = 0; s < 8; ++s) v[s] = x[at[s]];
+    }
+};
+
+// Max pooling: tree nodes of level cml-1.  Visiting order = APR-particle children in
 // slot order (dz, dx, dy), then upgraded-node children in slot order; strict '>' against an initial
 // -1e17 with index 0 (pyapr/aprnet/src/maxpool.hpp:51-52,105-142).
 template<typename T>
 __global__ void maxpool_kernel(const int32_t* __restrict__ child, ll n_tree, ll tb, ll te, ll out_off,
                                const T* __restrict__ in, ll ld_in, T* __restrict__ out, long long* __restrict__ idx,
                                ll ld_out, int C, ll up_off) {
+    constexpr int CB = 2;
     const ll t = tb + (ll) blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= te) return;
-    int32_t ch[8];
-#pragma unroll
-    for (int s = 0; s < 8; ++s) ch[s] = child[(ll) s * n_tree + t];
+    const Children<T> ch(child, n_tree, t, up_off);
     const int c0 = blockIdx.y * CH_PER_BLOCK, c1 = min(C, c0 + CH_PER_BLOCK);
-    for (int c = c0; c < c1; ++c) {
-        const T* x = in + (ll) c * ld_in;
-        T best = (T) -1e17f;
-        ll arg = 0;
+    for (int c = c0; c < c1; c += CB) {
+        T v[CB][8];
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            const int32_t v = ch[s];
-            if (v >= 0) { const T val = x[v]; if (val > best) { best = val; arg = v; } }
-        }
+        for (int k = 0; k < CB; ++k) ch.load(in + (ll) min(c + k, C - 1) * ld_in, v[k]);
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            const int32_t v = ch[s];
-            if (v < APRNET_NONE) { const ll q = aprnet_dec_tree(v) + up_off; const T val = x[q]; if (val > best) { best = val; arg = q; } }
+        for (int k = 0; k < CB; ++k) {
+            if (c + k >= c1) break;
+            T best = (T) -1e17f;
+            ll arg = 0;
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if ((ch.particle >> s & 1) && v[k][s] > best) { best = v[k][s]; arg = ch.at[s]; }
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if ((ch.node >> s & 1) && v[k][s] > best) { best = v[k][s]; arg = ch.at[s]; }
+            out[(ll) (c + k) * ld_out + t + out_off] = best;
+            idx[(ll) (c + k) * ld_out + t + out_off] = arg;
         }
-        out[(ll) c * ld_out + t + out_off] = best;
-        idx[(ll) c * ld_out + t + out_off] = arg;
     }
 }
 
 template<typename T>
 __global__ void maxpool_backward_kernel(const T* __restrict__ gout, const long long* __restrict__ idx, ll ld_out,
                                         T* __restrict__ gin, ll ld_in, ll nfixed, ll m, int C) {
+    constexpr int CB = 4;
     const ll i = (ll) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const int c0 = blockIdx.y * CH_PER_BLOCK, c1 = min(C, c0 + CH_PER_BLOCK);
-    for (int c = c0; c < c1; ++c) {
-        const T g = gout[(ll) c * ld_out + i];
-        const ll dst = i < nfixed ? i : idx[(ll) c * ld_out + i];
-        gin[(ll) c * ld_in + dst] = g;
+    const bool fixed = i < nfixed;
+    for (int c = c0; c < c1; c += CB) {
+        T g[CB];
+        ll dst[CB];
+#pragma unroll
+        for (int k = 0; k < CB; ++k) {
+            const ll at = (ll) min(c + k, C - 1) * ld_out + i;
+            g[k] = gout[at];
+            dst[k] = fixed ? i : idx[at];
+        }
+#pragma unroll
+        for (int k = 0; k < CB; ++k)
+            if (c + k < c1) gin[(ll) (c + k) * ld_in + dst[k]] = g[k];
     }
 }
 
@@ -199,30 +236,39 @@ __global__ void maxpool_backward_kernel(const T* __restrict__ gout, const long l
 template<typename T, bool BACKWARD>
 __global__ void upsample_kernel(const int32_t* __restrict__ child, ll n_tree, ll tb, ll te, ll in_off, ll out_off,
                                 const T* __restrict__ src, ll ld_src, T* __restrict__ dst, ll ld_dst, int C) {
+    constexpr int CB = BACKWARD ? 2 : 4;
     const ll t = tb + (ll) blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= te) return;
-    int32_t ch[8];
-#pragma unroll
-    for (int s = 0; s < 8; ++s) ch[s] = child[(ll) s * n_tree + t];
+    const Children<T> ch(child, n_tree, t, out_off);
     const int c0 = blockIdx.y * CH_PER_BLOCK, c1 = min(C, c0 + CH_PER_BLOCK);
-    for (int c = c0; c < c1; ++c) {
+    for (int c = c0; c < c1; c += CB) {
         if (!BACKWARD) {        // src = input (coarse), dst = output (fine)
-            const T v = src[(ll) c * ld_src + t + in_off];
-            T* o = dst + (ll) c * ld_dst;
+            T v[CB];
 #pragma unroll
-            for (int s = 0; s < 8; ++s) {
-                const int32_t q = ch[s];
-                if (q >= 0) o[q] = v; else if (q != APRNET_NONE) o[aprnet_dec_tree(q) + out_off] = v;
+            for (int k = 0; k < CB; ++k) v[k] = src[(ll) min(c + k, C - 1) * ld_src + t + in_off];
+#pragma unroll
+            for (int k = 0; k < CB; ++k) {
+                if (c + k >= c1) break;
+                T* o = dst + (ll) (c + k) * ld_dst;
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    if ((ch.particle | ch.node) >> s & 1) o[ch.at[s]] = v[k];
             }
         } else {                // src = grad_output (fine), dst = grad_input (coarse)
-            const T* go = src + (ll) c * ld_src;
-            T s_part = 0, s_tree = 0;
+            T v[CB][8];
 #pragma unroll
-            for (int s = 0; s < 8; ++s) {
-                const int32_t q = ch[s];
-                if (q >= 0) s_part += go[q]; else if (q != APRNET_NONE) s_tree += go[aprnet_dec_tree(q) + out_off];
+            for (int k = 0; k < CB; ++k) ch.load(src + (ll) min(c + k, C - 1) * ld_src, v[k]);
+#pragma unroll
+            for (int k = 0; k < CB; ++k) {
+                if (c + k >= c1) break;
+                T s_part = 0, s_tree = 0;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    if (ch.particle >> s & 1) s_part += v[k][s];
+                    if (ch.node >> s & 1) s_tree += v[k][s];
+                }
+                dst[(ll) (c + k) * ld_dst + t + in_off] = s_part + s_tree;
             }
-            dst[(ll) c * ld_dst + t + in_off] = s_part + s_tree;
         }
     }
 }
