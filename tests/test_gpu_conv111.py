@@ -1,0 +1,44 @@
+"""1x1x1 layers on the tensor cores at the edges of their tiles (pairs of 128 locations, pieces of 16 channels, 128-byte lines): with
+one stencil the layer is one matrix product over all locations.  Operands are exact in bf16 and at most 256 products are added in
+fp32, each rounding at most 2^-24 of the sum of magnitudes so far: |error| <= 2^-16 of that sum for the forward pass and the input
+gradient.  The weight gradient adds over all locations, in blocks: 2-norm error at most 1e-5, the rounding errors of random sign."""
+import pytest
+import torch
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+WIDTHS = [(8, 8), (16, 17), (24, 16), (33, 40), (64, 128), (130, 72), (256, 128), (128, 250)]
+
+
+@pytest.mark.parametrize("name", ["blob", "odd", "many"])
+@pytest.mark.parametrize("cin,cout", WIDTHS)
+def test_conv111_edges(name, cin, cout):
+    import pyapr
+    from pyapr.aprnet import cuda as ops
+    from _pyaprwrapper.aprnet import cuda as C
+    a = H.blob_arrays((64, 128, 128), 40, 11) if name == "many" else (H.arrays(name) if name in H.APR_CASES else H.blob_arrays())
+    apr = pyapr.apr_from_arrays(a)
+    apr.init_cuda()
+    torch.manual_seed(cin * 300 + cout)
+    exact = lambda *s: torch.randn(*s, device="cuda").bfloat16().float()
+    for dl in range(0, min(H.max_dl(a), 2) + 1):
+        n = int(pyapr.aprnet.utils.number_particles(apr, dl))
+        conv = ops.APRConv(cin, cout, nstencils=1, kernel_size=(1, 1, 1), precision="bf16").cuda()
+        with torch.no_grad():
+            conv.weight.copy_(exact(*conv.weight.shape))
+        x, g = exact(1, cin, n).requires_grad_(True), exact(1, cout, n)
+        out = conv(x, [apr], torch.full((1,), dl, dtype=torch.int32))
+        out.backward(g)
+        assert C.tc_error_flag() == 0
+        w, xd, gd = conv.weight.detach().double().reshape(cout, cin), x.detach()[0].double(), g[0].double()
+        want, size = w @ xd, w.abs() @ xd.abs()
+        if conv.bias is not None:
+            b = conv.bias.detach().double().reshape(-1, 1)
+            want, size = want + b, size + b.abs()
+        assert bool(((out.detach()[0].double() - want).abs() <= size * 2.0 ** -16).all()), dl
+        want, size = w.t() @ gd, w.t().abs() @ gd.abs()
+        assert bool(((x.grad[0].double() - want).abs() <= size * 2.0 ** -16).all()), dl
+        want = gd @ xd.t()
+        assert float((conv.weight.grad.double().reshape(cout, cin) - want).norm() / want.norm()) <= 1e-5, dl
