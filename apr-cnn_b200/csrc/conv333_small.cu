@@ -47,53 +47,81 @@ __global__ void small_stage_kernel(const float* __restrict__ x, ll ld_x, ll n, c
         vals[(ll) ci * R + r] = r < n ? x[(ll) ci * ld_x + r] : (r < n + t ? tree[(ll) ci * ld_tree + (r - n)] : 0.f);
 }
 
-// forward: thread = output location x block of 32 output channels; weights of the level's stencil in
-// shared memory as [tap][ci][32] (read four at a time)
-template<int CIN>
-__global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable segs, const int32_t* __restrict__ nbr, ll N, ll T,
+// forward: thread = output location x block of 32 output channels; weights of the level's stencil in shared memory as [tap][ci][32],
+// read four at a time.  What bounds it: the latency of the gathers, and per block the staging of the weights (27 strided values per
+// thread row, as many cache lines as the gathers of a tile touch).  So a block takes up to eight tiles with one staging, and the taps
+// go in thirds: the next third's table entries are on their way during the multiply-adds.  1 -> 32 channels: 28 M locations 5.5 -> 3.6 ms,
+// 3.5 M 0.71 -> 0.53; 2 -> 32: 9.3 -> 6.8.  (Two locations per thread, half the weight reads: 5.7 ms, too few warps.)
+template<int CIN, int TAPS>
+__global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable segs, int tiles, const int32_t* __restrict__ nbr, ll N, ll T,
                                                                     const float* __restrict__ vals, const float* __restrict__ w,
                                                                     int cout, const float* __restrict__ bias, float* __restrict__ out, ll ld_out) {
     __shared__ F4 ws[27 * CIN * 8];
+    __shared__ float bias_s[32];
     int seg = 0;
     while (seg + 1 < segs.n && (int) blockIdx.x >= segs.tile_begin[seg + 1]) ++seg;
-    const ll p = segs.begin[seg] + (ll) (blockIdx.x - segs.tile_begin[seg]) * 128 + threadIdx.x;
     const int co0 = blockIdx.y * 32;
     const float* wslot = w + (ll) segs.slot[seg] * cout * CIN * 27;
     for (int e = threadIdx.x; e < 27 * CIN * 32; e += 128) {
         const int co = e & 31, ci = (e >> 5) % CIN, tap = e / (32 * CIN);
         reinterpret_cast<float*>(ws)[e] = co0 + co < cout ? wslot[((ll) (co0 + co) * CIN + ci) * 27 + tap] : 0.f;
     }
+    if (threadIdx.x < 32) bias_s[threadIdx.x] = bias && co0 + (int) threadIdx.x < cout ? bias[co0 + threadIdx.x] : 0.f;
     __syncthreads();
-    if (p >= segs.end[seg]) return;
-    const ll R = N + T + 1;
-    float acc[32];
+    const ll R = N + T + 1, end = segs.end[seg];
+    ll p = segs.begin[seg] + (ll) (blockIdx.x - segs.tile_begin[seg]) * 128 * tiles + threadIdx.x;
+    const int nco = min(32, cout - co0);
+    for (int i = 0; i < tiles && p < end; ++i, p += 128) {
+        float acc[32];
 #pragma unroll
-    for (int o = 0; o < 32; ++o) acc[o] = 0.f;
-    // all 27 table entries, then all 27 values of a channel, are requested before any is used (the kernel is bound by
-    // the latency of these gathers, not by a unit); row numbers fit 32 bits (N + T + 1 < 2^31, checked by the driver)
-    int32_t rows[27];
+        for (int o = 0; o < 32; ++o) acc[o] = 0.f;
+        // TAPS table entries and then TAPS values are requested before any is used; row numbers fit 32 bits (N + T + 1 < 2^31, checked by
+        // the driver)
+        int32_t rows[TAPS];
+        auto request = [&](int tap0) {
+            const int32_t* e = nbr + (ll) tap0 * N + p;
 #pragma unroll
-    for (int tap = 0; tap < 27; ++tap) rows[tap] = (int32_t) resolve_row(__ldg(nbr + (ll) tap * N + p), N, N + T);
+            for (int t = 0; t < TAPS; ++t) rows[t] = (int32_t) resolve_row(__ldg(e + (ll) t * N), N, N + T);
+        };
+        request(0);
 #pragma unroll 1
-    for (int ci = 0; ci < CIN; ++ci) {
-        float v[27];
-        const float* vc = vals + (ll) ci * R;
+        for (int ci = 0; ci < CIN; ++ci) {
+            const float* vc = vals + (ll) ci * R;
+#pragma unroll 1
+            for (int tap0 = 0; tap0 < 27; tap0 += TAPS) {
+                float v[TAPS];
 #pragma unroll
-        for (int tap = 0; tap < 27; ++tap) v[tap] = __ldg(vc + rows[tap]);
+                for (int t = 0; t < TAPS; ++t) v[t] = __ldg(vc + rows[t]);
+                if (TAPS < 27) {
+                    if (tap0 + TAPS < 27) request(tap0 + TAPS);
+                    else if (ci + 1 < CIN) request(0);
+                }
 #pragma unroll
-        for (int tap = 0; tap < 27; ++tap) {
-            const F4* wr = ws + (tap * CIN + ci) * 8;
+                for (int t = 0; t < TAPS; ++t) {
+                    const F4* wr = ws + ((tap0 + t) * CIN + ci) * 8;
 #pragma unroll
-            for (int o4 = 0; o4 < 8; ++o4) {
-                const F4 q = wr[o4];
+                    for (int o4 = 0; o4 < 8; ++o4) {
+                        const F4 q = wr[o4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) acc[4 * o4 + k] = fmaf(v[tap], q.a[k], acc[4 * o4 + k]);
+                        for (int k = 0; k < 4; ++k) acc[4 * o4 + k] = fmaf(v[t], q.a[k], acc[4 * o4 + k]);
+                    }
+                }
             }
         }
-    }
+        if (bias) {
 #pragma unroll
-    for (int o = 0; o < 32; ++o)
-        if (co0 + o < cout) out[(ll) (co0 + o) * ld_out + p] = bias ? acc[o] + __ldg(bias + co0 + o) : acc[o];
+            for (int o = 0; o < 32; ++o) acc[o] += bias_s[o];
+        }
+        float* dst = out + (ll) co0 * ld_out + p;
+        if (nco == 32) {
+#pragma unroll
+            for (int o = 0; o < 32; ++o) dst[(ll) o * ld_out] = acc[o];
+        } else {
+#pragma unroll
+            for (int o = 0; o < 32; ++o)
+                if (o < nco) dst[(ll) o * ld_out] = acc[o];
+        }
+    }
 }
 
 // weight gradient: block = range of locations of one level x block of 32 output channels, one launch over all levels.  The 27 x CIN
@@ -203,20 +231,27 @@ int aprnet_small_stage(const float* x, ll ld_x, ll n, const float* tree, ll ld_t
 int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, const float* bias, float* out, ll ld_out, cudaStream_t st) {
     const AprPlan* plan = aprnet_get_plan(a, dl, st);
     if (!plan) return APRNET_ERR_CUDA;
-    const SegTable segs = make_seg_table(aprnet_segments(a, dl, slots, false), 128);
-    const int tiles = segs.tile_begin[segs.n];
-    if (tiles == 0) return APRNET_OK;
-    dim3 grid((unsigned) tiles, (unsigned) aprnet_ceil_div(cout, 32));
+    const std::vector<Segment> list = aprnet_segments(a, dl, slots, false);
+    ll total = 0;
+    for (const Segment& g : list) total += g.end - g.begin;
+    // several tiles per block once eight blocks per SM have one each; where two blocks per SM hold everything, the time is that of one
+    // tile and all its taps are requested at once (2 -> 32 channels on 7 k locations: 17 us, in thirds 21)
+    const ll tiles = aprnet_ceil_div(total, 128), groups = aprnet_ceil_div(cout, 32);
+    const int per_block = (int) std::min<ll>(8, std::max<ll>(1, tiles * groups / (148 * 8)));
+    const bool few = tiles * groups <= 148 * 2;
+    const SegTable segs = make_seg_table(list, 128 * per_block);
+    if (segs.tile_begin[segs.n] == 0) return APRNET_OK;
+    dim3 grid((unsigned) segs.tile_begin[segs.n], (unsigned) groups);
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_small_fwd:ci%d:co%d:dl%d", cin, cout, dl);
     AprnetProfScope _prof(pname, st);
+#define SMALL_CASE(CIN_) case CIN_: (few ? conv333_small_forward_kernel<CIN_, 27> : conv333_small_forward_kernel<CIN_, 9>)<<<grid, 128, 0, st>>>( \
+        segs, per_block, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
     switch (cin) {
-        case 1: conv333_small_forward_kernel<1><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
-        case 2: conv333_small_forward_kernel<2><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
-        case 3: conv333_small_forward_kernel<3><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
-        case 4: conv333_small_forward_kernel<4><<<grid, 128, 0, st>>>(segs, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
+        SMALL_CASE(1) SMALL_CASE(2) SMALL_CASE(3) SMALL_CASE(4)
         default: aprnet_set_error("small-Cin path called with cin = %d", cin); return APRNET_ERR_ARG;
     }
+#undef SMALL_CASE
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
