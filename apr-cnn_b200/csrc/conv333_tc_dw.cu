@@ -40,6 +40,7 @@ constexpr int DW_THREADS = (4 * NGROUP + 1) * 32;
 constexpr int DW_MAX_STAGES = 6;
 constexpr int A_STAGE = 2 * PT * 128;         // 128 accumulator rows = two 64-element swizzle atoms per slot
 constexpr int G_ROWS = PT + 8;                // dO of slots -1 .. 128 of the chunk, whole 8-row groups
+constexpr int DO_PHASES = NGROUP;             // "dO chunk read" barriers: chunk modulo DO_PHASES (the buffers alternate between two)
 
 constexpr int DW_MAX_SEGS = APRNET_MAX_LEVELS;
 struct DwParams {
@@ -79,8 +80,8 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
     uint64_t* full = bars;                       // [nstage] gathered rows landed (4 warps x 32 lanes)
     uint64_t* empty = bars + DW_MAX_STAGES;      // [nstage] MMAs that read the stage completed
     uint64_t* dfull = empty + DW_MAX_STAGES;     // [2] dO chunk landed
-    uint64_t* dempty = dfull + 2;                // [2] MMAs that read the dO chunk completed
-    uint64_t* done = dempty + 2;                 // all MMAs of the range completed
+    uint64_t* dempty = dfull + 2;                // [4] MMAs that read the dO chunk completed, by chunk modulo 4
+    uint64_t* done = dempty + DO_PHASES;         // all MMAs of the range completed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -101,7 +102,8 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
 
     if (tid == 0) {
         for (int i = 0; i < nstage; ++i) { mbar_init(smem_u32(full + i), 128); mbar_init(smem_u32(empty + i), 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(dfull + i), 128); mbar_init(smem_u32(dempty + i), 1); }
+        for (int i = 0; i < 2; ++i) mbar_init(smem_u32(dfull + i), 128);
+        for (int i = 0; i < DO_PHASES; ++i) mbar_init(smem_u32(dempty + i), 1);
         mbar_init(smem_u32(done), 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -155,9 +157,11 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
             const uint32_t slot = (uint32_t) s % (uint32_t) nstage, use = (uint32_t) s / (uint32_t) nstage;
             if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
             if (mt == 0) {
-                // this warp's rows of the dO chunk
-                const uint32_t db = chunk & 1, duse = chunk >> 1;
-                if (duse > 0 && !mbar_wait_warp(smem_u32(dempty + db), (duse - 1) & 1, abort_flag)) { failed = true; break; }
+                // this warp's rows of the dO chunk, into the buffer of chunk - 2.  A wait by parity must know the phase before the awaited
+                // one complete: the group that fills chunk c also filled c - 4 (groups take the stages modulo four), so with a barrier per
+                // chunk modulo four every warp waits for all phases of the barriers it uses, one after the other.
+                const uint32_t db = chunk & 1, before = (uint32_t) chunk - 2;
+                if (chunk >= 2 && !mbar_wait_warp(smem_u32(dempty + before % DO_PHASES), (before / DO_PHASES) & 1, abort_flag)) { failed = true; break; }
                 unsigned char* g_s = g_ring + db * G_BYTES;
                 constexpr int GP = NCOL / 8;                           // 16-byte pieces of a dO row
                 const int cc = lane % GP;
@@ -225,7 +229,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                         }
                     }
                     umma_commit(smem_u32(empty + slot));
-                    if (mt == MT - 1) umma_commit(smem_u32(dempty + db));
+                    if (mt == MT - 1) umma_commit(smem_u32(dempty + chunk % DO_PHASES));
                     if (++slot == (uint32_t) nstage) { slot = 0; ++use; }
                 }
             }
@@ -273,12 +277,10 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
 template<int CIB, int NCOL>
 int launch_dw(const DwParams& P, int nranges, int blocks_y, cudaStream_t st, const char* pname) {
     constexpr size_t G_BYTES = ((size_t) G_ROWS * (NCOL == 32 ? 64 : 128) * (NCOL == 128 ? 2 : 1) + 1023) / 1024 * 1024;
-    const size_t fixed = 2 * G_BYTES + (2 * DW_MAX_STAGES + 5) * 8 + 16 + 1024;
-    // Every wait on a barrier must find the phase before the awaited one complete (its parity test cannot tell two phases apart).  For
-    // the ring that holds with at least NGROUP stages; for the two dO buffers, filled for chunk c after chunk c - 2 has been read, also
-    // when a chunk is one stage only if the ring has at most four: chunk c - 4 has then been read when stage c is filled.
-    const bool one_tile = (9 - P.d_per_group * (P.groups - 1)) * CIB <= 128 || P.d_per_group * CIB <= 128;
-    const int nstage = (int) std::min<size_t>(one_tile ? 4 : DW_MAX_STAGES, (227 * 1024 - fixed) / A_STAGE);
+    const size_t fixed = 2 * G_BYTES + (2 * DW_MAX_STAGES + 2 + DO_PHASES + 1) * 8 + 16 + 1024;
+    // A wait for a ring slot must find the phase before the awaited one complete (its parity test cannot tell two phases apart): with at
+    // least NGROUP stages the group has by then seen a later stage of that round read.  The dO buffers have barriers of their own.
+    const int nstage = (int) std::min<size_t>(DW_MAX_STAGES, (227 * 1024 - fixed) / A_STAGE);
     if (nstage < NGROUP) { aprnet_set_error("conv333 tensor-core weight gradient: ring of %d stages", nstage); return APRNET_ERR_UNSUPPORTED; }
     const size_t smem = (size_t) nstage * A_STAGE + fixed;
     auto kern = conv333_tc_dw_kernel<CIB, NCOL>;

@@ -1,7 +1,12 @@
-"""The run kernels (9 gathered rows per slot, y taps as shifted reads) against the kernels that gather every tap by itself, at the
-edges of their tile shapes.  The forward pass keeps the order of the products: equal bit for bit.  The input gradient may add the
-same products in another order: relative difference (2-norm) at most 2e-6, a few fp32 roundings of sums of unit scale.  The same
-bound holds for the weight gradient, whose sums run over all locations."""
+"""The run kernels (9 gathered rows per slot, y taps as shifted reads) at the edges of their tile shapes.
+
+Forward pass and input gradient against the kernels that gather every tap by itself (`runs` = 0).  The forward pass keeps the order
+of the products: equal bit for bit (from 128 channels on each side both arms are the tap kernel).  The input gradient may add
+the same products in another order: relative difference (2-norm) at most 2e-6, a few fp32 roundings of sums of unit scale.
+
+The weight gradient always runs over the slots; it is held against the float64 kernel on the same operands: features and gradients
+that are exact in bf16, and the tree means as they are rounded to bf16.  What is left is the rounding of fp32 sums: the tensor cores truncate, so an accumulator that takes DEPTH products of 16 slots one after the
+other loses at most DEPTH * 2^-23 of sums of its own size."""
 import numpy as np
 import pytest
 import torch
@@ -42,5 +47,41 @@ def test_run_kernels_match_the_tap_kernels(name, cin, cout):
         got = _run(apr, dl, cin, cout, n)
         assert C.tc_error_flag() == 0
         assert torch.equal(got[0], want[0]), (dl, int((got[0] != want[0]).sum()))
-        for k in (1, 2):
-            assert float((got[k] - want[k]).norm() / want[k].norm()) <= 2e-6, (dl, k)
+        assert float((got[1] - want[1]).norm() / want[1].norm()) <= 2e-6, dl
+
+
+# widths with one stage per chunk of slots (more than 64 output channels, the last neighbour group of wide inputs) and with several
+DW_WIDTHS = [(8, 8), (16, 40), (33, 33), (64, 32), (24, 120), (32, 128), (128, 64), (128, 128), (130, 32), (48, 200)]
+
+
+@pytest.mark.parametrize("name", ["blob", "odd", "plane", "many_chunks"])
+@pytest.mark.parametrize("cin,cout", DW_WIDTHS)
+def test_weight_gradient_matches_float64(name, cin, cout):
+    import pyapr
+    from _pyaprwrapper.aprnet import cuda as C
+    from _pyaprwrapper.data_containers import APRPtrVector
+    if name == "many_chunks":              # hundreds of chunks per block: the dO buffers and the ring go round many times
+        a = H.blob_arrays((128, 128, 128), 200, 12)
+    else:
+        a = H.arrays(name) if name in H.APR_CASES else H.blob_arrays()
+    apr = pyapr.apr_from_arrays(a)
+    apr.init_cuda()
+    L = a.level_max - a.level_min + 1
+    for dl in (0,) if name == "many_chunks" else range(0, H.max_dl(a) + 1):
+        n = int(pyapr.aprnet.utils.number_particles(apr, dl))
+        ld = torch.full((1,), dl, dtype=torch.int32)
+        torch.manual_seed(2)
+        x = torch.randn(1, cin, n, device="cuda").bfloat16().float()
+        g = torch.randn(1, cout, n, device="cuda").bfloat16().float()
+        w = torch.randn(L, cout, cin, 3, 3, 3, device="cuda") / (27 * cin) ** 0.5
+        v = APRPtrVector([apr])
+        _, rows = C.conv333_forward_keep_rows(v, x, w, ld, "bf16")
+        runs = [C.conv333_backward_with_rows(v, rows, w, g, ld, False, "bf16")[1] for _ in range(3)]
+        assert C.tc_error_flag() == 0
+        assert all(torch.equal(r, runs[0]) for r in runs[1:])          # one order of summation
+        tree = C.conv333_forward_keep_tree(v, x, w, ld, "fp32")[1]
+        if cin > 4: tree = tree.bfloat16()
+        want = C.conv333_backward_pretree(v, x.double(), tree.double(), torch.empty(0, dtype=torch.uint8, device="cuda"), w.double(),
+                                          g.double(), ld, False)[2]
+        depth = 1.27 * n / 16          # all slots in one accumulator: more than any block takes
+        assert float((runs[0] - want).norm() / want.norm()) <= depth * 2.0 ** -23, (dl, float((runs[0] - want).norm() / want.norm()))
