@@ -65,6 +65,7 @@ __device__ __forceinline__ unsigned long long pack2(float x, float y) {
 __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
+__device__ __forceinline__ void add2(unsigned long long& acc, unsigned long long a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
 __device__ __forceinline__ float2 unpack2(unsigned long long v) {
     float2 r;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
@@ -309,12 +310,19 @@ __global__ void __launch_bounds__(256) vrow_reduce_f32_kernel(const int32_t* __r
 // ring slot holds 16 locations of both operands as they lie in memory (rows of channels), which is the order in which a
 // thread's 4 x TN results want them.  The blocks of a level take its units of 64 locations in turn, so that blocks that run
 // together gather from neighbouring rows.  Block sums go to a workspace and are added in a fixed order.
+//
+// A result of the block would be one chain of additions, and its rounding error grows with the chain.  So the chain starts again
+// after seg_flush slots: narrow tiles (TN <= 8) keep the sum of the finished chains in registers; wide ones, whose accumulators take
+// them, add it to the block's sum in the workspace (only one thread ever touches a sum, so its reductions are applied in program order:
+// one order of summation).  Relative error against float64 on 2 M locations, one chain / chains: 16 -> 16 6.6e-7 / 2.3e-7, 33 -> 33
+// 15e-7 / 8.1e-7, 128 -> 128 34e-7 / 8.6e-7; it costs 0 (16 -> 16) to 4 % (64 -> 64) of the kernel's time.
 constexpr int DW_UNIT = 64;
 
 struct F32DwParams {
     int n_segs;
     ll seg_begin[MAX_SEGS], seg_end[MAX_SEGS];
     int range_first[MAX_SEGS + 1];
+    int seg_flush[MAX_SEGS];               // ring slots per chain of additions
     const int32_t* nbr; ll N;
     const float* xrows; int xpad; ll tree_base, zero_row;
     const float* grows; int gpad; ll g_zero_row;
@@ -379,55 +387,77 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
         if (++islot == RING) islot = 0;
     };
 
-    unsigned long long acc[4][TN / 2];
+    constexpr bool IN_REGISTERS = TN <= 8;
+    unsigned long long acc[4][TN / 2], done[IN_REGISTERS ? 4 : 1][IN_REGISTERS ? TN / 2 : 1];
+    if (IN_REGISTERS) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int n = 0; n < TN / 2; ++n) acc[i][n] = 0ull;
+            for (int n = 0; n < TN / 2; ++n) done[i][n] = 0ull;
+    }
 
     request(0);
 #pragma unroll
     for (int s = 0; s < RING - 1; ++s) { issue(); cp_async_commit(); }
     const int m0 = wm * 128 + lane * 4;            // this thread's rows: m0 .. m0 + 3
     const int a_off = (m0 / CIB) * TAP_STRIDE + m0 % CIB, n_off = wn * TN;
-    int slot = 0;
-    for (int s = 0; s < total; ++s) {
-        cp_async_wait<RING - 2>();
-        __syncthreads();
-        issue();
-        cp_async_commit();
-        const float* a_s = ring + slot * SLOT;
-        const float* b_s = a_s + A_ELEMS + n_off;
+    int slot = 0, s = 0;
+    do {
+        const int s0 = s, s1 = min(total, s + P.seg_flush[seg]);
 #pragma unroll
-        for (int k = 0; k < KS; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(a_s + a_off + k * CIB);
-            const unsigned long long a2[4] = {pack2(a.x, a.x), pack2(a.y, a.y), pack2(a.z, a.z), pack2(a.w, a.w)};
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int h = 0; h < TN / 4; ++h) {
-                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(b_s + k * NT + h * 4);
+            for (int n = 0; n < TN / 2; ++n) acc[i][n] = 0ull;
+        for (; s < s1; ++s) {
+            cp_async_wait<RING - 2>();
+            __syncthreads();
+            issue();
+            cp_async_commit();
+            const float* a_s = ring + slot * SLOT;
+            const float* b_s = a_s + A_ELEMS + n_off;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) { fma2(acc[i][2 * h], a2[i], b.x); fma2(acc[i][2 * h + 1], a2[i], b.y); }
+            for (int k = 0; k < KS; ++k) {
+                const float4 a = *reinterpret_cast<const float4*>(a_s + a_off + k * CIB);
+                const unsigned long long a2[4] = {pack2(a.x, a.x), pack2(a.y, a.y), pack2(a.z, a.z), pack2(a.w, a.w)};
+#pragma unroll
+                for (int h = 0; h < TN / 4; ++h) {
+                    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(b_s + k * NT + h * 4);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { fma2(acc[i][2 * h], a2[i], b.x); fma2(acc[i][2 * h + 1], a2[i], b.y); }
+                }
+            }
+            if (++slot == RING) slot = 0;
+        }
+        if (IN_REGISTERS) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int n = 0; n < TN / 2; ++n) add2(done[i][n], acc[i][n]);
+        }
+        if (IN_REGISTERS && s < total) continue;
+        // a thread's four rows are four input channels of one tap, the lanes of a warp lie along them (opaque to the compiler, so that
+        // it keeps no addresses in registers during the main loop)
+        int m = m0;
+        asm volatile("" : "+r"(m));
+        const int tap = tap0 + m / CIB, ci = c0 + m % CIB;
+        if (tap >= 27) continue;
+        float* dst = P.partial + (((ll) blockIdx.x * 27 + tap) * P.cout + o0 + n_off) * P.cin + ci;
+#pragma unroll
+        for (int n = 0; n < TN; ++n, dst += P.cin) {
+            if (o0 + n_off + n >= P.cout) break;
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { const float2 pair = unpack2(IN_REGISTERS ? done[IN_REGISTERS ? i : 0][IN_REGISTERS ? n / 2 : 0] : acc[i][n / 2]); v[i] = n & 1 ? pair.y : pair.x; }
+            if (!IN_REGISTERS && s0 > 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (ci + i < P.cin) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + i), "f"(v[i]) : "memory");
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (ci + i < P.cin) dst[i] = v[i];
             }
         }
-        if (++slot == RING) slot = 0;
-    }
+    } while (s < total);
     cp_async_wait<0>();
-
-    // a thread's four rows are four input channels of one tap, the lanes of a warp lie along them
-    const int tap = tap0 + m0 / CIB, ci = c0 + m0 % CIB;
-    if (tap < 27) {
-        float* dst = P.partial + ((ll) blockIdx.x * 27 + tap) * P.cin * P.cout + ci;
-#pragma unroll
-        for (int n = 0; n < TN; ++n) {
-            const int co = o0 + n_off + n;
-            if (co >= P.cout) continue;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 pair = unpack2(acc[i][n / 2]);
-                if (ci + i < P.cin) dst[(ll) co * P.cin + i] = n & 1 ? pair.y : pair.x;
-            }
-        }
-    }
 }
 
 // grad_weights[slot][filter][tap] = (+=) the block sums [range][tap][filter] of the slot's ranges, filter = co * cin + ci.  Block = 32
@@ -553,6 +583,10 @@ inline DwGeom dw_geometry(int cin, int cout) {
     return g;
 }
 
+// ring slots (16 locations) per chain of a block, for a level of `len` locations and tiles of nt output channels.  In registers: 128
+// locations.  In the workspace, where the end of a chain writes the block's sums: at least 512 locations, and 1 / 256 of the level.
+inline int dw_flush_slots(ll len, int nt) { return nt <= 16 ? 128 / KS : (int) std::max<ll>(512 / KS, (len / 256 + KS - 1) / KS); }
+
 // ranges of the whole launch: enough blocks for four waves of three per SM, bounded by 64 Mi partial sums
 inline int dw_max_ranges(int cin, int cout) {
     const DwGeom g = dw_geometry(cin, cout);
@@ -592,7 +626,7 @@ int run_dw(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* xro
     sr.n = 0;
     P.range_first[0] = 0;
     for (int i = 0; i < P.n_segs; ++i) {
-        P.seg_begin[i] = segs[i].begin; P.seg_end[i] = segs[i].end;
+        P.seg_begin[i] = segs[i].begin; P.seg_end[i] = segs[i].end; P.seg_flush[i] = dw_flush_slots(segs[i].end - segs[i].begin, g.nt);
         P.range_first[i + 1] = P.range_first[i] + (int) (((segs[i].end - segs[i].begin + DW_UNIT - 1) / DW_UNIT + per_block - 1) / per_block);
         // levels are listed coarse to fine, so those that share a slot (the last one) are neighbours
         if (sr.n == 0 || sr.slot[sr.n - 1] != segs[i].slot) { sr.first[sr.n] = P.range_first[i]; sr.slot[sr.n++] = segs[i].slot; }

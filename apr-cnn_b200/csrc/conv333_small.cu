@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable seg
 // gathered values and the 32 dO values of KP locations are staged in shared memory (all table entries of a step, then all values, are
 // requested before any is used: the staging is bound by their latency); a thread owns a 4 x 4
 // tile of (tap, ci) x co products; the 4 thread groups of a block take different quarters of every staged
-// step and are combined in a fixed order.  partial[range][tap][co][ci].
+// step and are combined in a fixed order.  The products of a quarter (8 or 16 locations) are summed before they are added to the
+// thread's sums: short chains of additions whatever the length of the range.  partial[range][tap][co][ci].
 struct SmallRanges { int n; ll begin[MAX_SEGS], end[MAX_SEGS], len[MAX_SEGS]; int first[MAX_SEGS + 1]; };
 
 template<int CIN>
@@ -178,19 +179,26 @@ __global__ void __launch_bounds__(256) conv333_small_dw_kernel(SmallRanges rg, c
 #pragma unroll
         for (int i = 0; i < NG; ++i) { const int e = threadIdx.x + i * 256, k = e % KP, co = e / KP; gs[k][co >> 2].a[co & 3] = gv[i]; }
         __syncthreads();
+#pragma unroll
+        for (int ps = 0; ps < PASSES; ++ps) {
+            if (ps * 8 + rq >= RQ) continue;
+            float part[4][4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) part[a][b] = 0.f;
 #pragma unroll 4
-        for (int k = grp * (KP / 4); k < (grp + 1) * (KP / 4); ++k) {
-            const F4 g = gs[k][cq];
+            for (int k = grp * (KP / 4); k < (grp + 1) * (KP / 4); ++k) {
+                const F4 g = gs[k][cq], x = xs[k][ps * 8 + rq];
 #pragma unroll
-            for (int ps = 0; ps < PASSES; ++ps) {
-                if (ps * 8 + rq < RQ) {
-                    const F4 x = xs[k][ps * 8 + rq];
+                for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int a = 0; a < 4; ++a)
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) acc[ps][a][b] = fmaf(x.a[a], g.a[b], acc[ps][a][b]);
-                }
+                    for (int b = 0; b < 4; ++b) part[a][b] = fmaf(x.a[a], g.a[b], part[a][b]);
             }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[ps][a][b] += part[a][b];
         }
         __syncthreads();
     }
