@@ -498,6 +498,7 @@ int conv333_bwd_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, con
 
 #define CONV_CHECKS()                                                                                           \
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0, "bad argument");                \
+    APRNET_DEVICE_CHECK(a);                                                                                     \
     APRNET_ARG_CHECK(a->cml(dl) <= a->meta.level_max, "level_delta out of range");                              \
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), \
                      "leading dimension too small")

@@ -35,6 +35,7 @@ int pack_input(const aprnet_apr* a, int dl, int precision, int cin, const float*
 int forward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const float* in, ll ld_in, const float* w, const float* bias,
                  float* out, ll ld_out, float* tree, ll ld_tree, bool tree_valid, void* workspace, cudaStream_t st) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && in && w && out && tree && workspace, "bad argument");
+    APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), "leading dimension too small");
     int rc = tree_valid ? APRNET_OK : aprnet_fill_tree_mean_forward(a, dl, APRNET_F32, cin, in, ld_in, tree, ld_tree, st);
     if (rc) return rc;
@@ -49,6 +50,7 @@ int forward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int sl
 int backward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const void* rows, const float* gout, ll ld_out, const float* w,
                   float* gin, ll ld_in, float* gw, int accumulate, float* gtree, ll ld_tree, float* partial, void* ws, bool fold_tree, cudaStream_t st) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && gout && (gin || gw) && (!gin || (w && gtree)) && ws && (!gw || (rows && partial)), "bad argument");
+    APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_out >= a->number_parts(dl) && (!gin || (ld_in >= a->number_parts(dl) && ld_tree >= a->tree_size(dl))), "leading dimension too small");
     const ll n = a->number_parts(dl);
     const int gpad = aprnet_tc_pad(cout);
@@ -118,6 +120,7 @@ extern "C" int aprnet_conv333_rows_forward(aprnet_apr* a, int dl, int precision,
 extern "C" int aprnet_conv333_rows_pack(aprnet_apr* a, int dl, int precision, int cin, const float* in, int64_t ld_in, float* tree, int64_t ld_tree, int tree_is_valid,
                                         void* rows, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && in && tree && rows && precision_ok(precision), "bad argument");
+    APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), "leading dimension too small");
     const int rc = tree_is_valid ? APRNET_OK : aprnet_fill_tree_mean_forward(a, dl, APRNET_F32, cin, in, ld_in, tree, ld_tree, stream);
     return rc ? rc : pack_input(a, dl, precision, cin, in, ld_in, tree, ld_tree, rows, (cudaStream_t) stream);

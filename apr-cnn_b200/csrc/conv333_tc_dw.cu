@@ -310,6 +310,7 @@ extern "C" int64_t aprnet_conv333_tc_dw_partial_elems(int cin, int cout) {
 int aprnet_tc_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* xrows, int xpad, const void* grows, int gpad, float* gw, int accumulate,
                                float* partial, cudaStream_t st) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && xrows && grows && gw && partial, "bad argument");
+    APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(xpad % 16 == 0 && gpad % 16 == 0 && xpad >= cin && gpad >= cout, "packed row widths must be multiples of 16");
     const RunPlan* rp = aprnet_get_run_plan(a, dl, st);
     if (!rp) return APRNET_ERR_CUDA;

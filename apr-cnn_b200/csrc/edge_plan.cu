@@ -338,6 +338,7 @@ EdgePlan* aprnet_get_edge_plan(aprnet_apr* a, int dl, cudaStream_t st) {
 // Builds (once; cached) the cross-level edge lists of a level delta.  Allocates; call it up front.
 extern "C" int aprnet_edge_plan_build(aprnet_apr* a, int dl, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl), "bad handle or level_delta");
+    APRNET_DEVICE_CHECK(a);
     return aprnet_get_edge_plan(a, dl, (cudaStream_t) stream) ? APRNET_OK : APRNET_ERR_CUDA;
 }
 
@@ -358,6 +359,7 @@ int aprnet_cross_level_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, c
                           long long ld_in, float* gtree, long long ld_tree, void* wp_ws, void* edge_ws, long long edge_ws_bytes, void* stream,
                           bool tree_adjoint) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && grows && w && gin && gtree && wp_ws && edge_ws, "bad argument");
+    APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(gpad == aprnet_tc_pad(cout), "packed row width does not match the padded channel count");
     cudaStream_t st = (cudaStream_t) stream;
     EdgePlan* ep = aprnet_get_edge_plan(a, dl, st);
@@ -404,6 +406,7 @@ extern "C" int aprnet_conv333_backward_input_cross_level_tc(aprnet_apr* a, int d
                                                             int64_t ld_in, float* gtree, int64_t ld_tree, void* wp_ws,
                                                             void* edge_ws, int64_t edge_ws_bytes, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && w && wp_ws, "bad argument");
+    APRNET_DEVICE_CHECK(a);
     const int rc = aprnet_tc_pack_weights(a, dl, w, slots, cin, cout, 1, wp_ws, (cudaStream_t) stream);
     return rc ? rc : aprnet_cross_level_tc(a, dl, cin, cout, slots, grows, gpad, w, gin, ld_in, gtree, ld_tree, wp_ws, edge_ws, edge_ws_bytes, stream, true);
 }

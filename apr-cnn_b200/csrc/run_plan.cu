@@ -212,5 +212,6 @@ int aprnet_fill_nbr_table(aprnet_apr* a, int dl, int32_t* nbr, ll n, cudaStream_
 // Builds (once; cached) the run plan of a level delta.  Allocates; call it up front.
 extern "C" int aprnet_run_plan_build(aprnet_apr* a, int dl, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl), "bad handle or level_delta");
+    APRNET_DEVICE_CHECK(a);
     return aprnet_get_run_plan(a, dl, (cudaStream_t) stream) ? APRNET_OK : APRNET_ERR_CUDA;
 }

@@ -1,0 +1,64 @@
+"""Every convolution entry point of the C ABI checks that the current device is the handle's before it launches or copies anything.
+
+Runs only without a GPU: there the check is the one call that fails with "no current CUDA device"; an entry point that got past it
+would report its first launch or copy instead.  (On a GPU the same calls would reach kernels with the made-up pointers.)"""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "apr-cnn_b200")
+NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    if torch.cuda.is_available():
+        pytest.skip("with a GPU a missing check would launch kernels on made-up pointers")
+    if not os.path.exists(NVCC):
+        pytest.skip("needs nvcc")
+    out = str(tmp_path_factory.mktemp("dc") / "helper.so")
+    subprocess.check_call([NVCC, "-shared", "-Xcompiler", "-fPIC", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
+                           os.path.join(ROOT, "tests", "device_check_helper.cu"), "-o", out])
+    lib = C.CDLL(os.path.join(PKG, "libaprnet_b200.so"), mode=C.RTLD_GLOBAL)
+    lib.aprnet_last_error.restype = C.c_char_p
+    helper = C.CDLL(out)
+    helper.fake_handle.restype = C.c_void_p
+    return lib, C.c_void_p(helper.fake_handle(3))
+
+
+p, n = C.c_void_p(0x1000), C.c_int64(64)          # never dereferenced on the host
+i = C.c_int
+CALLS = {
+    "aprnet_plan_build": (i(0), None),
+    "aprnet_run_plan_build": (i(0), None),
+    "aprnet_edge_plan_build": (i(0), None),
+    "aprnet_conv333_forward": (i(0), i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, None),
+    "aprnet_conv333_forward_pretree": (i(0), i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, None),
+    "aprnet_conv333_backward_input": (i(0), i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, None),
+    "aprnet_conv333_backward_input_pretree": (i(0), i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, None),
+    "aprnet_conv333_backward_input_cross_level": (i(0), i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, None),
+    "aprnet_conv333_backward_weights": (i(0), i(0), i(8), i(8), i(1), p, n, p, n, p, n, p, p, None),
+    "aprnet_conv333_rows_forward": (i(0), i(0), i(8), i(8), i(1), p, n, p, None, p, n, p, n, i(1), p, None),
+    "aprnet_conv333_rows_pack": (i(0), i(1), i(8), p, n, p, n, i(1), p, None),
+    "aprnet_conv333_rows_backward": (i(0), i(1), i(8), i(8), i(1), p, p, n, p, p, n, p, i(0), p, n, i(1), p, p, None),
+    "aprnet_conv333_forward_tc": (i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, p, None),
+    "aprnet_conv333_forward_tc_pretree": (i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, p, None),
+    "aprnet_conv333_backward_tc": (i(0), i(8), i(8), i(1), p, n, p, n, p, p, p, p, i(1), p, n, p, p, None),
+    "aprnet_conv333_backward_tc_rows": (i(0), i(8), i(8), i(1), p, p, n, p, p, n, p, p, n, p, p, None),
+    "aprnet_conv333_backward_tc_rows_pretree": (i(0), i(8), i(8), i(1), p, p, n, p, p, n, p, p, n, p, p, None),
+    "aprnet_conv333_backward_weights_tc": (i(0), i(8), i(8), i(1), p, i(16), p, i(16), p, p, None),
+    "aprnet_conv333_backward_input_cross_level_tc": (i(0), i(8), i(8), i(1), p, i(16), p, p, n, p, n, p, p, n, None),
+    "aprnet_conv111_forward": (i(0), i(0), i(8), i(8), i(1), p, n, p, p, n, None),
+    "aprnet_conv111_forward_tc": (i(0), i(8), i(8), i(1), p, n, p, p, n, None),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CALLS))
+def test_refused_before_anything_is_launched(lib, name):
+    lib, handle = lib
+    assert getattr(lib, name)(handle, *CALLS[name]) < 0
+    assert lib.aprnet_last_error() == b"no current CUDA device"
