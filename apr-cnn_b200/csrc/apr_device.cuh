@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 #include <map>
+#include <algorithm>
 #include <cuda_runtime.h>
 #include "../../include/aprnet_b200.h"
 
@@ -53,9 +54,23 @@ struct EdgePlan {
     int32_t* vnbr = nullptr;       // [27][n_active]
     std::vector<ActiveSeg> segs;   // by level, in active[] order
     // coarse map for splitting the work when the virtual rows do not fit the workspace: chunk k starts at
-    // active index chunk_a[k] and virtual row chunk_v[k]; chunks hold about VROW_GRANULE rows
+    // active index chunk_a[k] and virtual row chunk_v[k]; a chunk holds at most APRNET_VROW_CHUNK rows
     std::vector<long long> chunk_a, chunk_v;
 };
+
+// A chunk ends with the target that reaches the granule, which adds at most 27 rows.  The workspace of the virtual rows is bounded by
+// 8 GiB, but never smaller than one chunk, whatever the width of a row; one pass takes as many chunks as fit.
+constexpr long long APRNET_VROW_GRANULE = 64ll << 10, APRNET_VROW_CHUNK = APRNET_VROW_GRANULE + 27;
+inline long long aprnet_vrow_workspace_bytes(long long n_vrows, long long row_bytes) {
+    const long long cap = std::max(8ll << 30, (APRNET_VROW_CHUNK + 2) * row_bytes);
+    return std::max<long long>(256, std::min(cap, (n_vrows + 2) * row_bytes));
+}
+// first chunk that no longer fits a pass of cap_rows rows from chunk k0 on
+inline int aprnet_vrow_pass_end(const std::vector<long long>& chunk_v, int k0, long long cap_rows) {
+    int k1 = k0 + 1;
+    while (k1 + 1 < (int) chunk_v.size() && chunk_v[k1 + 1] - chunk_v[k0] <= cap_rows) ++k1;
+    return k1;
+}
 
 // Output locations of a level delta in runs along y (run_plan.cu): slot s is a cell of its level, loc[s] the location it holds
 // (-1: none), src[d][s] what fills the cell (dz, dx) = (d / 3 - 1, d % 3 - 1) away (encoded like the neighbour table).

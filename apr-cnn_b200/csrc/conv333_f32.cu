@@ -663,8 +663,7 @@ int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* 
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_bwd_cross_pull:ci%d:co%d:dl%d", cin, cout, dl);
     for (int k0 = 0, k1; k0 < nk; k0 = k1) {
-        k1 = k0 + 1;
-        while (k1 < nk && ep->chunk_v[k1 + 1] - ep->chunk_v[k0] <= cap_rows) ++k1;
+        k1 = aprnet_vrow_pass_end(ep->chunk_v, k0, cap_rows);
         const ll v0 = ep->chunk_v[k0], v1 = ep->chunk_v[k1], a0 = ep->chunk_a[k0], a1 = ep->chunk_a[k1];
         if (v1 - v0 > cap_rows) { aprnet_set_error("edge workspace too small for %lld virtual rows", v1 - v0); return APRNET_ERR_ARG; }
         if (v1 > v0) {
@@ -691,10 +690,8 @@ int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* 
 }
 
 inline size_t edge_bytes(const aprnet_apr* a, int dl, int cout) {
-    const ll cap = 8ll << 30, row = (ll) pad4(cout) * 4;      // bounds the sums' workspace; smaller = more passes
     const auto it = a->edge_plans.find(dl);
-    const ll rows = it != a->edge_plans.end() ? it->second.n_vrows + 2 : 27 * a->number_parts(dl) + 2;
-    return align256((size_t) std::max<ll>(256, std::min(cap, rows * row)));
+    return align256((size_t) aprnet_vrow_workspace_bytes(it != a->edge_plans.end() ? it->second.n_vrows : 27 * a->number_parts(dl), (ll) pad4(cout) * 4));
 }
 
 } // namespace

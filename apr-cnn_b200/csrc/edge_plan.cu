@@ -124,13 +124,14 @@ __global__ void vrow_fill_kernel(const int32_t* __restrict__ active, ll n_active
     });
 }
 
-// out[k] = first index i of sorted[0, n) with sorted[i] >= key[k]
-__global__ void lower_bound_kernel(const int32_t* __restrict__ sorted, ll n, const ll* __restrict__ key, int nkeys, ll* __restrict__ out) {
+// out[k] = first index i of sorted[0, n) with sorted[i] >= key[k]; value (may be null): sorted[out[k]], readable up to sorted[n]
+__global__ void lower_bound_kernel(const int32_t* __restrict__ sorted, ll n, const ll* __restrict__ key, int nkeys, ll* __restrict__ out, ll* __restrict__ value) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nkeys) return;
     ll lo = 0, hi = n;
     while (lo < hi) { const ll m = (lo + hi) >> 1; if ((ll) sorted[m] < key[k]) lo = m + 1; else hi = m; }
     out[k] = lo;
+    if (value) value[k] = sorted[lo];
 }
 
 // pass 1: thread = (VPT consecutive virtual rows, 8-channel chunk); sums the dO rows of each row's locations in
@@ -180,8 +181,6 @@ __global__ void __launch_bounds__(256) vrow_reduce_kernel(const int32_t* __restr
         *reinterpret_cast<uint4*>(out + (vb + u - v0) * gpad + c * 8) = *reinterpret_cast<const uint4*>(o);
     }
 }
-
-constexpr ll VROW_GRANULE = 4ll << 20;      // virtual rows per entry of the chunk map
 
 template<typename T>
 int dev_alloc(T** p, size_t n, long long* bytes, cudaStream_t st) {
@@ -284,12 +283,12 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
     }
     key_h.push_back(NT); key_level.push_back(-1);
     const int nkeys = (int) key_h.size();
-    const int nchunk = (int) (n_vrows / VROW_GRANULE) + 1;
-    EP_ALLOC(keys, std::max(nkeys, nchunk + 1));
-    EP_ALLOC(found, std::max(nkeys, nchunk + 1));
-    std::vector<ll> found_h(std::max(nkeys, nchunk + 1));
+    const int nchunk = (int) (n_vrows / APRNET_VROW_GRANULE) + 1, nk = std::max(nkeys, nchunk + 1);
+    EP_ALLOC(keys, nk);
+    EP_ALLOC(found, 2 * nk);                                  // indices, values
+    std::vector<ll> found_h(2 * nk);
     EP_CHECK(cudaMemcpyAsync(keys, key_h.data(), nkeys * sizeof(ll), cudaMemcpyHostToDevice, st));
-    lower_bound_kernel<<<1, 64, 0, st>>>(ep.active, n_active, keys, nkeys, found);
+    lower_bound_kernel<<<1, 64, 0, st>>>(ep.active, n_active, keys, nkeys, found, nullptr);
     EP_CHECK(cudaMemcpyAsync(found_h.data(), found, nkeys * sizeof(ll), cudaMemcpyDeviceToHost, st));
     EP_CHECK(cudaStreamSynchronize(st));
     ep.segs.clear();
@@ -299,21 +298,17 @@ static int build_edge_plan(aprnet_apr* a, int dl, const AprPlan* plan, EdgePlan&
         else if (sg.end > sg.begin) { aprnet_set_error("edge plan: edges from level %d outside [%d, %d]", sg.location_level, a->meta.level_min, cml); cleanup(); return APRNET_ERR_CUDA; }
     }
     std::vector<ll> ckey(nchunk + 1);
-    for (int k = 0; k < nchunk; ++k) ckey[k] = (ll) k * VROW_GRANULE;
+    for (int k = 0; k < nchunk; ++k) ckey[k] = (ll) k * APRNET_VROW_GRANULE;
     ckey[nchunk] = (ll) n_vrows + 1;        // beyond the last value: maps to n_active
     EP_CHECK(cudaMemcpyAsync(keys, ckey.data(), (nchunk + 1) * sizeof(ll), cudaMemcpyHostToDevice, st));
-    lower_bound_kernel<<<aprnet_ceil_div(nchunk + 1, 64), 64, 0, st>>>(vfirst, n_active, keys, nchunk + 1, found);
-    EP_CHECK(cudaMemcpyAsync(found_h.data(), found, (nchunk + 1) * sizeof(ll), cudaMemcpyDeviceToHost, st));
+    lower_bound_kernel<<<aprnet_ceil_div(nchunk + 1, 64), 64, 0, st>>>(vfirst, n_active, keys, nchunk + 1, found, found + nk);
+    EP_CHECK(cudaMemcpyAsync(found_h.data(), found, 2 * nk * sizeof(ll), cudaMemcpyDeviceToHost, st));
     EP_CHECK(cudaStreamSynchronize(st));
-    std::vector<int32_t> vf(nchunk + 1);
     ep.chunk_a.clear(); ep.chunk_v.clear();
     for (int k = 0; k <= nchunk; ++k) {
-        const ll ca = std::min<ll>(found_h[k], n_active);
+        const ll ca = found_h[k];
         if (!ep.chunk_a.empty() && ep.chunk_a.back() == ca) continue;
-        int32_t v = 0;
-        EP_CHECK(cudaMemcpyAsync(&v, vfirst + ca, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        EP_CHECK(cudaStreamSynchronize(st));
-        ep.chunk_a.push_back(ca); ep.chunk_v.push_back(v);
+        ep.chunk_a.push_back(ca); ep.chunk_v.push_back(found_h[nk + k]);
     }
     if (ep.chunk_a.back() != n_active) { ep.chunk_a.push_back(n_active); ep.chunk_v.push_back(n_vrows); }
     EP_CHECK(cudaGetLastError());
@@ -344,11 +339,8 @@ extern "C" int aprnet_edge_plan_build(aprnet_apr* a, int dl, void* stream) {
 
 extern "C" int64_t aprnet_edge_workspace_bytes(const aprnet_apr* a, int dl, int cout) {
     if (!a || !a->valid_dl(dl)) return -1;
-    const ll cap = 8ll << 30;     // bounds the virtual-row workspace; smaller = more passes
-    const ll row = (ll) aprnet_tc_pad(cout) * 2;
-    auto it = a->edge_plans.find(dl);
-    const ll rows = it != a->edge_plans.end() ? it->second.n_vrows + 2 : 27 * a->number_parts(dl) + 2;
-    return (int64_t) std::max<ll>(256, std::min(cap, rows * row));
+    const auto it = a->edge_plans.find(dl);
+    return (int64_t) aprnet_vrow_workspace_bytes(it != a->edge_plans.end() ? it->second.n_vrows : 27 * a->number_parts(dl), (ll) aprnet_tc_pad(cout) * 2);
 }
 
 // Cross-level part of the input gradient (added to grad_input, which holds the same-level part, and to
@@ -383,8 +375,7 @@ int aprnet_cross_level_tc(aprnet_apr* a, int dl, int cin, int cout, int slots, c
         const int nk = (int) ep->chunk_a.size() - 1;
         int k0 = 0;
         while (k0 < nk) {
-            int k1 = k0 + 1;
-            while (k1 < nk && ep->chunk_v[k1 + 1] - ep->chunk_v[k0] <= cap_rows) ++k1;
+            const int k1 = aprnet_vrow_pass_end(ep->chunk_v, k0, cap_rows);
             const ll v0 = ep->chunk_v[k0], v1 = ep->chunk_v[k1], a0 = ep->chunk_a[k0], a1 = ep->chunk_a[k1];
             if (v1 - v0 > cap_rows) { aprnet_set_error("edge workspace too small for %lld virtual rows", v1 - v0); return APRNET_ERR_ARG; }
             if (v1 > v0) {

@@ -1,7 +1,10 @@
-"""Every convolution entry point of the C ABI checks that the current device is the handle's before it launches or copies anything.
+"""Host logic of the C ABI that needs no GPU, with handles and tables that are made up.
 
-Runs only without a GPU: there the check is the one call that fails with "no current CUDA device"; an entry point that got past it
-would report its first launch or copy instead.  (On a GPU the same calls would reach kernels with the made-up pointers.)"""
+Device check: every convolution entry point checks that the current device is the handle's before it launches or copies anything.
+Without a GPU the check is the one call that fails with "no current CUDA device"; an entry point that got past it would report its
+first launch or copy instead.  (On a GPU the same calls would reach kernels with the made-up pointers.)
+
+Cross-level input gradient: the sums per (target, tap) go through a bounded workspace in passes; no width may be refused."""
 import ctypes as C
 import os
 import subprocess
@@ -15,18 +18,23 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 
 @pytest.fixture(scope="module")
-def lib(tmp_path_factory):
-    if torch.cuda.is_available():
-        pytest.skip("with a GPU a missing check would launch kernels on made-up pointers")
+def helper(tmp_path_factory):
     if not os.path.exists(NVCC):
         pytest.skip("needs nvcc")
-    out = str(tmp_path_factory.mktemp("dc") / "helper.so")
+    out = str(tmp_path_factory.mktemp("host") / "helper.so")
     subprocess.check_call([NVCC, "-shared", "-Xcompiler", "-fPIC", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
-                           os.path.join(ROOT, "tests", "device_check_helper.cu"), "-o", out])
-    lib = C.CDLL(os.path.join(PKG, "libaprnet_b200.so"), mode=C.RTLD_GLOBAL)
-    lib.aprnet_last_error.restype = C.c_char_p
+                           os.path.join(ROOT, "tests", "host_helper.cu"), "-o", out])
     helper = C.CDLL(out)
     helper.fake_handle.restype = C.c_void_p
+    helper.vrow_worst_pass.restype = helper.vrow_chunk.restype = C.c_longlong
+    return helper
+
+
+@pytest.fixture(scope="module")
+def lib(helper):
+    lib = C.CDLL(os.path.join(PKG, "libaprnet_b200.so"), mode=C.RTLD_GLOBAL)
+    lib.aprnet_last_error.restype = C.c_char_p
+    lib.aprnet_edge_workspace_bytes.restype = lib.aprnet_conv333_rows_backward_workspace_bytes.restype = C.c_int64
     return lib, C.c_void_p(helper.fake_handle(3))
 
 
@@ -59,6 +67,20 @@ CALLS = {
 
 @pytest.mark.parametrize("name", sorted(CALLS))
 def test_refused_before_anything_is_launched(lib, name):
+    if torch.cuda.is_available():
+        pytest.skip("with a GPU a missing check would launch kernels on made-up pointers")
     lib, handle = lib
     assert getattr(lib, name)(handle, *CALLS[name]) < 0
     assert lib.aprnet_last_error() == b"no current CUDA device"
+
+
+@pytest.mark.parametrize("cout", [1, 64, 500, 512, 1024, 2048, 5000, 65536])
+def test_cross_level_passes_fit_their_workspace(helper, lib, cout):
+    lib, handle = lib
+    for row in ((cout + 3) // 4 * 16, (cout + 15) // 16 * 32):                  # packed rows: fp32, bf16
+        for n in (0, 1, 65535, 65536, 65537, 3 << 20, 4 << 20, (4 << 20) + 1, 40_000_000):
+            assert helper.vrow_worst_pass(C.c_longlong(n), C.c_longlong(row)) <= 0, (row, n)
+    helper.set_vrows(handle, C.c_longlong(40_000_000))
+    # the workspaces that the library reports hold a chunk of the plan at any width
+    assert lib.aprnet_edge_workspace_bytes(handle, 0, cout) >= helper.vrow_chunk() * ((cout + 15) // 16 * 32)
+    assert lib.aprnet_conv333_rows_backward_workspace_bytes(handle, 0, 0, 8, cout, 1, 1) >= helper.vrow_chunk() * ((cout + 3) // 4 * 16)
