@@ -447,7 +447,8 @@ std::vector<torch::Tensor> conv333_backward_pretree(std::vector<APR*>& aprs, tor
         const int mode = bf16 ? APRNET_PREC_BF16 : APRNET_PREC_F32;
         auto rows = bf16 ? kept : conv333_pack(aprs, input, level_delta, mode, tree);
         auto r = conv333_backward_rows(aprs, rows, weights, grad_output, level_delta, mode, need_grad_input, false, ldt);
-        return {r[0], need_grad_input ? r[2] : torch::zeros({nb, cin, ldt}, grad_output.options()), r[1]};
+        if (need_grad_input) return {r[0], r[2], r[1]};
+        return {bf16 ? r[0] : torch::zeros({nb, cin, n}, grad_output.options()), torch::zeros({nb, cin, ldt}, grad_output.options()), r[1]};
     }
     void* st = stream_of(grad_output);
     auto grad_tree = torch::zeros({nb, cin, ldt}, grad_output.options());

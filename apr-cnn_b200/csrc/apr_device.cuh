@@ -168,6 +168,9 @@ extern "C" int aprnet_conv333_backward_input_cross_level(aprnet_apr* a, int dl, 
                                                          const void* gout, int64_t ld_out, const void* w, void* gin,
                                                          int64_t ld_in, void* gtree, int64_t ld_tree, void* stream);
 
+// cross-level part by atomic adds (fp32; grad_tree is zero-filled and, with tree_adjoint, folded into grad_input)
+int aprnet_cross_level_scatter(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* gout, long long ld_out, const float* w, float* gin, long long ld_in,
+                               float* gtree, long long ld_tree, bool tree_adjoint, cudaStream_t st);
 const RunPlan* aprnet_get_run_plan(aprnet_apr* apr, int dl, cudaStream_t stream);                // nullptr on failure
 EdgePlan* aprnet_get_edge_plan(aprnet_apr* apr, int dl, cudaStream_t stream);
 void aprnet_free_edge_plan(EdgePlan& ep, cudaStream_t st);

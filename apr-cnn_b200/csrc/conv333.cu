@@ -601,3 +601,8 @@ extern "C" int aprnet_conv333_backward_input_cross_level(aprnet_apr* a, int dl, 
     DISPATCH(dtype, conv333_bwd_input<float>(a, dl, cin, cout, slots, (const float*) gout, ld_out, (const float*) w, (float*) gin, ld_in, (float*) gtree, ld_tree, st, 1),
              conv333_bwd_input<double>(a, dl, cin, cout, slots, (const double*) gout, ld_out, (const double*) w, (double*) gin, ld_in, (double*) gtree, ld_tree, st, 1));
 }
+
+int aprnet_cross_level_scatter(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* gout, ll ld_out, const float* w, float* gin, ll ld_in,
+                               float* gtree, ll ld_tree, bool tree_adjoint, cudaStream_t st) {
+    return conv333_bwd_input<float>(a, dl, cin, cout, slots, gout, ld_out, w, gin, ld_in, gtree, ld_tree, st, 1, tree_adjoint);
+}

@@ -790,8 +790,7 @@ int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slot
     if (27 * n + 1 >= (1ll << 31)) {
         // more than 79.5 M locations: the 32-bit edge ids of the edge plan run out; the cross-level part is scattered with
         // atomic adds instead (correct, but the summation order is no longer fixed)
-        if (!tree_adjoint) { aprnet_set_error("the split backward form needs the edge plan, which supports up to 79.5 M locations"); return APRNET_ERR_UNSUPPORTED; }
-        return aprnet_conv333_backward_input_cross_level(a, dl, APRNET_F32, cin, cout, slots, gout, ld_out, w, gin, ld_in, gtree, ld_tree, st);
+        return aprnet_cross_level_scatter(a, dl, cin, cout, slots, gout, ld_out, w, gin, ld_in, gtree, ld_tree, tree_adjoint, st);
     }
     if (ts > 0) APRNET_CUDA_CHECK(cudaMemset2DAsync(gtree, (size_t) ld_tree * sizeof(float), 0, (size_t) ts * sizeof(float), (size_t) cin, st));
     if ((rc = run_cross(a, dl, cin, cout, slots, grows, gin, ld_in, gtree, ld_tree, wp, vrows, (ll) edge_bytes(a, dl, cout), st))) return rc;
