@@ -283,10 +283,18 @@ int copy_rows(T* dst, ll ld_dst, const T* src, ll ld_src, ll count, int C, cudaS
     return APRNET_OK;
 }
 
-// Fills the tree bottom-up.  A level of more than COARSE_NODES nodes is a launch of its own; the levels above the first one
-// with fewer (the coarser, the fewer) share one launch: a launch costs the host 4 us, which is what small structures wait for, and
-// the device about 2 us; inside the shared one a level costs about 2 us per CLUSTER * COARSE_TPB nodes.
+// Fills the tree bottom-up.  The coarsest levels, as long as they have at most COARSE_NODES nodes each, share one launch: a launch
+// costs the host 4 us, which is what small structures wait for, and the device about 2 us; inside the shared one a level costs about
+// 2 us per CLUSTER * COARSE_TPB nodes.  Every finer level is a launch of its own, also one with few nodes: where fine cells are
+// rare, a level below it has many, and one cluster would walk them with 8 of the SMs.
 constexpr ll COARSE_NODES = 2 * CLUSTER * COARSE_TPB;
+
+// last level of the shared launch (level_min - 2: none)
+int last_coarse_level(const LevelMeta& m, int cml) {
+    int l = m.level_min - 1;
+    while (l <= cml - 1 && m.tlvl_begin[l + 1] - m.tlvl_begin[l] <= COARSE_NODES) ++l;
+    return l - 1;
+}
 
 template<typename T, bool MAX>
 int fill_tree(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree, ll ld_tree, const char* pname, cudaStream_t st) {
@@ -297,11 +305,12 @@ int fill_tree(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree
     const unsigned gx = (unsigned) aprnet_ceil_div(C, CH);
     LevelList coarse;
     coarse.n = 0;
+    const int last = last_coarse_level(m, cml);
     for (int lp = cml - 1; lp >= m.level_min - 1; --lp) {
         const ll tb = m.tlvl_begin[lp], te = m.tlvl_begin[lp + 1];
         if (te <= tb) continue;
         const int use_up = (dl > 0 && lp + 1 == cml) ? 1 : 0;
-        if (te - tb <= COARSE_NODES || coarse.n > 0) {
+        if (lp <= last) {
             coarse.begin[coarse.n] = tb; coarse.end[coarse.n] = te; coarse.use_up[coarse.n] = use_up;
             ++coarse.n;
             continue;
