@@ -44,8 +44,16 @@ __device__ __forceinline__ void restrict_table(int S, int k, T (*coef)[CROW]) {
     }
 }
 
+// The grid of an extra slot is at least twice coarser, so along an axis the middle fine tap lies in the middle coarse tap and an outer
+// one in the middle and in its own: 125 of the 729 pairs overlap.  The others are left out, not multiplied by zero: a value that is not
+// finite stays in the taps that it belongs to.
+__host__ __device__ constexpr bool restrict_axis(int fine, int coarse) { return coarse == 1 || (fine != 1 && fine == coarse); }
+__host__ __device__ constexpr bool restrict_overlaps(int fine, int coarse) {
+    return restrict_axis(fine / 9, coarse / 9) && restrict_axis(fine / 3 % 3, coarse / 3 % 3) && restrict_axis(fine % 3, coarse % 3);
+}
+
 // grid (filter blocks, level slots).  A thread holds the 27 values of its filter and adds the products of a result in ascending order
-// of the fine taps; the coefficients are broadcast reads.  (A coefficient of zero leaves the sum as it is.)
+// of the fine taps; the coefficients are broadcast reads.
 template<typename T>
 __global__ void __launch_bounds__(FB) restrict333_forward_kernel(int S, ll filters, const T* __restrict__ src, T* __restrict__ dst) {
     __shared__ T stage[FB * 27];
@@ -67,11 +75,11 @@ __global__ void __launch_bounds__(FB) restrict333_forward_kernel(int S, ll filte
     T fine[27];
 #pragma unroll
     for (int t = 0; t < 27; ++t) fine[t] = stage[threadIdx.x * 27 + t];
-#pragma unroll 3
+#pragma unroll
     for (int o = 0; o < 27; ++o) {
         T acc = 0;
 #pragma unroll
-        for (int t = 0; t < 27; ++t) acc += coef[o][t] * fine[t];
+        for (int t = 0; t < 27; ++t) if (restrict_overlaps(t, o)) acc += coef[o][t] * fine[t];
         stage[threadIdx.x * 27 + o] = acc;             // this thread's own values
     }
     __syncthreads();
@@ -113,11 +121,11 @@ __global__ void __launch_bounds__(FB) restrict333_backward_kernel(int S, int L, 
         restrict_table<T>(S, k, coef);
         __syncthreads();
         if (k + 1 < L) request(k + 1);
-#pragma unroll 3
+#pragma unroll
         for (int o = 0; o < 27; ++o) {
             const T c = stage[threadIdx.x * 27 + o];
 #pragma unroll
-            for (int t = 0; t < 27; ++t) acc[t] += coef[o][t] * c;
+            for (int t = 0; t < 27; ++t) if (restrict_overlaps(t, o)) acc[t] += coef[o][t] * c;
         }
     }
     __syncthreads();
