@@ -17,6 +17,14 @@ from _pyaprwrapper.aprnet.cuda import (conv111_backward, conv111_forward, conv33
                                        restrict_kernel333_backward, restrict_kernel333_forward)
 
 
+def _kernel_bias(bias, inputs, weights):
+    """The bias as the kernels add it (contiguous, one value per output channel, the features' type and device); None where torch has
+    to add it afterwards by its own rules (another type, a broadcast value) or there is none."""
+    if bias is None or bias.dtype != inputs.dtype or bias.device != inputs.device or bias.numel() != weights.shape[1]:
+        return None
+    return bias.contiguous()
+
+
 class Conv333Function(Function):
     """3x3x3 stencil: the given stencils are expanded to one per level, then applied per level."""
 
@@ -32,9 +40,10 @@ class Conv333Function(Function):
         ctx.packed = inputs.dtype == torch.float32
         if ctx.packed:
             ctx.precision = precision or get_conv_precision()
-            out, rows = conv333_forward_keep_rows(APRPtrVector(aprs), inputs, expanded, level_deltas, ctx.precision, bias)
+            fused = _kernel_bias(bias, inputs, weights)
+            out, rows = conv333_forward_keep_rows(APRPtrVector(aprs), inputs, expanded, level_deltas, ctx.precision, fused)
             ctx.save_for_backward(expanded, bias, level_deltas.clone(), rows)
-            return out
+            return out if bias is None or fused is not None else out + bias.view(1, -1, 1)
         # float64: the tree means computed by the forward pass are kept (1/7 of the input's size) so that the
         # backward pass does not have to fill the tree again
         out, tree = conv333_forward_keep_tree(APRPtrVector(aprs), inputs, expanded, level_deltas)
@@ -68,7 +77,9 @@ class Conv111Function(Function):
         ctx.aprs = aprs
         ctx.precision = precision or ""
         ctx.save_for_backward(inputs, weights, bias, level_deltas.clone())
-        return conv111_forward(APRPtrVector(aprs), inputs, weights, level_deltas, ctx.precision, bias)
+        fused = _kernel_bias(bias, inputs, weights)
+        out = conv111_forward(APRPtrVector(aprs), inputs, weights, level_deltas, ctx.precision, fused)
+        return out if bias is None or fused is not None else out + bias.view(1, -1, 1)
 
     @staticmethod
     def backward(ctx, grad_output):
