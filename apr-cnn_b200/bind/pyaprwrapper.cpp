@@ -331,15 +331,16 @@ std::vector<torch::Tensor> conv333_forward_keep_tree(std::vector<APR*>& aprs, to
 }
 
 // float32 forward that keeps the packed rows of the input (particles, tree means, zero row) for the backward pass instead
-// of the input and the tree means: returns {output, rows (B, bytes) uint8}.  bias: added to the output, padding included.
+// of the input and the tree means: returns {output, rows (B, bytes) uint8}.  bias: added to the output, padding included.  Without
+// `keep` the rows are one item's scratch and an empty tensor is returned.
 std::vector<torch::Tensor> conv333_forward_keep_rows(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights, torch::Tensor level_delta,
-                                                     const std::string& precision, c10::optional<torch::Tensor> bias) {
+                                                     const std::string& precision, c10::optional<torch::Tensor> bias, bool keep) {
     CHECK_INPUT(input); CHECK_INPUT(weights);
     check_conv333(input, weights);
     TORCH_CHECK(input.scalar_type() == torch::kFloat32, "the packed-row path takes float32 tensors");
     c10::cuda::CUDAGuard guard(input.device());
-    auto r = conv333_forward_rows(aprs, input, weights, level_delta, resolve_mode(precision), false, true, torch::Tensor(), bias);
-    return {r[0], r[2]};
+    auto r = conv333_forward_rows(aprs, input, weights, level_delta, resolve_mode(precision), false, keep, torch::Tensor(), bias);
+    return {r[0], keep ? r[2] : torch::empty({0, 0}, r[2].options())};
 }
 
 std::vector<torch::Tensor> conv333_backward_with_rows(std::vector<APR*>& aprs, torch::Tensor rows, torch::Tensor weights, torch::Tensor grad_output,
@@ -973,7 +974,7 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
     cuda.def("conv333_forward_keep_tree", &conv333_forward_keep_tree, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "");
     cuda.def("conv333_backward_with_tree", &conv333_backward_with_tree, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "tree"_a, "need_grad_input"_a = true,
              "precision"_a = "");
-    cuda.def("conv333_forward_keep_rows", &conv333_forward_keep_rows, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "bf16", "bias"_a = py::none());
+    cuda.def("conv333_forward_keep_rows", &conv333_forward_keep_rows, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "bf16", "bias"_a = py::none(), "keep"_a = true);
     cuda.def("conv333_backward_with_rows", &conv333_backward_with_rows, "aprs"_a, "rows"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "need_grad_input"_a = true, "precision"_a = "bf16");
     cuda.def("upsample_const_forward", &upsample_const_forward, "aprs"_a, "input"_a, "level_delta"_a);
     cuda.def("upsample_const_backward", &upsample_const_backward, "aprs"_a, "grad_output"_a, "level_delta"_a);

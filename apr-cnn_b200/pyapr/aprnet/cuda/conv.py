@@ -29,7 +29,9 @@ class Conv333Function(Function):
     """3x3x3 stencil: the given stencils are expanded to one per level, then applied per level."""
 
     @staticmethod
-    def forward(ctx, inputs, weights, bias, aprs, level_deltas, precision=None):
+    def forward(ctx, inputs, weights, bias, aprs, level_deltas, precision=None, keep=True):
+        # keep: something for a backward pass is kept (False where no gradient can be wanted: one item's scratch instead of the
+        # packed rows of the whole batch)
         num_levels = max(a.level_max() - a.level_min() + 1 for a in aprs)
         expanded = restrict_kernel333_forward(weights, num_levels)
         ctx.aprs = aprs
@@ -41,8 +43,9 @@ class Conv333Function(Function):
         if ctx.packed:
             ctx.precision = precision or get_conv_precision()
             fused = _kernel_bias(bias, inputs, weights)
-            out, rows = conv333_forward_keep_rows(APRPtrVector(aprs), inputs, expanded, level_deltas, ctx.precision, fused)
-            ctx.save_for_backward(expanded, bias, level_deltas.clone(), rows)
+            out, rows = conv333_forward_keep_rows(APRPtrVector(aprs), inputs, expanded, level_deltas, ctx.precision, fused, keep)
+            if keep:
+                ctx.save_for_backward(expanded, bias, level_deltas.clone(), rows)
             return out if bias is None or fused is not None else out + bias.view(1, -1, 1)
         # float64: the tree means computed by the forward pass are kept (1/7 of the input's size) so that the
         # backward pass does not have to fill the tree again
@@ -61,12 +64,12 @@ class Conv333Function(Function):
                                                                    bool(ctx.needs_input_grad[0]), ctx.precision)
             grad_weights = restrict_kernel333_backward(grad_expanded, ctx.num_stencils)
             grad_bias = grad_output.sum(dim=(0, 2)) if bias is not None else None
-            return grad_input, grad_weights, grad_bias, None, None, None
+            return grad_input, grad_weights, grad_bias, None, None, None, None
         inputs, expanded, bias, level_deltas, tree = ctx.saved_tensors
         grad_input, grad_expanded = conv333_backward_with_tree(APRPtrVector(ctx.aprs), inputs, expanded, grad_output, level_deltas, tree)
         grad_weights = restrict_kernel333_backward(grad_expanded, ctx.num_stencils)
         grad_bias = grad_output.sum(dim=(0, 2)) if bias is not None else None
-        return grad_input, grad_weights, grad_bias, None, None, None
+        return grad_input, grad_weights, grad_bias, None, None, None, None
 
 
 class Conv111Function(Function):
@@ -126,4 +129,7 @@ class APRConv(nn.Module):
             init.uniform_(self.bias, -bound, bound)
 
     def forward(self, input_features, aprs, level_deltas):
-        return self._function.apply(input_features, self.weight, self.bias, aprs, level_deltas, self.precision)
+        if self._function is Conv111Function:
+            return Conv111Function.apply(input_features, self.weight, self.bias, aprs, level_deltas, self.precision)
+        keep = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (input_features, self.weight, self.bias))
+        return Conv333Function.apply(input_features, self.weight, self.bias, aprs, level_deltas, self.precision, keep)
