@@ -935,7 +935,6 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
         .def("cuda_device_bytes", [](APR& a) { return a.dev ? aprnet_device_bytes(a.dev) : (int64_t) 0; })
         .def("plan", [](APR& a, int dl) { TORCH_CHECK(a.dev, "APR.init_cuda() must be called first");
                                           c10::cuda::CUDAGuard guard((c10::DeviceIndex) a.dev_index);      // the tables live on the APR's device
-                                          if (g_conv_mode == 1) check(aprnet_run_plan_build(a.dev, dl, nullptr), "run plan");        // first: the others are derived from it
                                           check(aprnet_plan_build(a.dev, dl, nullptr), "plan");
                                           if (g_conv_mode == 1) check(aprnet_edge_plan_build(a.dev, dl, nullptr), "edge plan"); }, "level_delta"_a,
              "Build (and cache) the neighbour table of a level delta ahead of the first convolution")

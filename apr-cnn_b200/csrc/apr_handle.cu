@@ -372,6 +372,7 @@ const int32_t* aprnet_loc_parent_table(const aprnet_apr* a, int dl, cudaStream_t
 extern "C" int aprnet_plan_build(aprnet_apr* a, int dl, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl), "bad handle or level_delta");
     APRNET_DEVICE_CHECK(a);
+    if (!aprnet_get_run_plan(a, dl, (cudaStream_t) stream)) return APRNET_ERR_CUDA;          // first: the neighbour table is derived from it
     if (!aprnet_get_plan(a, dl, (cudaStream_t) stream)) return APRNET_ERR_CUDA;
     if (!aprnet_node_parent_table(a, (cudaStream_t) stream) || !aprnet_loc_parent_table(a, dl, (cudaStream_t) stream)) return APRNET_ERR_CUDA;
     return APRNET_OK;
