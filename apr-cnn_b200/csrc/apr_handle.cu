@@ -26,13 +26,15 @@ extern "C" const char* aprnet_last_error(void) { return g_last_error.c_str(); }
 // ---- memory of the cached tables and of their construction ------------------------------------------
 // One stream-ordered pool per device, shared by all handles.  cudaMalloc / cudaFree cost about 0.9 and 0.5 ms per table, which was
 // most of the time it took to prepare an access structure.  What is freed (temporaries, the tables of a destroyed handle) stays for
-// the next structure up to POOL_SPARE bytes above what is in use; the driver gives the rest back at the next synchronisation.
+// the next structure up to POOL_SPARE bytes above what is in use; the driver gives the rest back at the next synchronisation.  When a
+// device's last structure is destroyed, all but POOL_IDLE goes back.
 // The driver's allocator is safe with several threads and streams.
 namespace {
-constexpr unsigned long long POOL_SPARE = 2ull << 30;
+constexpr unsigned long long POOL_SPARE = 2ull << 30, POOL_IDLE = 256ull << 20;
 constexpr int POOL_DEVICES = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pools[POOL_DEVICES] = {};
+int g_structures[POOL_DEVICES] = {};           // alive on the device
 
 cudaMemPool_t pool_of_device() {
     int dev = 0;
@@ -55,6 +57,14 @@ void pool_keep(cudaMemPool_t pool) {          // reserved memory the pool may ho
     used += POOL_SPARE;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &used);
 }
+}
+
+static void count_structure(int device, int change) {
+    if (device < 0 || device >= POOL_DEVICES) return;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    g_structures[device] += change;
+    if (g_structures[device] > 0 || change > 0 || !g_pools[device]) return;
+    if (cudaStreamSynchronize(0) != cudaSuccess || cudaMemPoolTrimTo(g_pools[device], POOL_IDLE) != cudaSuccess) cudaGetLastError();
 }
 
 int aprnet_pool_alloc(void** p, size_t bytes, cudaStream_t st) {
@@ -242,6 +252,7 @@ extern "C" int aprnet_apr_create(aprnet_apr** out, int level_min, int level_max,
         return APRNET_ERR_UNSUPPORTED;
     }
     static_assert(sizeof(long long) == sizeof(int64_t), "int64 layout");
+    count_structure(device, +1);
     int rc;
     if ((rc = upload(&a->row_ptr, (const long long*) row_ptr, (size_t) a->n_rows + 1, &a->device_bytes))) { aprnet_apr_destroy(a); return rc; }
     if ((rc = upload(&a->y, y, (size_t) a->n_particles, &a->device_bytes))) { aprnet_apr_destroy(a); return rc; }
@@ -259,9 +270,14 @@ extern "C" int aprnet_apr_create(aprnet_apr** out, int level_min, int level_max,
         const int blocks = aprnet_ceil_div(rows * 32, 128);
         build_child_table_kernel<<<blocks, 128>>>(m, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, a->child,
                                                   a->tree_scale, a->n_tree, l);
-        APRNET_LAUNCH_CHECK();
     }
-    APRNET_CUDA_CHECK(cudaDeviceSynchronize());
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {
+        aprnet_set_error("aprnet_apr_create: child table: %s", cudaGetErrorString(e));
+        aprnet_apr_destroy(a);
+        return APRNET_ERR_CUDA;
+    }
     *out = a;
     return APRNET_OK;
 }
@@ -278,6 +294,7 @@ extern "C" void aprnet_apr_destroy(aprnet_apr* a) {
     for (auto& kv : a->loc_parent) aprnet_pool_free(kv.second, 0);
     for (auto& kv : a->edge_plans) aprnet_free_edge_plan(kv.second, 0);
     for (auto& kv : a->run_plans) { aprnet_pool_free(kv.second.loc, 0); aprnet_pool_free(kv.second.src, 0); }
+    count_structure(a->device, -1);
     delete a;
     if (prev >= 0) cudaSetDevice(prev);
 }
