@@ -113,6 +113,13 @@ struct aprnet_apr {
 };
 
 void aprnet_set_error(const char* fmt, ...);
+
+// Packed operands have a row per location, per tree node and one of zeros; the kernels hold row numbers in 32 bits.
+inline bool aprnet_rows_overflow(const aprnet_apr* a, int dl) {
+    if (a->number_parts(dl) + a->tree_size(dl) + 1 < (1ll << 31)) return false;
+    aprnet_set_error("%lld locations and %lld tree nodes exceed the 32-bit row numbers of the convolutions", a->number_parts(dl), a->tree_size(dl));
+    return true;
+}
 int aprnet_check_device(const aprnet_apr* a);      // APRNET_OK when the current device is the handle's device
 
 #define APRNET_CUDA_CHECK(expr)                                                                     \

@@ -320,6 +320,7 @@ const AprPlan* aprnet_get_plan(aprnet_apr* a, int dl, cudaStream_t stream) {
     if (aprnet_check_device(a) != APRNET_OK) return nullptr;
     auto it = a->plans.find(dl);
     if (it != a->plans.end()) return &it->second;
+    if (aprnet_rows_overflow(a, dl)) return nullptr;
     AprPlan p;
     p.level_delta = dl;
     p.n = a->number_parts(dl);

@@ -75,8 +75,7 @@ __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable seg
         float acc[32];
 #pragma unroll
         for (int o = 0; o < 32; ++o) acc[o] = 0.f;
-        // TAPS table entries and then TAPS values are requested before any is used; row numbers fit 32 bits (N + T + 1 < 2^31, checked by
-        // the driver)
+        // TAPS table entries and then TAPS values are requested before any is used; row numbers fit 32 bits (aprnet_rows_overflow)
         int32_t rows[TAPS];
         auto request = [&](int tap0) {
             const int32_t* e = nbr + (ll) tap0 * N + p;

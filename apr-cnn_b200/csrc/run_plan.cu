@@ -45,20 +45,22 @@ __device__ __forceinline__ RunRow run_row(const LevelMeta& m, const ll* row_ptr,
     return r;
 }
 
-// one thread per row; first pass (slot_y == null): count[row] = slots of the row; second pass: the slots from first[row] on
+// one thread per row; first pass (slot_y == null): count[row] = slots of the row, *total = slots of all rows; second pass: the slots
+// from first[row] on
 __global__ void run_slots_kernel(LevelMeta m, RunLevels R, const ll* __restrict__ row_ptr, const uint16_t* __restrict__ y, const ll* __restrict__ trow_ptr,
                                  const uint16_t* __restrict__ ty, int32_t* __restrict__ count, const int32_t* __restrict__ first,
-                                 int32_t* __restrict__ slot_y, int32_t* __restrict__ slot_loc) {
+                                 int32_t* __restrict__ slot_y, int32_t* __restrict__ slot_loc, unsigned long long* __restrict__ total) {
     const ll g = (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= R.begin[R.cml + 1]) return;
-    const int l = level_of_row(R, g);
+    const bool inside = g < R.begin[R.cml + 1];
+    const int l = inside ? level_of_row(R, g) : R.cml;
     const ll row = g - R.begin[l], tree_off = R.tree_off;
     const int with_tree = R.dl > 0 && l == R.cml;
-    RunRow r = run_row(m, row_ptr, y, trow_ptr, ty, l, row, with_tree);
+    RunRow r = {};
+    if (inside) r = run_row(m, row_ptr, y, trow_ptr, ty, l, row, with_tree);
     int last = -3, n = 0, yy;
     ll index;
     bool from_b;
-    const ll base = slot_y ? first[g] : 0;
+    const ll base = slot_y && inside ? first[g] : 0;
     while (r.next(&yy, &index, &from_b)) {
         for (int c = max(yy - 1, last + 1); c <= yy + 1; ++c) {
             if (slot_y) { slot_y[base + n] = c; slot_loc[base + n] = -1; }
@@ -67,7 +69,10 @@ __global__ void run_slots_kernel(LevelMeta m, RunLevels R, const ll* __restrict_
         last = yy + 1;
         if (slot_y) slot_loc[base + n - 2] = (int32_t) (from_b ? index + tree_off : index);
     }
-    if (!slot_y) count[g] = n;
+    if (slot_y) return;
+    if (inside) count[g] = n;
+    const unsigned sum = __reduce_add_sync(0xffffffffu, (unsigned) n);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(total, (unsigned long long) sum);
 }
 
 __device__ __forceinline__ ll find_cell(const uint16_t* __restrict__ y, ll b, ll e, int target) {
@@ -147,32 +152,40 @@ int build_run_plan(aprnet_apr* a, int dl, RunPlan& rp, cudaStream_t st) {
     for (int l = m.level_min; l <= cml; ++l) { R.begin[l] = rows; rows += (ll) m.z_num[l] * m.x_num[l]; }
     R.begin[cml + 1] = rows;
     int32_t *first = nullptr, *slot_y = nullptr, *picked = nullptr;
+    unsigned long long* total = nullptr;
     int rc = APRNET_OK;
     void* temp = nullptr;
     size_t temp_bytes = 0;
-    auto cleanup = [&]() { aprnet_pool_free(first, st); aprnet_pool_free(slot_y, st); aprnet_pool_free(picked, st); aprnet_pool_free(temp, st); };
+    auto cleanup = [&]() { aprnet_pool_free(first, st); aprnet_pool_free(slot_y, st); aprnet_pool_free(picked, st); aprnet_pool_free(temp, st); aprnet_pool_free(total, st); };
 #define RP_ALLOC(p, bytes) do { if ((rc = aprnet_pool_alloc((void**) &(p), (bytes), st))) { cleanup(); return rc; } } while (0)
 #define RP_CHECK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) { aprnet_set_error("%s failed: %s", #expr, cudaGetErrorString(_e)); cudaGetLastError(); cleanup(); return APRNET_ERR_CUDA; } } while (0)
+    // rows of packed operands and slots are 32-bit in the kernels
+    if (aprnet_rows_overflow(a, dl)) return APRNET_ERR_UNSUPPORTED;
+    RP_ALLOC(total, sizeof(ll));
+    RP_CHECK(cudaMemsetAsync(total, 0, sizeof(ll), st));
     RP_ALLOC(first, (size_t) (rows + 1) * sizeof(int32_t));
     RP_CHECK(cudaMemsetAsync(first + rows, 0, sizeof(int32_t), st));
-    run_slots_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, first, nullptr, nullptr, nullptr);
-    RP_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, first, first, (int) (rows + 1), st));
+    run_slots_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, first, nullptr, nullptr, nullptr, total);
+    RP_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, first, first, rows + 1, st));
     RP_ALLOC(temp, std::max<size_t>(temp_bytes, 1));
-    RP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, first, first, (int) (rows + 1), st));
+    RP_CHECK(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, first, first, rows + 1, st));
     std::vector<int32_t> at(cml + 2, 0);
     Picks picks;
     for (int l = m.level_min; l <= cml + 1; ++l) picks.at[l - m.level_min] = R.begin[l];
     RP_ALLOC(picked, sizeof(int32_t) * (APRNET_MAX_LEVELS + 2));
     pick_kernel<<<1, 32, 0, st>>>(first, picks, cml + 2 - m.level_min, picked);
     RP_CHECK(cudaMemcpyAsync(at.data() + m.level_min, picked, sizeof(int32_t) * (cml + 2 - m.level_min), cudaMemcpyDeviceToHost, st));
+    unsigned long long all = 0;
+    RP_CHECK(cudaMemcpyAsync(&all, total, sizeof(all), cudaMemcpyDeviceToHost, st));
     RP_CHECK(cudaStreamSynchronize(st));
+    if (all >= (1ull << 31) - 256) { aprnet_set_error("run plan: %llu slots exceed the 32-bit tables", all); cleanup(); return APRNET_ERR_UNSUPPORTED; }
     const ll S = at[cml + 1];
     rp.n_slots = S;
     rp.level_begin.assign(at.begin(), at.end());
     RP_ALLOC(slot_y, (size_t) std::max<ll>(S, 1) * sizeof(int32_t));
     RP_ALLOC(rp.loc, (size_t) std::max<ll>(S, 1) * sizeof(int32_t));
     RP_ALLOC(rp.src, (size_t) std::max<ll>(S, 1) * 9 * sizeof(int32_t));
-    run_slots_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, nullptr, first, slot_y, rp.loc);
+    run_slots_kernel<<<aprnet_ceil_div(rows, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, nullptr, first, slot_y, rp.loc, nullptr);
     run_sources_kernel<<<aprnet_ceil_div(rows * 32, 128), 128, 0, st>>>(m, R, a->row_ptr, a->y, a->tree_row_ptr, a->tree_y, first, slot_y, S, rp.src);
     RP_CHECK(cudaGetLastError());
     RP_CHECK(cudaStreamSynchronize(st));

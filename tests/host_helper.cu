@@ -34,3 +34,11 @@ extern "C" long long vrow_worst_pass(long long n_vrows, long long row_bytes) {
 }
 extern "C" void set_vrows(aprnet_apr* a, long long n) { a->edge_plans[0].n_vrows = n; }
 extern "C" long long vrow_chunk() { return APRNET_VROW_CHUNK; }
+
+extern "C" int rows_overflow(aprnet_apr* a, long long particles, long long nodes) {
+    const LevelMeta kept = a->meta;
+    for (int l = 2; l <= APRNET_MAX_LEVELS; ++l) { a->meta.lvl_begin[l] = particles; a->meta.tlvl_begin[l] = nodes; }
+    const int over = aprnet_rows_overflow(a, 0);
+    a->meta = kept;
+    return over;
+}

@@ -4,7 +4,9 @@ Device check: every convolution entry point checks that the current device is th
 Without a GPU the check is the one call that fails with "no current CUDA device"; an entry point that got past it would report its
 first launch or copy instead.  (On a GPU the same calls would reach kernels with the made-up pointers.)
 
-Cross-level input gradient: the sums per (target, tap) go through a bounded workspace in passes; no width may be refused."""
+Cross-level input gradient: the sums per (target, tap) go through a bounded workspace in passes; no width may be refused.
+
+Row numbers: the kernels hold them in 32 bits; structures beyond that are refused when a plan is built."""
 import ctypes as C
 import os
 import subprocess
@@ -24,6 +26,7 @@ def helper(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("host") / "helper.so")
     subprocess.check_call([NVCC, "-shared", "-Xcompiler", "-fPIC", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
                            os.path.join(ROOT, "tests", "host_helper.cu"), "-o", out])
+    C.CDLL(os.path.join(PKG, "libaprnet_b200.so"), mode=C.RTLD_GLOBAL)
     helper = C.CDLL(out)
     helper.fake_handle.restype = C.c_void_p
     helper.vrow_worst_pass.restype = helper.vrow_chunk.restype = C.c_longlong
@@ -84,3 +87,11 @@ def test_cross_level_passes_fit_their_workspace(helper, lib, cout):
     # the workspaces that the library reports hold a chunk of the plan at any width
     assert lib.aprnet_edge_workspace_bytes(handle, 0, cout) >= helper.vrow_chunk() * ((cout + 15) // 16 * 32)
     assert lib.aprnet_conv333_rows_backward_workspace_bytes(handle, 0, 0, 8, cout, 1, 1) >= helper.vrow_chunk() * ((cout + 3) // 4 * 16)
+
+
+@pytest.mark.parametrize("particles,nodes,over", [(16, 2, 0), (2 ** 31 - 1000, 998, 0), (2 ** 31 - 1000, 999, 1), (2 ** 31 - 3, 2 ** 31 - 3, 1)])
+def test_row_numbers_fit_32_bits(helper, lib, particles, nodes, over):
+    lib, handle = lib
+    assert helper.rows_overflow(handle, C.c_longlong(particles), C.c_longlong(nodes)) == over
+    if over:
+        assert b"32-bit row numbers" in lib.aprnet_last_error()
