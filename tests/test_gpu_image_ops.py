@@ -17,16 +17,23 @@ def oracle():
     return apr_oracle
 
 
+def _arrays(name):
+    if name == "long":                      # rows of 1101 cells: more than a warp holds at a time (512), odd extents
+        from pyapr import synthetic
+        return synthetic.random_apr((5, 7, 1101), 21, density=0.02)
+    return H.arrays(name) if name in H.APR_CASES else H.blob_arrays()
+
+
 def _apr(name):
     import pyapr
-    a = H.arrays(name) if name in H.APR_CASES else H.blob_arrays()
+    a = _arrays(name)
     apr = pyapr.apr_from_arrays(a, name)
     apr.init_cuda()
     return a, apr
 
 
 @pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-13), (torch.float32, 1e-6)])
-@pytest.mark.parametrize("name", ["blob", "odd", "odd2", "plane", "ref_shape"])
+@pytest.mark.parametrize("name", ["blob", "odd", "odd2", "plane", "ref_shape", "long"])
 def test_image_ops_match_oracle(name, dtype, tol, oracle):
     from _pyaprwrapper.data_containers import APRPtrVector
     from _pyaprwrapper.aprnet import cuda as C
