@@ -18,9 +18,10 @@ def oracle():
 
 
 def _arrays(name):
-    if name == "long":                      # rows of 1101 cells: more than a warp holds at a time (512), odd extents
+    if name == "long":                      # rows of 1101 cells: more than a warp holds at a time (512), odd extents, cells of up to 8^3
         from pyapr import synthetic
-        return synthetic.random_apr((5, 7, 1101), 21, density=0.02)
+        gen = torch.Generator().manual_seed(21)
+        return synthetic.apr_from_level_map(torch.randint(8, 12, (3, 4, 551), generator=gen).to(torch.int16), (5, 7, 1101))
     return H.arrays(name) if name in H.APR_CASES else H.blob_arrays()
 
 
