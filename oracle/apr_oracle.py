@@ -206,7 +206,7 @@ def _cells(a, dl):
         n_le = int(a.row_ptr[row_off[cml] + a.dims[cml][0] * a.dims[cml][1]])                # particles of levels <= cml
         t_begin = int(a.tree_row_ptr[tree_row_off[cml]])
         out.append(level_cells(a.tree_row_ptr, a.tree_y, tree_row_off[cml], cml, 1, n_le - t_begin))
-    return out, a.dims[cml]
+    return [c for c in out if len(c[0])], a.dims[cml]        # (the operators loop over the voxels of a cell: not for empty levels)
 
 
 def reconstruct_forward(a, x, dl):
