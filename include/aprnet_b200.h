@@ -4,8 +4,19 @@
  * Drop-in boundary for the operator set that AdaptiveParticles/APR-CNN exposes to Python as
  * `_pyaprwrapper.aprnet.cuda` (wrappers/pythonBind.cpp:162-181).  Every entry point takes plain
  * pointers and sizes, returns 0 on success or a negative status (never aborts), launches on the
- * stream it is given and performs no device-wide synchronisation and no allocation on the hot path:
- * outputs and scratch buffers are owned by the caller.
+ * stream it is given and performs no device-wide synchronisation: outputs and workspaces are owned by
+ * the caller.
+ *
+ * What allocates:
+ *   - aprnet_apr_create, and the first use of a level delta: the cached tables (aprnet_plan_build and,
+ *     for input gradients, aprnet_edge_plan_build build them up front; both wait for the stream);
+ *   - stream-ordered scratch of one call (cudaMallocAsync, given back in the same call; a CUDA graph can
+ *     capture it), where the signature has no workspace: float32 aprnet_conv333_{forward, backward_input,
+ *     backward_weights} and their _pretree forms (packed rows, packed weights and sums; with a workspace:
+ *     aprnet_conv333_rows_*), aprnet_reconstruct_* and aprnet_sample_particles_* (the levels below the
+ *     image; with a workspace: aprnet_cells_to_image / aprnet_image_to_cells);
+ *   - the same in aprnet_conv333_backward_input_cross_level_tc when edge_ws does not lie behind the rows
+ *     (rows and sums are addressed from one base: a joint copy otherwise).
  *
  * Conventions
  *   - feature tensors are channel-major: element (c, p) of a tensor lives at base[c * ld + p], with
@@ -82,7 +93,8 @@ int64_t aprnet_device_bytes(const aprnet_apr* apr);
  * location and each of the 27 stencil taps, which value fills that cell.  Replaces the per-call
  * non-empty-row enumeration and dense-patch staging of the reference
  * (pyapr/aprnet/cuda/src/nonempty_rows.cu:26-230, conv333_gpu.cu:63-118).  Called implicitly by the
- * conv333 entry points; call it up front to keep allocation out of timed regions. */
+ * conv333 entry points; call it up front to keep allocation out of timed regions and graph captures.  Also builds the
+ * run plan that the table is derived from and the parent tables of the tree adjoint. */
 int aprnet_plan_build(aprnet_apr* apr, int level_delta, void* stream);
 /* Test hooks: copy the cached tables to host memory.  nbr: int32[27][N]; child: int32[8][T]. */
 int aprnet_plan_copy_nbr_table(aprnet_apr* apr, int level_delta, int32_t* host_out);
@@ -234,7 +246,8 @@ int aprnet_conv333_backward_input_cross_level(aprnet_apr* apr, int level_delta, 
  * Limit: 27 * N(level_delta) < 2^31, i.e. up to 79.5 M locations (32-bit edge ids); beyond it
  * aprnet_conv333_backward_tc(_rows) falls back to aprnet_conv333_backward_input_cross_level (atomic adds). */
 int aprnet_edge_plan_build(aprnet_apr* apr, int level_delta, void* stream);
-/* The same for the run plan of the tensor-core gather kernels (output locations in runs along y; built once per level delta). */
+/* The run plan of the tensor-core gather kernels alone (output locations in runs along y; built once per level delta; part of
+ * aprnet_plan_build). */
 int aprnet_run_plan_build(aprnet_apr* apr, int level_delta, void* stream);
 int64_t aprnet_edge_workspace_bytes(const aprnet_apr* apr, int level_delta, int cout);
 int aprnet_conv333_backward_input_cross_level_tc(aprnet_apr* apr, int level_delta, int cin, int cout, int num_slots,
@@ -252,7 +265,9 @@ int aprnet_tc_selftest_wait_timeout(int max_polls, void* stream);
  * stage, "wps" = producer warps that fill one stage together (both must be set, and the pair must be a compiled
  * shape whose ring fits shared memory, else the automatic choice stays), "tma_taps" = how many of a stage's taps the TMA
  * unit fetches (tile::gather4) instead of cp.async (with "taps" and "wps"), "ks" = channels per stage (16, 32, 64),
- * "runs" = 0: gather every tap by itself instead of runs of cells, "dw_waves" = waves of blocks of the weight-gradient kernel. */
+ * "runs" = 0: gather every tap by itself instead of runs of cells, "dw_waves" = waves of blocks of the weight-gradient kernel.  "taps",
+ * "wps" and "tma_taps" act where every tap is gathered by itself ("runs" = 0, wide layers, the cross-level part) and leave the results as
+ * they are; the others change the order of the sums, i.e. the last bits of outputs ("ks") or gradients. */
 int aprnet_tc_set_option(const char* name, int value);
 
 /* ---- 1x1x1 convolution -----------------------------------------------------------------------
