@@ -1,5 +1,5 @@
-// 3x3x3 particle convolution on the tensor cores over runs of cells (bf16 operands, fp32 accumulation; forward pass and
-// same-level input gradient of layers with at most 128 result channels).
+// 3x3x3 particle convolution on the tensor cores over runs of cells (bf16 operands, fp32 accumulation): forward pass of layers with at
+// most 128 result channels (above 64 only where all source channels are in one stage), same-level input gradient of any width.
 //
 // The kernel of conv333_tc.cu gathers every source row once per tap, 27 rows per location.  Here the M dimension of a tile is not
 // 128 locations but 128 * H consecutive slots of the run plan (run_plan.cu).  For each of the 9 rows of cells (dz, dx) the tile's
