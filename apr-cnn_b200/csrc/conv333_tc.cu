@@ -146,19 +146,28 @@ constexpr int WS_MAX_STAGES = 20;
 constexpr int WS_MAX_ACC = 4;
 constexpr int WS_NIDX = 3;
 
-struct TileInfo { ll lo, hi, p0; int slot, ntile; };
-
-__device__ __forceinline__ TileInfo tile_info(const TcParams& P, int work) {
-    TileInfo t;
-    const int tile = P.n_tiles == 1 ? work : work / P.n_tiles;
-    t.ntile = P.n_tiles == 1 ? 0 : work % P.n_tiles;
-    int seg = 0;
-    while (seg + 1 < P.segs.n && tile >= P.segs.tile_begin[seg + 1]) ++seg;
-    t.lo = P.segs.begin[seg]; t.hi = P.segs.end[seg];
-    t.p0 = t.lo + (ll) (tile - P.segs.tile_begin[seg]) * TILE_M;
-    t.slot = P.segs.slot[seg];
-    return t;
-}
+// The tiles of a block, one after the other: work items blockIdx.x, + gridDim.x, ... over (tile, result tile).  The segment is found by going
+// on from the previous tile's: searching the parameters' table for every tile in every role cost some 500 cycles of dependent reads each time.
+struct TileWalk {
+    int tile, ntile, seg = -1, seg_first = 0, seg_end = 0, slot = 0;
+    const int dt, dn;                       // step of (tile, result tile) from one work item to the next
+    ll lo = 0, hi = 0;
+    __device__ __forceinline__ explicit TileWalk(const TcParams& P)
+        : tile(blockIdx.x / P.n_tiles), ntile(blockIdx.x % P.n_tiles), dt(gridDim.x / P.n_tiles), dn(gridDim.x % P.n_tiles) { settle(P); }
+    __device__ __forceinline__ void settle(const TcParams& P) {
+        while (tile >= seg_end && seg + 1 < P.segs.n) {
+            ++seg;
+            seg_first = P.segs.tile_begin[seg]; seg_end = P.segs.tile_begin[seg + 1];
+            lo = P.segs.begin[seg]; hi = P.segs.end[seg]; slot = P.segs.slot[seg];
+        }
+    }
+    __device__ __forceinline__ void next(const TcParams& P) {
+        tile += dt; ntile += dn;
+        if (ntile >= P.n_tiles) { ntile -= P.n_tiles; ++tile; }
+        settle(P);
+    }
+    __device__ __forceinline__ ll p0() const { return lo + (ll) (tile - seg_first) * TILE_M; }
+};
 
 template<int NT, int KS, int TAPS, int WPS, int TT, int NACC>
 __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcParams P, const int stages, const __grid_constant__ CUtensorMap row_map) {
@@ -229,15 +238,15 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
             const int32_t* idx = idx_s;
             const unsigned char* wsrc = nullptr;
             const ll w_tap_stride = (ll) P.n_tiles * P.kpad * NT * 2;
+            TileWalk walk(P);
             while (g < total_stages) {
-                while (step >= steps_per_tile) { step -= steps_per_tile; ++it; }
+                while (step >= steps_per_tile) { step -= steps_per_tile; ++it; walk.next(P); }
                 if (it != cur_it) {
                     cur_it = it;
                     if (!mbar_wait_warp(smem_u32(idx_full + it % NIDX), (it / NIDX) & 1, abort_flag)) { failed = true; break; }
                     idx = idx_s + (it % NIDX) * 27 * TILE_M + r0;
                     if (sub == 0 && lane == 0) {      // packed weights of one (slot, tap, n tile) are [k chunk][n][8]; a stage takes KS / 8 chunks of TAPS taps
-                        const TileInfo ti = tile_info(P, blockIdx.x + it * gridDim.x);
-                        wsrc = reinterpret_cast<const unsigned char*>(P.wp + ((ll) ti.slot * 27 * P.n_tiles + ti.ntile) * ((ll) P.kpad * NT));
+                        wsrc = reinterpret_cast<const unsigned char*>(P.wp + ((ll) walk.slot * 27 * P.n_tiles + walk.ntile) * ((ll) P.kpad * NT));
                     }
                 }
                 const int tg = step / kchunks, kc = step - tg * kchunks;
@@ -327,33 +336,33 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
         const int q = warp & 3;                           // TMEM lane group this warp may read
         const int row = q * 32 + lane;
         int32_t v[27];
+        TileWalk walk(P), ahead(P);                       // the tile that is read back, the one whose table entries are requested
         auto request_idx = [&](int it) {                  // table entries of this thread's row of tile `it` -> registers
             if (it >= my_tiles) return;
-            const TileInfo ti = tile_info(P, blockIdx.x + it * gridDim.x);
-            const ll p = ti.p0 + row;
+            const ll p = ahead.p0() + row;
+            const int32_t* src = P.nbr + p;
 #pragma unroll
-            for (int tap = 0; tap < 27; ++tap) v[tap] = (p < ti.hi) ? __ldg(P.nbr + (ll) tap * P.N + p) : APRNET_NONE;
+            for (int tap = 0; tap < 27; ++tap, src += P.N) v[tap] = (p < ahead.hi) ? __ldg(src) : APRNET_NONE;
         };
-        auto publish_idx = [&](int it) {                  // decode and hand the rows to the producers
+        auto publish_idx = [&](int it) {                  // decode and hand the rows to the producers (row numbers fit 32 bits)
             if (it >= my_tiles) return;
-            const TileInfo ti = tile_info(P, blockIdx.x + it * gridDim.x);
             int32_t* dst = idx_s + (it % NIDX) * 27 * TILE_M;
+            const int32_t zero = (int32_t) P.zero_row, tree = (int32_t) P.tree_base - 2, shift = (int32_t) P.v_shift, lo = (int32_t) ahead.lo, hi = (int32_t) ahead.hi;
 #pragma unroll
             for (int tap = 0; tap < 27; ++tap) {
-                ll r = P.zero_row;
-                if (P.same_level_only) { if (v[tap] >= ti.lo && v[tap] < ti.hi) r = v[tap]; }
-                else if (v[tap] >= 0) r = v[tap] + P.v_shift;
-                else if (v[tap] != APRNET_NONE) r = P.tree_base + aprnet_dec_tree(v[tap]);
-                dst[tap * TILE_M + row] = (int32_t) r;
+                int32_t r;
+                if (P.same_level_only) r = v[tap] >= lo && v[tap] < hi ? v[tap] : zero;
+                else r = v[tap] >= 0 ? v[tap] + shift : (v[tap] != APRNET_NONE ? tree - v[tap] : zero);
+                dst[tap * TILE_M + row] = r;
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(idx_full + it % NIDX));
+            ahead.next(P);
         };
         for (int it = 0; it < NIDX; ++it) { request_idx(it); publish_idx(it); }
-        for (int it = 0; it < my_tiles; ++it) {
-            const TileInfo ti = tile_info(P, blockIdx.x + it * gridDim.x);
-            const ll p = ti.p0 + row;
-            const bool valid = p < ti.hi;
+        for (int it = 0; it < my_tiles; ++it, walk.next(P)) {
+            const ll p = walk.p0() + row;
+            const bool valid = p < walk.hi;
             float* acc_dst = nullptr; ll acc_ld = 0;
             if (P.out_map && valid) {
                 const ll t = P.out_map[p];
@@ -372,30 +381,24 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
                 if (P.bias) {                // apart from the stores: a choice per element there cost the whole kernel 10 to 20 %
 #pragma unroll
                     for (int jj = 0; jj < 32; ++jj) {
-                        const int n = ti.ntile * NT + c0 + jj;
+                        const int n = walk.ntile * NT + c0 + jj;
                         if (n < P.n_dim) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + __ldg(P.bias + n));
                     }
                 }
                 if (valid && !P.out_map) {
 #pragma unroll
                     for (int jj = 0; jj < 32; ++jj) {
-                        const int n = ti.ntile * NT + c0 + jj;
+                        const int n = walk.ntile * NT + c0 + jj;
                         if (n < P.n_dim) P.out[(ll) n * P.ld_out + p] = __uint_as_float(r[jj]);
                     }
-                } else if (valid) {          // this thread is the only writer of its target: read all, then add and write
+                } else if (valid) {
+                    // this thread is the only writer of its target, so the order of the additions is fixed.  They happen in L2: with loads here the
+                    // four warps waited out the latency of scattered DRAM accesses twice per 32 channels.  Together with the walk over the
+                    // tiles, cross-level part of 32 -> 32, 64 -> 32 (3.5 M locations), 128 -> 64 (level delta 1): 494, 681, 404 -> 299, 381, 274 us.
 #pragma unroll
-                    for (int h = 0; h < 32; h += 16) {        // 16 independent loads at a time
-                        float old[16];
-#pragma unroll
-                        for (int jj = 0; jj < 16; ++jj) {
-                            const int n = ti.ntile * NT + c0 + h + jj;
-                            old[jj] = n < P.n_dim ? acc_dst[(ll) n * acc_ld] : 0.f;
-                        }
-#pragma unroll
-                        for (int jj = 0; jj < 16; ++jj) {
-                            const int n = ti.ntile * NT + c0 + h + jj;
-                            if (n < P.n_dim) acc_dst[(ll) n * acc_ld] = old[jj] + __uint_as_float(r[h + jj]);
-                        }
+                    for (int jj = 0; jj < 32; ++jj) {
+                        const int n = walk.ntile * NT + c0 + jj;
+                        if (n < P.n_dim) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(acc_dst + (ll) n * acc_ld), "f"(__uint_as_float(r[jj])) : "memory");
                     }
                 }
             }
