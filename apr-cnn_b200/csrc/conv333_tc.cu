@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
         // ---------------- MMA issue ----------------
         if (lane == 0) {
             uint32_t slot = 0, use = 0;
+            bool ready = false;                   // the next stage is known to be there
             for (int it = 0; it < my_tiles && !failed; ++it) {
                 const uint32_t acc = (uint32_t) it % NACC, acc_use = (uint32_t) it / NACC;
                 if (acc_use > 0 && !mbar_wait(smem_u32(tmem_empty + acc), (acc_use - 1) & 1, abort_flag)) { failed = true; break; }
@@ -308,15 +309,18 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
                 const uint32_t d_addr = tmem_d + acc * NT;
                 int t0 = 0, kc = 0;
                 for (int step = 0; step < steps_per_tile; ++step) {
-                    if (!mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
+                    if (!ready && !mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
                     fence_proxy_async();          // generic-proxy writes of the cp.async copies -> tensor-core (async proxy) reads
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(stage_base + (size_t) slot * STAGE_BYTES);
                     // descriptors of the stage's first MMA; the others add the encoded byte offset of their operand
                     const uint64_t da0 = make_desc(a_addr, 16, 8 * ROW_BYTES, A_LAYOUT);
                     const uint64_t db0 = make_desc(a_addr + TAPS * A_TAP, NT * 16, 128, 0);
+                    const uint32_t used = slot;
+                    if (++slot == (uint32_t) stages) { slot = 0; ++use; }
 #pragma unroll
                     for (int t = 0; t < TAPS; ++t) {
+                        if (t == TAPS / 2) ready = mbar_test(smem_u32(full + slot), use & 1);
                         if (t0 + t < 27) {
 #pragma unroll
                             for (int k = 0; k < KS / 16; ++k)
@@ -324,8 +328,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
                                           IDESC, (step > 0 || t > 0 || k > 0) ? 1u : 0u);
                         }
                     }
-                    umma_commit(smem_u32(empty + slot));
-                    if (++slot == (uint32_t) stages) { slot = 0; ++use; }
+                    umma_commit(smem_u32(empty + used));
                     if (++kc == kchunks) { kc = 0; t0 += TAPS; }
                 }
                 if (!failed) umma_commit(smem_u32(tmem_full + acc));

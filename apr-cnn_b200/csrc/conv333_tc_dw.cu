@@ -65,6 +65,7 @@ template<int CIB, int NCOL>
 __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwParams P, const int nstage) {
     constexpr int TPT = 128 / CIB;                      // neighbours per 128-row accumulator tile
     constexpr int PC = CIB / 8;                         // 16-byte chunks per gathered row piece
+    constexpr int PB = PC < 8 ? PC : 8;                 // copies whose rows are handed round together
     constexpr int G_ROW = NCOL == 32 ? 64 : 128;        // bytes of a dO row in one swizzle atom
     constexpr int G_ATOM = G_ROWS * G_ROW;              // one atom (32 or 64 columns) of a dO chunk
     constexpr int G_BYTES = (G_ATOM * (NCOL == 128 ? 2 : 1) + 1023) / 1024 * 1024;
@@ -126,8 +127,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
         // table entries of this lane's slot for stage s: requested here, decoded only when the stage is issued, so that the load
         // latency overlaps the copies of the stage in between; with a chunk's first stage also the locations of its dO rows (row r of
         // the dO chunk is slot r - 1; the last two rows belong to the last quarter)
-        auto request = [&](int s) {
-            const int chunk = s / MT, mt = s - chunk * MT;
+        auto request = [&](int chunk, int mt) {
             const ll c0 = sb + ((ll) rl + (ll) chunk * cnt) * PT, slot = c0 + wq * 32 + lane;
 #pragma unroll
             for (int tl = 0; tl < TPT; ++tl) {
@@ -140,22 +140,28 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                 loc_extra = wq == 3 && lane < 2 && q < se ? __ldg(P.loc + q) : -1;
             }
         };
+        const int32_t zero = (int32_t) P.zero_row, tree = (int32_t) P.tree_base - 2;      // row numbers fit 32 bits
         auto decode = [&]() {
 #pragma unroll
             for (int tl = 0; tl < TPT; ++tl) {
                 const int32_t v = raw_nxt[tl];
-                rows_cur[tl] = (int32_t) (v >= 0 ? (ll) v : (v == APRNET_NONE ? P.zero_row : P.tree_base + aprnet_dec_tree(v)));
+                rows_cur[tl] = v >= 0 ? v : (v == APRNET_NONE ? zero : tree - v);
             }
             g_row = loc_nxt >= 0 ? loc_nxt : (int32_t) P.g_zero_row;
             g_extra = loc_extra >= 0 ? loc_extra : (int32_t) P.g_zero_row;
         };
-        int s = gq;
-        if (s < total_stages) { request(s); decode(); }
-        while (s < total_stages) {
-            const int s_nxt = s + NGROUP;
-            if (s_nxt < total_stages) request(s_nxt);      // in flight while this stage is issued
-            const int chunk = s / MT, mt = s - chunk * MT;
-            const uint32_t slot = (uint32_t) s % (uint32_t) nstage, use = (uint32_t) s / (uint32_t) nstage;
+        int chunk_nxt = 0, mt_nxt = gq;                    // chunk and accumulator tile of the next stage of this group
+        auto advance = [&]() { while (mt_nxt >= MT) { mt_nxt -= MT; ++chunk_nxt; } };
+        advance();
+        if (gq < total_stages) { request(chunk_nxt, mt_nxt); decode(); }
+        uint32_t slot = gq, use = 0;                       // (the ring has at least NGROUP stages)
+        for (int s = gq; s < total_stages; s += NGROUP, slot += NGROUP) {
+            if (slot >= (uint32_t) nstage) { slot -= nstage; ++use; }
+            const int chunk = chunk_nxt, mt = mt_nxt;
+            mt_nxt += NGROUP;
+            advance();
+            const bool more = s + NGROUP < total_stages;
+            if (more) request(chunk_nxt, mt_nxt);          // in flight while this stage is issued
             if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
             if (mt == 0) {
                 // this warp's rows of the dO chunk, into the buffer of chunk - 2.  A wait by parity must know the phase before the awaited
@@ -190,17 +196,20 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                 const uint32_t dst0 = smem_u32(a_s + (m >> 6) * ATOM_STRIDE);
                 const int cc = (m & 63) >> 3;
 #pragma unroll
-                for (int pi = 0; pi < PC; ++pi) {
-                    const int pl = pi * RPI + r0;
-                    const int32_t r = __shfl_sync(0xffffffffu, rows_cur[tl], pl);
-                    const int k = wq * 32 + pl;
-                    if (c < cpieces) cp_async16(dst0 + k * 128 + ((cc ^ (k & 7)) << 4), src0 + (ll) r * P.xpad);
+                for (int p0 = 0; p0 < PC; p0 += PB) {      // copies and shuffles keep their order: the rows of several copies are handed round first
+                    int32_t r[PB];
+#pragma unroll
+                    for (int pi = 0; pi < PB; ++pi) r[pi] = __shfl_sync(0xffffffffu, rows_cur[tl], (p0 + pi) * RPI + r0);
+#pragma unroll
+                    for (int pi = 0; pi < PB; ++pi) {
+                        const int k = wq * 32 + (p0 + pi) * RPI + r0;
+                        if (c < cpieces) cp_async16(dst0 + k * 128 + ((cc ^ (k & 7)) << 4), src0 + (ll) r[pi] * P.xpad);
+                    }
                 }
             }
             // the stage's barrier receives this thread's arrival when the copies above have landed
             cp_async_arrive_noinc(smem_u32(full + slot));
-            if (s_nxt < total_stages) decode();
-            s = s_nxt;
+            if (more) decode();
         }
         cp_async_commit();
         cp_async_wait<0>();
@@ -208,20 +217,23 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
         // ---------------- MMA issue ----------------
         if (lane == 0) {
             uint32_t slot = 0, use = 0;
+            bool ready = false;                   // the next stage is known to be there
             for (int chunk = 0; chunk < nchunks && !failed; ++chunk) {
                 const uint32_t db = chunk & 1, duse = chunk >> 1;
                 const uint32_t b_addr = smem_u32(g_ring + db * G_BYTES);
                 for (int mt = 0; mt < MT; ++mt) {
-                    if (!mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
-                    if (mt == 0 && !mbar_wait(smem_u32(dfull + db), duse & 1, abort_flag)) { failed = true; break; }
+                    if (!ready && !mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
+                    if (mt == 0 && !mbar_test(smem_u32(dfull + db), duse & 1) && !mbar_wait(smem_u32(dfull + db), duse & 1, abort_flag)) { failed = true; break; }
                     fence_proxy_async();          // generic-proxy writes of the cp.async copies -> tensor-core (async proxy) reads
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(a_ring + (size_t) slot * A_STAGE);
+                    const uint32_t a_addr = smem_u32(a_ring + (size_t) slot * A_STAGE), used = slot;
+                    if (++slot == (uint32_t) nstage) { slot = 0; ++use; }
 #pragma unroll
                     for (int k = 0; k < PT / 16; ++k) {
                         // 16 slots = two 8-row groups; atoms along M are ATOM_STRIDE apart, along N one row (the next shift) or, for
                         // 128 columns, one atom
                         const uint64_t da = make_desc(a_addr + k * 2048, ATOM_STRIDE, 1024, 2);
+                        if (k == PT / 32) ready = mbar_test(smem_u32(full + slot), use & 1);
 #pragma unroll
                         for (int i = 0; i < MMAS; ++i) {
                             const uint64_t dbd = NCOL == 32 ? make_desc(b_addr + k * 1024, 64, 512, 4)
@@ -229,9 +241,8 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                             umma_bf16(tmem_d + mt * COLS + i * NCOL, da, dbd, IDESC, (chunk > 0 || k > 0) ? 1u : 0u);
                         }
                     }
-                    umma_commit(smem_u32(empty + slot));
+                    umma_commit(smem_u32(empty + used));
                     if (mt == MT - 1) umma_commit(smem_u32(dempty + chunk % DO_PHASES));
-                    if (++slot == (uint32_t) nstage) { slot = 0; ++use; }
                 }
             }
             if (!failed) umma_commit(smem_u32(done));

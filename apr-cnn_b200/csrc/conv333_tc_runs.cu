@@ -53,17 +53,32 @@ template<int KS> __device__ __forceinline__ int swizzled_chunk(int row, int c) {
     return KS == 64 ? (c ^ (row & 7)) : (KS == 32 ? (c ^ ((row >> 1) & 3)) : (c ^ ((row >> 2) & 1)));
 }
 
-struct Tile { ll s0, sb, se, lo, hi; int wslot, ntile; };       // s0: slot of staged row 0
-
-__device__ __forceinline__ Tile tile_of(const RunParams& P, int work, int rows) {
-    const int tile = work / P.n_tiles;
-    int seg = 0;
-    while (seg + 1 < P.n_segs && tile >= P.tile_begin[seg + 1]) ++seg;
-    Tile t;
-    t.sb = P.slot_begin[seg]; t.se = P.slot_end[seg]; t.lo = P.lo[seg]; t.hi = P.hi[seg]; t.wslot = P.wslot[seg]; t.ntile = work - tile * P.n_tiles;
-    t.s0 = t.sb - 1 + (ll) (tile - P.tile_begin[seg]) * (rows - 2);      // the first and the last row have no neighbour on one side
-    return t;
-}
+// The tiles of a block, one after the other: work items blockIdx.x, + gridDim.x, ... over (tile, result tile).  The segment is found by going
+// on from the previous tile's: searching the parameters' table for every tile in every role cost some 500 cycles of dependent reads each time.
+struct TileWalk {
+    int tile, ntile, seg = -1, seg_first = 0, seg_end = 0, wslot = 0;
+    int32_t lo = 0, hi = 0;                 // locations of the tile's level
+    const int dt, dn;                       // step of (tile, result tile) from one work item to the next
+    ll sb = 0, se = 0;                      // its slots
+    __device__ __forceinline__ explicit TileWalk(const RunParams& P)
+        : tile(blockIdx.x / P.n_tiles), ntile(blockIdx.x % P.n_tiles), dt(gridDim.x / P.n_tiles), dn(gridDim.x % P.n_tiles) { settle(P); }
+    __device__ __forceinline__ void settle(const RunParams& P) {
+        while (tile >= seg_end && seg + 1 < P.n_segs) {
+            ++seg;
+            seg_first = P.tile_begin[seg]; seg_end = P.tile_begin[seg + 1];
+            sb = P.slot_begin[seg]; se = P.slot_end[seg]; lo = (int32_t) P.lo[seg]; hi = (int32_t) P.hi[seg]; wslot = P.wslot[seg];
+        }
+    }
+    __device__ __forceinline__ void next(const RunParams& P) {
+        tile += dt; ntile += dn;
+        if (ntile >= P.n_tiles) { ntile -= P.n_tiles; ++tile; }
+        settle(P);
+    }
+    // slot of staged row 0; the first and the last of the `rows` rows have no neighbour on one side.  The rows [first, end) are slots of the level
+    __device__ __forceinline__ ll s0(int rows) const { return sb - 1 + (ll) (tile - seg_first) * (rows - 2); }
+    __device__ __forceinline__ int first() const { return tile == seg_first ? 1 : 0; }
+    __device__ __forceinline__ int end(int rows) const { return (int) min(se - s0(rows), (ll) rows); }
+};
 
 // Roles of the warps of the persistent block:
 //   0-7         producers, in groups of WPS; a stage (neighbour row x KS channels x 128 H slots, and the weights of its three taps) belongs to one
@@ -81,6 +96,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     constexpr int RW = 32 / CH;                              // rows per copy instruction of a warp
     constexpr int ROWS = 128 * H, WROWS = ROWS / WPS;        // slots of a tile, rows a producer warp copies
     constexpr int NI = WROWS / RW, LR = (WROWS + 31) / 32;   // its copy instructions per stage, table entries per lane
+    constexpr int NB = NI < 8 ? NI : 8;                      // copies whose rows are handed round together
     constexpr int NACC = 512 / (H * NT) < MAX_ACC ? 512 / (H * NT) : MAX_ACC;      // accumulators in flight per block of 128 rows
     constexpr int ISSUERS = H < 2 ? 1 : 2;
     constexpr int ROW_BYTES = KS * 2;
@@ -89,7 +105,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     constexpr int B_TAP = NT * KS * 2;
     constexpr int STAGE_BYTES = A_BYTES + 3 * B_TAP;
     constexpr uint32_t IDESC = make_idesc(NT, false, false);
-    static_assert(STAGE_BYTES % 1024 == 0 && H * NT <= 512 && WROWS % 32 == 0, "stages keep the swizzle alignment; accumulators fit TMEM");
+    static_assert(STAGE_BYTES % 1024 == 0 && H * NT <= 512 && WROWS % 32 == 0 && NI % NB == 0, "stages keep the swizzle alignment; accumulators fit TMEM");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ float bias_s[MAX_N];
     // ring at a multiple of 1024 bytes, with 1024 bytes in front of it (row -1 of the first stage is read, its results are not used)
@@ -129,54 +145,59 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
             const int j = lane % CH, rsub = lane / CH;
             const uint32_t total = (uint32_t) my_tiles * (uint32_t) steps;
             const ll w_tile = (ll) P.kpad * NT * 2, w_tap_stride = P.n_tiles * w_tile;
-            uint32_t g = grp, slot = grp, use = 0;
-            int it = 0, step = grp, cur_it = -1;
-            Tile t;
+            uint32_t slot = grp, use = 0;
+            uint32_t left = grp < (int) total ? (total - grp + ngroups - 1) / ngroups : 0;       // stages of this group
+            TileWalk walk(P);
+            int d = 0, kc = grp;                             // the stage's neighbour row and channels
+            auto locate = [&]() {
+                while (kc >= kchunks) { kc -= kchunks; ++d; }
+                while (d >= 9) { d -= 9; walk.next(P); }
+            };
             int32_t raw[LR], cur[LR];
-            auto request = [&](int d) {                      // table entries of this lane's rows
+            auto request = [&]() {                           // table entries of this lane's rows
+                const int first = walk.first(), end = walk.end(ROWS);
+                const int32_t* src = P.src + (ll) d * P.S + walk.s0(ROWS) + sub * WROWS + lane;
 #pragma unroll
                 for (int i = 0; i < LR; ++i) {
-                    const ll s = t.s0 + sub * WROWS + 32 * i + lane;
-                    raw[i] = (s >= t.sb && s < t.se) ? __ldg(P.src + (ll) d * P.S + s) : APRNET_NONE;
+                    const int row = sub * WROWS + 32 * i + lane;
+                    raw[i] = row >= first && row < end ? __ldg(src + 32 * i) : APRNET_NONE;
                 }
             };
-            auto locate = [&]() {                            // tile and stage of g
-                while (step >= steps) { step -= steps; ++it; }
-                if (it != cur_it) { cur_it = it; t = tile_of(P, blockIdx.x + it * gridDim.x, ROWS); }
-            };
-            if (g < total) { locate(); request(step / kchunks); }
-            while (g < total) {
-                const int d = step / kchunks, kc = step - d * kchunks;
+            const int32_t zero = (int32_t) P.zero_row, tree = (int32_t) P.tree_base - 2;       // row numbers fit 32 bits
+            if (left > 0) { locate(); request(); }
+            for (; left > 0; --left) {
 #pragma unroll
                 for (int i = 0; i < LR; ++i) {
                     const int32_t v = raw[i];
-                    ll r = P.zero_row;
-                    if (P.same_level_only) { if (v >= t.lo && v < t.hi) r = v; }
-                    else if (v >= 0) r = v;
-                    else if (v != APRNET_NONE) r = P.tree_base + aprnet_dec_tree(v);
-                    cur[i] = (int32_t) r;
+                    if (P.same_level_only) cur[i] = v >= walk.lo && v < walk.hi ? v : zero;
+                    else cur[i] = v >= 0 ? v : (v != APRNET_NONE ? tree - v : zero);
                 }
-                const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(P.wp) + (ll) t.wslot * 27 * w_tap_stride + t.ntile * w_tile;
-                step += ngroups;
-                if (g + ngroups < total) { locate(); request(step / kchunks); }      // in flight while this stage is copied
+                const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(P.wp) + ((ll) walk.wslot * 27 + (P.same_level_only ? 26 - 3 * d : 3 * d)) * w_tap_stride + walk.ntile * w_tile + (ll) kc * KS * NT * 2;
+                const __nv_bfloat16* src0 = P.rows + kc * KS + j * 8;
+                kc += ngroups;
+                if (left > 1) { locate(); request(); }       // in flight while this stage is copied
                 if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
                 unsigned char* a_s = ring + (size_t) slot * STAGE_BYTES;
                 if (sub == 0 && lane == 0) {
                     mbar_expect_tx(smem_u32(full + slot), 3 * B_TAP);
 #pragma unroll
                     for (int dy = 0; dy < 3; ++dy)
-                        bulk_copy_g2s(smem_u32(a_s + A_BYTES + dy * B_TAP), wsrc + (P.same_level_only ? 26 - 3 * d - dy : 3 * d + dy) * w_tap_stride + (ll) kc * KS * NT * 2, B_TAP, smem_u32(full + slot));
+                        bulk_copy_g2s(smem_u32(a_s + A_BYTES + dy * B_TAP), wsrc + (P.same_level_only ? -dy : dy) * w_tap_stride, B_TAP, smem_u32(full + slot));
                     bulk_issued = true;
                 }
-                const __nv_bfloat16* src0 = P.rows + kc * KS + j * 8;
 #pragma unroll
-                for (int i = 0; i < NI; ++i) {
-                    const int row = sub * WROWS + i * RW + rsub;
-                    const int32_t r = __shfl_sync(0xffffffffu, cur[i * RW / 32], (i * RW + rsub) & 31);
-                    cp_async16(smem_u32(a_s + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) r * P.kpad);
+                for (int i0 = 0; i0 < NI; i0 += NB) {        // copies and shuffles keep their order: the rows of several copies are handed round first
+                    int32_t r[NB];
+#pragma unroll
+                    for (int i = 0; i < NB; ++i) r[i] = __shfl_sync(0xffffffffu, cur[(i0 + i) * RW / 32], ((i0 + i) * RW + rsub) & 31);
+#pragma unroll
+                    for (int i = 0; i < NB; ++i) {
+                        const int row = sub * WROWS + (i0 + i) * RW + rsub;
+                        cp_async16(smem_u32(a_s + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) r[i] * P.kpad);
+                    }
                 }
                 cp_async_arrive_noinc(smem_u32(full + slot));        // this thread's arrival when its copies have landed
-                g += ngroups; slot += ngroups;
+                slot += ngroups;
                 if (slot >= (uint32_t) stages) { slot -= stages; ++use; }
             }
             cp_async_commit();
@@ -186,34 +207,34 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
         // ---------------- MMA issue, every second block of 128 rows ----------------
         const int h0 = warp - MMA_WARP;
         if (lane == 0 && h0 < ISSUERS) {
+            constexpr int MMAS = 3 * (KS / 16);
             uint32_t slot = 0, use = 0;
+            bool ready = false;                   // the next stage is known to be there
             for (int it = 0; it < my_tiles && !failed; ++it) {
                 const uint32_t acc = (uint32_t) it % NACC, acc_use = (uint32_t) it / NACC;
                 if (acc_use > 0 && !mbar_wait(smem_u32(tmem_empty + h0 * MAX_ACC + acc), (acc_use - 1) & 1, abort_flag)) { failed = true; break; }
                 tc_fence_after();
                 for (int step = 0; step < steps; ++step) {
-                    if (!mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
+                    if (!ready && !mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
                     fence_proxy_async();          // generic-proxy writes of the cp.async copies -> tensor-core (async proxy) reads
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(ring + (size_t) slot * STAGE_BYTES);
                     const uint64_t db0 = make_desc(a_addr + A_BYTES, NT * 16, 128, 0);
+                    const uint32_t used = slot;
+                    if (++slot == (uint32_t) stages) { slot = 0; ++use; }
 #pragma unroll
                     for (int h = 0; h < H; h += ISSUERS) {
                         const uint64_t da0 = make_desc(a_addr + (h + h0) * 128 * ROW_BYTES - ROW_BYTES, 16, 8 * ROW_BYTES, A_LAYOUT);      // dy = -1
                         const uint32_t d_addr = tmem_d + ((h + h0) * NACC + acc) * NT;
 #pragma unroll
-                        for (int ko = 0; ko < KS / KORD; ++ko)
-#pragma unroll
-                            for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-                                for (int kk = 0; kk < KORD / 16; ++kk) {
-                                    const int k = ko * (KORD / 16) + kk;
-                                    umma_bf16(d_addr, da0 + (uint64_t) ((dy * ROW_BYTES + k * 32) >> 4), db0 + (uint64_t) ((dy * B_TAP + k * 2 * (NT * 16)) >> 4),
-                                              IDESC, (step > 0 || ko > 0 || dy > 0 || kk > 0) ? 1u : 0u);
-                                }
+                        for (int m = 0; m < MMAS; ++m) {          // blocks of KORD channels, dy, 16 channels
+                            const int ko = m / (3 * (KORD / 16)), dy = m / (KORD / 16) % 3, k = ko * (KORD / 16) + m % (KORD / 16);
+                            if (h + ISSUERS >= H && m == MMAS / 2) ready = mbar_test(smem_u32(full + slot), use & 1);
+                            umma_bf16(d_addr, da0 + (uint64_t) ((dy * ROW_BYTES + k * 32) >> 4), db0 + (uint64_t) ((dy * B_TAP + k * 2 * (NT * 16)) >> 4),
+                                      IDESC, (step > 0 || m > 0) ? 1u : 0u);
+                        }
                     }
-                    umma_commit(smem_u32(empty + slot));
-                    if (++slot == (uint32_t) stages) { slot = 0; ++use; }
+                    umma_commit(smem_u32(empty + used));
                 }
                 if (!failed) umma_commit(smem_u32(tmem_full + h0 * MAX_ACC + acc));
             }
@@ -221,19 +242,19 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     } else if ((warp - EPI_WARP) / 4 < ISSUERS) {
         // ---------------- epilogue of one issuer's blocks ----------------
         const int h0 = (warp - EPI_WARP) >> 2, q = warp & 3;         // q: TMEM lanes this warp may read
+        TileWalk walk(P);                                            // the tile after the one that is read back
         auto location = [&](int it, int h) {
             const int m = h * 128 + q * 32 + lane;
             if (it >= my_tiles || m == 0 || m == ROWS - 1) return (int32_t) -1;
-            const Tile t = tile_of(P, blockIdx.x + it * gridDim.x, ROWS);
-            const ll s = t.s0 + m;
-            return s >= t.sb && s < t.se ? __ldg(P.loc + s) : -1;
+            return m >= walk.first() && m < walk.end(ROWS) ? __ldg(P.loc + walk.s0(ROWS) + m) : -1;
         };
         constexpr int BLOCKS = H / ISSUERS;
         int32_t p_next[BLOCKS];
 #pragma unroll
         for (int b = 0; b < BLOCKS; ++b) p_next[b] = location(0, h0 + b * ISSUERS);
         for (int it = 0; it < my_tiles; ++it) {
-            const int n0 = (int) ((blockIdx.x + it * gridDim.x) % (unsigned) P.n_tiles) * NT;
+            const int n0 = walk.ntile * NT;
+            walk.next(P);
             int32_t p_cur[BLOCKS];
 #pragma unroll
             for (int b = 0; b < BLOCKS; ++b) { p_cur[b] = p_next[b]; p_next[b] = location(it + 1, h0 + b * ISSUERS); }
