@@ -270,14 +270,20 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
             dst = t < P.out_split ? P.out + t : P.out2 + (t - P.out_split);
             ld = t < P.out_split ? P.ld_out : P.ld_out2;
         }
+        // target mode adds to what is there (this thread is the only writer of its target in this launch): all of it is requested before any is
+        // written, an addition after the other waited TN times for scattered accesses
+        float add[TN];
 #pragma unroll
         for (int n = 0; n < TN; ++n) {
             const int co = nt * NT + n_off + n;
-            if (co >= P.n_dim) continue;
+            add[n] = co >= P.n_dim ? 0.f : (P.out_map ? dst[(ll) co * ld] : (P.bias ? P.bias[co] : 0.f));
+        }
+#pragma unroll
+        for (int n = 0; n < TN; ++n) {
+            const int co = nt * NT + n_off + n;
             const float2 pair = unpack2(acc[i][n / 2]);
             const float v = n & 1 ? pair.y : pair.x;
-            if (P.out_map) dst[(ll) co * ld] += v;          // the only writer of its target in this launch
-            else dst[(ll) co * ld] = P.bias ? v + P.bias[co] : v;
+            if (co < P.n_dim) dst[(ll) co * ld] = P.out_map || P.bias ? v + add[n] : v;
         }
     }
 }
