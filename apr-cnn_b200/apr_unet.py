@@ -30,9 +30,12 @@ class ConvNormAct(nn.Module):
         else:
             self.norm = nn.GroupNorm(groups, cout)
             self.act = nn.ReLU()
+        self._conv_norm = getattr(ops, "conv_norm", None)
 
     def forward(self, x, aprs, level_deltas):
-        return self.act(self.norm(self.conv(x, aprs, level_deltas)))
+        conv_norm = getattr(self, "_conv_norm", None)
+        y = conv_norm(self.conv, self.norm, x, aprs, level_deltas) if conv_norm else self.norm(self.conv(x, aprs, level_deltas))
+        return self.act(y)
 
 
 class Stage(nn.Module):

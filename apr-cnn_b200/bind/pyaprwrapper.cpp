@@ -286,6 +286,37 @@ static std::vector<torch::Tensor> conv333_backward_rows(std::vector<APR*>& aprs,
     return {grad_input, grad_weights, grad_tree};
 }
 
+// GroupNorm + ReLU and the convolution in front of it (one batch item, bf16 arithmetic): {grad_input or undefined, grad_weights, grad_gamma, grad_beta}
+std::vector<torch::Tensor> conv333_norm_backward(std::vector<APR*>& aprs, torch::Tensor rows, torch::Tensor weights, torch::Tensor conv_out, torch::Tensor grad_y,
+                                                 c10::optional<torch::Tensor> gamma, c10::optional<torch::Tensor> beta, torch::Tensor mean, torch::Tensor rstd,
+                                                 int64_t groups, bool relu, torch::Tensor level_delta, bool need_grad_input) {
+    CHECK_INPUT(weights); CHECK_INPUT(conv_out); CHECK_INPUT(grad_y); CHECK_INPUT(rows); CHECK_INPUT(mean); CHECK_INPUT(rstd);
+    TORCH_CHECK(conv_out.sizes() == grad_y.sizes() && conv_out.dim() == 3 && conv_out.size(0) == 1 && conv_out.size(1) == weights.size(1), "one batch item, gradient of the output's shape");
+    TORCH_CHECK(conv_out.scalar_type() == torch::kFloat32 && grad_y.scalar_type() == torch::kFloat32 && weights.scalar_type() == torch::kFloat32, "float32 tensors");
+    TORCH_CHECK(groups > 0 && conv_out.size(1) % groups == 0 && mean.numel() == groups && rstd.numel() == groups, "statistics do not match the input");
+    c10::cuda::CUDAGuard guard(conv_out.device());
+    const Batch B(aprs, conv_out, level_delta);
+    const int cin = (int) weights.size(2), cout = (int) weights.size(1), slots = (int) weights.size(0);
+    const int64_t n = conv_out.size(2);
+    TORCH_CHECK(rows.dim() == 2 && rows.size(0) == 1 && rows.scalar_type() == torch::kUInt8 &&
+                rows.size(1) >= B.most_bytes([&](aprnet_apr* h, int dl) { return aprnet_conv333_rows_bytes(h, dl, APRNET_PREC_BF16, cin); }), "rows buffer too small for this APR");
+    if (need_grad_input) check(aprnet_edge_plan_build(B.h[0], B.dl[0], stream_of(grad_y)), "edge plan");
+    const int64_t bytes = aprnet_conv333_rows_backward_workspace_bytes(B.h[0], B.dl[0], APRNET_PREC_BF16, cin, cout, slots, need_grad_input ? 1 : 0);
+    auto grad_tree = need_grad_input ? torch::empty({cin, B.max_tree}, grad_y.options()) : torch::Tensor();
+    auto grad_input = need_grad_input ? torch::empty({1, cin, n}, grad_y.options()) : torch::Tensor();
+    auto grad_weights = torch::empty_like(weights), dgamma = torch::empty({cout}, grad_y.options()), dbeta = torch::empty({cout}, grad_y.options());
+    auto ws = bytes_like(bytes, grad_y), norm_ws = bytes_like(aprnet_groupnorm_workspace_bytes(1, cout, (int) groups), grad_y);
+    auto partial = torch::empty({aprnet_conv333_rows_partial_elems(APRNET_PREC_BF16, cin, cout)}, grad_y.options());
+    const auto g = gamma.has_value() && gamma->defined() ? gamma->contiguous() : torch::Tensor(), be = beta.has_value() && beta->defined() ? beta->contiguous() : torch::Tensor();
+    check(aprnet_conv333_norm_backward(B.h[0], B.dl[0], cin, cout, slots, rows.data_ptr(), conv_out.data_ptr<float>(), n, (int) groups, g.defined() ? g.data_ptr<float>() : nullptr,
+                                       be.defined() ? be.data_ptr<float>() : nullptr, mean.data_ptr<float>(), rstd.data_ptr<float>(), relu ? 1 : 0, grad_y.data_ptr<float>(),
+                                       weights.data_ptr<float>(), need_grad_input ? grad_input.data_ptr<float>() : nullptr, n, grad_weights.data_ptr<float>(),
+                                       need_grad_input ? grad_tree.data_ptr<float>() : nullptr, B.max_tree, dgamma.data_ptr<float>(), dbeta.data_ptr<float>(),
+                                       partial.data_ptr<float>(), ws.data_ptr(), norm_ws.data_ptr(), stream_of(grad_y)), "conv333_norm_backward");
+    if (need_grad_input) fill_padding(grad_input, B.n);
+    return {grad_input, grad_weights, dgamma, dbeta};
+}
+
 // packed rows of an input whose forward call did not keep them (tree: its tree means per batch item, or undefined)
 static torch::Tensor conv333_pack(std::vector<APR*>& aprs, const torch::Tensor& input, const torch::Tensor& level_delta, int mode, const torch::Tensor& tree) {
     const Batch B(aprs, input, level_delta);
@@ -963,6 +994,8 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
     utils.def("number_parts", [](APR& a, int dl) { return a.number_parts(dl); }, "apr"_a, "level_delta"_a);
 
     py::module cuda = aprnet.def_submodule("cuda");
+    cuda.def("conv333_norm_backward", &conv333_norm_backward, "aprs"_a, "rows"_a, "weights"_a, "conv_out"_a, "grad_y"_a, "gamma"_a, "beta"_a, "mean"_a, "rstd"_a,
+             "groups"_a, "relu"_a, "level_delta"_a, "need_grad_input"_a);
     cuda.def("maxpool_forward_cuda", &maxpool_forward_cuda, "aprs"_a, "input"_a, "level_delta"_a);
     cuda.def("maxpool_backward_cuda", &maxpool_backward_cuda, "aprs"_a, "grad_output"_a, "max_indices"_a, "level_delta"_a);
     cuda.def("conv111_forward", &conv111_forward, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "", "bias"_a = py::none());

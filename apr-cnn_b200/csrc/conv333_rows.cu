@@ -46,10 +46,10 @@ int forward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int sl
     return aprnet_tc_gather_conv(a, dl, 0, cin, cout, slots, workspace, aprnet_tc_pad(cin), n, n + t, w, wp, bias, out, ld_out, st);
 }
 
-// `ws`: grad_bytes() bytes.  gin == null: no input gradient; gw == null: no weight gradient; fold_tree: grad_tree is folded into gin
+// `ws`: grad_bytes() bytes.  gout == null: `ws` starts with the packed rows of grad_output already (bf16, Cin > 4).  gin == null: no input gradient; gw == null: no weight gradient; fold_tree: grad_tree is folded into gin
 int backward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const void* rows, const float* gout, ll ld_out, const float* w,
                   float* gin, ll ld_in, float* gw, int accumulate, float* gtree, ll ld_tree, float* partial, void* ws, bool fold_tree, cudaStream_t st) {
-    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && gout && (gin || gw) && (!gin || (w && gtree)) && ws && (!gw || (rows && partial)), "bad argument");
+    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && (gout || (is_bf16(precision) && !aprnet_small_cin(cin) && 27 * a->number_parts(dl) + 1 < (1ll << 31))) && (gin || gw) && (!gin || (w && gtree)) && ws && (!gw || (rows && partial)), "bad argument");
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_out >= a->number_parts(dl) && (!gin || (ld_in >= a->number_parts(dl) && ld_tree >= a->tree_size(dl))), "leading dimension too small");
     const ll n = a->number_parts(dl);
@@ -57,7 +57,7 @@ int backward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int s
     const bool bf16 = is_bf16(precision);
     int rc;
     // the weight gradient of a first layer reads grad_output itself
-    if (gin || !aprnet_small_cin(cin)) {
+    if (gout && (gin || !aprnet_small_cin(cin))) {
         rc = bf16 ? aprnet_tc_pack_rows(gout, ld_out, n, nullptr, 0, 0, cout, gpad, ws, st) : aprnet_f32_pack_grad(a, dl, cout, gout, ld_out, ws, st);
         if (rc) return rc;
     }
@@ -187,4 +187,23 @@ extern "C" int aprnet_conv333_backward_tc(aprnet_apr* a, int dl, int cin, int co
     const int rc = aprnet_conv333_rows_pack(a, dl, APRNET_PREC_BF16, cin, in, ld_in, tree, ld_tree, tree_valid, workspace, stream);
     if (rc) return rc;
     return aprnet_conv333_backward_tc_rows(a, dl, cin, cout, slots, workspace, gout, ld_out, w, gin, ld_in, gw, gtree, ld_tree, partial, workspace, stream);
+}
+
+// GroupNorm + ReLU and the convolution in front of it, backward in one call for one batch item (float32 tensors, bf16 arithmetic, Cin > 4): conv_out is the
+// output of the convolution, n its row length; the gradient of it exists only as packed rows in `workspace`
+// (aprnet_conv333_rows_backward_workspace_bytes()).  norm_ws: aprnet_groupnorm_workspace_bytes(1, cout, groups)
+int aprnet_groupnorm_relu_backward_rows(int C, ll n, ll n_rows, int groups, const float* x, const float* dy, const float* gamma, const float* beta,
+                                        const float* mean, const float* rstd, float* dgamma, float* dbeta, int cpad, void* rows_out, double* ws, int relu, cudaStream_t st);
+
+extern "C" int aprnet_conv333_norm_backward(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* rows, const float* conv_out, int64_t n, int groups,
+                                            const float* gamma, const float* beta, const float* mean, const float* rstd, int relu, const float* grad_y, const float* w,
+                                            float* gin, int64_t ld_in, float* gw, float* gtree, int64_t ld_tree, float* dgamma, float* dbeta, float* partial,
+                                            void* workspace, void* norm_ws, void* stream) {
+    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && !aprnet_small_cin(cin) && gw && workspace && norm_ws && n >= a->number_parts(dl), "bad argument");
+    APRNET_DEVICE_CHECK(a);
+    cudaStream_t st = (cudaStream_t) stream;
+    const int rc = aprnet_groupnorm_relu_backward_rows(cout, n, a->number_parts(dl), groups, conv_out, grad_y, gamma, beta, mean, rstd, dgamma, dbeta,
+                                                       aprnet_tc_pad(cout), workspace, (double*) norm_ws, relu, st);
+    if (rc) return rc;
+    return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, rows, nullptr, n, w, gin, ld_in, gw, 0, gtree, ld_tree, partial, workspace, true, st);
 }

@@ -189,6 +189,15 @@ int aprnet_conv333_rows_backward(aprnet_apr* apr, int level_delta, int precision
                                  const void* packed_rows, const float* grad_output, int64_t ld_out, const float* weights,
                                  float* grad_input, int64_t ld_in, float* grad_weights, int accumulate, float* grad_tree,
                                  int64_t ld_tree, int fold_tree, float* partial, void* workspace, void* stream);
+/* GroupNorm + ReLU and the 3x3x3 convolution in front of it, backward in one call: one batch item, float32 tensors, bf16 arithmetic, cin > 4.
+ * conv_out (cout, n): output of the convolution, mean / rstd (groups) its statistics, grad_y (cout, n) the gradient behind the ReLU.  Same results as
+ * aprnet_groupnorm_relu_backward followed by aprnet_conv333_rows_backward (grad_weights written, tree gradient folded into grad_input), without the
+ * gradient of conv_out in memory.  grad_input null: not wanted.  norm_workspace: aprnet_groupnorm_workspace_bytes(1, cout, groups). */
+int aprnet_conv333_norm_backward(aprnet_apr* apr, int level_delta, int cin, int cout, int num_slots, const void* packed_input_rows, const float* conv_out,
+                                 int64_t n, int groups, const float* gamma, const float* beta, const float* mean, const float* rstd, int relu,
+                                 const float* grad_y, const float* weights, float* grad_input, int64_t ld_in, float* grad_weights, float* grad_tree,
+                                 int64_t ld_tree, float* grad_gamma, float* grad_beta, float* partial, void* workspace, void* norm_workspace, void* stream);
+
 
 /* ---- 3x3x3 convolution on the tensor cores (bf16 operands, fp32 accumulation) ------------------
  * No counterpart in the reference (its kernels are CUDA-core only).  Same contract as

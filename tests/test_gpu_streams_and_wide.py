@@ -1,0 +1,109 @@
+"""Sizes at which the copies of pooling, the GroupNorm kernels, the sums of the cross-level part and the wide forward layers change their shape."""
+import numpy as np
+import pytest
+import torch
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+def _apr(a):
+    import pyapr
+    apr = pyapr.apr_from_arrays(a)
+    apr.init_cuda()
+    return apr
+
+
+# rows of one tile and less, of a tile and one more, of many tiles per block; every alignment of a row comes up where n is odd
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("c,n", [(3, 1), (5, 31), (3, 993), (7, 1024), (4, 2049), (1, 300001)])
+def test_groupnorm_row_lengths(c, n, dtype):
+    from pyapr.aprnet import cuda as ops
+    torch.manual_seed(4)
+    x = torch.randn(2, c, n, dtype=dtype, device="cuda").requires_grad_(True)
+    m = ops.GroupNormReLU(1, c).to("cuda", dtype)
+    g = torch.randn_like(x)
+    y = m(x)
+    y.backward(g)
+    xd = x.detach().double().requires_grad_(True)
+    want = torch.relu(torch.nn.functional.group_norm(xd, 1, eps=1e-5))
+    # the ReLU's gate is taken from the computed output: a value within rounding of zero has either
+    want.backward(torch.where((y > 0) == (want > 0), g, torch.zeros_like(g)).double())
+    eps = 2.0 ** -23 if dtype == torch.float32 else 2.0 ** -52
+    assert float((y - want).abs().max()) <= 8 * eps * float(want.abs().max())
+    same = (y > 0) == (want > 0)
+    assert float((~same).sum()) <= 1e-4 * n * c + 1
+    if bool(same.all()):
+        assert float((x.grad - xd.grad).norm()) <= 64 * eps * float(xd.grad.norm()) + 1e-30
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+def test_pooling_keeps_coarse_particles(channels):
+    """More kept particles than a block copies, rows of odd length: they come through pooling and up-sampling bit for bit."""
+    import pyapr
+    from pyapr.aprnet import cuda as ops
+    a = H.blob_arrays((64, 96, 112), 40, 8)
+    apr = _apr(a)
+    for dtype in (torch.float32, torch.float64):
+        x = torch.randn(1, channels, a.n_particles + 5, dtype=dtype, device="cuda")
+        ld = torch.zeros(1, dtype=torch.int32)
+        pooled = ops.MaxPool()(x, [apr], ld)
+        up = ops.UpSampleConst()(pooled, [apr], ld)
+        n1 = int(pyapr.aprnet.utils.number_particles(apr, 1))
+        kept = int((up[0, 0, :a.n_particles] == x[0, 0, :a.n_particles]).cumprod(0).sum())       # leading entries that agree
+        assert kept > 4096 and torch.equal(pooled[..., :kept], x[..., :kept]) and torch.equal(up[..., :kept], x[..., :kept]) and pooled.shape[2] == n1
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 40), (16, 272), (24, 520)])
+def test_cross_level_sums_of_ragged_widths(cin, cout):
+    """Row widths that do not divide a block's threads and that take several columns of blocks, against the float64 kernels on operands that are exact in
+    bf16: what is left is the rounding of the sums (to bf16, 2^-9) and of the tree means."""
+    import pyapr
+    from _pyaprwrapper.aprnet import cuda as C
+    from _pyaprwrapper.data_containers import APRPtrVector
+    a = H.blob_arrays((48, 64, 64), 8, 5)
+    apr = _apr(a)
+    L = a.level_max - a.level_min + 1
+    n = int(pyapr.aprnet.utils.number_particles(apr, 0))
+    ld = torch.zeros(1, dtype=torch.int32)
+    torch.manual_seed(5)
+    w = (torch.randn(L, cout, cin, 3, 3, 3, device="cuda") / (27 * cout) ** 0.5).bfloat16().float()
+    g = torch.randn(1, cout, n, device="cuda").bfloat16().float()
+    x = torch.randn(1, cin, n, device="cuda")
+    v = APRPtrVector([apr])
+    _, rows = C.conv333_forward_keep_rows(v, x, w, ld, "bf16")
+    got = C.conv333_backward_with_rows(v, rows, w, g, ld, True, "bf16")[0]
+    want = C.conv333_backward(v, x.double(), w.double(), g.double(), ld)[0]
+    assert C.tc_error_flag() == 0
+    assert float((got - want).norm() / want.norm()) <= 2.0 ** -9
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 130), (48, 256), (64, 200), (160, 264)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_wide_forward_layers(cin, cout, bias):
+    """Several result tiles of 128: over runs of cells as by the kernel that gathers every tap, bit for bit; a bias of more than 256 channels takes the latter."""
+    import pyapr
+    from pyapr.aprnet import cuda as ops
+    from _pyaprwrapper.aprnet import cuda as C
+    for a in (H.arrays("odd"), H.blob_arrays((64, 96, 96), 30, 6)):
+        apr = _apr(a)
+        n = int(pyapr.aprnet.utils.number_particles(apr, 0))
+        torch.manual_seed(6)
+        conv = ops.APRConv(cin, cout, nstencils=2, bias=bias, precision="bf16").cuda()
+        x = torch.randn(1, cin, n, device="cuda")
+        ld = torch.zeros(1, dtype=torch.int32)
+        out = {}
+        with torch.no_grad():
+            for runs in (0, 1):
+                C.tc_set_option("runs", runs)
+                try:
+                    out[runs] = conv(x, [apr], ld)
+                finally:
+                    C.tc_set_option("runs", 1)
+        assert C.tc_error_flag() == 0 and torch.equal(out[0], out[1])
+        if bias:
+            with torch.no_grad():
+                plain = ops.APRConv(cin, cout, nstencils=2, bias=False, precision="bf16").cuda()
+                plain.weight.copy_(conv.weight)
+                assert torch.equal(out[1], plain(x, [apr], ld) + conv.bias.view(1, -1, 1))
