@@ -9,6 +9,7 @@
 // pyapr/aprnet/src/maxpool.hpp:70-230 and pyapr/aprnet/src/upsample.hpp:70-236.
 #include "apr_device.cuh"
 #include <algorithm>
+#include <cmath>
 
 namespace {
 
@@ -39,18 +40,22 @@ __device__ __forceinline__ void tree_node(const int32_t* __restrict__ child, con
         const T* src = v[s] >= 0 ? xin + v[s] : xtree + aprnet_dec_tree(v[s]);
         const ll ld = v[s] >= 0 ? ld_in : ld_coded;
 #pragma unroll
-        for (int k = 0; k < CH; ++k) vals[k][s] = (v[s] != APRNET_NONE && k < nch) ? src[k * ld] : T(0);
+        for (int k = 0; k < CH; ++k) vals[k][s] = (v[s] != APRNET_NONE && k < nch) ? src[k * ld] : (MAX ? T(-INFINITY) : T(0));
+    }
+    int first = 8;
+    if (MAX) {
+#pragma unroll
+        for (int s = 7; s >= 0; --s) if (v[s] != APRNET_NONE) first = s;
     }
     T* dst = tree + (ll) c0 * ld_tree + t;
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
         if (k >= nch) break;
-        if (MAX) {
-            bool seen = false;
+        if (MAX) {              // the first child's value, then what exceeds it (an absent child is -infinity); 0 where there is none
             T best = 0;
 #pragma unroll
             for (int s = 0; s < 8; ++s)
-                if (v[s] != APRNET_NONE && (!seen || vals[k][s] > best)) { best = vals[k][s]; seen = true; }
+                if (vals[k][s] > best || s == first) best = vals[k][s];
             dst[(ll) k * ld_tree] = best;
         } else {
             T s_part = 0, s_tree = 0;       // particles first, then tree children (fixed order)
