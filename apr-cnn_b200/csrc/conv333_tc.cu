@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
 #pragma unroll
                         for (int i = 0; i < NI; ++i) {
                             const int row = r0 + i * RW;
-                            cp_async16(smem_u32(a_s + t * A_TAP + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) src_row[i] * P.kpad);
+                            cp_async16_or_zero(smem_u32(a_s + t * A_TAP + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) src_row[i] * P.kpad, src_row[i] != (int32_t) P.zero_row);
                         }
                     }
                 }

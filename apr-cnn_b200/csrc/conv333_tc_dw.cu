@@ -177,13 +177,13 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
                     const int pl = i * (32 / GP) + lane / GP, r = wq * 32 + pl;
                     const int32_t a = __shfl_sync(0xffffffffu, g_row, pl);
                     const uint32_t off = NCOL == 32 ? r * 64 + ((cc ^ ((r >> 1) & 3)) << 4) : (cc >> 3) * G_ATOM + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
-                    if (cc < gpieces) cp_async16(smem_u32(g_s) + off, P.grows + (ll) a * P.gpad + cob * NCOL + cc * 8);
+                    if (cc < gpieces) cp_async16_or_zero(smem_u32(g_s) + off, P.grows + (ll) a * P.gpad + cob * NCOL + cc * 8, a != (int32_t) P.g_zero_row);
                 }
                 if (wq == 3) {                                         // rows 128 and 129
                     const int pl = lane / GP, r = PT + pl;
                     const int32_t a = __shfl_sync(0xffffffffu, g_extra, pl & 1);
                     const uint32_t off = NCOL == 32 ? r * 64 + ((cc ^ ((r >> 1) & 3)) << 4) : (cc >> 3) * G_ATOM + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
-                    if (pl < 2 && cc < gpieces) cp_async16(smem_u32(g_s) + off, P.grows + (ll) a * P.gpad + cob * NCOL + cc * 8);
+                    if (pl < 2 && cc < gpieces) cp_async16_or_zero(smem_u32(g_s) + off, P.grows + (ll) a * P.gpad + cob * NCOL + cc * 8, a != (int32_t) P.g_zero_row);
                 }
                 cp_async_arrive_noinc(smem_u32(dfull + db));
             }
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
 #pragma unroll
                     for (int pi = 0; pi < PB; ++pi) {
                         const int k = wq * 32 + (p0 + pi) * RPI + r0;
-                        if (c < cpieces) cp_async16(dst0 + k * 128 + ((cc ^ (k & 7)) << 4), src0 + (ll) r[pi] * P.xpad);
+                        if (c < cpieces) cp_async16_or_zero(dst0 + k * 128 + ((cc ^ (k & 7)) << 4), src0 + (ll) r[pi] * P.xpad, r[pi] != zero);
                     }
                 }
             }
