@@ -443,22 +443,20 @@ inline int pick_nt(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 12
 struct TcGeom { int kpad, ks, nt, n_tiles, order_nt; size_t rows_bytes, w_bytes; };
 
 int g_runs_off = 0;          // aprnet_tc_set_option("runs", 0 / 1): 0 = always this file's kernel, measurement switch
-int g_ks_override = 0;       // aprnet_tc_set_option("ks", n): channels per stage of this file's kernel with runs = 0, measurement switch
+int g_ks_override = 0;       // aprnet_tc_set_option("ks", n): channels per stage, measurement switch
 
 // tiles: tiles of 128 locations of the layer.  The width of the result tiles also fixes the channels and taps of a stage, that is the
 // order of the products; few locations get narrower tiles, so that all SMs work, in the order of the wide ones (order_nt).
-// 256 -> 256 channels on 1.9 k locations: 71 us with one 256-wide tile per 128 locations (15 blocks).  Wide layers take tiles of 128 in
-// stages of three taps, an order that the run kernel has too: 128 -> 128 on 0.55 M locations 0.61 -> 0.41 ms, 256 -> 128 1.15 -> 0.79 ms; 256 -> 256 on
-// 121 k locations 0.42 (one tile of 256, rows gathered once per tap) -> 0.31 ms (two tiles, rows gathered once per slot each).
+// 256 -> 256 channels on 1.9 k locations: 71 us with one 256-wide tile per 128 locations (15 blocks).
 TcGeom tc_geometry(ll rows, int k_dim, int n_dim, int slots, ll tiles, bool free_order) {
     TcGeom g;
     g.kpad = pad_to(k_dim, 16);
-    g.nt = g.order_nt = std::min(128, pick_nt(n_dim));
-    g.ks = (g.kpad % 64 == 0) ? 64 : ((g.kpad % 32 == 0) ? 32 : 16);
+    g.nt = g.order_nt = free_order ? std::min(128, pick_nt(n_dim)) : pick_nt(n_dim);
+    g.ks = (g.kpad % 64 == 0 && g.nt <= 128) ? 64 : ((g.kpad % 32 == 0) ? 32 : 16);
     // 64 output channels: stages of 3 taps x 32 channels (5 ring slots, 4 producer groups) measured 3-10 % faster than
-    // 2 taps x 64 channels (3 slots, 2 groups); for 32 outputs and in the cross-level part of 128 the 64-channel stages win
-    if (g.ks == 64 && (g.nt == 64 || (g.nt == 128 && !free_order))) g.ks = 32;
-    if (g_ks_override > 0 && g_runs_off && g.kpad % g_ks_override == 0) g.ks = g_ks_override;
+    // 2 taps x 64 channels (3 slots, 2 groups); for 32 and 128 outputs the 64-channel stages win
+    if (g.nt == 64 && g.ks == 64) g.ks = 32;
+    if (g_ks_override > 0 && g.kpad % g_ks_override == 0 && (g_ks_override < 64 || g.nt <= 128)) g.ks = g_ks_override;
     while (g.nt > 32 && tiles * ((n_dim + g.nt - 1) / g.nt) < 148) g.nt /= 2;
     if (free_order) { g.order_nt = g.nt; if (g.nt == 64 && g.ks == 64) g.ks = 32; }
     g.n_tiles = (n_dim + g.nt - 1) / g.nt;
@@ -487,7 +485,8 @@ inline int ws_stages(int nt, int ks, int taps) {
     X(32, 16, 1, 1) X(32, 16, 3, 1) X(32, 16, 9, 2) X(32, 32, 1, 1) X(32, 32, 3, 1) X(32, 32, 3, 2) X(32, 32, 9, 4) \
     X(32, 64, 1, 1) X(32, 64, 1, 2) X(32, 32, 2, 2) X(32, 64, 3, 2) X(32, 64, 3, 4) \
     X(64, 16, 1, 1) X(64, 16, 3, 1) X(64, 16, 9, 2) X(64, 32, 1, 1) X(64, 32, 3, 2) X(64, 32, 2, 2) X(64, 64, 1, 1) X(64, 64, 1, 2) X(64, 64, 2, 2) X(64, 64, 2, 4) X(64, 64, 3, 4) \
-    X(128, 16, 1, 1) X(128, 16, 3, 2) X(128, 32, 1, 1) X(128, 32, 2, 2) X(128, 32, 3, 4) X(128, 64, 1, 1) X(128, 64, 1, 2) X(128, 64, 2, 4)
+    X(128, 16, 1, 1) X(128, 16, 3, 2) X(128, 32, 1, 1) X(128, 32, 2, 2) X(128, 32, 3, 4) X(128, 64, 1, 1) X(128, 64, 1, 2) X(128, 64, 2, 4) \
+    X(256, 16, 1, 1) X(256, 16, 3, 2) X(256, 32, 1, 1) X(256, 32, 2, 2) X(256, 32, 2, 4)
 
 // the same with the last TT taps of every stage fetched by the TMA unit
 #define TC_TMA_VARIANTS(X) \
@@ -552,7 +551,7 @@ int make_row_map(CUtensorMap* map, const void* rows, ll n_rows, int kpad, int ks
 template<int NT, int KS, int TAPS, int WPS, int TT>
 int launch_tc_ws(const TcParams& P, int total_tiles, cudaStream_t st, const char* pname) {
     constexpr size_t STAGE = (size_t) TAPS * ((size_t) TILE_M * KS * 2 + (size_t) NT * KS * 2);
-    constexpr int NACC = 4;                          // accumulators in flight: the SM's 512 TMEM columns hold four of the widest
+    constexpr int NACC = NT <= 128 ? 4 : 2;          // accumulators in flight: the SM's 512 TMEM columns, at most 4
     auto kern = conv333_tc_ws_kernel<NT, KS, TAPS, WPS, TT, NACC>;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -627,7 +626,7 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
     if ((rc = aprnet_pack_weights(a, dl, true, w, slots, cin, cout, backward, g.nt, g.n_tiles, g.kpad, wp, st))) return rc;
     char pname[64];
     snprintf(pname, sizeof(pname), "%s:ci%d:co%d:dl%d", backward ? "conv333_tc_bwd_gather" : "conv333_tc_fwd", cin, cout, dl);
-    const int run_order = g_runs_off ? 0 : aprnet_tc_runs_order(backward, g.kpad, g.ks, bias != nullptr, g.n_tiles * g.nt);
+    const int run_order = g_runs_off ? 0 : aprnet_tc_runs_order(backward, g.kpad, g.order_nt, g.ks);
     if (run_order) return aprnet_tc_run_conv(a, dl, backward, slots, g.nt, run_order, rows, g.kpad, tree_base, zero_row, wp, bias, out, ld_out, n_dim, g_error_flag_dev, st, pname);
     TcParams P;
     P.segs = make_seg_table(aprnet_segments(a, dl, slots, false), TILE_M);

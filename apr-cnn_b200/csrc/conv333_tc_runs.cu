@@ -1,5 +1,5 @@
-// 3x3x3 particle convolution on the tensor cores over runs of cells (bf16 operands, fp32 accumulation): forward pass and same-level input
-// gradient.
+// 3x3x3 particle convolution on the tensor cores over runs of cells (bf16 operands, fp32 accumulation): forward pass of layers with at
+// most 128 result channels (above 64 only where all source channels are in one stage), same-level input gradient of any width.
 //
 // The kernel of conv333_tc.cu gathers every source row once per tap, 27 rows per location.  Here the M dimension of a tile is not
 // 128 locations but 128 * H consecutive slots of the run plan (run_plan.cu).  For each of the 9 rows of cells (dz, dx) the tile's
@@ -7,8 +7,8 @@
 // tap dy starts dy rows further.  (The swizzle of a K-major operand is a function of the shared-memory address, so a start address
 // inside the pattern is an ordinary one.)  That is 9 x 1.07 .. 1.27 gathered rows per location instead of 27; slots without a
 // location are the price, 7 to 27 % more multiply-adds.  Each weight tile that is fetched meets H blocks of 128 rows.
-// What bounds it now: the data pipe of the SM's shared memory.  For 32 -> 32 channels the tensor core's operand reads keep it busy for 56 % of
-// the time and the load-store unit (copies, whose sectors land one by one, shuffles, stores of the results) for 51 %.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
+// What bounds it now: rows and weights arrive from L2 at 6.5 to 7 TB/s (64 -> 64 channels), and the MMAs of narrow tiles read
+// shared memory for longer than they multiply.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
 // 32 -> 32 layer that takes 0.48.)
 //
 // Every result of the forward pass is the same sequence of MMAs (neighbour row, channel block, dy, 16 channels) as in
@@ -340,12 +340,14 @@ inline int pick_h(const RunParams& P, int nt, int ks, int max_h, int sms) {
 
 } // namespace
 
-// Channels between two changes of dy (the order of the products) of this kernel for kpad source channels; 0: not this kernel, which holds the
-// bias of at most MAX_N channels.  ks: channels per stage that conv333_tc.cu takes for the layer.  The forward pass keeps its order, stages of
-// `ks` channels that hold three taps.  The input gradient is free: nothing that follows depends on its last bit.
-int aprnet_tc_runs_order(int backward, int kpad, int ks, bool bias, int n) {
-    if (bias && n > MAX_N) return 0;
-    return backward ? (kpad % 32 == 0 ? 32 : 16) : ks;
+// Channels between two changes of dy (the order of the products) of this kernel for kpad source channels; 0: not this kernel.
+// nt_order, ks: tile width and channels per stage that conv333_tc.cu takes for the layer.  The forward pass keeps its order: stages of
+// `ks` channels that hold three taps for nt_order <= 64 (the same order as here) but fewer for wider tiles (the same only when all
+// channels are in one stage of one tap).  The input gradient is free: nothing that follows depends on its last bit.
+int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int ks) {
+    if (backward) return kpad % 32 == 0 ? 32 : 16;
+    if (nt_order <= 64) return ks;
+    return nt_order == 128 && kpad == ks ? ks : 0;
 }
 
 int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, ll tree_base, ll zero_row, const void* wp,
@@ -375,12 +377,12 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     RUN_CASE(32, 16, 16, 1, 2) RUN_CASE(32, 16, 16, 2, 2) RUN_CASE(32, 16, 16, 4, 2) RUN_CASE(32, 16, 16, 8, 4)
     RUN_CASE(32, 32, 32, 1, 2) RUN_CASE(32, 32, 32, 2, 2) RUN_CASE(32, 32, 32, 4, 2)
     RUN_CASE(32, 64, 64, 1, 2) RUN_CASE(32, 64, 64, 2, 2) RUN_CASE(32, 64, 64, 4, 4)
-    RUN_CASE(32, 64, 32, 1, 2) RUN_CASE(32, 64, 32, 2, 2) RUN_CASE(32, 64, 32, 4, 4)
+    RUN_CASE(32, 64, 32, 1, 2) RUN_CASE(32, 64, 32, 2, 2) RUN_CASE(32, 64, 32, 4, 4) RUN_CASE(64, 64, 64, 1, 2) RUN_CASE(64, 64, 64, 2, 4) RUN_CASE(64, 64, 64, 4, 4)
     RUN_CASE(64, 16, 16, 1, 2) RUN_CASE(64, 16, 16, 2, 2) RUN_CASE(64, 16, 16, 4, 2)
     RUN_CASE(64, 32, 32, 1, 2) RUN_CASE(64, 32, 32, 2, 2) RUN_CASE(64, 32, 32, 4, 2)
     RUN_CASE(64, 64, 32, 1, 2) RUN_CASE(64, 64, 32, 2, 4) RUN_CASE(64, 64, 32, 4, 4)
     RUN_CASE(128, 16, 16, 1, 2) RUN_CASE(128, 16, 16, 2, 2) RUN_CASE(128, 32, 32, 1, 2) RUN_CASE(128, 32, 32, 2, 2)
-    RUN_CASE(128, 64, 32, 1, 4) RUN_CASE(128, 64, 32, 2, 4)
+    RUN_CASE(128, 64, 32, 1, 4) RUN_CASE(128, 64, 32, 2, 4) RUN_CASE(128, 64, 64, 1, 4) RUN_CASE(128, 64, 64, 2, 4)
 #undef RUN_CASE
     aprnet_set_error("conv333 tensor-core path: unsupported run geometry nt=%d ks=%d order=%d h=%d", nt, ks, order, h);
     return APRNET_ERR_UNSUPPORTED;
