@@ -31,6 +31,8 @@ inline SegTable make_seg_table(const std::vector<Segment>& segs, ll tile) {
     return t;
 }
 
+constexpr int SMALL_STEP = 4 * 30;       // slots whose results a block of the forward kernel yields per tile
+
 struct alignas(16) F4 { float a[4]; };
 
 __device__ __forceinline__ ll resolve_row(int32_t v, ll n, ll zero_row) {
@@ -47,14 +49,16 @@ __global__ void small_stage_kernel(const float* __restrict__ x, ll ld_x, ll n, c
         vals[(ll) ci * R + r] = r < n ? x[(ll) ci * ld_x + r] : (r < n + t ? tree[(ll) ci * ld_tree + (r - n)] : 0.f);
 }
 
-// forward: thread = output location x block of 32 output channels; weights of the level's stencil in shared memory as [tap][ci][32],
-// read four at a time.  What bounds it: the latency of the gathers, and per block the staging of the weights (27 strided values per
-// thread row, as many cache lines as the gathers of a tile touch).  So a block takes up to eight tiles with one staging, and the taps
-// go in thirds: the next third's table entries are on their way during the multiply-adds.  1 -> 32 channels: 28 M locations 5.5 -> 3.6 ms,
-// 3.5 M 0.71 -> 0.53; 2 -> 32: 9.3 -> 6.8.  (Two locations per thread, half the weight reads: 5.7 ms, too few warps.)
-template<int CIN, int TAPS>
-__global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable segs, int tiles, const int32_t* __restrict__ nbr, ll N, ll T,
-                                                                    const float* __restrict__ vals, const float* __restrict__ w,
+// forward: thread = slot of the run plan x block of 32 output channels; weights of the level's stencil in shared memory as [tap][ci][32],
+// read four at a time.  A lane loads the 9 values that lie beside its cell (dz, dx) and gets those of the y neighbours from the lanes next to it, so a warp
+// yields 30 slots and gathers 9 values per slot where the neighbour table needs 27 entries and 27 values per location.  What bounds it is the latency of
+// these gathers: the table entries of the next tile are on their way during the multiply-adds, and a block takes up to eight tiles with one
+// staging of the weights.  1 -> 32 channels on 3.5 M locations 522 -> 311 us against one thread per
+// location and the neighbour table, 2 -> 32 889 -> 596, 4 -> 40 on 1.9 M 1415 -> 1124; 1 -> 16 on 7 k locations 10.7 -> 6.1.  (Paired multiply-adds: 0 to 10 % slower.)
+// The chain of multiply-adds of a result is channel by channel, tap by tap.
+template<int CIN>
+__global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable segs, int tiles, const int32_t* __restrict__ src, ll S, const int32_t* __restrict__ loc,
+                                                                    ll N, ll T, const float* __restrict__ vals, const float* __restrict__ w,
                                                                     int cout, const float* __restrict__ bias, float* __restrict__ out, ll ld_out) {
     __shared__ F4 ws[27 * CIN * 8];
     __shared__ float bias_s[32];
@@ -68,41 +72,46 @@ __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable seg
     }
     if (threadIdx.x < 32) bias_s[threadIdx.x] = bias && co0 + (int) threadIdx.x < cout ? bias[co0 + threadIdx.x] : 0.f;
     __syncthreads();
-    const ll R = N + T + 1, end = segs.end[seg];
-    ll p = segs.begin[seg] + (ll) (blockIdx.x - segs.tile_begin[seg]) * 128 * tiles + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const ll R = N + T + 1, begin = segs.begin[seg], end = segs.end[seg];
+    // the warp's first tile: lane 0 is the slot in front of its 30; consecutive tiles of a block are SMALL_STEP slots apart
+    ll s = begin + (ll) (blockIdx.x - segs.tile_begin[seg]) * SMALL_STEP * tiles + (threadIdx.x >> 5) * 30 - 1 + lane;
     const int nco = min(32, cout - co0);
-    for (int i = 0; i < tiles && p < end; ++i, p += 128) {
+    int32_t rows[9], p_next;
+    auto request = [&]() {                             // row numbers fit 32 bits (aprnet_rows_overflow)
+        const bool in = s >= begin && s < end;
+#pragma unroll
+        for (int d = 0; d < 9; ++d) rows[d] = in ? __ldg(src + d * S + s) : APRNET_NONE;
+        p_next = in && lane > 0 && lane < 31 ? __ldg(loc + s) : -1;
+    };
+    request();
+    for (int i = 0; i < tiles && s - lane + 1 < end; ++i) {
         float acc[32];
 #pragma unroll
         for (int o = 0; o < 32; ++o) acc[o] = 0.f;
-        // TAPS table entries and then TAPS values are requested before any is used; row numbers fit 32 bits (aprnet_rows_overflow)
-        int32_t rows[TAPS];
-        auto request = [&](int tap0) {
-            const int32_t* e = nbr + (ll) tap0 * N + p;
+        int32_t at[9];
 #pragma unroll
-            for (int t = 0; t < TAPS; ++t) rows[t] = (int32_t) resolve_row(__ldg(e + (ll) t * N), N, N + T);
-        };
-        request(0);
+        for (int d = 0; d < 9; ++d) at[d] = (int32_t) resolve_row(rows[d], N, N + T);
+        const int32_t p = p_next;
+        s += SMALL_STEP;
+        float v[9];
+#pragma unroll
+        for (int d = 0; d < 9; ++d) v[d] = __ldg(vals + at[d]);
+        request();
 #pragma unroll 1
         for (int ci = 0; ci < CIN; ++ci) {
-            const float* vc = vals + (ll) ci * R;
-#pragma unroll 1
-            for (int tap0 = 0; tap0 < 27; tap0 += TAPS) {
-                float v[TAPS];
 #pragma unroll
-                for (int t = 0; t < TAPS; ++t) v[t] = __ldg(vc + rows[t]);
-                if (TAPS < 27) {
-                    if (tap0 + TAPS < 27) request(tap0 + TAPS);
-                    else if (ci + 1 < CIN) request(0);
-                }
+            for (int d = 0; d < 9; ++d) {
+                const float beside[3] = {__shfl_up_sync(0xffffffffu, v[d], 1), v[d], __shfl_down_sync(0xffffffffu, v[d], 1)};
+                if (ci + 1 < CIN) v[d] = __ldg(vals + (ll) (ci + 1) * R + at[d]);
 #pragma unroll
-                for (int t = 0; t < TAPS; ++t) {
-                    const F4* wr = ws + ((tap0 + t) * CIN + ci) * 8;
+                for (int dy = 0; dy < 3; ++dy) {
+                    const F4* wr = ws + ((d * 3 + dy) * CIN + ci) * 8;
 #pragma unroll
                     for (int o4 = 0; o4 < 8; ++o4) {
                         const F4 q = wr[o4];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) acc[4 * o4 + k] = fmaf(v[t], q.a[k], acc[4 * o4 + k]);
+                        for (int k = 0; k < 4; ++k) acc[4 * o4 + k] = fmaf(beside[dy], q.a[k], acc[4 * o4 + k]);
                     }
                 }
             }
@@ -111,6 +120,7 @@ __global__ void __launch_bounds__(128) conv333_small_forward_kernel(SegTable seg
 #pragma unroll
             for (int o = 0; o < 32; ++o) acc[o] += bias_s[o];
         }
+        if (p < 0) continue;
         float* dst = out + (ll) co0 * ld_out + p;
         if (nco == 32) {
 #pragma unroll
@@ -247,24 +257,21 @@ int aprnet_small_stage(const float* x, ll ld_x, ll n, const float* tree, ll ld_t
 }
 
 int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, const float* bias, float* out, ll ld_out, cudaStream_t st) {
-    const AprPlan* plan = aprnet_get_plan(a, dl, st);
-    if (!plan) return APRNET_ERR_CUDA;
-    const std::vector<Segment> list = aprnet_segments(a, dl, slots, false);
-    ll total = 0;
-    for (const Segment& g : list) total += g.end - g.begin;
-    // several tiles per block once eight blocks per SM have one each; where two blocks per SM hold everything, the time is that of one
-    // tile and all its taps are requested at once (2 -> 32 channels on 7 k locations: 17 us, in thirds 21)
-    const ll tiles = aprnet_ceil_div(total, 128), groups = aprnet_ceil_div(cout, 32);
+    const RunPlan* rp = aprnet_get_run_plan(a, dl, st);
+    if (!rp) return APRNET_ERR_CUDA;
+    std::vector<Segment> list = aprnet_segments(a, dl, slots, false);
+    for (Segment& g : list) { g.begin = rp->level_begin[g.level]; g.end = rp->level_begin[g.level + 1]; }
+    // several tiles per block once eight blocks per SM have one each
+    const ll tiles = aprnet_ceil_div(rp->n_slots, SMALL_STEP), groups = aprnet_ceil_div(cout, 32);
     const int per_block = (int) std::min<ll>(8, std::max<ll>(1, tiles * groups / (148 * 8)));
-    const bool few = tiles * groups <= 148 * 2;
-    const SegTable segs = make_seg_table(list, 128 * per_block);
+    const SegTable segs = make_seg_table(list, SMALL_STEP * per_block);
     if (segs.tile_begin[segs.n] == 0) return APRNET_OK;
     dim3 grid((unsigned) segs.tile_begin[segs.n], (unsigned) groups);
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_small_fwd:ci%d:co%d:dl%d", cin, cout, dl);
     AprnetProfScope _prof(pname, st);
-#define SMALL_CASE(CIN_) case CIN_: (few ? conv333_small_forward_kernel<CIN_, 27> : conv333_small_forward_kernel<CIN_, 9>)<<<grid, 128, 0, st>>>( \
-        segs, per_block, plan->nbr, plan->n, plan->tree_size, vals, w, cout, bias, out, ld_out); break;
+#define SMALL_CASE(CIN_) case CIN_: conv333_small_forward_kernel<CIN_><<<grid, 128, 0, st>>>(segs, per_block, rp->src, rp->n_slots, rp->loc, a->number_parts(dl), \
+        a->tree_size(dl), vals, w, cout, bias, out, ld_out); break;
     switch (cin) {
         SMALL_CASE(1) SMALL_CASE(2) SMALL_CASE(3) SMALL_CASE(4)
         default: aprnet_set_error("small-Cin path called with cin = %d", cin); return APRNET_ERR_ARG;
