@@ -82,7 +82,7 @@ def test_cross_level_sums_of_ragged_widths(cin, cout):
 @pytest.mark.parametrize("cin,cout", [(16, 130), (48, 256), (64, 200), (160, 264)])
 @pytest.mark.parametrize("bias", [False, True])
 def test_wide_forward_layers(cin, cout, bias):
-    """Several result tiles of 128: over runs of cells as by the kernel that gathers every tap, bit for bit; a bias of more than 256 channels takes the latter."""
+    """More than 128 result channels, with and without a bias of any width: the same bits with and without gathers over runs of cells."""
     import pyapr
     from pyapr.aprnet import cuda as ops
     from _pyaprwrapper.aprnet import cuda as C
