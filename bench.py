@@ -160,7 +160,7 @@ def unet_conv_layers(base, depth):
     return layers
 
 
-GN_BYTES = {"groupnorm_stats": 4.0, "groupnorm_relu_apply": 8.0, "groupnorm_bwd_reduce": 8.0, "groupnorm_bwd_apply": 12.0}
+GN_BYTES = {"groupnorm_stats": 4.0, "groupnorm_relu_apply": 8.0, "groupnorm_bwd_reduce": 8.0, "groupnorm_bwd_apply": 12.0, "groupnorm_bwd_apply_rows": 10.0}
 
 
 def kernel_table(prof, steps, nparts, ntree, peaks, layers, bf16, fma_tflops=None):
@@ -171,7 +171,8 @@ def kernel_table(prof, steps, nparts, ntree, peaks, layers, bf16, fma_tflops=Non
     input gradient or weight gradient);
     4 * c * (N + 2 T) + 36 T for a tree fill (children read, node written and read by its parent, child table) and
     4 * c * (2 N + 2 T) + 36 T for its adjoint; 6 * c * rows for a packing pass; 4 / 8 / 8 / 12 bytes per element for
-    the four GroupNorm passes.  Pooling / up-sampling (part kernel, part strided copy) and the per-(target, tap) sums of the
+    the four GroupNorm passes, 10 for the last one where it leaves packed rows (the layers behind a bf16 3x3x3 convolution of more than
+    four channels, whose gradient is then not packed by itself).  Pooling / up-sampling and the per-(target, tap) sums of the
     cross-level input gradient are listed with their time only."""
     e_in = 2.0 if bf16 else 4.0
     ridge = peaks["tflops"] * 1e12 / (peaks["hbm_gbs"] * 1e9)
@@ -179,10 +180,11 @@ def kernel_table(prof, steps, nparts, ntree, peaks, layers, bf16, fma_tflops=Non
     c111 = [(ci, co, dl) for k, ci, co, dl in layers if k == "111"]
     gn = [(co, dl) for k, ci, co, dl in layers[:-1]]                          # every convolution but the head is followed by GroupNorm
     first = c333[0]
+    joint = [(co, dl) for ci, co, dl in c333 if ci > 4] if "groupnorm_bwd_apply_rows" in prof else []
     agg = {
         "tree_mean_fwd": sum(4.0 * ci * (nparts[dl] + 2 * ntree[dl]) + 36.0 * ntree[dl] for ci, co, dl in c333),
         "tree_mean_bwd": sum(4.0 * ci * (2 * nparts[dl] + 2 * ntree[dl]) + 36.0 * ntree[dl] for ci, co, dl in c333 if (ci, co, dl) != first),
-        "pack_rows_bf16": sum(6.0 * ci * (nparts[dl] + ntree[dl]) for ci, co, dl in c333 if ci > 4) + sum(6.0 * co * nparts[dl] for ci, co, dl in c333 if (ci, co, dl) != first),
+        "pack_rows_bf16": sum(6.0 * ci * (nparts[dl] + ntree[dl]) for ci, co, dl in c333 if ci > 4) + (0.0 if joint else sum(6.0 * co * nparts[dl] for ci, co, dl in c333 if (ci, co, dl) != first)),
     }
     # 1x1x1 passes: the tensor-core forward / input-gradient kernel carries its shape in the name (conv111_tc:ci..:co..:dl..,
     # channel roles swapped in the input gradient); the CUDA-core kernel "conv111" ran the layers no such name covers.
@@ -199,7 +201,8 @@ def kernel_table(prof, steps, nparts, ntree, peaks, layers, bf16, fma_tflops=Non
         dw111 = None                                                   # mixed: no per-name split
     agg["conv111_dw"] = agg["conv111_tc_dw"] = dw111
     for name, bpe in GN_BYTES.items():
-        agg[name] = sum(bpe * c * nparts[dl] for c, dl in gn)
+        agg[name] = sum(bpe * c * nparts[dl] for c, dl in (joint if name.endswith("_rows") else gn))
+    agg["groupnorm_bwd_apply"] -= sum(GN_BYTES["groupnorm_bwd_apply"] * c * nparts[dl] for c, dl in joint)
     rows = []
     for name, (calls, ms) in sorted(prof.items(), key=lambda kv: -kv[1][1]):
         parts = name.split(":")
