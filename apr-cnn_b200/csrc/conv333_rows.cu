@@ -130,6 +130,7 @@ extern "C" int aprnet_conv333_rows_backward(aprnet_apr* a, int dl, int precision
                                             const float* w, float* gin, int64_t ld_in, float* gw, int accumulate, float* gtree, int64_t ld_tree, int fold_tree,
                                             float* partial, void* workspace, void* stream) {
     APRNET_ARG_CHECK(precision_ok(precision), "unknown precision");
+    APRNET_ARG_CHECK(gout, "bad argument");
     return backward_rows(a, dl, precision, cin, cout, slots, rows, gout, ld_out, w, gin, ld_in, gw, accumulate, gtree, ld_tree, partial, workspace, fold_tree != 0, (cudaStream_t) stream);
 }
 
@@ -162,7 +163,7 @@ static void* grad_area(const aprnet_apr* a, int dl, int cin, void* workspace) {
 extern "C" int aprnet_conv333_backward_tc_rows(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* packed_input_rows,
                                                const float* gout, int64_t ld_out, const float* w, float* gin, int64_t ld_in, float* gw,
                                                float* gtree, int64_t ld_tree, float* partial, void* workspace, void* stream) {
-    APRNET_ARG_CHECK(gw, "bad argument");
+    APRNET_ARG_CHECK(gw && gout, "bad argument");
     return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, 1, gtree, ld_tree, partial,
                          grad_area(a, dl, cin, workspace), true, (cudaStream_t) stream);
 }
@@ -172,7 +173,7 @@ extern "C" int aprnet_conv333_backward_tc_rows(aprnet_apr* a, int dl, int cin, i
 extern "C" int aprnet_conv333_backward_tc_rows_pretree(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* packed_input_rows,
                                                        const float* gout, int64_t ld_out, const float* w, float* gin, int64_t ld_in, float* gw,
                                                        float* gtree, int64_t ld_tree, float* partial, void* workspace, void* stream) {
-    APRNET_ARG_CHECK(gw, "bad argument");
+    APRNET_ARG_CHECK(gw && gout, "bad argument");
     return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, packed_input_rows, gout, ld_out, w, gin, ld_in, gw, 1, gtree, ld_tree, partial,
                          grad_area(a, dl, cin, workspace), false, (cudaStream_t) stream);
 }
