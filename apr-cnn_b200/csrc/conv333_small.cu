@@ -3,7 +3,7 @@
 // carry one useful value in 32 bytes and the 27 x Cin x Cout products per location are far too few to
 // amortise a gathered operand tile.  Values are read from a channel-major buffer
 //     vals[ci][r],  r in [0, N) particles, [N, N + T) tree means, r = N + T: zero
-// through the cached neighbour table, so a tap is one 4-byte load per input channel.
+// through the run plan (forward) or the cached neighbour table (weight gradient), one 4-byte load per entry and input channel.
 // Arithmetic: pyapr/aprnet/src/helpers.hpp:505-575 (forward) and :624-702 (weight gradient).
 #include "apr_device.cuh"
 #include <algorithm>
