@@ -363,51 +363,77 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
             ahead.next(P);
         };
         for (int it = 0; it < NIDX; ++it) { request_idx(it); publish_idx(it); }
-        for (int it = 0; it < my_tiles; ++it, walk.next(P)) {
+        // target mode: what this thread's row of the tile is added to (-1: none)
+        auto target_of = [&](int it) { return P.out_map && it < my_tiles && walk.p0() + row < walk.hi ? __ldg(P.out_map + walk.p0() + row) : -1; };
+        int32_t target = target_of(0);
+        for (int it = 0; it < my_tiles; ++it) {
             const ll p = walk.p0() + row;
             const bool valid = p < walk.hi;
-            float* acc_dst = nullptr; ll acc_ld = 0;
-            if (P.out_map && valid) {
-                const ll t = P.out_map[p];
-                acc_dst = t < P.out_split ? P.out + t : P.out2 + (t - P.out_split);
-                acc_ld = t < P.out_split ? P.ld_out : P.ld_out2;
-            }
             const uint32_t acc = (uint32_t) it % NACC, acc_use = (uint32_t) it / NACC;
             request_idx(it + NIDX);       // lands while this warp waits for the accumulator
+            const int n0 = walk.ntile * NT, n_end = min(NT, P.n_dim - n0);
+            float held[2][16];            // target mode: what the target holds, 32 channels ahead
+            auto request_held = [&](float (&h)[16], int c0) {
+                ll ld = target < P.out_split ? P.ld_out : P.ld_out2;
+                asm volatile("" : "+l"(ld));              // else its multiples are kept for the whole loop: 30 registers, spilled
+                const float* src = (target < P.out_split ? P.out + target : P.out2 + (target - P.out_split)) + (n0 + c0) * ld;
+#pragma unroll
+                for (int jj = 0; jj < 16; ++jj, src += ld) h[jj] = target >= 0 && c0 + jj < n_end ? __ldcg(src) : 0.f;
+            };
+            if (P.out_map) { request_held(held[0], 0); request_held(held[1], 16); }
             if (!mbar_wait_warp(smem_u32(tmem_full + acc), acc_use & 1, abort_flag)) { failed = true; break; }
             tc_fence_after();
+            const uint32_t taddr = tmem_d + ((uint32_t) (q * 32) << 16) + acc * NT;
+            if (P.out_map) {
+                // This thread is the only writer of its target in this launch, so the order of the additions is fixed.  A load, an addition and a store:
+                // an addition in L2 (red.global.add.f32) would flush subnormal values.  What costs is the latency of the scattered loads, so
+                // 32 channels are requested before the wait for the products and each next 16 before the stores of the last.  Cross-level part of
+                // 32 -> 32, 64 -> 32 (3.5 M locations), 64 -> 64, 128 -> 64 (level delta 1): 508, 697, 289, 415 us with all loads after the wait and tiles that were
+                // searched, 335, 492, 237, 313 with 16 channels ahead, now 303, 445, 234, 308 (additions in L2: 277, 321, 220, 287; prefetching the
+                // targets of a later tile into L2: no change).
+                auto add = [&](float (&h)[16], int c0) {
+                    uint32_t r[16];
+                    tmem_ld16(taddr + c0, r);
+                    tmem_ld_wait();
 #pragma unroll
-            for (int c0 = 0; c0 < NT; c0 += 32) {
-                uint32_t r[32];
-                tmem_ld32(tmem_d + ((uint32_t) (q * 32) << 16) + acc * NT + c0, r);
-                tmem_ld_wait();
-                if (P.bias) {                // apart from the stores: a choice per element there cost the whole kernel 10 to 20 %
+                    for (int jj = 0; jj < 16; ++jj) r[jj] = __float_as_uint(h[jj] + __uint_as_float(r[jj]));
+                    request_held(h, c0 + 32);
+                    ll ld = target < P.out_split ? P.ld_out : P.ld_out2;
+                    asm volatile("" : "+l"(ld));
+                    float* dst = (target < P.out_split ? P.out + target : P.out2 + (target - P.out_split)) + (n0 + c0) * ld;
 #pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
-                        const int n = walk.ntile * NT + c0 + jj;
-                        if (n < P.n_dim) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + __ldg(P.bias + n));
+                    for (int jj = 0; jj < 16; ++jj, dst += ld)
+                        if (target >= 0 && c0 + jj < n_end) *dst = __uint_as_float(r[jj]);
+                };
+#pragma unroll 1
+                for (int c0 = 0; c0 < n_end; c0 += 32) { add(held[0], c0); add(held[1], c0 + 16); }
+            } else {
+#pragma unroll
+                for (int c0 = 0; c0 < NT; c0 += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + c0, r);
+                    tmem_ld_wait();
+                    if (P.bias) {            // apart from the stores: a choice per element there cost the whole kernel 10 to 20 %
+#pragma unroll
+                        for (int jj = 0; jj < 32; ++jj) {
+                            const int n = n0 + c0 + jj;
+                            if (n < P.n_dim) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + __ldg(P.bias + n));
+                        }
                     }
-                }
-                if (valid && !P.out_map) {
+                    if (valid) {
 #pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
-                        const int n = walk.ntile * NT + c0 + jj;
-                        if (n < P.n_dim) P.out[(ll) n * P.ld_out + p] = __uint_as_float(r[jj]);
-                    }
-                } else if (valid) {
-                    // this thread is the only writer of its target, so the order of the additions is fixed.  They happen in L2: with loads here the
-                    // four warps waited out the latency of scattered DRAM accesses twice per 32 channels.  Together with the walk over the
-                    // tiles, cross-level part of 32 -> 32, 64 -> 32 (3.5 M locations), 128 -> 64 (level delta 1): 494, 681, 404 -> 299, 381, 274 us.
-#pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
-                        const int n = walk.ntile * NT + c0 + jj;
-                        if (n < P.n_dim) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(acc_dst + (ll) n * acc_ld), "f"(__uint_as_float(r[jj])) : "memory");
+                        for (int jj = 0; jj < 32; ++jj) {
+                            const int n = n0 + c0 + jj;
+                            if (n < P.n_dim) P.out[(ll) n * P.ld_out + p] = __uint_as_float(r[jj]);
+                        }
                     }
                 }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(tmem_empty + acc));
+            walk.next(P);
+            target = target_of(it + 1);
             // every copy that read the source rows of tile `it` has landed (its accumulator is complete)
             publish_idx(it + NIDX);
         }

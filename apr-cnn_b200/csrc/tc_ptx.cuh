@@ -14,7 +14,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
 // The same past L1, whose 28 KB beside a full shared memory hit little in the kernels that gather widely spread rows, or 16 bytes of zeros where not `valid` (`src`, an address of the operand, is not read then: one row of zeros for all would be a
-// hot spot in L2).  Cross-level part 32 -> 32, 64 -> 32 on 3.5 M locations 295 -> 272, 379 -> 317 us; weight gradients 32 -> 32 506 -> 484, 32 -> 64 and 128 -> 64 at
+// hot spot in L2).  Cross-level part 32 -> 32, 64 -> 32 on 3.5 M locations 295 -> 272, 379 -> 317 us (with the additions of its epilogue in L2); weight gradients 32 -> 32 506 -> 484, 32 -> 64 and 128 -> 64 at
 // level delta 1 388 -> 355, 1043 -> 953.  (The run kernel, whose tiles overlap, is 1 % faster through L1 in its forward pass and 7 % in the input gradient.)
 __device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");

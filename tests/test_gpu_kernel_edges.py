@@ -79,6 +79,31 @@ def test_cross_level_sums_of_ragged_widths(cin, cout):
     assert float((got - want).norm() / want.norm()) <= 2.0 ** -9
 
 
+@pytest.mark.parametrize("cin,cout", [(16, 16), (33, 40), (72, 17), (130, 24)])
+@pytest.mark.parametrize("dl", [0, 1])
+def test_cross_level_sums_keep_subnormal_values(cin, cout, dl):
+    """Gradients below the smallest normal number: the operands are small whole numbers times powers of two, so every product, sum and tree
+    adjoint (factors 1/8 to 1) is exact, and scaling the operands scales the input gradient bit for bit down to 2^-149."""
+    import pyapr
+    from _pyaprwrapper.aprnet import cuda as C
+    from _pyaprwrapper.data_containers import APRPtrVector
+    a = H.arrays("odd")
+    apr = _apr(a)
+    n = int(pyapr.aprnet.utils.number_particles(apr, dl))
+    ld = torch.full((1,), dl, dtype=torch.int32)
+    torch.manual_seed(1)
+    w = torch.randint(-2, 3, (a.level_max - a.level_min + 1, cout, cin, 3, 3, 3), device="cuda").float()
+    g = torch.randint(-3, 4, (1, cout, n), device="cuda").float()
+    v, x = APRPtrVector([apr]), torch.zeros(1, cin, n, device="cuda")
+    _, rows = C.conv333_forward_keep_rows(v, x, w, ld, "bf16")
+    plain = C.conv333_backward_with_rows(v, rows, w, g, ld, True, "bf16")[0].double()
+    assert torch.equal(plain, C.conv333_backward(v, x.double(), w.double(), g.double(), ld)[0])
+    want = plain * 2.0 ** -133
+    assert int(((want != 0) & (want.abs() < 2.0 ** -126)).sum()) > n and bool((want * 2.0 ** 149 == (want * 2.0 ** 149).round()).all())
+    got = C.conv333_backward_with_rows(v, rows, w * 2.0 ** -66, g * 2.0 ** -67, ld, True, "bf16")[0].double()
+    assert C.tc_error_flag() == 0 and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("cin,cout", [(16, 130), (48, 256), (64, 200), (160, 264)])
 @pytest.mark.parametrize("bias", [False, True])
 def test_wide_forward_layers(cin, cout, bias):
