@@ -200,7 +200,13 @@ extern "C" int aprnet_conv333_norm_backward(aprnet_apr* a, int dl, int cin, int 
                                             const float* gamma, const float* beta, const float* mean, const float* rstd, int relu, const float* grad_y, const float* w,
                                             float* gin, int64_t ld_in, float* gw, float* gtree, int64_t ld_tree, float* dgamma, float* dbeta, float* partial,
                                             void* workspace, void* norm_ws, void* stream) {
-    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && !aprnet_small_cin(cin) && gw && workspace && norm_ws && n >= a->number_parts(dl), "bad argument");
+    // all of it before the first launch, which overwrites grad_gamma, grad_beta and the workspace
+    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && !aprnet_small_cin(cin) && rows && conv_out && n > 0 && groups > 0 && cout % groups == 0 &&
+                     mean && rstd && grad_y && gw && (!gin || (w && gtree)) && dgamma && dbeta && partial && workspace && norm_ws, "bad argument");
+    APRNET_ARG_CHECK(((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(workspace)) & 15) == 0, "packed rows and workspace must be 16-byte aligned");
+    const ll parts = a->number_parts(dl);
+    APRNET_ARG_CHECK(n >= parts && (!gin || (ld_in >= parts && ld_tree >= a->tree_size(dl))), "leading dimension too small");
+    if (27 * parts + 1 >= (1ll << 31)) { aprnet_set_error("%s: supports up to 79.5 M locations", __func__); return APRNET_ERR_UNSUPPORTED; }
     APRNET_DEVICE_CHECK(a);
     cudaStream_t st = (cudaStream_t) stream;
     const int rc = aprnet_groupnorm_relu_backward_rows(cout, n, a->number_parts(dl), groups, conv_out, grad_y, gamma, beta, mean, rstd, dgamma, dbeta,

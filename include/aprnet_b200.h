@@ -192,7 +192,10 @@ int aprnet_conv333_rows_backward(aprnet_apr* apr, int level_delta, int precision
 /* GroupNorm + ReLU and the 3x3x3 convolution in front of it, backward in one call: one batch item, float32 tensors, bf16 arithmetic, cin > 4.
  * conv_out (cout, n): output of the convolution, mean / rstd (groups) its statistics, grad_y (cout, n) the gradient behind the ReLU.  Same results as
  * aprnet_groupnorm_relu_backward followed by aprnet_conv333_rows_backward (grad_weights written, tree gradient folded into grad_input), without the
- * gradient of conv_out in memory.  grad_input null: not wanted.  norm_workspace: aprnet_groupnorm_workspace_bytes(1, cout, groups). */
+ * gradient of conv_out in memory.  grad_input null: not wanted (weights, grad_tree, ld_in and ld_tree are not used then).
+ * workspace: aprnet_conv333_rows_backward_workspace_bytes(), 16-byte aligned like packed_input_rows; norm_workspace:
+ * aprnet_groupnorm_workspace_bytes(1, cout, groups).  A call that is refused has launched nothing: APRNET_ERR_UNSUPPORTED for more than
+ * 79.5 M locations (27 N + 1 >= 2^31, with or without grad_input), APRNET_ERR_ARG for the others. */
 int aprnet_conv333_norm_backward(aprnet_apr* apr, int level_delta, int cin, int cout, int num_slots, const void* packed_input_rows, const float* conv_out,
                                  int64_t n, int groups, const float* gamma, const float* beta, const float* mean, const float* rstd, int relu,
                                  const float* grad_y, const float* weights, float* grad_input, int64_t ld_in, float* grad_weights, float* grad_tree,

@@ -33,6 +33,7 @@ extern "C" long long vrow_worst_pass(long long n_vrows, long long row_bytes) {
     return seen == n_vrows ? worst - cap : 1ll << 60;
 }
 extern "C" void set_vrows(aprnet_apr* a, long long n) { a->edge_plans[0].n_vrows = n; }
+extern "C" void set_particles(aprnet_apr* a, long long n) { for (int l = 3; l <= APRNET_MAX_LEVELS; ++l) a->meta.lvl_begin[l] = n; }
 extern "C" long long vrow_chunk() { return APRNET_VROW_CHUNK; }
 
 extern "C" int rows_overflow(aprnet_apr* a, long long particles, long long nodes) {
