@@ -83,12 +83,13 @@ def _plain(m, kind):
 
 def conv_norm(conv, norm, x, aprs, level_deltas):
     """`norm(conv(x, aprs, level_deltas))` for an `APRConv` followed by a `GroupNormReLU`, as one function where both are plain modules and a
-    backward pass in bf16 arithmetic over one batch item can follow; as two calls otherwise.  (More than four input channels: the weight gradient
+    backward pass of the convolution in bf16 arithmetic over one batch item can follow; as two calls otherwise, also where only the
+    normalisation wants gradients: the convolution then keeps nothing and has no backward pass.  (More than four input channels: the weight gradient
     of a first layer reads the gradient channel by channel; up to 79.5 M locations: beyond them the input gradient does.)"""
     if (_plain(conv, APRConv) and _plain(norm, GroupNormReLU) and conv._function is Conv333Function and conv.bias is None and x.is_cuda and x.dim() == 3 and
             x.shape[0] == 1 and len(aprs) == 1 and 4 < x.shape[1] == conv.in_channels and norm.num_channels == conv.out_channels and
             27 * x.shape[2] + 1 < 2 ** 31 and (conv.precision or get_conv_precision()) == "bf16" and torch.is_grad_enabled()):
         tensors = [t for t in (x, conv.weight, norm.weight, norm.bias) if t is not None]
-        if any(t.requires_grad for t in tensors) and all(t.dtype == torch.float32 and t.device == x.device for t in tensors):
+        if (x.requires_grad or conv.weight.requires_grad) and all(t.dtype == torch.float32 and t.device == x.device for t in tensors):
             return ConvGroupNormReLUFunction.apply(x, conv.weight, norm.weight, norm.bias, aprs, level_deltas, norm.num_groups, norm.eps, norm.relu)
     return norm(conv(x, aprs, level_deltas))

@@ -61,3 +61,32 @@ def test_conv_norm_calls_modules_that_are_observed():
     for p, other in (("fp32", norm), ("bf16", torch.nn.GroupNorm(8, 8).cuda())):
         conv.precision = p
         assert type(ops.conv_norm(conv, other, x, [apr], ld).grad_fn).__name__ != "ConvGroupNormReLUFunctionBackward"
+
+
+@pytest.mark.parametrize("affine", [True, False])
+def test_a_convolution_that_is_not_trained_keeps_nothing(affine):
+    """Input and weights without a gradient: the two functions, whose convolution has no backward pass and keeps no rows for one."""
+    import pyapr
+    from pyapr.aprnet import cuda as ops
+    a = H.blob_arrays((64, 64, 128), 40, 5)
+    apr = pyapr.apr_from_arrays(a)
+    apr.init_cuda()
+    conv, norm = ops.APRConv(32, 32, bias=False, precision="bf16").cuda(), ops.GroupNormReLU(32, 32, affine=affine).cuda()
+    conv.requires_grad_(False)
+    x, ld = torch.randn(1, 32, a.n_particles, device="cuda"), torch.zeros(1, dtype=torch.int32)
+    g = torch.randn(1, 32, a.n_particles, device="cuda")
+    res = []
+    for call in (lambda: norm(conv(x, [apr], ld)), lambda: ops.conv_norm(conv, norm, x, [apr], ld)):
+        norm.zero_grad(set_to_none=True)
+        y = call()
+        del y
+        before = torch.cuda.memory_allocated()
+        y = call()
+        held = torch.cuda.memory_allocated() - before
+        assert y.requires_grad == affine
+        if affine:
+            assert type(y.grad_fn).__name__ == "GroupNormReLUFunctionBackward"
+            y.backward(g)
+        res.append((held, [y.detach()] + [p.grad for p in norm.parameters()]))
+    assert res[1][0] <= res[0][0]
+    assert all(torch.equal(u, v) for u, v in zip(res[0][1], res[1][1]))
