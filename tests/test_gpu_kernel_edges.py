@@ -38,21 +38,34 @@ def test_groupnorm_row_lengths(c, n, dtype):
         assert float((x.grad - xd.grad).norm()) <= 64 * eps * float(xd.grad.norm()) + 1e-30
 
 
-@pytest.mark.parametrize("channels", [1, 3])
-def test_pooling_keeps_coarse_particles(channels):
-    """More kept particles than a block copies, rows of odd length: they come through pooling and up-sampling bit for bit."""
+def _two_levels(refined):
+    """5 x 10 x 41 cells of one level, the first few of every 700 divided once: 2050 - refined particles below the finest level."""
+    from pyapr import synthetic
+    level_map = torch.full((5, 10, 41), 6, dtype=torch.int32)
+    level_map.view(-1)[torch.arange(refined) * 700] = 7
+    return synthetic.apr_from_level_map(level_map, (10, 20, 82))
+
+
+# the copy kernel's blocks take 2048 entries each, shifted by where a row starts in its 128-byte line: one entry less, as many, one more, and
+# several blocks with a ragged end.  Five channels of rows of odd length start at five places of a line
+@pytest.mark.parametrize("refined,count", [(3, 2047), (2, 2048), (1, 2049), (None, None)])
+@pytest.mark.parametrize("channels", [1, 5])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_pooling_keeps_coarse_particles(refined, count, channels, dtype):
+    """The particles below the finest level come through pooling and up-sampling bit for bit."""
     import pyapr
     from pyapr.aprnet import cuda as ops
-    a = H.blob_arrays((64, 96, 112), 40, 8)
+    a = H.blob_arrays((64, 96, 112), 40, 8) if refined is None else _two_levels(refined)
+    kept = int(a.row_ptr[sum(a.dims[l][0] * a.dims[l][1] for l in range(a.level_min, a.level_max))])
+    assert kept == count if count else kept > 4096
     apr = _apr(a)
-    for dtype in (torch.float32, torch.float64):
-        x = torch.randn(1, channels, a.n_particles + 5, dtype=dtype, device="cuda")
+    for pad in (1, 2):
+        x = torch.randn(1, channels, a.n_particles + pad, dtype=dtype, device="cuda")
         ld = torch.zeros(1, dtype=torch.int32)
         pooled = ops.MaxPool()(x, [apr], ld)
+        assert pooled.shape[2] == int(pyapr.aprnet.utils.number_particles(apr, 1))
         up = ops.UpSampleConst()(pooled, [apr], ld)
-        n1 = int(pyapr.aprnet.utils.number_particles(apr, 1))
-        kept = int((up[0, 0, :a.n_particles] == x[0, 0, :a.n_particles]).cumprod(0).sum())       # leading entries that agree
-        assert kept > 4096 and torch.equal(pooled[..., :kept], x[..., :kept]) and torch.equal(up[..., :kept], x[..., :kept]) and pooled.shape[2] == n1
+        assert torch.equal(pooled[..., :kept], x[..., :kept]) and torch.equal(up[..., :kept], x[..., :kept])
 
 
 @pytest.mark.parametrize("cin,cout", [(16, 40), (16, 272), (24, 520)])
