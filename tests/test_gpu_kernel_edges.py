@@ -1,4 +1,5 @@
-"""Sizes at which the copies of pooling, the GroupNorm kernels, the sums of the cross-level part and the wide forward layers change their shape."""
+"""Sizes at which the copies of pooling, the GroupNorm kernels, the sums of the cross-level part and the wide forward layers change their shape; sums of
+subnormal values."""
 import numpy as np
 import pytest
 import torch
@@ -117,31 +118,55 @@ def test_cross_level_sums_keep_subnormal_values(cin, cout, dl):
     assert C.tc_error_flag() == 0 and torch.equal(got, want)
 
 
-@pytest.mark.parametrize("cin,cout", [(16, 130), (48, 256), (64, 200), (160, 264)])
-@pytest.mark.parametrize("bias", [False, True])
-def test_wide_forward_layers(cin, cout, bias):
-    """More than 128 result channels, with and without a bias of any width: the same bits with and without gathers over runs of cells."""
+# narrow result tiles on few tiles of locations, one and two blocks of 128 slots per tile on many
+STRUCTURES = [("odd",), ((64, 96, 96), 30, 6), ((128, 128, 256), 200, 6)]
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 65), (16, 128), (32, 100), (64, 127), (64, 128)])
+@pytest.mark.parametrize("structure", STRUCTURES)
+def test_wide_forward_layers_over_runs(cin, cout, structure):
+    """65 to 128 result channels with all source channels in one stage: over runs of cells (`runs` = 1) the same bits as tap by tap (0)."""
     import pyapr
     from pyapr.aprnet import cuda as ops
     from _pyaprwrapper.aprnet import cuda as C
-    for a in (H.arrays("odd"), H.blob_arrays((64, 96, 96), 30, 6)):
-        apr = _apr(a)
-        n = int(pyapr.aprnet.utils.number_particles(apr, 0))
-        torch.manual_seed(6)
-        conv = ops.APRConv(cin, cout, nstencils=2, bias=bias, precision="bf16").cuda()
-        x = torch.randn(1, cin, n, device="cuda")
-        ld = torch.zeros(1, dtype=torch.int32)
-        out = {}
-        with torch.no_grad():
-            for runs in (0, 1):
-                C.tc_set_option("runs", runs)
-                try:
-                    out[runs] = conv(x, [apr], ld)
-                finally:
-                    C.tc_set_option("runs", 1)
-        assert C.tc_error_flag() == 0 and torch.equal(out[0], out[1])
-        if bias:
-            with torch.no_grad():
-                plain = ops.APRConv(cin, cout, nstencils=2, bias=False, precision="bf16").cuda()
-                plain.weight.copy_(conv.weight)
-                assert torch.equal(out[1], plain(x, [apr], ld) + conv.bias.view(1, -1, 1))
+    apr = _apr(H.blob_arrays(*structure) if len(structure) > 1 else H.arrays(*structure))
+    n = int(pyapr.aprnet.utils.number_particles(apr, 0))
+    torch.manual_seed(6)
+    conv = ops.APRConv(cin, cout, nstencils=2, precision="bf16").cuda()
+    x = torch.randn(1, cin, n, device="cuda")
+    ld = torch.zeros(1, dtype=torch.int32)
+    out = {}
+    with torch.no_grad():
+        for runs in (0, 1):
+            C.tc_set_option("runs", runs)
+            try:
+                out[runs] = conv(x, [apr], ld)
+            finally:
+                C.tc_set_option("runs", 1)
+    assert C.tc_error_flag() == 0 and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 130), (48, 256), (64, 200), (160, 264), (128, 128)])
+@pytest.mark.parametrize("structure", STRUCTURES[:2])
+def test_wide_forward_layers_tap_by_tap(cin, cout, structure):
+    """Wider layers, against the float64 kernel on operands that are exact in bf16 (features, stencils, tree means as they are rounded): an accumulator takes
+    27 products of 16 channels per block of them, one after the other, and the tensor cores truncate each sum by at most 2^-23 of its size.  A
+    bias is one addition more."""
+    import pyapr
+    from _pyaprwrapper.aprnet import cuda as C
+    from _pyaprwrapper.data_containers import APRPtrVector
+    a = H.blob_arrays(*structure) if len(structure) > 1 else H.arrays(*structure)
+    apr = _apr(a)
+    n = int(pyapr.aprnet.utils.number_particles(apr, 0))
+    ld = torch.zeros(1, dtype=torch.int32)
+    torch.manual_seed(7)
+    w = (torch.randn(a.level_max - a.level_min + 1, cout, cin, 3, 3, 3, device="cuda") / (27 * cin) ** 0.5).bfloat16().float()
+    x = torch.randn(1, cin, n, device="cuda").bfloat16().float()
+    v = APRPtrVector([apr])
+    got, _ = C.conv333_forward_keep_rows(v, x, w, ld, "bf16")
+    tree = C.conv333_forward_keep_tree(v, x, w, ld, "fp32")[1].bfloat16()
+    want = C.conv333_forward_pretree(v, x.double(), tree.double(), w.double(), ld, "fp32")[0]
+    assert C.tc_error_flag() == 0
+    assert float((got - want).norm() / want.norm()) <= 27 * ((cin + 15) // 16) * 2.0 ** -23
+    bias = torch.randn(cout, device="cuda")
+    assert torch.equal(C.conv333_forward_keep_rows(v, x, w, ld, "bf16", bias)[0], got + bias.view(1, -1, 1))
