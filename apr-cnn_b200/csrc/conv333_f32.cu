@@ -114,7 +114,7 @@ struct F32Params {
     ll tree_base, zero_row;                // row of tree node 0 and of the zero row
     const float* wp; int mirror;           // packed weights (weights.cu); mirror: tap t meets the weights of tap 26 - t
     int n_dim, n_tiles;
-    int same_level_only;                   // mask table entries outside the tile's own level
+    int same_level_only;                   // mask table entries outside the tile's own level (as a constant of the mode: 16 -> 16 3.5 % slower)
     float* out; ll ld_out;
     const float* bias;                     // added to every output channel (null: none)
     // target mode (cross-level input gradient): location a stands for target out_map[a]; the result is added to
@@ -124,18 +124,26 @@ struct F32Params {
     ll v_shift;                            // added to table entries >= 0 (virtual rows)
 };
 
+enum { FORWARD, SAME_LEVEL, TARGETS };        // forward pass, the two parts of the input gradient
+
 // Block = 128 * WM locations x NT = TN * WN output channels, WM x WN warps; a thread owns the locations lane + 32 i (i < 4) of its
 // warp's 128 and TN channels.  A ring slot holds 16 channels of the tile's rows for one tap and the matching weights; 16-byte
 // pieces of a row are exchanged so that eight consecutive rows read at the same channel fall on different banks.  Table
 // entries are requested one tap ahead of the copies that need them.
 //
-// Order of the products.  KMAJOR == false: taps outer, 16 channels of one tap per slot.  KMAJOR == true (forward pass): blocks of
+// Order of the products.  Input gradient: taps outer, 16 channels of one tap per slot.  KMAJOR (forward pass): blocks of
 // 8 channels outer, taps inner, a slot holds two consecutive (block, tap) pairs.  A result is then the same chain of
 // multiply-adds whatever the tile (blocks of 8 channels, tap by tap, channel by channel): ReLU and max-pooling behind a
 // convolution turn a difference in its last bit into another gate or another child, so the forward pass keeps one order.
-template<int WM, int WN, int TN, bool KMAJOR>
+//
+// ZEROS: absent neighbours are zeros that are not read instead of the row of zeros in L1.  In the cross-level part, where most taps have none, that
+// takes 4 to 25 % off (32 -> 32 on 1.2 M locations 522 -> 465 us, with the sums below), in the same-level part up to 7 % where the tile is at most 32 channels wide
+// (32 -> 32 1805 -> 1753) and minus 3 to 10 % where it is 64 (33 -> 33 3220 -> 3333, 64 -> 64 at level delta 1 2595 -> 2663: the test costs more than
+// the reads).  The forward pass has next to none (neighbours outside the volume).
+template<int WM, int WN, int TN, int MODE>
 __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f32_gather_kernel(const F32Params P) {
     constexpr int T = 32 * WM * WN, M = 128 * WM, NT = TN * WN;
+    constexpr bool KMAJOR = MODE == FORWARD, ZEROS = MODE == TARGETS || (MODE == SAME_LEVEL && NT < 64);
     constexpr int RPT = M * (KS / 4) / T;          // row pieces a thread copies per slot
     constexpr int RSTEP = T / (KS / 4);            // distance of their rows
     constexpr int A_ELEMS = M * KS, B_ELEMS = KS * NT, SLOT = A_ELEMS + B_ELEMS;
@@ -173,12 +181,11 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
             src[i] = (int32_t) r;
         }
     };
-    auto copy_rows = [&](float* a_s, int k) {      // channels [k, k + 4) of the rows src[]; beyond the row and for absent neighbours zeros that are not read (16 -> 16 on 3.5 M
-        // locations, both parts of the input gradient 2051 -> 2022 us, 32 -> 32 at level delta 1 3400 -> 3268 and forward 3090 -> 3005)
+    auto copy_rows = [&](float* a_s, int k) {      // channels [k, k + 4) of the rows src[]; beyond the row: zeros
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
             const int row = prow + i * RSTEP;
-            cp_async16_zfill(smem_u32(a_s + row * KS + ((piece ^ ((row >> 1) & 3)) << 2)), P.rows + (ll) src[i] * P.kpad + k, k < P.kpad && src[i] != (int32_t) P.zero_row);
+            cp_async16_zfill(smem_u32(a_s + row * KS + ((piece ^ ((row >> 1) & 3)) << 2)), P.rows + (ll) src[i] * P.kpad + k, k < P.kpad && (!ZEROS || src[i] != (int32_t) P.zero_row));
         }
     };
     int itap = KMAJOR ? piece >> 1 : 0, ikc = 0, islot = 0, is = 0;       // KMAJOR: the (block, tap) pair of this thread's half of a slot
@@ -266,26 +273,35 @@ __global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f3
         if (p >= hi) continue;
         float* dst = P.out + p;
         ll ld = P.ld_out;
-        if (P.out_map) {
+        if (MODE == TARGETS) {
             const ll t = P.out_map[p];
             dst = t < P.out_split ? P.out + t : P.out2 + (t - P.out_split);
             ld = t < P.out_split ? P.ld_out : P.ld_out2;
-        }
-        // target mode adds to what is there (this thread is the only writer of its target in this launch): all of it is requested before any is
-        // written, an addition after the other waited TN times for scattered accesses
-        float add[TN];
+            // adds to what is there (this thread is the only writer of its target in this launch): all of it is requested before any is
+            // written, an addition after the other waited TN times for scattered accesses.  (In a kernel shared with the other parts this cost
+            // their epilogues up to 9 %: 8 -> 33, forward, on 1.2 M locations 814 -> 875 us, now 805.)
+            float held[TN];
 #pragma unroll
-        for (int n = 0; n < TN; ++n) {
-            const int co = nt * NT + n_off + n;
-            add[n] = co >= P.n_dim ? 0.f : (P.out_map ? dst[(ll) co * ld] : (P.bias ? P.bias[co] : 0.f));
-        }
+            for (int n = 0; n < TN; ++n) held[n] = nt * NT + n_off + n < P.n_dim ? dst[(ll) (nt * NT + n_off + n) * ld] : 0.f;
 #pragma unroll
-        for (int n = 0; n < TN; ++n) {
-            const int co = nt * NT + n_off + n;
-            const float2 pair = unpack2(acc[i][n / 2]);
-            const float v = n & 1 ? pair.y : pair.x;
-            if (co < P.n_dim) dst[(ll) co * ld] = P.out_map || P.bias ? v + add[n] : v;
+            for (int n = 0; n < TN; ++n) {
+                const int co = nt * NT + n_off + n;
+                const float2 pair = unpack2(acc[i][n / 2]);
+                if (co < P.n_dim) dst[(ll) co * ld] = (n & 1 ? pair.y : pair.x) + held[n];
+            }
+            continue;
         }
+        auto store = [&](bool bias) {
+#pragma unroll
+            for (int n = 0; n < TN; ++n) {
+                const int co = nt * NT + n_off + n;
+                if (co >= P.n_dim) continue;
+                const float2 pair = unpack2(acc[i][n / 2]);
+                const float v = n & 1 ? pair.y : pair.x;
+                dst[(ll) co * ld] = bias ? v + P.bias[co] : v;
+            }
+        };
+        if (MODE == FORWARD && P.bias) store(true); else store(false);
     }
 }
 
@@ -548,11 +564,11 @@ int run_pack_weights(const aprnet_apr* a, int dl, const float* w, int slots, int
     return aprnet_pack_weights(a, dl, false, w, slots, cin, cout, transposed, nt, (n_dim + nt - 1) / nt, pad4(transposed ? cout : cin), wp, st);
 }
 
-template<int WM, int WN, int TN, bool KMAJOR>
+template<int WM, int WN, int TN, int MODE>
 int launch_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
     constexpr int M = 128 * WM, NT = TN * WN;
     constexpr size_t smem = (size_t) RING * (M + NT) * KS * sizeof(float);
-    auto kern = conv333_f32_gather_kernel<WM, WN, TN, KMAJOR>;
+    auto kern = conv333_f32_gather_kernel<WM, WN, TN, MODE>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     P.segs = make_seg_table(segs, M);
     P.n_tiles = (P.n_dim + NT - 1) / NT;
@@ -564,13 +580,13 @@ int launch_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t s
     return APRNET_OK;
 }
 
-template<bool KMAJOR>
+template<int MODE>
 int run_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
     switch (pick_nt(P.n_dim)) {
-        case 64: return launch_gather<1, 4, 16, KMAJOR>(P, segs, st, pname);
-        case 32: return launch_gather<2, 2, 16, KMAJOR>(P, segs, st, pname);
-        case 16: return launch_gather<2, 2, 8, KMAJOR>(P, segs, st, pname);
-        default: return launch_gather<2, 2, 4, KMAJOR>(P, segs, st, pname);
+        case 64: return launch_gather<1, 4, 16, MODE>(P, segs, st, pname);
+        case 32: return launch_gather<2, 2, 16, MODE>(P, segs, st, pname);
+        case 16: return launch_gather<2, 2, 8, MODE>(P, segs, st, pname);
+        default: return launch_gather<2, 2, 4, MODE>(P, segs, st, pname);
     }
 }
 
@@ -690,7 +706,7 @@ int run_cross(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* 
         P.nbr = ep->vnbr; P.N = ep->n_active; P.rows = grows; P.kpad = gpad; P.zero_row = a->number_parts(dl); P.tree_base = 0; P.v_shift = off - v0;
         P.wp = wp; P.n_dim = cin;
         P.out = gin; P.ld_out = ld_in; P.out_map = ep->active; P.out_split = a->number_parts(dl); P.out2 = gtree; P.ld_out2 = ld_tree;
-        if ((rc = run_gather<false>(P, segs, st, pname))) return rc;
+        if ((rc = run_gather<TARGETS>(P, segs, st, pname))) return rc;
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -766,7 +782,7 @@ int aprnet_f32_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, cons
     P.wp = wp; P.n_dim = cout; P.out = out; P.ld_out = ld_out; P.bias = bias;
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_fwd:ci%d:co%d:dl%d", cin, cout, dl);
-    return run_gather<true>(P, aprnet_segments(a, dl, slots, false), st, pname);
+    return run_gather<FORWARD>(P, aprnet_segments(a, dl, slots, false), st, pname);
 }
 
 int aprnet_f32_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* rows, const float* gout, ll ld_out, const void* grows,
@@ -793,7 +809,7 @@ int aprnet_f32_backward_input(aprnet_apr* a, int dl, int cin, int cout, int slot
     P.wp = wp; P.n_dim = cin; P.out = gin; P.ld_out = ld_in;
     char pname[64];
     snprintf(pname, sizeof(pname), "conv333_bwd_input:ci%d:co%d:dl%d", cin, cout, dl);
-    if ((rc = run_gather<false>(P, aprnet_segments(a, dl, slots, false), st, pname))) return rc;
+    if ((rc = run_gather<SAME_LEVEL>(P, aprnet_segments(a, dl, slots, false), st, pname))) return rc;
     if (27 * n + 1 >= (1ll << 31)) {
         // more than 79.5 M locations: the 32-bit edge ids of the edge plan run out; the cross-level part is scattered with
         // atomic adds instead (correct, but the summation order is no longer fixed)
