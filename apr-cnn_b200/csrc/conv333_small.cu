@@ -53,7 +53,8 @@ __global__ void small_stage_kernel(const float* __restrict__ x, ll ld_x, ll n, c
 // read four at a time.  A lane loads the 9 values that lie beside its cell (dz, dx) and gets those of the y neighbours from the lanes next to it, so a warp
 // yields 30 slots and gathers 9 values per slot where the neighbour table needs 27 entries and 27 values per location.  What bounds it is the latency of
 // these gathers: the table entries of the next tile are on their way during the multiply-adds, and a block takes up to eight tiles with one
-// staging of the weights.  1 -> 32 channels on 3.5 M locations 522 -> 311 us against one thread per
+// staging of the weights.  (They are requested behind a block's last tile too: a condition costs registers, 1 -> 16 on 3.5 M locations
+// 303 -> 320 us, and is no faster with one tile per block, on 7 k and 64 k locations.)  1 -> 32 channels on 3.5 M locations 522 -> 311 us against one thread per
 // location and the neighbour table, 2 -> 32 889 -> 596, 4 -> 40 on 1.9 M 1415 -> 1124; 1 -> 16 on 7 k locations 10.7 -> 6.1.  (Paired multiply-adds: 0 to 10 % slower.)
 // The chain of multiply-adds of a result is channel by channel, tap by tap.
 template<int CIN>

@@ -7,8 +7,9 @@
 // tap dy starts dy rows further.  (The swizzle of a K-major operand is a function of the shared-memory address, so a start address
 // inside the pattern is an ordinary one.)  That is 9 x 1.07 .. 1.27 gathered rows per location instead of 27; slots without a
 // location are the price, 7 to 27 % more multiply-adds.  Each weight tile that is fetched meets H blocks of 128 rows.
-// What bounds it now: the data pipe of the SM's shared memory.  For 32 -> 32 channels the tensor core's operand reads keep it busy for 56 % of
-// the time and the load-store unit (copies, whose sectors land one by one, shuffles, stores of the results) for 51 %.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
+// What bounds it: no unit is saturated.  Shares of each unit's own peak for 32 -> 32 and 64 -> 64 channels, which overlap: operand reads of the tensor
+// core (l1tex__data_pipe_tc_wavefronts) 59 and 70 %, load-store unit (copies, whose sectors land one by one, shuffles, stores of the results;
+// l1tex__data_pipe_lsu_wavefronts) 52 and 55 %, issue slots 51 and 45 %, tensor pipe 25 and 49 %; the rest is waiting between the roles.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
 // 32 -> 32 layer that takes 0.48.)
 //
 // Every result of the forward pass is the same sequence of MMAs (neighbour row, channel block, dy, 16 channels) as in

@@ -258,8 +258,10 @@ __global__ void __launch_bounds__(GN_TPB) gn_backward_apply_kernel(const T* __re
 
 // Stage 3 for a convolution in front of the normalisation whose backward pass works from packed bf16 rows of its output's gradient: the same
 // dx, rounded and written as rows [0, n_rows) of cpad channels, row n_rows zero, instead of a channel-major tensor that would be read once
-// more to be packed (12 + 6 bytes per value; here 10).  HBM-bound; the 13 layers
+// more to be packed (12 + 6 bytes per value; here 10).  The 13 layers
 // of a training step on 3.5 M locations took 2.1 + 1.35 ms in two passes and take 2.26 ms, on 28 M locations 18.7 ms.  One batch item; a block has 32 channels x 128 entries.
+// What bounds it: the loads in flight.  A block has one tile and, between its loads and its stores, nothing of another under way: 0.77 of the copy rate with
+// 48 % of the warps active, which wait for loads (6.9 issue slots per instruction) and at the block's barriers (2.6); issue slots 51 %.
 __global__ void __launch_bounds__(256) gn_backward_apply_rows_kernel(const float* __restrict__ x, const float* __restrict__ dy, ll n, ll n_rows, int C, int ch_per_group,
                                                                      const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean,
                                                                      const float* __restrict__ rstd, const float* __restrict__ group_terms, const double* __restrict__ partial,
