@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + C1_MAX_ACC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
     for (int c = tid; c < ACC_COLS; c += C1_THREADS) bias_s[c] = P.bias && c < P.n_out ? P.bias[c] : 0.f;
     if (tid == 0) {
         for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), 4); mbar_init(smem_u32(empty + i), 1); }
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
 
         if (warp < C1_MMA) {
             // ---------------- producers ----------------
-            const int grp = tid >> 7, row = tid & 127;
+            const int grp = warp >> 2, row = tid & 127;
             for (int it = grp; grp < ngroups && it < mine && !failed; it += ngroups) {
                 const uint32_t j = j_base + (uint32_t) it, slot = j % (uint32_t) stages, use = j / (uint32_t) stages;
                 const float* src = P.in + min(tile_begin(it) + row, se - 1);     // rows past the end repeat the last location and are not stored
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
             }
         } else if (warp == C1_MMA) {
             // ---------------- MMA issue ----------------
-            if (lane == 0) {
+            if (elect_one()) {
                 for (int it = 0; it < mine && !failed; ++it) {
                     const uint32_t j = j_base + (uint32_t) it, slot = j % (uint32_t) stages, use = j / (uint32_t) stages;
                     const uint32_t acc = j % NACC, acc_use = j / NACC;
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
     uint64_t* done = empty + C1_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
     const uint32_t tmem_cols = mtiles * NT <= 32 ? 32u : (mtiles * NT <= 64 ? 64u : (mtiles * NT <= 128 ? 128u : (mtiles * NT <= 256 ? 256u : 512u)));
     if (tid == 0) {
         for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), 8); mbar_init(smem_u32(empty + i), 1); }
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
         }
     } else if (warp == DW_MMA) {
         // ---------------- MMA issue ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             for (int it = 0; it < mine && !failed; ++it) {
                 const uint32_t slot = (uint32_t) it % (uint32_t) stages, use = (uint32_t) it / (uint32_t) stages;
                 if (!mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }

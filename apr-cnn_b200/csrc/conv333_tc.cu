@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(idx_full + WS_MAX_ACC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
     const int kchunks = P.kpad / KS;
     const int steps_per_tile = NTG * kchunks;
     const int total_tiles = P.segs.tile_begin[P.segs.n] * P.n_tiles;
@@ -245,15 +245,14 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
                     cur_it = it;
                     if (!mbar_wait_warp(smem_u32(idx_full + it % NIDX), (it / NIDX) & 1, abort_flag)) { failed = true; break; }
                     idx = idx_s + (it % NIDX) * 27 * TILE_M + r0;
-                    if (sub == 0 && lane == 0) {      // packed weights of one (slot, tap, n tile) are [k chunk][n][8]; a stage takes KS / 8 chunks of TAPS taps
-                        wsrc = reinterpret_cast<const unsigned char*>(P.wp + ((ll) walk.slot * 27 * P.n_tiles + walk.ntile) * ((ll) P.kpad * NT));
-                    }
+                    // packed weights of one (slot, tap, n tile) are [k chunk][n][8]; a stage takes KS / 8 chunks of TAPS taps
+                    wsrc = reinterpret_cast<const unsigned char*>(P.wp + ((ll) walk.slot * 27 * P.n_tiles + walk.ntile) * ((ll) P.kpad * NT));
                 }
                 const int tg = step / kchunks, kc = step - tg * kchunks;
                 const int t0 = tg * TAPS;
                 if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
                 unsigned char* a_s = stage_base + (size_t) slot * STAGE_BYTES;
-                if (sub == 0 && lane == 0) {
+                if (sub == 0 && elect_one()) {
                     const int nt = min(TAPS, 27 - t0);
                     mbar_expect_tx(smem_u32(full + slot), nt * B_TAP + max(0, nt - (TAPS - TT)) * A_TAP);
                     for (int t = 0; t < nt; ++t)
@@ -299,7 +298,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv333_tc_ws_kernel(const TcPa
         }
     } else if (warp == WS_NPROD) {
         // ---------------- MMA issue ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t slot = 0, use = 0;
             bool ready = false;                   // the next stage is known to be there
             for (int it = 0; it < my_tiles && !failed; ++it) {

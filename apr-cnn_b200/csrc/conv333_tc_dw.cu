@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
     const int grp = blockIdx.y % P.groups, cib = (blockIdx.y / P.groups) % P.ci_blocks, cob = blockIdx.y / (P.groups * P.ci_blocks);
     const int d0 = grp * P.d_per_group;
     const int nd = min(P.d_per_group, 9 - d0);
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv333_tc_dw_kernel(const DwPa
         cp_async_wait<0>();
     } else if (warp == MMA_WARP && total_stages > 0) {
         // ---------------- MMA issue ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t slot = 0, use = 0;
             bool ready = false;                   // the next stage is known to be there
             for (int chunk = 0; chunk < nchunks && !failed; ++chunk) {

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2 * MAX_ACC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
     const int kchunks = P.kpad / KS, steps = 9 * kchunks;
     const int total_tiles = P.tile_begin[P.n_segs] * P.n_tiles;
     const int my_tiles = (int) blockIdx.x < total_tiles ? (total_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
                 if (left > 1) { locate(); request(); }       // in flight while this stage is copied
                 if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
                 unsigned char* a_s = ring + (size_t) slot * STAGE_BYTES;
-                if (sub == 0 && lane == 0) {
+                if (sub == 0 && elect_one()) {
                     mbar_expect_tx(smem_u32(full + slot), 3 * B_TAP);
 #pragma unroll
                     for (int dy = 0; dy < 3; ++dy)
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     } else if (warp < EPI_WARP) {
         // ---------------- MMA issue, every second block of 128 rows ----------------
         const int h0 = warp - MMA_WARP;
-        if (lane == 0 && h0 < ISSUERS) {
+        if (h0 < ISSUERS && elect_one()) {
             constexpr int MMAS = 3 * (KS / 16);
             uint32_t slot = 0, use = 0;
             bool ready = false;                   // the next stage is known to be there

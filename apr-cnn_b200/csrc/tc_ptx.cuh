@@ -76,14 +76,32 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     *abort_flag = 1;
     return false;
 }
-// one lane polls, the warp follows
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
+// ---- one value per warp ----------------------------------------------------------------------------------
+// The kernels give their warps roles.  Where the compiler cannot see that a branch or a loop goes the same way in all lanes, it treats what is inside as
+// divergent: every shuffle and vote there is preceded by a convergence of the warp, and instructions that take uniform registers (tcgen05.mma, bulk copies) are
+// issued in a loop over the lanes.  That was what the roles waited for: with the warp's number, the results of waits and the electing of one lane as
+// below, 3x3x3 layers on 3.5 M locations, 32 -> 32 forward 0.50 -> 0.38 ms, weight gradients 32 -> 32 and 64 -> 32 0.52 -> 0.35 and 0.81 -> 0.50 ms; 128 -> 128 at level delta 2
+// 10 to 22 % less; 1x1x1 weight gradient 64 -> 128 0.58 -> 0.51 ms.
+
+// the warp's number
+__device__ __forceinline__ int warp_number() { return __shfl_sync(0xffffffffu, (int) threadIdx.x >> 5, 0); }
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(ok));
     return ok != 0;
 }
-
+// bounded wait of the (converged) warp: every lane polls
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    bool ok = false;
+    for (unsigned it = 0; it < SPIN_LIMIT; ++it) {
+        ok = mbar_try_wait(bar, parity);
+        if (ok || ((it & 63) == 63 && *abort_flag)) break;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) *abort_flag = 1;
+    return ok;
+}
 // ---- proxies and tcgen05 fences --------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
