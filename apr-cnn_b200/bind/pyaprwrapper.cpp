@@ -559,8 +559,9 @@ torch::Tensor conv111_forward(std::vector<APR*>& aprs, torch::Tensor input, torc
     return output;
 }
 
-std::vector<torch::Tensor> conv111_backward(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights,
-                                            torch::Tensor grad_output, torch::Tensor level_delta, const std::string& precision) {
+// {grad_input, grad_weights} and, where it is wanted, the gradient of a bias: the sum of grad_output over batch and particle axis
+static std::vector<torch::Tensor> conv111_backward_impl(std::vector<APR*>& aprs, const torch::Tensor& input, const torch::Tensor& weights,
+                                                        const torch::Tensor& grad_output, const torch::Tensor& level_delta, const std::string& precision, bool with_bias) {
     CHECK_INPUT(input); CHECK_INPUT(weights); CHECK_INPUT(grad_output);
     check_batch(aprs, input);
     TORCH_CHECK(grad_output.dim() == 3 && grad_output.size(1) == weights.size(1) && grad_output.size(2) == input.size(2), "grad_output shape does not match");
@@ -570,14 +571,22 @@ std::vector<torch::Tensor> conv111_backward(std::vector<APR*>& aprs, torch::Tens
     auto grad_input = torch::empty_like(input);
     auto grad_weights = torch::zeros_like(weights);
     auto partial = torch::empty({aprnet_conv111_partial_elems((int) cin, (int) cout)}, input.options());
+    torch::Tensor grad_bias;
     const int dt = dtype_id(input);
     const bool tc = resolve_mode(precision) == 1 && dt == APRNET_F32;
     void* st = stream_of(input);
+    // the joint pass sums over the particles of one item; entries behind them would count, too
+    const bool sums = with_bias && input.size(0) == 1 && aprs[0]->number_parts(dl[0]) == n;
     for (int64_t b = 0; b < input.size(0); ++b) {
         check_level_delta(*aprs[b], dl[b]);
         aprnet_apr* h = aprs[b]->handle(input);
         int rc = APRNET_ERR_UNSUPPORTED;
         if (tc) {
+            auto gb = sums ? torch::empty({cout}, grad_output.options()) : torch::Tensor();
+            rc = aprnet_conv111_backward_tc(h, dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(input, b), n, (const float*) row(grad_output, b), n,
+                                            (const float*) weights.data_ptr(), (float*) row(grad_input, b), n, (float*) grad_weights.data_ptr(),
+                                            sums ? gb.data_ptr<float>() : nullptr, (float*) partial.data_ptr(), partial.numel(), st);
+            if (rc != APRNET_ERR_UNSUPPORTED) { check(rc, "conv111_backward (tensor cores)"); grad_bias = gb; continue; }
             rc = aprnet_conv111_backward_input_tc(h, dl[b], (int) cin, (int) cout, (int) weights.size(0), (const float*) row(grad_output, b), n,
                                                   (const float*) weights.data_ptr(), (float*) row(grad_input, b), n, st);
             if (rc != APRNET_ERR_UNSUPPORTED) check(rc, "conv111_backward_input (tensor cores)");
@@ -598,7 +607,19 @@ std::vector<torch::Tensor> conv111_backward(std::vector<APR*>& aprs, torch::Tens
               "conv111_backward_weights");
     }
     fill_padding(grad_input, valid_of(aprs, dl));
-    return {grad_input, grad_weights};
+    if (with_bias && !grad_bias.defined()) grad_bias = grad_output.sum(at::IntArrayRef{0, 2});
+    return {grad_input, grad_weights, grad_bias};
+}
+
+std::vector<torch::Tensor> conv111_backward(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights,
+                                            torch::Tensor grad_output, torch::Tensor level_delta, const std::string& precision) {
+    auto r = conv111_backward_impl(aprs, input, weights, grad_output, level_delta, precision, false);
+    return {r[0], r[1]};
+}
+
+std::vector<torch::Tensor> conv111_backward_with_bias(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights,
+                                                      torch::Tensor grad_output, torch::Tensor level_delta, const std::string& precision) {
+    return conv111_backward_impl(aprs, input, weights, grad_output, level_delta, precision, true);
 }
 
 // ---- restriction --------------------------------------------------------------------------------
@@ -1000,6 +1021,7 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
     cuda.def("maxpool_backward_cuda", &maxpool_backward_cuda, "aprs"_a, "grad_output"_a, "max_indices"_a, "level_delta"_a);
     cuda.def("conv111_forward", &conv111_forward, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "", "bias"_a = py::none());
     cuda.def("conv111_backward", &conv111_backward, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "precision"_a = "");
+    cuda.def("conv111_backward_with_bias", &conv111_backward_with_bias, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "precision"_a = "");
     cuda.def("conv333_forward", &conv333_forward, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a);
     cuda.def("conv333_backward", &conv333_backward, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a);
     // extensions: keep the tree means of the forward pass for the backward pass

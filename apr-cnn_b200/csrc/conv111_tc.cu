@@ -68,6 +68,57 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// One unit (two neighbouring tiles, 256 locations) of the channel-major result from its accumulators, by the eight epilogue warps: TMEM -> shared memory ->
+// stores that each cover what one line holds.  w8: the warp among the eight, which are two sets of four; has: this set's tile exists; piece: 16-channel pieces staged so far.  (A failed warp keeps the pace of the barriers.)
+__device__ __forceinline__ void store_unit(float* __restrict__ out, ll ld_out, int n_out, const float* bias_s, ll p0, int cnt, bool has, uint32_t acc_addr, uint32_t full_bar, uint32_t full_parity,
+                                           uint32_t empty_bar, float* out_s, int w8, int& piece, bool& failed, volatile int* abort_flag) {
+    constexpr int LINES = 2 * TILE_M / 32 + 1;
+    const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3, set = w8 >> 2;         // q: TMEM lane group this warp may read
+    if (has && !failed && !mbar_wait_warp(full_bar, full_parity, abort_flag)) failed = true;
+    const bool live = has && !failed;
+    tc_fence_after();
+    const uint32_t taddr = acc_addr + ((uint32_t) (q * 32) << 16);
+    uint32_t r[C1_OUT_CH];
+    if (live) tmem_ld16(taddr, r);
+#pragma unroll 1
+    for (int c0 = 0; c0 < n_out; c0 += C1_OUT_CH) {
+        float* buf = out_s + (piece++ & 1 ? C1_OUT_CH * 2 * TILE_M : 0);
+        if (live) {
+            tmem_ld_wait();
+            float* dst = buf + set * TILE_M + q * 32 + lane;
+#pragma unroll
+            for (int jj = 0; jj < C1_OUT_CH; ++jj) dst[jj * 2 * TILE_M] = __uint_as_float(r[jj]);
+            if (c0 + C1_OUT_CH < n_out) tmem_ld16(taddr + c0 + C1_OUT_CH, r);      // read while this piece is stored
+        }
+        // the buffer is written again after the barrier of the other one
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (failed) continue;
+#pragma unroll
+        for (int k = 0; k < C1_OUT_CH / 8; ++k) {
+            const int c = k * 8 + w8;
+            if (c0 + c >= n_out) break;
+            float* o = out + (ll) (c0 + c) * ld_out + p0;
+            const int e0 = lane - (int) ((reinterpret_cast<uintptr_t>(o) >> 2) & 31);
+            const float* src = buf + c * 2 * TILE_M + e0;
+            float v[LINES];
+#pragma unroll
+            for (int i = 0; i < LINES; ++i) v[i] = e0 + i * 32 >= 0 && e0 + i * 32 < 2 * TILE_M ? src[i * 32] : 0.f;
+            if (bias_s) {
+                const float bias = bias_s[c0 + c];
+#pragma unroll
+                for (int i = 0; i < LINES; ++i) v[i] += bias;
+            }
+            o += e0;
+#pragma unroll
+            for (int i = 0; i < LINES; ++i)
+                if (e0 + i * 32 >= 0 && e0 + i * 32 < cnt) o[i * 32] = v[i];
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (live && lane == 0) mbar_arrive(empty_bar);
+}
+
 template<int NT, int KS>
 __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Params P, const int stages) {
     constexpr int ACC_COLS = NT < 32 ? 32 : NT;                 // TMEM columns per accumulator
@@ -110,6 +161,7 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
     bool failed = false;
     const int ngroups = min(C1_GROUPS, stages);      // (a ring at least as long as the groups keeps the phases that a wait can meet apart)
     int piece = 0;                          // 16-channel pieces the epilogue has staged
+    const int w8 = warp - C1_MMA - 1, set = w8 >> 2;       // epilogue: two sets of four warps on the two tiles of a unit
     uint32_t j_base = 0;                    // tiles this block has been given in the levels before the current one
 
     for (int seg = 0; seg < P.n_segs; ++seg) {
@@ -204,58 +256,11 @@ __global__ void __launch_bounds__(C1_THREADS, 1) conv111_tc_kernel(const C1Param
             }
         } else {
             // ---------------- epilogue ----------------
-            const int q = warp & 3;                           // TMEM lane group this warp may read
-            const int w8 = warp - C1_MMA - 1, set = w8 >> 2;
-            for (int u = 0; u < units; ++u) {                 // (a failed warp keeps the pace of the barriers)
+            for (int u = 0; u < units; ++u) {
                 const int it = (u << pair) + set;
-                const bool has = set <= pair && it < mine;
-                const uint32_t j = j_base + (uint32_t) it, acc = j % NACC, acc_use = j / NACC;
-                const ll p0 = tile_begin(u << pair);
-                const int cnt = (int) min(se - p0, (ll) (TILE_M << pair));
-                if (has && !failed && !mbar_wait_warp(smem_u32(tmem_full + acc), acc_use & 1, abort_flag)) failed = true;
-                const bool live = has && !failed;
-                constexpr int LINES = 2 * TILE_M / 32 + 1;
-                tc_fence_after();
-                const uint32_t taddr = tmem_d + ((uint32_t) (q * 32) << 16) + acc * ACC_COLS;
-                uint32_t r[C1_OUT_CH];
-                if (live) tmem_ld16(taddr, r);
-#pragma unroll 1
-                for (int c0 = 0; c0 < P.n_out; c0 += C1_OUT_CH) {
-                    float* buf = out_s + (piece++ & 1 ? C1_OUT_CH * 2 * TILE_M : 0);
-                    if (live) {
-                        tmem_ld_wait();
-                        float* dst = buf + set * TILE_M + q * 32 + lane;
-#pragma unroll
-                        for (int jj = 0; jj < C1_OUT_CH; ++jj) dst[jj * 2 * TILE_M] = __uint_as_float(r[jj]);
-                        if (c0 + C1_OUT_CH < P.n_out) tmem_ld16(taddr + c0 + C1_OUT_CH, r);      // read while this piece is stored
-                    }
-                    // the buffer is written again after the barrier of the other one
-                    asm volatile("bar.sync 1, 256;" ::: "memory");
-                    if (failed) continue;
-#pragma unroll
-                    for (int k = 0; k < C1_OUT_CH / 8; ++k) {
-                        const int c = k * 8 + w8;
-                        if (c0 + c >= P.n_out) break;
-                        float* o = P.out + (ll) (c0 + c) * P.ld_out + p0;
-                        const int e0 = lane - (int) ((reinterpret_cast<uintptr_t>(o) >> 2) & 31);
-                        const float* src = buf + c * 2 * TILE_M + e0;
-                        const float bias = bias_s[c0 + c];
-                        float v[LINES];
-#pragma unroll
-                        for (int i = 0; i < LINES; ++i) v[i] = e0 + i * 32 >= 0 && e0 + i * 32 < 2 * TILE_M ? src[i * 32] : 0.f;
-                        if (P.bias) {
-#pragma unroll
-                            for (int i = 0; i < LINES; ++i) v[i] += bias;
-                        }
-                        o += e0;
-#pragma unroll
-                        for (int i = 0; i < LINES; ++i)
-                            if (e0 + i * 32 >= 0 && e0 + i * 32 < cnt) o[i * 32] = v[i];
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (live && lane == 0) mbar_arrive(smem_u32(tmem_empty + acc));
+                const uint32_t j = j_base + (uint32_t) it;
+                store_unit(P.out, P.ld_out, P.n_out, P.bias ? bias_s : nullptr, tile_begin(u << pair), (int) min(se - tile_begin(u << pair), (ll) (TILE_M << pair)), set <= pair && it < mine,
+                           tmem_d + (j % NACC) * ACC_COLS, smem_u32(tmem_full + j % NACC), (j / NACC) & 1, smem_u32(tmem_empty + j % NACC), out_s, w8, piece, failed, abort_flag);
             }
         }
         if (failed) *abort_flag = 1;
@@ -475,12 +480,281 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
     if (warp == DW_MMA) tmem_dealloc(tmem_d, tmem_cols);
 }
 
-__global__ void c1_reduce_partial_kernel(const float* __restrict__ partial, int nblocks, ll elems, float* __restrict__ dst) {
-    const ll e = (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= elems) return;
+// ---- both gradients in one pass ----------------------------------------------------------------------------
+// grad_in[i][p] = sum_o w[slot][o][i] * gout[o][p] and gw[slot][o][i] = sum_p gout[o][p] * in[i][p], and the sums of gout over the locations (the gradient of a
+// bias), from one reading of gout and in.  The three passes apart read gout three times and round it twice: 64 -> 128 channels on 3.5 M locations 0.69 + 0.51 + 0.32 ms,
+// 0.81 together (0.56 at the rate of a copy).
+// One persistent block per SM, 25 warps, over tiles of 128 locations, the weights of one level in shared memory:
+//   warps 0-15  producers in groups of 2, 4 or 8 warps (8 channel rows a warp, so that narrow layers have as much under way), which take the tiles in turn.  A warp reads
+//               whole rows, 128 locations of a channel, rounds them to bf16 and leaves, as conv111_tc_dw_kernel does, rows of channels whose locations lie in two
+//               swizzled halves: K-major operands of the weight gradient, and as MN-major operand that of the input gradient, so that one rounding and one
+//               write to shared memory serve both.  (A thread that owns a location and reads 32 of its channels, as in conv111_tc_kernel, has its warp fetch 128
+//               bytes of 32 rows, whose lines, at any multiple of four bytes, its neighbours fetch again: the pass took 1.03 ms; row pieces by bulk copies, which are
+//               issued one after the other, 1.5.)  The sums of gout add the fp32 values before they are rounded;
+//   warp 16     one thread issues the tcgen05.mma of a tile: cout / 16 for the input gradient, 8 for every 128 rows of the weight gradient, whose accumulators
+//               (mtiles x nt columns) stay in TMEM over all tiles of a level range, next to those of the input gradient, two or four tiles in flight;
+//   warps 17-24 epilogue as in conv111_tc_kernel, and the weight sums at the end of a level range.
+struct C1JointParams {
+    int n_segs;
+    ll seg_begin[C1_MAX_SEGS], seg_end[C1_MAX_SEGS];
+    int seg_slot[C1_MAX_SEGS];
+    const float* in; ll ld_in; int cin;
+    const float* gout; ll ld_out; int cout;
+    const float* w;                                // [slot][cout][cin]
+    float* gin; ll ld_gin;
+    float* partial;                                // [segment][block][cout][cin]
+    float* sums;                                   // [block][cout] (null: not wanted)
+    int stages, nt, mtiles, nacc;                  // ring; cin padded; 128-row accumulators of the weight gradient; accumulators of the input gradient
+    uint32_t idesc_x, idesc_w;
+    int* error_flag;
+};
+
+constexpr int C1J_PROD = 16, C1J_MMA = C1J_PROD, C1J_EPI = C1J_PROD + 1, C1J_THREADS = (C1J_EPI + 8) * 32;
+
+template<int WPG>
+__global__ void __launch_bounds__(C1J_THREADS, 1) conv111_tc_joint_kernel(const __grid_constant__ C1JointParams P) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int nt = P.nt, nacc = P.nacc, stages = P.stages;
+    const int kpad = (P.cout + 15) / 16 * 16, half_bytes = (kpad + nt) * 128, stage_bytes = 2 * half_bytes;
+    unsigned char* b_s = smem + (size_t) stages * stage_bytes;                      // [kpad / 8][nt][8] bf16
+    float* out_s = reinterpret_cast<float*>(b_s + (size_t) nt * kpad * 2);          // [2][C1_OUT_CH][256]
+    float* sums_s = out_s + C1_OUT_BYTES / 4;                                       // [groups][kpad]: a channel belongs to one warp of each group
+    constexpr int groups = C1J_PROD / WPG;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sums_s + groups * kpad);
+    uint64_t* full = bars;                              // [stages] operands written (the warps of a group)
+    uint64_t* empty = bars + C1_MAX_STAGES;             // [stages] MMAs that read the stage completed
+    uint64_t* tmem_full = empty + C1_MAX_STAGES;        // [nacc]   accumulator of the input gradient complete
+    uint64_t* tmem_empty = tmem_full + C1_MAX_ACC;      // [nacc]   read back (4 epilogue warps)
+    uint64_t* done = tmem_empty + C1_MAX_ACC;           //          all MMAs of the level range completed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < stages; ++i) { mbar_init(smem_u32(full + i), WPG); mbar_init(smem_u32(empty + i), 1); }
+        for (int i = 0; i < nacc; ++i) { mbar_init(smem_u32(tmem_full + i), 1); mbar_init(smem_u32(tmem_empty + i), 4); }
+        mbar_init(smem_u32(done), 1);
+        *abort_flag = 0;
+        fence_mbar_init();
+    }
+    // the rows that pad the contraction are zeros that nobody writes again
+    const int pad_rows = kpad - P.cout;
+    for (int e = tid; e < stages * 2 * pad_rows * 8; e += C1J_THREADS)
+        *reinterpret_cast<uint4*>(smem + (e / (pad_rows * 8)) * half_bytes + P.cout * 128 + e % (pad_rows * 8) * 16) = make_uint4(0, 0, 0, 0);
+    for (int e = tid; e < groups * kpad; e += C1J_THREADS) sums_s[e] = 0.f;
+    if (warp == C1J_MMA) { tmem_alloc(smem_u32(tmem_slot), 512); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_w = *tmem_slot, tmem_x = tmem_w + P.mtiles * nt;
+    bool failed = false;
+    int piece = 0;
+    const int w8 = warp - C1J_EPI, set = w8 >> 2;
+    uint32_t j_base = 0;                                // tiles of the level ranges before
+    uint32_t done_phase = 0;
+
+    for (int seg = 0; seg < P.n_segs; ++seg) {
+        const ll sb = P.seg_begin[seg], se = P.seg_end[seg];
+        const int seg_tiles = (int) ((se - sb + TILE_M - 1) / TILE_M);
+        const int pair = seg_tiles > (int) gridDim.x ? 1 : 0;
+        const int seg_units = (seg_tiles + pair) >> pair;
+        const int units = (int) blockIdx.x < seg_units ? (seg_units - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
+        const int mine = (units << pair) - (units > 0 && (seg_tiles & pair) && (seg_units - 1) % (int) gridDim.x == (int) blockIdx.x ? 1 : 0);
+        auto tile_begin = [&](int it) { return sb + ((((ll) blockIdx.x + (ll) (it >> pair) * gridDim.x) << pair) + (it & pair)) * TILE_M; };
+        // ---- the level's weights -> B operand (every accumulator of the previous level range has been read back) ----
+        tc_fence_before();
+        __syncthreads();
+        {
+            const float* wslot = P.w + (ll) P.seg_slot[seg] * P.cout * P.cin;
+            for (int e = tid; e < nt * kpad / 8; e += C1J_THREADS) {
+                const int n = e % nt, k8 = e / nt;
+                float v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int k = k8 * 8 + q;
+                    v[q] = (n < P.cin && k < P.cout) ? __ldg(wslot + (ll) k * P.cin + n) : 0.f;
+                }
+                uint4 pk;
+                pk.x = pack_bf16x2(v[0], v[1]); pk.y = pack_bf16x2(v[2], v[3]); pk.z = pack_bf16x2(v[4], v[5]); pk.w = pack_bf16x2(v[6], v[7]);
+                *reinterpret_cast<uint4*>(b_s + ((size_t) k8 * nt + n) * 16) = pk;
+            }
+            fence_proxy_async();
+        }
+        __syncthreads();
+        tc_fence_after();
+
+        if (warp < C1J_PROD) {
+            // ---------------- producers ----------------
+            const int grp = warp / WPG, sub = warp % WPG, used = min(groups, stages);      // (a ring at least as long as the groups keeps the phases that a wait can meet apart)
+            const int nrows = P.cout + P.cin;      // channel rows of a tile
+            float* sums = sums_s + grp * kpad;
+            for (int it = grp; grp < used && it < mine && !failed; it += used) {
+                const uint32_t j = j_base + (uint32_t) it, slot = j % (uint32_t) stages, use = j / (uint32_t) stages;
+                const ll p0 = tile_begin(it);
+                if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
+                unsigned char* st = smem + (size_t) slot * stage_bytes;
+                const bool whole = p0 + TILE_M <= se;
+                for (int r0 = sub; r0 < nrows; r0 += 8 * WPG) {      // 8 rows of this warp x 4 quarters of 32 locations in flight
+                    float v[8][4];
+                    auto source = [&](int r) { return (r < P.cout ? P.gout + (ll) r * P.ld_out : P.in + (ll) (r - P.cout) * P.ld_in) + p0 + lane; };
+                    if (whole) {                                     // no condition per load: a branch each costs more than the loads
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const float* src = source(min(r0 + u * WPG, nrows - 1));      // (the rows that repeat are not stored)
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) v[u][q] = src[q * 32];
+                        }
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const float* src = source(min(r0 + u * WPG, nrows - 1));
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) v[u][q] = p0 + q * 32 + lane < se ? src[q * 32] : 0.f;       // locations past the end are zeros
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int r = r0 + u * WPG;
+                        if (r >= nrows) break;
+                        const int orow = r < P.cout ? r : kpad + (r - P.cout);
+                        unsigned char* dst = st + (size_t) orow * 128 + ((lane & 7) << 1);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)                  // location 32 q + lane: half q >> 1, 16-byte piece 4 (q & 1) + lane / 8, swizzled
+                            *reinterpret_cast<__nv_bfloat16*>(dst + (q >> 1) * half_bytes + (((((q & 1) << 2) + (lane >> 3)) ^ (orow & 7)) << 4)) = __float2bfloat16(v[u][q]);
+                    }
+                    if (P.sums && r0 < P.cout) {                     // the fp32 values, before they are rounded: 8 rows in 9 shuffles
+                        float s[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) s[u] = (v[u][0] + v[u][1]) + (v[u][2] + v[u][3]);       // (of rows that repeat or are not of gout, not used)
+#pragma unroll
+                        for (int h = 4; h > 0; h >>= 1)              // lane l keeps the rows whose bit h is that of l
+#pragma unroll
+                            for (int u = 0; u < h; ++u) { const float x = s[u], y = s[u + h]; s[u] = ((lane & h) ? y : x) + __shfl_xor_sync(0xffffffffu, (lane & h) ? x : y, h); }
+                        s[0] += __shfl_xor_sync(0xffffffffu, s[0], 8);
+                        s[0] += __shfl_xor_sync(0xffffffffu, s[0], 16);
+                        const int r = r0 + lane * WPG;
+                        if (lane < 8 && r < P.cout) sums[r] += s[0];
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(full + slot));   // the MMA thread fences the generic-proxy writes after its wait
+            }
+        } else if (warp == C1J_MMA) {
+            // ---------------- MMA issue ----------------
+            if (elect_one()) {
+                const uint64_t dw0 = make_desc(smem_u32(b_s), nt * 16, 128, 0);
+                const int ksteps = kpad / 16;
+                for (int it = 0; it < mine && !failed; ++it) {
+                    const uint32_t j = j_base + (uint32_t) it, slot = j % (uint32_t) stages, use = j / (uint32_t) stages;
+                    const uint32_t acc = j % (uint32_t) nacc, acc_use = j / (uint32_t) nacc;
+                    if (acc_use > 0 && !mbar_wait(smem_u32(tmem_empty + acc), (acc_use - 1) & 1, abort_flag)) { failed = true; break; }
+                    if (!mbar_wait(smem_u32(full + slot), use & 1, abort_flag)) { failed = true; break; }
+                    fence_proxy_async();          // generic-proxy writes of the producers -> tensor-core (async proxy) reads
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + (size_t) slot * stage_bytes);
+                    const uint64_t da0 = make_desc(a_addr, half_bytes, 1024, 2);                 // 128 locations = two halves, 16 channels = 16 rows
+                    for (int k = 0; k < ksteps; ++k)
+                        umma_bf16(tmem_x + acc * nt, da0 + (uint64_t) ((k * 2048) >> 4), dw0 + (uint64_t) ((k * 2 * nt * 16) >> 4), P.idesc_x, k > 0 ? 1u : 0u);
+                    umma_commit(smem_u32(tmem_full + acc));
+                    for (int half = 0; half < 2; ++half) {
+                        const uint32_t hb = a_addr + half * half_bytes;
+                        const uint64_t db = make_desc(hb + kpad * 128, 16, 1024, 2);
+                        for (int mt = 0; mt < P.mtiles; ++mt) {
+                            // (128 rows: behind those of gout lies what follows them in shared memory, and results that nobody reads)
+                            const uint64_t da = make_desc(hb + mt * 128 * 128, 16, 1024, 2);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                umma_bf16(tmem_w + mt * nt, da + (uint64_t) ((k * 32) >> 4), db + (uint64_t) ((k * 32) >> 4), P.idesc_w, (it > 0 || half > 0 || k > 0) ? 1u : 0u);
+                        }
+                    }
+                    umma_commit(smem_u32(empty + slot));
+                }
+                if (!failed && mine > 0) umma_commit(smem_u32(done));
+            }
+        } else {
+            // ---------------- epilogue ----------------
+            for (int u = 0; u < units; ++u) {
+                const int it = (u << pair) + set;
+                const uint32_t j = j_base + (uint32_t) it, acc = j % (uint32_t) nacc;
+                store_unit(P.gin, P.ld_gin, P.cin, nullptr, tile_begin(u << pair), (int) min(se - tile_begin(u << pair), (ll) (TILE_M << pair)), set <= pair && it < mine,
+                           tmem_x + acc * nt, smem_u32(tmem_full + acc), (j / (uint32_t) nacc) & 1, smem_u32(tmem_empty + acc), out_s, w8, piece, failed, abort_flag);
+            }
+            // weight sums of the level range: set 0 the even, set 1 the odd pieces of 16 columns
+            float* dst = P.partial + ((ll) seg * gridDim.x + blockIdx.x) * P.cout * P.cin;
+            if (mine == 0) {
+                for (int e = tid - C1J_EPI * 32; e < P.cout * P.cin; e += 256) dst[e] = 0.f;     // this block still owns its slice
+            } else if (!failed && mbar_wait_warp(smem_u32(done), done_phase & 1, abort_flag)) {
+                tc_fence_after();
+                const int q = warp & 3;
+#pragma unroll 1
+                for (int mt = 0; mt < P.mtiles; ++mt) {
+                    const int o = mt * 128 + q * 32 + lane;
+#pragma unroll 1
+                    for (int c0 = set * 16; c0 < P.cin; c0 += 32) {
+                        uint32_t r[16];
+                        tmem_ld16(tmem_w + ((uint32_t) (q * 32) << 16) + mt * nt + c0, r);
+                        tmem_ld_wait();
+                        if (o < P.cout) {
+#pragma unroll
+                            for (int jj = 0; jj < 16; ++jj)
+                                if (c0 + jj < P.cin) dst[(ll) o * P.cin + c0 + jj] = __uint_as_float(r[jj]);
+                        }
+                    }
+                }
+            } else failed = true;
+        }
+        if (mine > 0) ++done_phase;
+        if (failed) *abort_flag = 1;
+        j_base += (uint32_t) mine;
+    }
+
+    if (failed) {
+        *abort_flag = 1;
+        if (P.error_flag) *P.error_flag = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (P.sums)
+        for (int c = tid; c < P.cout; c += C1J_THREADS) {
+            float v = 0.f;
+            for (int k = 0; k < groups; ++k) v += sums_s[k * kpad + c];
+            P.sums[(ll) blockIdx.x * P.cout + c] = v;
+        }
+    if (warp == C1J_MMA) tmem_dealloc(tmem_w, 512);
+}
+
+// dst[slot of segment y][e] += the blocks' partial sums; the last y (bias): dst_bias[e] = those of the bias.  A block has 32 entries, warp w adds
+// every eighth of the blocks' sums; the warps' sums are added in order.
+struct C1Reduce { int n_segs; int slot[C1_MAX_SEGS]; };
+__global__ void __launch_bounds__(256) c1_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ bias_partial, C1Reduce R, int nblocks, int elems, int cout,
+                                                        float* __restrict__ gw, float* __restrict__ gbias) {
+    __shared__ float sums[8][32];
+    const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane, seg = blockIdx.y;
+    const bool bias = seg == R.n_segs;
+    const int n = bias ? cout : elems;
+    if ((int) blockIdx.x * 32 >= n) return;
+    const float* src = bias ? bias_partial : partial + (ll) seg * nblocks * elems;
     float s = 0.f;
-    for (int c = 0; c < nblocks; ++c) s += partial[(ll) c * elems + e];
-    dst[e] += s;
+    if (e < n)
+#pragma unroll 4
+        for (int b = wrp; b < nblocks; b += 8) s += src[(ll) b * n + e];
+    sums[wrp][lane] = s;
+    __syncthreads();
+    if (wrp == 0 && e < n) {
+        for (int k = 1; k < 8; ++k) s += sums[k][lane];
+        if (bias) gbias[e] = s; else gw[(ll) R.slot[seg] * elems + e] += s;
+    }
+}
+
+template<int WPG>
+int launch_c1_joint(const C1JointParams& P, int grid, size_t smem, cudaStream_t st) {
+    auto kern = conv111_tc_joint_kernel<WPG>;
+    APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    AprnetProfScope _prof("conv111_tc_dw:joint", st);
+    kern<<<grid, C1J_THREADS, smem, st>>>(P);
+    APRNET_LAUNCH_CHECK();
+    return APRNET_OK;
 }
 
 template<int NT>
@@ -557,8 +831,61 @@ extern "C" int aprnet_conv111_backward_weights_tc(const aprnet_apr* a, int dl, i
         }
         if (rc) return rc;
         { AprnetProfScope _prof("conv111_dw_reduce", st);
-        c1_reduce_partial_kernel<<<aprnet_ceil_div(elems, 256), 256, 0, st>>>(partial, grid, elems, gw + (ll) sg.slot * elems);
+        C1Reduce R;
+        R.n_segs = 1; R.slot[0] = sg.slot;
+        c1_reduce_kernel<<<(unsigned) aprnet_ceil_div(elems, 32), 256, 0, st>>>(partial, nullptr, R, grid, (int) elems, cout, gw, nullptr);
         }
+    }
+    APRNET_LAUNCH_CHECK();
+    return APRNET_OK;
+}
+
+// All gradients of a layer in one pass: grad_input (written), grad_weights (accumulated into) and, where grad_bias is not null, the sums of grad_output over the
+// structure's locations (written).  APRNET_ERR_UNSUPPORTED where a channel count is below 8 or above 256, cin above 4 cout, the operands of two tiles do not fit shared memory or the
+// accumulators TMEM: the passes apart then.
+extern "C" int aprnet_conv111_backward_tc(const aprnet_apr* a, int dl, int cin, int cout, int S, const float* in, int64_t ld_in, const float* gout, int64_t ld_out,
+                                          const float* w, float* gin, int64_t ld_gin, float* gw, float* gbias, float* partial, int64_t partial_elems, void* stream) {
+    APRNET_ARG_CHECK(a && a->valid_dl(dl) && in && gout && w && gin && gw && partial && cin > 0 && cout > 0 && S > 0, "bad argument");
+    APRNET_DEVICE_CHECK(a);
+    const ll n = a->number_parts(dl), elems = (ll) cin * cout;
+    APRNET_ARG_CHECK(ld_in >= n && ld_out >= n && ld_gin >= n, "leading dimension too small");
+    if (cin < 8 || cout < 8 || cin > 256 || cout > 256) return APRNET_ERR_UNSUPPORTED;
+    // what is saved is reading gout twice more: 16 -> 16 channels 0.21 ms instead of 0.33, 64 -> 32 0.59 instead of 0.67, but 128 -> 8 0.97 instead of 0.94
+    if (4 * cout < cin) return APRNET_ERR_UNSUPPORTED;
+    C1JointParams P;
+    C1Reduce R;
+    ll tiles = 0;
+    P.n_segs = 0;
+    for (const Segment& sg : aprnet_segments(a, dl, S, true)) {
+        if (P.n_segs >= C1_MAX_SEGS) return APRNET_ERR_UNSUPPORTED;
+        P.seg_begin[P.n_segs] = sg.begin; P.seg_end[P.n_segs] = sg.end; P.seg_slot[P.n_segs] = R.slot[P.n_segs] = sg.slot;
+        tiles = std::max<ll>(tiles, (sg.end - sg.begin + TILE_M - 1) / TILE_M);
+        ++P.n_segs;
+    }
+    if (P.n_segs == 0) return APRNET_ERR_UNSUPPORTED;
+    R.n_segs = P.n_segs;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int blocks = (int) std::min<ll>(tiles, sms), grid = (int) std::min<ll>(blocks, partial_elems / (P.n_segs * elems + cout));
+    if (grid < 1 || grid < blocks / 2) return APRNET_ERR_UNSUPPORTED;            // too little workspace
+    P.in = in; P.ld_in = ld_in; P.cin = cin; P.gout = gout; P.ld_out = ld_out; P.cout = cout; P.w = w; P.gin = gin; P.ld_gin = ld_gin;
+    P.partial = partial; P.sums = gbias ? partial + (ll) grid * P.n_segs * elems : nullptr;
+    P.nt = pick_nt(cin); P.mtiles = (cout + 127) / 128; P.nacc = P.nt <= 64 ? 4 : 2;
+    P.idesc_x = make_idesc(P.nt, true, false); P.idesc_w = make_idesc(P.nt, false, false);
+    P.error_flag = aprnet_tc_error_flag_device();
+    const int kpad = (cout + 15) / 16 * 16, wpg = cin + cout <= 16 ? 2 : (cin + cout <= 32 ? 4 : 8);
+    const size_t stage = (size_t) (kpad + P.nt) * 256, smem_max = 227 * 1024;
+    const size_t fixed = (size_t) P.nt * kpad * 2 + C1_OUT_BYTES + (size_t) C1J_PROD / wpg * kpad * 4 + (2 * C1_MAX_STAGES + 2 * C1_MAX_ACC + 1) * 8 + 16 + 1024;
+    if ((P.mtiles + P.nacc) * P.nt > 512 || fixed + 2 * stage > smem_max) return APRNET_ERR_UNSUPPORTED;
+    P.stages = (int) std::min<size_t>(C1_MAX_STAGES, (smem_max - fixed) / stage);
+    const size_t smem = P.stages * stage + fixed;
+    cudaStream_t st = (cudaStream_t) stream;
+    const int rc = wpg == 2 ? launch_c1_joint<2>(P, grid, smem, st) : (wpg == 4 ? launch_c1_joint<4>(P, grid, smem, st) : launch_c1_joint<8>(P, grid, smem, st));
+    if (rc) return rc;
+    { AprnetProfScope _prof("conv111_dw_reduce", st);
+    c1_reduce_kernel<<<dim3((unsigned) aprnet_ceil_div(std::max<ll>(elems, gbias ? cout : 0), 32), (unsigned) (P.n_segs + (gbias ? 1 : 0))), 256, 0, st>>>(
+        partial, P.sums, R, grid, (int) elems, cout, gw, gbias);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;

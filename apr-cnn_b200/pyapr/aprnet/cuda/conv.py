@@ -12,7 +12,7 @@ from torch.autograd import Function
 from torch.nn import init
 
 from _pyaprwrapper.data_containers import APRPtrVector
-from _pyaprwrapper.aprnet.cuda import (conv111_backward, conv111_forward, conv333_backward_with_rows, conv333_backward_with_tree,
+from _pyaprwrapper.aprnet.cuda import (conv111_backward, conv111_backward_with_bias, conv111_forward, conv333_backward_with_rows, conv333_backward_with_tree,
                                        conv333_forward_keep_rows, conv333_forward_keep_tree, get_conv_precision,
                                        restrict_kernel333_backward, restrict_kernel333_forward)
 
@@ -88,9 +88,9 @@ class Conv111Function(Function):
     def backward(ctx, grad_output):
         inputs, weights, bias, level_deltas = ctx.saved_tensors
         grad_output = grad_output.contiguous()
-        grad_input, grad_weights = conv111_backward(APRPtrVector(ctx.aprs), inputs, weights, grad_output, level_deltas, ctx.precision)
-        grad_bias = grad_output.sum(dim=(0, 2)) if bias is not None else None
-        return grad_input, grad_weights, grad_bias, None, None, None
+        backward = conv111_backward if bias is None else conv111_backward_with_bias
+        grad_input, grad_weights, *grad_bias = backward(APRPtrVector(ctx.aprs), inputs, weights, grad_output, level_deltas, ctx.precision)
+        return grad_input, grad_weights, grad_bias[0] if grad_bias else None, None, None, None
 
 
 _FUNCTIONS = {(1, 1, 1): Conv111Function, (3, 3, 3): Conv333Function}

@@ -197,9 +197,11 @@ def kernel_table(prof, steps, nparts, ntree, peaks, layers, bf16, fma_tflops=Non
             tc111.update([(a, b, d), (b, a, d)])
     agg["conv111"] = sum(2 * 4.0 * (ci + co) * nparts[dl] for ci, co, dl in c111 if (ci, co, dl) not in tc111)
     dw111 = sum(4.0 * (ci + co) * nparts[dl] for ci, co, dl in c111)
-    if "conv111_tc_dw" in prof and "conv111_dw" in prof:
-        dw111 = None                                                   # mixed: no per-name split
+    joint111 = sum(4.0 * (2 * ci + co) * nparts[dl] for ci, co, dl in c111)      # with the input gradient
+    if sum(name in prof for name in ("conv111_tc_dw", "conv111_tc_dw:joint", "conv111_dw")) > 1:
+        dw111 = joint111 = None                                        # mixed: no per-name split
     agg["conv111_dw"] = agg["conv111_tc_dw"] = dw111
+    agg["conv111_tc_dw:joint"] = joint111
     for name, bpe in GN_BYTES.items():
         agg[name] = sum(bpe * c * nparts[dl] for c, dl in (joint if name.endswith("_rows") else gn))
     agg["groupnorm_bwd_apply"] -= sum(GN_BYTES["groupnorm_bwd_apply"] * c * nparts[dl] for c, dl in joint)

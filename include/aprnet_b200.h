@@ -313,6 +313,13 @@ int aprnet_conv111_backward_input_tc(const aprnet_apr* apr, int level_delta, int
 int aprnet_conv111_backward_weights_tc(const aprnet_apr* apr, int level_delta, int cin, int cout, int num_stencils,
                                        const float* input, int64_t ld_in, const float* grad_output, int64_t ld_out,
                                        float* grad_weights, float* partial, int64_t partial_elems, void* stream);
+/* Both gradients in one pass over grad_output and input: grad_input is written, grad_weights accumulated into; grad_bias (Cout),
+ * or NULL, receives the sums of grad_output over the structure's locations.  partial as above.  APRNET_ERR_UNSUPPORTED below 8 or above 256
+ * channels, with cin > 4 cout, where the weights and two tiles do not fit an SM, or with a partial that is too small: call the entries above then. */
+int aprnet_conv111_backward_tc(const aprnet_apr* apr, int level_delta, int cin, int cout, int num_stencils, const float* input,
+                               int64_t ld_in, const float* grad_output, int64_t ld_out, const float* weights, float* grad_input,
+                               int64_t ld_grad_in, float* grad_weights, float* grad_bias, float* partial, int64_t partial_elems,
+                               void* stream);
 int64_t aprnet_conv111_partial_elems(int cin, int cout);
 int aprnet_conv111_backward_weights(const aprnet_apr* apr, int level_delta, int dtype, int cin, int cout,
                                     int num_stencils, const void* input, int64_t ld_in, const void* grad_output,

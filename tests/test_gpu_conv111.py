@@ -42,3 +42,42 @@ def test_conv111_edges(name, cin, cout):
         assert bool(((x.grad[0].double() - want).abs() <= size * 2.0 ** -16).all()), dl
         want = gd @ xd.t()
         assert float((conv.weight.grad.double().reshape(cout, cin) - want).norm() / want.norm()) <= 1e-5, dl
+
+
+@pytest.mark.parametrize("cin,cout", [(8, 8), (17, 16), (16, 33), (64, 24), (100, 128), (24, 200), (128, 31), (64, 256)])
+def test_conv111_joint_gradients(cin, cout):
+    """All gradients of a layer with a stencil per level and a bias, one item and a padded batch.  A bias gradient adds the fp32 values of at most 14 k locations
+    in chains of at most 64 after 7 halvings, the blocks' sums in chains of at most 20: |error| <= (64 + 7 + 20 + 8) 2^-24 < 2^-17 of the sum of magnitudes."""
+    import pyapr
+    from pyapr.aprnet import cuda as ops
+    arrays = [H.blob_arrays((64, 128, 128), 40, 11), H.arrays("odd")]
+    aprs = [pyapr.apr_from_arrays(a) for a in arrays]
+    for a in aprs:
+        a.init_cuda()
+    torch.manual_seed(cin + 1000 * cout)
+    exact = lambda *s: torch.randn(*s, device="cuda").bfloat16().float()
+    counts = [int(pyapr.aprnet.utils.number_particles(a, 0)) for a in aprs]
+    for items in ([0], [1], [0, 1]):
+        n = max(counts[k] for k in items)
+        conv = ops.APRConv(cin, cout, nstencils=3, kernel_size=(1, 1, 1), precision="bf16").cuda()
+        with torch.no_grad():
+            conv.weight.copy_(exact(*conv.weight.shape))
+        x, g = exact(len(items), cin, n).requires_grad_(True), torch.randn(len(items), cout, n, device="cuda")
+        gb = g.bfloat16().float()
+        conv(x, [aprs[k] for k in items], torch.zeros(len(items), dtype=torch.int32)).backward(g)
+        want_w = torch.zeros(3, cout, cin, device="cuda", dtype=torch.double)
+        for b, k in enumerate(items):
+            a, begin, row = arrays[k], 0, 0
+            for level in range(a.level_min, a.level_max + 1):
+                row += a.dims[level][0] * a.dims[level][1]
+                end = int(a.row_ptr[row])
+                slot = min(a.level_max - level, 2)
+                gd, xd, w = gb[b, :, begin:end].double(), x.detach()[b, :, begin:end].double(), conv.weight.detach()[slot].double().reshape(cout, cin)
+                size = w.t().abs() @ gd.abs()
+                assert bool(((x.grad[b, :, begin:end].double() - w.t() @ gd).abs() <= size * 2.0 ** -16).all()), (items, level)
+                want_w[slot] += gd @ xd.t()
+                begin = end
+            assert end == counts[k] and bool((x.grad[b, :, end:] == 0).all())
+        assert float((conv.weight.grad.double().reshape(3, cout, cin) - want_w).norm() / want_w.norm()) <= 1e-5
+        want = g.double().sum(dim=(0, 2))
+        assert bool(((conv.bias.grad.double() - want).abs() <= g.double().abs().sum(dim=(0, 2)) * 2.0 ** -17).all())

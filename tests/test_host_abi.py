@@ -65,6 +65,7 @@ CALLS = {
     "aprnet_conv333_backward_input_cross_level_tc": (i(0), i(8), i(8), i(1), p, i(16), p, p, n, p, n, p, p, n, None),
     "aprnet_conv111_forward": (i(0), i(0), i(8), i(8), i(1), p, n, p, p, n, None),
     "aprnet_conv111_forward_tc": (i(0), i(8), i(8), i(1), p, n, p, p, n, None),
+    "aprnet_conv111_backward_tc": (i(0), i(8), i(8), i(1), p, n, p, n, p, p, n, p, p, p, C.c_int64(1 << 20), None),
 }
 
 
