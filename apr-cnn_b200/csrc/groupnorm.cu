@@ -95,6 +95,8 @@ constexpr int GN_UNROLL = 4, GN_TILE = GN_UNROLL * GN_TPB;
 template<typename T> __device__ __forceinline__ ll first_of(const T* row) {
     return (ll) blockIdx.x * GN_TILE + threadIdx.x - (ll) ((reinterpret_cast<uintptr_t>(row) & 127) / sizeof(T));
 }
+// all threads of the block have all entries of the tile: no condition per access then (forward in a batch of four 3.43 -> 3.34 ms)
+__device__ __forceinline__ bool whole_tile(ll i0, ll n) { const ll b = i0 - threadIdx.x; return b >= 0 && b + GN_TILE <= n; }
 // Their blocks per row: four waves over the chip, so that a block's statistics (sums of the partials, a division and a square root in double
 // precision, about 1 us) are spread over many tiles, but at least two tiles.  With 2048 entries per block whatever the row, the forward kernel took 4.92 ms
 // in a batch of four tensors of 1.8 M locations (2.5 times the statistics, which read what it reads and writes), now 3.43; on one of 3.5 M locations
@@ -127,6 +129,16 @@ __global__ void __launch_bounds__(GN_TPB) gn_relu_apply_kernel(const T* __restri
     T* yr = y + row * n;
     for (ll i0 = first_of(yr); i0 < n; i0 += (ll) gridDim.x * GN_TILE) {
         T v[GN_UNROLL];
+        if (whole_tile(i0, n)) {
+#pragma unroll
+            for (int u = 0; u < GN_UNROLL; ++u) v[u] = xr[i0 + u * GN_TPB];
+#pragma unroll
+            for (int u = 0; u < GN_UNROLL; ++u) {
+                const T r = (v[u] - mu) * rs * ga + be;
+                yr[i0 + u * GN_TPB] = (relu && r < T(0)) ? T(0) : r;
+            }
+            continue;
+        }
 #pragma unroll
         for (int u = 0; u < GN_UNROLL; ++u) { const ll i = i0 + u * GN_TPB; if (i >= 0 && i < n) v[u] = xr[i]; }
 #pragma unroll
@@ -242,6 +254,18 @@ __global__ void __launch_bounds__(GN_TPB) gn_backward_apply_kernel(const T* __re
     T* o = dx + row * n;
     for (ll i0 = first_of(o); i0 < n; i0 += (ll) gridDim.x * GN_TILE) {
         T xv[GN_UNROLL], dv[GN_UNROLL];
+        if (whole_tile(i0, n)) {
+#pragma unroll
+            for (int u = 0; u < GN_UNROLL; ++u) { xv[u] = xr[i0 + u * GN_TPB]; dv[u] = dr[i0 + u * GN_TPB]; }
+#pragma unroll
+            for (int u = 0; u < GN_UNROLL; ++u) {
+                const T xh = (xv[u] - mu) * rs;
+                T d = dv[u];
+                if (relu && xh * ga + be <= T(0)) d = T(0);
+                o[i0 + u * GN_TPB] = rs * (d * ga - mA - xh * mB);
+            }
+            continue;
+        }
 #pragma unroll
         for (int u = 0; u < GN_UNROLL; ++u) { const ll i = i0 + u * GN_TPB; if (i >= 0 && i < n) { xv[u] = xr[i]; dv[u] = dr[i]; } }
 #pragma unroll
@@ -258,18 +282,18 @@ __global__ void __launch_bounds__(GN_TPB) gn_backward_apply_kernel(const T* __re
 
 // Stage 3 for a convolution in front of the normalisation whose backward pass works from packed bf16 rows of its output's gradient: the same
 // dx, rounded and written as rows [0, n_rows) of cpad channels, row n_rows zero, instead of a channel-major tensor that would be read once
-// more to be packed (12 + 6 bytes per value; here 10).  The 13 layers
-// of a training step on 3.5 M locations took 2.1 + 1.35 ms in two passes and take 2.26 ms, on 28 M locations 18.7 ms.  One batch item; a block has 32 channels x 128 entries.
-// What bounds it: the loads in flight.  A block has one tile and, between its loads and its stores, nothing of another under way: 0.77 of the copy rate with
-// 48 % of the warps active, which wait for loads (6.9 issue slots per instruction) and at the block's barriers (2.6); issue slots 51 %.
-__global__ void __launch_bounds__(256) gn_backward_apply_rows_kernel(const float* __restrict__ x, const float* __restrict__ dy, ll n, ll n_rows, int C, int ch_per_group,
+// more to be packed (12 + 6 bytes per value; here 10: 2.1 + 1.35 ms in two passes where one now takes 2.00).  One batch item; a block has 32 channels x 128 entries at a time.
+// A block walks its tiles, the next one's loads in flight while a tile is stored: with a tile per block nothing of another was under way between its loads and its
+// stores, and each block added up its partial sums for one tile: the 13 layers of a
+// training step on 3.5 M locations 2.28 ms, now 2.00 (8C + 2C bytes per row at 0.87 of the copy rate).
+constexpr int GN_ROWS_BLOCKS = 4;       // blocks per SM
+__global__ void __launch_bounds__(256, GN_ROWS_BLOCKS) gn_backward_apply_rows_kernel(const float* __restrict__ x, const float* __restrict__ dy, ll n, ll n_rows, int C, int ch_per_group,
                                                                      const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean,
                                                                      const float* __restrict__ rstd, const float* __restrict__ group_terms, const double* __restrict__ partial,
                                                                      int nchunks, float* __restrict__ dgamma, float* __restrict__ dbeta, int relu, int cpad,
                                                                      __nv_bfloat16* __restrict__ out) {
-    __shared__ float tile[32][129], par[32][6];            // mean, rstd, gamma, beta, mA, mB
+    __shared__ float tile[2][32][129], par[32][6];         // par: mean, rstd, gamma, beta, mA, mB
     const int c0 = blockIdx.y * 32, lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
-    const ll r0 = (ll) blockIdx.x * 128;
     if (threadIdx.x < 32 && c0 + (int) threadIdx.x < C) {
         const int c = c0 + threadIdx.x, g = c / ch_per_group;
         float mA, mB;
@@ -289,41 +313,58 @@ __global__ void __launch_bounds__(256) gn_backward_apply_rows_kernel(const float
         float* p = par[threadIdx.x];
         p[0] = mean[g]; p[1] = rstd[g]; p[2] = gamma ? gamma[c] : 1.f; p[3] = beta ? beta[c] : 0.f; p[4] = mA; p[5] = mB;
     }
+    const ll tiles = n_rows / 128 + 1;                     // with the row of zeros
     float xv[4][4], dv[4][4];
+    auto request = [&](ll r0) {
+        if (r0 + 128 <= n_rows && c0 + 32 <= C) {          // no condition per load
+            const ll at = (ll) (c0 + wrp) * n + r0 + lane;
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-        const int ch = c0 + wrp + 8 * cc;
+            for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const ll r = r0 + lane + 32 * k;
-            const bool in = ch < C && r < n_rows;
-            xv[cc][k] = in ? x[(ll) ch * n + r] : 0.f;
-            dv[cc][k] = in ? dy[(ll) ch * n + r] : 0.f;
+                for (int k = 0; k < 4; ++k) { xv[cc][k] = x[at + 8 * cc * n + 32 * k]; dv[cc][k] = dy[at + 8 * cc * n + 32 * k]; }
+            return;
         }
-    }
-    __syncthreads();
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-        const int t = wrp + 8 * cc;
-        const float mu = par[t][0], rs = par[t][1], ga = par[t][2], be = par[t][3], mA = par[t][4], mB = par[t][5];
+        for (int cc = 0; cc < 4; ++cc) {
+            const int ch = c0 + wrp + 8 * cc;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float xh = (xv[cc][k] - mu) * rs;
-            float d = dv[cc][k];
-            if (relu && xh * ga + be <= 0.f) d = 0.f;
-            tile[t][lane + 32 * k] = c0 + t < C && r0 + lane + 32 * k < n_rows ? rs * (d * ga - mA - xh * mB) : 0.f;
+            for (int k = 0; k < 4; ++k) {
+                const ll r = r0 + lane + 32 * k;
+                const bool in = ch < C && r < n_rows;
+                xv[cc][k] = in ? x[(ll) ch * n + r] : 0.f;
+                dv[cc][k] = in ? dy[(ll) ch * n + r] : 0.f;
+            }
         }
-    }
-    __syncthreads();
+    };
+    request((ll) blockIdx.x * 128);
+    __syncthreads();                                       // par
+    int buf = 0;
+    for (ll t = blockIdx.x; t < tiles; t += gridDim.x, buf ^= 1) {
+        const ll r0 = t * 128;
 #pragma unroll
-    for (int e = threadIdx.x; e < 128 * 4; e += 256) {     // consecutive threads take consecutive 8-channel pieces of a row
-        const int rr = e >> 2, piece = e & 3;
-        const ll r = r0 + rr;
-        if (r <= n_rows && c0 + piece * 8 < cpad) {
-            __nv_bfloat162 h[4];
+        for (int cc = 0; cc < 4; ++cc) {
+            const int ch = wrp + 8 * cc;
+            const float mu = par[ch][0], rs = par[ch][1], ga = par[ch][2], be = par[ch][3], mA = par[ch][4], mB = par[ch][5];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(tile[piece * 8 + 2 * i][rr], tile[piece * 8 + 2 * i + 1][rr]);
-            *reinterpret_cast<uint4*>(out + r * cpad + c0 + piece * 8) = *reinterpret_cast<uint4*>(h);
+            for (int k = 0; k < 4; ++k) {
+                const float xh = (xv[cc][k] - mu) * rs;
+                float d = dv[cc][k];
+                if (relu && xh * ga + be <= 0.f) d = 0.f;
+                tile[buf][ch][lane + 32 * k] = c0 + ch < C && r0 + lane + 32 * k < n_rows ? rs * (d * ga - mA - xh * mB) : 0.f;
+            }
+        }
+        __syncthreads();                                   // (the other buffer is written after the next one)
+        if (t + gridDim.x < tiles) request((t + gridDim.x) * 128);      // in flight while this tile is stored
+#pragma unroll
+        for (int e = threadIdx.x; e < 128 * 4; e += 256) { // consecutive threads take consecutive 8-channel pieces of a row
+            const int rr = e >> 2, piece = e & 3;
+            const ll r = r0 + rr;
+            if (r <= n_rows && c0 + piece * 8 < cpad) {
+                __nv_bfloat162 h[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(tile[buf][piece * 8 + 2 * i][rr], tile[buf][piece * 8 + 2 * i + 1][rr]);
+                *reinterpret_cast<uint4*>(out + r * cpad + c0 + piece * 8) = *reinterpret_cast<uint4*>(h);
+            }
         }
     }
 }
@@ -394,7 +435,8 @@ int aprnet_groupnorm_relu_backward_rows(int C, ll n, ll n_rows, int groups, cons
     if (!fused) gn_backward_finalize_kernel<float><<<aprnet_ceil_div(C, 128), 128, 0, st>>>(row_sums, 1, C, cpg, n, gamma, dgamma, dbeta, group_terms);
     }
     { AprnetProfScope _p("groupnorm_bwd_apply_rows", st);
-    gn_backward_apply_rows_kernel<<<dim3((unsigned) aprnet_ceil_div(n_rows + 1, 128), (unsigned) aprnet_ceil_div(cpad, 32)), 256, 0, st>>>(
+    const int gy = aprnet_ceil_div(cpad, 32);
+    gn_backward_apply_rows_kernel<<<dim3((unsigned) std::min<ll>(aprnet_ceil_div(n_rows + 1, 128), aprnet_ceil_div(148 * GN_ROWS_BLOCKS, gy)), (unsigned) gy), 256, 0, st>>>(
         x, dy, n, n_rows, C, cpg, gamma, beta, mean, rstd, group_terms, fused ? ws : nullptr, nchunks, dgamma, dbeta, relu, cpad, (__nv_bfloat16*) rows_out);
     }
     APRNET_LAUNCH_CHECK();
