@@ -7,17 +7,17 @@
 //
 // Arithmetic follows pyapr/aprnet/cuda/src/reconstruct_gpu.cu:5-157 and sample_particles_gpu.cu:5-170.  The
 // reference launches one block per (image row, level) and combines the rows of a coarse cell with atomicAdd.
-// Here both directions run level by level over a pyramid of dense images (level l has 1/8 of the cells of level
-// l + 1, so the whole pyramid costs 1/7 of the image in traffic and scratch):
-//   to the image:    dense_l = the level's particles painted over the two-fold enlarged dense_(l - 1); cells that are
-//                    subdivided hold whatever lies above them and are always painted over further down, because the
-//                    particles tile the volume.  The last level is the image itself.
-//   from the image:  a particle of level l is one cell of S_l, and S_(l - 1) = sums of 2x2x2 cells of S_l (S of the
-//                    last level is the image), clipped at the border like the cells are.
-// The image is written / read exactly once, in whole rows, by one warp per row; every value has one writer and a
-// fixed order of summation.  (One warp per particle sweeping its own cell, the former kernel, touched the rows of an
-// image 8 to 32 bytes at a time: 4.0 ms for image -> particles -> image with both gradients on two channels of
-// 256 x 320 x 384 voxels, 6 % of the HBM rate.)
+// Here every value has one writer and a fixed order of summation:
+//   to the image:    one launch, one warp per row of the image.  The particles tile the volume, so a row is put together from the cells of all levels that cover
+//                    it, each voxel once, in shared memory, and stored in whole lines.  (A pyramid of dense images, each level painted over the two-fold enlarged
+//                    coarser one, wrote and read the voxels of subdivided cells once per level and took a launch per level: 157 us for two channels of
+//                    256 x 320 x 384 voxels, now 91; 39 us at the rate of a copy.)
+//   from the image:  level by level over a pyramid of sums: a particle of level l is one cell of S_l, and S_(l - 1) = sums of 2x2x2 cells of S_l (S of the
+//                    last level is the image), clipped at the border like the cells are.  Level l has 1/8 of the cells of level l + 1, so the
+//                    pyramid costs 1/7 of the image in traffic and scratch.  The image is read once, in whole rows, by one warp per row (pairs of
+//                    voxels where rows are aligned to them: 113 -> 97 us for the same two channels).
+// (One warp per particle sweeping its own cell, the first kernel, touched the rows of an image 8 to 32 bytes at a time: 4.0 ms for image -> particles ->
+// image with both gradients on these two channels, 6 % of the HBM rate.)
 #include "apr_device.cuh"
 #include <algorithm>
 
@@ -26,7 +26,8 @@ namespace {
 typedef long long ll;
 constexpr int WARPS = 8;                 // rows per block
 constexpr int TPB = WARPS * 32;
-constexpr int CHUNK = 512;               // cells of a row that a warp holds in shared memory at a time
+constexpr int CHUNK_BYTES = 2048;        // of a row that a warp holds in shared memory at a time, for each of PAINT_CH channels
+constexpr int PAINT_CH = 2;              // channels that are painted together, with their cells looked up once
 constexpr int CH_PER_BLOCK = 4;          // channels a warp loops over with its row pointers resolved once
 
 // the cells that hold a value at one level: particles, and at the last level of a pooled tensor its upgraded tree nodes
@@ -56,63 +57,97 @@ __device__ __forceinline__ ll cell_volume(const ImageLevel& L, int z, int x, int
     return (ll) (min((z + 1) * s, L.Z) - z * s) * (min((x + 1) * s, L.X) - x * s) * (min((y + 1) * s, L.Y) - y * s);
 }
 
-// dense[c][z][x][:] = the parent level's row enlarged two-fold, then the row's own cells over it
+// the cells of every level (and, behind them, the upgraded nodes of a pooled tensor), which together tile the image
+struct PaintLevels {
+    int n, Z, X, Y, mean;
+    CellRows rows[APRNET_MAX_LEVELS + 1];
+    int k[APRNET_MAX_LEVELS + 1], x_num[APRNET_MAX_LEVELS + 1];
+};
+
+template<typename T> __device__ __forceinline__ void store_equal(T* p, T v, int count) {      // `count` values from an address that is aligned to them (1, 2 or 4)
+    if (count == 1) { *p = v; return; }
+    if (sizeof(T) == 8) {
+        *reinterpret_cast<double2*>(p) = make_double2(v, v);
+        if (count == 4) *reinterpret_cast<double2*>(p + 2) = make_double2(v, v);
+    } else if (count == 4) *reinterpret_cast<float4*>(p) = make_float4(v, v, v, v);
+    else *reinterpret_cast<float2*>(p) = make_float2(v, v);
+}
+
 template<typename T>
-__global__ void __launch_bounds__(TPB) paint_level_kernel(ImageLevel L, const T* __restrict__ parts, ll ld, const T* __restrict__ parent,
-                                                          int parent_x, int parent_y, ll parent_stride, T* __restrict__ dense, int C) {
-    __shared__ T buf_s[WARPS][CHUNK];
-    const int lane = threadIdx.x & 31;
-    T* buf = buf_s[threadIdx.x >> 5];
-    const ll r = (ll) blockIdx.x * WARPS + (threadIdx.x >> 5);
-    if (r >= (ll) L.z_num * L.x_num) return;
-    const int z = (int) (r / L.x_num), x = (int) (r % L.x_num);
-    const ll stride = (ll) L.z_num * L.x_num * L.y_num;
-    const int c0 = blockIdx.y * CH_PER_BLOCK, c1 = min(C, c0 + CH_PER_BLOCK);
-    ll rb[2] = {0, 0}, re[2] = {0, 0};
-    for (int s = 0; s < L.n_rows_sets; ++s) { rb[s] = L.rows[s].row_ptr[r]; re[s] = L.rows[s].row_ptr[r + 1]; }
-    const T* prow = parent ? parent + ((ll) (z >> 1) * parent_x + (x >> 1)) * parent_y : nullptr;
-    for (int y0 = 0; y0 < L.y_num; y0 += CHUNK) {
-        const int len = min(CHUNK, L.y_num - y0);
-        ll pb[2], pe[2];
-        for (int s = 0; s < 2; ++s) {
-            pb[s] = rb[s]; pe[s] = re[s];
-            if (L.y_num > CHUNK && pe[s] > pb[s]) {
-                pb[s] = first_at_or_after(L.rows[s].y, rb[s], re[s], y0);
-                pe[s] = first_at_or_after(L.rows[s].y, pb[s], re[s], y0 + CHUNK);
+__global__ void __launch_bounds__(TPB) paint_rows_kernel(const __grid_constant__ PaintLevels L, const T* __restrict__ parts, ll ld, T* __restrict__ image, int C) {
+    constexpr int CHUNK = CHUNK_BYTES / sizeof(T), VEC = 16 / sizeof(T);
+    __shared__ __align__(16) T buf_s[WARPS][PAINT_CH][CHUNK];
+    const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int) threadIdx.x >> 5, 0);      // (one value per warp, also to the compiler)
+    const ll r = (ll) blockIdx.x * WARPS + w;
+    if (r >= (ll) L.Z * L.X) return;
+    const int z = (int) (r / L.X), x = (int) (r % L.X);
+    // the row pointers of all levels at once, a lane per level
+    ll first = 0, last = 0;
+    if (lane < L.n) {
+        const int k = L.k[lane];
+        const ll* rp = L.rows[lane].row_ptr + (ll) (z >> k) * L.x_num[lane] + (x >> k);
+        first = rp[0]; last = rp[1];
+    }
+    const ll stride = (ll) L.Z * L.X * L.Y;
+    const int c0 = blockIdx.y * PAINT_CH, nc = min(PAINT_CH, C - c0);
+    for (int y0 = 0; y0 < L.Y; y0 += CHUNK) {
+        const int len = min(CHUNK, L.Y - y0);
+        for (int i = 0; i < L.n; ++i) {
+            ll pb = __shfl_sync(0xffffffffu, first, i), pe = __shfl_sync(0xffffffffu, last, i);
+            if (pe <= pb) continue;
+            const int k = L.k[i];
+            const uint16_t* __restrict__ ys = L.rows[i].y;
+            if (L.Y > CHUNK) {              // the cells that reach into this piece of the row
+                pb = first_at_or_after(ys, pb, pe, y0 >> k);
+                pe = first_at_or_after(ys, pb, pe, ((y0 + len - 1) >> k) + 1);
+            }
+            const T* __restrict__ src = parts + (ll) c0 * ld + L.rows[i].index_offset;
+            // a lane writes `width` equal voxels of a cell; 2^shift lanes share a cell
+            const int shift = max(k - 2, 0), width = k == 0 ? 1 : (k == 1 ? 2 : 4);
+            const ll total = (pe - pb) << shift;
+            for (ll e = lane; e < total; e += 32) {
+                const ll p = pb + (e >> shift);
+                const int cell = ys[p], at = (cell << k) + (((int) e & ((1 << shift) - 1)) << 2) - y0;
+                T v[PAINT_CH];
+#pragma unroll
+                for (int c = 0; c < PAINT_CH; ++c) v[c] = src[min(c, nc - 1) * ld + p];
+                if (at < 0 || at >= len) continue;
+                if (L.mean && k > 0) {
+                    const int s = 1 << k, cz = z >> k, cx = x >> k;
+                    const T inv = T(1) / (T) ((ll) (min((cz + 1) * s, L.Z) - cz * s) * (min((cx + 1) * s, L.X) - cx * s) * (min((cell + 1) * s, L.Y) - cell * s));
+#pragma unroll
+                    for (int c = 0; c < PAINT_CH; ++c) v[c] *= inv;
+                }
+#pragma unroll
+                for (int c = 0; c < PAINT_CH; ++c) store_equal(&buf_s[w][c][at], v[c], width);      // (what a clipped cell writes behind the row stays in the buffer)
             }
         }
-        for (int c = c0; c < c1; ++c) {
-            if (prow) {
-                const T* ps = prow + c * parent_stride + (y0 >> 1);
-#pragma unroll 4
-                for (int e = lane; e < (len + 1) >> 1; e += 32) {       // CHUNK is even: one parent value covers cells 2e and 2e + 1
-                    const T v = ps[e];
-                    buf[2 * e] = v; buf[2 * e + 1] = v;
-                }
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < PAINT_CH; ++c) {
+            if (c >= nc) break;
+            T* dst = image + (c0 + c) * stride + r * L.Y + y0;
+            const T* b = buf_s[w][c];
+            int e = lane;
+            if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+                for (int q = lane; q < len / VEC; q += 32) reinterpret_cast<int4*>(dst)[q] = reinterpret_cast<const int4*>(b)[q];
+                e += len / VEC * VEC;
             }
-            __syncwarp();
-            for (int s = 0; s < L.n_rows_sets; ++s) {
-                const T* src = parts + c * ld + L.rows[s].index_offset;
-                for (ll p = pb[s] + lane; p < pe[s]; p += 32) {
-                    const int y = L.rows[s].y[p];
-                    T v = src[p];
-                    if (L.mean && L.k > 0) v *= T(1) / (T) cell_volume(L, z, x, y);
-                    buf[y - y0] = v;
-                }
-            }
-            __syncwarp();
-            T* dst = dense + c * stride + r * L.y_num + y0;
 #pragma unroll 4
-            for (int e = lane; e < len; e += 32) dst[e] = buf[e];
-            __syncwarp();
+            for (; e < len; e += 32) dst[e] = b[e];
         }
+        __syncwarp();
     }
 }
+
+template<typename T> struct Pair;
+template<> struct Pair<float> { typedef float2 type; };
+template<> struct Pair<double> { typedef double2 type; };
 
 // S_(l - 1) = 2x2x2 sums of S_l, and the level's particles read from S_l.  One warp per row of the parent level (up to four
 // rows of the level, which the particles then find in L1); parent == nullptr: only the particles are wanted.
 template<typename T>
-__global__ void __launch_bounds__(TPB) gather_level_kernel(ImageLevel L, T* __restrict__ parts, ll ld, const T* __restrict__ dense,
+__global__ void __launch_bounds__(TPB) gather_level_kernel(const __grid_constant__ ImageLevel L, T* __restrict__ parts, ll ld, const T* __restrict__ dense,
                                                            T* __restrict__ parent, int parent_z, int parent_x, int parent_y, int C) {
     const int lane = threadIdx.x & 31;
     const ll pr = (ll) blockIdx.x * WARPS + (threadIdx.x >> 5);
@@ -126,6 +161,17 @@ __global__ void __launch_bounds__(TPB) gather_level_kernel(ImageLevel L, T* __re
             const T* src = dense + c * stride + ((ll) z0 * L.x_num + x0) * L.y_num;
             T* dst = parent + c * parent_stride + pr * parent_y;
             const ll off[4] = {0, (ll) L.y_num, (ll) L.x_num * L.y_num, ((ll) L.x_num + 1) * L.y_num};
+            if (nz == 2 && nx == 2 && L.y_num % 2 == 0 && (reinterpret_cast<uintptr_t>(src) & (2 * sizeof(T) - 1)) == 0) {       // rows of whole pairs
+                typedef typename Pair<T>::type P2;
+#pragma unroll 4
+                for (int e = lane; e < parent_y; e += 32) {
+                    P2 v[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) v[q] = reinterpret_cast<const P2*>(src + off[q])[e];
+                    dst[e] = ((v[0].x + v[0].y) + (v[1].x + v[1].y)) + ((v[2].x + v[2].y) + (v[3].x + v[3].y));
+                }
+                continue;
+            }
 #pragma unroll 2
             for (int e = lane; e < parent_y; e += 32) {
                 const bool two = 2 * e + 1 < L.y_num;
@@ -171,46 +217,49 @@ ll pyramid_elems(const aprnet_apr* a, int dl) {
     return n;
 }
 
-template<typename T, bool TO_IMAGE>
-int run_levels(const aprnet_apr* a, int dl, int C, T* parts, ll ld, T* image, int mean, T* scratch, cudaStream_t st) {
+// the cells of level l, and at the last level of a pooled tensor the upgraded tree nodes behind the particles
+int cell_rows(const aprnet_apr* a, int dl, int l, CellRows (&rows)[2]) {
+    const LevelMeta& m = a->meta;
+    rows[0].row_ptr = a->row_ptr + m.row_off[l]; rows[0].y = a->y; rows[0].index_offset = 0;
+    rows[1] = rows[0];
+    if (l < a->cml(dl) || dl == 0) return 1;
+    rows[1].row_ptr = a->tree_row_ptr + m.trow_off[l]; rows[1].y = a->tree_y; rows[1].index_offset = a->tree_offset(l);
+    return 2;
+}
+
+template<typename T>
+int run_paint(const aprnet_apr* a, int dl, int C, const T* parts, ll ld, T* image, int mean, cudaStream_t st) {
+    const LevelMeta& m = a->meta;
+    const int cml = a->cml(dl);
+    PaintLevels L;
+    L.n = 0; L.Z = m.z_num[cml]; L.X = m.x_num[cml]; L.Y = m.y_num[cml]; L.mean = mean;
+    for (int l = first_level(a, cml); l <= cml; ++l) {
+        CellRows rows[2];
+        const int sets = cell_rows(a, dl, l, rows);
+        for (int i = 0; i < sets; ++i) { L.rows[L.n] = rows[i]; L.k[L.n] = cml - l; L.x_num[L.n] = m.x_num[l]; ++L.n; }
+    }
+    AprnetProfScope _prof("cells_to_image", st);
+    paint_rows_kernel<T><<<dim3((unsigned) aprnet_ceil_div((ll) L.Z * L.X, WARPS), (unsigned) aprnet_ceil_div(C, PAINT_CH)), TPB, 0, st>>>(L, parts, ld, image, C);
+    APRNET_LAUNCH_CHECK();
+    return APRNET_OK;
+}
+
+template<typename T>
+int run_gather(const aprnet_apr* a, int dl, int C, T* parts, ll ld, const T* image, int mean, T* scratch, cudaStream_t st) {
     const int cml = a->cml(dl), l0 = first_level(a, cml);
     const LevelMeta& m = a->meta;
-    std::vector<T*> dense(cml + 1, nullptr);
-    T* next = scratch;
-    for (int l = l0; l < cml; ++l) { dense[l] = next; next += (ll) C * m.z_num[l] * m.x_num[l] * m.y_num[l]; }
-    dense[cml] = image;
-    auto level = [&](int l) {
+    std::vector<T*> sums(cml + 1, nullptr);
+    for (int l = l0; l < cml; ++l) { sums[l] = scratch; scratch += (ll) C * m.z_num[l] * m.x_num[l] * m.y_num[l]; }
+    for (int l = cml; l >= l0; --l) {
         ImageLevel L;
-        L.rows[0].row_ptr = a->row_ptr + m.row_off[l]; L.rows[0].y = a->y; L.rows[0].index_offset = 0;
-        L.rows[1] = L.rows[0];
-        L.n_rows_sets = 1;
-        if (l == cml && dl > 0) {      // upgraded tree nodes, stored behind the particles
-            L.rows[1].row_ptr = a->tree_row_ptr + m.trow_off[l]; L.rows[1].y = a->tree_y; L.rows[1].index_offset = a->tree_offset(l);
-            L.n_rows_sets = 2;
-        }
+        L.n_rows_sets = cell_rows(a, dl, l, L.rows);
         L.z_num = m.z_num[l]; L.x_num = m.x_num[l]; L.y_num = m.y_num[l]; L.k = cml - l;
         L.Z = m.z_num[cml]; L.X = m.x_num[cml]; L.Y = m.y_num[cml];
         L.mean = mean;
-        return L;
-    };
-    const unsigned gy = (unsigned) aprnet_ceil_div(C, CH_PER_BLOCK);
-    if (TO_IMAGE) {
-        for (int l = l0; l <= cml; ++l) {
-            const ImageLevel L = level(l);
-            const bool top = l == l0;
-            AprnetProfScope _prof("cells_to_image", st);
-            paint_level_kernel<T><<<dim3((unsigned) aprnet_ceil_div((ll) L.z_num * L.x_num, WARPS), gy), TPB, 0, st>>>(
-                L, parts, ld, top ? nullptr : dense[l - 1], top ? 0 : m.x_num[l - 1], top ? 0 : m.y_num[l - 1],
-                top ? 0 : (ll) m.z_num[l - 1] * m.x_num[l - 1] * m.y_num[l - 1], dense[l], C);
-        }
-    } else {
-        for (int l = cml; l >= l0; --l) {
-            const ImageLevel L = level(l);
-            const int pz = (L.z_num + 1) / 2, px = (L.x_num + 1) / 2, py = (L.y_num + 1) / 2;
-            AprnetProfScope _prof("image_to_cells", st);
-            gather_level_kernel<T><<<dim3((unsigned) aprnet_ceil_div((ll) pz * px, WARPS), gy), TPB, 0, st>>>(
-                L, parts, ld, dense[l], l == l0 ? nullptr : dense[l - 1], pz, px, py, C);
-        }
+        const int pz = (L.z_num + 1) / 2, px = (L.x_num + 1) / 2, py = (L.y_num + 1) / 2;
+        AprnetProfScope _prof("image_to_cells", st);
+        gather_level_kernel<T><<<dim3((unsigned) aprnet_ceil_div((ll) pz * px, WARPS), (unsigned) aprnet_ceil_div(C, CH_PER_BLOCK)), TPB, 0, st>>>(
+            L, parts, ld, l == cml ? image : sums[l], l == l0 ? nullptr : sums[l - 1], pz, px, py, C);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -223,13 +272,15 @@ int dispatch(const aprnet_apr* a, int dl, int dtype, int C, void* parts, ll ld, 
     APRNET_ARG_CHECK(ld >= a->number_parts(dl), "leading dimension too small");
     if (dtype != APRNET_F32 && dtype != APRNET_F64) { aprnet_set_error("unsupported dtype %d", dtype); return APRNET_ERR_ARG; }
     cudaStream_t st = (cudaStream_t) stream;
+    if (TO_IMAGE) return dtype == APRNET_F32 ? run_paint<float>(a, dl, C, (const float*) parts, ld, (float*) image, mean, st)
+                                             : run_paint<double>(a, dl, C, (const double*) parts, ld, (double*) image, mean, st);
     void* own = nullptr;                 // without a workspace from the caller: stream-ordered allocation for the call
     if (!workspace) {
         APRNET_CUDA_CHECK(cudaMallocAsync(&own, (size_t) aprnet_image_workspace_bytes(a, dl, dtype, C), st));
         workspace = own;
     }
-    const int rc = dtype == APRNET_F32 ? run_levels<float, TO_IMAGE>(a, dl, C, (float*) parts, ld, (float*) image, mean, (float*) workspace, st)
-                                       : run_levels<double, TO_IMAGE>(a, dl, C, (double*) parts, ld, (double*) image, mean, (double*) workspace, st);
+    const int rc = dtype == APRNET_F32 ? run_gather<float>(a, dl, C, (float*) parts, ld, (const float*) image, mean, (float*) workspace, st)
+                                       : run_gather<double>(a, dl, C, (double*) parts, ld, (const double*) image, mean, (double*) workspace, st);
     if (own) cudaFreeAsync(own, st);
     return rc;
 }

@@ -89,3 +89,29 @@ def test_image_ops_gradcheck(name):
     img = aprnet.Reconstruct()(x.detach(), [apr], ld.clone())
     im = torch.rand_like(img).requires_grad_(True)
     assert gradcheck(lambda t: aprnet.SampleParticles()(t, [apr], ld.clone()), (im,), eps=1e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("channels", [1, 2, 3])
+@pytest.mark.parametrize("shape", [(16, 24, 32), (8, 8, 516), (9, 7, 1030)])
+def test_image_rows_at_any_alignment(shape, channels):
+    """Rows are read in pairs of voxels and stored in 16-byte pieces where their addresses allow it: an image that starts one element further gives the same
+    particles bit for bit, and whole, ragged and several pieces of a row give back each cell's value (all of it copies)."""
+    from _pyaprwrapper.data_containers import APRPtrVector
+    from _pyaprwrapper.aprnet import cuda as C
+    import pyapr
+    from pyapr import synthetic
+    arrays = synthetic.random_apr(shape, 3, density=0.02)
+    apr = pyapr.apr_from_arrays(arrays)
+    apr.init_cuda()
+    ld = torch.zeros(1, dtype=torch.int32)
+    torch.manual_seed(5)
+    for dtype in (torch.float32, torch.float64):
+        flat = torch.randn(1 + channels * shape[0] * shape[1] * shape[2], device="cuda", dtype=dtype)
+        shifted = flat[1:].view(1, channels, *shape)
+        aligned = shifted.clone()
+        parts = C.sample_particles_forward(APRPtrVector([apr]), aligned, ld)
+        assert torch.equal(C.sample_particles_forward(APRPtrVector([apr]), shifted, ld), parts)
+        image = C.reconstruct_forward(APRPtrVector([apr]), parts, ld)
+        fine = C.sample_particles_forward(APRPtrVector([apr]), image, ld)
+        assert torch.allclose(fine, parts, rtol=1e-5 if dtype == torch.float32 else 1e-13, atol=0)
+        assert torch.equal(image, C.reconstruct_forward(APRPtrVector([apr]), parts, ld))
