@@ -5,7 +5,7 @@ blocks of unet_parts.py:6-83): every stage is `n_conv` x [APRConv 3x3x3 (no bias
 ReLU]; going down a stage starts with MaxPool; going up, a 1x1x1 conv block halves the channels,
 UpSampleConst restores the finer level, the skip tensor is concatenated in front, and a stage of conv
 blocks follows; a biased 1x1x1 conv maps to the output classes.  Channel widths double per level.
-GroupNorm / ReLU / cat are ordinary torch operators, as in the reference.
+GroupNorm / ReLU / cat are ordinary torch operators, as in the reference, where `ops` offers no fused form.
 
 `ops` is any namespace providing `APRConv`, `MaxPool` and `UpSampleConst` with the reference's
 constructor and call signatures: `pyapr.aprnet.cuda` for the GPU path, or the CPU reference modules
@@ -32,10 +32,13 @@ class ConvNormAct(nn.Module):
             self.act = nn.ReLU()
         self._conv_norm = getattr(ops, "conv_norm", None)
 
-    def forward(self, x, aprs, level_deltas):
+    def forward(self, x, aprs, level_deltas, skip=None):
+        """skip: a tensor in front of x along the channels"""
         conv_norm = getattr(self, "_conv_norm", None)
-        y = conv_norm(self.conv, self.norm, x, aprs, level_deltas) if conv_norm else self.norm(self.conv(x, aprs, level_deltas))
-        return self.act(y)
+        if conv_norm:
+            return self.act(conv_norm(self.conv, self.norm, x, aprs, level_deltas, skip))
+        x = x if skip is None else torch.cat([skip, x], dim=1)
+        return self.act(self.norm(self.conv(x, aprs, level_deltas)))
 
 
 class Stage(nn.Module):
@@ -45,9 +48,9 @@ class Stage(nn.Module):
         self.blocks = nn.ModuleList(ConvNormAct(ops, widths[i], widths[i + 1], nstencils, (3, 3, 3), num_groups, fused_norm)
                                     for i in range(n_conv))
 
-    def forward(self, x, aprs, level_deltas):
+    def forward(self, x, aprs, level_deltas, skip=None):
         for b in self.blocks:
-            x = b(x, aprs, level_deltas)
+            x, skip = b(x, aprs, level_deltas, skip), None
         return x
 
 
@@ -81,6 +84,5 @@ class APRUNet(nn.Module):
         for k in range(self.depth):
             y = self.reduce[k](y, aprs, level_deltas)
             y = self.ups[k](y, aprs, level_deltas)
-            y = torch.cat([skips[self.depth - 1 - k], y], dim=1)
-            y = self.dec[k](y, aprs, level_deltas)
+            y = self.dec[k](y, aprs, level_deltas, skips[self.depth - 1 - k])
         return self.head(y, aprs, level_deltas)

@@ -317,6 +317,50 @@ std::vector<torch::Tensor> conv333_norm_backward(std::vector<APR*>& aprs, torch:
     return {grad_input, grad_weights, dgamma, dbeta};
 }
 
+// 3x3x3 convolution without a bias, GroupNorm and ReLU, forward, float32: {y}, or {y, mean, rstd, convolution's output, packed rows} where `keep`.  input1: the
+// channels behind those of `input` (a concatenation that is not written out).  Without `keep` nobody sees the convolution's output, and the entries behind
+// the particles of an item are neither written nor read.
+std::vector<torch::Tensor> conv333_norm_forward(std::vector<APR*>& aprs, torch::Tensor input, c10::optional<torch::Tensor> input1, torch::Tensor weights, torch::Tensor level_delta,
+                                                const std::string& precision, c10::optional<torch::Tensor> gamma, c10::optional<torch::Tensor> beta, int64_t groups, double eps,
+                                                bool relu, bool keep) {
+    CHECK_INPUT(input); CHECK_INPUT(weights);
+    const bool pair = input1.has_value() && input1->defined();
+    const int64_t c0 = input.size(1), cin = c0 + (pair ? input1->size(1) : 0), cout = weights.size(1), nb = input.size(0), n = input.size(2);
+    TORCH_CHECK(input.dim() == 3 && weights.dim() == 6 && weights.size(3) == 3 && weights.size(4) == 3 && weights.size(5) == 3 && weights.size(2) == cin, "input tensor shape does not match weights tensor");
+    TORCH_CHECK(input.scalar_type() == torch::kFloat32 && weights.scalar_type() == torch::kFloat32 && groups > 0 && cout % groups == 0, "float32 tensors, channels divisible by groups");
+    if (pair) { CHECK_INPUT((*input1)); TORCH_CHECK(input1->dim() == 3 && input1->size(0) == nb && input1->size(2) == n && input1->scalar_type() == torch::kFloat32, "the two inputs do not match"); }
+    c10::cuda::CUDAGuard guard(input.device());
+    const Batch B(aprs, input, level_delta);
+    const int mode = resolve_mode(precision), slots = (int) weights.size(0);
+    auto out = torch::empty({nb, cout, n}, input.options()), tree = torch::empty({1, cin, B.max_tree}, input.options());
+    const int64_t bytes = B.most_bytes([&](aprnet_apr* h, int dl) { return aprnet_conv333_rows_forward_workspace_bytes(h, dl, mode, (int) cin, (int) cout, slots); });
+    auto ws = torch::empty({keep ? nb : 1, (bytes + 255) / 256 * 256}, input.options().dtype(torch::kUInt8));
+    for (int64_t b = 0; b < nb; ++b) {
+        void* w = row(ws, keep ? b : 0);
+        if (pair)
+            check(aprnet_conv333_rows_forward_pair(B.h[b], B.dl[b], mode, (int) cin, (int) cout, slots, (const float*) row(input, b), n, (int) c0, (const float*) row(*input1, b), n,
+                                                   weights.data_ptr<float>(), nullptr, (float*) row(out, b), n, tree.data_ptr<float>(), tree.size(2), w, stream_of(input)), "conv333_forward");
+        else
+            check(aprnet_conv333_rows_forward(B.h[b], B.dl[b], mode, (int) cin, (int) cout, slots, (const float*) row(input, b), n, weights.data_ptr<float>(), nullptr,
+                                              (float*) row(out, b), n, tree.data_ptr<float>(), tree.size(2), 0, w, stream_of(input)), "conv333_forward");
+    }
+    bool ragged = !keep && nb <= 64, padded = false;
+    for (int64_t v : B.n) padded = padded || v < n;
+    if (!ragged || !padded) { ragged = false; fill_padding(out, B.n); }
+    tree = torch::Tensor();
+    if (!keep) ws = torch::Tensor();
+    auto y = torch::empty_like(out), mean = torch::empty({nb * groups}, input.options()), rstd = torch::empty({nb * groups}, input.options());
+    auto norm_ws = bytes_like(aprnet_groupnorm_workspace_bytes((int) nb, (int) cout, (int) groups), input);
+    const auto g = gamma.has_value() && gamma->defined() ? gamma->contiguous() : torch::Tensor(), be = beta.has_value() && beta->defined() ? beta->contiguous() : torch::Tensor();
+    const void *gp = g.defined() ? g.data_ptr() : nullptr, *bp = be.defined() ? be.data_ptr() : nullptr;
+    check(ragged ? aprnet_groupnorm_relu_forward_valid(APRNET_F32, (int) nb, (int) cout, n, B.n.data(), (int) groups, out.data_ptr(), gp, bp, eps, y.data_ptr(), mean.data_ptr(),
+                                                       rstd.data_ptr(), norm_ws.data_ptr(), relu ? 1 : 0, stream_of(input))
+                 : aprnet_groupnorm_relu_forward(APRNET_F32, (int) nb, (int) cout, n, (int) groups, out.data_ptr(), gp, bp, eps, y.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+                                                 norm_ws.data_ptr(), relu ? 1 : 0, stream_of(input)), "groupnorm_relu_forward");
+    if (!keep) return {y};
+    return {y, mean, rstd, out, ws};
+}
+
 // packed rows of an input whose forward call did not keep them (tree: its tree means per batch item, or undefined)
 static torch::Tensor conv333_pack(std::vector<APR*>& aprs, const torch::Tensor& input, const torch::Tensor& level_delta, int mode, const torch::Tensor& tree) {
     const Batch B(aprs, input, level_delta);
@@ -646,7 +690,8 @@ torch::Tensor restrict_kernel_333_backward(torch::Tensor grad_weights_expanded, 
 }
 
 // ---- max pooling --------------------------------------------------------------------------------
-std::vector<torch::Tensor> maxpool_forward_cuda(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor level_delta) {
+// with_indices: false leaves the second result empty (nothing for a backward pass)
+std::vector<torch::Tensor> maxpool_forward_cuda(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor level_delta, bool with_indices) {
     CHECK_INPUT(input);
     check_batch(aprs, input);
     c10::cuda::CUDAGuard guard(input.device());
@@ -657,11 +702,14 @@ std::vector<torch::Tensor> maxpool_forward_cuda(std::vector<APR*>& aprs, torch::
         max_size = std::max(max_size, aprs[i]->number_parts(dl[i] + 1));
     }
     auto output = torch::empty({input.size(0), input.size(1), max_size}, input.options());
-    auto max_indices = torch::zeros({input.size(0), input.size(1), max_size}, input.options().dtype(torch::kLong));
+    auto max_indices = with_indices ? torch::zeros({input.size(0), input.size(1), max_size}, input.options().dtype(torch::kLong))
+                                    : torch::empty({0}, input.options().dtype(torch::kLong));
     const int dt = dtype_id(input);
     for (int64_t b = 0; b < input.size(0); ++b) {
-        check(aprnet_maxpool_forward(aprs[b]->handle(input), dl[b], dt, (int) input.size(1), row(input, b), input.size(2), row(output, b),
-                                     (int64_t*) row(max_indices, b), max_size, stream_of(input)), "maxpool_forward");
+        check(with_indices ? aprnet_maxpool_forward(aprs[b]->handle(input), dl[b], dt, (int) input.size(1), row(input, b), input.size(2), row(output, b),
+                                                    (int64_t*) row(max_indices, b), max_size, stream_of(input))
+                           : aprnet_maxpool_forward_values(aprs[b]->handle(input), dl[b], dt, (int) input.size(1), row(input, b), input.size(2), row(output, b),
+                                                           max_size, stream_of(input)), "maxpool_forward");
     }
     fill_padding(output, valid_of(aprs, dl, +1));
     return {output, max_indices};
@@ -1017,8 +1065,10 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
     py::module cuda = aprnet.def_submodule("cuda");
     cuda.def("conv333_norm_backward", &conv333_norm_backward, "aprs"_a, "rows"_a, "weights"_a, "conv_out"_a, "grad_y"_a, "gamma"_a, "beta"_a, "mean"_a, "rstd"_a,
              "groups"_a, "relu"_a, "level_delta"_a, "need_grad_input"_a);
-    cuda.def("maxpool_forward_cuda", &maxpool_forward_cuda, "aprs"_a, "input"_a, "level_delta"_a);
+    cuda.def("maxpool_forward_cuda", &maxpool_forward_cuda, "aprs"_a, "input"_a, "level_delta"_a, "with_indices"_a = true);
     cuda.def("maxpool_backward_cuda", &maxpool_backward_cuda, "aprs"_a, "grad_output"_a, "max_indices"_a, "level_delta"_a);
+    cuda.def("conv333_norm_forward", &conv333_norm_forward, "aprs"_a, "input"_a, "input1"_a, "weights"_a, "level_delta"_a, "precision"_a, "gamma"_a, "beta"_a, "groups"_a, "eps"_a,
+             "relu"_a, "keep"_a);
     cuda.def("conv111_forward", &conv111_forward, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "", "bias"_a = py::none());
     cuda.def("conv111_backward", &conv111_backward, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "precision"_a = "");
     cuda.def("conv111_backward_with_bias", &conv111_backward_with_bias, "aprs"_a, "input"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "precision"_a = "");

@@ -73,9 +73,9 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
 }
 
 // ---- operand packing --------------------------------------------------------------------------------
-// rows [0, n): x[:, p]; rows [n, n + t): tree[:, p - n]; row n + t: zeros.  Channels padded with zeros to cpad (multiple of 4).
-__global__ void __launch_bounds__(256) pack_rows_f32_kernel(const float* __restrict__ x, ll ld_x, ll n, const float* __restrict__ tree, ll ld_tree, ll t,
-                                                            int c, int cpad, float* __restrict__ out) {
+// rows [0, n): x[:, p], from channel `split` on x1[:, p]; rows [n, n + t): tree[:, p - n]; row n + t: zeros.  Channels padded with zeros to cpad (multiple of 4).
+__global__ void __launch_bounds__(256) pack_rows_f32_kernel(const float* __restrict__ x, ll ld_x, int split, const float* __restrict__ x1, ll ld_x1, ll n,
+                                                            const float* __restrict__ tree, ll ld_tree, ll t, int c, int cpad, float* __restrict__ out) {
     // tile: 32 channels x 64 rows, read along the particle axis, written as 16-byte pieces of the rows
     __shared__ float tile[32][65];
     const ll r0 = (ll) blockIdx.x * 64;
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) pack_rows_f32_kernel(const float* __restr
         for (int k = 0; k < 2; ++k) {
             const int ch = c0 + wrp + 8 * cc;
             const ll r = r0 + lane + 32 * k;
-            v[cc][k] = (ch < c && r < n + t) ? (r < n ? x[(ll) ch * ld_x + r] : tree[(ll) ch * ld_tree + (r - n)]) : 0.f;
+            v[cc][k] = (ch < c && r < n + t) ? (r < n ? (ch < split ? x[(ll) ch * ld_x + r] : x1[(ll) (ch - split) * ld_x1 + r]) : tree[(ll) ch * ld_tree + (r - n)]) : 0.f;
         }
 #pragma unroll
     for (int cc = 0; cc < 4; ++cc)
@@ -551,10 +551,10 @@ inline size_t weight_bytes(int k_dim, int n_dim, int slots) {
     return align256((size_t) slots * 27 * ((n_dim + nt - 1) / nt * nt) * pad4(k_dim) * sizeof(float));
 }
 
-int run_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, ll t, int c, float* out, cudaStream_t st) {
+int run_pack_rows(const float* x, ll ld_x, int split, const float* x1, ll ld_x1, ll n, const float* tree, ll ld_tree, ll t, int c, float* out, cudaStream_t st) {
     dim3 grid((unsigned) aprnet_ceil_div(n + t + 1, 64), (unsigned) aprnet_ceil_div(pad4(c), 32));
     AprnetProfScope _prof("pack_rows_f32", st);
-    pack_rows_f32_kernel<<<grid, 256, 0, st>>>(x, ld_x, n, tree, ld_tree, t, c, pad4(c), out);
+    pack_rows_f32_kernel<<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, pad4(c), out);
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
@@ -760,11 +760,15 @@ int64_t aprnet_f32_partial_elems(int cin, int cout) {
 int aprnet_f32_pack_input(const aprnet_apr* a, int dl, int cin, const float* in, ll ld_in, const float* tree, ll ld_tree, void* rows, cudaStream_t st) {
     const ll n = a->number_parts(dl), t = a->tree_size(dl);
     if (aprnet_small_cin(cin)) return aprnet_small_stage(in, ld_in, n, tree, ld_tree, t, cin, (float*) rows, st);
-    return run_pack_rows(in, ld_in, n, tree, ld_tree, t, cin, (float*) rows, st);
+    return run_pack_rows(in, ld_in, cin, in, ld_in, n, tree, ld_tree, t, cin, (float*) rows, st);
+}
+
+int aprnet_f32_pack_pair(const aprnet_apr* a, int dl, int cin, const float* in0, ll ld0, int c0, const float* in1, ll ld1, const float* tree, ll ld_tree, void* rows, cudaStream_t st) {
+    return run_pack_rows(in0, ld0, c0, in1, ld1, a->number_parts(dl), tree, ld_tree, a->tree_size(dl), cin, (float*) rows, st);
 }
 
 int aprnet_f32_pack_grad(const aprnet_apr* a, int dl, int cout, const float* gout, ll ld_out, void* grows, cudaStream_t st) {
-    return run_pack_rows(gout, ld_out, a->number_parts(dl), nullptr, 0, 0, cout, (float*) grows, st);
+    return run_pack_rows(gout, ld_out, cout, gout, ld_out, a->number_parts(dl), nullptr, 0, 0, cout, (float*) grows, st);
 }
 
 // forward from the packed input rows at the start of `workspace` (aprnet_f32_forward_bytes)

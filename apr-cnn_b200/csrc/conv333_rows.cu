@@ -13,6 +13,9 @@
 typedef long long ll;
 
 int aprnet_tc_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st);
+int aprnet_tc_pack_rows_pair(const float* x0, ll ld0, int c0, const float* x1, ll ld1, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st);
+int aprnet_f32_pack_pair(const aprnet_apr* a, int dl, int cin, const float* in0, ll ld0, int c0, const float* in1, ll ld1, const float* tree, ll ld_tree, void* rows, cudaStream_t st);
+int aprnet_fill_tree_mean_pair(const aprnet_apr* a, int dl, int C, const float* in0, ll ld0, int c0, const float* in1, ll ld1, float* tree, ll ld_tree, cudaStream_t st);
 int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout, int slots, const void* rows, int kpad,
                           ll tree_base, ll zero_row, const float* w, void* wp_ws, const float* bias, float* out, ll ld_out, cudaStream_t st);
 
@@ -32,6 +35,14 @@ int pack_input(const aprnet_apr* a, int dl, int precision, int cin, const float*
                               : aprnet_f32_pack_input(a, dl, cin, in, ld_in, tree, ld_tree, rows, st);
 }
 
+// forward product from the packed rows at the start of `workspace`
+int product(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const float* w, const float* bias, float* out, ll ld_out, void* workspace, cudaStream_t st) {
+    if (!is_bf16(precision) || aprnet_small_cin(cin)) return aprnet_f32_forward(a, dl, cin, cout, slots, w, bias, out, ld_out, workspace, st);
+    const ll n = a->number_parts(dl), t = a->tree_size(dl);
+    void* wp = (char*) workspace + aprnet_tc_rows_bytes(n + t + 1, cin);
+    return aprnet_tc_gather_conv(a, dl, 0, cin, cout, slots, workspace, aprnet_tc_pad(cin), n, n + t, w, wp, bias, out, ld_out, st);
+}
+
 int forward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const float* in, ll ld_in, const float* w, const float* bias,
                  float* out, ll ld_out, float* tree, ll ld_tree, bool tree_valid, void* workspace, cudaStream_t st) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && in && w && out && tree && workspace, "bad argument");
@@ -40,10 +51,7 @@ int forward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int sl
     int rc = tree_valid ? APRNET_OK : aprnet_fill_tree_mean_forward(a, dl, APRNET_F32, cin, in, ld_in, tree, ld_tree, st);
     if (rc) return rc;
     if ((rc = pack_input(a, dl, precision, cin, in, ld_in, tree, ld_tree, workspace, st))) return rc;
-    if (!is_bf16(precision) || aprnet_small_cin(cin)) return aprnet_f32_forward(a, dl, cin, cout, slots, w, bias, out, ld_out, workspace, st);
-    const ll n = a->number_parts(dl), t = a->tree_size(dl);
-    void* wp = (char*) workspace + aprnet_tc_rows_bytes(n + t + 1, cin);
-    return aprnet_tc_gather_conv(a, dl, 0, cin, cout, slots, workspace, aprnet_tc_pad(cin), n, n + t, w, wp, bias, out, ld_out, st);
+    return product(a, dl, precision, cin, cout, slots, w, bias, out, ld_out, workspace, st);
 }
 
 // `ws`: grad_bytes() bytes.  gout == null: `ws` starts with the packed rows of grad_output already (bf16, Cin > 4).  gin == null: no input gradient; gw == null: no weight gradient; fold_tree: grad_tree is folded into gin
@@ -115,6 +123,23 @@ extern "C" int aprnet_conv333_rows_forward(aprnet_apr* a, int dl, int precision,
                                            const float* bias, float* out, int64_t ld_out, float* tree, int64_t ld_tree, int tree_is_valid, void* workspace, void* stream) {
     APRNET_ARG_CHECK(precision_ok(precision), "unknown precision");
     return forward_rows(a, dl, precision, cin, cout, slots, in, ld_in, w, bias, out, ld_out, tree, ld_tree, tree_is_valid != 0, workspace, (cudaStream_t) stream);
+}
+
+// Forward pass over the concatenation of two tensors of cin0 and cin - cin0 channels, which is never written out: tree means and packed rows are made from both.
+extern "C" int aprnet_conv333_rows_forward_pair(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const float* in0, int64_t ld0, int cin0, const float* in1, int64_t ld1,
+                                                const float* w, const float* bias, float* out, int64_t ld_out, float* tree, int64_t ld_tree, void* workspace, void* stream) {
+    APRNET_ARG_CHECK(precision_ok(precision), "unknown precision");
+    APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && in0 && in1 && w && out && tree && workspace, "bad argument");
+    APRNET_DEVICE_CHECK(a);
+    APRNET_ARG_CHECK(cin0 > 0 && cin0 < cin && cin0 % 4 == 0 && !aprnet_small_cin(cin), "the first tensor's channels must be a multiple of four, both together more than four");
+    const ll n = a->number_parts(dl), t = a->tree_size(dl);
+    APRNET_ARG_CHECK(ld0 >= n && ld1 >= n && ld_out >= n && ld_tree >= t, "leading dimension too small");
+    cudaStream_t st = (cudaStream_t) stream;
+    int rc = aprnet_fill_tree_mean_pair(a, dl, cin, in0, ld0, cin0, in1, ld1, tree, ld_tree, st);
+    if (rc) return rc;
+    rc = is_bf16(precision) ? aprnet_tc_pack_rows_pair(in0, ld0, cin0, in1, ld1, n, tree, ld_tree, t, cin, aprnet_tc_pad(cin), workspace, st)
+                            : aprnet_f32_pack_pair(a, dl, cin, in0, ld0, cin0, in1, ld1, tree, ld_tree, workspace, st);
+    return rc ? rc : product(a, dl, precision, cin, cout, slots, w, bias, out, ld_out, workspace, st);
 }
 
 extern "C" int aprnet_conv333_rows_pack(aprnet_apr* a, int dl, int precision, int cin, const float* in, int64_t ld_in, float* tree, int64_t ld_tree, int tree_is_valid,

@@ -60,25 +60,26 @@ template<int KS> __device__ __forceinline__ int swizzled_chunk(int row, int c) {
 }
 
 // ---- operand packing --------------------------------------------------------------------------------
-// rows [0, n): x[:, p]; rows [n, n + t): tree[:, p - n]; row n + t: zeros.  Channels padded to cpad.
+// rows [0, n): x[:, p], from channel `split` on x1[:, p]; rows [n, n + t): tree[:, p - n]; row n + t: zeros.  Channels padded to cpad.
 // HBM-bound.  A block walks tiles of 32 channels x 128 rows; reads are coalesced along the row (particle) axis of the channel-major source, writes are 16-byte
 // pieces (8 channels) of the packed rows, and the next tile's loads are in flight while a tile is stored.
 // The 13 layers of a training step on 3.5 M locations: 1.79 ms with a tile per block and a condition per load, now 1.50; a batch of four in inference 2.05 -> 1.75.
 constexpr int PACK_BLOCKS = 4;          // blocks per SM
-__global__ void __launch_bounds__(256, PACK_BLOCKS) pack_rows_bf16_kernel(const float* __restrict__ x, ll ld_x, ll n, const float* __restrict__ tree, ll ld_tree, ll t,
-                                                            int c, int cpad, __nv_bfloat16* __restrict__ out) {
+__global__ void __launch_bounds__(256, PACK_BLOCKS) pack_rows_bf16_kernel(const float* __restrict__ x, ll ld_x, int split, const float* __restrict__ x1, ll ld_x1, ll n,
+                                                            const float* __restrict__ tree, ll ld_tree, ll t, int c, int cpad, __nv_bfloat16* __restrict__ out) {
     __shared__ float tile[2][32][129];
     const int c0 = blockIdx.y * 32;
     const ll rows = n + t + 1, tiles = (rows + 127) / 128;
     const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;      // 8 warps
     float v[4][4];
     auto request = [&](ll r0) {
-        if (r0 + 128 <= n && c0 + 32 <= c) {                        // no condition per load
-            const float* src = x + (c0 + wrp) * ld_x + r0 + lane;
+        if (r0 + 128 <= n && c0 + 32 <= c && (c0 + 32 <= split || c0 >= split)) {      // no condition per load
+            const ll ld = c0 < split ? ld_x : ld_x1;
+            const float* src = (c0 < split ? x + (c0 + wrp) * ld : x1 + (c0 - split + wrp) * ld) + r0 + lane;
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) v[cc][k] = src[8 * cc * ld_x + 32 * k];
+                for (int k = 0; k < 4; ++k) v[cc][k] = src[8 * cc * ld + 32 * k];
             return;
         }
 #pragma unroll
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(256, PACK_BLOCKS) pack_rows_bf16_kernel(const 
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const ll r = r0 + lane + 32 * k;
-                v[cc][k] = ch < c && r < n + t ? (r < n ? x[(ll) ch * ld_x + r] : tree[(ll) ch * ld_tree + (r - n)]) : 0.f;
+                v[cc][k] = ch < c && r < n + t ? (r < n ? (ch < split ? x[(ll) ch * ld_x + r] : x1[(ll) (ch - split) * ld_x1 + r]) : tree[(ll) ch * ld_tree + (r - n)]) : 0.f;
             }
         }
     };
@@ -635,11 +636,11 @@ int dispatch_tc(const TcParams& P, const TcGeom& g, int total_tiles, cudaStream_
     return APRNET_ERR_UNSUPPORTED;
 }
 
-int run_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, __nv_bfloat16* out, cudaStream_t st) {
+int run_pack_rows(const float* x, ll ld_x, int split, const float* x1, ll ld_x1, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, __nv_bfloat16* out, cudaStream_t st) {
     const int gy = aprnet_ceil_div(cpad, 32);
     const dim3 grid((unsigned) std::min<ll>(aprnet_ceil_div(n + t + 1, 128), aprnet_ceil_div(148 * PACK_BLOCKS, gy)), (unsigned) gy);
     { AprnetProfScope _prof("pack_rows_bf16", st);
-    pack_rows_bf16_kernel<<<grid, 256, 0, st>>>(x, ld_x, n, tree, ld_tree, t, c, cpad, out);
+    pack_rows_bf16_kernel<<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, cpad, out);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -650,7 +651,12 @@ int run_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, 
 int* aprnet_tc_error_flag_device() { return ensure_error_flag() == APRNET_OK ? g_error_flag_dev : nullptr; }
 
 int aprnet_tc_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st) {
-    return run_pack_rows(x, ld_x, n, tree, ld_tree, t, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st);
+    return run_pack_rows(x, ld_x, c, x, ld_x, n, tree, ld_tree, t, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st);
+}
+
+// the same for the concatenation of two tensors of c0 and c - c0 channels
+int aprnet_tc_pack_rows_pair(const float* x0, ll ld0, int c0, const float* x1, ll ld1, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st) {
+    return run_pack_rows(x0, ld0, c0, x1, ld1, n, tree, ld_tree, t, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st);
 }
 
 // Gather-GEMM over packed rows.  backward == 0: out[n = co] from rows of the input (k = ci);

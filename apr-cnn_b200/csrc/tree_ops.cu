@@ -66,13 +66,25 @@ __device__ __forceinline__ void tree_node(const int32_t* __restrict__ child, con
     }
 }
 
+// channels [0, split) of the features, then those of a second tensor (a concatenation that is not written out, 1.46 of 25.6 ms of an inference batch of four); split is a
+// multiple of a thread's channels
+template<typename T>
+struct Features {
+    const T* in0; ll ld0;
+    const T* in1; ll ld1;
+    int split;
+    // row 0 as if the channels of c0's tensor began at channel 0
+    __device__ __forceinline__ const T* base(int c0) const { return c0 < split ? in0 : in1 - split * ld1; }
+    __device__ __forceinline__ ll ld(int c0) const { return c0 < split ? ld0 : ld1; }
+};
+
 template<typename T, int CH, bool MAX>
 __global__ void __launch_bounds__(TPB) tree_level_kernel(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree,
-                                                         ll tb, ll te, const T* __restrict__ in, ll ld_in, T* tree,
+                                                         ll tb, ll te, const Features<T> in, T* tree,
                                                          ll ld_tree, int C, ll up_off, int use_up) {
     const ll t = tb + (ll) blockIdx.y * TPB + threadIdx.x;
     const int c0 = blockIdx.x * CH;
-    if (t < te) tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, use_up);
+    if (t < te) tree_node<T, CH, MAX>(child, scale, n_tree, t, in.base(c0), in.ld(c0), tree, ld_tree, c0, min(CH, C - c0), up_off, use_up);
 }
 
 // The coarse end of the tree in one launch: a cluster of blocks owns CH channels and walks the levels [0, n) of `lv` (fine to
@@ -88,18 +100,18 @@ __device__ __forceinline__ void cluster_barrier() {
 
 template<typename T, int CH, bool MAX>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(COARSE_TPB) tree_coarse_kernel(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree,
-                                                                 LevelList lv, const T* __restrict__ in, ll ld_in, T* tree, ll ld_tree, int C, ll up_off) {
+                                                                 LevelList lv, const Features<T> in, T* tree, ll ld_tree, int C, ll up_off) {
     const int c0 = (int) (blockIdx.x / CLUSTER) * CH, first = (int) (blockIdx.x % CLUSTER) * COARSE_TPB + threadIdx.x;
     int i = 0;
     for (; i < lv.n && lv.end[i] - lv.begin[i] > ALONE_NODES; ++i) {
         for (ll t = lv.begin[i] + first; t < lv.end[i]; t += CLUSTER * COARSE_TPB)
-            tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
+            tree_node<T, CH, MAX>(child, scale, n_tree, t, in.base(c0), in.ld(c0), tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
         cluster_barrier();
     }
     if (first >= COARSE_TPB) return;
     for (; i < lv.n; ++i) {
         for (ll t = lv.begin[i] + first; t < lv.end[i]; t += COARSE_TPB)
-            tree_node<T, CH, MAX>(child, scale, n_tree, t, in, ld_in, tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
+            tree_node<T, CH, MAX>(child, scale, n_tree, t, in.base(c0), in.ld(c0), tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
         __syncthreads();
     }
 }
@@ -208,7 +220,7 @@ __global__ void maxpool_kernel(const int32_t* __restrict__ child, ll n_tree, ll 
             for (int s = 0; s < 8; ++s)
                 if ((ch.node >> s & 1) && v[k][s] > best) { best = v[k][s]; arg = ch.at[s]; }
             out[(ll) (c + k) * ld_out + t + out_off] = best;
-            idx[(ll) (c + k) * ld_out + t + out_off] = arg;
+            if (idx) idx[(ll) (c + k) * ld_out + t + out_off] = arg;
         }
     }
 }
@@ -323,7 +335,7 @@ int last_coarse_level(const LevelMeta& m, int cml) {
 }
 
 template<typename T, bool MAX>
-int fill_tree(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree, ll ld_tree, const char* pname, cudaStream_t st) {
+int fill_tree(const aprnet_apr* a, int dl, int C, const Features<T>& in, T* tree, ll ld_tree, const char* pname, cudaStream_t st) {
     constexpr int CH = 4;
     const LevelMeta& m = a->meta;
     const int cml = a->cml(dl);
@@ -344,17 +356,20 @@ int fill_tree(const aprnet_apr* a, int dl, int C, const T* in, ll ld_in, T* tree
         for (ll b = tb; b < te; b += 65535ll * TPB) {              // grid.y holds 65535 blocks
             AprnetProfScope _prof(pname, st);
             const ll e = std::min(te, b + 65535ll * TPB);
-            tree_level_kernel<T, CH, MAX><<<dim3(gx, (unsigned) aprnet_ceil_div(e - b, TPB)), TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, b, e, in, ld_in,
+            tree_level_kernel<T, CH, MAX><<<dim3(gx, (unsigned) aprnet_ceil_div(e - b, TPB)), TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, b, e, in,
                                                                                                           tree, ld_tree, C, up, use_up);
         }
     }
     if (coarse.n > 0) {
         AprnetProfScope _prof(pname, st);
-        tree_coarse_kernel<T, CH, MAX><<<gx * CLUSTER, COARSE_TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, coarse, in, ld_in, tree, ld_tree, C, up);
+        tree_coarse_kernel<T, CH, MAX><<<gx * CLUSTER, COARSE_TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, coarse, in, tree, ld_tree, C, up);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
+
+template<typename T>
+inline Features<T> one_tensor(const T* in, ll ld, int C) { return Features<T>{in, ld, in, ld, C}; }
 
 template<typename T>
 int fill_tree_mean_bwd(const aprnet_apr* a, int dl, int C, T* gin, ll ld_in, T* gtree, ll ld_tree, cudaStream_t st) {
@@ -449,14 +464,19 @@ int upsample_impl(const aprnet_apr* a, int dl, int C, const T* src, ll ld_src, T
         default: aprnet_set_error("%s: unknown dtype %d", __func__, dtype); return APRNET_ERR_ARG; \
     }
 
+// tree means of the concatenation of two float32 tensors of c0 and C - c0 channels (c0 a multiple of four)
+int aprnet_fill_tree_mean_pair(const aprnet_apr* a, int dl, int C, const float* in0, ll ld0, int c0, const float* in1, ll ld1, float* tree, ll ld_tree, cudaStream_t st) {
+    return fill_tree<float, false>(a, dl, C, Features<float>{in0, ld0, in1, ld1, c0}, tree, ld_tree, "tree_mean_fwd", st);
+}
+
 extern "C" int aprnet_fill_tree_mean_forward(const aprnet_apr* a, int dl, int dtype, int C, const void* in, int64_t ld_in,
                                              void* tree, int64_t ld_tree, void* stream) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && in && tree && C > 0, "bad argument");
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_tree >= a->tree_size(dl), "leading dimension too small");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, (fill_tree<float, false>(a, dl, C, (const float*) in, ld_in, (float*) tree, ld_tree, "tree_mean_fwd", st)),
-             (fill_tree<double, false>(a, dl, C, (const double*) in, ld_in, (double*) tree, ld_tree, "tree_mean_fwd", st)));
+    DISPATCH(dtype, (fill_tree<float, false>(a, dl, C, one_tensor((const float*) in, ld_in, C), (float*) tree, ld_tree, "tree_mean_fwd", st)),
+             (fill_tree<double, false>(a, dl, C, one_tensor((const double*) in, ld_in, C), (double*) tree, ld_tree, "tree_mean_fwd", st)));
 }
 
 extern "C" int aprnet_fill_tree_mean_full(const aprnet_apr* a, int dtype, int C, const void* in, int64_t ld_in, void* tree,
@@ -480,8 +500,8 @@ extern "C" int aprnet_fill_tree_max(const aprnet_apr* a, int dtype, int C, const
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_in >= a->n_particles && ld_tree >= a->n_tree, "leading dimension too small");
     cudaStream_t st = (cudaStream_t) stream;
-    DISPATCH(dtype, (fill_tree<float, true>(a, 0, C, (const float*) in, ld_in, (float*) tree, ld_tree, "tree_max", st)),
-             (fill_tree<double, true>(a, 0, C, (const double*) in, ld_in, (double*) tree, ld_tree, "tree_max", st)));
+    DISPATCH(dtype, (fill_tree<float, true>(a, 0, C, one_tensor((const float*) in, ld_in, C), (float*) tree, ld_tree, "tree_max", st)),
+             (fill_tree<double, true>(a, 0, C, one_tensor((const double*) in, ld_in, C), (double*) tree, ld_tree, "tree_max", st)));
 }
 
 extern "C" int aprnet_maxpool_forward(const aprnet_apr* a, int dl, int dtype, int C, const void* in, int64_t ld_in,
@@ -492,6 +512,16 @@ extern "C" int aprnet_maxpool_forward(const aprnet_apr* a, int dl, int dtype, in
     cudaStream_t st = (cudaStream_t) stream;
     DISPATCH(dtype, maxpool_fwd<float>(a, dl, C, (const float*) in, ld_in, (float*) out, (long long*) idx, ld_out, st),
              maxpool_fwd<double>(a, dl, C, (const double*) in, ld_in, (double*) out, (long long*) idx, ld_out, st));
+}
+
+// the same without indices, where no backward pass follows
+extern "C" int aprnet_maxpool_forward_values(const aprnet_apr* a, int dl, int dtype, int C, const void* in, int64_t ld_in, void* out, int64_t ld_out, void* stream) {
+    APRNET_ARG_CHECK(a && a->valid_dl(dl) && a->valid_dl(dl + 1) && in && out && C > 0, "bad argument");
+    APRNET_DEVICE_CHECK(a);
+    APRNET_ARG_CHECK(ld_in >= a->number_parts(dl) && ld_out >= a->number_parts(dl + 1), "leading dimension too small");
+    cudaStream_t st = (cudaStream_t) stream;
+    DISPATCH(dtype, maxpool_fwd<float>(a, dl, C, (const float*) in, ld_in, (float*) out, nullptr, ld_out, st),
+             maxpool_fwd<double>(a, dl, C, (const double*) in, ld_in, (double*) out, nullptr, ld_out, st));
 }
 
 extern "C" int aprnet_maxpool_backward(const aprnet_apr* a, int dl, int dtype, int C, const void* gout, const int64_t* idx,

@@ -9,9 +9,11 @@ from _pyaprwrapper.aprnet.cuda import maxpool_backward_cuda, maxpool_forward_cud
 class MaxPoolFunction(Function):
     @staticmethod
     def forward(ctx, inputs, aprs, level_deltas, increment_level_deltas):
-        output, max_indices = maxpool_forward_cuda(APRPtrVector(aprs), inputs, level_deltas)
-        ctx.aprs = aprs
-        ctx.save_for_backward(max_indices, level_deltas.clone())
+        keep = ctx.needs_input_grad[0]
+        output, max_indices = maxpool_forward_cuda(APRPtrVector(aprs), inputs, level_deltas, keep)
+        if keep:
+            ctx.aprs = aprs
+            ctx.save_for_backward(max_indices, level_deltas.clone())
         if increment_level_deltas:
             level_deltas.add_(1)        # shared state: later layers see the pooled resolution
         return output

@@ -12,7 +12,7 @@ from torch.autograd import Function
 
 from torch.nn.modules import module as _module
 
-from _pyaprwrapper.aprnet.cuda import (conv333_forward_keep_rows, conv333_norm_backward, get_conv_precision, groupnorm_relu_backward,
+from _pyaprwrapper.aprnet.cuda import (conv333_norm_backward, conv333_norm_forward, get_conv_precision, groupnorm_relu_backward,
                                        groupnorm_relu_forward, restrict_kernel333_backward, restrict_kernel333_forward)
 from _pyaprwrapper.data_containers import APRPtrVector
 
@@ -51,27 +51,32 @@ class GroupNormReLU(nn.Module):
 
 
 class ConvGroupNormReLUFunction(Function):
-    """3x3x3 convolution without a bias, GroupNorm and ReLU for one batch item in bf16 arithmetic.  The forward pass is that of the two
-    functions; in the backward pass the gradient between them exists only as the packed bf16 rows that the convolution works from, written
-    by the normalisation (same values, 8 of 18 bytes less per value)."""
+    """3x3x3 convolution without a bias, GroupNorm and ReLU on float32 tensors.  The forward pass is that of the two functions, over `inputs` or the
+    concatenation of `inputs` and `inputs1` along the channels, which is not written out.  keep (one batch item, bf16 arithmetic): a backward pass can follow, in which
+    the gradient between the two exists only as the packed bf16 rows that the convolution works from, written by the normalisation (same values, 8 of
+    18 bytes less per value).  Without it nothing is kept, and the entries behind the particles of a shorter item are not written between the two."""
 
     @staticmethod
-    def forward(ctx, inputs, weights, gamma, beta, aprs, level_deltas, groups, eps, relu):
+    def forward(ctx, inputs, inputs1, weights, gamma, beta, aprs, level_deltas, groups, eps, relu, precision, keep):
         num_levels = max(a.level_max() - a.level_min() + 1 for a in aprs)
         expanded = restrict_kernel333_forward(weights, num_levels)
-        out, rows = conv333_forward_keep_rows(APRPtrVector(aprs), inputs, expanded, level_deltas, "bf16", None, True)
-        y, mean, rstd = groupnorm_relu_forward(out, gamma, beta, groups, eps, relu)
-        ctx.save_for_backward(expanded, level_deltas.clone(), rows, out, gamma, beta, mean, rstd)
-        ctx.aprs, ctx.num_stencils, ctx.groups, ctx.relu = aprs, weights.shape[0], groups, relu
+        y, *kept = conv333_norm_forward(APRPtrVector(aprs), inputs, inputs1, expanded, level_deltas, precision, gamma, beta, groups, eps, relu, keep)
+        if keep:
+            mean, rstd, out, rows = kept
+            ctx.save_for_backward(expanded, level_deltas.clone(), rows, out, gamma, beta, mean, rstd)
+            ctx.aprs, ctx.num_stencils, ctx.groups, ctx.relu, ctx.split = aprs, weights.shape[0], groups, relu, inputs.shape[1]
         return y
 
     @staticmethod
     def backward(ctx, grad_y):
         expanded, level_deltas, rows, out, gamma, beta, mean, rstd = ctx.saved_tensors
+        wanted = ctx.needs_input_grad
         grad_input, grad_expanded, dgamma, dbeta = conv333_norm_backward(APRPtrVector(ctx.aprs), rows, expanded, out, grad_y.contiguous(), gamma, beta, mean, rstd,
-                                                                         ctx.groups, ctx.relu, level_deltas, bool(ctx.needs_input_grad[0]))
-        return (grad_input, restrict_kernel333_backward(grad_expanded, ctx.num_stencils), dgamma if gamma is not None else None,
-                dbeta if beta is not None else None, None, None, None, None, None)
+                                                                         ctx.groups, ctx.relu, level_deltas, bool(wanted[0] or wanted[1]))
+        # two inputs: each has its channels of one gradient
+        grad_input0 = grad_input if not wanted[0] or ctx.split == expanded.shape[2] else grad_input[:, :ctx.split]
+        return (grad_input0 if wanted[0] else None, grad_input[:, ctx.split:] if wanted[1] else None, restrict_kernel333_backward(grad_expanded, ctx.num_stencils),
+                dgamma if gamma is not None else None, dbeta if beta is not None else None, None, None, None, None, None, None, None)
 
 
 def _plain(m, kind):
@@ -81,15 +86,28 @@ def _plain(m, kind):
                  _module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks or _module._global_backward_pre_hooks))
 
 
-def conv_norm(conv, norm, x, aprs, level_deltas):
-    """`norm(conv(x, aprs, level_deltas))` for an `APRConv` followed by a `GroupNormReLU`, as one function where both are plain modules and a
-    backward pass of the convolution in bf16 arithmetic over one batch item can follow; as two calls otherwise, also where only the
-    normalisation wants gradients: the convolution then keeps nothing and has no backward pass.  (More than four input channels: the weight gradient
-    of a first layer reads the gradient channel by channel; up to 79.5 M locations: beyond them the input gradient does.)"""
-    if (_plain(conv, APRConv) and _plain(norm, GroupNormReLU) and conv._function is Conv333Function and conv.bias is None and x.is_cuda and x.dim() == 3 and
-            x.shape[0] == 1 and len(aprs) == 1 and 4 < x.shape[1] == conv.in_channels and norm.num_channels == conv.out_channels and
-            27 * x.shape[2] + 1 < 2 ** 31 and (conv.precision or get_conv_precision()) == "bf16" and torch.is_grad_enabled()):
-        tensors = [t for t in (x, conv.weight, norm.weight, norm.bias) if t is not None]
-        if (x.requires_grad or conv.weight.requires_grad) and all(t.dtype == torch.float32 and t.device == x.device for t in tensors):
-            return ConvGroupNormReLUFunction.apply(x, conv.weight, norm.weight, norm.bias, aprs, level_deltas, norm.num_groups, norm.eps, norm.relu)
+def conv_norm(conv, norm, x, aprs, level_deltas, skip=None):
+    """`norm(conv(x, aprs, level_deltas))` for an `APRConv` followed by a `GroupNormReLU`; with `skip`, x is `torch.cat([skip, x], 1)`.  One function where both
+    are plain modules and either no gradient is wanted or a backward pass of the convolution in bf16 arithmetic over one batch item can follow; two
+    calls (and the concatenation) otherwise, also where only the normalisation wants gradients: the convolution then keeps nothing and has no backward pass.
+    (More than four input channels in a backward pass: the weight gradient of a first layer reads the gradient channel by channel; up to 79.5 M
+    locations: beyond them the input gradient does.)"""
+    features = (x,) if skip is None else (skip, x)
+    if (_plain(conv, APRConv) and _plain(norm, GroupNormReLU) and conv._function is Conv333Function and conv.bias is None and
+            all(t.is_cuda and t.dim() == 3 and t.is_contiguous() for t in features) and len(aprs) == x.shape[0] and x.shape[0] > 0 and
+            sum(t.shape[1] for t in features) == conv.in_channels and norm.num_channels == conv.out_channels):
+        tensors = [t for t in (*features, conv.weight, norm.weight, norm.bias) if t is not None]
+        wanted = torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
+        precision = conv.precision or get_conv_precision()
+        joint = all(t.dtype == torch.float32 and t.device == x.device for t in tensors)
+        if skip is not None:
+            joint = joint and skip.shape[0] == x.shape[0] and skip.shape[2] == x.shape[2] and skip.shape[1] > 0 and skip.shape[1] % 4 == 0 and conv.in_channels > 4
+        if wanted:
+            joint = (joint and x.shape[0] == 1 and 4 < conv.in_channels and 27 * x.shape[2] + 1 < 2 ** 31 and precision == "bf16" and
+                     (conv.weight.requires_grad or any(t.requires_grad for t in features)))
+        if joint:
+            return ConvGroupNormReLUFunction.apply(features[0], features[1] if skip is not None else None, conv.weight, norm.weight, norm.bias, aprs, level_deltas,
+                                                   norm.num_groups, norm.eps, norm.relu, precision, wanted)
+    if skip is not None:
+        x = torch.cat([skip, x], dim=1)
     return norm(conv(x, aprs, level_deltas))

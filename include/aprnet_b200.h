@@ -177,6 +177,11 @@ int aprnet_conv333_rows_forward(aprnet_apr* apr, int level_delta, int precision,
                                 const float* input, int64_t ld_in, const float* weights, const float* bias,
                                 float* output, int64_t ld_out, float* tree, int64_t ld_tree, int tree_is_valid,
                                 void* workspace, void* stream);
+/* Forward pass over the concatenation of two tensors of cin0 (a multiple of four) and cin - cin0 channels that is never written out;
+ * cin above four; otherwise as aprnet_conv333_rows_forward without given tree means. */
+int aprnet_conv333_rows_forward_pair(aprnet_apr* apr, int level_delta, int precision, int cin, int cout, int num_slots, const float* input0,
+                                     int64_t ld_in0, int cin0, const float* input1, int64_t ld_in1, const float* weights, const float* bias,
+                                     float* output, int64_t ld_out, float* tree, int64_t ld_tree, void* workspace, void* stream);
 int aprnet_conv333_rows_pack(aprnet_apr* apr, int level_delta, int precision, int cin, const float* input, int64_t ld_in,
                              float* tree, int64_t ld_tree, int tree_is_valid, void* packed_rows, void* stream);
 /* grad_input (Cin, ld_in) is written (NULL: not computed); grad_weights (num_slots, Cout, Cin, 27) is written or, with
@@ -356,6 +361,11 @@ int64_t aprnet_groupnorm_workspace_bytes(int batch, int channels, int groups);
 int aprnet_groupnorm_relu_forward(int dtype, int batch, int channels, int64_t n, int groups, const void* x,
                                   const void* gamma, const void* beta, double eps, void* y, void* mean, void* rstd,
                                   void* workspace, int relu, void* stream);
+/* The forward pass over a batch (at most 64 items, APRNET_ERR_UNSUPPORTED beyond) whose items hold host_valid[item] <= n entries: what lies
+ * behind them counts as zeros and is not read; y is written whole. */
+int aprnet_groupnorm_relu_forward_valid(int dtype, int batch, int channels, int64_t n, const int64_t* host_valid, int groups, const void* x,
+                                        const void* gamma, const void* beta, double eps, void* y, void* mean, void* rstd, void* workspace,
+                                        int relu, void* stream);
 int aprnet_groupnorm_relu_backward(int dtype, int batch, int channels, int64_t n, int groups, const void* x,
                                    const void* grad_y, const void* gamma, const void* beta, const void* mean,
                                    const void* rstd, void* grad_x, void* grad_gamma, void* grad_beta,
@@ -386,6 +396,9 @@ int aprnet_maxpool_forward(const aprnet_apr* apr, int level_delta, int dtype, in
                            const void* input, int64_t ld_in, void* output, int64_t* max_indices, int64_t ld_out,
                            void* stream);
 /* grad_input must be zero-filled by the caller (only the kept particles and the arg-max positions are written). */
+/* without indices, where no backward pass follows */
+int aprnet_maxpool_forward_values(const aprnet_apr* apr, int level_delta, int dtype, int channels, const void* input, int64_t ld_in,
+                                  void* output, int64_t ld_out, void* stream);
 int aprnet_maxpool_backward(const aprnet_apr* apr, int level_delta, int dtype, int channels,
                             const void* grad_output, const int64_t* max_indices, int64_t ld_out,
                             void* grad_input, int64_t ld_in, void* stream);
