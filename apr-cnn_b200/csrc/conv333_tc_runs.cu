@@ -90,7 +90,10 @@ struct TileWalk {
 //               cycles than it costs the tensor pipe) and commits the stage's free barrier;
 //   10-17       epilogue, four warps per issuer: TMEM -> registers -> global;
 // All waits are bounded and poll the block's abort flag (see conv333_tc.cu).
-template<int NT, int KS, int KORD, int H, int WPS>
+//
+// KUSE: channels of a stage that exist, the others of its KS-wide rows are neither copied nor multiplied.  48 channels (33 to 48, padded) in stages of 16 took three
+// stages per neighbour row, each with rows of 32 bytes: 48 -> 48 on 3.5 M locations 1.04 ms, now 0.76; 96 -> 48, input gradient at level delta 1, 1.40 -> 0.53.
+template<int NT, int KS, int KUSE, int KORD, int H, int WPS>
 __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunParams P, const int stages) {
     constexpr int NG = NPROD / WPS;                          // stages in issue at once
     constexpr int CH = KS / 8;                               // 16-byte chunks per row piece
@@ -103,7 +106,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     constexpr int ROW_BYTES = KS * 2;
     constexpr uint32_t A_LAYOUT = KS == 64 ? 2u : (KS == 32 ? 4u : 6u);     // SWIZZLE_128B / 64B / 32B
     constexpr int A_BYTES = ROWS * ROW_BYTES;
-    constexpr int B_TAP = NT * KS * 2;
+    constexpr int B_TAP = NT * KUSE * 2;
     constexpr int STAGE_BYTES = A_BYTES + 3 * B_TAP;
     constexpr uint32_t IDESC = make_idesc(NT, false, false);
     static_assert(STAGE_BYTES % 1024 == 0 && H * NT <= 512 && WROWS % 32 == 0 && NI % NB == 0, "stages keep the swizzle alignment; accumulators fit TMEM");
@@ -120,7 +123,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
-    const int kchunks = P.kpad / KS, steps = 9 * kchunks;
+    const int kchunks = P.kpad / KUSE, steps = 9 * kchunks;
     const int total_tiles = P.tile_begin[P.n_segs] * P.n_tiles;
     const int my_tiles = (int) blockIdx.x < total_tiles ? (total_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
     const int ngroups = min(NG, stages);
@@ -173,8 +176,8 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
                     if (P.same_level_only) cur[i] = v >= walk.lo && v < walk.hi ? v : zero;
                     else cur[i] = v >= 0 ? v : (v != APRNET_NONE ? tree - v : zero);
                 }
-                const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(P.wp) + ((ll) walk.wslot * 27 + (P.same_level_only ? 26 - 3 * d : 3 * d)) * w_tap_stride + walk.ntile * w_tile + (ll) kc * KS * NT * 2;
-                const __nv_bfloat16* src0 = P.rows + kc * KS + j * 8;
+                const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(P.wp) + ((ll) walk.wslot * 27 + (P.same_level_only ? 26 - 3 * d : 3 * d)) * w_tap_stride + walk.ntile * w_tile + (ll) kc * KUSE * NT * 2;
+                const __nv_bfloat16* src0 = P.rows + kc * KUSE + j * 8;
                 kc += ngroups;
                 if (left > 1) { locate(); request(); }       // in flight while this stage is copied
                 if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
 #pragma unroll
                     for (int i = 0; i < NB; ++i) {
                         const int row = sub * WROWS + (i0 + i) * RW + rsub;
-                        cp_async16(smem_u32(a_s + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) r[i] * P.kpad);
+                        if (KUSE == KS || j < KUSE / 8) cp_async16(smem_u32(a_s + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) r[i] * P.kpad);
                     }
                 }
                 cp_async_arrive_noinc(smem_u32(full + slot));        // this thread's arrival when its copies have landed
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
         // ---------------- MMA issue, every second block of 128 rows ----------------
         const int h0 = warp - MMA_WARP;
         if (h0 < ISSUERS && elect_one()) {
-            constexpr int MMAS = 3 * (KS / 16);
+            constexpr int MMAS = 3 * (KUSE / 16);
             uint32_t slot = 0, use = 0;
             bool ready = false;                   // the next stage is known to be there
             for (int it = 0; it < my_tiles && !failed; ++it) {
@@ -304,14 +307,14 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
 // ---- host side ----------------------------------------------------------------------------------------
 constexpr size_t FIXED = (2 * MAX_STAGES + 4 * MAX_ACC) * 8 + 16 + 2048 + 1024;      // barriers, the rows in front of and behind the ring, alignment
 
-inline size_t stage_bytes(int nt, int ks, int h) { return (size_t) 128 * h * ks * 2 + 3 * (size_t) nt * ks * 2; }
-inline int run_stages(int nt, int ks, int h) { return (int) std::min<size_t>(MAX_STAGES, (226 * 1024 - FIXED) / stage_bytes(nt, ks, h)); }
+inline size_t stage_bytes(int nt, int ks, int kuse, int h) { return (size_t) 128 * h * ks * 2 + 3 * (size_t) nt * kuse * 2; }
+inline int run_stages(int nt, int ks, int kuse, int h) { return (int) std::min<size_t>(MAX_STAGES, (226 * 1024 - FIXED) / stage_bytes(nt, ks, kuse, h)); }
 
-template<int NT, int KS, int KORD, int H, int WPS>
+template<int NT, int KS, int KUSE, int KORD, int H, int WPS>
 int launch_runs(RunParams& P, int sms, cudaStream_t st, const char* pname) {
-    auto kern = conv333_tc_runs_kernel<NT, KS, KORD, H, WPS>;
-    const int stages = run_stages(NT, KS, H);
-    const size_t smem = (size_t) stages * stage_bytes(NT, KS, H) + FIXED;
+    auto kern = conv333_tc_runs_kernel<NT, KS, KUSE, KORD, H, WPS>;
+    const int stages = run_stages(NT, KS, KUSE, H);
+    const size_t smem = (size_t) stages * stage_bytes(NT, KS, KUSE, H) + FIXED;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     for (int i = 0; i < P.n_segs; ++i) P.tile_begin[i + 1] = P.tile_begin[i] + aprnet_ceil_div(P.slot_end[i] - P.slot_begin[i], 128 * H - 2);
     if (P.tile_begin[P.n_segs] == 0) return APRNET_OK;
@@ -326,14 +329,14 @@ int launch_runs(RunParams& P, int sms, cudaStream_t st, const char* pname) {
 // roles whatever the stage holds.  Tall tiles spread that and the weights over more rows; few rows want short tiles on all SMs.
 // (16 -> 16, 32 -> 32, 64 -> 32 at level delta 0 and 64 -> 64 at level delta 1 of 1.8 M particles, forward: H = 2: 0.22, 0.30,
 // 0.45, 0.26 ms; H = 4: 0.16, 0.24, 0.39, 0.25 ms; conv333_tc.cu: 0.52 for 32 -> 32, 0.48 for 64 -> 64.)
-inline int pick_h(const RunParams& P, int nt, int ks, int max_h, int sms) {
+inline int pick_h(const RunParams& P, int nt, int ks, int kuse, int max_h, int sms) {
     int best = 1;
     double cost = 0;
     for (int h = 1; h <= max_h; h *= 2) {
         ll tiles = 0;
         for (int i = 0; i < P.n_segs; ++i) tiles += aprnet_ceil_div(P.slot_end[i] - P.slot_begin[i], 128 * h - 2);
-        const double stage = 550 + h * 3 * (ks / 16) * (32 + nt / 4) + 1.3 * stage_bytes(nt, ks, h) / 128;
-        const double c = (double) ((tiles * P.n_tiles + sms - 1) / sms) * (9 * P.kpad / ks) * stage;
+        const double stage = 550 + h * 3 * (kuse / 16) * (32 + nt / 4) + 1.3 * stage_bytes(nt, ks, kuse, h) / 128;
+        const double c = (double) ((tiles * P.n_tiles + sms - 1) / sms) * (9 * P.kpad / kuse) * stage;
         if (h == 1 || c < cost) { cost = c; best = h; }
     }
     return best;
@@ -343,12 +346,12 @@ inline int pick_h(const RunParams& P, int nt, int ks, int max_h, int sms) {
 
 // Channels between two changes of dy (the order of the products) of this kernel for kpad source channels; 0: not this kernel.
 // nt_order, ks: tile width and channels per stage that conv333_tc.cu takes for the layer.  The forward pass keeps its order: stages of
-// `ks` channels that hold three taps for nt_order <= 64 (the same order as here) but fewer for wider tiles (the same only when all
-// channels are in one stage of one tap).  The input gradient is free: nothing that follows depends on its last bit.
+// `ks` channels that hold three taps for nt_order <= 64, and for 128 where ks < 64 (the same order as here); one tap at a time for 128 and ks = 64 (the same only when all
+// channels are in one stage), pairs of taps for 256.  The input gradient is free: nothing that follows depends on its last bit.
 int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int ks) {
     if (backward) return kpad % 32 == 0 ? 32 : 16;
     if (nt_order <= 64) return ks;
-    return nt_order == 128 && kpad == ks ? ks : 0;
+    return nt_order == 128 && (ks < 64 || kpad == ks) ? ks : 0;
 }
 
 int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, ll tree_base, ll zero_row, const void* wp,
@@ -371,9 +374,9 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // channels per stage: whole 128-byte rows where the width allows (64 -> 64: 0.25 instead of 0.29 ms with 32)
-    const int ks = kpad % 64 == 0 && order >= 32 ? 64 : order;
-    const int h = pick_h(P, nt, ks, nt == 128 ? 2 : (nt == 32 && ks == 16 ? 8 : 4), sms);
-#define RUN_CASE(NT_, KS_, KORD_, H_, WPS_) if (nt == NT_ && ks == KS_ && order == KORD_ && h == H_) return launch_runs<NT_, KS_, KORD_, H_, WPS_>(P, sms, st, pname);
+    const int kuse = kpad == 48 && order == 16 ? 48 : (kpad % 64 == 0 && order >= 32 ? 64 : order), ks = kuse == 48 ? 64 : kuse;
+    const int h = pick_h(P, nt, ks, kuse, nt == 128 ? 2 : (nt == 32 && ks == 16 ? 8 : 4), sms);
+#define RUN_CASE(NT_, KS_, KORD_, H_, WPS_) if (nt == NT_ && kuse == KS_ && order == KORD_ && h == H_) return launch_runs<NT_, KS_ == 48 ? 64 : KS_, KS_, KORD_, H_, WPS_>(P, sms, st, pname);
     // warps per stage: two, so that four stages are in issue at once; four where the ring holds only two or three stages
     RUN_CASE(32, 16, 16, 1, 2) RUN_CASE(32, 16, 16, 2, 2) RUN_CASE(32, 16, 16, 4, 2) RUN_CASE(32, 16, 16, 8, 4)
     RUN_CASE(32, 32, 32, 1, 2) RUN_CASE(32, 32, 32, 2, 2) RUN_CASE(32, 32, 32, 4, 2)
@@ -383,6 +386,8 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     RUN_CASE(64, 32, 32, 1, 2) RUN_CASE(64, 32, 32, 2, 2) RUN_CASE(64, 32, 32, 4, 2)
     RUN_CASE(64, 64, 32, 1, 2) RUN_CASE(64, 64, 32, 2, 4) RUN_CASE(64, 64, 32, 4, 4)
     RUN_CASE(128, 16, 16, 1, 2) RUN_CASE(128, 16, 16, 2, 2) RUN_CASE(128, 32, 32, 1, 2) RUN_CASE(128, 32, 32, 2, 2)
+    RUN_CASE(32, 48, 16, 1, 2) RUN_CASE(32, 48, 16, 2, 2) RUN_CASE(32, 48, 16, 4, 4)
+    RUN_CASE(64, 48, 16, 1, 2) RUN_CASE(64, 48, 16, 2, 4) RUN_CASE(64, 48, 16, 4, 4) RUN_CASE(128, 48, 16, 1, 4) RUN_CASE(128, 48, 16, 2, 4)
     RUN_CASE(128, 64, 32, 1, 4) RUN_CASE(128, 64, 32, 2, 4) RUN_CASE(128, 64, 64, 1, 4) RUN_CASE(128, 64, 64, 2, 4)
 #undef RUN_CASE
     aprnet_set_error("conv333 tensor-core path: unsupported run geometry nt=%d ks=%d order=%d h=%d", nt, ks, order, h);

@@ -50,6 +50,26 @@ def test_run_kernels_match_the_tap_kernels(name, cin, cout):
         assert float((got[1] - want[1]).norm() / want[1].norm()) <= 2e-6, dl
 
 
+@pytest.mark.parametrize("cin,cout", [(16, 128), (40, 72), (48, 128), (96, 128), (160, 100), (33, 20), (48, 64), (128, 48)])
+def test_run_kernels_of_padded_and_wide_layers(cin, cout):
+    """Stages of 48 channels, and forward layers of 65 to 128 result channels whose stages of the tap kernel hold three taps; several tiles per block."""
+    import pyapr
+    from _pyaprwrapper.aprnet import cuda as C
+    apr = pyapr.apr_from_arrays(H.blob_arrays((64, 128, 128), 40, 11))
+    apr.init_cuda()
+    for dl in (0, 1):
+        n = int(pyapr.aprnet.utils.number_particles(apr, dl))
+        try:
+            C.tc_set_option("runs", 0)
+            want = _run(apr, dl, cin, cout, n)
+        finally:
+            C.tc_set_option("runs", 1)
+        got = _run(apr, dl, cin, cout, n)
+        assert C.tc_error_flag() == 0
+        assert torch.equal(got[0], want[0]), (dl, int((got[0] != want[0]).sum()))
+        assert float((got[1] - want[1]).norm() / want[1].norm()) <= 2e-6, dl
+
+
 # widths with one stage per chunk of slots (more than 64 output channels, the last neighbour group of wide inputs) and with several
 DW_WIDTHS = [(8, 8), (16, 40), (33, 33), (64, 32), (24, 120), (32, 128), (128, 64), (128, 128), (130, 32), (48, 200)]
 
