@@ -29,7 +29,6 @@ using tcptx::cp_async_wait;
 typedef long long ll;
 constexpr int MAX_SEGS = APRNET_MAX_LEVELS;
 constexpr int KS = 16;                   // channels (gather) or locations (weight gradient) per ring slot
-constexpr int RING = 4;                  // ring slots
 
 struct SegTable {
     int n;
@@ -73,9 +72,10 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
 }
 
 // ---- operand packing --------------------------------------------------------------------------------
-// rows [0, n): x[:, p], from channel `split` on x1[:, p]; rows [n, n + t): tree[:, p - n]; row n + t: zeros.  Channels padded with zeros to cpad (multiple of 4).
-__global__ void __launch_bounds__(256) pack_rows_f32_kernel(const float* __restrict__ x, ll ld_x, int split, const float* __restrict__ x1, ll ld_x1, ll n,
-                                                            const float* __restrict__ tree, ll ld_tree, ll t, int c, int cpad, float* __restrict__ out) {
+// rows [0, n): x[:, p], with PAIR from channel `split` on x1[:, p] (a kernel of its own: the choice cost one tensor's packing 12 %); rows [n, n + t): tree[:, p - n]; row n + t: zeros.  Channels padded with zeros to cpad (multiple of 4).
+template<bool PAIR>
+__global__ void __launch_bounds__(256) pack_rows_f32_kernel(const float* __restrict__ x, ll ld_x, int split, const float* __restrict__ x1, ll ld_x1, ll n, const float* __restrict__ tree, ll ld_tree, ll t,
+                                                            int c, int cpad, float* __restrict__ out) {
     // tile: 32 channels x 64 rows, read along the particle axis, written as 16-byte pieces of the rows
     __shared__ float tile[32][65];
     const ll r0 = (ll) blockIdx.x * 64;
@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(256) pack_rows_f32_kernel(const float* __restr
         for (int k = 0; k < 2; ++k) {
             const int ch = c0 + wrp + 8 * cc;
             const ll r = r0 + lane + 32 * k;
-            v[cc][k] = (ch < c && r < n + t) ? (r < n ? (ch < split ? x[(ll) ch * ld_x + r] : x1[(ll) (ch - split) * ld_x1 + r]) : tree[(ll) ch * ld_tree + (r - n)]) : 0.f;
+            const float* from = PAIR && ch >= split ? x1 + (ll) (ch - split) * ld_x1 : x + (ll) ch * ld_x;
+            v[cc][k] = (ch < c && r < n + t) ? (r < n ? from[r] : tree[(ll) ch * ld_tree + (r - n)]) : 0.f;
         }
 #pragma unroll
     for (int cc = 0; cc < 4; ++cc)
@@ -140,8 +141,16 @@ enum { FORWARD, SAME_LEVEL, TARGETS };        // forward pass, the two parts of 
 // takes 4 to 25 % off (32 -> 32 on 1.2 M locations 522 -> 465 us, with the sums below), in the same-level part up to 7 % where the tile is at most 32 channels wide
 // (32 -> 32 1805 -> 1753) and minus 3 to 10 % where it is 64 (33 -> 33 3220 -> 3333, 64 -> 64 at level delta 1 2595 -> 2663: the test costs more than
 // the reads).  The forward pass has next to none (neighbours outside the volume).
+// Threads per SM and ring slots.  16 warps of 128 registers instead of 12 of 168 give little, because the register file bounds the loop (paired multiply-adds read
+// four registers a cycle): input gradient of 32 channels 4.94 -> 4.56 ms (32 -> 32, 3.5 M locations, three slots), forward pass of 64 9.01 -> 8.90 ms (64 -> 64 at level
+// delta 1), weight gradient of 16 x 32 tiles 8.16 -> 7.98 (33 -> 24); the other shapes lose 1 to 14 %.
+template<int WM, int TN, int MODE> struct GatherShape {
+    static constexpr bool MORE = TN == 16 && ((MODE == FORWARD && WM == 1) || (MODE == SAME_LEVEL && WM == 2));
+    static constexpr int THREADS = MORE ? 512 : 384, RING = MORE && WM == 2 ? 3 : 4;
+};
 template<int WM, int WN, int TN, int MODE>
-__global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f32_gather_kernel(const F32Params P) {
+__global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, MODE>::THREADS / (32 * WM * WN)) conv333_f32_gather_kernel(const F32Params P) {
+    constexpr int RING = GatherShape<WM, TN, MODE>::RING;
     constexpr int T = 32 * WM * WN, M = 128 * WM, NT = TN * WN;
     constexpr bool KMAJOR = MODE == FORWARD, ZEROS = MODE == TARGETS || (MODE == SAME_LEVEL && NT < 64);
     constexpr int RPT = M * (KS / 4) / T;          // row pieces a thread copies per slot
@@ -353,8 +362,13 @@ struct F32DwParams {
     int cin, cout, ci_blocks, groups;
 };
 
+template<int CIB, int WM, int TN> struct DwShape {
+    static constexpr bool MORE = CIB == 16 && WM == 2 && TN == 16;
+    static constexpr int THREADS = MORE ? 512 : 384, RING = MORE ? 3 : 4;
+};
 template<int CIB, int WM, int WN, int TN>
-__global__ void __launch_bounds__(32 * WM * WN, 384 / (32 * WM * WN)) conv333_f32_dw_kernel(const F32DwParams P) {
+__global__ void __launch_bounds__(32 * WM * WN, DwShape<CIB, WM, TN>::THREADS / (32 * WM * WN)) conv333_f32_dw_kernel(const F32DwParams P) {
+    constexpr int RING = DwShape<CIB, WM, TN>::RING;
     constexpr int T = 32 * WM * WN, M = 128 * WM, NT = TN * WN;
     constexpr int TS = M / CIB;                    // taps of a block
     constexpr int PC = CIB / 4;                    // 16-byte pieces of a gathered row
@@ -554,7 +568,8 @@ inline size_t weight_bytes(int k_dim, int n_dim, int slots) {
 int run_pack_rows(const float* x, ll ld_x, int split, const float* x1, ll ld_x1, ll n, const float* tree, ll ld_tree, ll t, int c, float* out, cudaStream_t st) {
     dim3 grid((unsigned) aprnet_ceil_div(n + t + 1, 64), (unsigned) aprnet_ceil_div(pad4(c), 32));
     AprnetProfScope _prof("pack_rows_f32", st);
-    pack_rows_f32_kernel<<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, pad4(c), out);
+    if (split < c) pack_rows_f32_kernel<true><<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, pad4(c), out);
+    else pack_rows_f32_kernel<false><<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, pad4(c), out);
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
@@ -567,7 +582,7 @@ int run_pack_weights(const aprnet_apr* a, int dl, const float* w, int slots, int
 template<int WM, int WN, int TN, int MODE>
 int launch_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
     constexpr int M = 128 * WM, NT = TN * WN;
-    constexpr size_t smem = (size_t) RING * (M + NT) * KS * sizeof(float);
+    constexpr size_t smem = (size_t) GatherShape<WM, TN, MODE>::RING * (M + NT) * KS * sizeof(float);
     auto kern = conv333_f32_gather_kernel<WM, WN, TN, MODE>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     P.segs = make_seg_table(segs, M);
@@ -621,7 +636,7 @@ inline int dw_max_ranges(int cin, int cout) {
 template<int CIB, int WM, int WN, int TN>
 int launch_dw(const F32DwParams& P, int nranges, int blocks_y, cudaStream_t st, const char* pname) {
     constexpr int TS = 128 * WM / CIB, TAP_STRIDE = KS * CIB + (CIB < 32 ? CIB : 0);
-    constexpr size_t smem = (size_t) RING * (TS * TAP_STRIDE + KS * TN * WN) * sizeof(float);
+    constexpr size_t smem = (size_t) DwShape<CIB, WM, TN>::RING * (TS * TAP_STRIDE + KS * TN * WN) * sizeof(float);
     auto kern = conv333_f32_dw_kernel<CIB, WM, WN, TN>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     AprnetProfScope _prof(pname, st);
