@@ -70,16 +70,16 @@ __global__ void __launch_bounds__(256, PACK_BLOCKS) pack_rows_bf16_kernel(const 
     __shared__ float tile[2][32][129];
     const int c0 = blockIdx.y * 32;
     const ll rows = n + t + 1, tiles = (rows + 127) / 128;
-    const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;      // 8 warps
+    const int lane = threadIdx.x & 31, wrp = __shfl_sync(0xffffffffu, (int) threadIdx.x >> 5, 0);      // 8 warps
     float v[4][4];
     auto request = [&](ll r0) {
-        if (r0 + 128 <= n && c0 + 32 <= c && (c0 + 32 <= split || c0 >= split)) {      // no condition per load
+        if (r0 + 128 <= n && (c0 + 32 <= split || c0 >= split)) {      // one condition per channel, the same for a warp
             const ll ld = c0 < split ? ld_x : ld_x1;
             const float* src = (c0 < split ? x + (c0 + wrp) * ld : x1 + (c0 - split + wrp) * ld) + r0 + lane;
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) v[cc][k] = src[8 * cc * ld + 32 * k];
+                for (int k = 0; k < 4; ++k) v[cc][k] = c0 + wrp + 8 * cc < c ? src[8 * cc * ld + 32 * k] : 0.f;
             return;
         }
 #pragma unroll

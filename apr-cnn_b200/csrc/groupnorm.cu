@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(256, GN_ROWS_BLOCKS) gn_backward_apply_rows_ke
                                                                      int nchunks, float* __restrict__ dgamma, float* __restrict__ dbeta, int relu, int cpad,
                                                                      __nv_bfloat16* __restrict__ out) {
     __shared__ float tile[2][32][129], par[32][6];         // par: mean, rstd, gamma, beta, mA, mB
-    const int c0 = blockIdx.y * 32, lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
+    const int c0 = blockIdx.y * 32, lane = threadIdx.x & 31, wrp = __shfl_sync(0xffffffffu, (int) threadIdx.x >> 5, 0);
     if (threadIdx.x < 32 && c0 + (int) threadIdx.x < C) {
         const int c = c0 + threadIdx.x, g = c / ch_per_group;
         float mA, mB;
@@ -336,12 +336,15 @@ __global__ void __launch_bounds__(256, GN_ROWS_BLOCKS) gn_backward_apply_rows_ke
     const ll tiles = n_rows / 128 + 1;                     // with the row of zeros
     float xv[4][4], dv[4][4];
     auto request = [&](ll r0) {
-        if (r0 + 128 <= n_rows && c0 + 32 <= C) {          // no condition per load
+        if (r0 + 128 <= n_rows) {                          // one condition per channel, the same for a warp
             const ll at = (ll) (c0 + wrp) * n + r0 + lane;
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) { xv[cc][k] = x[at + 8 * cc * n + 32 * k]; dv[cc][k] = dy[at + 8 * cc * n + 32 * k]; }
+                for (int k = 0; k < 4; ++k) {
+                    const bool in = c0 + wrp + 8 * cc < C;
+                    xv[cc][k] = in ? x[at + 8 * cc * n + 32 * k] : 0.f; dv[cc][k] = in ? dy[at + 8 * cc * n + 32 * k] : 0.f;
+                }
             return;
         }
 #pragma unroll
