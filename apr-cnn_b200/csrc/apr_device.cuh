@@ -194,7 +194,8 @@ int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, co
 int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* gout, long long ld_out,
                                   float* gw, int accumulate, float* partial, cudaStream_t st);
 // tensor-core gather over runs (conv333_tc_runs.cu)
-int aprnet_tc_runs_order(int backward, int kpad, int nt, int ks);
+constexpr int APRNET_TAP_KERNEL = 1;      // of aprnet_tc_run_conv: nothing was launched, the kernel that gathers every tap is the faster one
+int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int nt, int ks);
 int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, long long tree_base, long long zero_row, const void* wp,
                        const float* bias, float* out, long long ld_out, int n_dim, int* error_flag, cudaStream_t st, const char* pname);
 int aprnet_pack_weights(const aprnet_apr* a, int dl, bool bf16, const float* w, int slots, int cin, int cout, int transposed, int nt, int n_tiles, int kpad,

@@ -675,8 +675,11 @@ int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout
     if ((rc = aprnet_pack_weights(a, dl, true, w, slots, cin, cout, backward, g.nt, g.n_tiles, g.kpad, wp, st))) return rc;
     char pname[64];
     snprintf(pname, sizeof(pname), "%s:ci%d:co%d:dl%d", backward ? "conv333_tc_bwd_gather" : "conv333_tc_fwd", cin, cout, dl);
-    const int run_order = g_runs_off ? 0 : aprnet_tc_runs_order(backward, g.kpad, g.order_nt, g.ks);
-    if (run_order) return aprnet_tc_run_conv(a, dl, backward, slots, g.nt, run_order, rows, g.kpad, tree_base, zero_row, wp, bias, out, ld_out, n_dim, g_error_flag_dev, st, pname);
+    const int run_order = g_runs_off ? 0 : aprnet_tc_runs_order(backward, g.kpad, g.order_nt, g.nt, g.ks);
+    if (run_order) {
+        rc = aprnet_tc_run_conv(a, dl, backward, slots, g.nt, run_order, rows, g.kpad, tree_base, zero_row, wp, bias, out, ld_out, n_dim, g_error_flag_dev, st, pname);
+        if (rc != APRNET_TAP_KERNEL) return rc;
+    }
     TcParams P;
     P.segs = make_seg_table(aprnet_segments(a, dl, slots, false), TILE_M);
     P.nbr = plan->nbr; P.N = plan->n; P.rows = reinterpret_cast<const __nv_bfloat16*>(rows); P.kpad = g.kpad;

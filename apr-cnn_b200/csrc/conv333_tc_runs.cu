@@ -304,6 +304,209 @@ __global__ void __launch_bounds__(THREADS, 1) conv333_tc_runs_kernel(const RunPa
     if (warp == MMA_WARP) tmem_dealloc(tmem_d, H * NACC * NT);
 }
 
+// Forward pass of layers with 65 to 128 result channels and several chunks of 64 source channels, over runs of cells, in the order of conv333_tc.cu for them: one tap
+// after the other, each over all chunks.  A tap's products run through all source channels before the next tap's, so all chunks of a neighbour row
+// have to be there before its first tap is finished: the rows (pieces of 128 H slots x 64 channels) and the weights (tiles of one tap and chunk) have rings of
+// their own; a piece is given back after the last of its row's three taps, a weight tile after its MMAs.  Gathering every tap by itself the layers were
+// bound by the gather (27 rows per location past L1): 128 -> 128 on 553 k locations 0.52 ms, now 0.45; 256 -> 128 0.99, now 0.86.
+// Roles of the warps: 0-7 producers of pieces, in two groups of four; 8 weights (bulk copies of one thread); 9 MMA issue (one thread); 10-17 epilogue, one set of four warps
+// for every block of 128 rows (H = 1: the first set).
+constexpr int WIDE_MAX_PIECES = 14, WIDE_MAX_TILES = 8;
+template<int NT, int H>
+__global__ void __launch_bounds__(THREADS, 1) conv333_tc_wide_kernel(const RunParams P, const int pieces, const int tiles) {
+    constexpr int KS = 64, CH = 8, RW = 4, WPS = 4;
+    constexpr int ROWS = 128 * H, WROWS = ROWS / WPS, NI = WROWS / RW, LR = WROWS / 32;
+    constexpr int NACC = 512 / (H * NT) < MAX_ACC ? 512 / (H * NT) : MAX_ACC;
+    constexpr int ROW_BYTES = 128, PIECE = ROWS * ROW_BYTES, B_TILE = NT * KS * 2;
+    constexpr uint32_t IDESC = make_idesc(NT, false, false);
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ float bias_s[MAX_N];
+    // the ring of pieces at a multiple of 1024 bytes, with 1024 bytes in front of it and behind it (rows that are read next to a piece's first and last, for results that are not used)
+    unsigned char* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u) + 1024;
+    unsigned char* b_ring = ring + (size_t) pieces * PIECE + 1024;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(b_ring + (size_t) tiles * B_TILE);
+    uint64_t* full = bars;                                   // [pieces] rows landed
+    uint64_t* empty = full + WIDE_MAX_PIECES;                // [pieces] the last tap's MMAs completed
+    uint64_t* w_full = empty + WIDE_MAX_PIECES;              // [tiles]  weights landed
+    uint64_t* w_empty = w_full + WIDE_MAX_TILES;             // [tiles]  MMAs that read them completed
+    uint64_t* tmem_full = w_empty + WIDE_MAX_TILES;          // [NACC]   accumulators of a tile complete
+    uint64_t* tmem_empty = tmem_full + MAX_ACC;              // [NACC]   read back (four warps per block of 128 rows)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + MAX_ACC);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = warp_number(), lane = tid & 31;
+    const int kchunks = P.kpad / KS, steps = 9 * kchunks;    // pieces of a tile
+    const int total_tiles = P.tile_begin[P.n_segs] * P.n_tiles;
+    const int my_tiles = (int) blockIdx.x < total_tiles ? (total_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x : 0;
+
+    if (P.bias) for (int c = tid; c < min(MAX_N, P.n_tiles * NT); c += THREADS) bias_s[c] = c < P.n_dim ? P.bias[c] : 0.f;
+    if (tid == 0) {
+        for (int i = 0; i < pieces; ++i) { mbar_init(smem_u32(full + i), WPS * 32); mbar_init(smem_u32(empty + i), 1); }
+        for (int i = 0; i < tiles; ++i) { mbar_init(smem_u32(w_full + i), 1); mbar_init(smem_u32(w_empty + i), 1); }
+        for (int i = 0; i < NACC; ++i) { mbar_init(smem_u32(tmem_full + i), 1); mbar_init(smem_u32(tmem_empty + i), 4 * H); }
+        *abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == MMA_WARP + 1) { tmem_alloc(smem_u32(tmem_slot), H * NACC * NT); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_d = *tmem_slot;
+    bool failed = false, bulk_issued = false;
+
+    if (warp < NPROD) {
+        // ---------------- rows ----------------
+        const int grp = warp / WPS, sub = warp % WPS, j = lane % CH, rsub = lane / CH;
+        const uint32_t total = (uint32_t) my_tiles * (uint32_t) steps;
+        uint32_t slot = grp, use = 0;                        // (two groups, at least three pieces)
+        uint32_t left = grp < (int) total ? (total - grp + 1) / 2 : 0;
+        TileWalk walk(P);
+        int d = 0, kc = grp;                                 // the piece's neighbour row and channels
+        auto locate = [&]() {
+            while (kc >= kchunks) { kc -= kchunks; ++d; }
+            while (d >= 9) { d -= 9; walk.next(P); }
+        };
+        int32_t raw[LR], cur[LR];
+        auto request = [&]() {                               // table entries of this lane's rows
+            const int first = walk.first(), end = walk.end(ROWS);
+            const int32_t* src = P.src + (ll) d * P.S + walk.s0(ROWS) + sub * WROWS + lane;
+#pragma unroll
+            for (int i = 0; i < LR; ++i) {
+                const int row = sub * WROWS + 32 * i + lane;
+                raw[i] = row >= first && row < end ? __ldg(src + 32 * i) : APRNET_NONE;
+            }
+        };
+        const int32_t zero = (int32_t) P.zero_row, tree = (int32_t) P.tree_base - 2;       // row numbers fit 32 bits
+        if (left > 0) { locate(); request(); }
+        for (; left > 0; --left) {
+#pragma unroll
+            for (int i = 0; i < LR; ++i) { const int32_t v = raw[i]; cur[i] = v >= 0 ? v : (v != APRNET_NONE ? tree - v : zero); }
+            const __nv_bfloat16* src0 = P.rows + kc * KS + j * 8;
+            kc += 2;
+            if (left > 1) { locate(); request(); }           // in flight while this piece is copied
+            if (use > 0 && !mbar_wait_warp(smem_u32(empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
+            unsigned char* a_s = ring + (size_t) slot * PIECE;
+#pragma unroll
+            for (int i0 = 0; i0 < NI; i0 += 8) {             // copies and shuffles keep their order: the rows of several copies are handed round first
+                int32_t r[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) r[i] = __shfl_sync(0xffffffffu, cur[(i0 + i) * RW / 32], ((i0 + i) * RW + rsub) & 31);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int row = sub * WROWS + (i0 + i) * RW + rsub;
+                    cp_async16(smem_u32(a_s + row * ROW_BYTES + (swizzled_chunk<KS>(row, j) << 4)), src0 + (ll) r[i] * P.kpad);
+                }
+            }
+            cp_async_arrive_noinc(smem_u32(full + slot));
+            slot += 2;
+            if (slot >= (uint32_t) pieces) { slot -= pieces; ++use; }
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+    } else if (warp == MMA_WARP) {
+        // ---------------- weights: tap by tap, chunk by chunk ----------------
+        if (elect_one()) {
+            const ll w_tile = (ll) P.kpad * NT * 2, w_tap = P.n_tiles * w_tile;
+            TileWalk walk(P);
+            uint32_t slot = 0, use = 0;
+            for (int it = 0; it < my_tiles && !failed; ++it, walk.next(P)) {
+                const unsigned char* src = reinterpret_cast<const unsigned char*>(P.wp) + (ll) walk.wslot * 27 * w_tap + walk.ntile * w_tile;
+                for (int tap = 0; tap < 27 && !failed; ++tap, src += w_tap)
+                    for (int kc = 0; kc < kchunks; ++kc) {
+                        if (use > 0 && !mbar_wait(smem_u32(w_empty + slot), (use - 1) & 1, abort_flag)) { failed = true; break; }
+                        mbar_expect_tx(smem_u32(w_full + slot), B_TILE);
+                        bulk_copy_g2s(smem_u32(b_ring + (size_t) slot * B_TILE), src + (ll) kc * B_TILE, B_TILE, smem_u32(w_full + slot));
+                        bulk_issued = true;
+                        if (++slot == (uint32_t) tiles) { slot = 0; ++use; }
+                    }
+            }
+        }
+    } else if (warp == MMA_WARP + 1) {
+        // ---------------- MMA issue ----------------
+        if (elect_one()) {
+            uint32_t p0 = 0, p0_use = 0, ws = 0, wu = 0;     // first piece of the neighbour row; weight tile
+            for (int it = 0; it < my_tiles && !failed; ++it) {
+                const uint32_t acc = (uint32_t) it % NACC, acc_use = (uint32_t) it / NACC;
+                if (acc_use > 0 && !mbar_wait(smem_u32(tmem_empty + acc), (acc_use - 1) & 1, abort_flag)) { failed = true; break; }
+                tc_fence_after();
+                for (int d = 0; d < 9 && !failed; ++d) {
+                    for (int dy = 0; dy < 3 && !failed; ++dy) {
+                        uint32_t p = p0, pu = p0_use;
+                        for (int kc = 0; kc < kchunks; ++kc) {
+                            if (dy == 0 && !mbar_test(smem_u32(full + p), pu & 1) && !mbar_wait(smem_u32(full + p), pu & 1, abort_flag)) { failed = true; break; }
+                            if (!mbar_test(smem_u32(w_full + ws), wu & 1) && !mbar_wait(smem_u32(w_full + ws), wu & 1, abort_flag)) { failed = true; break; }
+                            if (dy == 0) fence_proxy_async();        // generic-proxy writes of the cp.async copies -> tensor-core (async proxy) reads
+                            tc_fence_after();
+                            const uint64_t db0 = make_desc(smem_u32(b_ring + (size_t) ws * B_TILE), NT * 16, 128, 0);
+#pragma unroll
+                            for (int h = 0; h < H; ++h) {
+                                const uint64_t da0 = make_desc(smem_u32(ring + (size_t) p * PIECE) + (h * 128 + dy - 1) * ROW_BYTES, 16, 8 * ROW_BYTES, 2u);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k)
+                                    umma_bf16(tmem_d + (h * NACC + acc) * NT, da0 + (uint64_t) ((k * 32) >> 4), db0 + (uint64_t) ((k * 2 * (NT * 16)) >> 4), IDESC, (d > 0 || dy > 0 || kc > 0 || k > 0) ? 1u : 0u);
+                            }
+                            umma_commit(smem_u32(w_empty + ws));
+                            if (dy == 2) umma_commit(smem_u32(empty + p));
+                            if (++ws == (uint32_t) tiles) { ws = 0; ++wu; }
+                            if (++p == (uint32_t) pieces) { p = 0; ++pu; }
+                        }
+                        if (dy == 2) { p0 = p; p0_use = pu; }
+                    }
+                }
+                if (!failed) umma_commit(smem_u32(tmem_full + acc));
+            }
+        }
+    } else if ((warp - EPI_WARP) / 4 < H) {
+        // ---------------- epilogue of one block of 128 rows ----------------
+        const int h = (warp - EPI_WARP) >> 2, q = warp & 3;          // q: TMEM lanes this warp may read
+        TileWalk walk(P);                                            // the tile after the one that is read back
+        auto location = [&](int it) {
+            const int m = h * 128 + q * 32 + lane;
+            if (it >= my_tiles || m == 0 || m == ROWS - 1) return (int32_t) -1;
+            return m >= walk.first() && m < walk.end(ROWS) ? __ldg(P.loc + walk.s0(ROWS) + m) : -1;
+        };
+        int32_t next = location(0);
+        for (int it = 0; it < my_tiles; ++it) {
+            const int n0 = walk.ntile * NT;
+            walk.next(P);
+            const int32_t p = next;
+            next = location(it + 1);
+            const uint32_t acc = (uint32_t) it % NACC, acc_use = (uint32_t) it / NACC;
+            if (!mbar_wait_warp(smem_u32(tmem_full + acc), acc_use & 1, abort_flag)) { failed = true; break; }
+            tc_fence_after();
+#pragma unroll 1
+            for (int c0 = 0; c0 < NT; c0 += 32) {
+                uint32_t r[32];
+                tmem_ld32(tmem_d + ((uint32_t) (q * 32) << 16) + (h * NACC + acc) * NT + c0, r);
+                tmem_ld_wait();
+                if (P.bias) {
+#pragma unroll
+                    for (int jj = 0; jj < 32; ++jj) r[jj] = __float_as_uint(__uint_as_float(r[jj]) + bias_s[n0 + c0 + jj]);
+                }
+                if (p >= 0) {
+                    float* dst = P.out + (ll) (n0 + c0) * P.ld_out + p;
+#pragma unroll
+                    for (int jj = 0; jj < 32; ++jj)
+                        if (n0 + c0 + jj < P.n_dim) dst[(ll) jj * P.ld_out] = __uint_as_float(r[jj]);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(tmem_empty + acc));
+        }
+    }
+
+    // teardown as in conv333_tc_runs_kernel
+    if (failed) {
+        *abort_flag = 1;
+        if (P.error_flag) *P.error_flag = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (bulk_issued && *abort_flag) for (int i = 0; i < 2000; ++i) __nanosleep(100);
+    if (warp == MMA_WARP + 1) tmem_dealloc(tmem_d, H * NACC * NT);
+}
+
 // ---- host side ----------------------------------------------------------------------------------------
 constexpr size_t FIXED = (2 * MAX_STAGES + 4 * MAX_ACC) * 8 + 16 + 2048 + 1024;      // barriers, the rows in front of and behind the ring, alignment
 
@@ -344,15 +547,48 @@ inline int pick_h(const RunParams& P, int nt, int ks, int kuse, int max_h, int s
     return best;
 }
 
+constexpr size_t WIDE_FIXED = (2 * WIDE_MAX_PIECES + 2 * WIDE_MAX_TILES + 2 * MAX_ACC) * 8 + 16 + 2048 + 1024;
+constexpr size_t WIDE_SMEM = 227 * 1024 - 1024;          // (the biases are static)
+
+// Rings of a layer of kpad source channels: all pieces of a neighbour row and one more, and three weight tiles; what is left goes to the pieces of a second row, then to the weights.
+// false: they do not fit
+inline bool wide_shape(int nt, int h, int kpad, int* pieces, int* tiles) {
+    const size_t piece = (size_t) 128 * h * 128, tile = (size_t) nt * 128, room = WIDE_SMEM - WIDE_FIXED;
+    const int kchunks = kpad / 64;
+    if (kchunks + 1 > WIDE_MAX_PIECES || (kchunks + 1) * piece + 3 * tile > room) return false;
+    *tiles = 3;
+    *pieces = (int) std::min<size_t>(std::min(2 * kchunks, WIDE_MAX_PIECES), (room - 3 * tile) / piece);
+    *pieces = std::max(*pieces, kchunks + 1);
+    *tiles = (int) std::min<size_t>(WIDE_MAX_TILES, (room - *pieces * piece) / tile);
+    return *pieces >= 3;
+}
+
+template<int NT, int H>
+int launch_wide(RunParams& P, int sms, cudaStream_t st, const char* pname) {
+    int pieces, tiles;
+    if (!wide_shape(NT, H, P.kpad, &pieces, &tiles)) return APRNET_ERR_UNSUPPORTED;
+    auto kern = conv333_tc_wide_kernel<NT, H>;
+    const size_t smem = (size_t) pieces * 128 * H * 128 + (size_t) tiles * NT * 128 + WIDE_FIXED;
+    APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    for (int i = 0; i < P.n_segs; ++i) P.tile_begin[i + 1] = P.tile_begin[i] + aprnet_ceil_div(P.slot_end[i] - P.slot_begin[i], 128 * H - 2);
+    if (P.tile_begin[P.n_segs] == 0) return APRNET_OK;
+    AprnetProfScope _prof(pname, st);
+    kern<<<std::min(P.tile_begin[P.n_segs] * P.n_tiles, sms), THREADS, smem, st>>>(P, pieces, tiles);
+    APRNET_LAUNCH_CHECK();
+    return APRNET_OK;
+}
+
 } // namespace
 
 // Channels between two changes of dy (the order of the products) of this kernel for kpad source channels; 0: not this kernel.
 // nt_order, ks: tile width and channels per stage that conv333_tc.cu takes for the layer.  The forward pass keeps its order: stages of
 // `ks` channels that hold three taps for nt_order <= 64, and for 128 where ks < 64 (the same order as here); one tap at a time for 128 and ks = 64 (the same only when all
 // channels are in one stage), pairs of taps for 256.  The input gradient is free: nothing that follows depends on its last bit.
-int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int ks) {
+// -1: one tap after the other over all channels, in the kernel for that (APRNET_TAP_KERNEL where the tap kernel is the faster one).
+int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int nt, int ks) {
     if (backward) return kpad % 32 == 0 ? 32 : 16;
     if (nt_order <= 64) return ks;
+    if (nt_order == 128 && ks == 64 && kpad > 64) { int pieces, tiles; return nt == 128 && wide_shape(nt, 1, kpad, &pieces, &tiles) ? -1 : 0; }
     return nt_order == 128 && (ks < 64 || kpad == ks) ? ks : 0;
 }
 
@@ -375,6 +611,22 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (order < 0) {
+        // Microseconds of a wave of tiles for 128 source channels, and before the first one, of this kernel with two and with one block of 128 rows per tile and of the tap kernel,
+        // as fitted to 128 -> 128 layers: 553 k locations 455, 538, 522; 170 k 158, 177, 186; 61 k 80, 85, 83; 33 k 55, 53, 49; 32 k (fewer tiles of two than SMs) -, 39, 49.
+        // Result tiles narrower than 128 (few locations) are 10 to 15 % faster in the tap kernel: 9 k locations 42 against 37.
+        ll t2 = 0, t1 = 0, taps = 0;
+        for (int i = 0; i < P.n_segs; ++i) {
+            const ll slots_ = P.slot_end[i] - P.slot_begin[i];
+            t2 += aprnet_ceil_div(slots_, 254); t1 += aprnet_ceil_div(slots_, 126); taps += aprnet_ceil_div(P.hi[i] - P.lo[i], 128);
+        }
+        const double k = kpad / 128.0;
+        auto time = [&](ll tiles, double wave, double start) { return (double) ((tiles + sms - 1) / sms) * wave * k + start; };
+        int pieces, wtiles;
+        const double two = wide_shape(nt, 2, kpad, &pieces, &wtiles) ? time(t2, 27.0, 3.0) : 1e30, one = time(t1, 15.8, 7.0);
+        if (nt != 128 || std::min(one, two) > time(taps, 17.4, 14.0)) return APRNET_TAP_KERNEL;
+        return two < one ? launch_wide<128, 2>(P, sms, st, pname) : launch_wide<128, 1>(P, sms, st, pname);
+    }
     // channels per stage: whole 128-byte rows where the width allows (64 -> 64: 0.25 instead of 0.29 ms with 32)
     const int kuse = kpad == 48 && order == 16 ? 48 : (kpad % 64 == 0 && order >= 32 ? 64 : order), ks = kuse == 48 ? 64 : kuse;
     const int h = pick_h(P, nt, ks, kuse, nt >= 64 ? 2 : (ks == 16 ? 8 : 4), sms);

@@ -70,6 +70,33 @@ def test_run_kernels_of_padded_and_wide_layers(cin, cout):
         assert float((got[1] - want[1]).norm() / want[1].norm()) <= 2e-6, dl
 
 
+@pytest.mark.parametrize("cin,cout", [(128, 128), (113, 65), (192, 100), (256, 128), (320, 72), (448, 128), (1024, 70)])
+@pytest.mark.parametrize("name", ["odd", "volume", "large"])
+def test_wide_forward_layers_keep_their_order(name, cin, cout):
+    """Forward layers whose taps run one after the other over all source channels: tiles of one and two blocks of rows, up to
+    the widths whose rows no longer fit, and structures that stay with the tap kernel; bit for bit what the kernel that gathers every tap gives."""
+    import pyapr
+    from pyapr.aprnet import cuda as ops
+    from _pyaprwrapper.aprnet import cuda as C
+    a = H.arrays(name) if name == "odd" else H.blob_arrays((64, 128, 128), 40, 11) if name == "volume" else H.blob_arrays((128, 128, 160), 200, 3)
+    apr = pyapr.apr_from_arrays(a)
+    apr.init_cuda()
+    torch.manual_seed(2)
+    conv = ops.APRConv(cin, cout, nstencils=3, precision="bf16").cuda()
+    for dl in (0, 1): 
+        n = int(pyapr.aprnet.utils.number_particles(apr, dl))
+        x, ld = torch.randn(1, cin, n, device="cuda"), torch.full((1,), dl, dtype=torch.int32)
+        with torch.no_grad():
+            try:
+                C.tc_set_option("runs", 0)
+                want = conv(x, [apr], ld)
+            finally:
+                C.tc_set_option("runs", 1)
+            got = conv(x, [apr], ld)
+        assert C.tc_error_flag() == 0
+        assert torch.equal(got, want), (dl, int((got != want).sum()))
+
+
 # widths with one stage per chunk of slots (more than 64 output channels, the last neighbour group of wide inputs) and with several
 DW_WIDTHS = [(8, 8), (16, 40), (33, 33), (64, 32), (24, 120), (32, 128), (128, 64), (128, 128), (130, 32), (48, 200)]
 
