@@ -258,7 +258,8 @@ static std::vector<torch::Tensor> conv333_forward_rows(std::vector<APR*>& aprs, 
 
 // float32 backward from the packed rows (B, bytes): {grad_input or undefined, grad_weights, grad_tree}
 static std::vector<torch::Tensor> conv333_backward_rows(std::vector<APR*>& aprs, const torch::Tensor& rows, const torch::Tensor& weights, const torch::Tensor& grad_output,
-                                                        const torch::Tensor& level_delta, int mode, bool need_grad_input, bool fold_tree, int64_t ld_tree = 0) {
+                                                        const torch::Tensor& level_delta, int mode, bool need_grad_input, bool fold_tree, int64_t ld_tree = 0,
+                                                        torch::Tensor* grad_bias = nullptr) {
     const Batch B(aprs, grad_output, level_delta);
     TORCH_CHECK(grad_output.size(1) == weights.size(1) && grad_output.scalar_type() == torch::kFloat32, "grad_output shape does not match");
     const int cin = (int) weights.size(2), cout = (int) weights.size(1), slots = (int) weights.size(0);
@@ -276,6 +277,18 @@ static std::vector<torch::Tensor> conv333_backward_rows(std::vector<APR*>& aprs,
     auto grad_weights = nb > 0 ? torch::empty_like(weights) : torch::zeros_like(weights);
     auto ws = bytes_like(bytes, grad_output);
     auto partial = torch::empty({aprnet_conv333_rows_partial_elems(mode, cin, cout)}, grad_output.options());
+    if (grad_bias) {
+        // taken along over the particles of one item (entries behind them would count, too); a sum of its own otherwise
+        if (mode == APRNET_PREC_BF16 && cin > 4 && nb == 1 && B.n[0] == n && fold_tree) {
+            *grad_bias = torch::empty({cout}, grad_output.options());
+            const int rc = aprnet_conv333_rows_backward_bias(B.h[0], B.dl[0], cin, cout, slots, row(rows, 0), (const float*) row(grad_output, 0), n, weights.data_ptr<float>(),
+                                                             need_grad_input ? (float*) row(grad_input, 0) : nullptr, n, grad_weights.data_ptr<float>(),
+                                                             need_grad_input ? (float*) row(grad_tree, 0) : nullptr, ld_tree, grad_bias->data_ptr<float>(), partial.data_ptr<float>(),
+                                                             ws.data_ptr(), stream_of(grad_output));
+            if (rc != APRNET_ERR_UNSUPPORTED) { check(rc, "conv333_backward (tensor cores)"); return {grad_input, grad_weights, grad_tree}; }
+        }
+        *grad_bias = grad_output.sum(at::IntArrayRef{0, 2});
+    }
     for (int64_t b = 0; b < nb; ++b)
         check(aprnet_conv333_rows_backward(B.h[b], B.dl[b], mode, cin, cout, slots, row(rows, b), (const float*) row(grad_output, b), n, weights.data_ptr<float>(),
                                            need_grad_input ? (float*) row(grad_input, b) : nullptr, n, grad_weights.data_ptr<float>(), b > 0 ? 1 : 0,
@@ -424,6 +437,16 @@ std::vector<torch::Tensor> conv333_backward_with_rows(std::vector<APR*>& aprs, t
     c10::cuda::CUDAGuard guard(grad_output.device());
     auto r = conv333_backward_rows(aprs, rows, weights, grad_output, level_delta, resolve_mode(precision), need_grad_input, true);
     return {r[0], r[1]};
+}
+
+// the same and the gradient of a bias: the sum of grad_output over batch and particle axis
+std::vector<torch::Tensor> conv333_backward_with_rows_bias(std::vector<APR*>& aprs, torch::Tensor rows, torch::Tensor weights, torch::Tensor grad_output,
+                                                           torch::Tensor level_delta, bool need_grad_input, const std::string& precision) {
+    CHECK_INPUT(weights); CHECK_INPUT(grad_output); CHECK_INPUT(rows);
+    c10::cuda::CUDAGuard guard(grad_output.device());
+    torch::Tensor grad_bias;
+    auto r = conv333_backward_rows(aprs, rows, weights, grad_output, level_delta, resolve_mode(precision), need_grad_input, true, 0, &grad_bias);
+    return {r[0], r[1], grad_bias};
 }
 
 static std::vector<torch::Tensor> conv333_backward_impl(std::vector<APR*>& aprs, torch::Tensor input, torch::Tensor weights,
@@ -1080,6 +1103,7 @@ PYBIND11_MODULE(_pyaprwrapper, m) {
              "precision"_a = "");
     cuda.def("conv333_forward_keep_rows", &conv333_forward_keep_rows, "aprs"_a, "input"_a, "weights"_a, "level_delta"_a, "precision"_a = "bf16", "bias"_a = py::none(), "keep"_a = true);
     cuda.def("conv333_backward_with_rows", &conv333_backward_with_rows, "aprs"_a, "rows"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "need_grad_input"_a = true, "precision"_a = "bf16");
+    cuda.def("conv333_backward_with_rows_bias", &conv333_backward_with_rows_bias, "aprs"_a, "rows"_a, "weights"_a, "grad_output"_a, "level_delta"_a, "need_grad_input"_a = true, "precision"_a = "bf16");
     cuda.def("upsample_const_forward", &upsample_const_forward, "aprs"_a, "input"_a, "level_delta"_a);
     cuda.def("upsample_const_backward", &upsample_const_backward, "aprs"_a, "grad_output"_a, "level_delta"_a);
     cuda.def("reconstruct_forward", &reconstruct_forward, "aprs"_a, "input"_a, "level_delta"_a);

@@ -14,6 +14,8 @@ typedef long long ll;
 
 int aprnet_tc_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st);
 int aprnet_tc_pack_rows_pair(const float* x0, ll ld0, int c0, const float* x1, ll ld1, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st);
+int aprnet_tc_pack_rows_sums(const float* x, ll ld_x, ll n, int c, int cpad, void* out, double* sums, float* sums_out, cudaStream_t st);
+size_t aprnet_tc_pack_sums_bytes(int c);
 int aprnet_f32_pack_pair(const aprnet_apr* a, int dl, int cin, const float* in0, ll ld0, int c0, const float* in1, ll ld1, const float* tree, ll ld_tree, void* rows, cudaStream_t st);
 int aprnet_fill_tree_mean_pair(const aprnet_apr* a, int dl, int C, const float* in0, ll ld0, int c0, const float* in1, ll ld1, float* tree, ll ld_tree, cudaStream_t st);
 int aprnet_tc_gather_conv(aprnet_apr* a, int dl, int backward, int cin, int cout, int slots, const void* rows, int kpad,
@@ -56,7 +58,7 @@ int forward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int sl
 
 // `ws`: grad_bytes() bytes.  gout == null: `ws` starts with the packed rows of grad_output already (bf16, Cin > 4).  gin == null: no input gradient; gw == null: no weight gradient; fold_tree: grad_tree is folded into gin
 int backward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int slots, const void* rows, const float* gout, ll ld_out, const float* w,
-                  float* gin, ll ld_in, float* gw, int accumulate, float* gtree, ll ld_tree, float* partial, void* ws, bool fold_tree, cudaStream_t st) {
+                  float* gin, ll ld_in, float* gw, int accumulate, float* gtree, ll ld_tree, float* partial, void* ws, bool fold_tree, cudaStream_t st, float* gbias = nullptr) {
     APRNET_ARG_CHECK(a && a->valid_dl(dl) && cin > 0 && cout > 0 && slots > 0 && (gout || (is_bf16(precision) && !aprnet_small_cin(cin) && 27 * a->number_parts(dl) + 1 < (1ll << 31))) && (gin || gw) && (!gin || (w && gtree)) && ws && (!gw || (rows && partial)), "bad argument");
     APRNET_DEVICE_CHECK(a);
     APRNET_ARG_CHECK(ld_out >= a->number_parts(dl) && (!gin || (ld_in >= a->number_parts(dl) && ld_tree >= a->tree_size(dl))), "leading dimension too small");
@@ -66,7 +68,9 @@ int backward_rows(aprnet_apr* a, int dl, int precision, int cin, int cout, int s
     int rc;
     // the weight gradient of a first layer reads grad_output itself
     if (gout && (gin || !aprnet_small_cin(cin))) {
-        rc = bf16 ? aprnet_tc_pack_rows(gout, ld_out, n, nullptr, 0, 0, cout, gpad, ws, st) : aprnet_f32_pack_grad(a, dl, cout, gout, ld_out, ws, st);
+        // (the sums' buffer is the weight gradient's, which comes afterwards)
+        rc = gbias ? aprnet_tc_pack_rows_sums(gout, ld_out, n, cout, gpad, ws, (double*) partial, gbias, st)
+           : bf16 ? aprnet_tc_pack_rows(gout, ld_out, n, nullptr, 0, 0, cout, gpad, ws, st) : aprnet_f32_pack_grad(a, dl, cout, gout, ld_out, ws, st);
         if (rc) return rc;
     }
     if (gw) {
@@ -157,6 +161,15 @@ extern "C" int aprnet_conv333_rows_backward(aprnet_apr* a, int dl, int precision
     APRNET_ARG_CHECK(precision_ok(precision), "unknown precision");
     APRNET_ARG_CHECK(gout, "bad argument");
     return backward_rows(a, dl, precision, cin, cout, slots, rows, gout, ld_out, w, gin, ld_in, gw, accumulate, gtree, ld_tree, partial, workspace, fold_tree != 0, (cudaStream_t) stream);
+}
+
+// The backward pass in bf16 arithmetic (cin > 4) with the sums of grad_output over the structure's locations, the gradient of a bias, in grad_bias (cout): taken along where
+// grad_output is packed.  partial: aligned to 8 bytes
+extern "C" int aprnet_conv333_rows_backward_bias(aprnet_apr* a, int dl, int cin, int cout, int slots, const void* rows, const float* gout, int64_t ld_out, const float* w,
+                                                 float* gin, int64_t ld_in, float* gw, float* gtree, int64_t ld_tree, float* gbias, float* partial, void* workspace, void* stream) {
+    APRNET_ARG_CHECK(gout && gw && gbias && partial && (reinterpret_cast<uintptr_t>(partial) & 7) == 0 && cin > 0 && !aprnet_small_cin(cin) && cout > 0, "bad argument");
+    if (aprnet_tc_pack_sums_bytes(cout) > (size_t) aprnet_conv333_tc_dw_partial_elems(cin, cout) * sizeof(float)) { aprnet_set_error("%s: the weight gradient's buffer is too small for the sums", __func__); return APRNET_ERR_UNSUPPORTED; }
+    return backward_rows(a, dl, APRNET_PREC_BF16, cin, cout, slots, rows, gout, ld_out, w, gin, ld_in, gw, 0, gtree, ld_tree, partial, workspace, true, (cudaStream_t) stream, gbias);
 }
 
 // ---- the tensor-core entry points ------------------------------------------------------------------------

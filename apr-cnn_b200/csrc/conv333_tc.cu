@@ -65,8 +65,12 @@ template<int KS> __device__ __forceinline__ int swizzled_chunk(int row, int c) {
 // pieces (8 channels) of the packed rows, and the next tile's loads are in flight while a tile is stored.
 // The 13 layers of a training step on 3.5 M locations: 1.79 ms with a tile per block and a condition per load, now 1.50; a batch of four in inference 2.05 -> 1.75.
 constexpr int PACK_BLOCKS = 4;          // blocks per SM
+// SUMS: the sums of x over its rows are taken along (the gradient of a bias, from the gradient that is packed): four values of a tile in fp32, then in double precision, the
+// warps' sums in sums[block][channel], which channel_sums_kernel adds in order (a pass of its own over 1.2 M rows of 33 channels took
+// 57 us, the packing with sums and their addition 7 us more than without).
+template<bool SUMS>
 __global__ void __launch_bounds__(256, PACK_BLOCKS) pack_rows_bf16_kernel(const float* __restrict__ x, ll ld_x, int split, const float* __restrict__ x1, ll ld_x1, ll n,
-                                                            const float* __restrict__ tree, ll ld_tree, ll t, int c, int cpad, __nv_bfloat16* __restrict__ out) {
+                                                            const float* __restrict__ tree, ll ld_tree, ll t, int c, int cpad, __nv_bfloat16* __restrict__ out, double* __restrict__ sums) {
     __shared__ float tile[2][32][129];
     const int c0 = blockIdx.y * 32;
     const ll rows = n + t + 1, tiles = (rows + 127) / 128;
@@ -94,11 +98,14 @@ __global__ void __launch_bounds__(256, PACK_BLOCKS) pack_rows_bf16_kernel(const 
     };
     request((ll) blockIdx.x * 128);
     int buf = 0;
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
     for (ll i = blockIdx.x; i < tiles; i += gridDim.x, buf ^= 1) {
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc)
+        for (int cc = 0; cc < 4; ++cc) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) tile[buf][wrp + 8 * cc][lane + 32 * k] = v[cc][k];
+            if (SUMS) sum[cc] += (double) ((v[cc][0] + v[cc][1]) + (v[cc][2] + v[cc][3]));       // (entries behind the rows are zeros)
+        }
         __syncthreads();                                            // (the other buffer is written after the next one)
         if (i + gridDim.x < tiles) request((i + gridDim.x) * 128);
         // 128 rows x 4 pieces of 8 channels; consecutive threads take consecutive pieces of a row
@@ -113,6 +120,31 @@ __global__ void __launch_bounds__(256, PACK_BLOCKS) pack_rows_bf16_kernel(const 
                 *reinterpret_cast<uint4*>(out + r * cpad + c0 + piece * 8) = *reinterpret_cast<uint4*>(h);
             }
         }
+    }
+    if (SUMS) {
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum[cc] += __shfl_xor_sync(0xffffffffu, sum[cc], o);
+            const int ch = c0 + wrp + 8 * cc;
+            if (lane == 0 && ch < c) sums[(ll) blockIdx.x * c + ch] = sum[cc];
+        }
+    }
+}
+
+// out[ch] = the blocks' sums of the channel, added in a fixed order: a block has 32 channels, warp w takes every eighth block's
+__global__ void __launch_bounds__(256) channel_sums_kernel(const double* __restrict__ sums, int blocks, int c, float* __restrict__ out) {
+    __shared__ double part[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ch = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (ch < c)
+#pragma unroll 8
+        for (int b = w; b < blocks; b += 8) s += sums[(ll) b * c + ch];
+    part[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && ch < c) {
+        for (int k = 1; k < 8; ++k) s += part[k][lane];
+        out[ch] = (float) s;
     }
 }
 
@@ -636,12 +668,15 @@ int dispatch_tc(const TcParams& P, const TcGeom& g, int total_tiles, cudaStream_
     return APRNET_ERR_UNSUPPORTED;
 }
 
-int run_pack_rows(const float* x, ll ld_x, int split, const float* x1, ll ld_x1, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, __nv_bfloat16* out, cudaStream_t st) {
+int run_pack_rows(const float* x, ll ld_x, int split, const float* x1, ll ld_x1, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, __nv_bfloat16* out, cudaStream_t st,
+                  double* sums = nullptr, float* sums_out = nullptr) {
     const int gy = aprnet_ceil_div(cpad, 32);
     const dim3 grid((unsigned) std::min<ll>(aprnet_ceil_div(n + t + 1, 128), aprnet_ceil_div(148 * PACK_BLOCKS, gy)), (unsigned) gy);
     { AprnetProfScope _prof("pack_rows_bf16", st);
-    pack_rows_bf16_kernel<<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, cpad, out);
+    if (sums) pack_rows_bf16_kernel<true><<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, cpad, out, sums);
+    else pack_rows_bf16_kernel<false><<<grid, 256, 0, st>>>(x, ld_x, split, x1, ld_x1, n, tree, ld_tree, t, c, cpad, out, nullptr);
     }
+    if (sums) channel_sums_kernel<<<(unsigned) aprnet_ceil_div(c, 32), 256, 0, st>>>(sums, (int) grid.x, c, sums_out);
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }
@@ -653,6 +688,12 @@ int* aprnet_tc_error_flag_device() { return ensure_error_flag() == APRNET_OK ? g
 int aprnet_tc_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st) {
     return run_pack_rows(x, ld_x, c, x, ld_x, n, tree, ld_tree, t, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st);
 }
+
+// rows of grad_output, and its sums over them in sums_out (c); sums: aprnet_tc_pack_sums_bytes(c)
+int aprnet_tc_pack_rows_sums(const float* x, ll ld_x, ll n, int c, int cpad, void* out, double* sums, float* sums_out, cudaStream_t st) {
+    return run_pack_rows(x, ld_x, c, x, ld_x, n, nullptr, 0, 0, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st, sums, sums_out);
+}
+size_t aprnet_tc_pack_sums_bytes(int c) { return (size_t) 148 * PACK_BLOCKS * c * sizeof(double); }
 
 // the same for the concatenation of two tensors of c0 and c - c0 channels
 int aprnet_tc_pack_rows_pair(const float* x0, ll ld0, int c0, const float* x1, ll ld1, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st) {

@@ -12,7 +12,8 @@ from torch.autograd import Function
 from torch.nn import init
 
 from _pyaprwrapper.data_containers import APRPtrVector
-from _pyaprwrapper.aprnet.cuda import (conv111_backward, conv111_backward_with_bias, conv111_forward, conv333_backward_with_rows, conv333_backward_with_tree,
+from _pyaprwrapper.aprnet.cuda import (conv111_backward, conv111_backward_with_bias, conv111_forward, conv333_backward_with_rows,
+                                       conv333_backward_with_rows_bias, conv333_backward_with_tree,
                                        conv333_forward_keep_rows, conv333_forward_keep_tree, get_conv_precision,
                                        restrict_kernel333_backward, restrict_kernel333_forward)
 
@@ -60,11 +61,10 @@ class Conv333Function(Function):
         grad_output = grad_output.contiguous()
         if ctx.packed:
             expanded, bias, level_deltas, rows = ctx.saved_tensors
-            grad_input, grad_expanded = conv333_backward_with_rows(APRPtrVector(ctx.aprs), rows, expanded, grad_output, level_deltas,
-                                                                   bool(ctx.needs_input_grad[0]), ctx.precision)
+            backward = conv333_backward_with_rows if bias is None else conv333_backward_with_rows_bias
+            grad_input, grad_expanded, *grad_bias = backward(APRPtrVector(ctx.aprs), rows, expanded, grad_output, level_deltas, bool(ctx.needs_input_grad[0]), ctx.precision)
             grad_weights = restrict_kernel333_backward(grad_expanded, ctx.num_stencils)
-            grad_bias = grad_output.sum(dim=(0, 2)) if bias is not None else None
-            return grad_input, grad_weights, grad_bias, None, None, None, None
+            return grad_input, grad_weights, grad_bias[0] if grad_bias else None, None, None, None, None
         inputs, expanded, bias, level_deltas, tree = ctx.saved_tensors
         grad_input, grad_expanded = conv333_backward_with_tree(APRPtrVector(ctx.aprs), inputs, expanded, grad_output, level_deltas, tree)
         grad_weights = restrict_kernel333_backward(grad_expanded, ctx.num_stencils)

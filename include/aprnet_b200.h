@@ -194,6 +194,13 @@ int aprnet_conv333_rows_backward(aprnet_apr* apr, int level_delta, int precision
                                  const void* packed_rows, const float* grad_output, int64_t ld_out, const float* weights,
                                  float* grad_input, int64_t ld_in, float* grad_weights, int accumulate, float* grad_tree,
                                  int64_t ld_tree, int fold_tree, float* partial, void* workspace, void* stream);
+/* The same in bf16 arithmetic (cin > 4), grad_weights written and the tree gradient folded into grad_input, with the sums of grad_output over the
+ * structure's locations in grad_bias (cout).  partial: aligned to 8 bytes.  APRNET_ERR_UNSUPPORTED where it is too small for the sums (very many
+ * channels): take them apart then. */
+int aprnet_conv333_rows_backward_bias(aprnet_apr* apr, int level_delta, int cin, int cout, int num_slots, const void* packed_rows,
+                                      const float* grad_output, int64_t ld_out, const float* weights, float* grad_input, int64_t ld_in,
+                                      float* grad_weights, float* grad_tree, int64_t ld_tree, float* grad_bias, float* partial,
+                                      void* workspace, void* stream);
 /* GroupNorm + ReLU and the 3x3x3 convolution in front of it, backward in one call: one batch item, float32 tensors, bf16 arithmetic, cin > 4.
  * conv_out (cout, n): output of the convolution, mean / rstd (groups) its statistics, grad_y (cout, n) the gradient behind the ReLU.  Same results as
  * aprnet_groupnorm_relu_backward followed by aprnet_conv333_rows_backward (grad_weights written, tree gradient folded into grad_input), without the

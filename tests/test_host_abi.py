@@ -57,6 +57,7 @@ CALLS = {
     "aprnet_conv333_rows_forward_pair": (i(0), i(1), i(8), i(8), i(1), p, n, i(4), p, n, p, None, p, n, p, n, p, None),
     "aprnet_conv333_rows_pack": (i(0), i(1), i(8), p, n, p, n, i(1), p, None),
     "aprnet_conv333_rows_backward": (i(0), i(1), i(8), i(8), i(1), p, p, n, p, p, n, p, i(0), p, n, i(1), p, p, None),
+    "aprnet_conv333_rows_backward_bias": (i(0), i(8), i(8), i(1), p, p, n, p, p, n, p, p, n, p, p, p, None),
     "aprnet_conv333_forward_tc": (i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, p, None),
     "aprnet_conv333_forward_tc_pretree": (i(0), i(8), i(8), i(1), p, n, p, p, n, p, n, p, None),
     "aprnet_conv333_backward_tc": (i(0), i(8), i(8), i(1), p, n, p, n, p, p, p, p, i(1), p, n, p, p, None),
