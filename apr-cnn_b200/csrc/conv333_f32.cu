@@ -127,8 +127,9 @@ struct F32Params {
 
 enum { FORWARD, SAME_LEVEL, TARGETS };        // forward pass, the two parts of the input gradient
 
-// Block = 128 * WM locations x NT = TN * WN output channels, WM x WN warps; a thread owns the locations lane + 32 i (i < 4) of its
-// warp's 128 and TN channels.  A ring slot holds 16 channels of the tile's rows for one tap and the matching weights; 16-byte
+// Block = 32 * R * WM locations x NT = TN * WN output channels, WM x WN warps; a thread owns the locations lane + 32 i (i < R) of its
+// warp's 32 R and TN channels.  R = 4 where the blocks fill the chip; few blocks are a serial chain of slots each, and with R = 1 a slot takes a quarter of the
+// multiply-adds and four times the blocks share the work: gathers of 64-wide tiles in a training step on 9.7 k locations 7.3 -> 4.2 ms.  Each result is the same chain.  A ring slot holds 16 channels of the tile's rows for one tap and the matching weights; 16-byte
 // pieces of a row are exchanged so that eight consecutive rows read at the same channel fall on different banks.  Table
 // entries are requested one tap ahead of the copies that need them.
 //
@@ -144,14 +145,14 @@ enum { FORWARD, SAME_LEVEL, TARGETS };        // forward pass, the two parts of 
 // Threads per SM and ring slots.  16 warps of 128 registers instead of 12 of 168 give little, because the register file bounds the loop (paired multiply-adds read
 // four registers a cycle): input gradient of 32 channels 4.94 -> 4.56 ms (32 -> 32, 3.5 M locations, three slots), forward pass of 64 9.01 -> 8.90 ms (64 -> 64 at level
 // delta 1), weight gradient of 16 x 32 tiles 8.16 -> 7.98 (33 -> 24); the other shapes lose 1 to 14 %.
-template<int WM, int TN, int MODE> struct GatherShape {
-    static constexpr bool MORE = TN == 16 && ((MODE == FORWARD && WM == 1) || (MODE == SAME_LEVEL && WM == 2));
-    static constexpr int THREADS = MORE ? 512 : 384, RING = MORE && WM == 2 ? 3 : 4;
+template<int WM, int TN, int R, int MODE> struct GatherShape {
+    static constexpr bool MORE = R == 4 && TN == 16 && ((MODE == FORWARD && WM == 1) || (MODE == SAME_LEVEL && WM == 2));
+    static constexpr int THREADS = R == 1 ? 768 : (MORE ? 512 : 384), RING = MORE && WM == 2 ? 3 : 4;
 };
-template<int WM, int WN, int TN, int MODE>
-__global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, MODE>::THREADS / (32 * WM * WN)) conv333_f32_gather_kernel(const F32Params P) {
-    constexpr int RING = GatherShape<WM, TN, MODE>::RING;
-    constexpr int T = 32 * WM * WN, M = 128 * WM, NT = TN * WN;
+template<int WM, int WN, int TN, int R, int MODE>
+__global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, R, MODE>::THREADS / (32 * WM * WN)) conv333_f32_gather_kernel(const F32Params P) {
+    constexpr int RING = GatherShape<WM, TN, R, MODE>::RING;
+    constexpr int T = 32 * WM * WN, M = 32 * R * WM, NT = TN * WN;
     constexpr bool KMAJOR = MODE == FORWARD, ZEROS = MODE == TARGETS || (MODE == SAME_LEVEL && NT < 64);
     constexpr int RPT = M * (KS / 4) / T;          // row pieces a thread copies per slot
     constexpr int RSTEP = T / (KS / 4);            // distance of their rows
@@ -223,16 +224,16 @@ __global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, MODE>::THREA
         if (++islot == RING) islot = 0;
     };
 
-    unsigned long long acc[4][TN / 2];             // pairs of output channels
+    unsigned long long acc[R][TN / 2];             // pairs of output channels
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int n = 0; n < TN / 2; ++n) acc[i][n] = 0ull;
 
     request(itap);
 #pragma unroll
     for (int s = 0; s < RING - 1; ++s) { issue(); cp_async_commit(); }
-    const int sw = (lane >> 1) & 3, arow = (wm * 128 + lane) * KS, n_off = wn * TN;
+    const int sw = (lane >> 1) & 3, arow = (wm * 32 * R + lane) * KS, n_off = wn * TN;
     int slot = 0, kc = 0;
     for (int s = 0; s < total; ++s) {
         cp_async_wait<RING - 2>();
@@ -242,15 +243,15 @@ __global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, MODE>::THREA
         const float* a_s = ring + slot * SLOT + arow;
         const float* b_s = ring + slot * SLOT + A_ELEMS + n_off;
         auto quad = [&](int q) {                   // four channels
-            float4 a[4];
+            float4 a[R];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(a_s + i * 32 * KS + ((q ^ sw) << 2));
+            for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4*>(a_s + i * 32 * KS + ((q ^ sw) << 2));
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 const float* bk = b_s + (q * 4 + kk) * NT;
-                unsigned long long a2[4];
+                unsigned long long a2[R];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < R; ++i) {
                     const float av = kk == 0 ? a[i].x : (kk == 1 ? a[i].y : (kk == 2 ? a[i].z : a[i].w));
                     a2[i] = pack2(av, av);
                 }
@@ -258,9 +259,9 @@ __global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, MODE>::THREA
                 for (int h = 0; h < TN / 4; ++h) {
                     const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(bk + h * 4);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) fma2(acc[i][2 * h], a2[i], b.x);
+                    for (int i = 0; i < R; ++i) fma2(acc[i][2 * h], a2[i], b.x);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) fma2(acc[i][2 * h + 1], a2[i], b.y);
+                    for (int i = 0; i < R; ++i) fma2(acc[i][2 * h + 1], a2[i], b.y);
                 }
             }
         };
@@ -277,8 +278,8 @@ __global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, MODE>::THREA
     cp_async_wait<0>();
 
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const ll p = p0 + wm * 128 + lane + i * 32;
+    for (int i = 0; i < R; ++i) {
+        const ll p = p0 + wm * 32 * R + lane + i * 32;
         if (p >= hi) continue;
         float* dst = P.out + p;
         ll ld = P.ld_out;
@@ -579,11 +580,11 @@ int run_pack_weights(const aprnet_apr* a, int dl, const float* w, int slots, int
     return aprnet_pack_weights(a, dl, false, w, slots, cin, cout, transposed, nt, (n_dim + nt - 1) / nt, pad4(transposed ? cout : cin), wp, st);
 }
 
-template<int WM, int WN, int TN, int MODE>
+template<int WM, int WN, int TN, int R, int MODE>
 int launch_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
-    constexpr int M = 128 * WM, NT = TN * WN;
-    constexpr size_t smem = (size_t) GatherShape<WM, TN, MODE>::RING * (M + NT) * KS * sizeof(float);
-    auto kern = conv333_f32_gather_kernel<WM, WN, TN, MODE>;
+    constexpr int M = 32 * R * WM, NT = TN * WN;
+    constexpr size_t smem = (size_t) GatherShape<WM, TN, R, MODE>::RING * (M + NT) * KS * sizeof(float);
+    auto kern = conv333_f32_gather_kernel<WM, WN, TN, R, MODE>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     P.segs = make_seg_table(segs, M);
     P.n_tiles = (P.n_dim + NT - 1) / NT;
@@ -595,13 +596,24 @@ int launch_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t s
     return APRNET_OK;
 }
 
+// One location per lane where four leave SMs without a block: training steps on 9.7 k, 26 k and 106 k locations 10.7 -> 7.5, 12.0 -> 9.8 and 19.1 -> 18.0 ms.  With the line at 222 or
+// 320 blocks 106 k take 18.7 ms, 68 k (at 320) 15.3 instead of 14.2.
+constexpr int FEW_BLOCKS = 148;
+template<int WM, int WN, int TN, int MODE>
+int launch_tiles(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
+    ll blocks = 0;
+    for (const Segment& s : segs) blocks += aprnet_ceil_div(s.end - s.begin, 128 * WM);
+    blocks *= (P.n_dim + TN * WN - 1) / (TN * WN);
+    return blocks <= FEW_BLOCKS ? launch_gather<WM, WN, TN, 1, MODE>(P, segs, st, pname) : launch_gather<WM, WN, TN, 4, MODE>(P, segs, st, pname);
+}
+
 template<int MODE>
 int run_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
     switch (pick_nt(P.n_dim)) {
-        case 64: return launch_gather<1, 4, 16, MODE>(P, segs, st, pname);
-        case 32: return launch_gather<2, 2, 16, MODE>(P, segs, st, pname);
-        case 16: return launch_gather<2, 2, 8, MODE>(P, segs, st, pname);
-        default: return launch_gather<2, 2, 4, MODE>(P, segs, st, pname);
+        case 64: return launch_tiles<1, 4, 16, MODE>(P, segs, st, pname);
+        case 32: return launch_tiles<2, 2, 16, MODE>(P, segs, st, pname);
+        case 16: return launch_tiles<2, 2, 8, MODE>(P, segs, st, pname);
+        default: return launch_tiles<2, 2, 4, MODE>(P, segs, st, pname);
     }
 }
 
