@@ -133,6 +133,25 @@ int aprnet_check_device(const aprnet_apr* a);      // APRNET_OK when the current
 
 #define APRNET_LAUNCH_CHECK() APRNET_CUDA_CHECK(cudaGetLastError())
 
+// Chains of short kernels: a kernel launched with `behind` starts while the launch before it on the stream still runs, once all blocks of that one have started and called
+// let_next_grid_start() or have ended.  Up to wait_for_grid_before() it may only read what was there before the chain's first launch, which is an ordinary one: tables and
+// inputs, not what the chain writes; it writes nothing up to there.  Every block of such a kernel waits, so that the end of one launch is the end of all before it.
+// (Reads behind the wait go through pointers without __restrict__: loads of what the compiler takes for constant are free to move.)
+template<typename... P, typename... A>
+inline void aprnet_launch(bool behind, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.attrs = &attr; cfg.numAttrs = behind ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);             // (an error stays for APRNET_LAUNCH_CHECK)
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void let_next_grid_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_grid_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 #define APRNET_ARG_CHECK(cond, msg)                                                                 \
     do { if (!(cond)) { aprnet_set_error("%s: %s", __func__, msg); return APRNET_ERR_ARG; } } while (0)
 

@@ -24,13 +24,16 @@ template<> struct DT<double> { static constexpr int id = APRNET_F64; };
 // One tree level: node t = scale[t] * sum(children) (MAX: their maximum).  A thread owns a node and CH channels; the
 // block's channel group is the fast grid axis, so that the groups of the same nodes run together and find the 36-byte
 // table entries of a node in L2.  All CH x 8 child values are requested before any is used.
-template<typename T, int CH, bool MAX>
+// The levels are a chain of short launches, each of which reads what the one before wrote: a launch starts behind the running one and has its table entries when that one
+// ends (8 channels on 256 x 512 x 512, mean and maximum of all levels: 122 -> 104 us; one launch after the other, each began with a gap and the latency of the table).
+template<typename T, int CH, bool MAX, bool BEHIND = false>
 __device__ __forceinline__ void tree_node(const int32_t* __restrict__ child, const float* __restrict__ scale, ll n_tree, ll t,
                                           const T* __restrict__ in, ll ld_in, T* tree, ll ld_tree, int c0, int nch, ll up_off, int use_up) {
     int32_t v[8];
 #pragma unroll
     for (int s = 0; s < 8; ++s) v[s] = __ldg(child + (ll) s * n_tree + t);
     const T f = MAX ? T(1) : (T) __ldg(scale + t);
+    if (BEHIND) wait_for_grid_before();         // for the finer level's nodes
     const T* xin = in + (ll) c0 * ld_in;
     const T* xtree = use_up ? xin + up_off : tree + (ll) c0 * ld_tree;     // coded children: upgraded nodes in the features, else the tree scratch
     const ll ld_coded = use_up ? ld_in : ld_tree;
@@ -84,7 +87,8 @@ __global__ void __launch_bounds__(TPB) tree_level_kernel(const int32_t* __restri
                                                          ll ld_tree, int C, ll up_off, int use_up) {
     const ll t = tb + (ll) blockIdx.y * TPB + threadIdx.x;
     const int c0 = blockIdx.x * CH;
-    if (t < te) tree_node<T, CH, MAX>(child, scale, n_tree, t, in.base(c0), in.ld(c0), tree, ld_tree, c0, min(CH, C - c0), up_off, use_up);
+    let_next_grid_start();
+    if (t < te) tree_node<T, CH, MAX, true>(child, scale, n_tree, t, in.base(c0), in.ld(c0), tree, ld_tree, c0, min(CH, C - c0), up_off, use_up);
 }
 
 // The coarse end of the tree in one launch: a cluster of blocks owns CH channels and walks the levels [0, n) of `lv` (fine to
@@ -103,6 +107,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(COARSE_TPB) tr
                                                                  LevelList lv, const Features<T> in, T* tree, ll ld_tree, int C, ll up_off) {
     const int c0 = (int) (blockIdx.x / CLUSTER) * CH, first = (int) (blockIdx.x % CLUSTER) * COARSE_TPB + threadIdx.x;
     int i = 0;
+    wait_for_grid_before();
     for (; i < lv.n && lv.end[i] - lv.begin[i] > ALONE_NODES; ++i) {
         for (ll t = lv.begin[i] + first; t < lv.end[i]; t += CLUSTER * COARSE_TPB)
             tree_node<T, CH, MAX>(child, scale, n_tree, t, in.base(c0), in.ld(c0), tree, ld_tree, c0, min(CH, C - c0), up_off, lv.use_up[i]);
@@ -121,16 +126,17 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(COARSE_TPB) tr
 // axis is streamed (coalesced read-modify-write, one writer per entry), the parents' values come from a few cache lines
 // per warp.  The parent-centric form (one thread per parent, eight scattered children) touched every sector of the
 // gradient half at a time and ran at half this speed.  dst and gtree may be the same array (node levels): a level only
-// reads the level above it.
-template<typename T>
+// reads the level above it.  A launch starts behind the one before it and has its table entries and the old values by the time the parents are there.
+template<typename T, bool BEHIND = false>
 __device__ __forceinline__ void tree_backward_child(const int32_t* __restrict__ parent, const float* __restrict__ scale, ll u, T* dst, ll ld_dst,
                                                     const T* gtree, ll ld_tree, int c0, int C) {
     T old[CH_PER_BLOCK];
 #pragma unroll
     for (int k = 0; k < CH_PER_BLOCK; ++k) old[k] = dst[(ll) min(c0 + k, C - 1) * ld_dst + u];        // independent of the parent
     const int32_t t = parent[u];
+    const T f = t < 0 ? T(0) : (T) scale[t];
+    if (BEHIND) wait_for_grid_before();         // for the parents' gradients
     if (t < 0) return;
-    const T f = (T) scale[t];
     T g[CH_PER_BLOCK];
 #pragma unroll
     for (int k = 0; k < CH_PER_BLOCK; ++k) g[k] = gtree[(ll) min(c0 + k, C - 1) * ld_tree + t];
@@ -143,7 +149,8 @@ template<typename T>
 __global__ void __launch_bounds__(TPB) tree_mean_backward_children_kernel(const int32_t* __restrict__ parent, const float* __restrict__ scale,
                                                                           ll ub, ll ue, T* dst, ll ld_dst, const T* gtree, ll ld_tree, int C) {
     const ll u = ub + (ll) blockIdx.x * blockDim.x + threadIdx.x;
-    if (u < ue) tree_backward_child<T>(parent, scale, u, dst, ld_dst, gtree, ld_tree, blockIdx.y * CH_PER_BLOCK, C);
+    let_next_grid_start();
+    if (u < ue) tree_backward_child<T, true>(parent, scale, u, dst, ld_dst, gtree, ld_tree, blockIdx.y * CH_PER_BLOCK, C);
 }
 
 // the coarse tree levels of `lv` (coarse to fine) in one launch, a cluster per channel group (see tree_coarse_kernel)
@@ -344,6 +351,7 @@ int fill_tree(const aprnet_apr* a, int dl, int C, const Features<T>& in, T* tree
     LevelList coarse;
     coarse.n = 0;
     const int last = last_coarse_level(m, cml);
+    bool behind = false;
     for (int lp = cml - 1; lp >= m.level_min - 1; --lp) {
         const ll tb = m.tlvl_begin[lp], te = m.tlvl_begin[lp + 1];
         if (te <= tb) continue;
@@ -356,13 +364,14 @@ int fill_tree(const aprnet_apr* a, int dl, int C, const Features<T>& in, T* tree
         for (ll b = tb; b < te; b += 65535ll * TPB) {              // grid.y holds 65535 blocks
             AprnetProfScope _prof(pname, st);
             const ll e = std::min(te, b + 65535ll * TPB);
-            tree_level_kernel<T, CH, MAX><<<dim3(gx, (unsigned) aprnet_ceil_div(e - b, TPB)), TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, b, e, in,
-                                                                                                          tree, ld_tree, C, up, use_up);
+            aprnet_launch(behind, tree_level_kernel<T, CH, MAX>, dim3(gx, (unsigned) aprnet_ceil_div(e - b, TPB)), TPB, 0, st, a->child, a->tree_scale, a->n_tree, b, e, in,
+                          tree, ld_tree, C, up, use_up);
+            behind = true;
         }
     }
     if (coarse.n > 0) {
         AprnetProfScope _prof(pname, st);
-        tree_coarse_kernel<T, CH, MAX><<<gx * CLUSTER, COARSE_TPB, 0, st>>>(a->child, a->tree_scale, a->n_tree, coarse, in, tree, ld_tree, C, up);
+        aprnet_launch(behind, tree_coarse_kernel<T, CH, MAX>, gx * CLUSTER, COARSE_TPB, 0, st, a->child, a->tree_scale, a->n_tree, coarse, in, tree, ld_tree, C, up);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
@@ -386,19 +395,21 @@ int fill_tree_mean_bwd(const aprnet_apr* a, int dl, int C, T* gin, ll ld_in, T* 
         if (m.tlvl_begin[l + 1] > m.tlvl_begin[l]) { coarse.begin[coarse.n] = m.tlvl_begin[l]; coarse.end[coarse.n] = m.tlvl_begin[l + 1]; ++coarse.n; }
     if (coarse.n > 0) {
         AprnetProfScope _prof("tree_mean_bwd", st);
-        tree_mean_backward_coarse_kernel<T><<<(unsigned) aprnet_ceil_div(C, CH_PER_BLOCK) * CLUSTER, COARSE_TPB, 0, st>>>(node_parent, a->tree_scale, coarse, gtree, ld_tree, C);
+        aprnet_launch(false, tree_mean_backward_coarse_kernel<T>, (unsigned) aprnet_ceil_div(C, CH_PER_BLOCK) * CLUSTER, COARSE_TPB, 0, st, node_parent, a->tree_scale, coarse, gtree, ld_tree, C);
     }
+    bool behind = coarse.n > 0;
     for (; l <= cml - 1; ++l) {
         const ll ub = m.tlvl_begin[l], ue = m.tlvl_begin[l + 1];
         if (ue <= ub) continue;
         AprnetProfScope _prof("tree_mean_bwd", st);
-        tree_mean_backward_children_kernel<T><<<node_grid(ue - ub, C), TPB, 0, st>>>(node_parent, a->tree_scale, ub, ue, gtree, ld_tree, gtree, ld_tree, C);
+        aprnet_launch(behind, tree_mean_backward_children_kernel<T>, node_grid(ue - ub, C), TPB, 0, st, node_parent, a->tree_scale, ub, ue, gtree, ld_tree, gtree, ld_tree, C);
+        behind = true;
     }
     // then every feature location (particles of all levels, upgraded nodes) from its parent node
     const ll n = a->number_parts(dl);
     if (n > 0) {
         AprnetProfScope _prof("tree_mean_bwd", st);
-        tree_mean_backward_children_kernel<T><<<node_grid(n, C), TPB, 0, st>>>(loc_parent, a->tree_scale, 0, n, gin, ld_in, gtree, ld_tree, C);
+        aprnet_launch(behind, tree_mean_backward_children_kernel<T>, node_grid(n, C), TPB, 0, st, loc_parent, a->tree_scale, 0, n, gin, ld_in, gtree, ld_tree, C);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
