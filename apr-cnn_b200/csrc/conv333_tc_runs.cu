@@ -1,5 +1,5 @@
 // 3x3x3 particle convolution on the tensor cores over runs of cells (bf16 operands, fp32 accumulation): forward pass of layers with at
-// most 128 result channels (above 64 only where all source channels are in one stage), same-level input gradient of any width.
+// most 128 result channels (above 64 and with several chunks of source channels by a kernel of its own, see there), same-level input gradient of any width.
 //
 // The kernel of conv333_tc.cu gathers every source row once per tap, 27 rows per location.  Here the M dimension of a tile is not
 // 128 locations but 128 * H consecutive slots of the run plan (run_plan.cu).  For each of the 9 rows of cells (dz, dx) the tile's
@@ -7,9 +7,9 @@
 // tap dy starts dy rows further.  (The swizzle of a K-major operand is a function of the shared-memory address, so a start address
 // inside the pattern is an ordinary one.)  That is 9 x 1.07 .. 1.27 gathered rows per location instead of 27; slots without a
 // location are the price, 7 to 27 % more multiply-adds.  Each weight tile that is fetched meets H blocks of 128 rows.
-// What bounds it: no unit is saturated.  Shares of each unit's own peak for 32 -> 32 and 64 -> 64 channels, which overlap: operand reads of the tensor
-// core (l1tex__data_pipe_tc_wavefronts) 59 and 70 %, load-store unit (copies, whose sectors land one by one, shuffles, stores of the results;
-// l1tex__data_pipe_lsu_wavefronts) 52 and 55 %, issue slots 51 and 45 %, tensor pipe 25 and 49 %; the rest is waiting between the roles.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
+// What bounds it: operand reads.  Shares of each unit's own peak for 32 -> 32 and 64 -> 64 channels, which overlap: operand reads of the tensor
+// core (l1tex__data_pipe_tc_wavefronts) 71 and 77 %, load-store unit (copies, whose sectors land one by one, shuffles, stores of the results;
+// l1tex__data_pipe_lsu_wavefronts) 67 and 60 %, issue slots 34 and 24 %, tensor pipe 31 and 52 %.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
 // 32 -> 32 layer that takes 0.48.)
 //
 // Every result of the forward pass is the same sequence of MMAs (neighbour row, channel block, dy, 16 channels) as in
