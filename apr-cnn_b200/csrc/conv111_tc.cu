@@ -490,7 +490,9 @@ __global__ void __launch_bounds__(C1_THREADS_DW, 1) conv111_tc_dw_kernel(const C
 //               swizzled halves: K-major operands of the weight gradient, and as MN-major operand that of the input gradient, so that one rounding and one
 //               write to shared memory serve both.  (A thread that owns a location and reads 32 of its channels, as in conv111_tc_kernel, has its warp fetch 128
 //               bytes of 32 rows, whose lines, at any multiple of four bytes, its neighbours fetch again: the pass took 1.03 ms; row pieces by bulk copies, which are
-//               issued one after the other, 1.5.)  The sums of gout add the fp32 values before they are rounded;
+//               issued one after the other, 1.5.)  The sums of gout add the fp32 values before they are rounded, those of a tile by halving in fp32, the tiles in
+//               double precision, each by an addition in L2 that nobody waits for (fp32 chains lost up to 1e-6 of a sum on 2.1 M locations and more with the volume; doubles in shared
+//               memory, 1 KB more, cost 64 -> 128 and 128 -> 128 channels 12 %: beyond 196 KB an SM's L1 shrinks);
 //   warp 16     one thread issues the tcgen05.mma of a tile: cout / 16 for the input gradient, 8 for every 128 rows of the weight gradient, whose accumulators
 //               (mtiles x nt columns) stay in TMEM over all tiles of a level range, next to those of the input gradient, two or four tiles in flight;
 //   warps 17-24 epilogue as in conv111_tc_kernel, and the weight sums at the end of a level range.
@@ -503,7 +505,7 @@ struct C1JointParams {
     const float* w;                                // [slot][cout][cin]
     float* gin; ll ld_gin;
     float* partial;                                // [segment][block][cout][cin]
-    float* sums;                                   // [block][cout] (null: not wanted)
+    double* sums;                                  // [block][group][cout] (null: not wanted)
     int stages, nt, mtiles, nacc;                  // ring; cin padded; 128-row accumulators of the weight gradient; accumulators of the input gradient
     uint32_t idesc_x, idesc_w;
     int* error_flag;
@@ -519,9 +521,8 @@ __global__ void __launch_bounds__(C1J_THREADS, 1) conv111_tc_joint_kernel(const 
     const int kpad = (P.cout + 15) / 16 * 16, half_bytes = (kpad + nt) * 128, stage_bytes = 2 * half_bytes;
     unsigned char* b_s = smem + (size_t) stages * stage_bytes;                      // [kpad / 8][nt][8] bf16
     float* out_s = reinterpret_cast<float*>(b_s + (size_t) nt * kpad * 2);          // [2][C1_OUT_CH][256]
-    float* sums_s = out_s + C1_OUT_BYTES / 4;                                       // [groups][kpad]: a channel belongs to one warp of each group
     constexpr int groups = C1J_PROD / WPG;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sums_s + groups * kpad);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + C1_OUT_BYTES / 4);
     uint64_t* full = bars;                              // [stages] operands written (the warps of a group)
     uint64_t* empty = bars + C1_MAX_STAGES;             // [stages] MMAs that read the stage completed
     uint64_t* tmem_full = empty + C1_MAX_STAGES;        // [nacc]   accumulator of the input gradient complete
@@ -542,7 +543,9 @@ __global__ void __launch_bounds__(C1J_THREADS, 1) conv111_tc_joint_kernel(const 
     const int pad_rows = kpad - P.cout;
     for (int e = tid; e < stages * 2 * pad_rows * 8; e += C1J_THREADS)
         *reinterpret_cast<uint4*>(smem + (e / (pad_rows * 8)) * half_bytes + P.cout * 128 + e % (pad_rows * 8) * 16) = make_uint4(0, 0, 0, 0);
-    for (int e = tid; e < groups * kpad; e += C1J_THREADS) sums_s[e] = 0.f;
+    // sums of gout: an entry belongs to one lane of the group, which sets it to zero and adds each tile of the group in turn
+    if (P.sums && warp < C1J_PROD && lane < 8)
+        for (int r = warp % WPG + lane * WPG; r < P.cout; r += 8 * WPG) P.sums[((ll) blockIdx.x * groups + warp / WPG) * P.cout + r] = 0.0;
     if (warp == C1J_MMA) { tmem_alloc(smem_u32(tmem_slot), 512); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
@@ -588,7 +591,6 @@ __global__ void __launch_bounds__(C1J_THREADS, 1) conv111_tc_joint_kernel(const 
             // ---------------- producers ----------------
             const int grp = warp / WPG, sub = warp % WPG, used = min(groups, stages);      // (a ring at least as long as the groups keeps the phases that a wait can meet apart)
             const int nrows = P.cout + P.cin;      // channel rows of a tile
-            float* sums = sums_s + grp * kpad;
             for (int it = grp; grp < used && it < mine && !failed; it += used) {
                 const uint32_t j = j_base + (uint32_t) it, slot = j % (uint32_t) stages, use = j / (uint32_t) stages;
                 const ll p0 = tile_begin(it);
@@ -634,7 +636,7 @@ __global__ void __launch_bounds__(C1J_THREADS, 1) conv111_tc_joint_kernel(const 
                         s[0] += __shfl_xor_sync(0xffffffffu, s[0], 8);
                         s[0] += __shfl_xor_sync(0xffffffffu, s[0], 16);
                         const int r = r0 + lane * WPG;
-                        if (lane < 8 && r < P.cout) sums[r] += s[0];
+                        if (lane < 8 && r < P.cout) atomicAdd(P.sums + ((ll) blockIdx.x * groups + grp) * P.cout + r, (double) s[0]);
                     }
                 }
                 __syncwarp();
@@ -715,35 +717,38 @@ __global__ void __launch_bounds__(C1J_THREADS, 1) conv111_tc_joint_kernel(const 
     }
     tc_fence_before();
     __syncthreads();
-    if (P.sums)
-        for (int c = tid; c < P.cout; c += C1J_THREADS) {
-            float v = 0.f;
-            for (int k = 0; k < groups; ++k) v += sums_s[k * kpad + c];
-            P.sums[(ll) blockIdx.x * P.cout + c] = v;
-        }
     if (warp == C1J_MMA) tmem_dealloc(tmem_w, 512);
 }
 
-// dst[slot of segment y][e] += the blocks' partial sums; the last y (bias): dst_bias[e] = those of the bias.  A block has 32 entries, warp w adds
-// every eighth of the blocks' sums; the warps' sums are added in order.
+// dst[slot of segment y][e] += the blocks' partial sums; the last y (bias): dst_bias[e] = the `nbias` sums of the bias.  A block has 32 entries, warp w adds
+// every eighth of the sums (in T); the warps' sums are added in order.
 struct C1Reduce { int n_segs; int slot[C1_MAX_SEGS]; };
-__global__ void __launch_bounds__(256) c1_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ bias_partial, C1Reduce R, int nblocks, int elems, int cout,
+template<typename T>
+__device__ __forceinline__ T c1_sums(const T* __restrict__ from, int count, int n, int e) {      // valid in warp 0
+    __shared__ T sums[8][32];
+    const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
+    T s = 0;
+    if (e < n)
+#pragma unroll 4
+        for (int b = wrp; b < count; b += 8) s += from[(ll) b * n + e];
+    sums[wrp][lane] = s;
+    __syncthreads();
+    if (wrp == 0) for (int k = 1; k < 8; ++k) s += sums[k][lane];
+    return s;
+}
+__global__ void __launch_bounds__(256) c1_reduce_kernel(const float* __restrict__ partial, const double* __restrict__ bias_partial, C1Reduce R, int nblocks, int nbias, int elems, int cout,
                                                         float* __restrict__ gw, float* __restrict__ gbias) {
-    __shared__ float sums[8][32];
-    const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane, seg = blockIdx.y;
+    const int e = blockIdx.x * 32 + (threadIdx.x & 31), seg = blockIdx.y;
     const bool bias = seg == R.n_segs;
     const int n = bias ? cout : elems;
     if ((int) blockIdx.x * 32 >= n) return;
-    const float* src = bias ? bias_partial : partial + (ll) seg * nblocks * elems;
-    float s = 0.f;
-    if (e < n)
-#pragma unroll 4
-        for (int b = wrp; b < nblocks; b += 8) s += src[(ll) b * n + e];
-    sums[wrp][lane] = s;
-    __syncthreads();
-    if (wrp == 0 && e < n) {
-        for (int k = 1; k < 8; ++k) s += sums[k][lane];
-        if (bias) gbias[e] = s; else gw[(ll) R.slot[seg] * elems + e] += s;
+    const bool writes = threadIdx.x < 32 && e < n;
+    if (bias) {
+        const double s = c1_sums(bias_partial, nbias, n, e);
+        if (writes) gbias[e] = (float) s;
+    } else {
+        const float s = c1_sums(partial + (ll) seg * nblocks * elems, nblocks, n, e);
+        if (writes) gw[(ll) R.slot[seg] * elems + e] += s;
     }
 }
 
@@ -833,7 +838,7 @@ extern "C" int aprnet_conv111_backward_weights_tc(const aprnet_apr* a, int dl, i
         { AprnetProfScope _prof("conv111_dw_reduce", st);
         C1Reduce R;
         R.n_segs = 1; R.slot[0] = sg.slot;
-        c1_reduce_kernel<<<(unsigned) aprnet_ceil_div(elems, 32), 256, 0, st>>>(partial, nullptr, R, grid, (int) elems, cout, gw, nullptr);
+        c1_reduce_kernel<<<(unsigned) aprnet_ceil_div(elems, 32), 256, 0, st>>>(partial, nullptr, R, grid, 0, (int) elems, cout, gw, nullptr);
         }
     }
     APRNET_LAUNCH_CHECK();
@@ -867,16 +872,18 @@ extern "C" int aprnet_conv111_backward_tc(const aprnet_apr* a, int dl, int cin, 
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int blocks = (int) std::min<ll>(tiles, sms), grid = (int) std::min<ll>(blocks, partial_elems / (P.n_segs * elems + cout));
+    const int wpg = cin + cout <= 16 ? 2 : (cin + cout <= 32 ? 4 : 8), groups = C1J_PROD / wpg;
+    // (behind the partial weight gradients the sums of gout, doubles at a multiple of eight bytes)
+    const int blocks = (int) std::min<ll>(tiles, sms), grid = (int) std::min<ll>(blocks, (partial_elems - 1) / (P.n_segs * elems + (gbias ? 2 * groups * cout : 0)));
     if (grid < 1 || grid < blocks / 2) return APRNET_ERR_UNSUPPORTED;            // too little workspace
     P.in = in; P.ld_in = ld_in; P.cin = cin; P.gout = gout; P.ld_out = ld_out; P.cout = cout; P.w = w; P.gin = gin; P.ld_gin = ld_gin;
-    P.partial = partial; P.sums = gbias ? partial + (ll) grid * P.n_segs * elems : nullptr;
+    P.partial = partial; P.sums = gbias ? reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(partial + (ll) grid * P.n_segs * elems) + 7) & ~(uintptr_t) 7) : nullptr;
     P.nt = pick_nt(cin); P.mtiles = (cout + 127) / 128; P.nacc = P.nt <= 64 ? 4 : 2;
     P.idesc_x = make_idesc(P.nt, true, false); P.idesc_w = make_idesc(P.nt, false, false);
     P.error_flag = aprnet_tc_error_flag_device();
-    const int kpad = (cout + 15) / 16 * 16, wpg = cin + cout <= 16 ? 2 : (cin + cout <= 32 ? 4 : 8);
+    const int kpad = (cout + 15) / 16 * 16;
     const size_t stage = (size_t) (kpad + P.nt) * 256, smem_max = 227 * 1024;
-    const size_t fixed = (size_t) P.nt * kpad * 2 + C1_OUT_BYTES + (size_t) C1J_PROD / wpg * kpad * 4 + (2 * C1_MAX_STAGES + 2 * C1_MAX_ACC + 1) * 8 + 16 + 1024;
+    const size_t fixed = (size_t) P.nt * kpad * 2 + C1_OUT_BYTES + (2 * C1_MAX_STAGES + 2 * C1_MAX_ACC + 1) * 8 + 16 + 1024;
     if ((P.mtiles + P.nacc) * P.nt > 512 || fixed + 2 * stage > smem_max) return APRNET_ERR_UNSUPPORTED;
     P.stages = (int) std::min<size_t>(C1_MAX_STAGES, (smem_max - fixed) / stage);
     const size_t smem = P.stages * stage + fixed;
@@ -885,7 +892,7 @@ extern "C" int aprnet_conv111_backward_tc(const aprnet_apr* a, int dl, int cin, 
     if (rc) return rc;
     { AprnetProfScope _prof("conv111_dw_reduce", st);
     c1_reduce_kernel<<<dim3((unsigned) aprnet_ceil_div(std::max<ll>(elems, gbias ? cout : 0), 32), (unsigned) (P.n_segs + (gbias ? 1 : 0))), 256, 0, st>>>(
-        partial, P.sums, R, grid, (int) elems, cout, gw, gbias);
+        partial, P.sums, R, grid, grid * groups, (int) elems, cout, gw, gbias);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;

@@ -81,3 +81,20 @@ def test_conv111_joint_gradients(cin, cout):
         assert float((conv.weight.grad.double().reshape(3, cout, cin) - want_w).norm() / want_w.norm()) <= 1e-5
         want = g.double().sum(dim=(0, 2))
         assert bool(((conv.bias.grad.double() - want).abs() <= g.double().abs().sum(dim=(0, 2)) * 2.0 ** -17).all())
+
+
+def test_conv111_bias_sums_of_equal_values_are_exact():
+    """2^21 locations, so that a block adds more than fifty tiles: 128 equal values of a tile add up exactly in fp32, the tiles exactly in double precision (24 + 21
+    bits), and the result is a float times a power of two.  Chains in fp32 round it off (mantissas chosen so that each addition loses nearly half a bit)."""
+    import pyapr
+    from pyapr import synthetic
+    from pyapr.aprnet import cuda as ops
+    apr = pyapr.apr_from_arrays(synthetic.apr_from_level_map(torch.full((64, 64, 64), 7, dtype=torch.int16), (128, 128, 128)))
+    apr.init_cuda()
+    n = int(pyapr.aprnet.utils.number_particles(apr, 0))
+    assert n == 2 ** 21
+    conv = ops.APRConv(32, 8, nstencils=1, kernel_size=(1, 1, 1), precision="bf16").cuda()
+    value = 1 + torch.tensor([912, 783, 752, 686352, 7748513, 31, 127, 8191], device="cuda").float() * 2.0 ** -23
+    x, g = torch.zeros(1, 32, n, device="cuda"), value.view(1, -1, 1).repeat(1, 1, n)
+    conv(x, [apr], torch.zeros(1, dtype=torch.int32)).backward(g)
+    assert torch.equal(conv.bias.grad, value * 2.0 ** 21)
