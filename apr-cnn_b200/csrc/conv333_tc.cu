@@ -65,6 +65,9 @@ template<int KS> __device__ __forceinline__ int swizzled_chunk(int row, int c) {
 // pieces (8 channels) of the packed rows, and the next tile's loads are in flight while a tile is stored.
 // The 13 layers of a training step on 3.5 M locations: 1.79 ms with a tile per block and a condition per load, now 1.50; a batch of four in inference 2.05 -> 1.75.
 constexpr int PACK_BLOCKS = 4;          // blocks per SM
+// `split` where there is no second tensor, so that no block of 32 channels has channels of two, the last one of a layer included (with the number of channels in its place that
+// block had a condition per load: 8, 16 and 48 channels on 2.0 M locations 69, 86 and 146 us, now 48, 52 and 114)
+constexpr int ONE_TENSOR = 1 << 30;
 // SUMS: the sums of x over its rows are taken along (the gradient of a bias, from the gradient that is packed): four values of a tile in fp32, then in double precision, the
 // warps' sums in sums[block][channel], which channel_sums_kernel adds in order (a pass of its own over 1.2 M rows of 33 channels took
 // 57 us, the packing with sums and their addition 7 us more than without).
@@ -686,12 +689,12 @@ int run_pack_rows(const float* x, ll ld_x, int split, const float* x1, ll ld_x1,
 int* aprnet_tc_error_flag_device() { return ensure_error_flag() == APRNET_OK ? g_error_flag_dev : nullptr; }
 
 int aprnet_tc_pack_rows(const float* x, ll ld_x, ll n, const float* tree, ll ld_tree, ll t, int c, int cpad, void* out, cudaStream_t st) {
-    return run_pack_rows(x, ld_x, c, x, ld_x, n, tree, ld_tree, t, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st);
+    return run_pack_rows(x, ld_x, ONE_TENSOR, x, ld_x, n, tree, ld_tree, t, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st);
 }
 
 // rows of grad_output, and its sums over them in sums_out (c); sums: aprnet_tc_pack_sums_bytes(c)
 int aprnet_tc_pack_rows_sums(const float* x, ll ld_x, ll n, int c, int cpad, void* out, double* sums, float* sums_out, cudaStream_t st) {
-    return run_pack_rows(x, ld_x, c, x, ld_x, n, nullptr, 0, 0, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st, sums, sums_out);
+    return run_pack_rows(x, ld_x, ONE_TENSOR, x, ld_x, n, nullptr, 0, 0, c, cpad, reinterpret_cast<__nv_bfloat16*>(out), st, sums, sums_out);
 }
 size_t aprnet_tc_pack_sums_bytes(int c) { return (size_t) 148 * PACK_BLOCKS * c * sizeof(double); }
 
