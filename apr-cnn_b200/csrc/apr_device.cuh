@@ -212,6 +212,11 @@ int aprnet_small_stage(const float* x, long long ld_x, long long n, const float*
 int aprnet_small_forward(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* w, const float* bias, float* out, long long ld_out, cudaStream_t st);
 int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int slots, const float* vals, const float* gout, long long ld_out,
                                   float* gw, int accumulate, float* partial, cudaStream_t st);
+// fp32 gather kernel (conv333_f32.cu): blocks of four locations per lane up to which the form with one location per lane, four times as many blocks, is the faster
+// one.  Its time grows with the blocks it puts on an SM.  Time of one location per lane / of four, where it puts 1, 2, 3 and 4 blocks on an SM (up to 37, 74, 111 and 148
+// blocks of four): tiles of 64 result channels, forward pass 0.52, 0.75, 0.88, 1.05 to 1.25, same-level input gradient 0.65, 0.95, 1.26, 1.43, cross-level 0.62, 0.9, 1.16, 1.35; 32
+// channels 0.47, 0.65, 0.77, 1.0 and 0.48, 0.66, 0.81, 1.05; 16 channels 0.5, 0.6, 0.72, 0.85 and 0.6, 0.78, 0.9, 1.08; 8 channels 0.55, 0.61, 0.7, 0.75 and 0.8, 0.9, 1.0, 1.1.
+inline int aprnet_f32_few_blocks(int tile_channels, bool forward) { return 37 * ((tile_channels == 64 ? 2 : 3) + (forward ? 1 : 0)); }
 // tensor-core gather over runs (conv333_tc_runs.cu)
 constexpr int APRNET_TAP_KERNEL = 1;      // of aprnet_tc_run_conv: nothing was launched, the kernel that gathers every tap is the faster one
 int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int nt, int ks);

@@ -596,15 +596,13 @@ int launch_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t s
     return APRNET_OK;
 }
 
-// One location per lane where four leave SMs without a block: training steps on 9.7 k, 26 k and 106 k locations 10.7 -> 7.5, 12.0 -> 9.8 and 19.1 -> 18.0 ms.  With the line at 222 or
-// 320 blocks 106 k take 18.7 ms, 68 k (at 320) 15.3 instead of 14.2.
-constexpr int FEW_BLOCKS = 148;
+// One location per lane where four leave SMs without work: training steps on 9.7 k and 26 k locations 10.7 -> 7.5 and 12.0 -> 9.8 ms.  Up to which number of blocks: aprnet_f32_few_blocks.
 template<int WM, int WN, int TN, int MODE>
 int launch_tiles(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
     ll blocks = 0;
     for (const Segment& s : segs) blocks += aprnet_ceil_div(s.end - s.begin, 128 * WM);
     blocks *= (P.n_dim + TN * WN - 1) / (TN * WN);
-    return blocks <= FEW_BLOCKS ? launch_gather<WM, WN, TN, 1, MODE>(P, segs, st, pname) : launch_gather<WM, WN, TN, 4, MODE>(P, segs, st, pname);
+    return blocks <= aprnet_f32_few_blocks(TN * WN, MODE == FORWARD) ? launch_gather<WM, WN, TN, 1, MODE>(P, segs, st, pname) : launch_gather<WM, WN, TN, 4, MODE>(P, segs, st, pname);
 }
 
 template<int MODE>

@@ -43,3 +43,5 @@ extern "C" int rows_overflow(aprnet_apr* a, long long particles, long long nodes
     a->meta = kept;
     return over;
 }
+
+extern "C" int f32_few_blocks(int tile_channels, int forward) { return aprnet_f32_few_blocks(tile_channels, forward != 0); }

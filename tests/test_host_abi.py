@@ -98,3 +98,9 @@ def test_row_numbers_fit_32_bits(helper, lib, particles, nodes, over):
     assert helper.rows_overflow(handle, C.c_longlong(particles), C.c_longlong(nodes)) == over
     if over:
         assert b"32-bit row numbers" in lib.aprnet_last_error()
+
+
+@pytest.mark.parametrize("width,forward,per_sm", [(64, 1, 3), (64, 0, 2), (32, 1, 4), (32, 0, 3), (16, 1, 4), (16, 0, 3), (8, 1, 4), (8, 0, 3)])
+def test_few_blocks_of_an_fp32_gather(helper, width, forward, per_sm):
+    """One location per lane is the faster form as long as it puts at most `per_sm` of its blocks, four for one, on each of 148 SMs."""
+    assert helper.f32_few_blocks(width, forward) * 4 == per_sm * 148
