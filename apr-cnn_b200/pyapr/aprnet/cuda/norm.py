@@ -86,12 +86,20 @@ def _plain(m, kind):
                  _module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks or _module._global_backward_pre_hooks))
 
 
+def _two_inputs(conv, skip, x):
+    """The kernels take the two tensors as they are: more than four channels together, the first tensor's a multiple of four."""
+    return (conv.in_channels > 4 and skip.dim() == x.dim() == 3 and skip.shape[1] % 4 == 0 and skip.shape[1] > 0 and x.shape[1] > 0 and
+            skip.shape[0] == x.shape[0] and skip.shape[2] == x.shape[2] and skip.dtype == x.dtype and skip.device == x.device and skip.is_contiguous() and x.is_contiguous())
+
+
 def conv_norm(conv, norm, x, aprs, level_deltas, skip=None):
-    """`norm(conv(x, aprs, level_deltas))` for an `APRConv` followed by a `GroupNormReLU`; with `skip`, x is `torch.cat([skip, x], 1)`.  One function where both
-    are plain modules and either no gradient is wanted or a backward pass of the convolution in bf16 arithmetic over one batch item can follow; two
-    calls (and the concatenation) otherwise, also where only the normalisation wants gradients: the convolution then keeps nothing and has no backward pass.
+    """`norm(conv(x, aprs, level_deltas))` for an `APRConv` followed by a `GroupNormReLU`; with `skip`, x is `torch.cat([skip, x], 1)`, which is written out where the
+    kernels do not take the two tensors.  One function where both are plain modules and either no gradient is wanted or a backward pass of the convolution in bf16
+    arithmetic over one batch item can follow; two calls otherwise, also where only the normalisation wants gradients: the convolution then keeps nothing and has no backward pass.
     (More than four input channels in a backward pass: the weight gradient of a first layer reads the gradient channel by channel; up to 79.5 M
     locations: beyond them the input gradient does.)"""
+    if skip is not None and not (type(conv) is APRConv and _two_inputs(conv, skip, x)):
+        x, skip = torch.cat([skip, x], dim=1), None
     features = (x,) if skip is None else (skip, x)
     if (_plain(conv, APRConv) and _plain(norm, GroupNormReLU) and conv._function is Conv333Function and conv.bias is None and
             all(t.is_cuda and t.dim() == 3 and t.is_contiguous() for t in features) and len(aprs) == x.shape[0] and x.shape[0] > 0 and
@@ -100,8 +108,6 @@ def conv_norm(conv, norm, x, aprs, level_deltas, skip=None):
         wanted = torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
         precision = conv.precision or get_conv_precision()
         joint = all(t.dtype == torch.float32 and t.device == x.device for t in tensors)
-        if skip is not None:
-            joint = joint and skip.shape[0] == x.shape[0] and skip.shape[2] == x.shape[2] and skip.shape[1] > 0 and skip.shape[1] % 4 == 0 and conv.in_channels > 4
         if wanted:
             joint = (joint and x.shape[0] == 1 and 4 < conv.in_channels and 27 * x.shape[2] + 1 < 2 ** 31 and precision == "bf16" and
                      (conv.weight.requires_grad or any(t.requires_grad for t in features)))

@@ -77,3 +77,32 @@ def test_pooling_without_indices(wanted):
     want = ops.MaxPool()(x.clone().requires_grad_(True), aprs, ld.clone()).detach()
     got = ops.MaxPool()(x.requires_grad_(wanted), aprs, ld.clone())
     assert torch.equal(got.detach(), want) and got.requires_grad == wanted
+
+
+@pytest.mark.parametrize("front,behind", [(33, 31), (6, 10), (1, 32), (32, 32), (0, 20)])
+def test_training_is_one_function_at_any_split(front, behind):
+    """A number of channels in front that the packing of two tensors does not take costs the concatenation, not the joint backward pass: the same bits as one tensor."""
+    from pyapr.aprnet import cuda as ops
+    aprs, n, ld = _setup(["volume"], 0, 0)
+    torch.manual_seed(front)
+    conv, norm = _modules(front + behind, 16, 4, "bf16")
+    whole, g = torch.randn(1, front + behind, n, device="cuda"), torch.randn(1, 16, n, device="cuda")
+    res = []
+    for split in (False, True):
+        conv.zero_grad(); norm.zero_grad()
+        x = whole.clone().requires_grad_(True)
+        y = ops.conv_norm(conv, norm, x[:, front:], aprs, ld, x[:, :front]) if split and front else ops.conv_norm(conv, norm, x, aprs, ld)
+        assert "ConvGroupNormReLUFunction" in y.grad_fn.name()
+        y.backward(g)
+        res.append([y.detach(), x.grad] + [p.grad.clone() for m in (conv, norm) for p in m.parameters()])
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
+def test_no_channels_behind():
+    """The tensor in front may be all of the input."""
+    from pyapr.aprnet import cuda as ops
+    aprs, n, ld = _setup(["odd"], 0, 0)
+    conv, norm = _modules(8, 8, 2, "bf16")
+    x = torch.randn(1, 8, n, device="cuda")
+    with torch.no_grad():
+        assert torch.equal(ops.conv_norm(conv, norm, x[:, 8:], aprs, ld, x), ops.conv_norm(conv, norm, x, aprs, ld))
