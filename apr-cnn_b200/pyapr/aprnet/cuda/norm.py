@@ -86,6 +86,28 @@ def _plain(m, kind):
                  _module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks or _module._global_backward_pre_hooks))
 
 
+def _backward_follows(conv, norm, x, skip, aprs):
+    """Whether the convolution and the normalisation are one function: None if not, else whether a backward pass can follow.  (What refuses most calls comes first: with all
+    checks made for every call, small layers that end in two calls took 7 us more.)"""
+    if type(conv) is not APRConv or type(norm) is not GroupNormReLU or conv.bias is not None:
+        return None
+    weight, gamma, beta = conv.weight, norm.weight, norm.bias
+    features = x.requires_grad or weight.requires_grad or (skip is not None and skip.requires_grad)
+    wanted = (features or (gamma is not None and gamma.requires_grad) or (beta is not None and beta.requires_grad)) and torch.is_grad_enabled()
+    if wanted and not (features and conv.in_channels > 4 and len(aprs) == 1 and (conv.precision or get_conv_precision()) == "bf16"):
+        return None
+    if not (x.is_cuda and x.dim() == 3 and x.is_contiguous() and _plain(conv, APRConv) and _plain(norm, GroupNormReLU) and conv._function is Conv333Function):
+        return None
+    batch, channels, n = x.shape
+    if (batch != len(aprs) or batch == 0 or channels + (0 if skip is None else skip.shape[1]) != conv.in_channels or norm.num_channels != conv.out_channels or
+            (wanted and 27 * n + 1 >= 2 ** 31)):
+        return None
+    for t in (x, weight, gamma, beta):
+        if t is not None and (t.dtype is not torch.float32 or t.device != x.device):
+            return None
+    return wanted
+
+
 def _two_inputs(conv, skip, x):
     """The kernels take the two tensors as they are: more than four channels together, the first tensor's a multiple of four."""
     return (conv.in_channels > 4 and skip.dim() == x.dim() == 3 and skip.shape[1] % 4 == 0 and skip.shape[1] > 0 and x.shape[1] > 0 and
@@ -100,20 +122,10 @@ def conv_norm(conv, norm, x, aprs, level_deltas, skip=None):
     locations: beyond them the input gradient does.)"""
     if skip is not None and not (type(conv) is APRConv and _two_inputs(conv, skip, x)):
         x, skip = torch.cat([skip, x], dim=1), None
-    features = (x,) if skip is None else (skip, x)
-    if (_plain(conv, APRConv) and _plain(norm, GroupNormReLU) and conv._function is Conv333Function and conv.bias is None and
-            all(t.is_cuda and t.dim() == 3 and t.is_contiguous() for t in features) and len(aprs) == x.shape[0] and x.shape[0] > 0 and
-            sum(t.shape[1] for t in features) == conv.in_channels and norm.num_channels == conv.out_channels):
-        tensors = [t for t in (*features, conv.weight, norm.weight, norm.bias) if t is not None]
-        wanted = torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
-        precision = conv.precision or get_conv_precision()
-        joint = all(t.dtype == torch.float32 and t.device == x.device for t in tensors)
-        if wanted:
-            joint = (joint and x.shape[0] == 1 and 4 < conv.in_channels and 27 * x.shape[2] + 1 < 2 ** 31 and precision == "bf16" and
-                     (conv.weight.requires_grad or any(t.requires_grad for t in features)))
-        if joint:
-            return ConvGroupNormReLUFunction.apply(features[0], features[1] if skip is not None else None, conv.weight, norm.weight, norm.bias, aprs, level_deltas,
-                                                   norm.num_groups, norm.eps, norm.relu, precision, wanted)
+    wanted = _backward_follows(conv, norm, x, skip, aprs)
+    if wanted is not None:
+        return ConvGroupNormReLUFunction.apply(x if skip is None else skip, None if skip is None else x, conv.weight, norm.weight, norm.bias, aprs, level_deltas,
+                                               norm.num_groups, norm.eps, norm.relu, conv.precision or get_conv_precision(), wanted)
     if skip is not None:
         x = torch.cat([skip, x], dim=1)
     return norm(conv(x, aprs, level_deltas))
