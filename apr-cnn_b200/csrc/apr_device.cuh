@@ -218,6 +218,7 @@ int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int 
 // channels 0.47, 0.65, 0.77, 1.0 and 0.48, 0.66, 0.81, 1.05; 16 channels 0.5, 0.6, 0.72, 0.85 and 0.6, 0.78, 0.9, 1.08; 8 channels 0.55, 0.61, 0.7, 0.75 and 0.8, 0.9, 1.0, 1.1.
 inline int aprnet_f32_few_blocks(int tile_channels, bool forward) { return 37 * ((tile_channels == 64 ? 2 : 3) + (forward ? 1 : 0)); }
 // tensor-core gather over runs (conv333_tc_runs.cu)
+inline int aprnet_run_max_height(int nt) { return nt >= 64 ? 2 : 4; }      // blocks of 128 rows in a tile of nt result channels, at most (pick_h has the times)
 constexpr int APRNET_TAP_KERNEL = 1;      // of aprnet_tc_run_conv: nothing was launched, the kernel that gathers every tap is the faster one
 int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int nt, int ks);
 int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, int order, const void* rows, int kpad, long long tree_base, long long zero_row, const void* wp,

@@ -533,7 +533,8 @@ int launch_runs(RunParams& P, int sms, cudaStream_t st, const char* pname) {
 // (16 -> 16, 32 -> 32, 64 -> 32 at level delta 0 and 64 -> 64 at level delta 1 of 1.8 M particles, forward: H = 2: 0.22, 0.30,
 // 0.45, 0.26 ms; H = 4: 0.16, 0.24, 0.39, 0.25 ms; conv333_tc.cu: 0.52 for 32 -> 32, 0.48 for 64 -> 64.)  Since the roles branch per warp, result tiles of
 // 64 channels are 6 % faster with H = 2 and its deeper ring (64 -> 64 at level delta 1 0.52 -> 0.49 ms, input gradient 64 -> 32 0.45 -> 0.41), those of 32 stay at 4
-// (32 -> 32 0.38 against 0.44).
+// (32 -> 32 0.38 against 0.44).  Stages of 16 channels had 8 until then: 16 -> 16 forward on 3.5 M and 263 k locations 306 and 38 us with 8, 267 and 31 with 4, input gradient 252 and 234; only
+// input gradients of up to 8 channels on millions of locations lose, 3 to 5 % (8 -> 8 219 and 229).
 inline int pick_h(const RunParams& P, int nt, int ks, int kuse, int max_h, int sms) {
     int best = 1;
     double cost = 0;
@@ -629,10 +630,10 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     }
     // channels per stage: whole 128-byte rows where the width allows (64 -> 64: 0.25 instead of 0.29 ms with 32)
     const int kuse = kpad == 48 && order == 16 ? 48 : (kpad % 64 == 0 && order >= 32 ? 64 : order), ks = kuse == 48 ? 64 : kuse;
-    const int h = pick_h(P, nt, ks, kuse, nt >= 64 ? 2 : (ks == 16 ? 8 : 4), sms);
+    const int h = pick_h(P, nt, ks, kuse, aprnet_run_max_height(nt), sms);
 #define RUN_CASE(NT_, KS_, KORD_, H_, WPS_) if (nt == NT_ && kuse == KS_ && order == KORD_ && h == H_) return launch_runs<NT_, KS_ == 48 ? 64 : KS_, KS_, KORD_, H_, WPS_>(P, sms, st, pname);
     // warps per stage: two, so that four stages are in issue at once; four where the ring holds only two or three stages
-    RUN_CASE(32, 16, 16, 1, 2) RUN_CASE(32, 16, 16, 2, 2) RUN_CASE(32, 16, 16, 4, 2) RUN_CASE(32, 16, 16, 8, 4)
+    RUN_CASE(32, 16, 16, 1, 2) RUN_CASE(32, 16, 16, 2, 2) RUN_CASE(32, 16, 16, 4, 2)
     RUN_CASE(32, 32, 32, 1, 2) RUN_CASE(32, 32, 32, 2, 2) RUN_CASE(32, 32, 32, 4, 2)
     RUN_CASE(32, 64, 64, 1, 2) RUN_CASE(32, 64, 64, 2, 2) RUN_CASE(32, 64, 64, 4, 4)
     RUN_CASE(32, 64, 32, 1, 2) RUN_CASE(32, 64, 32, 2, 2) RUN_CASE(32, 64, 32, 4, 4) RUN_CASE(64, 64, 64, 1, 2) RUN_CASE(64, 64, 64, 2, 4) RUN_CASE(64, 64, 64, 4, 4)

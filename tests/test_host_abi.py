@@ -104,3 +104,9 @@ def test_row_numbers_fit_32_bits(helper, lib, particles, nodes, over):
 def test_few_blocks_of_an_fp32_gather(helper, width, forward, per_sm):
     """One location per lane is the faster form as long as it puts at most `per_sm` of its blocks, four for one, on each of 148 SMs."""
     assert helper.f32_few_blocks(width, forward) * 4 == per_sm * 148
+
+
+@pytest.mark.parametrize("nt,blocks", [(32, 4), (64, 2), (128, 2)])
+def test_tallest_tile_over_runs(helper, nt, blocks):
+    """Whatever a stage holds: with roles that branch per warp, taller tiles are slower for every number of source channels."""
+    assert helper.run_max_height(nt) == blocks
