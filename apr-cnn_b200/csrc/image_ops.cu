@@ -26,7 +26,7 @@ namespace {
 typedef long long ll;
 constexpr int WARPS = 8;                 // rows per block
 constexpr int TPB = WARPS * 32;
-constexpr int CHUNK_BYTES = 2048;        // of a row that a warp holds in shared memory at a time, for each of PAINT_CH channels
+constexpr int ROW_BYTES = 4096;          // of its row that a warp holds in shared memory at a time, for all channels that are painted together
 constexpr int PAINT_CH = 2;              // channels that are painted together, with their cells looked up once
 constexpr int CH_PER_BLOCK = 4;          // channels a warp loops over with its row pointers resolved once
 
@@ -73,10 +73,13 @@ template<typename T> __device__ __forceinline__ void store_equal(T* p, T v, int 
     else *reinterpret_cast<float2*>(p) = make_float2(v, v);
 }
 
-template<typename T>
+// CH channels together.  PIECES: rows longer than a warp holds, painted piece by piece; the cells of a piece are looked for in all levels at once, a lane per level.  (Each level in
+// turn and from both ends, 20 loads one after the other, 256 x 512 x 1024 voxels took 551 and 571 us for one and two float32 channels, 256 x 512 x 512 442 and 464 for float64: more
+// than a pyramid; now 210 and 355, 170 and 313.)
+template<typename T, int CH, bool PIECES>
 __global__ void __launch_bounds__(TPB) paint_rows_kernel(const __grid_constant__ PaintLevels L, const T* __restrict__ parts, ll ld, T* __restrict__ image, int C) {
-    constexpr int CHUNK = CHUNK_BYTES / sizeof(T), VEC = 16 / sizeof(T);
-    __shared__ __align__(16) T buf_s[WARPS][PAINT_CH][CHUNK];
+    constexpr int CHUNK = ROW_BYTES / CH / sizeof(T), VEC = 16 / sizeof(T);
+    __shared__ __align__(16) T buf_s[WARPS][CH][CHUNK];
     const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int) threadIdx.x >> 5, 0);      // (one value per warp, also to the compiler)
     const ll r = (ll) blockIdx.x * WARPS + w;
     if (r >= (ll) L.Z * L.X) return;
@@ -89,42 +92,45 @@ __global__ void __launch_bounds__(TPB) paint_rows_kernel(const __grid_constant__
         first = rp[0]; last = rp[1];
     }
     const ll stride = (ll) L.Z * L.X * L.Y;
-    const int c0 = blockIdx.y * PAINT_CH, nc = min(PAINT_CH, C - c0);
+    const int c0 = blockIdx.y * CH, nc = min(CH, C - c0);
     for (int y0 = 0; y0 < L.Y; y0 += CHUNK) {
-        const int len = min(CHUNK, L.Y - y0);
+        const int len = PIECES ? min(CHUNK, L.Y - y0) : L.Y;
+        ll end = last, next = last;
+        if (PIECES && first < last) {       // the cells that reach into this piece; the next one begins with the last of them or behind it
+            const int k = L.k[lane], behind = ((y0 + len - 1) >> k) + 1;
+            const uint16_t* __restrict__ ys = L.rows[lane].y;
+            end = first_at_or_after(ys, first, min(last, first + behind - (y0 >> k)), behind);
+            next = end > first && ((int) ys[end - 1] + 1) << k > y0 + len ? end - 1 : end;
+        }
         for (int i = 0; i < L.n; ++i) {
-            ll pb = __shfl_sync(0xffffffffu, first, i), pe = __shfl_sync(0xffffffffu, last, i);
-            if (pe <= pb) continue;
+            const ll pb = __shfl_sync(0xffffffffu, first, i), pe = __shfl_sync(0xffffffffu, end, i);
             const int k = L.k[i];
             const uint16_t* __restrict__ ys = L.rows[i].y;
-            if (L.Y > CHUNK) {              // the cells that reach into this piece of the row
-                pb = first_at_or_after(ys, pb, pe, y0 >> k);
-                pe = first_at_or_after(ys, pb, pe, ((y0 + len - 1) >> k) + 1);
-            }
             const T* __restrict__ src = parts + (ll) c0 * ld + L.rows[i].index_offset;
             // a lane writes `width` equal voxels of a cell; 2^shift lanes share a cell
             const int shift = max(k - 2, 0), width = k == 0 ? 1 : (k == 1 ? 2 : 4);
             const ll total = (pe - pb) << shift;
+#pragma unroll 1
             for (ll e = lane; e < total; e += 32) {
                 const ll p = pb + (e >> shift);
                 const int cell = ys[p], at = (cell << k) + (((int) e & ((1 << shift) - 1)) << 2) - y0;
-                T v[PAINT_CH];
+                T v[CH];
 #pragma unroll
-                for (int c = 0; c < PAINT_CH; ++c) v[c] = src[min(c, nc - 1) * ld + p];
-                if (at < 0 || at >= len) continue;
+                for (int c = 0; c < CH; ++c) v[c] = src[min(c, nc - 1) * ld + p];
+                if (PIECES ? (unsigned) at >= (unsigned) len : at >= len) continue;
                 if (L.mean && k > 0) {
                     const int s = 1 << k, cz = z >> k, cx = x >> k;
                     const T inv = T(1) / (T) ((ll) (min((cz + 1) * s, L.Z) - cz * s) * (min((cx + 1) * s, L.X) - cx * s) * (min((cell + 1) * s, L.Y) - cell * s));
 #pragma unroll
-                    for (int c = 0; c < PAINT_CH; ++c) v[c] *= inv;
+                    for (int c = 0; c < CH; ++c) v[c] *= inv;
                 }
 #pragma unroll
-                for (int c = 0; c < PAINT_CH; ++c) store_equal(&buf_s[w][c][at], v[c], width);      // (what a clipped cell writes behind the row stays in the buffer)
+                for (int c = 0; c < CH; ++c) store_equal(&buf_s[w][c][at], v[c], width);      // (what a clipped cell writes behind the row stays in the buffer)
             }
         }
         __syncwarp();
 #pragma unroll
-        for (int c = 0; c < PAINT_CH; ++c) {
+        for (int c = 0; c < CH; ++c) {
             if (c >= nc) break;
             T* dst = image + (c0 + c) * stride + r * L.Y + y0;
             const T* b = buf_s[w][c];
@@ -137,6 +143,7 @@ __global__ void __launch_bounds__(TPB) paint_rows_kernel(const __grid_constant__
             for (; e < len; e += 32) dst[e] = b[e];
         }
         __syncwarp();
+        if (PIECES) first = next;
     }
 }
 
@@ -238,8 +245,19 @@ int run_paint(const aprnet_apr* a, int dl, int C, const T* parts, ll ld, T* imag
         const int sets = cell_rows(a, dl, l, rows);
         for (int i = 0; i < sets; ++i) { L.rows[L.n] = rows[i]; L.k[L.n] = cml - l; L.x_num[L.n] = m.x_num[l]; ++L.n; }
     }
+    const unsigned gx = (unsigned) aprnet_ceil_div((ll) L.Z * L.X, WARPS);
     AprnetProfScope _prof("cells_to_image", st);
-    paint_rows_kernel<T><<<dim3((unsigned) aprnet_ceil_div((ll) L.Z * L.X, WARPS), (unsigned) aprnet_ceil_div(C, PAINT_CH)), TPB, 0, st>>>(L, parts, ld, image, C);
+    if (L.Y * (ll) (PAINT_CH * sizeof(T)) <= ROW_BYTES)
+        paint_rows_kernel<T, PAINT_CH, false><<<dim3(gx, (unsigned) aprnet_ceil_div(C, PAINT_CH)), TPB, 0, st>>>(L, parts, ld, image, C);
+    else {      // longer rows: a channel that has no other beside it has the whole of the warp's shared memory
+        const int pairs = C / PAINT_CH * PAINT_CH;
+        if (pairs) paint_rows_kernel<T, PAINT_CH, true><<<dim3(gx, (unsigned) (pairs / PAINT_CH)), TPB, 0, st>>>(L, parts, ld, image, pairs);
+        for (int c = pairs; c < C; ++c) {
+            T* dst = image + (ll) c * L.Z * L.X * L.Y;
+            if (L.Y * (ll) sizeof(T) <= ROW_BYTES) paint_rows_kernel<T, 1, false><<<gx, TPB, 0, st>>>(L, parts + c * ld, ld, dst, 1);
+            else paint_rows_kernel<T, 1, true><<<gx, TPB, 0, st>>>(L, parts + c * ld, ld, dst, 1);
+        }
+    }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;
 }

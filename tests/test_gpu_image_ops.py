@@ -115,3 +115,50 @@ def test_image_rows_at_any_alignment(shape, channels):
         fine = C.sample_particles_forward(APRPtrVector([apr]), image, ld)
         assert torch.allclose(fine, parts, rtol=1e-5 if dtype == torch.float32 else 1e-13, atol=0)
         assert torch.equal(image, C.reconstruct_forward(APRPtrVector([apr]), parts, ld))
+
+
+@pytest.mark.parametrize("dtype,short,long", [(torch.float32, (64, 256, 512), (64, 128, 1024)), (torch.float64, (64, 256, 256), (64, 128, 512))])
+@pytest.mark.parametrize("channels", [1, 2, 3])
+def test_long_rows_are_painted_as_fast(dtype, short, long, channels):
+    """The same volume cut into rows that a warp holds and into rows twice as long: as many voxels, cells and bytes, so about the same time."""
+    from _pyaprwrapper.data_containers import APRPtrVector
+    from _pyaprwrapper.aprnet import cuda as C
+    import pyapr
+    from pyapr import synthetic
+    took, ld = [], torch.zeros(1, dtype=torch.int32)
+    for shape in (short, long):
+        apr = pyapr.apr_from_arrays(H.blob_arrays(shape, 80, 7))
+        apr.init_cuda()
+        x = torch.randn(1, channels, int(pyapr.aprnet.utils.number_particles(apr, 0)), device="cuda", dtype=dtype)
+        best = []
+        for _ in range(9):
+            C.reconstruct_forward(APRPtrVector([apr]), x, ld)
+            torch.cuda.synchronize()
+            C.profile_enable(True)
+            try:
+                C.reconstruct_forward(APRPtrVector([apr]), x, ld)
+                torch.cuda.synchronize()
+                best.append(C.profile_read()["cells_to_image"][1])
+            finally:
+                C.profile_enable(False)
+        took.append(min(best) / x.shape[2])
+    assert took[1] < 1.35 * took[0], took
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", [(3, 5, 256), (3, 5, 257), (3, 5, 511), (3, 5, 513), (2, 9, 1024), (2, 9, 1025), (4, 4, 2100)])
+@pytest.mark.parametrize("channels", [1, 2, 5])
+def test_rows_around_the_lengths_that_a_warp_holds(shape, channels, dtype):
+    """Each voxel is a copy of the value of the cell that covers it, for cells of all sizes, those that reach over several pieces of a row included."""
+    from _pyaprwrapper.data_containers import APRPtrVector
+    from _pyaprwrapper.aprnet import cuda as C
+    import pyapr
+    from pyapr import synthetic
+    import apr_oracle
+    arrays = synthetic.random_apr(shape, 11, density=0.05)
+    apr = pyapr.apr_from_arrays(arrays)
+    apr.init_cuda()
+    for dl in range(2):
+        x = torch.randn(1, channels, int(pyapr.aprnet.utils.number_particles(apr, dl)), device="cuda", dtype=dtype)
+        got = C.reconstruct_forward(APRPtrVector([apr]), x, torch.full((1,), dl, dtype=torch.int32))[0]
+        assert np.array_equal(H.t2n(got), apr_oracle.reconstruct_forward(arrays, H.t2n(x[0]), dl).astype(H.t2n(got).dtype))
