@@ -246,17 +246,23 @@ int run_paint(const aprnet_apr* a, int dl, int C, const T* parts, ll ld, T* imag
         for (int i = 0; i < sets; ++i) { L.rows[L.n] = rows[i]; L.k[L.n] = cml - l; L.x_num[L.n] = m.x_num[l]; ++L.n; }
     }
     const unsigned gx = (unsigned) aprnet_ceil_div((ll) L.Z * L.X, WARPS);
+    const ll voxels = (ll) L.Z * L.X * L.Y;
     AprnetProfScope _prof("cells_to_image", st);
-    if (L.Y * (ll) (PAINT_CH * sizeof(T)) <= ROW_BYTES)
-        paint_rows_kernel<T, PAINT_CH, false><<<dim3(gx, (unsigned) aprnet_ceil_div(C, PAINT_CH)), TPB, 0, st>>>(L, parts, ld, image, C);
-    else {      // longer rows: a channel that has no other beside it has the whole of the warp's shared memory
-        const int pairs = C / PAINT_CH * PAINT_CH;
-        if (pairs) paint_rows_kernel<T, PAINT_CH, true><<<dim3(gx, (unsigned) (pairs / PAINT_CH)), TPB, 0, st>>>(L, parts, ld, image, pairs);
-        for (int c = pairs; c < C; ++c) {
-            T* dst = image + (ll) c * L.Z * L.X * L.Y;
-            if (L.Y * (ll) sizeof(T) <= ROW_BYTES) paint_rows_kernel<T, 1, false><<<gx, TPB, 0, st>>>(L, parts + c * ld, ld, dst, 1);
-            else paint_rows_kernel<T, 1, true><<<gx, TPB, 0, st>>>(L, parts + c * ld, ld, dst, 1);
+    for (int c0 = 0, n; c0 < C; c0 += n) {                     // grid.y holds 65535 blocks
+        n = std::min(C - c0, 65535 * PAINT_CH);
+        const T* src = parts + c0 * ld;
+        T* dst = image + c0 * voxels;
+        const int pairs = n / PAINT_CH * PAINT_CH;
+        if (L.Y * (ll) (PAINT_CH * sizeof(T)) <= ROW_BYTES) {
+            paint_rows_kernel<T, PAINT_CH, false><<<dim3(gx, (unsigned) aprnet_ceil_div(n, PAINT_CH)), TPB, 0, st>>>(L, src, ld, dst, n);
+            continue;
         }
+        // longer rows: a channel that has no other beside it has the whole of the warp's shared memory
+        if (pairs) paint_rows_kernel<T, PAINT_CH, true><<<dim3(gx, (unsigned) (pairs / PAINT_CH)), TPB, 0, st>>>(L, src, ld, dst, pairs);
+        if (pairs == n) continue;
+        src += pairs * ld; dst += pairs * voxels;
+        if (L.Y * (ll) sizeof(T) <= ROW_BYTES) paint_rows_kernel<T, 1, false><<<gx, TPB, 0, st>>>(L, src, ld, dst, 1);
+        else paint_rows_kernel<T, 1, true><<<gx, TPB, 0, st>>>(L, src, ld, dst, 1);
     }
     APRNET_LAUNCH_CHECK();
     return APRNET_OK;

@@ -162,3 +162,17 @@ def test_rows_around_the_lengths_that_a_warp_holds(shape, channels, dtype):
         x = torch.randn(1, channels, int(pyapr.aprnet.utils.number_particles(apr, dl)), device="cuda", dtype=dtype)
         got = C.reconstruct_forward(APRPtrVector([apr]), x, torch.full((1,), dl, dtype=torch.int32))[0]
         assert np.array_equal(H.t2n(got), apr_oracle.reconstruct_forward(arrays, H.t2n(x[0]), dl).astype(H.t2n(got).dtype))
+
+
+def test_more_channels_than_a_grid_has_rows_of_blocks():
+    """131,073 channels: painted two at a time they are one more than 65,535 rows of blocks hold."""
+    from _pyaprwrapper.data_containers import APRPtrVector
+    from _pyaprwrapper.aprnet import cuda as C
+    import pyapr
+    from pyapr import synthetic
+    apr = pyapr.apr_from_arrays(synthetic.apr_from_level_map(torch.full((2, 2, 2), 2, dtype=torch.int16), (4, 4, 4)))
+    apr.init_cuda()
+    channels, ld = 131073, torch.zeros(1, dtype=torch.int32)
+    x = torch.randn(1, channels, 64, device="cuda")
+    image = C.reconstruct_forward(APRPtrVector([apr]), x, ld)
+    assert torch.equal(C.sample_particles_forward(APRPtrVector([apr]), image, ld), x)
