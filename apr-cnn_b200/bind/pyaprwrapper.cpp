@@ -812,6 +812,7 @@ static void check_same_extent(std::vector<APR*>& aprs, const std::vector<int>& d
     }
 }
 
+// sums of an image's cells per level (image -> particles)
 static torch::Tensor image_workspace(std::vector<APR*>& aprs, const std::vector<int>& dl, const torch::Tensor& like) {
     int64_t bytes = 256;
     for (size_t i = 0; i < aprs.size(); ++i)
@@ -828,10 +829,9 @@ torch::Tensor reconstruct_forward(std::vector<APR*>& aprs, torch::Tensor input, 
     const auto e = image_extent(aprs, dl, input);
     check_same_extent(aprs, dl, input, e);
     auto output = torch::empty({input.size(0), input.size(1), e[0], e[1], e[2]}, input.options());
-    auto ws = image_workspace(aprs, dl, input);
     for (int64_t b = 0; b < input.size(0); ++b)
         check(aprnet_cells_to_image(aprs[b]->handle(input), dl[b], dtype_id(input), (int) input.size(1), row(input, b), input.size(2),
-                                    row(output, b), 0, ws.data_ptr(), stream_of(input)), "reconstruct_forward");
+                                    row(output, b), 0, nullptr, stream_of(input)), "reconstruct_forward");
     return output;
 }
 
@@ -880,10 +880,9 @@ torch::Tensor sample_particles_backward(std::vector<APR*>& aprs, torch::Tensor g
     const auto e = image_extent(aprs, dl, grad_output);
     check_same_extent(aprs, dl, grad_output, e);
     auto grad_input = torch::empty({grad_output.size(0), grad_output.size(1), e[0], e[1], e[2]}, grad_output.options());
-    auto ws = image_workspace(aprs, dl, grad_output);
     for (int64_t b = 0; b < grad_output.size(0); ++b)
         check(aprnet_cells_to_image(aprs[b]->handle(grad_output), dl[b], dtype_id(grad_output), (int) grad_output.size(1), row(grad_output, b),
-                                    grad_output.size(2), row(grad_input, b), 1, ws.data_ptr(), stream_of(grad_output)), "sample_particles_backward");
+                                    grad_output.size(2), row(grad_input, b), 1, nullptr, stream_of(grad_output)), "sample_particles_backward");
     return grad_input;
 }
 

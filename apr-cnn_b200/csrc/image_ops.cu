@@ -337,10 +337,9 @@ extern "C" int aprnet_sample_particles_backward(const aprnet_apr* a, int dl, int
     return dispatch<true>(a, dl, dtype, C, const_cast<void*>(grad_output), ld_out, grad_image, 1, nullptr, stream);
 }
 
-// the same two transfers with the caller's workspace (aprnet_image_workspace_bytes)
-extern "C" int aprnet_cells_to_image(const aprnet_apr* a, int dl, int dtype, int C, const void* cells, int64_t ld, void* image, int mean, void* workspace, void* stream) {
-    APRNET_ARG_CHECK(workspace, "null workspace");
-    return dispatch<true>(a, dl, dtype, C, const_cast<void*>(cells), ld, image, mean, workspace, stream);
+// the same two transfers with the caller's workspace (aprnet_image_workspace_bytes), which only image -> particles uses
+extern "C" int aprnet_cells_to_image(const aprnet_apr* a, int dl, int dtype, int C, const void* cells, int64_t ld, void* image, int mean, void*, void* stream) {
+    return dispatch<true>(a, dl, dtype, C, const_cast<void*>(cells), ld, image, mean, nullptr, stream);
 }
 extern "C" int aprnet_image_to_cells(const aprnet_apr* a, int dl, int dtype, int C, const void* image, void* cells, int64_t ld, int mean, void* workspace, void* stream) {
     APRNET_ARG_CHECK(workspace, "null workspace");

@@ -435,8 +435,8 @@ int aprnet_sample_particles_forward(const aprnet_apr* apr, int level_delta, int 
 int aprnet_sample_particles_backward(const aprnet_apr* apr, int level_delta, int dtype, int channels,
                                      const void* grad_output, int64_t ld_out, void* grad_image, void* stream);
 
-/* The transfers behind the four functions above, with the workspace (aprnet_image_workspace_bytes bytes) from the
- * caller instead of a stream-ordered allocation per call.  mean = 0: values are copied / summed (reconstruct and its
+/* The transfers behind the four functions above, image -> cells with the workspace (aprnet_image_workspace_bytes bytes) from the
+ * caller instead of a stream-ordered allocation per call; cells -> image needs none (workspace: not used, may be NULL).  mean = 0: values are copied / summed (reconstruct and its
  * backward), mean = 1: they are divided by the cell volume (backward of sample_particles / sample_particles). */
 int64_t aprnet_image_workspace_bytes(const aprnet_apr* apr, int level_delta, int dtype, int channels);
 int aprnet_cells_to_image(const aprnet_apr* apr, int level_delta, int dtype, int channels, const void* cells, int64_t ld,

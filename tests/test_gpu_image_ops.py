@@ -176,3 +176,19 @@ def test_more_channels_than_a_grid_has_rows_of_blocks():
     x = torch.randn(1, channels, 64, device="cuda")
     image = C.reconstruct_forward(APRPtrVector([apr]), x, ld)
     assert torch.equal(C.sample_particles_forward(APRPtrVector([apr]), image, ld), x)
+
+
+@pytest.mark.parametrize("name", ["reconstruct_forward", "sample_particles_backward"])
+def test_painting_allocates_its_result_only(name):
+    from _pyaprwrapper.data_containers import APRPtrVector
+    from _pyaprwrapper.aprnet import cuda as C
+    a = H.blob_arrays((64, 128, 128), 40, 11)
+    import pyapr
+    apr = pyapr.apr_from_arrays(a)
+    apr.init_cuda()
+    x, ld = torch.randn(1, 8, a.n_particles, device="cuda"), torch.zeros(1, dtype=torch.int32)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    image = getattr(C, name)(APRPtrVector([apr]), x, ld)
+    assert torch.cuda.max_memory_allocated() - before <= image.numel() * 4 + 4096

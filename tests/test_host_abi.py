@@ -110,3 +110,14 @@ def test_few_blocks_of_an_fp32_gather(helper, width, forward, per_sm):
 def test_tallest_tile_over_runs(helper, nt, blocks):
     """Whatever a stage holds: with roles that branch per warp, taller tiles are slower for every number of source channels."""
     assert helper.run_max_height(nt) == blocks
+
+
+def test_painting_needs_no_workspace(lib):
+    """Cells to image: a null workspace is no bad argument (the device check comes after the arguments'); image to cells uses one."""
+    if torch.cuda.is_available():
+        pytest.skip("with a GPU the call would reach kernels with the made-up pointers")
+    lib, handle = lib
+    assert lib.aprnet_cells_to_image(handle, i(0), i(0), i(2), p, n, p, i(0), None, None) < 0
+    assert lib.aprnet_last_error() == b"no current CUDA device"
+    assert lib.aprnet_image_to_cells(handle, i(0), i(0), i(2), p, p, n, i(0), None, None) < 0
+    assert b"workspace" in lib.aprnet_last_error()
