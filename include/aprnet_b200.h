@@ -402,10 +402,10 @@ int aprnet_groupnorm_backward_apply(int dtype, int batch, int channels, int64_t 
 int aprnet_maxpool_forward(const aprnet_apr* apr, int level_delta, int dtype, int channels,
                            const void* input, int64_t ld_in, void* output, int64_t* max_indices, int64_t ld_out,
                            void* stream);
-/* grad_input must be zero-filled by the caller (only the kept particles and the arg-max positions are written). */
-/* without indices, where no backward pass follows */
+/* The same without indices, where no backward pass follows. */
 int aprnet_maxpool_forward_values(const aprnet_apr* apr, int level_delta, int dtype, int channels, const void* input, int64_t ld_in,
                                   void* output, int64_t ld_out, void* stream);
+/* grad_input must be zero-filled by the caller (only the kept particles and the arg-max positions are written). */
 int aprnet_maxpool_backward(const aprnet_apr* apr, int level_delta, int dtype, int channels,
                             const void* grad_output, const int64_t* max_indices, int64_t ld_out,
                             void* grad_input, int64_t ld_in, void* stream);

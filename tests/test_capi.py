@@ -42,3 +42,12 @@ def test_argument_errors_are_status_codes():
     rc = lib.aprnet_conv111_forward(None, 0, 0, 1, 1, 1, None, C.c_int64(0), None, None, C.c_int64(0), None)
     assert rc == -1
     assert lib.aprnet_conv333_partial_elems(32, 32) >= 27 * 32 * 32 * 4
+
+
+def test_preconditions_stand_at_their_functions():
+    """What a caller has to do before a call is said in the comment directly in front of it."""
+    text = open(HEADER).read()
+    for name, words in (("aprnet_maxpool_backward", "zero-filled by the caller"), ("aprnet_maxpool_forward_values", "no backward pass follows"),
+                        ("aprnet_groupnorm_relu_forward_valid", "not read"), ("aprnet_conv333_rows_backward_bias", "aligned to 8 bytes")):
+        comment = re.search(r"/\*((?:(?!\*/).)*)\*/\s*int " + name + r"\(", text, flags=re.S)
+        assert comment and words in comment.group(1), name
