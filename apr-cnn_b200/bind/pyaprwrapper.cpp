@@ -642,10 +642,10 @@ static std::vector<torch::Tensor> conv111_backward_impl(std::vector<APR*>& aprs,
     const int dt = dtype_id(input);
     const bool tc = resolve_mode(precision) == 1 && dt == APRNET_F32;
     void* st = stream_of(input);
+    for (size_t i = 0; i < aprs.size(); ++i) check_level_delta(*aprs[i], dl[i]);
     // the joint pass sums over the particles of one item; entries behind them would count, too
     const bool sums = with_bias && input.size(0) == 1 && aprs[0]->number_parts(dl[0]) == n;
     for (int64_t b = 0; b < input.size(0); ++b) {
-        check_level_delta(*aprs[b], dl[b]);
         aprnet_apr* h = aprs[b]->handle(input);
         int rc = APRNET_ERR_UNSUPPORTED;
         if (tc) {

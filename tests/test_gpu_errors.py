@@ -70,3 +70,18 @@ def test_handle_on_another_device_is_an_argument_error():
         assert torch.cuda.current_device() == 1
     del apr
     assert torch.cuda.current_device() == 0           # destroying an APR leaves the current device alone
+
+
+@pytest.mark.parametrize("name", ["conv111_backward", "conv111_backward_with_bias"])
+@pytest.mark.parametrize("dl", [-1, 40])
+def test_level_delta_out_of_range(name, dl):
+    """The same error with and without the gradient of a bias."""
+    import pyapr
+    from _pyaprwrapper.aprnet import cuda as C
+    from _pyaprwrapper.data_containers import APRPtrVector
+    a = H.blob_arrays()
+    apr = pyapr.apr_from_arrays(a)
+    apr.init_cuda()
+    x, w = torch.rand(1, 8, a.n_particles, device="cuda"), torch.rand(1, 8, 8, 1, 1, 1, device="cuda")
+    with pytest.raises(RuntimeError, match="level delta"):
+        getattr(C, name)(APRPtrVector([apr]), x, w, x, torch.full((1,), dl, dtype=torch.int32))
