@@ -585,7 +585,8 @@ int launch_wide(RunParams& P, int sms, cudaStream_t st, const char* pname) {
 // nt_order, ks: tile width and channels per stage that conv333_tc.cu takes for the layer.  The forward pass keeps its order: stages of
 // `ks` channels that hold three taps for nt_order <= 64, and for 128 where ks < 64 (the same order as here); one tap at a time for 128 and ks = 64 (the same only when all
 // channels are in one stage), pairs of taps for 256.  The input gradient is free: nothing that follows depends on its last bit.
-// -1: one tap after the other over all channels, in the kernel for that (APRNET_TAP_KERNEL where the tap kernel is the faster one).
+// -1: one tap after the other over all channels, in the kernel for that (APRNET_TAP_KERNEL where the tap kernel is the faster one; result tiles narrower than 128, that is few
+// locations, are 10 to 15 % faster in the tap kernel: 9 k locations 42 against 37 us).
 int aprnet_tc_runs_order(int backward, int kpad, int nt_order, int nt, int ks) {
     if (backward) return kpad % 32 == 0 ? 32 : 16;
     if (nt_order <= 64) return ks;
@@ -615,7 +616,6 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     if (order < 0) {
         // Microseconds of a wave of tiles for 128 source channels, and before the first one, of this kernel with two and with one block of 128 rows per tile and of the tap kernel,
         // as fitted to 128 -> 128 layers: 553 k locations 455, 538, 522; 170 k 158, 177, 186; 61 k 80, 85, 83; 33 k 55, 53, 49; 32 k (fewer tiles of two than SMs) -, 39, 49.
-        // Result tiles narrower than 128 (few locations) are 10 to 15 % faster in the tap kernel: 9 k locations 42 against 37.
         ll t2 = 0, t1 = 0, taps = 0;
         for (int i = 0; i < P.n_segs; ++i) {
             const ll slots_ = P.slot_end[i] - P.slot_begin[i];
@@ -625,7 +625,7 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
         auto time = [&](ll tiles, double wave, double start) { return (double) ((tiles + sms - 1) / sms) * wave * k + start; };
         int pieces, wtiles;
         const double two = wide_shape(nt, 2, kpad, &pieces, &wtiles) ? time(t2, 27.0, 3.0) : 1e30, one = time(t1, 15.8, 7.0);
-        if (nt != 128 || std::min(one, two) > time(taps, 17.4, 14.0)) return APRNET_TAP_KERNEL;
+        if (std::min(one, two) > time(taps, 17.4, 14.0)) return APRNET_TAP_KERNEL;
         return two < one ? launch_wide<128, 2>(P, sms, st, pname) : launch_wide<128, 1>(P, sms, st, pname);
     }
     // channels per stage: whole 128-byte rows where the width allows (64 -> 64: 0.25 instead of 0.29 ms with 32)
@@ -636,13 +636,13 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     RUN_CASE(32, 16, 16, 1, 2) RUN_CASE(32, 16, 16, 2, 2) RUN_CASE(32, 16, 16, 4, 2)
     RUN_CASE(32, 32, 32, 1, 2) RUN_CASE(32, 32, 32, 2, 2) RUN_CASE(32, 32, 32, 4, 2)
     RUN_CASE(32, 64, 64, 1, 2) RUN_CASE(32, 64, 64, 2, 2) RUN_CASE(32, 64, 64, 4, 4)
-    RUN_CASE(32, 64, 32, 1, 2) RUN_CASE(32, 64, 32, 2, 2) RUN_CASE(32, 64, 32, 4, 4) RUN_CASE(64, 64, 64, 1, 2) RUN_CASE(64, 64, 64, 2, 4) RUN_CASE(64, 64, 64, 4, 4)
-    RUN_CASE(64, 16, 16, 1, 2) RUN_CASE(64, 16, 16, 2, 2) RUN_CASE(64, 16, 16, 4, 2)
-    RUN_CASE(64, 32, 32, 1, 2) RUN_CASE(64, 32, 32, 2, 2) RUN_CASE(64, 32, 32, 4, 2)
-    RUN_CASE(64, 64, 32, 1, 2) RUN_CASE(64, 64, 32, 2, 4) RUN_CASE(64, 64, 32, 4, 4)
+    RUN_CASE(32, 64, 32, 1, 2) RUN_CASE(32, 64, 32, 2, 2) RUN_CASE(32, 64, 32, 4, 4) RUN_CASE(64, 64, 64, 1, 2) RUN_CASE(64, 64, 64, 2, 4)
+    RUN_CASE(64, 16, 16, 1, 2) RUN_CASE(64, 16, 16, 2, 2)
+    RUN_CASE(64, 32, 32, 1, 2) RUN_CASE(64, 32, 32, 2, 2)
+    RUN_CASE(64, 64, 32, 1, 2) RUN_CASE(64, 64, 32, 2, 4)
     RUN_CASE(128, 16, 16, 1, 2) RUN_CASE(128, 16, 16, 2, 2) RUN_CASE(128, 32, 32, 1, 2) RUN_CASE(128, 32, 32, 2, 2)
     RUN_CASE(32, 48, 16, 1, 2) RUN_CASE(32, 48, 16, 2, 2) RUN_CASE(32, 48, 16, 4, 4)
-    RUN_CASE(64, 48, 16, 1, 2) RUN_CASE(64, 48, 16, 2, 4) RUN_CASE(64, 48, 16, 4, 4) RUN_CASE(128, 48, 16, 1, 4) RUN_CASE(128, 48, 16, 2, 4)
+    RUN_CASE(64, 48, 16, 1, 2) RUN_CASE(64, 48, 16, 2, 4) RUN_CASE(128, 48, 16, 1, 4) RUN_CASE(128, 48, 16, 2, 4)
     RUN_CASE(128, 64, 32, 1, 4) RUN_CASE(128, 64, 32, 2, 4) RUN_CASE(128, 64, 64, 1, 4) RUN_CASE(128, 64, 64, 2, 4)
 #undef RUN_CASE
     aprnet_set_error("conv333 tensor-core path: unsupported run geometry nt=%d ks=%d order=%d h=%d", nt, ks, order, h);

@@ -9,6 +9,7 @@ Cross-level input gradient: the sums per (target, tap) go through a bounded work
 Row numbers: the kernels hold them in 32 bits; structures beyond that are refused when a plan is built."""
 import ctypes as C
 import os
+import re
 import subprocess
 
 import pytest
@@ -121,3 +122,11 @@ def test_painting_needs_no_workspace(lib):
     assert lib.aprnet_last_error() == b"no current CUDA device"
     assert lib.aprnet_image_to_cells(handle, i(0), i(0), i(2), p, p, n, i(0), None, None) < 0
     assert b"workspace" in lib.aprnet_last_error()
+
+
+def test_every_compiled_tile_over_runs_is_reached(helper):
+    """The variants of the run kernel are those that the choice of a tile's height can ask for."""
+    source = open(os.path.join(PKG, "csrc", "conv333_tc_runs.cu")).read()
+    cases = [tuple(int(v) for v in c.split(",")) for c in re.findall(r"RUN_CASE\(((?:\d+, ){4}\d+)\)", source)]
+    assert cases and {(nt, ks, order): max(h for a, b, c, h, _ in cases if (a, b, c) == (nt, ks, order)) for nt, ks, order, _, _ in cases} == {
+        (nt, ks, order): helper.run_max_height(nt) for nt, ks, order, _, _ in cases}
