@@ -8,8 +8,8 @@
 // inside the pattern is an ordinary one.)  That is 9 x 1.07 .. 1.27 gathered rows per location instead of 27; slots without a
 // location are the price, 7 to 27 % more multiply-adds.  Each weight tile that is fetched meets H blocks of 128 rows.
 // What bounds it: operand reads.  Shares of each unit's own peak for 32 -> 32 and 64 -> 64 channels, which overlap: operand reads of the tensor
-// core (l1tex__data_pipe_tc_wavefronts) 71 and 77 %, load-store unit (copies, whose sectors land one by one, shuffles, stores of the results;
-// l1tex__data_pipe_lsu_wavefronts) 67 and 60 %, issue slots 34 and 24 %, tensor pipe 31 and 52 %.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
+// core (l1tex__data_pipe_tc_wavefronts) 71 and 80 %, load-store unit (copies, whose sectors land one by one, shuffles, stores of the results;
+// l1tex__data_pipe_lsu_wavefronts) 67 and 60 %, issue slots 34 and 30 %, tensor pipe 31 and 54 %; 16 -> 16: 52, 61, 38 and 23 %.  (All rows by tile::gather4 instead of cp.async took 6.6 cycles per row: 0.96 ms for a
 // 32 -> 32 layer that takes 0.48.)
 //
 // Every result of the forward pass is the same sequence of MMAs (neighbour row, channel block, dy, 16 channels) as in
@@ -616,6 +616,7 @@ int aprnet_tc_run_conv(aprnet_apr* a, int dl, int backward, int slots, int nt, i
     if (order < 0) {
         // Microseconds of a wave of tiles for 128 source channels, and before the first one, of this kernel with two and with one block of 128 rows per tile and of the tap kernel,
         // as fitted to 128 -> 128 layers: 553 k locations 455, 538, 522; 170 k 158, 177, 186; 61 k 80, 85, 83; 33 k 55, 53, 49; 32 k (fewer tiles of two than SMs) -, 39, 49.
+        // The choice against the tap kernel at other widths, 9 k to 2 M locations: 192 and 256 source channels 0 to 30 % faster, 320 to 512 (whose rows leave room for tiles of one block only) 0 to 20 %.
         ll t2 = 0, t1 = 0, taps = 0;
         for (int i = 0; i < P.n_segs; ++i) {
             const ll slots_ = P.slot_end[i] - P.slot_begin[i];
