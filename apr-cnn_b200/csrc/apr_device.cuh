@@ -217,6 +217,10 @@ int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int 
 // blocks of four): tiles of 64 result channels, forward pass 0.52, 0.75, 0.88, 1.05 to 1.25, same-level input gradient 0.65, 0.95, 1.26, 1.43, cross-level 0.62, 0.9, 1.16, 1.35; 32
 // channels 0.47, 0.65, 0.77, 1.0 and 0.48, 0.66, 0.81, 1.05; 16 channels 0.5, 0.6, 0.72, 0.85 and 0.6, 0.78, 0.9, 1.08; 8 channels 0.55, 0.61, 0.7, 0.75 and 0.8, 0.9, 1.0, 1.1.
 inline int aprnet_f32_few_blocks(int tile_channels, bool forward) { return 37 * ((tile_channels == 64 ? 2 : 3) + (forward ? 1 : 0)); }
+// Blocks of four locations per lane from which 512 threads per SM are faster than 384 (forward pass of 64 result channels, same-level input gradient of 32): beyond the three blocks per
+// SM that 384 threads hold.  Time with 384 / with 512 threads up to 148, 296 and 444 blocks and beyond 900: 64 channels 0.96, 0.98, 0.98 and 1.01; 32 channels, 32 and more source
+// channels, 0.87, 0.98, 1.01 and 1.05; 24 0.81, 0.93, 0.95 and 1.01; 16 0.87, 0.95, 0.95 and 0.98; 8 0.86, 0.87, 0.89 and 0.88.
+inline bool aprnet_f32_many_blocks(int tile_channels, int source_channels, long long blocks) { return blocks > 3 * 148 && (tile_channels == 64 || source_channels > 16); }
 // tensor-core gather over runs (conv333_tc_runs.cu)
 inline int aprnet_run_max_height(int nt) { return nt >= 64 ? 2 : 4; }      // blocks of 128 rows in a tile of nt result channels, at most (pick_h has the times)
 constexpr int APRNET_TAP_KERNEL = 1;      // of aprnet_tc_run_conv: nothing was launched, the kernel that gathers every tap is the faster one

@@ -144,14 +144,14 @@ enum { FORWARD, SAME_LEVEL, TARGETS };        // forward pass, the two parts of 
 // the reads).  The forward pass has next to none (neighbours outside the volume).
 // Threads per SM and ring slots.  16 warps of 128 registers instead of 12 of 168 give little, because the register file bounds the loop (paired multiply-adds read
 // four registers a cycle): input gradient of 32 channels 4.94 -> 4.56 ms (32 -> 32, 3.5 M locations, three slots), forward pass of 64 9.01 -> 8.90 ms (64 -> 64 at level
-// delta 1), weight gradient of 16 x 32 tiles 8.16 -> 7.98 (33 -> 24); the other shapes lose 1 to 14 %.
-template<int WM, int TN, int R, int MODE> struct GatherShape {
-    static constexpr bool MORE = R == 4 && TN == 16 && ((MODE == FORWARD && WM == 1) || (MODE == SAME_LEVEL && WM == 2));
-    static constexpr int THREADS = R == 1 ? 768 : (MORE ? 512 : 384), RING = MORE && WM == 2 ? 3 : 4;
+// delta 1), weight gradient of 16 x 32 tiles 8.16 -> 7.98 (33 -> 24); the other shapes lose 1 to 14 %, and so do these where the blocks do not need the room (MANY: aprnet_f32_many_blocks).
+template<int WM, int TN, int MODE> constexpr bool MORE_THREADS = TN == 16 && ((MODE == FORWARD && WM == 1) || (MODE == SAME_LEVEL && WM == 2));
+template<int WM, int R, bool MANY> struct GatherShape {
+    static constexpr int THREADS = R == 1 ? 768 : (MANY ? 512 : 384), RING = MANY && WM == 2 ? 3 : 4;
 };
-template<int WM, int WN, int TN, int R, int MODE>
-__global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, TN, R, MODE>::THREADS / (32 * WM * WN)) conv333_f32_gather_kernel(const F32Params P) {
-    constexpr int RING = GatherShape<WM, TN, R, MODE>::RING;
+template<int WM, int WN, int TN, int R, int MODE, bool MANY>
+__global__ void __launch_bounds__(32 * WM * WN, GatherShape<WM, R, MANY>::THREADS / (32 * WM * WN)) conv333_f32_gather_kernel(const F32Params P) {
+    constexpr int RING = GatherShape<WM, R, MANY>::RING;
     constexpr int T = 32 * WM * WN, M = 32 * R * WM, NT = TN * WN;
     constexpr bool KMAJOR = MODE == FORWARD, ZEROS = MODE == TARGETS || (MODE == SAME_LEVEL && NT < 64);
     constexpr int RPT = M * (KS / 4) / T;          // row pieces a thread copies per slot
@@ -580,11 +580,11 @@ int run_pack_weights(const aprnet_apr* a, int dl, const float* w, int slots, int
     return aprnet_pack_weights(a, dl, false, w, slots, cin, cout, transposed, nt, (n_dim + nt - 1) / nt, pad4(transposed ? cout : cin), wp, st);
 }
 
-template<int WM, int WN, int TN, int R, int MODE>
+template<int WM, int WN, int TN, int R, int MODE, bool MANY = false>
 int launch_gather(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st, const char* pname) {
     constexpr int M = 32 * R * WM, NT = TN * WN;
-    constexpr size_t smem = (size_t) GatherShape<WM, TN, R, MODE>::RING * (M + NT) * KS * sizeof(float);
-    auto kern = conv333_f32_gather_kernel<WM, WN, TN, R, MODE>;
+    constexpr size_t smem = (size_t) GatherShape<WM, R, MANY>::RING * (M + NT) * KS * sizeof(float);
+    auto kern = conv333_f32_gather_kernel<WM, WN, TN, R, MODE, MANY>;
     APRNET_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     P.segs = make_seg_table(segs, M);
     P.n_tiles = (P.n_dim + NT - 1) / NT;
@@ -602,7 +602,10 @@ int launch_tiles(F32Params& P, const std::vector<Segment>& segs, cudaStream_t st
     ll blocks = 0;
     for (const Segment& s : segs) blocks += aprnet_ceil_div(s.end - s.begin, 128 * WM);
     blocks *= (P.n_dim + TN * WN - 1) / (TN * WN);
-    return blocks <= aprnet_f32_few_blocks(TN * WN, MODE == FORWARD) ? launch_gather<WM, WN, TN, 1, MODE>(P, segs, st, pname) : launch_gather<WM, WN, TN, 4, MODE>(P, segs, st, pname);
+    if (blocks <= aprnet_f32_few_blocks(TN * WN, MODE == FORWARD)) return launch_gather<WM, WN, TN, 1, MODE>(P, segs, st, pname);
+    if constexpr (MORE_THREADS<WM, TN, MODE>)
+        if (aprnet_f32_many_blocks(TN * WN, P.kpad, blocks)) return launch_gather<WM, WN, TN, 4, MODE, true>(P, segs, st, pname);
+    return launch_gather<WM, WN, TN, 4, MODE>(P, segs, st, pname);
 }
 
 template<int MODE>

@@ -46,3 +46,4 @@ extern "C" int rows_overflow(aprnet_apr* a, long long particles, long long nodes
 
 extern "C" int f32_few_blocks(int tile_channels, int forward) { return aprnet_f32_few_blocks(tile_channels, forward != 0); }
 extern "C" int run_max_height(int nt) { return aprnet_run_max_height(nt); }
+extern "C" int f32_many_blocks(int tile_channels, int source_channels, long long blocks) { return aprnet_f32_many_blocks(tile_channels, source_channels, blocks); }

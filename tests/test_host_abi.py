@@ -130,3 +130,9 @@ def test_every_compiled_tile_over_runs_is_reached(helper):
     cases = [tuple(int(v) for v in c.split(",")) for c in re.findall(r"RUN_CASE\(((?:\d+, ){4}\d+)\)", source)]
     assert cases and {(nt, ks, order): max(h for a, b, c, h, _ in cases if (a, b, c) == (nt, ks, order)) for nt, ks, order, _, _ in cases} == {
         (nt, ks, order): helper.run_max_height(nt) for nt, ks, order, _, _ in cases}
+
+
+@pytest.mark.parametrize("width,source,blocks,many", [(64, 8, 444, 0), (64, 8, 445, 1), (64, 128, 148, 0), (32, 16, 100000, 0), (32, 20, 444, 0), (32, 20, 445, 1), (32, 64, 148, 0)])
+def test_threads_per_sm_of_an_fp32_gather(helper, width, source, blocks, many):
+    """More threads, with fewer registers each, only where 384 do not hold all blocks at once, and not for narrow sources, whose loop is bound elsewhere."""
+    assert helper.f32_many_blocks(width, source, C.c_longlong(blocks)) == many
