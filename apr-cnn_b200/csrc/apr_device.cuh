@@ -214,8 +214,8 @@ int aprnet_small_backward_weights(aprnet_apr* a, int dl, int cin, int cout, int 
                                   float* gw, int accumulate, float* partial, cudaStream_t st);
 // fp32 gather kernel (conv333_f32.cu): blocks of four locations per lane up to which the form with one location per lane, four times as many blocks, is the faster
 // one.  Its time grows with the blocks it puts on an SM.  Time of one location per lane / of four, where it puts 1, 2, 3 and 4 blocks on an SM (up to 37, 74, 111 and 148
-// blocks of four): tiles of 64 result channels, forward pass 0.52, 0.75, 0.88, 1.05 to 1.25, same-level input gradient 0.65, 0.95, 1.26, 1.43, cross-level 0.62, 0.9, 1.16, 1.35; 32
-// channels 0.47, 0.65, 0.77, 1.0 and 0.48, 0.66, 0.81, 1.05; 16 channels 0.5, 0.6, 0.72, 0.85 and 0.6, 0.78, 0.9, 1.08; 8 channels 0.55, 0.61, 0.7, 0.75 and 0.8, 0.9, 1.0, 1.1.
+// blocks of four): tiles of 64 result channels, forward pass 0.6, 0.77, 0.92, 1.1 to 1.25, same-level input gradient 0.65, 0.95, 1.26, 1.43, cross-level 0.62, 0.9, 1.16, 1.35; 32
+// channels, forward pass and same-level input gradient, 0.47, 0.65, 0.77, 1.0 and 0.56, 0.77, 0.97, 1.2; 16 channels 0.5, 0.6, 0.72, 0.85 and 0.6, 0.78, 0.9, 1.08; 8 channels 0.55, 0.61, 0.7, 0.75 and 0.8, 0.9, 1.0, 1.1.
 inline int aprnet_f32_few_blocks(int tile_channels, bool forward) { return 37 * ((tile_channels == 64 ? 2 : 3) + (forward ? 1 : 0)); }
 // Blocks of four locations per lane from which 512 threads per SM are faster than 384 (forward pass of 64 result channels, same-level input gradient of 32): beyond the three blocks per
 // SM that 384 threads hold.  Time with 384 / with 512 threads up to 148, 296 and 444 blocks and beyond 900: 64 channels 0.96, 0.98, 0.98 and 1.01; 32 channels, 32 and more source
